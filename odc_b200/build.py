@@ -22,7 +22,7 @@ NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 CUDA_SOURCES = ["kernels/comm.cu", "kernels/elementwise.cu", "kernels/gemm_tcgen05.cu", "kernels/gemm_tcgen05_2cta.cu", "kernels/attention_tcgen05.cu",
                 "kernels/fused_comm_gemm.cu", "kernels/no_alloc.cu", "kernels/device_prims.cu"]
 CPP_SOURCES = ["heap/symm_heap.cpp", "kernels/tensor_map.cpp"]
-BINDING_SOURCES = ["bindings/bindings.cpp"]
+BINDING_SOURCES = ["bindings/bindings.cpp", "bindings/ops.cpp"]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--use_fast_math",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]
@@ -83,7 +83,7 @@ def build(verbose: bool = False, force: bool = False) -> str:
         src = os.path.join(CSRC, rel)
         flags = cxx_common + [f"-I{p}" for p in inc] + [f"-I{py_inc}", "-DTORCH_EXTENSION_NAME=_C",
                                                       "-DTORCH_API_INCLUDE_EXTENSION_H"]
-        hdrs = "".join(open(os.path.join(CSRC, h)).read() for h in ("kernels/api.h", "heap/symm_heap.h"))
+        hdrs = "".join(open(os.path.join(CSRC, h)).read() for h in ("kernels/api.h", "heap/symm_heap.h", "bindings/ops.h"))
         tag = _digest(src, " ".join(flags) + hashlib.sha1(hdrs.encode()).hexdigest())
         obj = os.path.join(OBJ, os.path.basename(rel) + "." + tag + ".o")
         jobs.append((obj, ["g++"] + flags + ["-c", src, "-o", obj]))

@@ -1,23 +1,13 @@
-// Python bindings: tensors in, raw pointers + current stream out to the launchers in kernels/api.h.
-#include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDAGuard.h>
-#include <torch/extension.h>
+// Python bindings of the heap, the communication primitives and the fused GEMMs: tensors in, raw pointers + current
+// stream out to the launchers in kernels/api.h.  The decoder's differentiable ops are in ops.cpp.
+#include "ops.h"
 
 #include <mutex>
 #include <unordered_map>
 
 #include "../heap/symm_heap.h"
-#include "../kernels/api.h"
-#include "../kernels/tensor_map.h"
 
-namespace py = pybind11;
-using torch::Tensor;
-
-namespace {
-
-void check(cudaError_t e, const char* what) {
-  TORCH_CHECK(e == cudaSuccess, what, ": ", cudaGetErrorString(e));
-}
+namespace odc_bind {
 
 int sm_count() {
   static int n = [] {
@@ -27,17 +17,6 @@ int sm_count() {
     return v > 0 ? v : 148;
   }();
   return n;
-}
-
-cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
-
-int kind_of(at::ScalarType t) {
-  switch (t) {
-    case at::kFloat: return odc::kF32;
-    case at::kBFloat16: return odc::kBF16;
-    case at::kHalf: return odc::kF16;
-    default: TORCH_CHECK(false, "unsupported dtype ", t);
-  }
 }
 
 // Ring of self-resetting completion counters used by scatter_accumulate launches.  A slot is zero again once the
@@ -60,6 +39,21 @@ unsigned int* next_done_slot(int device) {
   unsigned long long s = seq[device]++;
   return reinterpret_cast<unsigned int*>(it->second.data_ptr<int>()) + (s % kDoneSlots);
 }
+
+Tensor& device_status(int device) {
+  static std::mutex mu;
+  static std::unordered_map<int, Tensor> st;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = st.find(device);
+  if (it == st.end()) it = st.emplace(device, torch::zeros({4}, torch::dtype(torch::kInt32).device(torch::kCUDA, device))).first;
+  return it->second;
+}
+
+}  // namespace odc_bind
+
+namespace {
+
+using namespace odc_bind;
 
 // ---------------------------------------------------------------------------------------- heap
 uintptr_t heap_create(int rank, int world, int device, size_t bytes, const std::string& mode,
@@ -194,215 +188,6 @@ void wait_posted(Tensor slots, int64_t nprod, int64_t epoch, Tensor counter, int
         "wait_posted launch");
 }
 
-// ---------------------------------------------------------------------------------------- ops
-std::tuple<Tensor, Tensor> rmsnorm_fwd(Tensor x, Tensor w, double eps) {
-  c10::cuda::CUDAGuard g(x.device());
-  odc::bind_device(x.get_device());
-  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.scalar_type() == at::kBFloat16, "rmsnorm: x must be [T,H] bf16");
-  TORCH_CHECK(w.scalar_type() == at::kBFloat16 && w.is_contiguous(), "rmsnorm: weight must be bf16");
-  auto y = torch::empty_like(x);
-  auto rstd = torch::empty({x.size(0)}, x.options().dtype(at::kFloat));
-  check(odc::launch_rmsnorm_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(),
-                                static_cast<int>(x.size(0)), static_cast<int>(x.size(1)), static_cast<float>(eps),
-                                sm_count(), cur_stream()),
-        "rmsnorm_fwd");
-  return {y, rstd};
-}
-
-std::tuple<Tensor, Tensor> rmsnorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor rstd, bool fixed_order,
-                                       c10::optional<Tensor> dres) {
-  c10::cuda::CUDAGuard g(x.device());
-  odc::bind_device(x.get_device());
-  TORCH_CHECK(dy.is_contiguous() && x.is_contiguous() && dy.sizes() == x.sizes(), "rmsnorm_bwd: contiguous dy, x [T,H]");
-  const int rows = static_cast<int>(x.size(0)), cols = static_cast<int>(x.size(1));
-  auto dx = torch::empty_like(x);
-  const int grid = odc::rmsnorm_bwd_grid(rows, sm_count());
-  auto dw = torch::empty({cols}, x.options().dtype(at::kFloat));
-  Tensor partial;
-  float* partial_ptr = nullptr;
-  if (fixed_order) {  // per-CTA column sums added up in a fixed order by a second pass (bitwise reproducible)
-    partial = torch::empty({grid, cols}, x.options().dtype(at::kFloat));
-    partial_ptr = partial.data_ptr<float>();
-  }
-  const void* dres_ptr = nullptr;
-  if (dres.has_value()) {
-    TORCH_CHECK(dres->is_contiguous() && dres->sizes() == x.sizes() && dres->scalar_type() == at::kBFloat16,
-                "rmsnorm_bwd: residual gradient must be contiguous bf16 of x's shape");
-    dres_ptr = dres->data_ptr();
-  }
-  check(odc::launch_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(),
-                                partial_ptr, dw.data_ptr<float>(), rows, cols, grid, cur_stream(), dres_ptr),
-        "rmsnorm_bwd");
-  return {dx, dw};
-}
-
-Tensor rope_qkv(Tensor qkv, Tensor pos, int n_q, int n_kv, int head_dim, double theta, bool inverse) {
-  c10::cuda::CUDAGuard g(qkv.device());
-  odc::bind_device(qkv.get_device());
-  TORCH_CHECK(qkv.dim() == 2 && qkv.is_contiguous() && qkv.scalar_type() == at::kBFloat16, "rope: qkv [T,W] bf16");
-  TORCH_CHECK(qkv.size(1) == int64_t(n_q + 2 * n_kv) * head_dim, "rope: width mismatch");
-  TORCH_CHECK(pos.scalar_type() == at::kLong && pos.numel() == qkv.size(0), "rope: position_ids int64 [T]");
-  auto out = torch::empty_like(qkv);
-  check(odc::launch_rope_qkv(qkv.data_ptr(), out.data_ptr(), reinterpret_cast<const long long*>(pos.data_ptr<int64_t>()),
-                             static_cast<int>(qkv.size(0)), n_q, n_kv, head_dim, static_cast<float>(theta), inverse,
-                             cur_stream()),
-        "rope_qkv");
-  return out;
-}
-
-Tensor swiglu_fwd(Tensor gu) {
-  c10::cuda::CUDAGuard g(gu.device());
-  odc::bind_device(gu.get_device());
-  TORCH_CHECK(gu.is_contiguous() && gu.scalar_type() == at::kBFloat16, "swiglu: bf16 contiguous");
-  const int f = static_cast<int>(gu.size(-1) / 2);
-  auto sizes = gu.sizes().vec();
-  sizes.back() = f;
-  auto out = torch::empty(sizes, gu.options());
-  check(odc::launch_swiglu_fwd(gu.data_ptr(), out.data_ptr(), gu.numel() / (2 * f), f, sm_count(), cur_stream()),
-        "swiglu_fwd");
-  return out;
-}
-
-Tensor swiglu_bwd(Tensor dy, Tensor gu) {
-  c10::cuda::CUDAGuard g(gu.device());
-  odc::bind_device(gu.get_device());
-  const int f = static_cast<int>(gu.size(-1) / 2);
-  auto out = torch::empty_like(gu);
-  check(odc::launch_swiglu_bwd(dy.data_ptr(), gu.data_ptr(), out.data_ptr(), gu.numel() / (2 * f), f, sm_count(),
-                               cur_stream()),
-        "swiglu_bwd");
-  return out;
-}
-
-void ce_fwd_bwd(Tensor logits, Tensor labels, c10::optional<Tensor> loss_scale, Tensor loss, int64_t ignore_index) {
-  c10::cuda::CUDAGuard g(logits.device());
-  odc::bind_device(logits.get_device());
-  TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous() && logits.scalar_type() == at::kBFloat16, "ce: logits bf16");
-  TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous(), "ce: labels int64");
-  const float* ls = nullptr;
-  if (loss_scale.has_value()) {
-    TORCH_CHECK(loss_scale->scalar_type() == at::kFloat && loss_scale->is_contiguous(), "ce: loss_scale fp32");
-    ls = loss_scale->data_ptr<float>();
-  }
-  check(odc::launch_ce_fwd_bwd(logits.data_ptr(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()), ls,
-                               loss.data_ptr<float>(), static_cast<int>(logits.size(0)),
-                               static_cast<int>(logits.size(1)), ignore_index, cur_stream()),
-        "ce_fwd_bwd");
-}
-
-void token_logprobs(Tensor logits, Tensor labels, Tensor out, int64_t ignore_index) {
-  c10::cuda::CUDAGuard g(logits.device());
-  odc::bind_device(logits.get_device());
-  TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous() && logits.scalar_type() == at::kBFloat16, "token_logprobs: logits bf16");
-  TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous() && labels.numel() == logits.size(0),
-              "token_logprobs: one int64 label per row");
-  TORCH_CHECK(out.scalar_type() == at::kFloat && out.is_contiguous() && out.numel() == logits.size(0) && out.is_cuda(),
-              "token_logprobs: one fp32 output per row");
-  check(odc::launch_token_logprobs(logits.data_ptr(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()),
-                                   out.data_ptr<float>(), static_cast<int>(logits.size(0)),
-                                   static_cast<int>(logits.size(1)), ignore_index, cur_stream()),
-        "token_logprobs");
-}
-
-void adamw_step(Tensor p, Tensor g, Tensor m, Tensor v, c10::optional<Tensor> p_lowp, double lr, double beta1,
-                double beta2, double eps, double wd, int64_t step, double grad_scale) {
-  c10::cuda::CUDAGuard guard(p.device());
-  odc::bind_device(p.get_device());
-  TORCH_CHECK(p.scalar_type() == at::kFloat && m.scalar_type() == at::kFloat && v.scalar_type() == at::kFloat,
-              "adamw: fp32 master state");
-  TORCH_CHECK(p.is_contiguous() && g.is_contiguous() && m.is_contiguous() && v.is_contiguous(), "adamw: contiguous");
-  void* lp = nullptr;
-  if (p_lowp.has_value()) {
-    TORCH_CHECK(p_lowp->scalar_type() == at::kBFloat16 && p_lowp->numel() == p.numel(), "adamw: bf16 replica");
-    lp = p_lowp->data_ptr();
-  }
-  const float bc1 = 1.f - std::pow(static_cast<float>(beta1), static_cast<float>(step));
-  const float bc2 = 1.f - std::pow(static_cast<float>(beta2), static_cast<float>(step));
-  check(odc::launch_adamw(p.data_ptr<float>(), g.data_ptr(), kind_of(g.scalar_type()), m.data_ptr<float>(),
-                          v.data_ptr<float>(), lp, static_cast<size_t>(p.numel()), static_cast<float>(lr),
-                          static_cast<float>(beta1), static_cast<float>(beta2), static_cast<float>(eps),
-                          static_cast<float>(wd), bc1, bc2, static_cast<float>(grad_scale), sm_count(), cur_stream()),
-        "adamw");
-}
-
-void cast_f32_to_bf16(Tensor in, Tensor out) {
-  c10::cuda::CUDAGuard g(in.device());
-  odc::bind_device(in.get_device());
-  TORCH_CHECK(in.scalar_type() == at::kFloat && out.scalar_type() == at::kBFloat16 && in.numel() == out.numel() &&
-                  in.is_contiguous() && out.is_contiguous(), "cast: fp32 -> bf16, same numel, contiguous");
-  check(odc::launch_cast_f32_to_bf16(in.data_ptr<float>(), out.data_ptr(), static_cast<size_t>(in.numel()), sm_count(),
-                                     cur_stream()),
-        "cast");
-}
-
-void sumsq(Tensor x, Tensor out) {
-  c10::cuda::CUDAGuard g(x.device());
-  odc::bind_device(x.get_device());
-  TORCH_CHECK(x.is_contiguous() && out.scalar_type() == at::kFloat, "sumsq: contiguous input, fp32 output");
-  check(odc::launch_sumsq(x.data_ptr(), kind_of(x.scalar_type()), static_cast<size_t>(x.numel()), out.data_ptr<float>(),
-                          sm_count(), cur_stream()),
-        "sumsq");
-}
-
-Tensor& gemm_status(int device) {
-  static std::mutex mu;
-  static std::unordered_map<int, Tensor> st;
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = st.find(device);
-  if (it == st.end()) it = st.emplace(device, torch::zeros({4}, torch::dtype(torch::kInt32).device(torch::kCUDA, device))).first;
-  return it->second;
-}
-
-Tensor kernel_status() {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  return gemm_status(dev);
-}
-
-void gemm(Tensor a, Tensor b, Tensor c, const std::string& layout, c10::optional<Tensor> bias, bool accumulate,
-          c10::optional<Tensor> residual, int pair) {
-  c10::cuda::CUDAGuard g(a.device());
-  odc::bind_device(a.get_device());
-  TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && c.dim() == 2, "gemm: 2-D operands");
-  TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "gemm: bf16 inputs");
-  TORCH_CHECK(a.stride(1) == 1 && b.stride(1) == 1 && c.stride(1) == 1, "gemm: innermost stride must be 1");
-  int lay, M, N, K;
-  if (layout == "nt") {
-    lay = 0; M = a.size(0); K = a.size(1); N = b.size(0);
-    TORCH_CHECK(b.size(1) == K, "gemm nt: K mismatch");
-  } else if (layout == "nn") {
-    lay = 1; M = a.size(0); K = a.size(1); N = b.size(1);
-    TORCH_CHECK(b.size(0) == K, "gemm nn: K mismatch");
-  } else if (layout == "tn") {
-    lay = 2; K = a.size(0); M = a.size(1); N = b.size(1);
-    TORCH_CHECK(b.size(0) == K, "gemm tn: K mismatch");
-  } else {
-    TORCH_CHECK(false, "gemm: unknown layout ", layout);
-  }
-  TORCH_CHECK(c.size(0) == M && c.size(1) == N, "gemm: output shape mismatch");
-  const void* bias_ptr = nullptr;
-  if (bias.has_value()) {
-    TORCH_CHECK(bias->scalar_type() == at::kBFloat16 && bias->numel() == N && bias->is_contiguous(), "gemm: bias bf16 [N]");
-    bias_ptr = bias->data_ptr();
-  }
-  const void* res_ptr = nullptr;
-  long long ldr = 0;
-  if (residual.has_value()) {
-    TORCH_CHECK(residual->scalar_type() == at::kBFloat16 && residual->dim() == 2 && residual->size(0) == M &&
-                    residual->size(1) == N && residual->stride(1) == 1, "gemm: residual bf16 [M,N]");
-    res_ptr = residual->data_ptr();
-    ldr = residual->stride(0);
-  }
-  cudaError_t e = odc::gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), kind_of(c.scalar_type()), bias_ptr, M, N, K,
-                                 lay, accumulate, a.stride(0), b.stride(0), c.stride(0),
-                                 gemm_status(a.get_device()).data_ptr<int>(), sm_count(), cur_stream(), res_ptr, ldr,
-                                 pair);
-  TORCH_CHECK(e == cudaSuccess, "gemm(", layout, ") M=", M, " N=", N, " K=", K, " lda=", a.stride(0), " ldb=", b.stride(0),
-              " ldc=", c.stride(0), " align(a,b,c)=", reinterpret_cast<uintptr_t>(a.data_ptr()) % 16, ",",
-              reinterpret_cast<uintptr_t>(b.data_ptr()) % 16, ",", reinterpret_cast<uintptr_t>(c.data_ptr()) % 16, ": ",
-              cudaGetErrorString(e));
-}
-
 void gemm_wgrad_scatter(Tensor dy, Tensor x, Tensor acc_table, Tensor ctr_table, int64_t acc_offset,
                         int64_t rows_per_rank, double scale) {
   c10::cuda::CUDAGuard g(dy.device());
@@ -415,7 +200,7 @@ void gemm_wgrad_scatter(Tensor dy, Tensor x, Tensor acc_table, Tensor ctr_table,
                                 reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()), acc_offset,
                                 static_cast<int>(rows_per_rank), static_cast<int>(acc_table.numel()),
                                 static_cast<float>(scale), next_done_slot(dy.get_device()),
-                                gemm_status(dy.get_device()).data_ptr<int>(), sm_count(), cur_stream()),
+                                device_status(dy.get_device()).data_ptr<int>(), sm_count(), cur_stream()),
         "gemm_wgrad_scatter");
 }
 
@@ -431,7 +216,7 @@ bool gemm_wgrad_scatter_tma(Tensor dy, Tensor x, std::vector<int64_t> acc_addrs,
       dy.data_ptr(), x.data_ptr(), dy.size(0), dy.size(1), x.size(1), dy.stride(0), x.stride(0), addrs.data(),
       reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()), acc_offset, static_cast<int>(rows_per_rank),
       static_cast<int>(addrs.size()), static_cast<float>(scale), next_done_slot(dy.get_device()),
-      gemm_status(dy.get_device()).data_ptr<int>(), sm_count(), cur_stream(), start_rank);
+      device_status(dy.get_device()).data_ptr<int>(), sm_count(), cur_stream(), start_rank);
   if (e == cudaErrorNotSupported) return false;  // shape not eligible: the caller uses the red.add variant
   check(e, "gemm_wgrad_scatter_tma");
   return true;
@@ -464,7 +249,7 @@ Tensor gemm_gather(Tensor x, Tensor shard_table, Tensor w_local, c10::optional<T
                             w_local.data_ptr(), y.data_ptr(), bias_ptr, M, N, K, x.stride(0), y.stride(0),
                             static_cast<int>(rows_per_rank), static_cast<int>(shard_table.numel()), start_rank,
                             reinterpret_cast<unsigned int*>(flags.data_ptr<int>()),
-                            gemm_status(x.get_device()).data_ptr<int>(), sm_count(), cur_stream(), res_ptr, ldr),
+                            device_status(x.get_device()).data_ptr<int>(), sm_count(), cur_stream(), res_ptr, ldr),
         "gemm_gather");
   return y;
 }
@@ -483,64 +268,9 @@ Tensor gemm_gather_dgrad(Tensor dy, Tensor shard_table, Tensor w_local, int64_t 
                             w_local.data_ptr(), dx.data_ptr(), M, N, K, dy.stride(0), dx.stride(0),
                             static_cast<int>(rows_per_rank), static_cast<int>(shard_table.numel()),
                             reinterpret_cast<unsigned int*>(flags.data_ptr<int>()),
-                            gemm_status(dy.get_device()).data_ptr<int>(), sm_count(), cur_stream(), start_rank),
+                            device_status(dy.get_device()).data_ptr<int>(), sm_count(), cur_stream(), start_rank),
         "gemm_gather_dgrad");
   return dx;
-}
-
-std::tuple<Tensor, Tensor> attn_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens, int max_seqlen, bool causal,
-                                    double scale) {
-  c10::cuda::CUDAGuard g(q.device());
-  odc::bind_device(q.get_device());
-  TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && v.dim() == 3, "attention: q/k/v are [T, H, D]");
-  TORCH_CHECK(q.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16,
-              "attention: bf16 inputs");
-  const int T = q.size(0), hq = q.size(1), d = q.size(2), hkv = k.size(1);
-  TORCH_CHECK(q.stride(2) == 1 && q.stride(1) == d && k.stride(2) == 1 && k.stride(1) == d && v.stride(2) == 1 &&
-                  v.stride(1) == d, "attention: heads must be packed within a token");
-  TORCH_CHECK(k.stride(0) == v.stride(0), "attention: k and v must share a row stride");
-  TORCH_CHECK(cu_seqlens.scalar_type() == at::kInt && cu_seqlens.is_contiguous(), "attention: cu_seqlens int32");
-  auto o = torch::empty({T, hq, d}, q.options());
-  auto lse = torch::empty({hq, T}, q.options().dtype(at::kFloat));
-  check(odc::attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
-                      cu_seqlens.data_ptr<int>(), static_cast<int>(cu_seqlens.numel() - 1), T, max_seqlen, hq, hkv, d,
-                      q.stride(0), k.stride(0), o.stride(0), static_cast<float>(scale), causal,
-                      gemm_status(q.get_device()).data_ptr<int>(), sm_count(), cur_stream()),
-        "attn_fwd");
-  return {o, lse};
-}
-
-std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse,
-                                                    Tensor cu_seqlens, int max_seqlen, bool causal, double scale,
-                                                    bool fused_qkv) {
-  c10::cuda::CUDAGuard g(q.device());
-  odc::bind_device(q.get_device());
-  const int T = q.size(0), hq = q.size(1), d = q.size(2), hkv = k.size(1);
-  TORCH_CHECK(dout.is_contiguous() && dout.scalar_type() == at::kBFloat16, "attention bwd: dout contiguous bf16");
-  TORCH_CHECK(o.stride(2) == 1 && o.stride(1) == d, "attention bwd: o heads packed");
-  TORCH_CHECK(q.stride(2) == 1 && q.stride(1) == d && k.stride(2) == 1 && k.stride(1) == d && v.stride(2) == 1 &&
-                  v.stride(1) == d && k.stride(0) == v.stride(0), "attention bwd: q/k/v layout");
-  Tensor dq, dk, dv, dqkv;
-  if (fused_qkv) {
-    // one [T, (hq + 2 hkv) d] gradient; dq/dk/dv are column views of it, so slicing costs nothing in autograd
-    dqkv = torch::empty({T, int64_t(hq + 2 * hkv) * d}, q.options());
-    dq = dqkv.narrow(1, 0, int64_t(hq) * d).view({T, hq, d});
-    dk = dqkv.narrow(1, int64_t(hq) * d, int64_t(hkv) * d).view({T, hkv, d});
-    dv = dqkv.narrow(1, int64_t(hq + hkv) * d, int64_t(hkv) * d).view({T, hkv, d});
-  } else {
-    dq = torch::empty({T, hq, d}, q.options());
-    dk = torch::empty({T, hkv, d}, q.options());
-    dv = torch::empty({T, hkv, d}, q.options());
-  }
-  auto delta = torch::empty({hq, T}, q.options().dtype(at::kFloat));
-  auto dq_acc = torch::empty({T, hq, d}, q.options().dtype(at::kFloat));
-  check(odc::attn_bwd(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
-                      dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), dq_acc.data_ptr<float>(),
-                      cu_seqlens.data_ptr<int>(), static_cast<int>(cu_seqlens.numel() - 1), T, max_seqlen, hq, hkv, d,
-                      q.stride(0), k.stride(0), o.stride(0), dq.stride(0), dk.stride(0), static_cast<float>(scale),
-                      causal, gemm_status(q.get_device()).data_ptr<int>(), sm_count(), cur_stream()),
-        "attn_bwd");
-  return {dq, dk, dv, fused_qkv ? dqkv : dq};  // 4th: the fused gradient when requested
 }
 
 // --- single-primitive test entry points: addresses are plain integers so peers' mappings can be passed
@@ -604,19 +334,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("wait_counter", &wait_counter);
   m.def("post_counts", &post_counts);
   m.def("wait_posted", &wait_posted);
-  m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("dy"), py::arg("x"), py::arg("w"), py::arg("rstd"),
-        py::arg("fixed_order") = false, py::arg("dres") = py::none());
-  m.def("rope_qkv", &rope_qkv);
-  m.def("swiglu_fwd", &swiglu_fwd);
-  m.def("swiglu_bwd", &swiglu_bwd);
-  m.def("ce_fwd_bwd", &ce_fwd_bwd);
-  m.def("token_logprobs", &token_logprobs);
-  m.def("adamw_step", &adamw_step);
-  m.def("cast_f32_to_bf16", &cast_f32_to_bf16);
-  m.def("sumsq", &sumsq);
-  m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("c"), py::arg("layout"), py::arg("bias"),
-        py::arg("accumulate"), py::arg("residual") = py::none(), py::arg("pair") = -1);
   m.def("put_block", &put_block);
   m.def("get_block", &get_block);
   m.def("scalar_put_get", &scalar_put_get);
@@ -629,8 +346,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("rows_per_rank"), py::arg("start_rank"), py::arg("residual") = py::none());
   m.def("gemm_gather_dgrad", &gemm_gather_dgrad, py::arg("dy"), py::arg("shard_table"), py::arg("w_local"),
         py::arg("rows_per_rank"), py::arg("start_rank") = 0);
-  m.def("attn_fwd", &attn_fwd);
-  m.def("attn_bwd", &attn_bwd);
-  m.def("kernel_status", &kernel_status);
   m.def("sm_count", &sm_count);
+  register_ops(m);
 }

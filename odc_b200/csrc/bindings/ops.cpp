@@ -1,0 +1,640 @@
+// The decoder's ops: raw kernel entry points, and their differentiable forms as native autograd functions.
+//
+// A training step of a small model is bound by the host: a Python autograd function costs 15-25 us per direction, the
+// kernels behind it 3-10 us.  The native functions cost 3-5 us per direction and run their backward without the
+// interpreter lock (packed 2-layer, 512-wide decoder, two microbatches: see the figures at the Python wrappers).
+#include "ops.h"
+
+#include <torch/csrc/autograd/custom_function.h>
+
+#include <atomic>
+#include <cstdlib>
+#include <cstring>
+
+namespace odc_bind {
+namespace {
+
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+
+constexpr const char* kLayoutNames[3] = {"nt", "nn", "tn"};
+
+// kernels of this package launched by the ops so far (benchmark accounting)
+std::atomic<long long> g_launches{0};
+void count(int n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+
+std::tuple<Tensor, Tensor> rmsnorm_fwd(Tensor x, Tensor w, double eps) {
+  c10::cuda::CUDAGuard g(x.device());
+  odc::bind_device(x.get_device());
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.scalar_type() == at::kBFloat16, "rmsnorm: x must be [T,H] bf16");
+  TORCH_CHECK(w.scalar_type() == at::kBFloat16 && w.is_contiguous(), "rmsnorm: weight must be bf16");
+  auto y = at::empty_like(x);
+  auto rstd = at::empty({x.size(0)}, x.options().dtype(at::kFloat));
+  check(odc::launch_rmsnorm_fwd(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(),
+                                static_cast<int>(x.size(0)), static_cast<int>(x.size(1)), static_cast<float>(eps),
+                                sm_count(), cur_stream()),
+        "rmsnorm_fwd");
+  return {y, rstd};
+}
+
+std::tuple<Tensor, Tensor> rmsnorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor rstd, bool fixed_order,
+                                       c10::optional<Tensor> dres) {
+  c10::cuda::CUDAGuard g(x.device());
+  odc::bind_device(x.get_device());
+  TORCH_CHECK(dy.is_contiguous() && x.is_contiguous() && dy.sizes() == x.sizes(), "rmsnorm_bwd: contiguous dy, x [T,H]");
+  const int rows = static_cast<int>(x.size(0)), cols = static_cast<int>(x.size(1));
+  auto dx = at::empty_like(x);
+  const int grid = odc::rmsnorm_bwd_grid(rows, sm_count());
+  auto dw = at::empty({cols}, x.options().dtype(at::kFloat));
+  Tensor partial;
+  float* partial_ptr = nullptr;
+  if (fixed_order) {  // per-CTA column sums added up in a fixed order by a second pass (bitwise reproducible)
+    partial = at::empty({grid, cols}, x.options().dtype(at::kFloat));
+    partial_ptr = partial.data_ptr<float>();
+  }
+  const void* dres_ptr = nullptr;
+  if (dres.has_value()) {
+    TORCH_CHECK(dres->is_contiguous() && dres->sizes() == x.sizes() && dres->scalar_type() == at::kBFloat16,
+                "rmsnorm_bwd: residual gradient must be contiguous bf16 of x's shape");
+    dres_ptr = dres->data_ptr();
+  }
+  check(odc::launch_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(),
+                                partial_ptr, dw.data_ptr<float>(), rows, cols, grid, cur_stream(), dres_ptr),
+        "rmsnorm_bwd");
+  return {dx, dw};
+}
+
+Tensor rope_qkv(Tensor qkv, Tensor pos, int n_q, int n_kv, int head_dim, double theta, bool inverse) {
+  c10::cuda::CUDAGuard g(qkv.device());
+  odc::bind_device(qkv.get_device());
+  TORCH_CHECK(qkv.dim() == 2 && qkv.is_contiguous() && qkv.scalar_type() == at::kBFloat16, "rope: qkv [T,W] bf16");
+  TORCH_CHECK(qkv.size(1) == int64_t(n_q + 2 * n_kv) * head_dim, "rope: width mismatch");
+  TORCH_CHECK(pos.scalar_type() == at::kLong && pos.numel() == qkv.size(0), "rope: position_ids int64 [T]");
+  auto out = at::empty_like(qkv);
+  check(odc::launch_rope_qkv(qkv.data_ptr(), out.data_ptr(), reinterpret_cast<const long long*>(pos.data_ptr<int64_t>()),
+                             static_cast<int>(qkv.size(0)), n_q, n_kv, head_dim, static_cast<float>(theta), inverse,
+                             cur_stream()),
+        "rope_qkv");
+  return out;
+}
+
+Tensor swiglu_fwd(Tensor gu) {
+  c10::cuda::CUDAGuard g(gu.device());
+  odc::bind_device(gu.get_device());
+  TORCH_CHECK(gu.is_contiguous() && gu.scalar_type() == at::kBFloat16, "swiglu: bf16 contiguous");
+  const int f = static_cast<int>(gu.size(-1) / 2);
+  auto sizes = gu.sizes().vec();
+  sizes.back() = f;
+  auto out = at::empty(sizes, gu.options());
+  check(odc::launch_swiglu_fwd(gu.data_ptr(), out.data_ptr(), gu.numel() / (2 * f), f, sm_count(), cur_stream()),
+        "swiglu_fwd");
+  return out;
+}
+
+Tensor swiglu_bwd(Tensor dy, Tensor gu) {
+  c10::cuda::CUDAGuard g(gu.device());
+  odc::bind_device(gu.get_device());
+  const int f = static_cast<int>(gu.size(-1) / 2);
+  auto out = at::empty_like(gu);
+  check(odc::launch_swiglu_bwd(dy.data_ptr(), gu.data_ptr(), out.data_ptr(), gu.numel() / (2 * f), f, sm_count(),
+                               cur_stream()),
+        "swiglu_bwd");
+  return out;
+}
+
+void ce_fwd_bwd(Tensor logits, Tensor labels, c10::optional<Tensor> loss_scale, Tensor loss, int64_t ignore_index) {
+  c10::cuda::CUDAGuard g(logits.device());
+  odc::bind_device(logits.get_device());
+  TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous() && logits.scalar_type() == at::kBFloat16, "ce: logits bf16");
+  TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous(), "ce: labels int64");
+  const float* ls = nullptr;
+  if (loss_scale.has_value()) {
+    TORCH_CHECK(loss_scale->scalar_type() == at::kFloat && loss_scale->is_contiguous(), "ce: loss_scale fp32");
+    ls = loss_scale->data_ptr<float>();
+  }
+  check(odc::launch_ce_fwd_bwd(logits.data_ptr(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()), ls,
+                               loss.data_ptr<float>(), static_cast<int>(logits.size(0)),
+                               static_cast<int>(logits.size(1)), ignore_index, cur_stream()),
+        "ce_fwd_bwd");
+}
+
+void token_logprobs(Tensor logits, Tensor labels, Tensor out, int64_t ignore_index) {
+  c10::cuda::CUDAGuard g(logits.device());
+  odc::bind_device(logits.get_device());
+  TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous() && logits.scalar_type() == at::kBFloat16, "token_logprobs: logits bf16");
+  TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous() && labels.numel() == logits.size(0),
+              "token_logprobs: one int64 label per row");
+  TORCH_CHECK(out.scalar_type() == at::kFloat && out.is_contiguous() && out.numel() == logits.size(0) && out.is_cuda(),
+              "token_logprobs: one fp32 output per row");
+  check(odc::launch_token_logprobs(logits.data_ptr(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()),
+                                   out.data_ptr<float>(), static_cast<int>(logits.size(0)),
+                                   static_cast<int>(logits.size(1)), ignore_index, cur_stream()),
+        "token_logprobs");
+}
+
+void adamw_step(Tensor p, Tensor g, Tensor m, Tensor v, c10::optional<Tensor> p_lowp, double lr, double beta1,
+                double beta2, double eps, double wd, int64_t step, double grad_scale) {
+  c10::cuda::CUDAGuard guard(p.device());
+  odc::bind_device(p.get_device());
+  TORCH_CHECK(p.scalar_type() == at::kFloat && m.scalar_type() == at::kFloat && v.scalar_type() == at::kFloat,
+              "adamw: fp32 master state");
+  TORCH_CHECK(p.is_contiguous() && g.is_contiguous() && m.is_contiguous() && v.is_contiguous(), "adamw: contiguous");
+  void* lp = nullptr;
+  if (p_lowp.has_value()) {
+    TORCH_CHECK(p_lowp->scalar_type() == at::kBFloat16 && p_lowp->numel() == p.numel(), "adamw: bf16 replica");
+    lp = p_lowp->data_ptr();
+  }
+  const float bc1 = 1.f - std::pow(static_cast<float>(beta1), static_cast<float>(step));
+  const float bc2 = 1.f - std::pow(static_cast<float>(beta2), static_cast<float>(step));
+  check(odc::launch_adamw(p.data_ptr<float>(), g.data_ptr(), kind_of(g.scalar_type()), m.data_ptr<float>(),
+                          v.data_ptr<float>(), lp, static_cast<size_t>(p.numel()), static_cast<float>(lr),
+                          static_cast<float>(beta1), static_cast<float>(beta2), static_cast<float>(eps),
+                          static_cast<float>(wd), bc1, bc2, static_cast<float>(grad_scale), sm_count(), cur_stream()),
+        "adamw");
+}
+
+void cast_f32_to_bf16(Tensor in, Tensor out) {
+  c10::cuda::CUDAGuard g(in.device());
+  odc::bind_device(in.get_device());
+  TORCH_CHECK(in.scalar_type() == at::kFloat && out.scalar_type() == at::kBFloat16 && in.numel() == out.numel() &&
+                  in.is_contiguous() && out.is_contiguous(), "cast: fp32 -> bf16, same numel, contiguous");
+  check(odc::launch_cast_f32_to_bf16(in.data_ptr<float>(), out.data_ptr(), static_cast<size_t>(in.numel()), sm_count(),
+                                     cur_stream()),
+        "cast");
+}
+
+void sumsq(Tensor x, Tensor out) {
+  c10::cuda::CUDAGuard g(x.device());
+  odc::bind_device(x.get_device());
+  TORCH_CHECK(x.is_contiguous() && out.scalar_type() == at::kFloat, "sumsq: contiguous input, fp32 output");
+  check(odc::launch_sumsq(x.data_ptr(), kind_of(x.scalar_type()), static_cast<size_t>(x.numel()), out.data_ptr<float>(),
+                          sm_count(), cur_stream()),
+        "sumsq");
+}
+
+Tensor kernel_status() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return device_status(dev);
+}
+
+// ODC_GEMM=cublas: library products, to measure the hand-written kernels against (read at every call)
+bool library_gemm() {
+  const char* e = std::getenv("ODC_GEMM");
+  return e != nullptr && std::strcmp(e, "cublas") == 0;
+}
+
+enum Layout : int { kNT = 0, kNN = 1, kTN = 2 };  // C = A B^T (forward), A B (input gradient), A^T B (weight gradient)
+
+void gemm_into(const Tensor& a, const Tensor& b, const Tensor& c, int lay, const Tensor& bias = {}, bool accumulate = false,
+               const Tensor& residual = {}, int pair = -1) {
+  c10::cuda::CUDAGuard g(a.device());
+  odc::bind_device(a.get_device());
+  TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && c.dim() == 2, "gemm: 2-D operands");
+  TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16, "gemm: bf16 inputs");
+  TORCH_CHECK(a.stride(1) == 1 && b.stride(1) == 1 && c.stride(1) == 1, "gemm: innermost stride must be 1");
+  const int K = lay == kTN ? a.size(0) : a.size(1), M = lay == kTN ? a.size(1) : a.size(0);
+  const int N = lay == kNT ? b.size(0) : b.size(1);
+  TORCH_CHECK((lay == kNT ? b.size(1) : b.size(0)) == K, "gemm ", kLayoutNames[lay], ": K mismatch");
+  TORCH_CHECK(c.size(0) == M && c.size(1) == N, "gemm: output shape mismatch");
+  const void* bias_ptr = nullptr;
+  if (bias.defined()) {
+    TORCH_CHECK(bias.scalar_type() == at::kBFloat16 && bias.numel() == N && bias.is_contiguous(), "gemm: bias bf16 [N]");
+    bias_ptr = bias.data_ptr();
+  }
+  const void* res_ptr = nullptr;
+  long long ldr = 0;
+  if (residual.defined()) {
+    TORCH_CHECK(residual.scalar_type() == at::kBFloat16 && residual.dim() == 2 && residual.size(0) == M &&
+                    residual.size(1) == N && residual.stride(1) == 1, "gemm: residual bf16 [M,N]");
+    res_ptr = residual.data_ptr();
+    ldr = residual.stride(0);
+  }
+  cudaError_t e = odc::gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), kind_of(c.scalar_type()), bias_ptr, M, N, K,
+                                 lay, accumulate, a.stride(0), b.stride(0), c.stride(0),
+                                 device_status(a.get_device()).data_ptr<int>(), sm_count(), cur_stream(), res_ptr, ldr,
+                                 pair);
+  TORCH_CHECK(e == cudaSuccess, "gemm(", kLayoutNames[lay], ") M=", M, " N=", N, " K=", K, " lda=", a.stride(0), " ldb=",
+              b.stride(0), " ldc=", c.stride(0), " align(a,b,c)=", reinterpret_cast<uintptr_t>(a.data_ptr()) % 16, ",",
+              reinterpret_cast<uintptr_t>(b.data_ptr()) % 16, ",", reinterpret_cast<uintptr_t>(c.data_ptr()) % 16, ": ",
+              cudaGetErrorString(e));
+}
+
+void gemm(Tensor a, Tensor b, Tensor c, const std::string& layout, c10::optional<Tensor> bias, bool accumulate,
+          c10::optional<Tensor> residual, int pair) {
+  int lay = 0;
+  while (lay < 3 && layout != kLayoutNames[lay]) ++lay;
+  TORCH_CHECK(lay < 3, "gemm: unknown layout ", layout);
+  gemm_into(a, b, c, lay, bias.value_or(Tensor()), accumulate, residual.value_or(Tensor()), pair);
+}
+
+// the product the ops use: own kernel, or the library when asked for
+void product_into(const Tensor& a, const Tensor& b, const Tensor& c, int lay, const Tensor& bias = {}, bool accumulate = false,
+                  const Tensor& residual = {}) {
+  if (library_gemm()) {
+    Tensor r = at::matmul(lay == kTN ? a.t() : a, lay == kNT ? b.t() : b);
+    if (bias.defined()) r = r + bias;
+    if (residual.defined()) r = r + residual;
+    if (accumulate) c.add_(r.to(c.scalar_type())); else c.copy_(r);
+    return;
+  }
+  gemm_into(a, b, c, lay, bias, accumulate, residual);
+  count();
+}
+Tensor product(const Tensor& a, const Tensor& b, int lay, const Tensor& bias = {}, const Tensor& residual = {},
+               c10::optional<at::ScalarType> dtype = c10::nullopt) {
+  auto c = at::empty({lay == kTN ? a.size(1) : a.size(0), lay == kNT ? b.size(0) : b.size(1)},
+                     dtype ? a.options().dtype(*dtype) : a.options());
+  product_into(a, b, c, lay, bias, false, residual);
+  return c;
+}
+
+std::tuple<Tensor, Tensor> attn_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens, int max_seqlen, bool causal,
+                                    double scale) {
+  c10::cuda::CUDAGuard g(q.device());
+  odc::bind_device(q.get_device());
+  TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && v.dim() == 3, "attention: q/k/v are [T, H, D]");
+  TORCH_CHECK(q.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16,
+              "attention: bf16 inputs");
+  const int T = q.size(0), hq = q.size(1), d = q.size(2), hkv = k.size(1);
+  TORCH_CHECK(q.stride(2) == 1 && q.stride(1) == d && k.stride(2) == 1 && k.stride(1) == d && v.stride(2) == 1 &&
+                  v.stride(1) == d, "attention: heads must be packed within a token");
+  TORCH_CHECK(k.stride(0) == v.stride(0), "attention: k and v must share a row stride");
+  TORCH_CHECK(cu_seqlens.scalar_type() == at::kInt && cu_seqlens.is_contiguous(), "attention: cu_seqlens int32");
+  auto o = at::empty({T, hq, d}, q.options());
+  auto lse = at::empty({hq, T}, q.options().dtype(at::kFloat));
+  check(odc::attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
+                      cu_seqlens.data_ptr<int>(), static_cast<int>(cu_seqlens.numel() - 1), T, max_seqlen, hq, hkv, d,
+                      q.stride(0), k.stride(0), o.stride(0), static_cast<float>(scale), causal,
+                      device_status(q.get_device()).data_ptr<int>(), sm_count(), cur_stream()),
+        "attn_fwd");
+  return {o, lse};
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse,
+                                                    Tensor cu_seqlens, int max_seqlen, bool causal, double scale,
+                                                    bool fused_qkv) {
+  c10::cuda::CUDAGuard g(q.device());
+  odc::bind_device(q.get_device());
+  const int T = q.size(0), hq = q.size(1), d = q.size(2), hkv = k.size(1);
+  TORCH_CHECK(dout.is_contiguous() && dout.scalar_type() == at::kBFloat16, "attention bwd: dout contiguous bf16");
+  TORCH_CHECK(o.stride(2) == 1 && o.stride(1) == d, "attention bwd: o heads packed");
+  TORCH_CHECK(q.stride(2) == 1 && q.stride(1) == d && k.stride(2) == 1 && k.stride(1) == d && v.stride(2) == 1 &&
+                  v.stride(1) == d && k.stride(0) == v.stride(0), "attention bwd: q/k/v layout");
+  Tensor dq, dk, dv, dqkv;
+  if (fused_qkv) {
+    // one [T, (hq + 2 hkv) d] gradient; dq/dk/dv are column views of it, so slicing costs nothing in autograd
+    dqkv = at::empty({T, int64_t(hq + 2 * hkv) * d}, q.options());
+    dq = dqkv.narrow(1, 0, int64_t(hq) * d).view({T, hq, d});
+    dk = dqkv.narrow(1, int64_t(hq) * d, int64_t(hkv) * d).view({T, hkv, d});
+    dv = dqkv.narrow(1, int64_t(hq + hkv) * d, int64_t(hkv) * d).view({T, hkv, d});
+  } else {
+    dq = at::empty({T, hq, d}, q.options());
+    dk = at::empty({T, hkv, d}, q.options());
+    dv = at::empty({T, hkv, d}, q.options());
+  }
+  auto delta = at::empty({hq, T}, q.options().dtype(at::kFloat));
+  auto dq_acc = at::empty({T, hq, d}, q.options().dtype(at::kFloat));
+  check(odc::attn_bwd(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
+                      dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), dq_acc.data_ptr<float>(),
+                      cu_seqlens.data_ptr<int>(), static_cast<int>(cu_seqlens.numel() - 1), T, max_seqlen, hq, hkv, d,
+                      q.stride(0), k.stride(0), o.stride(0), dq.stride(0), dk.stride(0), static_cast<float>(scale),
+                      causal, device_status(q.get_device()).data_ptr<int>(), sm_count(), cur_stream()),
+        "attn_bwd");
+  return {dq, dk, dv, fused_qkv ? dqkv : dq};  // 4th: the fused gradient when requested
+}
+
+// ------------------------------------------------------------------------------------------------ differentiable ops
+bool env_on(const char* name) {
+  const char* e = std::getenv(name);
+  return e != nullptr && *e != 0 && std::strcmp(e, "0") != 0 && std::strcmp(e, "false") != 0;
+}
+bool wants_grad(const Tensor& t) { return at::GradMode::is_enabled() && t.defined() && t.requires_grad(); }
+// sum over the rows of a bf16 gradient (the bias gradient), fp32 inside
+Tensor column_sum(const Tensor& x) {
+  c10::cuda::CUDAGuard g(x.device());
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.scalar_type() == at::kBFloat16, "column_sum: contiguous bf16 [T,N]");
+  auto out = at::empty({x.size(1)}, x.options());
+  check(odc::launch_column_sum(x.data_ptr(), out.data_ptr(), nullptr, x.size(0), static_cast<int>(x.size(1)), cur_stream()),
+        "column_sum");
+  count();
+  return out;
+}
+
+Tensor rows2d(const Tensor& x) { return x.dim() == 2 ? x : x.reshape({-1, x.size(-1)}); }
+Tensor like(const Tensor& y2, const Tensor& x, int64_t last) {
+  if (x.dim() == 2) return y2;
+  auto sizes = x.sizes().vec();
+  sizes.back() = last;
+  return y2.view(sizes);
+}
+
+struct LinearFn : Function<LinearFn> {
+  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor w, c10::optional<Tensor> bias, c10::optional<Tensor> residual,
+                        bool need_dx, bool need_dw, bool need_db, bool need_dres) {
+    ctx->save_for_backward({x, w});
+    ctx->saved_data["need"] = static_cast<int64_t>(need_dx | need_dw << 1 | need_db << 2 | need_dres << 3);
+    Tensor res;
+    if (residual.has_value()) res = rows2d(*residual);  // added in the GEMM epilogue
+    return like(product(rows2d(x), w, kNT, bias.value_or(Tensor()), res), x, w.size(0));
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1], &dy = grads[0];
+    const int64_t need = ctx->saved_data["need"].toInt();
+    const Tensor dy2 = rows2d(dy).contiguous();
+    Tensor dx, dw, db;
+    if (need & 1) dx = product(dy2, w, kNN).view(x.sizes());
+    if (need & 2) dw = product(dy2, rows2d(x), kTN, {}, {}, w.scalar_type());
+    if (need & 4) db = column_sum(dy2);
+    return {dx, dw, db, (need & 8) ? dy : Tensor(), {}, {}, {}, {}};
+  }
+};
+
+Tensor linear(Tensor x, Tensor w, c10::optional<Tensor> bias, c10::optional<Tensor> residual) {
+  const bool db = bias.has_value() && wants_grad(*bias), dres = residual.has_value() && wants_grad(*residual);
+  return LinearFn::apply(x, w, bias, residual, wants_grad(x), wants_grad(w), db, dres);
+}
+
+// RMSNorm; with_residual also returns x, and backward forms d(norm) + d(residual) in one pass over the activation
+// instead of leaving a separate addition to autograd.  `sink` (fp32 [H]): the weight's gradient is added there by the
+// kernel and the weight itself gets none (engines that keep all small parameters in one flat accumulator).
+struct RMSNormFn : Function<RMSNormFn> {
+  static variable_list forward(AutogradContext* ctx, Tensor x, Tensor w, double eps, bool with_residual,
+                               c10::optional<Tensor> sink) {
+    const Tensor x2 = rows2d(x);
+    auto [y, rstd] = rmsnorm_fwd(x2, w, eps);
+    count();
+    ctx->save_for_backward({x2, w, rstd});
+    if (sink.has_value()) ctx->saved_data["sink"] = *sink;
+    ctx->saved_data["residual"] = with_residual;
+    ctx->saved_data["sizes"] = x.sizes().vec();
+    if (x.dim() != 2) y = y.view(x.sizes());
+    if (!with_residual) return {y};
+    return {y, x.view_as(x)};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x2 = saved[0], &w = saved[1], &rstd = saved[2];
+    const bool fixed = env_on("ODC_DETERMINISTIC");  // fixed-order column sums instead of in-kernel atomics
+    const Tensor dy2 = rows2d(grads[0]).contiguous();
+    c10::optional<Tensor> dres;
+    if (ctx->saved_data["residual"].toBool() && grads[1].defined()) dres = rows2d(grads[1]).contiguous();
+    auto it = ctx->saved_data.find("sink");
+    auto [dx, dw] = rmsnorm_bwd(dy2, x2, w, rstd, fixed, dres);
+    count(fixed ? 2 : 1);
+    if (it != ctx->saved_data.end()) {
+      it->second.toTensor().add_(dw);
+      dw = Tensor();
+    } else if (dw.scalar_type() != w.scalar_type()) {
+      dw = dw.to(w.scalar_type());
+    }
+    return {dx.view(ctx->saved_data["sizes"].toIntVector()), dw, {}, {}, {}};
+  }
+};
+
+Tensor rms_norm(Tensor x, Tensor w, double eps, c10::optional<Tensor> sink) {
+  return RMSNormFn::apply(x.contiguous(), w, eps, false, sink)[0];
+}
+std::tuple<Tensor, Tensor> rms_norm_residual(Tensor x, Tensor w, double eps, c10::optional<Tensor> sink) {
+  auto out = RMSNormFn::apply(x.contiguous(), w, eps, true, sink);
+  return {out[0], out[1]};
+}
+
+// rotary embedding of the q and k heads of a fused [T, (Hq+2Hkv)*D] projection; v passes through
+struct RopeFn : Function<RopeFn> {
+  static Tensor forward(AutogradContext* ctx, Tensor qkv, Tensor pos, int64_t n_q, int64_t n_kv, int64_t d, double theta) {
+    ctx->save_for_backward({pos});
+    ctx->saved_data["cfg"] = std::vector<int64_t>{n_q, n_kv, d};
+    ctx->saved_data["theta"] = theta;
+    auto out = rope_qkv(qkv, pos, n_q, n_kv, d, theta, false);
+    count();
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor pos = ctx->get_saved_variables()[0];
+    const auto cfg = ctx->saved_data["cfg"].toIntVector();
+    auto d = rope_qkv(grads[0].contiguous(), pos, cfg[0], cfg[1], cfg[2], ctx->saved_data["theta"].toDouble(), true);
+    count();
+    return {d, {}, {}, {}, {}, {}};
+  }
+};
+Tensor rope(Tensor qkv, Tensor pos, int64_t n_q, int64_t n_kv, int64_t d, double theta) {
+  return RopeFn::apply(qkv, pos, n_q, n_kv, d, theta);
+}
+
+struct SwiGLUFn : Function<SwiGLUFn> {
+  static Tensor forward(AutogradContext* ctx, Tensor gate_up) {
+    ctx->save_for_backward({gate_up});
+    count();
+    return swiglu_fwd(gate_up);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const Tensor gate_up = ctx->get_saved_variables()[0];
+    count();
+    return {swiglu_bwd(grads[0].contiguous(), gate_up)};
+  }
+};
+Tensor swiglu(Tensor gate_up) { return SwiGLUFn::apply(gate_up.contiguous()); }
+
+struct AttentionFn : Function<AttentionFn> {
+  static Tensor forward(AutogradContext* ctx, Tensor q, Tensor k, Tensor v, Tensor cu, int64_t max_seqlen, bool causal,
+                        double scale) {
+    auto [o, lse] = attn_fwd(q, k, v, cu, max_seqlen, causal, scale);
+    count();
+    ctx->save_for_backward({q, k, v, o, lse, cu});
+    ctx->saved_data["max"] = max_seqlen;
+    ctx->saved_data["causal"] = causal;
+    ctx->saved_data["scale"] = scale;
+    return o;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    auto [dq, dk, dv, all] = attn_bwd(grads[0].contiguous(), s[0], s[1], s[2], s[3], s[4], s[5], ctx->saved_data["max"].toInt(),
+                                      ctx->saved_data["causal"].toBool(), ctx->saved_data["scale"].toDouble(), false);
+    count(3);
+    return {dq, dk, dv, {}, {}, {}, {}};
+  }
+};
+Tensor attention(Tensor q, Tensor k, Tensor v, Tensor cu, int64_t max_seqlen, bool causal, double scale) {
+  return AttentionFn::apply(q, k, v, cu, max_seqlen, causal, scale);
+}
+
+// Attention straight on a fused projection: q/k/v are column views in forward, and the backward kernels write dq/dk/dv
+// into column views of ONE gradient tensor, so autograd never materialises zero-padded slices.
+struct AttentionQKVFn : Function<AttentionQKVFn> {
+  static std::array<Tensor, 3> parts(const Tensor& qkv, int64_t n_q, int64_t n_kv, int64_t d) {
+    const int64_t T = qkv.size(0), ld = qkv.stride(0);
+    auto view = [&](int64_t first, int64_t heads) {
+      return qkv.as_strided({T, heads, d}, {ld, d, 1}, qkv.storage_offset() + first * d);
+    };
+    return {view(0, n_q), view(n_q, n_kv), view(n_q + n_kv, n_kv)};
+  }
+  static Tensor forward(AutogradContext* ctx, Tensor qkv, int64_t n_q, int64_t n_kv, int64_t d, Tensor cu, int64_t max_seqlen,
+                        bool causal, double scale) {
+    TORCH_CHECK(qkv.dim() == 2 && qkv.size(1) == (n_q + 2 * n_kv) * d && qkv.stride(1) == 1, "attention: qkv [T,(Hq+2Hkv)*D]");
+    const auto [q, k, v] = parts(qkv, n_q, n_kv, d);
+    auto [o, lse] = attn_fwd(q, k, v, cu, max_seqlen, causal, scale);
+    count();
+    ctx->save_for_backward({qkv, o, lse, cu});
+    ctx->saved_data["cfg"] = std::vector<int64_t>{n_q, n_kv, d, max_seqlen, causal};
+    ctx->saved_data["scale"] = scale;
+    return o;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const auto cfg = ctx->saved_data["cfg"].toIntVector();
+    const auto [q, k, v] = parts(s[0], cfg[0], cfg[1], cfg[2]);
+    auto [dq, dk, dv, dqkv] = attn_bwd(grads[0].contiguous(), q, k, v, s[1], s[2], s[3], cfg[3], cfg[4] != 0,
+                                       ctx->saved_data["scale"].toDouble(), true);
+    count(3);
+    return {dqkv, {}, {}, {}, {}, {}, {}, {}};
+  }
+};
+Tensor attention_qkv(Tensor qkv, int64_t n_q, int64_t n_kv, int64_t d, Tensor cu, int64_t max_seqlen, bool causal, double scale) {
+  return AttentionQKVFn::apply(qkv, n_q, n_kv, d, cu, max_seqlen, causal, scale);
+}
+
+// ---- LM head ---------------------------------------------------------------------------------------------------------
+// Loss and both gradients (for a loss gradient of one) in one pass over token chunks; [T, vocab] logits never exist.
+// Same mathematics as the reference's chunked LM head (examples/llm_training/lm_head.py:7-59), but the gradients are
+// formed while the chunk's logits are at hand, so backward is a multiplication by the loss gradient.
+std::tuple<Tensor, Tensor, Tensor> lm_head_loss(const Tensor& h, const Tensor& w, const Tensor& labels,
+                                                const c10::optional<Tensor>& loss_scale, int64_t ignore_index, int64_t chunk,
+                                                bool need_dh, bool need_dw, c10::optional<Tensor> dw_out) {
+  const int64_t T = h.size(0), V = w.size(0), H = h.size(1);
+  auto loss = at::zeros({}, h.options().dtype(at::kFloat));
+  auto logits = at::empty({std::min(chunk, T), V}, h.options());
+  Tensor dh, dw;
+  if (need_dh) dh = at::empty_like(h);
+  if (need_dw) dw = dw_out.has_value() ? *dw_out : at::empty({V, H}, h.options().dtype(at::kFloat));
+  if (T == 0 && need_dw) dw.zero_();
+  for (int64_t s = 0; s < T; s += chunk) {
+    const int64_t n = std::min(chunk, T - s);
+    const Tensor hs = h.narrow(0, s, n), lg = logits.narrow(0, 0, n);
+    product_into(hs, w, lg, kNT);
+    // in place: logits -> loss_scale * (softmax - onehot); adds the chunk's loss
+    ce_fwd_bwd(lg, labels.narrow(0, s, n), loss_scale.has_value() ? c10::optional<Tensor>(loss_scale->narrow(0, s, n)) : c10::nullopt,
+               loss, ignore_index);
+    count();
+    if (need_dh) product_into(lg, w, dh.narrow(0, s, n), kNN);
+    if (need_dw) product_into(lg, hs, dw, kTN, {}, s > 0);
+  }
+  return {loss, dh, dw};
+}
+
+struct LinearCrossEntropyFn : Function<LinearCrossEntropyFn> {
+  static Tensor forward(AutogradContext* ctx, Tensor h, Tensor w, Tensor labels, c10::optional<Tensor> loss_scale,
+                        int64_t ignore_index, int64_t chunk, bool need_dh, bool need_dw) {
+    auto [loss, dh, dw] = lm_head_loss(h, w, labels, loss_scale, ignore_index, chunk, need_dh, need_dw, c10::nullopt);
+    ctx->save_for_backward({dh, dw});
+    ctx->saved_data["dtype"] = w.scalar_type();
+    return loss;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor& g = grads[0];
+    Tensor gh, gw;
+    if (s[0].defined()) gh = s[0] * g.to(s[0].scalar_type());
+    if (s[1].defined()) gw = (s[1] * g).to(ctx->saved_data["dtype"].toScalarType());
+    return {gh, gw, {}, {}, {}, {}, {}, {}};
+  }
+};
+Tensor linear_cross_entropy(Tensor h, Tensor w, Tensor labels, c10::optional<Tensor> loss_scale, int64_t ignore_index,
+                            int64_t chunk) {
+  if (loss_scale.has_value()) loss_scale = loss_scale->to(at::kFloat);  // FSDP's mixed-precision input cast may have narrowed it
+  return LinearCrossEntropyFn::apply(h.contiguous(), w, labels.contiguous(), loss_scale, ignore_index, chunk, wants_grad(h),
+                                     wants_grad(w));
+}
+
+// Per-token log-probability of `ids` under softmax(h w^T / temperature), in token chunks: the policy-gradient form of the
+// chunked LM head (the reference's FusedLinearForPPOFunction, examples/llm_training/lm_head.py:62-190).  The weights of
+// the tokens are only known in backward, so backward recomputes each chunk's logits and turns them in place into
+// dlogp / temperature * (onehot - softmax).
+struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
+  static Tensor forward(AutogradContext* ctx, Tensor h, Tensor w, Tensor ids, double temperature, int64_t ignore_index,
+                        int64_t chunk, bool need_dh, bool need_dw) {
+    const int64_t T = h.size(0);
+    auto out = at::empty({T}, h.options().dtype(at::kFloat));
+    auto logits = at::empty({std::min(chunk, T), w.size(0)}, h.options());
+    for (int64_t s = 0; s < T; s += chunk) {
+      const int64_t n = std::min(chunk, T - s);
+      const Tensor lg = logits.narrow(0, 0, n);
+      product_into(h.narrow(0, s, n), w, lg, kNT);
+      if (temperature != 1.0) lg.mul_(1.0 / temperature);
+      token_logprobs(lg, ids.narrow(0, s, n), out.narrow(0, s, n), ignore_index);
+      count();
+    }
+    ctx->save_for_backward({h, w, ids});
+    ctx->saved_data["cfg"] = std::vector<int64_t>{ignore_index, chunk, need_dh, need_dw};
+    ctx->saved_data["temperature"] = temperature;
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &h = saved[0], &w = saved[1], &ids = saved[2];
+    const auto cfg = ctx->saved_data["cfg"].toIntVector();
+    const double temperature = ctx->saved_data["temperature"].toDouble();
+    const int64_t T = h.size(0), chunk = cfg[1];
+    Tensor dh, dw;
+    if (cfg[2]) dh = at::empty_like(h);
+    if (cfg[3]) dw = at::empty(w.sizes(), w.options().dtype(at::kFloat));
+    if (T == 0 && cfg[3]) dw.zero_();
+    const Tensor scale = (grads[0].reshape({-1}).to(at::kFloat) * (-1.0 / temperature)).contiguous();
+    auto sink = at::zeros({}, scale.options());  // the kernel's loss output is not used here
+    auto logits = at::empty({std::min(chunk, T), w.size(0)}, h.options());
+    for (int64_t s = 0; s < T; s += chunk) {
+      const int64_t n = std::min(chunk, T - s);
+      const Tensor hs = h.narrow(0, s, n), lg = logits.narrow(0, 0, n);
+      product_into(hs, w, lg, kNT);
+      if (temperature != 1.0) lg.mul_(1.0 / temperature);
+      ce_fwd_bwd(lg, ids.narrow(0, s, n), scale.narrow(0, s, n), sink, cfg[0]);
+      count();
+      if (cfg[2]) product_into(lg, w, dh.narrow(0, s, n), kNN);
+      if (cfg[3]) product_into(lg, hs, dw, kTN, {}, s > 0);
+    }
+    return {dh, dw.defined() ? dw.to(w.scalar_type()) : dw, {}, {}, {}, {}, {}, {}};
+  }
+};
+Tensor linear_token_logprobs(Tensor h, Tensor w, Tensor ids, double temperature, int64_t ignore_index, int64_t chunk) {
+  return LinearTokenLogProbsFn::apply(h.contiguous(), w, ids.contiguous(), temperature, ignore_index, chunk, wants_grad(h),
+                                      wants_grad(w));
+}
+
+}  // namespace
+
+void register_ops(py::module_& m) {
+  m.def("kernel_launches", [] { return g_launches.load(std::memory_order_relaxed); });
+  m.def("count_launches", [](int n) { count(n); });
+  m.def("rmsnorm_fwd", &rmsnorm_fwd);
+  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("dy"), py::arg("x"), py::arg("w"), py::arg("rstd"),
+        py::arg("fixed_order") = false, py::arg("dres") = py::none());
+  m.def("rope_qkv", &rope_qkv);
+  m.def("swiglu_fwd", &swiglu_fwd);
+  m.def("swiglu_bwd", &swiglu_bwd);
+  m.def("ce_fwd_bwd", &ce_fwd_bwd);
+  m.def("token_logprobs", &token_logprobs);
+  m.def("adamw_step", &adamw_step);
+  m.def("cast_f32_to_bf16", &cast_f32_to_bf16);
+  m.def("sumsq", &sumsq);
+  m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("c"), py::arg("layout"), py::arg("bias"),
+        py::arg("accumulate"), py::arg("residual") = py::none(), py::arg("pair") = -1);
+  m.def("attn_fwd", &attn_fwd);
+  m.def("attn_bwd", &attn_bwd);
+  m.def("kernel_status", &kernel_status);
+  // differentiable forms
+  m.def("linear", &linear, py::arg("x"), py::arg("w"), py::arg("bias") = py::none(), py::arg("residual") = py::none());
+  m.def("rms_norm", &rms_norm, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());
+  m.def("rms_norm_residual", &rms_norm_residual, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());
+  m.def("rope", &rope);
+  m.def("swiglu", &swiglu);
+  m.def("attention", &attention);
+  m.def("attention_qkv", &attention_qkv);
+  m.def("linear_cross_entropy", &linear_cross_entropy);
+  m.def("linear_token_logprobs", &linear_token_logprobs);
+  m.def("lm_head_loss", &lm_head_loss, py::arg("h"), py::arg("w"), py::arg("labels"), py::arg("loss_scale"),
+        py::arg("ignore_index"), py::arg("chunk"), py::arg("need_dh"), py::arg("need_dw"), py::arg("dw_out") = py::none());
+}
+
+}  // namespace odc_bind

@@ -87,6 +87,8 @@ cudaError_t launch_token_logprobs(const void* logits, const long long* labels, f
 cudaError_t launch_adamw(float* p, const void* g, int g_kind, float* m, float* v, void* p_lowp, size_t n, float lr,
                          float beta1, float beta2, float eps, float wd, float bc1, float bc2, float grad_scale,
                          int sm_count, cudaStream_t stream);
+// column sums of a bf16 [rows, cols] matrix, fp32 inside: rounded into out (bf16) or added to sink (fp32); cols % 8 == 0
+cudaError_t launch_column_sum(const void* x, void* out, float* sink, long long rows, int cols, cudaStream_t stream);
 cudaError_t launch_cast_f32_to_bf16(const float* in, void* out, size_t n, int sm_count, cudaStream_t stream);
 cudaError_t launch_sumsq(const void* x, int kind, size_t n, float* out, int sm_count, cudaStream_t stream);
 

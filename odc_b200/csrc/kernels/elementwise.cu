@@ -238,6 +238,46 @@ __global__ void colsum_kernel(const float* __restrict__ partial, float* __restri
   out[c] = s;
 }
 
+// Column sums of a bf16 matrix (bias gradients): a CTA owns 64 columns and walks all rows, so there is one launch, no
+// zeroed scratch and a fixed order of additions.  Bound by the load latency of the walk: 1024 threads with four 16-byte
+// loads each keep 64 KiB in flight per CTA.
+constexpr int kColSumThreads = 1024;
+__global__ void __launch_bounds__(kColSumThreads)
+column_sum_kernel(const bf16* __restrict__ x, bf16* __restrict__ out, float* __restrict__ sink, long long rows, int cols) {
+  __shared__ float part[kColSumThreads / 32][64];
+  const int vec = threadIdx.x & 7, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int col = blockIdx.x * 64 + vec * 8;
+  constexpr int kRows = kColSumThreads / 8;
+  float s[8] = {};
+  if (col < cols) {
+    const bf16* p = x + col;
+#pragma unroll 4
+    for (long long r = threadIdx.x >> 3; r < rows; r += kRows) {
+      float f[8];
+      unpack8(*reinterpret_cast<const uint4*>(p + r * cols), f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s[i] += f[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    s[i] += __shfl_xor_sync(0xffffffffu, s[i], 8);
+    s[i] += __shfl_xor_sync(0xffffffffu, s[i], 16);
+  }
+  if (lane < 8) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part[warp][vec * 8 + i] = s[i];
+  }
+  __syncthreads();
+  const int c = blockIdx.x * 64 + threadIdx.x;
+  if (threadIdx.x < 64 && c < cols) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < kColSumThreads / 32; ++w) t += part[w][threadIdx.x];
+    if (sink != nullptr) sink[c] += t; else out[c] = __float2bfloat16(t);
+  }
+}
+
 // ------------------------------------------------------------------------- RoPE -------------
 // one CTA per token; cos/sin of the head_dim/2 angles computed once and reused by all heads
 __global__ void __launch_bounds__(128)
@@ -526,6 +566,14 @@ cudaError_t launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
     e = cudaGetLastError();
   }
   return e;
+}
+
+cudaError_t launch_column_sum(const void* x, void* out, float* sink, long long rows, int cols, cudaStream_t stream) {
+  if (cols % 8 != 0 || (out == nullptr) == (sink == nullptr)) return cudaErrorInvalidValue;
+  if (cols == 0) return cudaSuccess;
+  column_sum_kernel<<<(cols + 63) / 64, kColSumThreads, 0, stream>>>(static_cast<const bf16*>(x), static_cast<bf16*>(out), sink,
+                                                                    rows, cols);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_rope_qkv(const void* in, void* out, const long long* pos, int tokens, int n_q, int n_kv,
