@@ -49,145 +49,7 @@ Tensor& device_status(int device) {
   return it->second;
 }
 
-}  // namespace odc_bind
-
-namespace {
-
-using namespace odc_bind;
-
-// ---------------------------------------------------------------------------------------- heap
-uintptr_t heap_create(int rank, int world, int device, size_t bytes, const std::string& mode,
-                      const std::string& token) {
-  return reinterpret_cast<uintptr_t>(odc::heap_create(rank, world, device, bytes, mode, token));
-}
-odc::Heap* H(uintptr_t h) { return reinterpret_cast<odc::Heap*>(h); }
-
-Tensor tensor_from_ptr(uintptr_t ptr, int64_t numel, at::ScalarType dtype, int device) {
-  auto opts = torch::TensorOptions().dtype(dtype).device(torch::kCUDA, device);
-  return torch::from_blob(reinterpret_cast<void*>(ptr), {numel}, [](void*) {}, opts);
-}
-
-py::bytes get_ipc_handle(const Tensor& t) {
-  TORCH_CHECK(t.is_cuda(), "get_ipc_handle expects a CUDA tensor");
-  c10::cuda::CUDAGuard g(t.device());
-  odc::bind_device(t.get_device());
-  return py::bytes(odc::ipc_export(t.data_ptr()));
-}
-
-Tensor reconstruct_tensor(const std::string& blob, std::vector<int64_t> shape, at::ScalarType dtype) {
-  void* p = odc::ipc_import(blob);
-  int dev = 0;
-  cudaGetDevice(&dev);
-  auto opts = torch::TensorOptions().dtype(dtype).device(torch::kCUDA, dev);
-  return torch::from_blob(p, shape, [](void*) {}, opts);
-}
-
-// ---------------------------------------------------------------------------------------- comm
-void gather(Tensor out2d, Tensor table, int64_t n, at::ScalarType src_dtype, int my_index, bool checkb,
-            Tensor status, int64_t src_region_elems) {
-  c10::cuda::CUDAGuard g(out2d.device());
-  odc::bind_device(out2d.get_device());
-  const int nranks = static_cast<int>(table.numel());
-  TORCH_CHECK(out2d.is_contiguous() && out2d.numel() == n * nranks, "gather: bad output shape");
-  const int ssz = static_cast<int>(c10::elementSize(src_dtype));
-  const int dsz = static_cast<int>(out2d.element_size());
-  const bool narrow = (src_dtype == at::kFloat && out2d.scalar_type() == at::kBFloat16);
-  TORCH_CHECK(narrow || src_dtype == out2d.scalar_type(), "gather: only same-dtype or fp32->bf16");
-  check(odc::launch_gather(table.data_ptr<int64_t>() ? reinterpret_cast<const long long*>(table.data_ptr<int64_t>()) : nullptr,
-                           out2d.data_ptr(), static_cast<size_t>(n), ssz, dsz, narrow, nranks, my_index, checkb,
-                           status.data_ptr<int>(), sm_count(), cur_stream(),
-                           checkb ? static_cast<size_t>(src_region_elems) : 0),
-        "gather launch");
-}
-
-void scatter_accumulate(Tensor inp2d, Tensor acc_table, Tensor ctr_table, int64_t n, at::ScalarType acc_dtype,
-                        int my_index, double scale, bool checkb, Tensor status, int64_t acc_region_elems) {
-  c10::cuda::CUDAGuard g(inp2d.device());
-  odc::bind_device(inp2d.get_device());
-  const int nranks = static_cast<int>(acc_table.numel());
-  TORCH_CHECK(inp2d.is_contiguous() && inp2d.numel() == n * nranks, "scatter_accumulate: bad input shape");
-  check(odc::launch_scatter_accumulate(inp2d.data_ptr(), kind_of(inp2d.scalar_type()),
-                                       reinterpret_cast<const long long*>(acc_table.data_ptr<int64_t>()),
-                                       kind_of(acc_dtype),
-                                       reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()),
-                                       static_cast<size_t>(n), nranks, my_index, static_cast<float>(scale),
-                                       next_done_slot(inp2d.get_device()), sm_count(), cur_stream(),
-                                       status.data_ptr<int>(), checkb ? acc_region_elems : 0),
-        "scatter_accumulate launch");
-}
-
-bool scatter_accumulate_segments(std::vector<Tensor> grads, std::vector<int64_t> chunk_numels,
-                                 std::vector<int64_t> dst_offsets, Tensor acc_table, Tensor ctr_table,
-                                 at::ScalarType acc_dtype, int my_index, double scale, bool checkb,
-                                 c10::optional<Tensor> status, int64_t acc_region_elems) {
-  // Returns false (nothing launched) when the list does not fit this path; the caller then flattens the gradients.
-  if (grads.empty() || grads.size() > static_cast<size_t>(odc::kMaxScatterSegments) || acc_dtype != at::kFloat) return false;
-  TORCH_CHECK(grads.size() == chunk_numels.size() && grads.size() == dst_offsets.size(),
-              "scatter_accumulate_segments: one chunk size and one offset per gradient");
-  const auto dt = grads[0].scalar_type();
-  if (dt != at::kFloat && dt != at::kBFloat16) return false;
-  odc::ScatterSegments segs{};
-  segs.count = static_cast<int>(grads.size());
-  for (size_t i = 0; i < grads.size(); ++i) {
-    const Tensor& g = grads[i];
-    if (!g.is_cuda() || !g.is_contiguous() || g.scalar_type() != dt || g.device() != grads[0].device()) return false;
-    segs.src[i] = g.data_ptr();
-    segs.chunk[i] = chunk_numels[i];
-    segs.total[i] = g.numel();
-    segs.dst[i] = dst_offsets[i];
-  }
-  c10::cuda::CUDAGuard guard(grads[0].device());
-  odc::bind_device(grads[0].get_device());
-  const int nranks = static_cast<int>(acc_table.numel());
-  check(odc::launch_scatter_accumulate_segments(segs, kind_of(dt),
-                                                reinterpret_cast<const long long*>(acc_table.data_ptr<int64_t>()),
-                                                reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()), nranks,
-                                                my_index, static_cast<float>(scale),
-                                                next_done_slot(grads[0].get_device()), sm_count(), cur_stream(),
-                                                (checkb && status.has_value()) ? acc_region_elems : 0,
-                                                status.has_value() ? status->data_ptr<int>() : nullptr),
-        "scatter_accumulate_segments launch");
-  return true;
-}
-
-void wait_counter(Tensor counter, int64_t expected, int64_t timeout_ms, Tensor status) {
-  c10::cuda::CUDAGuard g(counter.device());
-  odc::bind_device(counter.get_device());
-  check(odc::launch_wait_counter(counter.data_ptr(), static_cast<unsigned long long>(expected),
-                                 static_cast<unsigned long long>(timeout_ms) * 1000000ull, status.data_ptr<int>(),
-                                 cur_stream()),
-        "wait_counter launch");
-}
-
-void post_counts(std::vector<int64_t> slot_addrs, std::vector<int64_t> counts, int64_t epoch, int device) {
-  c10::cuda::CUDAGuard g(c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(device)));
-  odc::bind_device(device);
-  TORCH_CHECK(slot_addrs.size() == counts.size() && slot_addrs.size() <= size_t(odc::kMaxPostedCounts),
-              "post_counts: at most ", odc::kMaxPostedCounts, " owners");
-  odc::PostedCounts pc{};
-  pc.n = static_cast<int>(slot_addrs.size());
-  for (int i = 0; i < pc.n; ++i) {
-    TORCH_CHECK(slot_addrs[i] != 0 && (slot_addrs[i] & 7) == 0, "post_counts: bad slot address");
-    TORCH_CHECK(counts[i] >= 0 && counts[i] < (int64_t(1) << 32), "post_counts: count out of range");
-    pc.slot_addr[i] = slot_addrs[i];
-    pc.value[i] = (static_cast<unsigned long long>(epoch) << 32) | static_cast<unsigned long long>(counts[i]);
-  }
-  check(odc::launch_post_counts(pc, cur_stream()), "post_counts launch");
-}
-
-void wait_posted(Tensor slots, int64_t nprod, int64_t epoch, Tensor counter, int64_t timeout_ms, Tensor status,
-                 Tensor expected_out) {
-  c10::cuda::CUDAGuard g(counter.device());
-  odc::bind_device(counter.get_device());
-  TORCH_CHECK(slots.scalar_type() == at::kLong && slots.numel() >= nprod && expected_out.scalar_type() == at::kLong,
-              "wait_posted: int64 slots (one per producer) and an int64 output word");
-  check(odc::launch_wait_posted(slots.data_ptr(), static_cast<int>(nprod), static_cast<unsigned long long>(epoch),
-                                counter.data_ptr(), static_cast<unsigned long long>(timeout_ms) * 1000000ull,
-                                status.data_ptr<int>(), reinterpret_cast<unsigned long long*>(expected_out.data_ptr()),
-                                cur_stream()),
-        "wait_posted launch");
-}
-
+// ---------------------------------------------------------------------------------------- GEMMs fused with the primitives
 void gemm_wgrad_scatter(Tensor dy, Tensor x, Tensor acc_table, Tensor ctr_table, int64_t acc_offset,
                         int64_t rows_per_rank, double scale) {
   c10::cuda::CUDAGuard g(dy.device());
@@ -273,6 +135,198 @@ Tensor gemm_gather_dgrad(Tensor dy, Tensor shard_table, Tensor w_local, int64_t 
   return dx;
 }
 
+}  // namespace odc_bind
+
+namespace {
+
+using namespace odc_bind;
+
+// ---------------------------------------------------------------------------------------- heap
+uintptr_t heap_create(int rank, int world, int device, size_t bytes, const std::string& mode,
+                      const std::string& token) {
+  return reinterpret_cast<uintptr_t>(odc::heap_create(rank, world, device, bytes, mode, token));
+}
+odc::Heap* H(uintptr_t h) { return reinterpret_cast<odc::Heap*>(h); }
+
+Tensor tensor_from_ptr(uintptr_t ptr, int64_t numel, at::ScalarType dtype, int device) {
+  auto opts = torch::TensorOptions().dtype(dtype).device(torch::kCUDA, device);
+  return torch::from_blob(reinterpret_cast<void*>(ptr), {numel}, [](void*) {}, opts);
+}
+
+py::bytes get_ipc_handle(const Tensor& t) {
+  TORCH_CHECK(t.is_cuda(), "get_ipc_handle expects a CUDA tensor");
+  c10::cuda::CUDAGuard g(t.device());
+  odc::bind_device(t.get_device());
+  return py::bytes(odc::ipc_export(t.data_ptr()));
+}
+
+Tensor reconstruct_tensor(const std::string& blob, std::vector<int64_t> shape, at::ScalarType dtype) {
+  void* p = odc::ipc_import(blob);
+  int dev = 0;
+  cudaGetDevice(&dev);
+  auto opts = torch::TensorOptions().dtype(dtype).device(torch::kCUDA, dev);
+  return torch::from_blob(p, shape, [](void*) {}, opts);
+}
+
+// ---------------------------------------------------------------------------------------- comm
+void gather(Tensor out2d, Tensor table, int64_t n, at::ScalarType src_dtype, int my_index, bool checkb,
+            Tensor status, int64_t src_region_elems) {
+  c10::cuda::CUDAGuard g(out2d.device());
+  odc::bind_device(out2d.get_device());
+  const int nranks = static_cast<int>(table.numel());
+  TORCH_CHECK(out2d.is_contiguous() && out2d.numel() == n * nranks, "gather: bad output shape");
+  const int ssz = static_cast<int>(c10::elementSize(src_dtype));
+  const int dsz = static_cast<int>(out2d.element_size());
+  const bool narrow = (src_dtype == at::kFloat && out2d.scalar_type() == at::kBFloat16);
+  TORCH_CHECK(narrow || src_dtype == out2d.scalar_type(), "gather: only same-dtype or fp32->bf16");
+  check(odc::launch_gather(table.data_ptr<int64_t>() ? reinterpret_cast<const long long*>(table.data_ptr<int64_t>()) : nullptr,
+                           out2d.data_ptr(), static_cast<size_t>(n), ssz, dsz, narrow, nranks, my_index, checkb,
+                           status.data_ptr<int>(), sm_count(), cur_stream(),
+                           checkb ? static_cast<size_t>(src_region_elems) : 0),
+        "gather launch");
+}
+
+void scatter_accumulate(Tensor inp2d, Tensor acc_table, Tensor ctr_table, int64_t n, at::ScalarType acc_dtype,
+                        int my_index, double scale, bool checkb, Tensor status, int64_t acc_region_elems,
+                        c10::optional<Tensor> scale_tensor) {
+  c10::cuda::CUDAGuard g(inp2d.device());
+  if (scale_tensor.has_value())
+    TORCH_CHECK(scale_tensor->is_cuda() && scale_tensor->scalar_type() == at::kFloat && scale_tensor->numel() == 1 &&
+                    acc_dtype == at::kFloat, "scatter_accumulate: the scale tensor is one fp32 value on the device");
+  odc::bind_device(inp2d.get_device());
+  const int nranks = static_cast<int>(acc_table.numel());
+  TORCH_CHECK(inp2d.is_contiguous() && inp2d.numel() == n * nranks, "scatter_accumulate: bad input shape");
+  check(odc::launch_scatter_accumulate(inp2d.data_ptr(), kind_of(inp2d.scalar_type()),
+                                       reinterpret_cast<const long long*>(acc_table.data_ptr<int64_t>()),
+                                       kind_of(acc_dtype),
+                                       reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()),
+                                       static_cast<size_t>(n), nranks, my_index, static_cast<float>(scale),
+                                       next_done_slot(inp2d.get_device()), sm_count(), cur_stream(),
+                                       status.data_ptr<int>(), checkb ? acc_region_elems : 0,
+                                       scale_tensor.has_value() ? scale_tensor->data_ptr<float>() : nullptr),
+        "scatter_accumulate launch");
+}
+
+bool scatter_accumulate_segments(std::vector<Tensor> grads, std::vector<int64_t> chunk_numels,
+                                 std::vector<int64_t> dst_offsets, Tensor acc_table, Tensor ctr_table,
+                                 at::ScalarType acc_dtype, int my_index, double scale, bool checkb,
+                                 c10::optional<Tensor> status, int64_t acc_region_elems) {
+  // Returns false (nothing launched) when the list does not fit this path; the caller then flattens the gradients.
+  if (grads.empty() || grads.size() > static_cast<size_t>(odc::kMaxScatterSegments) || acc_dtype != at::kFloat) return false;
+  TORCH_CHECK(grads.size() == chunk_numels.size() && grads.size() == dst_offsets.size(),
+              "scatter_accumulate_segments: one chunk size and one offset per gradient");
+  const auto dt = grads[0].scalar_type();
+  if (dt != at::kFloat && dt != at::kBFloat16) return false;
+  odc::ScatterSegments segs{};
+  segs.count = static_cast<int>(grads.size());
+  for (size_t i = 0; i < grads.size(); ++i) {
+    const Tensor& g = grads[i];
+    if (!g.is_cuda() || !g.is_contiguous() || g.scalar_type() != dt || g.device() != grads[0].device()) return false;
+    segs.src[i] = g.data_ptr();
+    segs.chunk[i] = chunk_numels[i];
+    segs.total[i] = g.numel();
+    segs.dst[i] = dst_offsets[i];
+  }
+  c10::cuda::CUDAGuard guard(grads[0].device());
+  odc::bind_device(grads[0].get_device());
+  const int nranks = static_cast<int>(acc_table.numel());
+  check(odc::launch_scatter_accumulate_segments(segs, kind_of(dt),
+                                                reinterpret_cast<const long long*>(acc_table.data_ptr<int64_t>()),
+                                                reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()), nranks,
+                                                my_index, static_cast<float>(scale),
+                                                next_done_slot(grads[0].get_device()), sm_count(), cur_stream(),
+                                                (checkb && status.has_value()) ? acc_region_elems : 0,
+                                                status.has_value() ? status->data_ptr<int>() : nullptr),
+        "scatter_accumulate_segments launch");
+  return true;
+}
+
+// rows of a bf16 lookup gradient [T, H] into the fp32 accumulators of the ranks that own the looked-up rows
+void embedding_scatter(Tensor ids, Tensor dx, Tensor acc_table, Tensor ctr_table, int64_t rows_per_rank, int64_t vocab,
+                       double scale) {
+  c10::cuda::CUDAGuard g(dx.device());
+  odc::bind_device(dx.get_device());
+  TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && dx.dim() == 2 && dx.is_contiguous() &&
+                  dx.scalar_type() == at::kBFloat16 && ids.numel() == dx.size(0) && dx.size(1) % 8 == 0,
+              "embedding_scatter: int64 ids [T], contiguous bf16 gradient [T, H], H a multiple of 8");
+  TORCH_CHECK(vocab <= rows_per_rank * acc_table.numel(), "embedding_scatter: more rows than the owners hold");
+  check(odc::launch_embedding_scatter(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), dx.data_ptr(),
+                                      static_cast<int>(dx.size(0)), static_cast<int>(dx.size(1)),
+                                      reinterpret_cast<const long long*>(acc_table.data_ptr<int64_t>()),
+                                      reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()), rows_per_rank, vocab,
+                                      static_cast<int>(acc_table.numel()), static_cast<float>(scale),
+                                      next_done_slot(dx.get_device()), sm_count(), cur_stream()),
+        "embedding_scatter launch");
+}
+
+void wait_counter(Tensor counter, int64_t expected, int64_t timeout_ms, Tensor status) {
+  c10::cuda::CUDAGuard g(counter.device());
+  odc::bind_device(counter.get_device());
+  check(odc::launch_wait_counter(counter.data_ptr(), static_cast<unsigned long long>(expected),
+                                 static_cast<unsigned long long>(timeout_ms) * 1000000ull, status.data_ptr<int>(),
+                                 cur_stream()),
+        "wait_counter launch");
+}
+
+odc::PostedCounts posted(const std::vector<int64_t>& slot_addrs, const std::vector<int64_t>& counts, int64_t epoch) {
+  TORCH_CHECK(slot_addrs.size() == counts.size() && slot_addrs.size() <= size_t(odc::kMaxPostedCounts),
+              "post_counts: at most ", odc::kMaxPostedCounts, " owners");
+  odc::PostedCounts pc{};
+  pc.n = static_cast<int>(slot_addrs.size());
+  for (int i = 0; i < pc.n; ++i) {
+    TORCH_CHECK(slot_addrs[i] != 0 && (slot_addrs[i] & 7) == 0, "post_counts: bad slot address");
+    TORCH_CHECK(counts[i] >= 0 && counts[i] < (int64_t(1) << 32), "post_counts: count out of range");
+    pc.slot_addr[i] = slot_addrs[i];
+    pc.value[i] = (static_cast<unsigned long long>(epoch) << 32) | static_cast<unsigned long long>(counts[i]);
+  }
+  return pc;
+}
+
+void post_counts(std::vector<int64_t> slot_addrs, std::vector<int64_t> counts, int64_t epoch, int device) {
+  c10::cuda::CUDAGuard g(c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(device)));
+  odc::bind_device(device);
+  check(odc::launch_post_counts(posted(slot_addrs, counts, epoch), cur_stream()), "post_counts launch");
+}
+
+// post_counts + wait_posted in one launch, then the current stream is synchronised; returns {code, detail, observed} of
+// the device's status word
+std::tuple<int, int, int> post_and_wait(std::vector<int64_t> slot_addrs, std::vector<int64_t> counts, int64_t epoch, Tensor slots,
+                                        int64_t nprod, Tensor counter, int64_t timeout_ms, Tensor status, Tensor status_host) {
+  c10::cuda::CUDAGuard g(counter.device());
+  odc::bind_device(counter.get_device());
+  TORCH_CHECK(slots.scalar_type() == at::kLong && slots.numel() >= nprod, "post_and_wait: int64 slots, one per producer");
+  TORCH_CHECK(status_host.scalar_type() == at::kInt && status_host.numel() >= 4 && status_host.is_pinned(),
+              "post_and_wait: four pinned ints");
+  int* host = status_host.data_ptr<int>();
+  int* mapped = nullptr;
+  check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&mapped), host, 0), "post_and_wait: status buffer");
+  const cudaStream_t stream = cur_stream();
+  check(odc::launch_post_and_wait(posted(slot_addrs, counts, epoch), slots.data_ptr(), static_cast<int>(nprod),
+                                  static_cast<unsigned long long>(epoch), counter.data_ptr(),
+                                  static_cast<unsigned long long>(timeout_ms) * 1000000ull, status.data_ptr<int>(), mapped, stream),
+        "post_and_wait launch");
+  cudaError_t e;
+  {
+    py::gil_scoped_release nogil;
+    e = cudaStreamSynchronize(stream);
+  }
+  check(e, "post_and_wait");
+  return {host[0], host[1], host[2]};
+}
+
+void wait_posted(Tensor slots, int64_t nprod, int64_t epoch, Tensor counter, int64_t timeout_ms, Tensor status,
+                 Tensor expected_out) {
+  c10::cuda::CUDAGuard g(counter.device());
+  odc::bind_device(counter.get_device());
+  TORCH_CHECK(slots.scalar_type() == at::kLong && slots.numel() >= nprod && expected_out.scalar_type() == at::kLong,
+              "wait_posted: int64 slots (one per producer) and an int64 output word");
+  check(odc::launch_wait_posted(slots.data_ptr(), static_cast<int>(nprod), static_cast<unsigned long long>(epoch),
+                                counter.data_ptr(), static_cast<unsigned long long>(timeout_ms) * 1000000ull,
+                                status.data_ptr<int>(), reinterpret_cast<unsigned long long*>(expected_out.data_ptr()),
+                                cur_stream()),
+        "wait_posted launch");
+}
+
 // --- single-primitive test entry points: addresses are plain integers so peers' mappings can be passed
 void put_block(uintptr_t remote_dst, Tensor local_src) {
   c10::cuda::CUDAGuard g(local_src.device());
@@ -327,13 +381,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("check"), py::arg("status"), py::arg("src_region_elems") = 0);
   m.def("scatter_accumulate", &scatter_accumulate, py::arg("inp2d"), py::arg("acc_table"), py::arg("ctr_table"),
         py::arg("n"), py::arg("acc_dtype"), py::arg("my_index"), py::arg("scale"), py::arg("check"), py::arg("status"),
-        py::arg("acc_region_elems") = 0);
+        py::arg("acc_region_elems") = 0, py::arg("scale_tensor") = py::none());
   m.def("scatter_accumulate_segments", &scatter_accumulate_segments, py::arg("grads"), py::arg("chunk_numels"),
         py::arg("dst_offsets"), py::arg("acc_table"), py::arg("ctr_table"), py::arg("acc_dtype"), py::arg("my_index"),
         py::arg("scale"), py::arg("check") = false, py::arg("status") = py::none(), py::arg("acc_region_elems") = 0);
+  m.def("embedding_scatter", &embedding_scatter);
   m.def("wait_counter", &wait_counter);
   m.def("post_counts", &post_counts);
   m.def("wait_posted", &wait_posted);
+  m.def("post_and_wait", &post_and_wait);
   m.def("put_block", &put_block);
   m.def("get_block", &get_block);
   m.def("scalar_put_get", &scalar_put_get);

@@ -38,15 +38,20 @@ std::tuple<Tensor, Tensor> rmsnorm_fwd(Tensor x, Tensor w, double eps) {
   return {y, rstd};
 }
 
+// sink (fp32 [H], not with fixed_order): dw is added there and an undefined tensor comes back in its place
 std::tuple<Tensor, Tensor> rmsnorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor rstd, bool fixed_order,
-                                       c10::optional<Tensor> dres) {
+                                       c10::optional<Tensor> dres, c10::optional<Tensor> sink) {
   c10::cuda::CUDAGuard g(x.device());
   odc::bind_device(x.get_device());
   TORCH_CHECK(dy.is_contiguous() && x.is_contiguous() && dy.sizes() == x.sizes(), "rmsnorm_bwd: contiguous dy, x [T,H]");
   const int rows = static_cast<int>(x.size(0)), cols = static_cast<int>(x.size(1));
   auto dx = at::empty_like(x);
   const int grid = odc::rmsnorm_bwd_grid(rows, sm_count());
-  auto dw = at::empty({cols}, x.options().dtype(at::kFloat));
+  const bool add = sink.has_value();
+  if (add)
+    TORCH_CHECK(!fixed_order && sink->scalar_type() == at::kFloat && sink->numel() == cols && sink->is_contiguous(),
+                "rmsnorm_bwd: sink is fp32 [H]");
+  auto dw = add ? *sink : at::empty({cols}, x.options().dtype(at::kFloat));
   Tensor partial;
   float* partial_ptr = nullptr;
   if (fixed_order) {  // per-CTA column sums added up in a fixed order by a second pass (bitwise reproducible)
@@ -60,9 +65,9 @@ std::tuple<Tensor, Tensor> rmsnorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor rst
     dres_ptr = dres->data_ptr();
   }
   check(odc::launch_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(),
-                                partial_ptr, dw.data_ptr<float>(), rows, cols, grid, cur_stream(), dres_ptr),
+                                partial_ptr, dw.data_ptr<float>(), rows, cols, grid, cur_stream(), dres_ptr, add),
         "rmsnorm_bwd");
-  return {dx, dw};
+  return {dx, add ? Tensor() : dw};
 }
 
 Tensor rope_qkv(Tensor qkv, Tensor pos, int n_q, int n_kv, int head_dim, double theta, bool inverse) {
@@ -322,6 +327,19 @@ Tensor column_sum(const Tensor& x) {
   return out;
 }
 
+// bf16(in * *scale) for a one-element scale on the device; in is fp32 or bf16
+Tensor scale_to_bf16(Tensor in, Tensor scale) {
+  c10::cuda::CUDAGuard g(in.device());
+  TORCH_CHECK(in.is_contiguous() && scale.numel() == 1 && scale.is_cuda(), "scale_to_bf16: contiguous input, one device value");
+  scale = scale.to(at::kFloat);
+  auto out = at::empty(in.sizes(), in.options().dtype(at::kBFloat16));
+  check(odc::launch_scale_to_bf16(in.data_ptr(), kind_of(in.scalar_type()), out.data_ptr(), scale.data_ptr<float>(),
+                                  static_cast<size_t>(in.numel()), sm_count(), cur_stream()),
+        "scale_to_bf16");
+  count();
+  return out;
+}
+
 Tensor rows2d(const Tensor& x) { return x.dim() == 2 ? x : x.reshape({-1, x.size(-1)}); }
 Tensor like(const Tensor& y2, const Tensor& x, int64_t last) {
   if (x.dim() == 2) return y2;
@@ -382,10 +400,12 @@ struct RMSNormFn : Function<RMSNormFn> {
     c10::optional<Tensor> dres;
     if (ctx->saved_data["residual"].toBool() && grads[1].defined()) dres = rows2d(grads[1]).contiguous();
     auto it = ctx->saved_data.find("sink");
-    auto [dx, dw] = rmsnorm_bwd(dy2, x2, w, rstd, fixed, dres);
+    c10::optional<Tensor> sink;
+    if (it != ctx->saved_data.end()) sink = it->second.toTensor();
+    auto [dx, dw] = rmsnorm_bwd(dy2, x2, w, rstd, fixed, dres, fixed ? c10::nullopt : sink);
     count(fixed ? 2 : 1);
-    if (it != ctx->saved_data.end()) {
-      it->second.toTensor().add_(dw);
+    if (sink.has_value()) {
+      if (fixed) sink->add_(dw);
       dw = Tensor();
     } else if (dw.scalar_type() != w.scalar_type()) {
       dw = dw.to(w.scalar_type());
@@ -529,15 +549,14 @@ struct LinearCrossEntropyFn : Function<LinearCrossEntropyFn> {
                         int64_t ignore_index, int64_t chunk, bool need_dh, bool need_dw) {
     auto [loss, dh, dw] = lm_head_loss(h, w, labels, loss_scale, ignore_index, chunk, need_dh, need_dw, c10::nullopt);
     ctx->save_for_backward({dh, dw});
-    ctx->saved_data["dtype"] = w.scalar_type();
     return loss;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
     const Tensor& g = grads[0];
     Tensor gh, gw;
-    if (s[0].defined()) gh = s[0] * g.to(s[0].scalar_type());
-    if (s[1].defined()) gw = (s[1] * g).to(ctx->saved_data["dtype"].toScalarType());
+    if (s[0].defined()) gh = scale_to_bf16(s[0], g);
+    if (s[1].defined()) gw = scale_to_bf16(s[1], g);
     return {gh, gw, {}, {}, {}, {}, {}, {}};
   }
 };
@@ -602,6 +621,102 @@ Tensor linear_token_logprobs(Tensor h, Tensor w, Tensor ids, double temperature,
                                       wants_grad(w));
 }
 
+// ---- linear layer of the sharded engine --------------------------------------------------------------------------------
+// Contributions sent by native code since the reduction service last asked (it adds them to its own books at `sync`).
+struct DispatchCounter : torch::CustomClassHolder {
+  std::atomic<int64_t> n{0};
+  int64_t take() { return n.exchange(0); }
+};
+
+// What one row-sharded matrix needs at every call: its shard, the peers' addresses, its accumulator.
+struct ShardedMatrix : torch::CustomClassHolder {
+  int64_t id = 0;                       // how the Python side knows it
+  Tensor shard;                         // [rows_per_rank, K] bf16, in the symmetric heap
+  Tensor table, acc_table, ctr_table;   // device tables of the owners' shards / accumulators / arrival counters
+  std::vector<int64_t> acc_addrs;
+  int64_t out_features = 0, rows_per_rank = 0, world = 1, index = 0;
+  double grad_scale = 1.0;
+  bool keep_weight = false;
+  bool local_pending = false;           // earlier microbatches left a gradient in the local buffer
+  c10::intrusive_ptr<DispatchCounter> dispatched;
+  Tensor whole() const { return shard.narrow(0, 0, out_features); }
+};
+
+std::atomic<bool> g_sync_grads{true};   // false: weight gradients are accumulated on the producing rank
+py::object* g_deferred = nullptr;       // Python: (id, dy2, x2) of a gradient that is not pushed straight away
+
+// Forward is the plain product for one rank, else the product that pulls the owners' rows inside the kernel; the weight
+// gradient is added into its owners from the epilogue of its product.  The weight is no autograd input.
+struct ShardedLinearFn : Function<ShardedLinearFn> {
+  static Tensor forward(AutogradContext* ctx, Tensor x, c10::optional<Tensor> bias, c10::optional<Tensor> residual,
+                        c10::intrusive_ptr<ShardedMatrix> m, c10::optional<Tensor> bias_sink, bool need_dx, bool need_db,
+                        bool need_dres) {
+    const Tensor x2 = rows2d(x);
+    c10::optional<Tensor> res;
+    if (residual.has_value()) res = rows2d(*residual);
+    Tensor y, w_full;
+    if (m->world == 1) {
+      y = product(x2, m->whole(), kNT, bias.value_or(Tensor()), res.value_or(Tensor()));
+    } else {
+      w_full = at::empty({m->out_features, m->shard.size(1)}, m->shard.options());
+      y = gemm_gather(x2, m->table, w_full, bias, m->rows_per_rank, m->index, res);
+      count();
+    }
+    if (!m->keep_weight) w_full = Tensor();  // dropped: backward pulls the shards again
+    ctx->save_for_backward({x, w_full});
+    ctx->saved_data["need"] = static_cast<int64_t>(need_dx | need_db << 1 | need_dres << 2);
+    if (bias_sink.has_value()) ctx->saved_data["sink"] = *bias_sink;
+    ctx->saved_data["m"] = c10::IValue::make_capsule(m);
+    return like(y, x, m->out_features);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor& x = saved[0];
+    auto capsule = ctx->saved_data["m"].toCapsule();
+    auto* m = static_cast<ShardedMatrix*>(capsule.get());
+    const int64_t need = ctx->saved_data["need"].toInt();
+    const Tensor dy2 = rows2d(grads[0]).contiguous(), x2 = rows2d(x).contiguous();
+    Tensor dx, db;
+    if (need & 1) {
+      if (m->world == 1) {
+        dx = product(dy2, m->whole(), kNN);
+      } else if (saved[1].defined()) {
+        dx = product(dy2, saved[1], kNN);
+      } else {
+        auto w_full = at::empty({m->out_features, m->shard.size(1)}, m->shard.options());
+        dx = gemm_gather_dgrad(dy2, m->table, w_full, m->rows_per_rank, m->index);
+        count();
+      }
+      dx = dx.view(x.sizes());
+    }
+    if (!g_sync_grads || m->local_pending) {
+      py::gil_scoped_acquire gil;
+      (*g_deferred)(m->id, dy2, x2);
+    } else {
+      // whole 128-row tiles per owner and at most 8 owners: output boxes added by the TMA unit; else per-thread reductions
+      if (!gemm_wgrad_scatter_tma(dy2, x2, m->acc_addrs, m->ctr_table, 0, m->rows_per_rank, m->grad_scale, m->index))
+        gemm_wgrad_scatter(dy2, x2, m->acc_table, m->ctr_table, 0, m->rows_per_rank, m->grad_scale);
+      count();
+      m->dispatched->n.fetch_add(1);
+    }
+    auto sink = ctx->saved_data.find("sink");
+    if (sink != ctx->saved_data.end()) {
+      const Tensor s = sink->second.toTensor();
+      check(odc::launch_column_sum(dy2.data_ptr(), nullptr, s.data_ptr<float>(), dy2.size(0), static_cast<int>(dy2.size(1)),
+                                   cur_stream()), "column_sum");
+      count();
+    } else if (need & 2) {
+      db = column_sum(dy2);
+    }
+    return {dx, db, (need & 4) ? grads[0] : Tensor(), {}, {}, {}, {}, {}};
+  }
+};
+Tensor sharded_linear(Tensor x, c10::optional<Tensor> bias, c10::optional<Tensor> residual, c10::intrusive_ptr<ShardedMatrix> m,
+                      c10::optional<Tensor> bias_sink) {
+  const bool db = bias.has_value() && wants_grad(*bias), dres = residual.has_value() && wants_grad(*residual);
+  return ShardedLinearFn::apply(x, bias, residual, m, bias_sink, wants_grad(x), db, dres);
+}
+
 }  // namespace
 
 void register_ops(py::module_& m) {
@@ -609,7 +724,7 @@ void register_ops(py::module_& m) {
   m.def("count_launches", [](int n) { count(n); });
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("dy"), py::arg("x"), py::arg("w"), py::arg("rstd"),
-        py::arg("fixed_order") = false, py::arg("dres") = py::none());
+        py::arg("fixed_order") = false, py::arg("dres") = py::none(), py::arg("sink") = py::none());
   m.def("rope_qkv", &rope_qkv);
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);
@@ -623,7 +738,31 @@ void register_ops(py::module_& m) {
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("kernel_status", &kernel_status);
+  m.def("scale_to_bf16", &scale_to_bf16);
+  py::class_<DispatchCounter, c10::intrusive_ptr<DispatchCounter>>(m, "DispatchCounter")
+      .def(py::init([] { return c10::make_intrusive<DispatchCounter>(); }))
+      .def("take", &DispatchCounter::take);
+  py::class_<ShardedMatrix, c10::intrusive_ptr<ShardedMatrix>>(m, "ShardedMatrix")
+      .def(py::init([](int64_t id, Tensor shard, Tensor table, Tensor acc_table, Tensor ctr_table, std::vector<int64_t> acc_addrs,
+                       int64_t out_features, int64_t index, double grad_scale, bool keep_weight,
+                       c10::intrusive_ptr<DispatchCounter> dispatched) {
+        auto p = c10::make_intrusive<ShardedMatrix>();
+        p->id = id; p->shard = shard; p->table = table; p->acc_table = acc_table; p->ctr_table = ctr_table;
+        p->world = static_cast<int64_t>(acc_addrs.size());
+        p->acc_addrs = std::move(acc_addrs);
+        p->out_features = out_features; p->rows_per_rank = shard.size(0); p->index = index; p->grad_scale = grad_scale;
+        p->keep_weight = keep_weight; p->dispatched = dispatched;
+        return p;
+      }))
+      .def_readwrite("local_pending", &ShardedMatrix::local_pending);
+  m.def("set_sync_grads", [](bool on) { g_sync_grads = on; });
+  m.def("set_deferred_weight_grad", [](py::object fn) {
+    if (g_deferred == nullptr) g_deferred = new py::object();  // never destroyed: backward threads may outlive the module
+    *g_deferred = fn;
+  });
   // differentiable forms
+  m.def("sharded_linear", &sharded_linear, py::arg("x"), py::arg("bias"), py::arg("residual"), py::arg("matrix"),
+        py::arg("bias_sink") = py::none());
   m.def("linear", &linear, py::arg("x"), py::arg("w"), py::arg("bias") = py::none(), py::arg("residual") = py::none());
   m.def("rms_norm", &rms_norm, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());
   m.def("rms_norm_residual", &rms_norm_residual, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());

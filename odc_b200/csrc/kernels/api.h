@@ -20,7 +20,13 @@ cudaError_t launch_gather(const long long* peers, void* out, size_t n, int src_e
 cudaError_t launch_scatter_accumulate(const void* inp, int in_kind, const long long* accs, int acc_kind,
                                       const long long* ctrs, size_t n, int nranks, int start, float scale,
                                       unsigned int* done_slot, int sm_count, cudaStream_t stream,
-                                      int* status_for_bulk = nullptr, long long acc_len = 0);
+                                      int* status_for_bulk = nullptr, long long acc_len = 0,
+                                      const float* scale_ptr = nullptr /* device factor on top of scale, fp32 accumulators */);
+// row t of dx (bf16 [tokens, width]) times scale is added to row ids[t] of a matrix whose rows are spread over nranks
+// fp32 accumulators, rows_per_rank each; ids outside [0, vocab) are skipped; then one arrival per owner
+cudaError_t launch_embedding_scatter(const long long* ids, const void* dx, int tokens, int width, const long long* accs,
+                                     const long long* ctrs, long long rows_per_rank, long long vocab, int nranks, float scale,
+                                     unsigned int* done_slot, int sm_count, cudaStream_t stream);
 // scatter_accumulate taken straight from up to kMaxScatterSegments contiguous gradient tensors (fp32 accumulators
 // only).  The caller fills count/src/chunk/total/dst; the launcher derives tile_prefix and vec.
 constexpr int kMaxScatterSegments = 32;
@@ -53,6 +59,10 @@ cudaError_t launch_post_counts(const PostedCounts& pc, cudaStream_t stream);
 cudaError_t launch_wait_posted(const void* slots, int nprod, unsigned long long epoch, const void* ctr,
                                unsigned long long budget_ns, int* status, unsigned long long* expected_out,
                                cudaStream_t stream);
+// Both in one launch: post to every owner, then wait; afterwards the status word is copied to status_host (four ints of
+// pinned host memory), so that the caller needs a stream synchronisation and no copy to look at it.
+cudaError_t launch_post_and_wait(const PostedCounts& pc, const void* slots, int nprod, unsigned long long epoch, const void* ctr,
+                                 unsigned long long budget_ns, int* status, int* status_host, cudaStream_t stream);
 
 // ---- single-primitive test kernels (device_prims.cu) ---------------------------------------------
 cudaError_t launch_put_block(void* remote_dst, const void* local_src, size_t bytes, cudaStream_t s);
@@ -70,7 +80,7 @@ cudaError_t launch_rmsnorm_fwd(const void* x, const void* w, void* y, float* rst
 // [rows, cols] gradient that reached x through a residual connection, added to dx in the same pass
 cudaError_t launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx,
                                float* partial, float* dw, int rows, int cols, int grid, cudaStream_t stream,
-                               const void* dres = nullptr);
+                               const void* dres = nullptr, bool add = false /* dw += instead of dw = */);
 int rmsnorm_bwd_grid(int rows, int sm_count);
 cudaError_t launch_rope_qkv(const void* in, void* out, const long long* pos, int tokens, int n_q, int n_kv,
                             int head_dim, float theta, bool inverse, cudaStream_t stream);
@@ -89,6 +99,9 @@ cudaError_t launch_adamw(float* p, const void* g, int g_kind, float* m, float* v
                          int sm_count, cudaStream_t stream);
 // column sums of a bf16 [rows, cols] matrix, fp32 inside: rounded into out (bf16) or added to sink (fp32); cols % 8 == 0
 cudaError_t launch_column_sum(const void* x, void* out, float* sink, long long rows, int cols, cudaStream_t stream);
+// out (bf16) = in (fp32 or bf16) * *scale
+cudaError_t launch_scale_to_bf16(const void* in, int in_kind, void* out, const float* scale, size_t n, int sm_count,
+                                 cudaStream_t stream);
 cudaError_t launch_cast_f32_to_bf16(const float* in, void* out, size_t n, int sm_count, cudaStream_t stream);
 cudaError_t launch_sumsq(const void* x, int kind, size_t n, float* out, int sm_count, cudaStream_t stream);
 

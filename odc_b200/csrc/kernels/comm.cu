@@ -196,7 +196,8 @@ template <typename InT>
 __global__ void __launch_bounds__(kThreads)
 scatter_acc_f32_kernel(const InT* __restrict__ inp, const long long* __restrict__ accs,
                        const long long* __restrict__ ctrs, size_t n, int nranks, int start, float scale,
-                       unsigned int* done_slot, int vec_ok, long long acc_len, int* status) {
+                       unsigned int* done_slot, int vec_ok, long long acc_len, int* status, const float* scale_ptr) {
+  if (scale_ptr != nullptr) scale *= *scale_ptr;
   if (const int refused = scatter_refused(accs, ctrs, nranks, start, static_cast<long long>(n), acc_len, status)) {
     if (refused == 1) finish_and_signal(ctrs, nranks, done_slot);
     return;
@@ -307,6 +308,29 @@ scatter_acc_segments_kernel(const __grid_constant__ ScatterSegments segs, const 
       const long long e1 = min(len, e0 + kTileElems);
       for (long long j = e0 + threadIdx.x; j < e1; j += kThreads) red_add_f32(acc + j, float(src[j]) * scale);
     }
+  }
+  finish_and_signal(ctrs, nranks, done_slot);
+}
+
+// ---------------------------------------------------------------- embedding lookup, backward ------
+// Row t of the gradient goes straight to the owner of row ids[t]: T x H values move instead of the whole V x H gradient
+// matrix (67 MB instead of 1 GB at 16384 tokens of a 128256 x 2048 table).  Bound by the reductions' L2 traffic.
+__global__ void __launch_bounds__(kThreads)
+embedding_scatter_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dx, int tokens, int width,
+                         const long long* __restrict__ accs, const long long* __restrict__ ctrs, long long rows_per_rank,
+                         long long vocab, int nranks, float scale, unsigned int* done_slot) {
+  const int per_row = width / 8;
+  const long long total = static_cast<long long>(tokens) * per_row;
+  for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<long long>(gridDim.x) * blockDim.x) {
+    const int t = static_cast<int>(i / per_row), c = static_cast<int>(i % per_row) * 8;
+    const long long id = ids[t];
+    if (id < 0 || id >= vocab) continue;
+    const int owner = static_cast<int>(id / rows_per_rank);
+    float* dst = reinterpret_cast<float*>(accs[owner]) + (id - owner * rows_per_rank) * width + c;
+    const uint4 u = *reinterpret_cast<const uint4*>(dx + static_cast<long long>(t) * width + c);
+    red_add_v4_f32(dst, bf16_lo(u.x) * scale, bf16_hi(u.x) * scale, bf16_lo(u.y) * scale, bf16_hi(u.y) * scale);
+    red_add_v4_f32(dst + 4, bf16_lo(u.z) * scale, bf16_hi(u.z) * scale, bf16_lo(u.w) * scale, bf16_hi(u.w) * scale);
   }
   finish_and_signal(ctrs, nranks, done_slot);
 }
@@ -432,9 +456,10 @@ __global__ void post_counts_kernel(const __grid_constant__ PostedCounts pc) {
     asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(pc.slot_addr[i]), "l"(pc.value[i]) : "memory");
 }
 
-__global__ void wait_posted_kernel(const unsigned long long* slots, int nprod, unsigned long long epoch,
-                                   const unsigned long long* ctr, unsigned long long budget_ns, int* status,
-                                   unsigned long long* expected_out) {
+// one warp; returns in lane 0 only
+__device__ __forceinline__ void collect_and_wait(const unsigned long long* slots, int nprod, unsigned long long epoch,
+                                                 const unsigned long long* ctr, unsigned long long budget_ns, int* status,
+                                                 unsigned long long* expected_out) {
   const int lane = threadIdx.x;
   unsigned long long sum = 0;
   bool ok = true;
@@ -460,6 +485,25 @@ __global__ void wait_posted_kernel(const unsigned long long* slots, int nprod, u
     const uint64_t spent = globaltimer_ns() - t0;
     bounded_wait_ge(ctr, sum, budget_ns > spent ? budget_ns - spent : 0, status, /*detail=*/0);
   }
+}
+
+__global__ void wait_posted_kernel(const unsigned long long* slots, int nprod, unsigned long long epoch,
+                                   const unsigned long long* ctr, unsigned long long budget_ns, int* status,
+                                   unsigned long long* expected_out) {
+  collect_and_wait(slots, nprod, epoch, ctr, budget_ns, status, expected_out);
+}
+
+// Post, collect, wait and hand the status word to the host: what `sync` does, as one launch of one warp (it was two
+// launches and a device-to-host copy; each costs the host about 3 us and the stream 2 us, and the copy as much again).
+__global__ void post_and_wait_kernel(const __grid_constant__ PostedCounts pc, const unsigned long long* slots, int nprod,
+                                     unsigned long long epoch, const unsigned long long* ctr, unsigned long long budget_ns,
+                                     int* status, int* status_host) {
+  for (int i = threadIdx.x; i < pc.n; i += 32)
+    asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(pc.slot_addr[i]), "l"(pc.value[i]) : "memory");
+  __syncwarp();
+  collect_and_wait(slots, nprod, epoch, ctr, budget_ns, status, nullptr);
+  __syncwarp();
+  if (threadIdx.x < 4) reinterpret_cast<volatile int*>(status_host)[threadIdx.x] = reinterpret_cast<volatile int*>(status)[threadIdx.x];
 }
 
 int grid_for(size_t tiles, int sm_count) {
@@ -499,8 +543,9 @@ cudaError_t launch_gather(const long long* peers, void* out, size_t n, int src_e
 cudaError_t launch_scatter_accumulate(const void* inp, int in_kind, const long long* accs, int acc_kind,
                                       const long long* ctrs, size_t n, int nranks, int start, float scale,
                                       unsigned int* done_slot, int sm_count, cudaStream_t stream, int* status_for_bulk,
-                                      long long acc_len) {
+                                      long long acc_len, const float* scale_ptr) {
   if (nranks == 0) return cudaSuccess;
+  if (scale_ptr != nullptr && acc_kind != kF32) return cudaErrorInvalidValue;
   const size_t tiles = ((n / 4 + kTileVecs - 1) / kTileVecs + 1) * nranks;
   const int grid = grid_for(tiles, sm_count);
   const int vec_ok = ((n % 4) == 0 || nranks == 1) && (reinterpret_cast<uintptr_t>(inp) % 16) == 0;
@@ -510,7 +555,7 @@ cudaError_t launch_scatter_accumulate(const void* inp, int in_kind, const long l
     const char* e = getenv("ODC_SCATTER_BULK");
     return e != nullptr && e[0] == '1';
   }();
-  if (bulk_enabled && acc_kind == kF32 && in_kind == kF32 && scale == 1.0f && (n % 4) == 0 && n * sizeof(float) >= 65536 &&
+  if (bulk_enabled && acc_kind == kF32 && in_kind == kF32 && scale == 1.0f && scale_ptr == nullptr && (n % 4) == 0 && n * sizeof(float) >= 65536 &&
       (reinterpret_cast<uintptr_t>(inp) % 16) == 0) {
     static bool attr_set = false;
     if (!attr_set) {
@@ -525,17 +570,28 @@ cudaError_t launch_scatter_accumulate(const void* inp, int in_kind, const long l
   } else if (acc_kind == kF32 && in_kind == kF32) {
     scatter_acc_f32_kernel<float><<<grid, kThreads, 0, stream>>>(static_cast<const float*>(inp), accs, ctrs, n,
                                                                  nranks, start, scale, done_slot, vec_ok, acc_len,
-                                                                 status_for_bulk);
+                                                                 status_for_bulk, scale_ptr);
   } else if (acc_kind == kF32 && in_kind == kBF16) {
     scatter_acc_f32_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(inp), accs, ctrs, n, nranks, start, scale, done_slot, vec_ok, acc_len,
-        status_for_bulk);
+        status_for_bulk, scale_ptr);
   } else if (acc_kind == kBF16 && in_kind == kBF16) {
     scatter_acc_bf16_kernel<<<grid, kThreads, 0, stream>>>(static_cast<const __nv_bfloat16*>(inp), accs, ctrs, n,
                                                           nranks, start, scale, done_slot, acc_len, status_for_bulk);
   } else {
     return cudaErrorInvalidValue;
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_embedding_scatter(const long long* ids, const void* dx, int tokens, int width, const long long* accs,
+                                     const long long* ctrs, long long rows_per_rank, long long vocab, int nranks, float scale,
+                                     unsigned int* done_slot, int sm_count, cudaStream_t stream) {
+  if (nranks == 0) return cudaSuccess;
+  if (width % 8 != 0 || rows_per_rank <= 0) return cudaErrorInvalidValue;
+  const size_t vecs = static_cast<size_t>(tokens) * (width / 8);
+  embedding_scatter_kernel<<<grid_for((vecs + kThreads - 1) / kThreads, sm_count), kThreads, 0, stream>>>(
+      ids, static_cast<const __nv_bfloat16*>(dx), tokens, width, accs, ctrs, rows_per_rank, vocab, nranks, scale, done_slot);
   return cudaGetLastError();
 }
 
@@ -583,6 +639,14 @@ cudaError_t launch_wait_posted(const void* slots, int nprod, unsigned long long 
                                cudaStream_t stream) {
   wait_posted_kernel<<<1, 32, 0, stream>>>(static_cast<const unsigned long long*>(slots), nprod, epoch,
                                            static_cast<const unsigned long long*>(ctr), budget_ns, status, expected_out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_post_and_wait(const PostedCounts& pc, const void* slots, int nprod, unsigned long long epoch, const void* ctr,
+                                 unsigned long long budget_ns, int* status, int* status_host, cudaStream_t stream) {
+  if (pc.n < 0 || pc.n > kMaxPostedCounts || status == nullptr || status_host == nullptr) return cudaErrorInvalidValue;
+  post_and_wait_kernel<<<1, 32, 0, stream>>>(pc, static_cast<const unsigned long long*>(slots), nprod, epoch,
+                                             static_cast<const unsigned long long*>(ctr), budget_ns, status, status_host);
   return cudaGetLastError();
 }
 

@@ -481,6 +481,28 @@ cast_f32_bf16_kernel(const float* __restrict__ in, bf16* __restrict__ out, size_
     for (size_t j = nvec * 8 + threadIdx.x; j < n; j += blockDim.x) out[j] = __float2bfloat16(in[j]);
 }
 
+// out = in * *scale, one pass from fp32 or bf16 (gradients that were formed for a loss gradient of one)
+template <typename T>
+__global__ void __launch_bounds__(256)
+scale_to_bf16_kernel(const T* __restrict__ in, bf16* __restrict__ out, const float* __restrict__ scale, size_t n) {
+  const float s = *scale;
+  const size_t nvec = n / 8;
+  for (size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x; v < nvec; v += size_t(gridDim.x) * blockDim.x) {
+    float f[8];
+    if constexpr (sizeof(T) == 4) {
+      const float4 a = *reinterpret_cast<const float4*>(in + v * 8), b = *reinterpret_cast<const float4*>(in + v * 8 + 4);
+      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+    } else {
+      unpack8(*reinterpret_cast<const uint4*>(in + v * 8), f);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] *= s;
+    *reinterpret_cast<uint4*>(out + v * 8) = pack8(f);
+  }
+  if (blockIdx.x == 0)
+    for (size_t j = nvec * 8 + threadIdx.x; j < n; j += blockDim.x) out[j] = __float2bfloat16(float(in[j]) * s);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ x, size_t n, float* __restrict__ out) {
   __shared__ float red[32];
@@ -544,14 +566,16 @@ int rmsnorm_bwd_grid(int rows, int sm_count) {
   return want < g ? (want < 1 ? 1 : want) : g;
 }
 
-// partial == nullptr: single launch, the CTAs add their column sums into dw (zeroed here first; the order of the
-// additions varies from run to run).  partial = [grid, cols] scratch: per-CTA sums, then a fixed-order column pass.
+// partial == nullptr: single launch, the CTAs add their column sums into dw (zeroed here first unless `add`; the order
+// of the additions varies from run to run).  partial = [grid, cols] scratch: per-CTA sums, then a fixed-order column pass.
 cudaError_t launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, void* dx,
                                float* partial, float* dw, int rows, int cols, int grid, cudaStream_t stream,
-                               const void* dres) {
-  if (cols % 8 != 0 || cols > 8192) return cudaErrorInvalidValue;
+                               const void* dres, bool add) {
+  if (cols % 8 != 0 || cols > 8192 || (add && partial != nullptr)) return cudaErrorInvalidValue;
   cudaError_t e;
-  if (partial == nullptr) {
+  if (add) {
+    if (rows == 0) return cudaSuccess;
+  } else if (partial == nullptr) {
     e = cudaMemsetAsync(dw, 0, sizeof(float) * cols, stream);
     if (e != cudaSuccess) return e;
     if (rows == 0) return cudaSuccess;
@@ -644,6 +668,19 @@ cudaError_t launch_cast_f32_to_bf16(const float* in, void* out, size_t n, int sm
   if (n == 0) return cudaSuccess;
   cast_f32_bf16_kernel<<<cap_grid(static_cast<long long>(n / 8 + 1), 256, sm_count, 16), 256, 0, stream>>>(
       in, static_cast<bf16*>(out), n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_scale_to_bf16(const void* in, int in_kind, void* out, const float* scale, size_t n, int sm_count,
+                                 cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  const int grid = cap_grid(static_cast<long long>(n / 8 + 1), 256, sm_count, 16);
+  if (in_kind == kF32)
+    scale_to_bf16_kernel<float><<<grid, 256, 0, stream>>>(static_cast<const float*>(in), static_cast<bf16*>(out), scale, n);
+  else if (in_kind == kBF16)
+    scale_to_bf16_kernel<bf16><<<grid, 256, 0, stream>>>(static_cast<const bf16*>(in), static_cast<bf16*>(out), scale, n);
+  else
+    return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 

@@ -70,7 +70,15 @@ class SmallGroup:
         self.grad32 = torch.zeros(self.shard * self.world, dtype=torch.float32, device=device)
         self.grad_scale = 1.0 / (self.world * L.replicas())
         self.dirty = False
-        self.full.register_post_accumulate_grad_hook(self._fold)
+        # On CUDA the layers use plain views of the gathered vector and their kernels add the gradients straight into
+        # views of the fp32 buffer: no autograd slices, no low-precision gradient of the whole vector per use.
+        self.native = self.full.is_cuda and lowp_dtype == torch.bfloat16
+        self._views = {}
+        if self.native:
+            flat = self.full.detach()
+            self._views = {name: (flat[o:o + n], self.grad32[o:o + n]) for name, (o, n) in self.slots.items()}
+        else:
+            self.full.register_post_accumulate_grad_hook(self._fold)
 
     def _fold(self, leaf):
         # one low-precision gradient per backward pass; the running sum over microbatches is kept in fp32
@@ -81,6 +89,24 @@ class SmallGroup:
     def view(self, name: str, shape) -> torch.Tensor:
         o, n = self.slots[name]
         return self.full[o:o + n].view(shape)
+
+    def norm(self, x, name: str, eps: float):
+        if self.native:
+            w, sink = self._views[name]
+            return ops._ext().rms_norm(x, w, eps, sink)
+        return ops.rms_norm(x, self.view(name, (x.shape[-1],)), eps)
+
+    def norm_residual(self, x, name: str, eps: float):
+        if self.native:
+            w, sink = self._views[name]
+            return ops._ext().rms_norm_residual(x, w, eps, sink)
+        return ops.rms_norm_residual(x, self.view(name, (x.shape[-1],)), eps)
+
+    def bias(self, name: str):
+        """``(bias, fp32 buffer for its gradient or None)``"""
+        if self.native:
+            return self._views[name]
+        return self.view(name, (self.slots[name][1],)), None
 
     def flat(self):
         return self.master, self.acc, self.m, self.v, self.lowp
@@ -111,9 +137,16 @@ class SmallGroup:
         dst.copy_(flat[self.index * self.shard:(self.index + 1) * self.shard])
 
 
+def _direct(p: ShardedParameter) -> bool:
+    """True when a gradient of ``p`` can go straight to the owners: pushes are on, nothing waits in the local buffer and
+    all owners are mapped."""
+    return L.requires_gradient_sync() and not p.local_dirty and bool(p.matrix())
+
+
 class _Embedding(torch.autograd.Function):
-    """Lookup in the gathered matrix; backward scatter-adds into the producing rank's fp32 buffer and (with
-    synchronisation on) pushes that buffer to the owners.  ``anchor`` only makes autograd call backward."""
+    """Lookup in the gathered matrix; backward adds the rows into the owners' accumulators, or (synchronisation off, or
+    earlier microbatches waiting) into the producing rank's fp32 buffer, which is then pushed with synchronisation on.
+    ``anchor`` only makes autograd call backward."""
 
     @staticmethod
     def forward(ctx, ids, anchor, model):
@@ -127,6 +160,16 @@ class _Embedding(torch.autograd.Function):
         model = ctx.model
         (ids,) = ctx.saved_tensors
         p = model.embed
+        model.small.dirty = True   # the lookup's backward is the last of a pass: every norm and bias has its gradient
+        if _direct(p):
+            service, reg = L._service(), SymmBufferRegistry.get_instance()
+            ops._ext().embedding_scatter(ids.reshape(-1), dx.reshape(-1, dx.shape[-1]).contiguous(),
+                                         reg.peer_ptr_table(service.scatter_target(p.key), p.ranks),
+                                         reg.peer_ptr_table(service.counter, p.ranks), p.rows_per_rank, p.out_features,
+                                         p.grad_scale)
+            ops._count()
+            service.note_dispatch(p.ranks)
+            return None, None, None
         p.wait_push()
         buf = p.local_buffer()
         buf.index_add_(0, ids.reshape(-1), dx.reshape(-1, dx.shape[-1]).float())
@@ -146,22 +189,12 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
         p = model.head_param()
         w = model.head_full()[:p.out_features]
         if h.is_cuda:
-            T, H = h.shape
-            ext = ops._ext()
-            dh = torch.empty_like(h)
-            dw32 = torch.empty(p.out_features, H, dtype=torch.float32, device=h.device)  # written by the first chunk
-            loss = torch.zeros((), dtype=torch.float32, device=h.device)
-            logits = torch.empty(min(chunk, T), p.out_features, dtype=torch.bfloat16, device=h.device)
-            if T == 0:
-                dw32.zero_()
-            for s in range(0, T, chunk):
-                e = min(T, s + chunk)
-                lg = logits[: e - s]
-                ops.gemm(h[s:e], w, "nt", out=lg)
-                ext.ce_fwd_bwd(lg, labels[s:e], None if loss_scale is None else loss_scale[s:e], loss, ignore_index)
-                ops._count()
-                ops.gemm(lg, w, "nn", out=dh[s:e])
-                ops.gemm(lg, h[s:e], "tn", out=dw32, accumulate=s > 0)
+            # room for the owners' padding rows, so that the whole buffer can be pushed as it is
+            dw32 = torch.empty(p.world * p.rows_per_rank, h.shape[1], dtype=torch.float32, device=h.device)
+            if dw32.shape[0] > p.out_features:
+                dw32[p.out_features:].zero_()
+            loss, dh, _ = ops._ext().lm_head_loss(h, w, labels, loss_scale, ignore_index, chunk, True, True,
+                                                  dw32[:p.out_features])
         else:
             with torch.enable_grad():
                 h_ = h.detach().requires_grad_()
@@ -178,9 +211,12 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
         dh, dw32 = ctx.saved_tensors
         model = ctx.model
         p = model.head_param()
+        if _direct(p):
+            p.push_direct(dw32, dloss)
+            return ops._ext().scale_to_bf16(dh, dloss), None, None, None, None, None
         p.wait_push()
         buf = p.local_buffer()
-        buf[:p.out_features].addcmul_(dw32, dloss.to(dw32.dtype))
+        buf[:p.out_features].addcmul_(dw32[:p.out_features], dloss.to(dw32.dtype))
         p.local_dirty = True
         if p is not model.embed and L.requires_gradient_sync():
             p.push_local(side_stream=True)   # a tied matrix is pushed by the lookup's backward, which runs last
@@ -236,14 +272,14 @@ class FusedDecoderLayer(nn.Module):
     def forward(self, x, position_ids, cu_seqlens, max_seqlen):
         c, s, i = self.cfg, self.small, self.i
         T = x.shape[0]
-        h, x = ops.rms_norm_residual(x, s.view(f"layers.{i}.attn_norm.weight", (c.hidden_size,)), c.rms_eps)
-        bias = s.view(f"layers.{i}.attn.bqkv", (c.qkv_dim,)) if c.qkv_bias else None
-        qkv = self.wqkv(h, bias=bias)
+        h, x = s.norm_residual(x, f"layers.{i}.attn_norm.weight", c.rms_eps)
+        bias, sink = s.bias(f"layers.{i}.attn.bqkv") if c.qkv_bias else (None, None)
+        qkv = self.wqkv(h, bias=bias, bias_sink=sink)
         qkv = ops.rope_qkv(qkv, position_ids, c.num_heads, c.num_kv_heads, c.head_dim, c.rope_theta,
                            c.rope_inv_freq(qkv.device))
         o = ops.varlen_attention_qkv(qkv, c.num_heads, c.num_kv_heads, c.head_dim, cu_seqlens, max_seqlen, causal=True)
         x = self.wo(o.reshape(T, c.num_heads * c.head_dim), residual=x)
-        h, x = ops.rms_norm_residual(x, s.view(f"layers.{i}.mlp_norm.weight", (c.hidden_size,)), c.rms_eps)
+        h, x = s.norm_residual(x, f"layers.{i}.mlp_norm.weight", c.rms_eps)
         return self.w_down(ops.swiglu(self.w_gate_up(h)), residual=x)
 
 
@@ -286,12 +322,16 @@ class FusedDecoderLM(nn.Module):
         if source.lm_head is not None:
             self.lm_head = ShardedParameter("lm_head", tuple(source.lm_head.shape), pg, device, full=source.lm_head.data,
                                             lowp_dtype=lowp_dtype)
-        self.embed_full = torch.empty(self.embed.world * self.embed.rows_per_rank, cfg.hidden_size, dtype=lowp_dtype,
-                                      device=device)
-        self.lm_head_full = None if self.lm_head is None else torch.empty(
-            self.lm_head.world * self.lm_head.rows_per_rank, cfg.hidden_size, dtype=lowp_dtype, device=device)
+        self.embed_full = self._whole(self.embed)
+        self.lm_head_full = None if self.lm_head is None else self._whole(self.lm_head)
         self._head_fresh = False
         del source
+
+    @staticmethod
+    def _whole(p: ShardedParameter) -> torch.Tensor:
+        """Where the matrix is pulled to; with one rank the shard is the matrix and nothing is pulled."""
+        return p.lowp if p.world == 1 else torch.empty(p.world * p.rows_per_rank, p.in_features, dtype=p.lowp.dtype,
+                                                       device=p.lowp.device)
 
     # -- parameters ------------------------------------------------------------------------------------
     def head_param(self) -> ShardedParameter:
@@ -344,8 +384,9 @@ class FusedDecoderLM(nn.Module):
     def hidden_states(self, input_ids, position_ids, cu_seqlens, max_seqlen):
         with torch.no_grad():
             # one pull per microbatch, like a root FSDP unit that stays unsharded from forward to backward
-            self.gather.gather_ranks(self.embed_full, self.embed.lowp, self.embed.ranks)
-            if self.lm_head is not None:
+            if self.embed.world > 1:
+                self.gather.gather_ranks(self.embed_full, self.embed.lowp, self.embed.ranks)
+            if self.lm_head is not None and self.lm_head.world > 1:
                 self.gather.gather_ranks(self.lm_head_full, self.lm_head.lowp, self.lm_head.ranks)
         x = _Embedding.apply(input_ids, self.small.full, self)
         for layer in self.layers:
@@ -353,7 +394,7 @@ class FusedDecoderLM(nn.Module):
                 x = checkpoint(layer, x, position_ids, cu_seqlens, max_seqlen, use_reentrant=False)
             else:
                 x = layer(x, position_ids, cu_seqlens, max_seqlen)
-        return ops.rms_norm(x, self.small.view("norm.weight", (self.cfg.hidden_size,)), self.cfg.rms_eps)
+        return self.small.norm(x, "norm.weight", self.cfg.rms_eps)
 
     def forward(self, input_ids, position_ids, cu_seqlens, max_seqlen, labels=None, loss_scale=None,
                 return_logprobs: bool = False, temperature: float = 1.0):

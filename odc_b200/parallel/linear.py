@@ -20,6 +20,7 @@ same two hot paths the reference patches into FSDP (odc/fsdp/fsdp2.py:218-313 an
 from __future__ import annotations
 
 import math
+import os
 from typing import List, Optional
 
 import torch
@@ -37,6 +38,7 @@ _params: List["ShardedParameter"] = []
 _reduction: Optional[ReductionService] = None
 _next_id = 0
 _sync_grads = True
+_native = False        # a matrix of this engine has been handed to the native extension
 _replicate_pg = None   # HSDP: the group of ranks that hold the same rows as this one (None: no replication)
 
 
@@ -64,6 +66,8 @@ def set_requires_gradient_sync(flag: bool) -> None:
     """False: following backward passes accumulate weight gradients locally instead of pushing them to the owners."""
     global _sync_grads
     _sync_grads = bool(flag)
+    if _native:
+        ops._ext().set_sync_grads(_sync_grads)
 
 
 def requires_gradient_sync() -> bool:
@@ -106,9 +110,46 @@ class ShardedParameter:
         self.grad_scale = 1.0 / (self.world * replicas())
         # deferred synchronisation: unsharded fp32 gradient of this rank's own microbatches
         self.local_grad: Optional[torch.Tensor] = None
-        self.local_dirty = False
+        self._local_dirty = False
         self.push_event = None
+        self._matrix = None
         _params.append(self)
+
+    @property
+    def local_dirty(self) -> bool:
+        return self._local_dirty
+
+    @local_dirty.setter
+    def local_dirty(self, flag: bool) -> None:
+        self._local_dirty = flag
+        if self._matrix:
+            self._matrix.local_pending = flag
+
+    def reaches_other_nodes(self) -> bool:
+        return fused._spans_nodes(SymmBufferRegistry.get_instance(), self.ranks)
+
+    def matrix(self, keep_weight: bool = False):
+        """What the native layer needs of this parameter (addresses of the owners' rows, accumulators and counters), or
+        False where the data path is not the mapped heap alone (CPU ranks, groups that span nodes)."""
+        if self._matrix is None:
+            if not self.lowp.is_cuda or self.lowp.dtype != torch.bfloat16 or self.reaches_other_nodes():
+                self._matrix = False
+            else:
+                global _native
+                service, reg, ext = _service(), SymmBufferRegistry.get_instance(), ops._ext()
+                target = service.scatter_target(self.key)
+                if self.rows_per_rank * self.in_features > target.numel() or target.dtype != torch.float32:
+                    raise ValueError("parameter does not fit in its fp32 accumulator")
+                self._matrix = ext.ShardedMatrix(
+                    _params.index(self), self.lowp, reg.peer_ptr_table(self.lowp, self.ranks),
+                    reg.peer_ptr_table(target, self.ranks), reg.peer_ptr_table(service.counter, self.ranks),
+                    reg.peer_ptrs(target, self.ranks), self.out_features, self.index, self.grad_scale, keep_weight,
+                    service.native_dispatches(self.ranks))
+                self._matrix.local_pending = self._local_dirty
+                ext.set_deferred_weight_grad(_deferred_weight_grad)
+                ext.set_sync_grads(_sync_grads)
+                _native = True
+        return self._matrix
 
     # -- views -----------------------------------------------------------------------------------------
     def grad(self) -> torch.Tensor:
@@ -147,6 +188,17 @@ class ShardedParameter:
             _service().scatter_accumulate(self.key, buf.view(-1), self.pg, scale=self.grad_scale)
             buf.zero_()
         self.local_dirty = False
+
+    def push_direct(self, grad: torch.Tensor, factor: torch.Tensor) -> None:
+        """Add ``factor * grad`` into the owners' accumulators (one-sided) on the side stream; ``grad`` is a rank-major
+        fp32 gradient this microbatch has formed itself, ``factor`` one value on the device."""
+        factor = factor.to(torch.float32)
+        stream = control.get_comm_stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            _service().scatter_accumulate(self.key, grad.view(-1), self.pg, scale=self.grad_scale, scale_tensor=factor)
+        grad.record_stream(stream)
+        factor.record_stream(stream)
 
     # -- whole-matrix access (collective; checkpoints and tests) ------------------------------------------
     def full_master(self) -> torch.Tensor:
@@ -227,6 +279,12 @@ class _OdcLinearFn(torch.autograd.Function):
         return dx, db, dres, None
 
 
+def _deferred_weight_grad(i: int, dy2: torch.Tensor, x2: torch.Tensor) -> None:
+    """The native layer's way back for a gradient that is accumulated locally, or that follows one that was."""
+    with torch.no_grad():
+        accumulate_weight_grad(_params[i], dy2, x2)
+
+
 def accumulate_weight_grad(p: ShardedParameter, dy2: torch.Tensor, x2: torch.Tensor) -> None:
     """``dW = dy2.T @ x2`` of one microbatch: straight into the owners (fused epilogue), or into the local buffer."""
     if _sync_grads:
@@ -262,8 +320,16 @@ class OdcLinear(nn.Module):
     def grad_scale(self) -> float:
         return self.weight.grad_scale
 
-    def forward(self, x, bias=None, residual=None):
-        return _OdcLinearFn.apply(x, bias if bias is not None else self.bias, residual, self)
+    def forward(self, x, bias=None, residual=None, bias_sink=None):
+        """``bias_sink``: fp32 vector the kernel adds the bias gradient to (native layer only; the bias then gets none)."""
+        bias = bias if bias is not None else self.bias
+        m = self.weight._matrix
+        if m is None:
+            m = self.weight.matrix(self.keep_weight)
+        if m and x.is_cuda and os.environ.get("ODC_WGRAD_SCATTER", "tma") == "tma":
+            return ops._ext().sharded_linear(x, bias, residual, m, bias_sink)
+        assert bias_sink is None
+        return _OdcLinearFn.apply(x, bias, residual, self)
 
 
 def sharded_parameters() -> List[ShardedParameter]:
@@ -273,9 +339,10 @@ def sharded_parameters() -> List[ShardedParameter]:
 def start_minibatch() -> None:
     """Zero the accumulators and publish the freshly written low-precision rows (collective)."""
     _service().clear_accumulations()
-    if torch.cuda.is_available():
-        torch.cuda.current_stream().synchronize()
-    control.host_barrier()
+    if control.world_size() > 1:      # a single rank has no peer that could read or add before this point
+        if torch.cuda.is_available():
+            torch.cuda.current_stream().synchronize()
+        control.host_barrier()
 
 
 def flush_local_grads() -> None:
@@ -302,10 +369,11 @@ def finish_minibatch(lr: float = 1e-3, betas=(0.9, 0.999), eps: float = 1e-8, we
 
 
 def reset() -> None:
-    global _reduction, _next_id, _sync_grads, _replicate_pg
+    global _reduction, _next_id, _sync_grads, _replicate_pg, _native
     _layers.clear()
     _params.clear()
     _reduction = None
     _next_id = 0
-    _sync_grads = True
+    set_requires_gradient_sync(True)
+    _native = False
     _replicate_pg = None

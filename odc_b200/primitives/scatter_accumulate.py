@@ -61,6 +61,7 @@ class ReductionService:
         self.posted = self.registry.get_or_create_symm_buffer(POSTED_KEY, (max(8, control.world_size()),), torch.int64)
         self.posted.zero_()
         self.epoch = 0
+        self._native: Dict[tuple, object] = {}
         control.heartbeat()  # starts publishing (if enabled) before the barrier, so every peer is seen alive after it
         self._sync_device()
         control.host_barrier()
@@ -90,7 +91,9 @@ class ReductionService:
 
     # -- hot path ----------------------------------------------------------------------------
     def scatter_accumulate(self, key: Hashable, input: torch.Tensor, pg: Optional[dist.ProcessGroup] = None,
-                           scale: float = 1.0) -> None:
+                           scale: float = 1.0, scale_tensor: Optional[torch.Tensor] = None) -> None:
+        """``scale_tensor``: one fp32 value on the input's device, a further factor (a loss gradient the host has not
+        seen)."""
         ranks = control.group_ranks(pg)
         n = len(ranks)
         if input.dim() != 1:
@@ -107,7 +110,10 @@ class ReductionService:
         my_index = ranks.index(me)
         target = self.scatter_target(key)
         with nvtx_range("odc::scatter_accumulate"):
-            self.transport.scatter_add(input.view(n, shard), target, self.counter, ranks, my_index, scale)
+            if scale_tensor is not None and not self.transport.scales_on_device(ranks):
+                scale, scale_tensor = scale * float(scale_tensor), None
+            self.transport.scatter_add(input.view(n, shard), target, self.counter, ranks, my_index, scale,
+                                       **({} if scale_tensor is None else {"scale_tensor": scale_tensor}))
         self.note_dispatch(ranks)
 
     def scatter_accumulate_segments(self, key: Hashable, grads, chunk_numels, dst_offsets,
@@ -129,11 +135,19 @@ class ReductionService:
             self.note_dispatch(ranks)
         return done
 
-    def note_dispatch(self, ranks) -> None:
-        """Record one contribution sent to each of ``ranks`` (also used by the fused weight-gradient GEMM)."""
+    def note_dispatch(self, ranks, count: int = 1) -> None:
+        """Record ``count`` contributions sent to each of ``ranks`` (also used by the fused weight-gradient GEMM)."""
         for r in ranks:
-            self.dispatched[r] = self.dispatched.get(r, 0) + 1
-        self.calls += 1
+            self.dispatched[r] = self.dispatched.get(r, 0) + count
+        self.calls += count
+
+    def native_dispatches(self, ranks):
+        """Counter for contributions that native code sends to ``ranks``; ``sync`` adds it to :attr:`dispatched`."""
+        key = tuple(ranks)
+        if key not in self._native:
+            from .. import _ext
+            self._native[key] = _ext.load().DispatchCounter()
+        return self._native[key]
 
     def get_accumulation(self, key: Hashable) -> torch.Tensor:
         return self.accumulations[key]
@@ -146,10 +160,9 @@ class ReductionService:
         return key in self.accumulations
 
     def clear_accumulations(self) -> None:
-        for acc in self.accumulations.values():
-            acc.zero_()
-        for slots in self.slots.values():
-            slots.zero_()
+        every = [*self.accumulations.values(), *self.slots.values()]
+        if every:
+            torch._foreach_zero_(every)   # a few launches for all parameters instead of one each
 
     # -- once per minibatch ------------------------------------------------------------------
     def sync(self, pg: Optional[dist.ProcessGroup] = None, payload=None) -> list:
@@ -161,14 +174,17 @@ class ReductionService:
         with nvtx_range("odc::scatter_accumulate_sync"):
             me = control.rank()
             world = list(range(control.world_size()))
+            for ranks, counter in self._native.items():
+                sent = counter.take()
+                if sent:
+                    self.note_dispatch(ranks, sent)
             self.epoch += 1
             control.check_peers_alive()  # host-side liveness first: a rank that left is reported, not waited for
             if payload is None and config.sync_by_posting() and self.transport.supports_posting(world):
                 # No host collective: every producer stores its cumulative count on each owner, and the owner's
                 # wait collects the postings of this synchronisation before it waits for the arrivals themselves.
-                self.transport.post_counts(self.posted, world, me, self.epoch,
-                                           [self.dispatched.get(r, 0) for r in world])
-                self.transport.wait_posted(self.posted, self.counter, len(world), self.epoch)
+                self.transport.post_and_wait(self.posted, world, me, self.epoch,
+                                             [self.dispatched.get(r, 0) for r in world], self.counter)
                 self.expected_total = None  # summed on the device; not brought back to the host
                 gathered = [(None, None)] * len(world)
             else:

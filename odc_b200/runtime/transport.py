@@ -38,6 +38,10 @@ class Transport:
         """``acc on ranks[i] += scale * inp2d[i]``, then one arrival on each owner's counter."""
         raise NotImplementedError
 
+    def scales_on_device(self, ranks: Sequence[int]) -> bool:
+        """True when ``scatter_add`` to these ranks also takes a factor held in a device tensor (``scale_tensor``)."""
+        return False
+
     def wait_arrivals(self, counter_local: torch.Tensor, expected: int) -> None:
         """Return once the local arrival counter has reached ``expected`` (bounded)."""
         raise NotImplementedError
@@ -66,6 +70,12 @@ class Transport:
     def wait_posted(self, slots_local: torch.Tensor, counter_local: torch.Tensor, nprod: int, epoch: int) -> None:
         """Collect one posting of ``epoch`` from each of ``nprod`` producers, then wait for that many arrivals."""
         raise NotImplementedError
+
+    def post_and_wait(self, slots_local: torch.Tensor, ranks: Sequence[int], my_slot: int, epoch: int, counts: Sequence[int],
+                      counter_local: torch.Tensor) -> None:
+        """``post_counts`` to ``ranks``, then ``wait_posted`` for as many producers."""
+        self.post_counts(slots_local, ranks, my_slot, epoch, counts)
+        self.wait_posted(slots_local, counter_local, len(ranks), epoch)
 
 
 class HostShmTransport(Transport):
@@ -168,11 +178,15 @@ class NvlinkP2PTransport(Transport):
                         self.status, src_local.numel())
         self.launches += 1
 
-    def scatter_add(self, inp2d, acc_local, counter_local, ranks, my_index, scale=1.0):
+    def scales_on_device(self, ranks):
+        return True
+
+    def scatter_add(self, inp2d, acc_local, counter_local, ranks, my_index, scale=1.0, scale_tensor=None):
         acc_table = self.registry.peer_ptr_table(acc_local, ranks)
         ctr_table = self.registry.peer_ptr_table(counter_local, ranks)
         self.ext.scatter_accumulate(inp2d, acc_table, ctr_table, inp2d.shape[1], acc_local.dtype,
-                                    my_index, float(scale), config.debug_bounds(), self.status, acc_local.numel())
+                                    my_index, float(scale), config.debug_bounds(), self.status, acc_local.numel(),
+                                    scale_tensor)
         self.launches += 1
 
     def scatter_add_segments(self, grads, chunk_numels, dst_offsets, acc_local, counter_local, ranks, my_index,
@@ -207,6 +221,15 @@ class NvlinkP2PTransport(Transport):
                              self._expected)
         self.launches += 1
         self.check()
+
+    def post_and_wait(self, slots_local, ranks, my_slot, epoch, counts, counter_local):
+        addrs = [a + 8 * my_slot for a in self.registry.peer_ptrs(slots_local, ranks)]
+        code, detail, seen = self.ext.post_and_wait(addrs, counts, epoch, slots_local, len(ranks), counter_local,
+                                                    config.wait_timeout_ms(), self.status, self._status_host)
+        self.launches += 1
+        if code != 0:
+            self.status.zero_()
+            check_status_word(code, detail, seen)
 
     def check(self) -> None:
         """Read the device status word (one small D2H copy + stream sync) and raise if a kernel gave up.
