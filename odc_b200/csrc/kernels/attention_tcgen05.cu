@@ -15,7 +15,7 @@
 // Backward: a pre-pass computes delta = rowsum(dO * O); the main kernel owns one (128 keys, kv
 // head) tile, keeps dK and dV in TMEM across all query tiles and query heads of the group, and
 // recomputes P from the saved log-sum-exp.  dQ tiles are staged in shared memory as fp32 and added into a
-// global fp32 buffer by the TMA unit (bulk reduce-add), then converted to bf16 by a post-pass.
+// global fp32 buffer by the TMA unit (bulk reduce-add), then scaled and converted to bf16 by a post-pass.
 //
 // The reference calls flash-attn 2 for this op (examples/llm_training/torch_fsdp2.py:85-103).
 #include <cuda.h>
@@ -392,24 +392,42 @@ struct BwdParams {
   int* status;
 };
 
+// One CTA owns (128 keys, kv head) and walks the query tiles of all heads of the group.  Scores are formed transposed
+// (S^T = K Q^T, keys in the TMEM lanes), so P^T is written back to tensor memory as the A operand of dV += P^T dO and
+// dS^T goes to shared memory once, where dK reads it K-major and dQ reads the same bytes MN-major.
+//   warp 0       TMA producer of Q / dO, and the log-sum-exp and delta of the tile's queries into shared memory
+//   warp 1       MMA issuer
+//   warps 2-9    P and dS: two warpgroups, each takes 64 of the 128 query columns
+//   warps 10-13  dQ tile from tensor memory -> fp32 staging -> TMA reduce-add
+// Every product of one tile runs under another step of the pipeline: S(i+1) is issued as soon as P(i) exists, dK(i) runs
+// while dQ(i) is read out, the exponentials of tile i+1 run under dQ(i), dK(i) and dP(i+1).  With one chain per tile
+// (scores -> P, dS -> dK, dV, dQ -> read-out) the tensor cores sat idle through every element-wise step: 32768 tokens,
+// 40 query and 8 key/value heads, D = 128: forward + backward 54.3 ms then, 42.4 ms with this pipeline.
+// Bound: shared memory.  At D = 128 the four products with both operands there read 256 KiB per tile at 128 B/clk, which
+// is also the tensor cores' time for them; staging and loads add 256 KiB.
 template <int D>
 struct BwdCfg {
-  static constexpr int kStages = (D == 64) ? 2 : 1;
-  static constexpr int kTile = 128 * D * 2;            // one [128][D] bf16 operand
-  static constexpr int kStageBytes = 2 * kTile;        // Q_i and dO_i
-  static constexpr int kPBytes = 128 * 128 * 2;
-  // fp32 staging tile for the dQ reduction: D = 64 has room for its own 32 KiB, so the next P/dS can be written
-  // while the TMA unit still reads it; D = 128 reuses the (consumed) P and dS buffers
-  static constexpr int kDqStageBytes = (D == 64) ? 128 * 64 * 4 : 0;
-  static constexpr int kSmem = 2 * kTile + kStages * kStageBytes + 2 * kPBytes + kDqStageBytes + 1024 + 256;
+  static constexpr int kQStages = 2;                       // Q(i+1) feeds S(i+1) while dK(i) still reads Q(i)
+  static constexpr int kDoStages = (D == 64) ? 2 : 1;      // shared memory is full at D = 128
+  static constexpr int kTile = 128 * D * 2;                // one [128][D] bf16 operand
+  static constexpr int kDsBytes = 128 * 128 * 2;
+  static constexpr int kStageBytes = 2 * 16384;            // two [128][32] fp32 boxes of the dQ reduction
+  static constexpr int kStatBytes = kQStages * 2 * 128 * 4;
+  static constexpr int kBarBytes = 256;
+  // the dynamic window starts 1024-byte aligned in practice; the kernel checks and reports otherwise
+  static constexpr int kAlignSlack = 768;
+  static constexpr int kSmem =
+      (2 + kQStages + kDoStages) * kTile + kDsBytes + kStageBytes + kStatBytes + kBarBytes + kAlignSlack;
+  // tensor memory columns.  D = 64 has room for P and dQ of their own; D = 128 fills all 512: P takes over the score
+  // columns it came from and dQ the columns of the consumed dP
+  static constexpr int kS = 0, kDp = 128, kDv = 256, kDk = 256 + D;
+  static constexpr bool kPrivate = (D == 64);
+  static constexpr int kDq = kPrivate ? 384 : kDp;
+  __host__ __device__ static constexpr int p_col(int half) { return kPrivate ? 448 + 32 * half : kS + 64 * half; }
 };
+static_assert(BwdCfg<128>::kSmem <= 232448, "shared memory of one CTA");
 
-__device__ __forceinline__ void red_add_v4_gpu(float* p, float a, float b, float c, float d) {
-  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
-
-constexpr int kBwdThreads = 32 * (2 + 8);  // TMA warp, MMA warp, two compute warpgroups (each takes half of the columns)
+constexpr int kBwdThreads = 32 * (2 + 8 + 4);
 
 template <int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
@@ -430,28 +448,25 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw);
-  const uint32_t k_smem = base, v_smem = base + C::kTile;
-  const uint32_t ring = v_smem + C::kTile;
-  const uint32_t p_smem = ring + C::kStages * C::kStageBytes;
-  const uint32_t ds_smem = p_smem + C::kPBytes;
-  uint8_t* p_ptr = smem + 2 * C::kTile + C::kStages * C::kStageBytes;
-  uint8_t* ds_ptr = p_ptr + C::kPBytes;
-  constexpr bool kOwnStage = C::kDqStageBytes > 0;
-  uint8_t* stage_ptr = kOwnStage ? ds_ptr + C::kPBytes : p_ptr;
-  const uint32_t stage_smem = kOwnStage ? ds_smem + C::kPBytes : p_smem;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ds_ptr + C::kPBytes + C::kDqStageBytes);
+  if (base - raw > static_cast<uint32_t>(C::kAlignSlack)) {  // cannot happen with a 1024-aligned window
+    if (threadIdx.x == 0) report(p.status, kErrBounds, 41, static_cast<int>(base - raw));
+    return;
+  }
+  constexpr int kQOff = 2 * C::kTile, kDoOff = kQOff + C::kQStages * C::kTile, kDsOff = kDoOff + C::kDoStages * C::kTile;
+  constexpr int kStageOff = kDsOff + C::kDsBytes, kStatOff = kStageOff + C::kStageBytes, kBarOff = kStatOff + C::kStatBytes;
+  const uint32_t k_smem = base, v_smem = base + C::kTile, ds_smem = base + kDsOff;
+  float* stats = reinterpret_cast<float*>(smem + kStatOff);  // [stage][-log2(e) * lse, delta][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kBarOff);
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t kv_full = bar0;
-  const uint32_t qdo_full0 = bar0 + 8;                      // [kStages]
-  const uint32_t qdo_empty0 = qdo_full0 + 8 * C::kStages;   // [kStages]
-  const uint32_t sdp_full = qdo_empty0 + 8 * C::kStages;
-  const uint32_t pds_full = sdp_full + 8;
-  const uint32_t dq_full = pds_full + 8;
-  const uint32_t dq_read = dq_full + 8;
-  const uint32_t dkv_full = dq_read + 8;
-  const uint32_t stg_ready = dkv_full + 8;  // dQ staging tile written by all compute warps
-  const uint32_t stg_free = stg_ready + 8;  // TMA has finished reading the staging tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 8);
+  const uint32_t q_full0 = bar0 + 8, q_empty0 = bar0 + 24, do_full0 = bar0 + 40, do_empty0 = bar0 + 56, stat_full0 = bar0 + 72;
+  const uint32_t s_full = bar0 + 88;    // S^T of this tile is complete
+  const uint32_t p_full = bar0 + 96;    // P^T is in tensor memory, the scores have been read
+  const uint32_t dp_full = bar0 + 104;  // dP^T is complete
+  const uint32_t ds_full = bar0 + 112;  // dS^T is in shared memory, dP^T has been read
+  const uint32_t ds_empty = bar0 + 120; // dK and dQ have read dS^T
+  const uint32_t dq_full = bar0 + 128, dq_read = bar0 + 136, dkv_full = bar0 + 144;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -459,17 +474,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int s = 0; s < C::kStages; ++s) {
-      mbar_init(qdo_full0 + 8 * s, 1);
-      mbar_init(qdo_empty0 + 8 * s, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(q_full0 + 8 * s, 1);
+      mbar_init(q_empty0 + 8 * s, 1);
+      mbar_init(do_full0 + 8 * s, 1);
+      mbar_init(do_empty0 + 8 * s, 1);
+      mbar_init(stat_full0 + 8 * s, 1);
     }
-    mbar_init(sdp_full, 1);
-    mbar_init(pds_full, 8);
+    mbar_init(s_full, 1);
+    mbar_init(p_full, 8);
+    mbar_init(dp_full, 1);
+    mbar_init(ds_full, 8);
+    mbar_init(ds_empty, 1);
     mbar_init(dq_full, 1);
-    mbar_init(dq_read, 8);
+    mbar_init(dq_read, 4);
     mbar_init(dkv_full, 1);
-    mbar_init(stg_ready, 8);
-    mbar_init(stg_free, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -481,11 +500,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tm_s = tmem_base, tm_dp = tmem_base + 128, tm_dv = tmem_base + 256, tm_dk = tmem_base + 256 + D;
-  // D = 64 leaves room for a private dQ tile, so the next S/dP can be issued while dQ is read out;
-  // D = 128 fills all 512 columns and dQ_i reuses the score columns once the scores have been consumed
-  constexpr bool kPrivateDq = (D == 64);
-  const uint32_t tm_dq = kPrivateDq ? tmem_base + 384 : tm_s;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -497,198 +511,275 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         tma_load_2d(k_smem + s * 16384, &tmap_k, kv_full, kv_head * D + 64 * s, seq_start + kv0);
         tma_load_2d(v_smem + s * 16384, &tmap_v, kv_full, kv_head * D + 64 * s, seq_start + kv0);
       }
-      bool ok = true;
-      for (int it = 0; it < total_iters && ok; ++it) {
-        const int head = kv_head * rep + it / iters_per_head;
-        const int i = i_first + it % iters_per_head;
-        const int st = it % C::kStages;
-        if (!(ok = mbar_wait(qdo_empty0 + 8 * st, ((it / C::kStages) & 1) ^ 1, wc, 31))) break;
-        const uint32_t bar = qdo_full0 + 8 * st;
-        mbar_arrive_expect_tx(bar, C::kStageBytes);
-        const uint32_t q_dst = ring + st * C::kStageBytes, do_dst = q_dst + C::kTile;
-        const int row = seq_start + i * 128;
+    }
+    int head = kv_head * rep, i = i_first;
+    for (int it = 0; it < total_iters; ++it) {
+      const int qs = it % C::kQStages, os = it % C::kDoStages;
+      const int row = seq_start + i * 128;
+      // a free Q stage also means that this slot's statistics have been read: dS was made from them
+      if (!__all_sync(0xffffffffu, mbar_wait(q_empty0 + 8 * qs, ((it / C::kQStages) & 1) ^ 1, wc, 31))) break;
+      if (lane == 0) {
+        const uint32_t bar = q_full0 + 8 * qs, dst = base + kQOff + qs * C::kTile;
+        mbar_arrive_expect_tx(bar, C::kTile);
 #pragma unroll
-        for (int s = 0; s < D / 64; ++s) {
-          tma_load_2d(q_dst + s * 16384, &tmap_q, bar, head * D + 64 * s, row);
-          tma_load_2d(do_dst + s * 16384, &tmap_do, bar, head * D + 64 * s, row);
-        }
+        for (int s = 0; s < D / 64; ++s) tma_load_2d(dst + s * 16384, &tmap_q, bar, head * D + 64 * s, row);
       }
+      float nl[4], dl[4];
+      const long long first = static_cast<long long>(head) * p.total_tokens + row;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int c = lane + 32 * e;
+        const bool in = i * 128 + c < seq_len;
+        nl[e] = in ? -kLog2e * p.lse[first + c] : 0.f;
+        dl[e] = in ? p.delta[first + c] : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        stats[qs * 256 + lane + 32 * e] = nl[e];
+        stats[qs * 256 + 128 + lane + 32 * e] = dl[e];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(stat_full0 + 8 * qs);
+      if (!__all_sync(0xffffffffu, mbar_wait(do_empty0 + 8 * os, ((it / C::kDoStages) & 1) ^ 1, wc, 30))) break;
+      if (lane == 0) {
+        const uint32_t bar = do_full0 + 8 * os, dst = base + kDoOff + os * C::kTile;
+        mbar_arrive_expect_tx(bar, C::kTile);
+#pragma unroll
+        for (int s = 0; s < D / 64; ++s) tma_load_2d(dst + s * 16384, &tmap_do, bar, head * D + 64 * s, row);
+      }
+      if (++i == n_qblocks) { i = i_first; ++head; }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // S, dP: both operands K-major
-      const uint32_t idesc_tt = make_idesc_bf16(128, D, true, true);      // dV, dK: A^T (MN-major) x MN-major
-      const uint32_t idesc_dq = make_idesc_bf16(128, D, false, true);     // dQ: K-major x MN-major
-      bool ok = mbar_wait(kv_full, 0, wc, 32);
-      for (int it = 0; it < total_iters && ok; ++it) {
-        const int st = it % C::kStages;
-        const uint32_t q_src = ring + st * C::kStageBytes, do_src = q_src + C::kTile;
-        if (!(ok = mbar_wait(qdo_full0 + 8 * st, (it / C::kStages) & 1, wc, 33))) break;
-        if (!kPrivateDq && it > 0) {  // the score columns still hold dQ of the previous tile until it has been read out
-          if (!(ok = mbar_wait(dq_read, (it - 1) & 1, wc, 34))) break;
-        }
-        tc_fence_after();
+      const uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);  // S^T, dP^T: both operands K-major
+      const uint32_t idesc_kn = make_idesc_bf16(128, D, false, true);    // dV (A in tensor memory), dK: K-major x MN-major
+      const uint32_t idesc_nn = make_idesc_bf16(128, D, true, true);     // dQ: dS^T read MN-major x MN-major
+      auto scores = [&](uint32_t d_col, uint32_t a_smem, uint32_t b_smem) {
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k >> 2) * 16384 + (k & 3) * 32;
-          umma_f16(tm_s, make_smem_desc(q_src + off, 16, 1024), make_smem_desc(k_smem + off, 16, 1024), idesc_s,
+          umma_f16(tmem_base + d_col, make_smem_desc(a_smem + off, 16, 1024), make_smem_desc(b_smem + off, 16, 1024), idesc_s,
                    k > 0 ? 1u : 0u);
         }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * 16384 + (k & 3) * 32;
-          umma_f16(tm_dp, make_smem_desc(do_src + off, 16, 1024), make_smem_desc(v_smem + off, 16, 1024), idesc_s,
-                   k > 0 ? 1u : 0u);
-        }
-        umma_commit(sdp_full);
-        if (!(ok = mbar_wait(pds_full, it & 1, wc, 35))) break;
+      };
+      auto issue_s = [&](int it) -> bool {
+        if (!mbar_wait(q_full0 + 8 * (it % C::kQStages), (it / C::kQStages) & 1, wc, 33)) return false;
         tc_fence_after();
-        // dV += P^T dO ; dK += dS^T Q   (reduction over the 128 query rows, 16 at a time)
+        scores(C::kS, k_smem, base + kQOff + (it % C::kQStages) * C::kTile);
+        umma_commit(s_full);
+        return true;
+      };
+      auto issue_dp = [&](int it) -> bool {
+        if (!mbar_wait(do_full0 + 8 * (it % C::kDoStages), (it / C::kDoStages) & 1, wc, 29)) return false;
+        tc_fence_after();
+        scores(C::kDp, v_smem, base + kDoOff + (it % C::kDoStages) * C::kTile);
+        umma_commit(dp_full);
+        return true;
+      };
+      auto issue_dk = [&](int it) {  // dK += dS^T Q, over the 128 query rows, 16 at a time
+        const uint32_t q_src = base + kQOff + (it % C::kQStages) * C::kTile;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          umma_f16(tm_dv, make_smem_desc(p_smem + k * 2048, 16384, 1024), make_smem_desc(do_src + k * 2048, 16384, 1024),
-                   idesc_tt, (it > 0 || k > 0) ? 1u : 0u);
-        }
+        for (int k = 0; k < 8; ++k)
+          umma_f16(tmem_base + C::kDk, make_smem_desc(ds_smem + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
+                   make_smem_desc(q_src + k * 2048, 16384, 1024), idesc_kn, (it > 0 || k > 0) ? 1u : 0u);
+        umma_commit(q_empty0 + 8 * (it % C::kQStages));
+      };
+      auto issue_dq = [&]() {  // dQ = dS K, over the 128 keys
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          umma_f16(tm_dk, make_smem_desc(ds_smem + k * 2048, 16384, 1024), make_smem_desc(q_src + k * 2048, 16384, 1024),
-                   idesc_tt, (it > 0 || k > 0) ? 1u : 0u);
-        }
-        umma_commit(qdo_empty0 + 8 * st);  // Q_i / dO_i are not read again: their stage can be refilled now
-        // dQ_i = dS K   (reduction over the 128 keys)
-        if (kPrivateDq && it > 0) {  // the private dQ tile of the previous query tile must have been read out
-          if (!(ok = mbar_wait(dq_read, (it - 1) & 1, wc, 34))) break;
-          tc_fence_after();
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          umma_f16(tm_dq, make_smem_desc(ds_smem + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024),
-                   make_smem_desc(k_smem + k * 2048, 16384, 1024), idesc_dq, k > 0 ? 1u : 0u);
-        }
+        for (int k = 0; k < 8; ++k)
+          umma_f16(tmem_base + C::kDq, make_smem_desc(ds_smem + k * 2048, 16384, 1024),
+                   make_smem_desc(k_smem + k * 2048, 16384, 1024), idesc_nn, k > 0 ? 1u : 0u);
         umma_commit(dq_full);
+      };
+      bool ok = mbar_wait(kv_full, 0, wc, 32) && issue_s(0) && issue_dp(0);
+      for (int it = 0; it < total_iters && ok; ++it) {
+        const bool more = it + 1 < total_iters;
+        if (!(ok = mbar_wait(p_full, it & 1, wc, 35))) break;
+        tc_fence_after();
+        if (C::kPrivate && more && !(ok = issue_s(it + 1))) break;
+        const uint32_t do_src = base + kDoOff + (it % C::kDoStages) * C::kTile;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)  // dV += P^T dO
+          umma_f16_ts(tmem_base + C::kDv, tmem_base + C::p_col(k >> 2) + (k & 3) * 8, make_smem_desc(do_src + k * 2048, 16384, 1024),
+                      idesc_kn, (it > 0 || k > 0) ? 1u : 0u);
+        umma_commit(do_empty0 + 8 * (it % C::kDoStages));
+        if (!C::kPrivate && more) {
+          // P lies in the score columns: they are free once dV(it) is complete
+          if (!(ok = mbar_wait(do_empty0 + 8 * (it % C::kDoStages), (it / C::kDoStages) & 1, wc, 28))) break;
+          if (!(ok = issue_s(it + 1))) break;
+        }
+        if (!(ok = mbar_wait(ds_full, it & 1, wc, 27))) break;
+        tc_fence_after();
+        if (C::kPrivate) {
+          if (more && !(ok = issue_dp(it + 1))) break;
+          issue_dk(it);
+          if (it > 0 && !(ok = mbar_wait(dq_read, (it - 1) & 1, wc, 34))) break;
+          tc_fence_after();
+          issue_dq();
+          umma_commit(ds_empty);
+        } else {
+          issue_dq();
+          issue_dk(it);
+          umma_commit(ds_empty);
+          if (more) {  // dP(it+1) takes the columns that dQ(it) is read from
+            if (!(ok = mbar_wait(dq_read, it & 1, wc, 34))) break;
+            if (!(ok = issue_dp(it + 1))) break;
+          }
+        }
       }
       if (ok) umma_commit(dkv_full);
     }
-  } else {
+  } else if (warp < 10) {
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;            // which 64 of the 128 key columns this warpgroup handles
-    const int row = quad * 32 + lane;
-    const uint32_t lane_sel = static_cast<uint32_t>(quad * 32) << 16;
+    const int half = (warp - 2) >> 2;            // which 64 of the 128 query columns this warpgroup handles
+    const int row = quad * 32 + lane;            // key within the tile
+    const int kv = kv0 + row;
+    const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     bool ok = true;
-    for (int it = 0; it < total_iters && ok; ++it) {
-      const int head = kv_head * rep + it / iters_per_head;
-      const int i = i_first + it % iters_per_head;
-      const int q_rel = i * 128 + row;
-      const bool q_valid = q_rel < seq_len;
-      const long long tok = seq_start + q_rel;
-      const float lse2 = q_valid ? p.lse[static_cast<long long>(head) * p.total_tokens + tok] * kLog2e : 0.f;
-      const float dlt = q_valid ? p.delta[static_cast<long long>(head) * p.total_tokens + tok] : 0.f;
-      if (!(ok = mbar_wait(sdp_full, it & 1, wc, 36))) break;
+    int i = i_first;
+    for (int it = 0; it < total_iters; ++it) {
+      const float4* nl = reinterpret_cast<const float4*>(stats + (it % C::kQStages) * 256 + half * 64);
+      if (!(ok = mbar_wait(stat_full0 + 8 * (it % C::kQStages), (it / C::kQStages) & 1, wc, 26))) break;
+      if (!(ok = mbar_wait(s_full, it & 1, wc, 36))) break;
       tc_fence_after();
-      // the P/dS buffers double as the staging tile of the previous dQ reduction: wait until TMA has read it
-      if (!kOwnStage && it > 0) {
-        if (!(ok = mbar_wait(stg_free, (it - 1) & 1, wc, 39))) break;
-      }
-      uint32_t rs[64], rd[64];
-      tmem_ld_32x32(tm_s + lane_sel + half * 64, rs);
-      tmem_ld_32x32(tm_s + lane_sel + half * 64 + 32, rs + 32);
-      tmem_ld_32x32(tm_dp + lane_sel + half * 64, rd);
-      tmem_ld_32x32(tm_dp + lane_sel + half * 64 + 32, rd + 32);
-      tmem_ld_wait();
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        float pf[8], df[8];
-#pragma unroll
-        for (int x = 0; x < 8; ++x) {
-          const int col = half * 64 + v * 8 + x;
-          const int kv = kv0 + col;
-          const bool okk = q_valid && kv < seq_len && (!p.causal || kv <= q_rel);
-          const float pv = okk ? exp2f(fmaf(__uint_as_float(rs[v * 8 + x]), p.scale_log2, -lse2)) : 0.f;
-          pf[x] = pv;
-          df[x] = pv * (__uint_as_float(rd[v * 8 + x]) - dlt) * p.scale;
-        }
-        uint4 a, b;
-        a.x = pack2(pf[0], pf[1]); a.y = pack2(pf[2], pf[3]); a.z = pack2(pf[4], pf[5]); a.w = pack2(pf[6], pf[7]);
-        b.x = pack2(df[0], df[1]); b.y = pack2(df[2], df[3]); b.z = pack2(df[4], df[5]); b.w = pack2(df[6], df[7]);
-        const uint32_t off = swz_chunk_offset(row, half * 8 + v);
-        *reinterpret_cast<uint4*>(p_ptr + off) = a;
-        *reinterpret_cast<uint4*>(ds_ptr + off) = b;
-      }
-      tc_fence_before();
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(pds_full);
-      // dQ tile -> fp32 staging in shared memory (over the consumed P/dS buffers) -> TMA reduce-add into the
-      // global accumulator; rows past the end of the sequence are staged as zeros
-      if (!(ok = mbar_wait(dq_full, it & 1, wc, 37))) break;
-      tc_fence_after();
-      if (kOwnStage && it > 0) {  // the private staging tile of the previous query tile must have been read
-        if (!(ok = mbar_wait(stg_free, (it - 1) & 1, wc, 39))) break;
-      }
-#pragma unroll 1
-      for (int c = 0; c < D / 64; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tm_dq + lane_sel + half * (D / 2) + c * 32, r);
+      float pr[64];
+      {
+        uint32_t* r = reinterpret_cast<uint32_t*>(pr);
+        tmem_ld_32x32(lanes + C::kS + half * 64, r);
+        tmem_ld_32x32(lanes + C::kS + half * 64 + 32, r + 32);
         tmem_ld_wait();
-        const int box = half * (D / 64) + c;
+      }
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          uint4 o = q_valid ? make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]) : make_uint4(0, 0, 0, 0);
-          *reinterpret_cast<uint4*>(stage_ptr + box * 16384 + row * 128 + ((v ^ (row & 7)) << 4)) = o;
+      for (int v = 0; v < 16; ++v) {
+        const float4 l4 = nl[v];
+        pr[4 * v] = exp2f(fmaf(pr[4 * v], p.scale_log2, l4.x));
+        pr[4 * v + 1] = exp2f(fmaf(pr[4 * v + 1], p.scale_log2, l4.y));
+        pr[4 * v + 2] = exp2f(fmaf(pr[4 * v + 2], p.scale_log2, l4.z));
+        pr[4 * v + 3] = exp2f(fmaf(pr[4 * v + 3], p.scale_log2, l4.w));
+      }
+      const int q0 = i * 128;
+      if (q0 + 128 > seq_len || kv0 + 128 > seq_len || (p.causal && i * 128 < kv0 + 128)) {
+        // queries [lo, hi) of this warpgroup's columns see the key
+        const int lo = (p.causal ? kv - q0 : 0) - half * 64, hi = (kv < seq_len ? seq_len - q0 : 0) - half * 64;
+#pragma unroll
+        for (int c = 0; c < 64; ++c)
+          if (c < lo || c >= hi) pr[c] = 0.f;
+      }
+      // S(it) may be complete before dV(it-1), which reads the previous P from its own columns
+      if (C::kPrivate && it > 0 &&
+          !(ok = mbar_wait(do_empty0 + 8 * ((it - 1) % C::kDoStages), ((it - 1) / C::kDoStages) & 1, wc, 24)))
+        break;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) pk[c] = pack2(pr[32 * h + 2 * c], pr[32 * h + 2 * c + 1]);
+        tmem_st_32x16(lanes + C::p_col(half) + 16 * h, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      if (!(ok = mbar_wait(dp_full, it & 1, wc, 37))) break;
+      tc_fence_after();
+      if (it > 0 && !(ok = mbar_wait(ds_empty, (it - 1) & 1, wc, 39))) break;
+      // dS without the score scale: dK takes it in its epilogue and dQ where it is narrowed to bf16
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t r[32];
+        tmem_ld_32x32(lanes + C::kDp + half * 64 + 32 * h, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const float4 a = nl[32 + 8 * h + 2 * v], b = nl[32 + 8 * h + 2 * v + 1];
+          const float* pv = pr + 32 * h + 8 * v;
+          const uint32_t* rv = r + 8 * v;
+          uint4 o;
+          o.x = pack2(pv[0] * (__uint_as_float(rv[0]) - a.x), pv[1] * (__uint_as_float(rv[1]) - a.y));
+          o.y = pack2(pv[2] * (__uint_as_float(rv[2]) - a.z), pv[3] * (__uint_as_float(rv[3]) - a.w));
+          o.z = pack2(pv[4] * (__uint_as_float(rv[4]) - b.x), pv[5] * (__uint_as_float(rv[5]) - b.y));
+          o.w = pack2(pv[6] * (__uint_as_float(rv[6]) - b.z), pv[7] * (__uint_as_float(rv[7]) - b.w));
+          *reinterpret_cast<uint4*>(smem + kDsOff + swz_chunk_offset(row, half * 8 + 4 * h + v)) = o;
         }
       }
       tc_fence_before();
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(stg_ready);
-        mbar_arrive(dq_read);
-      }
-      if (warp == 2 && lane == 0) {  // one thread hands the staged tile to the TMA unit and frees it once read
-        if (mbar_wait(stg_ready, it & 1, wc, 40)) {
-#pragma unroll
-          for (int b2 = 0; b2 < D / 32; ++b2)
-            tma_reduce_add_2d(&tmap_dq, stage_smem + b2 * 16384, head * D + 32 * b2, seq_start + i * 128);
-          bulk_commit_group();
-          bulk_wait_group_read0();
-        }
-        mbar_arrive(stg_free);
-      }
-      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_full);
+      if (++i == n_qblocks) i = i_first;
     }
-    if (warp == 2 && lane == 0) bulk_wait_group0();
     // dK / dV of this key tile: one warpgroup writes dV, the other dK
     if (ok) ok = mbar_wait(dkv_full, 0, wc, 38);
     if (ok) {
       tc_fence_after();
-      const int kv_rel = kv0 + row;
-      const bool kv_valid = kv_rel < seq_len;
-      const long long off = static_cast<long long>(seq_start + kv_rel) * p.dkv_stride + kv_head * D;
+      const long long off = static_cast<long long>(seq_start + kv) * p.dkv_stride + kv_head * D;
       __nv_bfloat16* dst = (half == 0 ? p.dv : p.dk) + off;
-      const uint32_t src = (half == 0 ? tm_dv : tm_dk) + lane_sel;
+      const uint32_t src = lanes + (half == 0 ? C::kDv : C::kDk);
+      const float f = half == 0 ? 1.f : p.scale;
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         uint32_t r[32];
-        if (total_iters > 0) {
-          tmem_ld_32x32(src + c * 32, r);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int x = 0; x < 32; ++x) r[x] = 0;
-        }
-        if (kv_valid) {
+        tmem_ld_32x32(src + c * 32, r);
+        tmem_ld_wait();
+        if (kv < seq_len) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             uint4 o;
-            o.x = pack2(__uint_as_float(r[8 * v]), __uint_as_float(r[8 * v + 1]));
-            o.y = pack2(__uint_as_float(r[8 * v + 2]), __uint_as_float(r[8 * v + 3]));
-            o.z = pack2(__uint_as_float(r[8 * v + 4]), __uint_as_float(r[8 * v + 5]));
-            o.w = pack2(__uint_as_float(r[8 * v + 6]), __uint_as_float(r[8 * v + 7]));
+            o.x = pack2(__uint_as_float(r[8 * v]) * f, __uint_as_float(r[8 * v + 1]) * f);
+            o.y = pack2(__uint_as_float(r[8 * v + 2]) * f, __uint_as_float(r[8 * v + 3]) * f);
+            o.z = pack2(__uint_as_float(r[8 * v + 4]) * f, __uint_as_float(r[8 * v + 5]) * f);
+            o.w = pack2(__uint_as_float(r[8 * v + 6]) * f, __uint_as_float(r[8 * v + 7]) * f);
             *reinterpret_cast<uint4*>(dst + c * 32 + v * 8) = o;
           }
         }
       }
     }
+  } else {
+    // dQ tile -> fp32 staging, 32 columns at a time in two alternating boxes -> TMA reduce-add into the global accumulator;
+    // rows past the end of the sequence are staged as zeros.  A warp that gives up keeps walking the named barriers.
+    const int quad = warp & 3;
+    const int row = quad * 32 + lane;
+    const uint32_t src = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + C::kDq;
+    const bool issuer = warp == 10 && lane == 0;
+    bool ok = true;
+    int head = kv_head * rep, i = i_first;
+    for (int it = 0; it < total_iters; ++it) {
+      ok = ok && mbar_wait(dq_full, it & 1, wc, 40);
+      tc_fence_after();
+      const bool q_valid = i * 128 + row < seq_len;
+#pragma unroll 1
+      for (int c = 0; c < D / 32; c += 2) {
+        uint32_t r[64];
+        tmem_ld_32x32(src + c * 32, r);
+        tmem_ld_32x32(src + c * 32 + 32, r + 32);
+        tmem_ld_wait();
+        if (c + 2 == D / 32) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dq_read);
+        }
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          if (issuer) bulk_wait_group_read1();  // the box two steps back has been read
+          named_barrier_sync(1, 128);
+          uint8_t* box = smem + kStageOff + b * 16384 + row * 128;
+#pragma unroll
+          for (int v = 0; v < 8; ++v) {
+            const uint32_t* x = r + 32 * b + 4 * v;
+            *reinterpret_cast<uint4*>(box + ((v ^ (row & 7)) << 4)) =
+                q_valid ? make_uint4(x[0], x[1], x[2], x[3]) : make_uint4(0, 0, 0, 0);
+          }
+          fence_proxy_async();
+          named_barrier_sync(1, 128);
+          if (issuer && ok) {
+            tma_reduce_add_2d(&tmap_dq, base + kStageOff + b * 16384, head * D + 32 * (c + b), seq_start + i * 128);
+            bulk_commit_group();
+          }
+        }
+      }
+      if (++i == n_qblocks) { i = i_first; ++head; }
+    }
+    if (issuer) bulk_wait_group0();
   }
 
   tc_fence_before();
@@ -732,10 +823,10 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* _
   }
 }
 
-// acc is dense [tokens, width] fp32; dq rows are dq_stride elements apart
+// dq = bf16(acc * scale); acc is dense [tokens, width] fp32; dq rows are dq_stride elements apart
 __global__ void __launch_bounds__(256)
 cast_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long n8, int width8,
-               long long dq_stride) {
+               long long dq_stride, float scale) {
   for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < n8;
        v += static_cast<long long>(gridDim.x) * blockDim.x) {
     const float4 a = *reinterpret_cast<const float4*>(acc + v * 8);
@@ -743,7 +834,8 @@ cast_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, lo
     const long long row = v / width8;
     const int col = static_cast<int>(v % width8) * 8;
     *reinterpret_cast<uint4*>(dq + row * dq_stride + col) =
-        make_uint4(pack2(a.x, a.y), pack2(a.z, a.w), pack2(b.x, b.y), pack2(b.z, b.w));
+        make_uint4(pack2(a.x * scale, a.y * scale), pack2(a.z * scale, a.w * scale), pack2(b.x * scale, b.y * scale),
+                   pack2(b.z * scale, b.w * scale));
   }
 }
 
@@ -849,7 +941,7 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
   long long g = (n8 + 255) / 256;
   if (g > sm_count * 16) g = sm_count * 16;
   cast_dq_kernel<<<static_cast<int>(g), 256, 0, stream>>>(dq_acc, static_cast<__nv_bfloat16*>(dq), n8,
-                                                          n_q * head_dim / 8, dq_stride);
+                                                          n_q * head_dim / 8, dq_stride, scale);
   return cudaGetLastError();
 }
 

@@ -75,3 +75,27 @@ def test_attention_on_fused_qkv_matches_reference():
     torch.testing.assert_close(o.float(), want, rtol=2e-2, atol=2e-2)
     err = (qkv.grad.float() - x.grad).abs().max().item()
     assert err <= 3e-2 * max(x.grad.abs().max().item(), 1.0), err
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("lens,hq,hkv,d", [([1, 127, 128, 129], 2, 2, 64), ([385, 64, 2], 6, 2, 64), ([640], 4, 1, 64),
+                                           ([1, 127, 128, 129], 2, 2, 128), ([385, 64, 2], 6, 2, 128),
+                                           ([257, 130], 10, 2, 128), ([640], 4, 1, 128)])
+def test_attention_tile_edges(lens, hq, hkv, d, causal):
+    """Ends of tiles, odd and even numbers of heads per group, one to five tiles in each pipeline, both mask forms.
+
+    Bounds: P, dS and the outputs are bf16 (2^-9 each) inside fp32 sums, so a few times 2^-8 of a tensor's norm."""
+    from odc_b200 import _ext, ops
+    from odc_b200.ops import reference as ref
+    q, k, v, cu = _case(lens, hq, hkv, d, seed=7)
+    q, k, v = (t.detach().clone().requires_grad_() for t in (q, k, v))
+    o = ops.varlen_attention(q, k, v, cu, max(lens), causal)
+    do = torch.randn_like(o)
+    o.backward(do)
+    assert _ext.load().kernel_status()[0].item() == 0, _ext.load().kernel_status().tolist()
+    qr, kr, vr = (t.detach().double().requires_grad_() for t in (q, k, v))
+    want = ref.varlen_attention(qr, kr, vr, cu.cpu(), causal, d ** -0.5)
+    want.backward(do.double())
+    for name, got, exp in (("o", o, want), ("dq", q.grad, qr.grad), ("dk", k.grad, kr.grad), ("dv", v.grad, vr.grad)):
+        rel = ((got.double() - exp).norm() / exp.norm()).item()
+        assert rel <= 4 * 2 ** -8, (name, rel)
