@@ -192,6 +192,23 @@ def test_adamw_matches_torch(ext):
     assert torch.equal(low, p.bfloat16())
 
 
+@pytest.mark.parametrize("grad", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,skip", [(1, 0), (3, 0), (4, 0), (1025, 0), (4098, 1), (4098, 4)])
+def test_adamw_accesses(ext, n, skip, grad):
+    """Wide and element-wise accesses, remainders, arrays that start off a 16-byte boundary: the same numbers."""
+    base = [torch.rand(n + skip, device="cuda") for _ in range(3)]
+    g = torch.randn(n + skip, device="cuda").to(grad)[skip:]
+    p, m, v = (t[skip:] for t in base)
+    low = torch.zeros(n + skip, dtype=torch.bfloat16, device="cuda")[skip:]
+    pd, md, vd, gd = p.double(), m.double(), v.double(), g.double() * 0.5
+    ext.adamw_step(p, g, m, v, low, 1e-2, 0.9, 0.95, 1e-8, 0.1, 3, 0.5)
+    md, vd = 0.9 * md + 0.1 * gd, 0.95 * vd + 0.05 * gd * gd
+    pd = pd * (1 - 1e-3) - 1e-2 / (1 - 0.9 ** 3) * md / (vd.sqrt() / (1 - 0.95 ** 3) ** 0.5 + 1e-8)
+    for got, exp in ((p, pd), (m, md), (v, vd)):
+        torch.testing.assert_close(got.double(), exp, rtol=2e-5, atol=2e-6)
+    assert torch.equal(low, p.bfloat16())
+
+
 # ------------------------------------------------------------------------------------ GEMM
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (256, 512, 256), (300, 1376, 200), (1000, 264, 1032),
