@@ -108,7 +108,8 @@ Tensor swiglu_bwd(Tensor dy, Tensor gu) {
   return out;
 }
 
-void ce_fwd_bwd(Tensor logits, Tensor labels, c10::optional<Tensor> loss_scale, Tensor loss, int64_t ignore_index) {
+void ce_fwd_bwd(Tensor logits, Tensor labels, c10::optional<Tensor> loss_scale, Tensor loss, int64_t ignore_index,
+                double inv_temp) {
   c10::cuda::CUDAGuard g(logits.device());
   odc::bind_device(logits.get_device());
   TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous() && logits.scalar_type() == at::kBFloat16, "ce: logits bf16");
@@ -120,11 +121,11 @@ void ce_fwd_bwd(Tensor logits, Tensor labels, c10::optional<Tensor> loss_scale, 
   }
   check(odc::launch_ce_fwd_bwd(logits.data_ptr(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()), ls,
                                loss.data_ptr<float>(), static_cast<int>(logits.size(0)),
-                               static_cast<int>(logits.size(1)), ignore_index, cur_stream()),
+                               static_cast<int>(logits.size(1)), ignore_index, cur_stream(), static_cast<float>(inv_temp)),
         "ce_fwd_bwd");
 }
 
-void token_logprobs(Tensor logits, Tensor labels, Tensor out, int64_t ignore_index) {
+void token_logprobs(Tensor logits, Tensor labels, Tensor out, int64_t ignore_index, double inv_temp) {
   c10::cuda::CUDAGuard g(logits.device());
   odc::bind_device(logits.get_device());
   TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous() && logits.scalar_type() == at::kBFloat16, "token_logprobs: logits bf16");
@@ -134,7 +135,7 @@ void token_logprobs(Tensor logits, Tensor labels, Tensor out, int64_t ignore_ind
               "token_logprobs: one fp32 output per row");
   check(odc::launch_token_logprobs(logits.data_ptr(), reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()),
                                    out.data_ptr<float>(), static_cast<int>(logits.size(0)),
-                                   static_cast<int>(logits.size(1)), ignore_index, cur_stream()),
+                                   static_cast<int>(logits.size(1)), ignore_index, cur_stream(), static_cast<float>(inv_temp)),
         "token_logprobs");
 }
 
@@ -536,7 +537,7 @@ std::tuple<Tensor, Tensor, Tensor> lm_head_loss(const Tensor& h, const Tensor& w
     product_into(hs, w, lg, kNT);
     // in place: logits -> loss_scale * (softmax - onehot); adds the chunk's loss
     ce_fwd_bwd(lg, labels.narrow(0, s, n), loss_scale.has_value() ? c10::optional<Tensor>(loss_scale->narrow(0, s, n)) : c10::nullopt,
-               loss, ignore_index);
+               loss, ignore_index, 1.0);
     count();
     if (need_dh) product_into(lg, w, dh.narrow(0, s, n), kNN);
     if (need_dw) product_into(lg, hs, dw, kTN, {}, s > 0);
@@ -581,8 +582,7 @@ struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
       const int64_t n = std::min(chunk, T - s);
       const Tensor lg = logits.narrow(0, 0, n);
       product_into(h.narrow(0, s, n), w, lg, kNT);
-      if (temperature != 1.0) lg.mul_(1.0 / temperature);
-      token_logprobs(lg, ids.narrow(0, s, n), out.narrow(0, s, n), ignore_index);
+      token_logprobs(lg, ids.narrow(0, s, n), out.narrow(0, s, n), ignore_index, 1.0 / temperature);
       count();
     }
     ctx->save_for_backward({h, w, ids});
@@ -598,7 +598,8 @@ struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
     const int64_t T = h.size(0), chunk = cfg[1];
     Tensor dh, dw;
     if (cfg[2]) dh = at::empty_like(h);
-    if (cfg[3]) dw = at::empty(w.sizes(), w.options().dtype(at::kFloat));
+    // several chunks are summed in fp32; the product of a single one is rounded once, in its own epilogue
+    if (cfg[3]) dw = at::empty(w.sizes(), T > chunk ? w.options().dtype(at::kFloat) : w.options());
     if (T == 0 && cfg[3]) dw.zero_();
     const Tensor scale = (grads[0].reshape({-1}).to(at::kFloat) * (-1.0 / temperature)).contiguous();
     auto sink = at::zeros({}, scale.options());  // the kernel's loss output is not used here
@@ -607,8 +608,7 @@ struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
       const int64_t n = std::min(chunk, T - s);
       const Tensor hs = h.narrow(0, s, n), lg = logits.narrow(0, 0, n);
       product_into(hs, w, lg, kNT);
-      if (temperature != 1.0) lg.mul_(1.0 / temperature);
-      ce_fwd_bwd(lg, ids.narrow(0, s, n), scale.narrow(0, s, n), sink, cfg[0]);
+      ce_fwd_bwd(lg, ids.narrow(0, s, n), scale.narrow(0, s, n), sink, cfg[0], 1.0 / temperature);
       count();
       if (cfg[2]) product_into(lg, w, dh.narrow(0, s, n), kNN);
       if (cfg[3]) product_into(lg, hs, dw, kTN, {}, s > 0);
@@ -728,8 +728,10 @@ void register_ops(py::module_& m) {
   m.def("rope_qkv", &rope_qkv);
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);
-  m.def("ce_fwd_bwd", &ce_fwd_bwd);
-  m.def("token_logprobs", &token_logprobs);
+  m.def("ce_fwd_bwd", &ce_fwd_bwd, py::arg("logits"), py::arg("labels"), py::arg("loss_scale"), py::arg("loss"),
+        py::arg("ignore_index"), py::arg("inv_temp") = 1.0);
+  m.def("token_logprobs", &token_logprobs, py::arg("logits"), py::arg("labels"), py::arg("out"), py::arg("ignore_index"),
+        py::arg("inv_temp") = 1.0);
   m.def("adamw_step", &adamw_step);
   m.def("cast_f32_to_bf16", &cast_f32_to_bf16);
   m.def("sumsq", &sumsq);

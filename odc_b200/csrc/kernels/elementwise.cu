@@ -373,11 +373,14 @@ swiglu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ gu, bf16
 // one CTA per row; pass 1: online max / sum-exp; pass 2: logits <- scale * (softmax - onehot)
 // kForwardOnly: pass 1 only, the logits stay as they are and the row's log-probability of its label
 // (0 for an ignored row) goes to per_token[row]; the scale and the summed loss are not used.
+// inv_temp multiplies every logit on the way in (fp32): dividing the stored logits by a temperature would be one more
+// pass over them and a second rounding to bf16.
 constexpr int kCeThreads = 1024;
 template <bool kForwardOnly>
 __global__ void __launch_bounds__(kCeThreads)
 ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ loss_scale,
-                  float* __restrict__ loss, int vocab, long long ignore_index, float* __restrict__ per_token) {
+                  float* __restrict__ loss, int vocab, long long ignore_index, float* __restrict__ per_token,
+                  float inv_temp) {
   __shared__ float red[32];
   const int row = blockIdx.x;
   bf16* lr = logits + size_t(row) * vocab;
@@ -399,6 +402,8 @@ ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ label
   for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
     float f[8];
     unpack8(lv[v], f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] *= inv_temp;
     float mx = f[0];
 #pragma unroll
     for (int i = 1; i < 8; ++i) mx = fmaxf(mx, f[i]);
@@ -410,7 +415,7 @@ ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ label
     for (int i = 0; i < 8; ++i) s += __expf(f[i] - m);
   }
   for (int j = nvec * 8 + threadIdx.x; j < vocab; j += blockDim.x) {
-    const float f = __bfloat162float(lr[j]);
+    const float f = __bfloat162float(lr[j]) * inv_temp;
     if (f > m) {
       s *= __expf(m - f);
       m = f;
@@ -422,10 +427,10 @@ ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ label
   const float gs = block_sum(s, red);
   const float lse = gm + logf(gs);
   if constexpr (kForwardOnly) {
-    if (threadIdx.x == 0) per_token[row] = __bfloat162float(lr[label]) - lse;
+    if (threadIdx.x == 0) per_token[row] = __bfloat162float(lr[label]) * inv_temp - lse;
     return;
   }
-  if (threadIdx.x == 0) atomicAdd(loss, scale * (lse - __bfloat162float(lr[label])));
+  if (threadIdx.x == 0) atomicAdd(loss, scale * (lse - __bfloat162float(lr[label]) * inv_temp));
   __syncthreads();  // the label logit is read above before anyone overwrites it
   const float inv = 1.f / gs;
   for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
@@ -434,14 +439,14 @@ ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ label
     const int base = v * 8;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      float p = __expf(f[i] - gm) * inv;
+      float p = __expf(f[i] * inv_temp - gm) * inv;
       if (base + i == label) p -= 1.f;
       f[i] = p * scale;
     }
     lv[v] = pack8(f);
   }
   for (int j = nvec * 8 + threadIdx.x; j < vocab; j += blockDim.x) {
-    float p = __expf(__bfloat162float(lr[j]) - gm) * inv;
+    float p = __expf(__bfloat162float(lr[j]) * inv_temp - gm) * inv;
     if (j == label) p -= 1.f;
     lr[j] = __float2bfloat16(p * scale);
   }
@@ -671,21 +676,21 @@ cudaError_t launch_swiglu_bwd(const void* dy, const void* gate_up, void* dgate_u
 }
 
 cudaError_t launch_ce_fwd_bwd(void* logits, const long long* labels, const float* loss_scale, float* loss,
-                              int rows, int vocab, long long ignore_index, cudaStream_t stream) {
+                              int rows, int vocab, long long ignore_index, cudaStream_t stream, float inv_temp) {
   if (rows == 0) return cudaSuccess;
   if (vocab % 8 != 0) return cudaErrorInvalidValue;  // rows must stay 16-byte aligned
   ce_fwd_bwd_kernel<false><<<rows, kCeThreads, 0, stream>>>(static_cast<bf16*>(logits), labels, loss_scale, loss, vocab,
-                                                            ignore_index, nullptr);
+                                                            ignore_index, nullptr, inv_temp);
   return cudaGetLastError();
 }
 
 cudaError_t launch_token_logprobs(const void* logits, const long long* labels, float* per_token, int rows, int vocab,
-                                  long long ignore_index, cudaStream_t stream) {
+                                  long long ignore_index, cudaStream_t stream, float inv_temp) {
   if (rows == 0) return cudaSuccess;
   if (vocab % 8 != 0 || per_token == nullptr) return cudaErrorInvalidValue;
   // the forward-only instantiation never writes through the logits pointer
   ce_fwd_bwd_kernel<true><<<rows, kCeThreads, 0, stream>>>(static_cast<bf16*>(const_cast<void*>(logits)), labels, nullptr,
-                                                           nullptr, vocab, ignore_index, per_token);
+                                                           nullptr, vocab, ignore_index, per_token, inv_temp);
   return cudaGetLastError();
 }
 

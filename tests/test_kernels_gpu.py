@@ -305,6 +305,26 @@ def test_linear_cross_entropy_matches_reference():
 
 
 @pytest.mark.parametrize("temperature", [1.0, 0.7])
+def test_linear_token_logprobs_one_chunk(temperature):
+    """One chunk (weight gradient straight to bf16) against several (fp32 sums): apart by bf16 roundings of the gradient
+    (2^-8 of its size), and the log-probabilities by nothing."""
+    from odc_b200 import ops
+    T, H, V = 384, 256, 1032
+    h = torch.randn(T, H, device="cuda").bfloat16().requires_grad_()
+    w = (0.05 * torch.randn(V, H, device="cuda")).bfloat16().requires_grad_()
+    ids, adv = torch.randint(0, V, (T,), device="cuda"), torch.randn(T, device="cuda")
+    got = []
+    for chunk in (128, T):
+        lp = ops.linear_token_logprobs(h, w, ids, temperature, chunk=chunk)
+        got.append((lp, *torch.autograd.grad(lp, [h, w], adv)))
+    want = torch.log_softmax(h.double() @ w.double().t() / temperature, -1).gather(1, ids[:, None])[:, 0]
+    torch.testing.assert_close(got[1][0].double(), want, rtol=0, atol=2e-2)  # bf16 logits of size 4: half a spacing is 2^-7
+    for a, b in zip(*got):
+        assert a.dtype == b.dtype
+        assert ((a - b).float().norm() <= 2 ** -8 * b.float().norm()).item()
+
+
+@pytest.mark.parametrize("temperature", [1.0, 0.7])
 def test_linear_token_logprobs_matches_reference(temperature):
     """Per-token log-probabilities and both gradients against the fp32 statement of the same head; a 3-D input,
     a ragged last chunk and ignored positions included."""
