@@ -1,13 +1,12 @@
 // Causal attention over packed variable-length sequences on tcgen05 tensor cores (sm_100a).
 //
-// Forward: one CTA per (128 query rows of one sequence, query head).
-//   warp 0     TMA producer: Q tile once, then K/V tiles of 128 keys through a small ring
-//   warp 1     MMA issuer:   S = Q K^T into one of two TMEM buffers, then O += P V
-//   warps 2-5  softmax:      one query row per thread; S from TMEM, online softmax in base 2 with
+// Forward: one or two tiles of 128 query rows of one sequence per CTA.
+//   warp 0     TMA producer: Q tiles once, then K/V tiles of 128 keys through a small ring
+//   warp 1     MMA issuer:   S = Q K^T into TMEM, then O += P V
+//   warps 2-   softmax:      four warps per tile, one query row per thread; S from TMEM, online softmax in base 2 with
 //                            lazy rescaling of O (only when a row maximum grows by more than 2^8),
-//                            P written to shared memory as a 128-byte-swizzled bf16 operand
-// S(j+1) is issued before P(j) is consumed, so the tensor core computes the next score tile while
-// the softmax warps work on the current one.  K and V tiles share one TMA box shape: K is read as
+//                            P written back to TMEM as the bf16 A operand of P V
+// K and V tiles share one TMA box shape: K is read as
 // a K-major operand (Q K^T) and V as an N-major operand (P V), so nothing is transposed in memory.
 // Rows/keys outside the sequence are masked; grouped-query attention maps query head h to
 // key/value head h / (Hq/Hkv).
@@ -55,6 +54,7 @@ struct FwdParams {
   const int* cu_seqlens;
   int num_seqs;
   int n_q, n_kv;
+  int heads_per_cta;
   __nv_bfloat16* o;
   long long o_stride;
   float* lse;  // [n_q, total_tokens]
@@ -80,61 +80,95 @@ __device__ __forceinline__ bool locate_block(const int* cu, int num_seqs, int bl
   return false;
 }
 
+// Two 128-row query tiles per SM keep the exponential units and the tensor cores busy at the same time: while the softmax
+// warps of one tile work, the products of the other run.  P goes back to tensor memory as the A operand of O += P V, so
+// it costs no shared memory and no shared-memory bandwidth.
+//   D = 64:  one tile per CTA in 256 TMEM columns, two CTAs per SM (tiles of short sequences see only 1-3 key blocks: the
+//            start of one CTA hides under the other).  P has its own columns, so S(j+1) is issued as soon as S(j) has
+//            been read and runs under the exponentials of block j.
+//   D = 128: two tiles in one CTA that read the same K and V tiles: two heads of a key/value group, or with an odd number
+//            of heads per group two consecutive tiles of one head.  All 512 TMEM columns are taken: P(j) overwrites the
+//            scores it came from, and S(j+1) follows P V(j) in the tensor cores' issue order.
+// Bound by the exponentials (16 per clock and SM) and the chain around them.  With one tile per CTA and P through shared
+// memory: 32768 tokens, 32/8 heads, D = 128: 10.4 ms (848 TFLOP/s), now 8.6 ms (1019); 16210 tokens in 12 sequences,
+// 32/8 heads, D = 64: 0.707 ms, now 0.600 ms.
 template <int D>
 struct FwdCfg {
-  // D = 64: one score buffer, 256 TMEM columns and 112 KiB of shared memory, so two CTAs share an SM
-  // and hide each other's latency chains (most tiles of short sequences see only 1-3 key blocks).
-  // D = 128: two score buffers, one CTA per SM.
-  static constexpr int kStages = 2;
-  static constexpr int kSBufs = (D == 64) ? 1 : 2;
+  static constexpr int kTiles = (D == 64) ? 1 : 2;
+  static constexpr int kStages = (D == 64) ? 3 : 2;
+  static constexpr bool kPrivateP = (D == 64);
   static constexpr int kTmemCols = (D == 64) ? 256 : 512;
-  static constexpr int kOCol = kSBufs * 128;
+  static constexpr int kOCol = kTiles * 128;
+  static constexpr int kPCol = kPrivateP ? 192 : 0;
   static constexpr int kCtasPerSm = (D == 64) ? 2 : 1;
+  static constexpr int kThreads = 64 + 128 * kTiles;
   static constexpr int kQBytes = kBlockQ * D * 2;
   static constexpr int kKBytes = kBlockKV * D * 2;
   static constexpr int kStageBytes = 2 * kKBytes;
-  static constexpr int kPBytes = kBlockQ * kBlockKV * 2;
-  // barriers take 128 bytes; the alignment slack is trimmed for D = 64 so that two CTAs fit in one SM's
-  // 228 KiB (the dynamic window starts 1024-byte aligned in practice; the kernel checks and reports otherwise)
-  static constexpr int kAlignSlack = (D == 64) ? 768 : 1024;
-  static constexpr int kSmem = kQBytes + kStages * kStageBytes + kPBytes + 128 + kAlignSlack;
+  static constexpr int kBarBytes = 256;
+  // the alignment slack is trimmed so that two CTAs fit in one SM's 228 KiB (the dynamic window starts 1024-byte aligned
+  // in practice; the kernel checks and reports otherwise)
+  static constexpr int kAlignSlack = 768;
+  static constexpr int kSmem = kTiles * kQBytes + kStages * kStageBytes + kBarBytes + kAlignSlack;
 };
 
+// a * b + c on two fp32 values in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return d;
+}
+
 template <int D>
-__global__ void __launch_bounds__(192, FwdCfg<D>::kCtasPerSm)
+__global__ void __launch_bounds__(FwdCfg<D>::kThreads, FwdCfg<D>::kCtasPerSm)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
   using C = FwdCfg<D>;
-  int seq, seq_start, seq_len, q0;
-  if (!locate_block(p.cu_seqlens, p.num_seqs, blockIdx.x, kBlockQ, &seq, &seq_start, &seq_len, &q0)) return;
-  const int head = blockIdx.y;
-  const int kv_head = head / (p.n_q / p.n_kv);
-  const int kv_end = p.causal ? min(seq_len, q0 + kBlockQ) : seq_len;
-  const int n_blocks = (kv_end + kBlockKV - 1) / kBlockKV;
+  // the tiles of one CTA: heads_per_cta heads, or consecutive query tiles of one head
+  const int rows = p.heads_per_cta == C::kTiles ? kBlockQ : kBlockQ * C::kTiles;
+  int seq, seq_start, seq_len, q_first;
+  // causal: the last tiles of a sequence see the most keys, so the grid is walked from the end
+  if (!locate_block(p.cu_seqlens, p.num_seqs, gridDim.x - 1 - blockIdx.x, rows, &seq, &seq_start, &seq_len, &q_first)) return;
+  const int head0 = blockIdx.y * p.heads_per_cta;
+  const int kv_head = head0 / (p.n_q / p.n_kv);
+  auto tile_head = [&](int t) { return p.heads_per_cta == C::kTiles ? head0 + t : head0; };
+  auto tile_q0 = [&](int t) { return p.heads_per_cta == C::kTiles ? q_first : q_first + t * kBlockQ; };
+  auto tile_blocks = [&](int t) {  // key blocks that tile t sees; 0 if it lies past the end of the sequence
+    const int q0 = tile_q0(t);
+    if (q0 >= seq_len) return 0;
+    return ((p.causal ? min(seq_len, q0 + kBlockQ) : seq_len) + kBlockKV - 1) / kBlockKV;
+  };
+  const int n_blocks = max(tile_blocks(0), tile_blocks(C::kTiles - 1));
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (base - raw);
   if (base - raw > static_cast<uint32_t>(C::kAlignSlack)) {  // cannot happen with a 1024-aligned window
-    if (threadIdx.x == 0) report(p.status, kErrBounds, 40, static_cast<int>(base - raw));
+    if (threadIdx.x == 0) report(p.status, kErrBounds, 42, static_cast<int>(base - raw));
     return;
   }
   const uint32_t q_smem = base;
-  const uint32_t kv_smem = q_smem + C::kQBytes;
-  const uint32_t p_smem = kv_smem + C::kStages * C::kStageBytes;
-  uint8_t* p_ptr = smem + C::kQBytes + C::kStages * C::kStageBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p_ptr + C::kPBytes);
+  const uint32_t kv_smem = q_smem + C::kTiles * C::kQBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kTiles * C::kQBytes + C::kStages * C::kStageBytes);
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t q_full = bar0;
   const uint32_t kv_full0 = bar0 + 8;                      // [kStages]
   const uint32_t kv_empty0 = kv_full0 + 8 * C::kStages;    // [kStages]
-  const uint32_t s_full0 = kv_empty0 + 8 * C::kStages;     // [2]
-  const uint32_t s_empty0 = s_full0 + 16;                  // [2]
-  const uint32_t p_full = s_empty0 + 16;
-  const uint32_t p_empty = p_full + 8;
-  const uint32_t o_ready = p_empty + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 8);
+  const uint32_t s_full0 = kv_empty0 + 8 * C::kStages;     // [2] per tile: scores complete
+  const uint32_t s_empty0 = s_full0 + 16;                  // [2] scores have been read
+  const uint32_t p_full0 = s_empty0 + 16;                  // [2] P is in tensor memory
+  const uint32_t o_ready0 = p_full0 + 16;                  // [2] P V complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::kStages + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -146,13 +180,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       mbar_init(kv_full0 + 8 * s, 1);
       mbar_init(kv_empty0 + 8 * s, 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(s_full0 + 8 * b, 1);
-      mbar_init(s_empty0 + 8 * b, 4);
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(s_full0 + 8 * t, 1);
+      mbar_init(s_empty0 + 8 * t, 4);
+      mbar_init(p_full0 + 8 * t, 4);
+      mbar_init(o_ready0 + 8 * t, 1);
     }
-    mbar_init(p_full, 4);
-    mbar_init(p_empty, 1);
-    mbar_init(o_ready, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -164,14 +197,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s0 = tmem_base, tmem_o = tmem_base + C::kOCol;
 
   if (warp == 0) {
     if (lane == 0) {
       prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
-      mbar_arrive_expect_tx(q_full, C::kQBytes);
+      mbar_arrive_expect_tx(q_full, C::kTiles * C::kQBytes);
 #pragma unroll
-      for (int s = 0; s < D / 64; ++s) tma_load_2d(q_smem + s * 16384, &tmap_q, q_full, head * D + 64 * s, seq_start + q0);
+      for (int t = 0; t < C::kTiles; ++t)
+#pragma unroll
+        for (int s = 0; s < D / 64; ++s)  // a tile past the end of the sequence reads rows that nobody uses
+          tma_load_2d(q_smem + t * C::kQBytes + s * 16384, &tmap_q, q_full, tile_head(t) * D + 64 * s, seq_start + tile_q0(t));
       bool ok = true;
       for (int j = 0; j < n_blocks && ok; ++j) {
         const int st = j % C::kStages;
@@ -193,68 +228,66 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const uint32_t idesc_s = make_idesc_bf16(kBlockQ, kBlockKV, false, false);
       const uint32_t idesc_o = make_idesc_bf16(kBlockQ, D, false, true);
       bool ok = mbar_wait(q_full, 0, wc, 12);
-      auto issue_s = [&](int j) {
+      auto issue_s = [&](int t, int j) -> bool {
         const int st = j % C::kStages;
-        const uint32_t k_src = kv_smem + st * C::kStageBytes;
-        const uint32_t d = tmem_s0 + (j % C::kSBufs) * 128;
+        if (!mbar_wait(kv_full0 + 8 * st, (j / C::kStages) & 1, wc, 13)) return false;
+        tc_fence_after();
+        const uint32_t q_src = q_smem + t * C::kQBytes, k_src = kv_smem + st * C::kStageBytes;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k >> 2) * 16384 + (k & 3) * 32;
-          umma_f16(d, make_smem_desc(q_smem + off, 16, 1024), make_smem_desc(k_src + off, 16, 1024), idesc_s,
+          umma_f16(tmem_base + t * 128, make_smem_desc(q_src + off, 16, 1024), make_smem_desc(k_src + off, 16, 1024), idesc_s,
                    k > 0 ? 1u : 0u);
         }
-        umma_commit(s_full0 + 8 * (j % C::kSBufs));
-      };
-      // S(j+1) may overwrite its buffer once the softmax of block j+1-kSBufs has read it
-      auto issue_next_s = [&](int j) -> bool {
-        if (j + 1 >= n_blocks) return true;
-        const int st1 = (j + 1) % C::kStages;
-        if (!mbar_wait(kv_full0 + 8 * st1, ((j + 1) / C::kStages) & 1, wc, 14)) return false;
-        const int use = (j + 1) / C::kSBufs;
-        if (use >= 1 && !mbar_wait(s_empty0 + 8 * ((j + 1) % C::kSBufs), (use - 1) & 1, wc, 15)) return false;
-        tc_fence_after();
-        issue_s(j + 1);
+        umma_commit(s_full0 + 8 * t);
         return true;
       };
-      if (ok && n_blocks > 0) {
-        ok = mbar_wait(kv_full0, 0, wc, 13);
-        if (ok) { tc_fence_after(); issue_s(0); }
+      int nb[C::kTiles];
+#pragma unroll
+      for (int t = 0; t < C::kTiles; ++t) {
+        nb[t] = tile_blocks(t);
+        if (ok && nb[t] > 0) ok = issue_s(t, 0);
       }
       for (int j = 0; j < n_blocks && ok; ++j) {
-        if (C::kSBufs == 2) {  // the next score tile runs while the softmax warps work on this one
-          if (!(ok = issue_next_s(j))) break;
-        }
-        if (!(ok = mbar_wait(p_full, j & 1, wc, 16))) break;
-        tc_fence_after();
-        if (C::kSBufs == 1) {  // single buffer: free as soon as P(j) exists; queue S(j+1) ahead of P V(j)
-          if (!(ok = issue_next_s(j))) break;
-        }
         const int st = j % C::kStages;
         const uint32_t v_src = kv_smem + st * C::kStageBytes + C::kKBytes;
 #pragma unroll
-        for (int k = 0; k < kBlockKV / 16; ++k) {
-          const uint64_t da = make_smem_desc(p_smem + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024);
-          const uint64_t db = make_smem_desc(v_src + k * 2048, 16384, 1024);
-          umma_f16(tmem_o, da, db, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+        for (int t = 0; t < C::kTiles; ++t) {
+          if (ok && C::kPrivateP && j + 1 < nb[t]) {
+            ok = mbar_wait(s_empty0 + 8 * t, j & 1, wc, 15);
+            if (ok) ok = issue_s(t, j + 1);
+          }
+          if (ok && j < nb[t]) {
+            ok = mbar_wait(p_full0 + 8 * t, j & 1, wc, 16);
+            if (ok) {
+              tc_fence_after();
+#pragma unroll
+              for (int k = 0; k < kBlockKV / 16; ++k)
+                umma_f16_ts(tmem_base + C::kOCol + t * D, tmem_base + C::kPCol + t * 128 + k * 8,
+                            make_smem_desc(v_src + k * 2048, 16384, 1024), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+              umma_commit(o_ready0 + 8 * t);
+            }
+          }
+          if (t == C::kTiles - 1) umma_commit(kv_empty0 + 8 * st);
+          if (ok && !C::kPrivateP && j + 1 < nb[t]) ok = issue_s(t, j + 1);
         }
-        umma_commit(kv_empty0 + 8 * st);
-        umma_commit(p_empty);
-        umma_commit(o_ready);
       }
     }
   } else {
     // ------------------------------------------------------------------ softmax / epilogue
     const int quad = warp & 3;
+    const int t = (warp - 2) >> 2;
     const int row = quad * 32 + lane;            // query row within the tile
+    const int head = tile_head(t), q0 = tile_q0(t), nb = tile_blocks(t);
     const int q_rel = q0 + row;                  // position inside the sequence
     const bool row_valid = q_rel < seq_len;
-    const uint32_t lane_sel = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t lanes = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    const uint32_t t_s = lanes + t * 128, t_p = lanes + C::kPCol + t * 128, t_o = lanes + C::kOCol + t * D;
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_blocks && ok; ++j) {
-      if (!(ok = mbar_wait(s_full0 + 8 * (j % C::kSBufs), (j / C::kSBufs) & 1, wc, 17))) break;
+    for (int j = 0; j < nb && ok; ++j) {
+      if (!(ok = mbar_wait(s_full0 + 8 * t, j & 1, wc, 17))) break;
       tc_fence_after();
-      const uint32_t t_s = tmem_s0 + (j % C::kSBufs) * 128 + lane_sel;
       const int kv0 = j * kBlockKV;
       const bool need_mask = (kv0 + kBlockKV > seq_len) || (p.causal && kv0 + kBlockKV > q0);
       // the whole score row (128 fp32) goes to registers with one wait; max, exp and packing run from there
@@ -262,8 +295,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + c * 32, sr + c * 32);
       tmem_ld_wait();
-      // four independent chains for the row maximum (and for the row sum below): a single running value would put
-      // 128 dependent operations on the critical path of every key block
+      if (C::kPrivateP) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_empty0 + 8 * t);
+      }
+      // independent chains for the row maximum and for the row sum: a single running value would put 128 dependent
+      // operations on the critical path of every key block
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
       if (need_mask) {
         // keys [kv0, kv_hi) are visible to this row; everything from kv_hi on is masked
@@ -281,73 +319,60 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const float m_new = fmaxf(m_used, mx * p.scale_log2);
       // lazy rescale of the running output (exact: P and l keep using m_used until it is bumped)
       const bool bump = (m_new - m_used > kRescaleThreshold) || (m_used == -INFINITY && m_new > -INFINITY);
+      // P V(j-1) is complete: O may be rescaled and P overwritten
+      if (j > 0 && !(ok = mbar_wait(o_ready0 + 8 * t, (j - 1) & 1, wc, 18))) break;
       if (j == 0) {
         m_used = m_new;
       } else if (__any_sync(0xffffffffu, bump)) {
-        if (!(ok = mbar_wait(o_ready, (j - 1) & 1, wc, 18))) break;
         tc_fence_after();
         const float alpha = (m_new == -INFINITY) ? 1.f : exp2f(m_used - m_new);
 #pragma unroll 1
         for (int c = 0; c < D / 32; ++c) {
           uint32_t r[32];
-          tmem_ld_32x32(tmem_o + lane_sel + c * 32, r);
+          tmem_ld_32x32(t_o + c * 32, r);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-          tmem_st_32x16(tmem_o + lane_sel + c * 32, r);
-          tmem_st_32x16(tmem_o + lane_sel + c * 32 + 16, r + 16);
+          tmem_st_32x16(t_o + c * 32, r);
+          tmem_st_32x16(t_o + c * 32 + 16, r + 16);
         }
-        tmem_st_wait();
         l *= alpha;
         m_used = m_new;
       }
-      // P may be overwritten once the previous P V has finished reading it
-      if (j > 0) {
-        if (!(ok = mbar_wait(p_empty, (j - 1) & 1, wc, 19))) break;
-      }
       const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), sub2 = make_float2(-m_sub, -m_sub);
+      float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-      for (int v = 0; v < 16; ++v) {
-        float f[8];
+      for (int v = 0; v < 4; ++v) {
+        uint32_t pk[16];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          f[i] = exp2f(fmaf(__uint_as_float(sr[8 * v + i]), p.scale_log2, -m_sub));
-          sum4[i & 3] += f[i];
+        for (int i = 0; i < 16; ++i) {
+          const int e = 32 * v + 2 * i;
+          float2 f = fma2(make_float2(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), scale2, sub2);
+          f.x = exp2f(f.x);
+          f.y = exp2f(f.y);
+          sum2[i & 1] = add2(sum2[i & 1], f);
+          pk[i] = pack2(f.x, f.y);
         }
-        uint4 o;
-        o.x = pack2(f[0], f[1]);
-        o.y = pack2(f[2], f[3]);
-        o.z = pack2(f[4], f[5]);
-        o.w = pack2(f[6], f[7]);
-        *reinterpret_cast<uint4*>(p_ptr + swz_chunk_offset(row, v)) = o;
+        tmem_st_32x16(t_p + 16 * v, pk);
       }
-      l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      // S buffer free for block j+2; P visible to the tensor core (async proxy)
+      l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
+      tmem_st_wait();
       tc_fence_before();
-      fence_proxy_async();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(s_empty0 + 8 * (j % C::kSBufs));
-        mbar_arrive(p_full);
-      }
+      if (lane == 0) mbar_arrive(p_full0 + 8 * t);
     }
     // epilogue: O / l -> bf16, log-sum-exp
-    if (ok && n_blocks > 0) ok = mbar_wait(o_ready, (n_blocks - 1) & 1, wc, 20);
-    if (ok) {
+    if (ok && nb > 0) ok = mbar_wait(o_ready0 + 8 * t, (nb - 1) & 1, wc, 20);
+    if (ok && nb > 0) {
       tc_fence_after();
       const float inv = (l > 0.f) ? 1.f / l : 0.f;
       __nv_bfloat16* orow = p.o + static_cast<long long>(seq_start + q_rel) * p.o_stride + head * D;
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         uint32_t r[32];
-        if (n_blocks > 0) {
-          tmem_ld_32x32(tmem_o + lane_sel + c * 32, r);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = 0;
-        }
+        tmem_ld_32x32(t_o + c * 32, r);
+        tmem_ld_wait();
         if (row_valid) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
@@ -863,8 +888,12 @@ cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float
   p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.n_q = n_q; p.n_kv = n_kv;
   p.o = static_cast<__nv_bfloat16*>(o); p.o_stride = o_stride; p.lse = lse; p.total_tokens = total_tokens;
   p.scale_log2 = scale * kLog2e; p.causal = causal ? 1 : 0; p.status = status;
-  const int blocks = (total_tokens + kBlockQ - 1) / kBlockQ + num_seqs;
-  dim3 grid(blocks, n_q);
+  // D = 128 takes two heads of a key/value group per CTA: both tiles then see the same keys, and a short sequence fills
+  // both.  An odd group is walked two query tiles at a time instead.
+  const int tiles = head_dim == 64 ? FwdCfg<64>::kTiles : FwdCfg<128>::kTiles;
+  p.heads_per_cta = (n_q / n_kv) % tiles == 0 ? tiles : 1;
+  const int rows = kBlockQ * tiles / p.heads_per_cta;
+  dim3 grid((total_tokens + rows - 1) / rows + num_seqs, n_q / p.heads_per_cta);
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
@@ -875,9 +904,9 @@ cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float
   });
   if (attr_err != cudaSuccess) return attr_err;
   if (head_dim == 64)
-    attn_fwd_kernel<64><<<grid, 192, FwdCfg<64>::kSmem, stream>>>(tq, tk, tv, p);
+    attn_fwd_kernel<64><<<grid, FwdCfg<64>::kThreads, FwdCfg<64>::kSmem, stream>>>(tq, tk, tv, p);
   else
-    attn_fwd_kernel<128><<<grid, 192, FwdCfg<128>::kSmem, stream>>>(tq, tk, tv, p);
+    attn_fwd_kernel<128><<<grid, FwdCfg<128>::kThreads, FwdCfg<128>::kSmem, stream>>>(tq, tk, tv, p);
   return cudaGetLastError();
 }
 
