@@ -64,20 +64,43 @@ struct FwdParams {
   int* status;
 };
 
-// find (sequence, query block) of a linear block index; returns false if out of range
-__device__ __forceinline__ bool locate_block(const int* cu, int num_seqs, int blk, int block_rows, int* seq,
-                                             int* start, int* len, int* q0) {
-  int acc = 0;
-  for (int s = 0; s < num_seqs; ++s) {
-    const int b = cu[s], e = cu[s + 1];
-    const int nb = (e - b + block_rows - 1) / block_rows;
-    if (blk < acc + nb) {
-      *seq = s; *start = b; *len = e - b; *q0 = (blk - acc) * block_rows;
+// The idx-th tile of the pack, longest work first; false if there are fewer.  A tile's work w is the number of tiles it meets
+// under the causal mask, 1 .. n for the n tiles of a sequence (query tiles from the front, key tiles from the back), so
+// sum over sequences of max(0, n - w + 1) tiles have at least w.  Tiles of a long sequence then start before those of
+// short ones wherever it lies in the pack: started in pack order, the last long tiles ran alone (T = 8192 in one
+// sequence, 16/4 heads: SMs idle for 23 % of the forward and 36 % of the backward; 16210 tokens in 12 sequences up to 8192, 32/8 heads, D = 64:
+// forward 0.600 ms, now 0.479, backward 1.388 ms, now 1.196).  Called by whole warps.
+__device__ __forceinline__ bool locate_tile(const int* cu, int num_seqs, int idx, int tile_rows, int* start, int* len, int* work) {
+  const int lane = threadIdx.x & 31;
+  auto tiles = [&](int s) { return s < num_seqs ? (cu[s + 1] - cu[s] + tile_rows - 1) / tile_rows : 0; };
+  const int own = tiles(lane);
+  auto at_least = [&](int w) {
+    int c = max(0, own - w + 1);
+    for (int s = lane + 32; s < num_seqs; s += 32) c += max(0, tiles(s) - w + 1);
+    return __reduce_add_sync(0xffffffffu, c);
+  };
+  int longest = own;
+  for (int s = lane + 32; s < num_seqs; s += 32) longest = max(longest, tiles(s));
+  int lo = 1, hi = __reduce_max_sync(0xffffffffu, longest);
+  if (hi < 1 || idx >= at_least(1)) return false;
+  while (lo < hi) {  // the largest w that more than idx tiles reach
+    const int mid = (lo + hi + 1) / 2;
+    if (at_least(mid) > idx) lo = mid; else hi = mid - 1;
+  }
+  int rank = idx - at_least(lo + 1);
+  for (int first = 0;; first += 32) {  // the rank-th sequence with at least lo tiles
+    const bool has = (first == 0 ? own : tiles(first + lane)) >= lo;
+    const unsigned int m = __ballot_sync(0xffffffffu, has);
+    if (rank < __popc(m)) {
+      const bool mine = has && __popc(m & ((1u << lane) - 1u)) == rank;
+      const int s = first + __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+      *start = cu[s];
+      *len = cu[s + 1] - cu[s];
+      *work = lo;
       return true;
     }
-    acc += nb;
+    rank -= __popc(m);
   }
-  return false;
 }
 
 // Two 128-row query tiles per SM keep the exponential units and the tensor cores busy at the same time: while the softmax
@@ -135,10 +158,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   using C = FwdCfg<D>;
   // the tiles of one CTA: heads_per_cta heads, or consecutive query tiles of one head
   const int rows = p.heads_per_cta == C::kTiles ? kBlockQ : kBlockQ * C::kTiles;
-  int seq, seq_start, seq_len, q_first;
-  // causal: the last tiles of a sequence see the most keys, so the grid is walked from the end
-  if (!locate_block(p.cu_seqlens, p.num_seqs, gridDim.x - 1 - blockIdx.x, rows, &seq, &seq_start, &seq_len, &q_first)) return;
-  const int head0 = blockIdx.y * p.heads_per_cta;
+  // heads vary fastest: the longest tiles of all heads start first
+  const int head_groups = p.n_q / p.heads_per_cta;
+  int seq_start, seq_len, work;
+  if (!locate_tile(p.cu_seqlens, p.num_seqs, blockIdx.x / head_groups, rows, &seq_start, &seq_len, &work)) return;
+  const int q_first = (work - 1) * rows;
+  const int head0 = (blockIdx.x % head_groups) * p.heads_per_cta;
   const int kv_head = head0 / (p.n_q / p.n_kv);
   auto tile_head = [&](int t) { return p.heads_per_cta == C::kTiles ? head0 + t : head0; };
   auto tile_q0 = [&](int t) { return p.heads_per_cta == C::kTiles ? q_first : q_first + t * kBlockQ; };
@@ -460,11 +485,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                 const __grid_constant__ CUtensorMap tmap_dq, const BwdParams p) {
   using C = BwdCfg<D>;
-  int seq, seq_start, seq_len, kv0;
-  if (!locate_block(p.cu_seqlens, p.num_seqs, blockIdx.x, 128, &seq, &seq_start, &seq_len, &kv0)) return;
-  const int kv_head = blockIdx.y;
+  int seq_start, seq_len, work;
+  if (!locate_tile(p.cu_seqlens, p.num_seqs, blockIdx.x / p.n_kv, 128, &seq_start, &seq_len, &work)) return;
+  const int kv_head = blockIdx.x % p.n_kv;
   const int rep = p.n_q / p.n_kv;
   const int n_qblocks = (seq_len + 127) / 128;
+  const int kv0 = (n_qblocks - work) * 128;
   const int i_first = p.causal ? kv0 / 128 : 0;
   const int iters_per_head = n_qblocks - i_first;
   const int total_iters = iters_per_head * rep;
@@ -893,7 +919,7 @@ cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float
   const int tiles = head_dim == 64 ? FwdCfg<64>::kTiles : FwdCfg<128>::kTiles;
   p.heads_per_cta = (n_q / n_kv) % tiles == 0 ? tiles : 1;
   const int rows = kBlockQ * tiles / p.heads_per_cta;
-  dim3 grid((total_tokens + rows - 1) / rows + num_seqs, n_q / p.heads_per_cta);
+  const unsigned int grid = ((total_tokens + rows - 1) / rows + num_seqs) * (n_q / p.heads_per_cta);
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
@@ -961,7 +987,7 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
                                       BwdCfg<128>::kSmem);
   });
   if (attr_err != cudaSuccess) return attr_err;
-  dim3 grid((total_tokens + 127) / 128 + num_seqs, n_kv);
+  const unsigned int grid = ((total_tokens + 127) / 128 + num_seqs) * n_kv;
   if (head_dim == 64)
     attn_bwd_kernel<64><<<grid, kBwdThreads, BwdCfg<64>::kSmem, stream>>>(tq, tk, tv, tdo, tdq, p);
   else
