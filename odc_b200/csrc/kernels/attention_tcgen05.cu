@@ -842,9 +842,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 }
 
 // delta[h, t] = sum_d dO[t, h, d] * O[t, h, d].  A thread takes 16 bytes of both tensors; the D/8 threads of one
-// (token, head) pair are neighbours in a warp and combine with shuffles.  A CTA covers 256 / (D/8) consecutive
-// tokens and walks the heads, so the loads of a warp are whole 128-byte rows and the stores of one head form one
-// contiguous run of tokens.
+// (token, head) pair are neighbours in a warp and combine with shuffles.  A CTA covers 256 / (D/8) consecutive tokens of
+// kDeltaHeads heads, all of them loaded at once, so the loads of a warp are whole 128-byte rows and the stores of one head
+// form one contiguous run of tokens.  (One CTA walking all heads, one load at a time: 765 tokens, 12 heads, D = 128,
+// 11.0 us, now 4.3; 16321 tokens, 32 heads, D = 64, 31.9 us, now 22.1.)
+constexpr int kDeltaHeads = 4;
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o, float* __restrict__ delta,
@@ -853,24 +855,29 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* _
   constexpr int kTokens = 256 / kLanes;       // tokens per CTA
   const int part = threadIdx.x % kLanes;
   const int t = blockIdx.x * kTokens + threadIdx.x / kLanes;
+  const int h0 = blockIdx.y * kDeltaHeads;
   const bool live = t < total_tokens;
   const __nv_bfloat16* a = dout + static_cast<long long>(live ? t : 0) * do_stride + part * 8;
   const __nv_bfloat16* b = o + static_cast<long long>(live ? t : 0) * o_stride + part * 8;
-  for (int h = 0; h < n_q; ++h) {
-    float s = 0.f;
-    if (live) {
-      const uint4 x = *reinterpret_cast<const uint4*>(a + h * D);
-      const uint4 y = *reinterpret_cast<const uint4*>(b + h * D);
-      const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+  uint4 x[kDeltaHeads], y[kDeltaHeads];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        s += __uint_as_float(xs[i] << 16) * __uint_as_float(ys[i] << 16);
-        s += __uint_as_float(xs[i] & 0xffff0000u) * __uint_as_float(ys[i] & 0xffff0000u);
-      }
+  for (int k = 0; k < kDeltaHeads; ++k) {
+    const int h = min(h0 + k, n_q - 1);
+    x[k] = *reinterpret_cast<const uint4*>(a + h * D);
+    y[k] = *reinterpret_cast<const uint4*>(b + h * D);
+  }
+#pragma unroll
+  for (int k = 0; k < kDeltaHeads; ++k) {
+    const uint32_t xs[4] = {x[k].x, x[k].y, x[k].z, x[k].w}, ys[4] = {y[k].x, y[k].y, y[k].z, y[k].w};
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      s += __uint_as_float(xs[i] << 16) * __uint_as_float(ys[i] << 16);
+      s += __uint_as_float(xs[i] & 0xffff0000u) * __uint_as_float(ys[i] & 0xffff0000u);
     }
 #pragma unroll
     for (int off = kLanes / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (live && part == 0) delta[static_cast<long long>(h) * total_tokens + t] = s;
+    if (live && part == 0 && h0 + k < n_q) delta[static_cast<long long>(h0 + k) * total_tokens + t] = s;
   }
 }
 
@@ -953,12 +960,13 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
     return cudaErrorInvalidValue;
   // dout is contiguous [T, n_q, D]; dq / dk / dv rows may be strided (views of one fused qkv gradient)
   const long long do_stride = static_cast<long long>(n_q) * head_dim;
+  const unsigned int delta_y = (n_q + kDeltaHeads - 1) / kDeltaHeads;
   if (head_dim == 64) {
-    attn_delta_kernel<64><<<(total_tokens + 31) / 32, 256, 0, stream>>>(
+    attn_delta_kernel<64><<<dim3((total_tokens + 31) / 32, delta_y), 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, total_tokens, n_q,
         do_stride, o_stride);
   } else {
-    attn_delta_kernel<128><<<(total_tokens + 15) / 16, 256, 0, stream>>>(
+    attn_delta_kernel<128><<<dim3((total_tokens + 15) / 16, delta_y), 256, 0, stream>>>(
         static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, total_tokens, n_q,
         do_stride, o_stride);
   }
