@@ -217,10 +217,18 @@ void gemm_into(const Tensor& a, const Tensor& b, const Tensor& c, int lay, const
     res_ptr = residual.data_ptr();
     ldr = residual.stride(0);
   }
+  Tensor parts;  // few tiles and a long reduction: scratch for the partial products
+  if (pair < 0 && !accumulate) {
+    const size_t bytes = odc::gemm_split_bytes(M, N, K, kind_of(c.scalar_type()), sm_count());
+    if (bytes > 0) {
+      parts = at::empty({static_cast<int64_t>(bytes / sizeof(float))}, a.options().dtype(at::kFloat));
+      count();
+    }
+  }
   cudaError_t e = odc::gemm_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), kind_of(c.scalar_type()), bias_ptr, M, N, K,
                                  lay, accumulate, a.stride(0), b.stride(0), c.stride(0),
                                  device_status(a.get_device()).data_ptr<int>(), sm_count(), cur_stream(), res_ptr, ldr,
-                                 pair);
+                                 pair, parts.defined() ? parts.data_ptr<float>() : nullptr);
   TORCH_CHECK(e == cudaSuccess, "gemm(", kLayoutNames[lay], ") M=", M, " N=", N, " K=", K, " lda=", a.stride(0), " ldb=",
               b.stride(0), " ldc=", c.stride(0), " align(a,b,c)=", reinterpret_cast<uintptr_t>(a.data_ptr()) % 16, ",",
               reinterpret_cast<uintptr_t>(b.data_ptr()) % 16, ",", reinterpret_cast<uintptr_t>(c.data_ptr()) % 16, ": ",
@@ -737,6 +745,7 @@ void register_ops(py::module_& m) {
   m.def("sumsq", &sumsq);
   m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("c"), py::arg("layout"), py::arg("bias"),
         py::arg("accumulate"), py::arg("residual") = py::none(), py::arg("pair") = -1);
+  m.def("gemm_split_bytes", [](int M, int N, int K) { return odc::gemm_split_bytes(M, N, K, odc::kBF16, sm_count()); });
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("kernel_status", &kernel_status);

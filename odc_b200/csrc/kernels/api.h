@@ -112,13 +112,17 @@ struct GemmPlan;
 cudaError_t gemm_bf16(const void* a, const void* b, void* c, int c_kind, const void* bias, int M, int N, int K,
                       int layout, bool accumulate, long long lda, long long ldb, long long ldc, int* status,
                       int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0,
-                      int pair_mode = -1 /* -1: ODC_GEMM_PAIR decides, 0: single-CTA kernel, 1: CTA-pair kernel */);
+                      int pair_mode = -1 /* -1: ODC_GEMM_PAIR decides, 0: single-CTA kernel, 1: CTA-pair kernel */,
+                      float* split_ws = nullptr);
+// Bytes of scratch (split_ws) with which the CTA-pair kernel would divide this product's reduction; 0: it would not.
+size_t gemm_split_bytes(int M, int N, int K, int c_kind, int sm_count);
 
 // Same contract on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles).  Returns cudaErrorNotSupported for shapes it
 // does not take (M or N below 256, bf16 accumulation); gemm_bf16 tries it first unless ODC_GEMM_PAIR=0.
 cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, const void* bias, int M, int N, int K,
                            int layout, bool accumulate, long long lda, long long ldb, long long ldc, int* status,
-                           int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0);
+                           int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0,
+                           float* split_ws = nullptr);
 
 cudaError_t gemm_wgrad_scatter_pair(const void* dy, const void* x, int tokens, int n_out, int k_in, long long ld_dy,
                                     long long ld_x, const long long* acc_addrs_host, const long long* ctr_ptrs,

@@ -50,6 +50,9 @@ struct Params {
   int c_is_f32, accumulate;
   int a_mn, b_mn;
   int tiles_m, tiles_n;   // in units of the pair's 256 x 256 tile
+  // kModePlain: a tile's k-blocks are divided over `splits` pairs (1: not divided), kb_split each; split s writes its fp32
+  // partial tile at row s * split_rows of C
+  int splits, kb_split, split_rows;
   int* status;
   // kModeScatter: the epilogue adds every 128-row output box into the fp32 accumulator of the rank that owns those rows
   const long long* ctr_ptrs;   // [nranks] arrival counters
@@ -153,8 +156,17 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int num_tiles = p.tiles_m * p.tiles_n;
-  const int k_blocks = (p.K + BK - 1) / BK;
+  const int splits = kMode == kModePlain ? p.splits : 1;
+  const int num_tiles = p.tiles_m * p.tiles_n * splits;   // work items: (tile, split), the splits of a tile adjacent
+  const int all_k_blocks = (p.K + BK - 1) / BK;
+  auto k_range = [&](int item, int* kb0, int* kb1) {
+    *kb0 = 0;
+    *kb1 = all_k_blocks;
+    if (kMode == kModePlain && splits > 1) {
+      *kb0 = item % splits * p.kb_split;
+      *kb1 = min(all_k_blocks, *kb0 + p.kb_split);
+    }
+  };
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
 
   if (warp == 0) {
@@ -202,14 +214,16 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         int tm, tn;
-        tile_coords(tile, p, &tm, &tn);
+        tile_coords(tile / splits, p, &tm, &tn);
+        int kb0, k_blocks;
+        k_range(tile, &kb0, &k_blocks);
         const int m0 = tm * 256 + static_cast<int>(cta) * BMH;   // this CTA's rows of A and C
         const int n0 = tn * BN + static_cast<int>(cta) * BNH;    // this CTA's rows of B
         if constexpr (kMode == kModeGather) {
           // B K-major (forward): the 256 weight rows this tile multiplies must have landed in local memory first
           if (!p.b_mn && !(ok = wait_group(tn))) break;
         }
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        for (int kb = kb0; kb < k_blocks; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
           if constexpr (kMode == kModeGather) {
@@ -251,7 +265,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (!(ok = mbar_wait(tempty0 + 8 * acc, acc_ph ^ 1, wc, 12))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+        int kb0, k_blocks;
+        k_range(tile, &kb0, &k_blocks);
+        for (int kb = kb0; kb < k_blocks; ++kb, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1;
           if (!(ok = mbar_wait(full0 + 8 * s, ph, wc, 13))) break;
@@ -262,7 +278,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           for (int j = 0; j < BK / 16; ++j) {
             const uint64_t da = make_smem_desc(sa + j * a_kstep, a_lbo, 1024);
             const uint64_t db = make_smem_desc(sb + j * b_kstep, b_lbo, 1024);
-            umma_f16_pair(d_tmem, da, db, idesc, (kb > 0 || j > 0) ? 1u : 0u);
+            umma_f16_pair(d_tmem, da, db, idesc, (kb > kb0 || j > 0) ? 1u : 0u);
           }
           // the stage is reusable in BOTH CTAs once these MMAs have read it
           umma_commit_pair(mapa_shared(empty0 + 8 * s, 0));
@@ -331,7 +347,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const uint32_t tempty_leader0 = mapa_shared(tempty0, 0);
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local_tile) {
       int tm, tn;
-      tile_coords(tile, p, &tm, &tn);
+      tile_coords(tile / splits, p, &tm, &tn);
+      const int c_row0 = splits > 1 ? tile % splits * p.split_rows : 0;
       const int m0 = tm * 256 + static_cast<int>(cta) * BMH;
       const int n0 = tn * BN;
       const uint32_t acc = local_tile & 1;
@@ -406,7 +423,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             } else if (p.accumulate) {
               tma_reduce_add_2d(&tmap_c, staging_u32 + buf * kStagingBytes, col0, m0);
             } else {
-              tma_store_2d(&tmap_c, staging_u32 + buf * kStagingBytes, col0, m0);
+              tma_store_2d(&tmap_c, staging_u32 + buf * kStagingBytes, col0, c_row0 + m0);
             }
             bulk_commit_group();
             if (box_ctr >= 1) {
@@ -453,6 +470,38 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   }
 }
 
+// C = sum over splits of the fp32 partial tiles, in order, + bias + residual, narrowed to bf16.  Eight columns per thread.
+__global__ void __launch_bounds__(256)
+split_sum_kernel(const float* __restrict__ part, long long part_stride, int splits, __nv_bfloat16* __restrict__ c, long long ldc,
+                 const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ residual, long long ldr, int M, int N) {
+  const int n8 = N / 8;
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= static_cast<long long>(M) * n8) return;
+  const int row = static_cast<int>(i / n8), col = static_cast<int>(i % n8) * 8;
+  const float* src = part + static_cast<long long>(row) * N + col;
+  float f[8] = {};
+  for (int s = 0; s < splits; ++s, src += part_stride) {
+    const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+    f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+    f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+  }
+  if (bias != nullptr) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) f[k] += __bfloat162float(bias[col + k]);
+  }
+  if (residual != nullptr) {
+    const uint4 r = *reinterpret_cast<const uint4*>(residual + row * ldr + col);
+    const uint32_t u[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      f[2 * k] += __uint_as_float(u[k] << 16);
+      f[2 * k + 1] += __uint_as_float(u[k] & 0xffff0000u);
+    }
+  }
+  *reinterpret_cast<uint4*>(c + row * ldc + col) =
+      make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
+}
+
 }  // namespace gemm_pair
 
 // ODC_GEMM_ROTATE: 0 (default) every rank walks the owners in address order; 1: the forward gather and the
@@ -469,10 +518,40 @@ static int rotate_mode() {
   return mode;
 }
 
+// How many ways to divide the reduction of a bf16 product whose tiles leave pairs idle (few rows, long reduction: the short
+// packs of a minibatch).  In units of a k-block (512 clocks of the tensor cores, 0.28 us): a product takes as many rounds as
+// its items need, each as long as its longest item; dividing it adds a second launch (3 us: 11 units) and writes and reads the
+// fp32 partials once (at 5 TB/s, 1.4 MB per unit).  Divided only where that is at least a tenth faster.  765 x 1536 with
+// K = 8960: 59 us whole, 29 us divided by four with the sum; K = 17920: 100 us and 42 us.
+static int plan_splits(int M, int N, int K, int sm_count, int* kb_split) {
+  using namespace gemm_pair;
+  const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + BN - 1) / BN), pairs = sm_count / 2;
+  const int kb = (K + BK - 1) / BK;
+  double best = 0.9 * static_cast<double>((tiles + pairs - 1) / pairs) * kb;
+  int splits = 1;
+  *kb_split = kb;
+  for (int want = 2; want <= 8 && tiles < pairs; ++want) {
+    const int each = (kb + want - 1) / want, s = (kb + each - 1) / each;   // no empty split
+    if (s < 2) break;
+    const double bytes = 2.0 * s * ((M + 255) / 256) * 256.0 * N * 4.0;
+    const double cost = static_cast<double>((tiles * s + pairs - 1) / pairs) * each + 11.0 + bytes / 1.4e6;
+    if (cost < best) { best = cost; splits = s; *kb_split = each; }
+  }
+  return splits;
+}
+
+size_t gemm_split_bytes(int M, int N, int K, int c_kind, int sm_count) {
+  using namespace gemm_pair;
+  if (c_kind != kBF16 || M < 256 || N < 256 || K < BK || sm_count < 2) return 0;
+  int kb_split;
+  const int splits = plan_splits(M, N, K, sm_count, &kb_split);
+  return splits == 1 ? 0 : static_cast<size_t>(splits) * ((M + 255) / 256 * 256) * N * sizeof(float);
+}
+
 // Returns cudaErrorNotSupported when the shape is not worth a CTA pair (the caller then uses the single-CTA kernel).
 cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, const void* bias, int M, int N, int K,
                            int layout, bool accumulate, long long lda, long long ldb, long long ldc, int* status,
-                           int sm_count, cudaStream_t stream, const void* residual, long long ldr) {
+                           int sm_count, cudaStream_t stream, const void* residual, long long ldr, float* split_ws) {
   using namespace gemm_pair;
   if (M < 256 || N < 256 || K < BK || sm_count < 2) return cudaErrorNotSupported;
   const bool a_mn = (layout == 2);
@@ -501,28 +580,45 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
   } else {
     if (!encode_tile_map_2d(&tb, b, N, K, ldb * 2, 64, 64)) return cudaErrorInvalidTexture;
   }
-  if (c_kind == kF32) {
+  Params p{};
+  p.tiles_m = (M + 255) / 256;
+  p.splits = 1;
+  if (split_ws != nullptr) {
+    p.splits = plan_splits(M, N, K, sm_count, &p.kb_split);
+    p.split_rows = p.tiles_m * 256;
+  }
+  const bool split = p.splits > 1;
+  if (split) {
+    if (!encode_tile_map_2d_f32(&tc, split_ws, N, static_cast<uint64_t>(p.splits) * p.split_rows, static_cast<uint64_t>(N) * 4, 32, BMH))
+      return cudaErrorInvalidValue;
+  } else if (c_kind == kF32) {
     if (!encode_tile_map_2d_f32(&tc, c, N, M, ldc * 4, 32, BMH)) return cudaErrorInvalidValue;
   } else {
     if (!encode_tile_map_2d(&tc, c, N, M, ldc * 2, 64, BMH)) return cudaErrorInvalidValue;
   }
-  Params p{};
-  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  if (!split) p.bias = static_cast<const __nv_bfloat16*>(bias);   // the sum of the splits adds it otherwise
   p.M = M; p.N = N; p.K = K;
-  p.c_is_f32 = (c_kind == kF32);
+  p.c_is_f32 = (split || c_kind == kF32);
   p.accumulate = accumulate ? 1 : 0;
   p.a_mn = a_mn; p.b_mn = b_mn;
-  p.tiles_m = (M + 255) / 256;
   p.tiles_n = (N + BN - 1) / BN;
   p.status = status;
   if (residual != nullptr) {
     if (c_kind != kBF16 || (ldr % 8) || (reinterpret_cast<uintptr_t>(residual) & 15)) return cudaErrorInvalidValue;
-    p.residual = static_cast<const __nv_bfloat16*>(residual);
+    if (!split) p.residual = static_cast<const __nv_bfloat16*>(residual);
     p.ldr = ldr;
   }
-  const int tiles = p.tiles_m * p.tiles_n;
+  const int tiles = p.tiles_m * p.tiles_n * p.splits;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
   gemm_bf16_pair_kernel<kModePlain><<<2 * pairs, kThreads, kSmemBytes, stream>>>(ta, tb, tc, OwnerMaps{}, p);
+  if (split) {
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const long long items = static_cast<long long>(M) * (N / 8);
+    split_sum_kernel<<<static_cast<unsigned int>((items + 255) / 256), 256, 0, stream>>>(
+        split_ws, static_cast<long long>(p.split_rows) * N, p.splits, static_cast<__nv_bfloat16*>(c), ldc,
+        static_cast<const __nv_bfloat16*>(bias), static_cast<const __nv_bfloat16*>(residual), ldr, M, N);
+  }
   return cudaGetLastError();
 }
 

@@ -269,6 +269,28 @@ def test_gemm_cta_pair_layouts(ext, layout, M, N, K):
     torch.testing.assert_close(c32, want, rtol=1e-2, atol=1e-2 * math.sqrt(K))
 
 
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("M,N,K,divided", [(256, 256, 2048, True), (264, 264, 4040, True), (765, 1536, 17920, True),
+                                           (520, 1544, 8968, True), (768, 2048, 1536, False), (2304, 2304, 4096, False)])
+def test_gemm_divided_reduction(ext, layout, M, N, K, divided):
+    """Few tiles and a long reduction: partial products and their sum, ragged tiles and a ragged last part included."""
+    M = (M + 7) // 8 * 8 if layout == "tn" else M
+    assert (ext.gemm_split_bytes(M, N, K) > 0) == divided
+    torch.manual_seed(M + N + K)
+    A, B = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+    bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N + 8, device="cuda").bfloat16()[:, :N]
+    a = A.t().contiguous() if layout == "tn" else A
+    b = B.t().contiguous() if layout == "nt" else B
+    want = A.double() @ B.double()
+    c = torch.empty(M, N + 16, dtype=torch.bfloat16, device="cuda")[:, :N]
+    for kw, exp in (((None, False), want), ((bias, False, res), want + bias.double() + res.double())):
+        ext.gemm(a, b, c, layout, *kw)
+        torch.cuda.synchronize()
+        assert ext.kernel_status()[0].item() == 0, ext.kernel_status().tolist()
+        # fp32 sums of K products (sqrt(K) 2^-24 each way, far below) and one rounding to bf16
+        assert ((c.double() - exp).abs() <= 2 ** -8 * exp.abs() + 1e-4 * K ** 0.5).all()
+
+
 def test_linear_autograd_matches_reference():
     from odc_b200 import ops
     x = torch.randn(3, 100, 512, device="cuda").bfloat16().requires_grad_()
