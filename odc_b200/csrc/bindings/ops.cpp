@@ -310,8 +310,12 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(Tensor dout, Tensor q, Tenso
   }
   auto delta = at::empty({hq, T}, q.options().dtype(at::kFloat));
   auto dq_acc = at::empty({T, hq, d}, q.options().dtype(at::kFloat));
+  const int n_parts = hkv > 0 && hq % hkv == 0 ? odc::attn_bwd_parts(T, hq, hkv, sm_count()) : 1;
+  Tensor kv_parts;
+  if (n_parts > 1) kv_parts = at::empty({n_parts, 2, T, hkv, d}, q.options().dtype(at::kFloat));
   check(odc::attn_bwd(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
                       dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), dq_acc.data_ptr<float>(),
+                      n_parts > 1 ? kv_parts.data_ptr<float>() : nullptr,
                       cu_seqlens.data_ptr<int>(), static_cast<int>(cu_seqlens.numel() - 1), T, max_seqlen, hq, hkv, d,
                       q.stride(0), k.stride(0), o.stride(0), dq.stride(0), dk.stride(0), static_cast<float>(scale),
                       causal, device_status(q.get_device()).data_ptr<int>(), sm_count(), cur_stream()),

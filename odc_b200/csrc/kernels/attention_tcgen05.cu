@@ -436,6 +436,8 @@ struct BwdParams {
   __nv_bfloat16* dk;   // rows of n_kv * D values, dkv_stride elements apart
   __nv_bfloat16* dv;
   long long dkv_stride;
+  int parts;           // CTAs that share the query heads of one (key tile, kv head); each takes n_q / n_kv / parts of them
+  float* kv_parts;     // parts > 1: [parts][dK, dV][total_tokens, n_kv, D] fp32, summed by the post-pass
   int total_tokens;
   float scale, scale_log2;
   int causal;
@@ -486,9 +488,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 const __grid_constant__ CUtensorMap tmap_dq, const BwdParams p) {
   using C = BwdCfg<D>;
   int seq_start, seq_len, work;
-  if (!locate_tile(p.cu_seqlens, p.num_seqs, blockIdx.x / p.n_kv, 128, &seq_start, &seq_len, &work)) return;
-  const int kv_head = blockIdx.x % p.n_kv;
-  const int rep = p.n_q / p.n_kv;
+  if (!locate_tile(p.cu_seqlens, p.num_seqs, blockIdx.x / (p.n_kv * p.parts), 128, &seq_start, &seq_len, &work)) return;
+  const int kv_head = blockIdx.x / p.parts % p.n_kv, part = blockIdx.x % p.parts;
+  const int rep = p.n_q / p.n_kv / p.parts;                     // query heads of this CTA
+  const int first_head = (kv_head * p.parts + part) * rep;
   const int n_qblocks = (seq_len + 127) / 128;
   const int kv0 = (n_qblocks - work) * 128;
   const int i_first = p.causal ? kv0 / 128 : 0;
@@ -563,7 +566,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         tma_load_2d(v_smem + s * 16384, &tmap_v, kv_full, kv_head * D + 64 * s, seq_start + kv0);
       }
     }
-    int head = kv_head * rep, i = i_first;
+    int head = first_head, i = i_first;
     for (int it = 0; it < total_iters; ++it) {
       const int qs = it % C::kQStages, os = it % C::kDoStages;
       const int row = seq_start + i * 128;
@@ -767,12 +770,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       __nv_bfloat16* dst = (half == 0 ? p.dv : p.dk) + off;
       const uint32_t src = lanes + (half == 0 ? C::kDv : C::kDk);
       const float f = half == 0 ? 1.f : p.scale;
+      float* sum = p.kv_parts + ((static_cast<long long>(2 * part + 1 - half) * p.total_tokens + seq_start + kv) * p.n_kv + kv_head) * D;
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         uint32_t r[32];
         tmem_ld_32x32(src + c * 32, r);
         tmem_ld_wait();
-        if (kv < seq_len) {
+        if (kv < seq_len && p.parts > 1) {
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<uint4*>(sum + c * 32 + v * 4) = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+        } else if (kv < seq_len) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             uint4 o;
@@ -793,7 +801,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const uint32_t src = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + C::kDq;
     const bool issuer = warp == 10 && lane == 0;
     bool ok = true;
-    int head = kv_head * rep, i = i_first;
+    int head = first_head, i = i_first;
     for (int it = 0; it < total_iters; ++it) {
       ok = ok && mbar_wait(dq_full, it & 1, wc, 40);
       tc_fence_after();
@@ -881,19 +889,34 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* _
   }
 }
 
-// dq = bf16(acc * scale); acc is dense [tokens, width] fp32; dq rows are dq_stride elements apart
+// dq = bf16(acc * scale); acc is dense [tokens, width] fp32; dq rows are dq_stride elements apart.  With parts > 1 also
+// dk = bf16(scale * sum over parts) and dv = bf16(sum over parts), in order, from dense [parts][2][tokens, kv width] fp32.
 __global__ void __launch_bounds__(256)
-cast_dq_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long n8, int width8,
-               long long dq_stride, float scale) {
-  for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < n8;
+narrow_grads_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long n8, int width8, long long dq_stride,
+                    float scale, const float* __restrict__ kv_parts, int parts, __nv_bfloat16* __restrict__ dk,
+                    __nv_bfloat16* __restrict__ dv, long long kv_n8, int kv_width8, long long dkv_stride) {
+  const long long total = n8 + (parts > 1 ? 2 * kv_n8 : 0);
+  for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < total;
        v += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float4 a = *reinterpret_cast<const float4*>(acc + v * 8);
-    const float4 b = *reinterpret_cast<const float4*>(acc + v * 8 + 4);
-    const long long row = v / width8;
-    const int col = static_cast<int>(v % width8) * 8;
-    *reinterpret_cast<uint4*>(dq + row * dq_stride + col) =
-        make_uint4(pack2(a.x * scale, a.y * scale), pack2(a.z * scale, a.w * scale), pack2(b.x * scale, b.y * scale),
-                   pack2(b.z * scale, b.w * scale));
+    const bool is_q = v < n8, is_v = v >= n8 + kv_n8;
+    const long long i = is_q ? v : v - n8 - (is_v ? kv_n8 : 0);
+    const float* src = is_q ? acc + v * 8 : kv_parts + (v - n8) * 8;
+    float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+    if (!is_q) {
+      for (int s = 1; s < parts; ++s) {
+        src += 16 * kv_n8;
+        const float4 c = *reinterpret_cast<const float4*>(src), d = *reinterpret_cast<const float4*>(src + 4);
+        a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
+        b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
+      }
+    }
+    const int w8 = is_q ? width8 : kv_width8;
+    const long long row = i / w8;
+    const int col = static_cast<int>(i % w8) * 8;
+    __nv_bfloat16* dst = is_q ? dq + row * dq_stride : (is_v ? dv : dk) + row * dkv_stride;
+    const float f = is_v ? 1.f : scale;
+    *reinterpret_cast<uint4*>(dst + col) =
+        make_uint4(pack2(a.x * f, a.y * f), pack2(a.z * f, a.w * f), pack2(b.x * f, b.y * f), pack2(b.z * f, b.w * f));
   }
 }
 
@@ -947,8 +970,21 @@ cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float
 
 namespace odc {
 
+// Into how many CTAs the query heads of one (key tile, kv head) are divided: the smallest divisor of the group that gives
+// every SM a CTA, or the whole group.  A short pack has few key tiles and each would walk all heads in turn (D = 128, 12/2
+// heads: 765 tokens 93 us, 45 us divided by six; 2048 tokens 275 us and 79 us).  With a CTA for every SM already there, the
+// partial sums (parts * 16 bytes of traffic per element of dK) cost more than they give: 4096 tokens, 32/8 heads, D = 64,
+// 256 tiles: 302 us whole, 323 us divided by two.
+int attn_bwd_parts(int total_tokens, int n_q, int n_kv, int sm_count) {
+  const int rep = n_q / n_kv;
+  const long long tiles = static_cast<long long>((total_tokens + 127) / 128) * n_kv;
+  int parts = 1;
+  while (parts < rep && (rep % parts != 0 || tiles * parts < sm_count)) ++parts;
+  return parts;
+}
+
 cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const float* lse,
-                     void* dq, void* dk, void* dv, float* delta, float* dq_acc, const int* cu_seqlens, int num_seqs,
+                     void* dq, void* dk, void* dv, float* delta, float* dq_acc, float* kv_parts, const int* cu_seqlens, int num_seqs,
                      int total_tokens, int max_seqlen, int n_q, int n_kv, int head_dim, long long q_stride,
                      long long kv_stride, long long o_stride, long long dq_stride, long long dkv_stride, float scale,
                      bool causal, int* status, int sm_count, cudaStream_t stream) {
@@ -986,6 +1022,9 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
   p.dq_acc = dq_acc; p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
   p.total_tokens = total_tokens; p.scale = scale; p.scale_log2 = scale * kLog2e; p.causal = causal ? 1 : 0;
   p.status = status; p.dkv_stride = dkv_stride;
+  p.parts = attn_bwd_parts(total_tokens, n_q, n_kv, sm_count);
+  p.kv_parts = kv_parts;
+  if (p.parts > 1 && kv_parts == nullptr) return cudaErrorInvalidValue;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
@@ -995,16 +1034,18 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
                                       BwdCfg<128>::kSmem);
   });
   if (attr_err != cudaSuccess) return attr_err;
-  const unsigned int grid = ((total_tokens + 127) / 128 + num_seqs) * n_kv;
+  const unsigned int grid = ((total_tokens + 127) / 128 + num_seqs) * n_kv * p.parts;
   if (head_dim == 64)
     attn_bwd_kernel<64><<<grid, kBwdThreads, BwdCfg<64>::kSmem, stream>>>(tq, tk, tv, tdo, tdq, p);
   else
     attn_bwd_kernel<128><<<grid, kBwdThreads, BwdCfg<128>::kSmem, stream>>>(tq, tk, tv, tdo, tdq, p);
   const long long n8 = static_cast<long long>(total_tokens) * n_q * head_dim / 8;
-  long long g = (n8 + 255) / 256;
+  const long long kv_n8 = static_cast<long long>(total_tokens) * n_kv * head_dim / 8;
+  long long g = (n8 + (p.parts > 1 ? 2 * kv_n8 : 0) + 255) / 256;
   if (g > sm_count * 16) g = sm_count * 16;
-  cast_dq_kernel<<<static_cast<int>(g), 256, 0, stream>>>(dq_acc, static_cast<__nv_bfloat16*>(dq), n8,
-                                                          n_q * head_dim / 8, dq_stride, scale);
+  narrow_grads_kernel<<<static_cast<int>(g), 256, 0, stream>>>(
+      dq_acc, static_cast<__nv_bfloat16*>(dq), n8, n_q * head_dim / 8, dq_stride, scale, kv_parts, p.parts,
+      static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), kv_n8, n_kv * head_dim / 8, dkv_stride);
   return cudaGetLastError();
 }
 
