@@ -291,6 +291,31 @@ def test_gemm_divided_reduction(ext, layout, M, N, K, divided):
         assert ((c.double() - exp).abs() <= 2 ** -8 * exp.abs() + 1e-4 * K ** 0.5).all()
 
 
+@pytest.mark.parametrize("T,H,F", [(24, 256, 512), (300, 512, 1536), (765, 1536, 8960)])
+def test_chained_kernels_see_their_predecessors(ext, T, H, F):
+    """A kernel may start before the one ahead of it has ended: a chain queued without a pause gives the bytes of one that is
+    waited for after every call, also when each link reuses the memory of the link before."""
+    torch.manual_seed(T)
+    x0 = torch.randn(T, H, device="cuda").bfloat16()
+    w = torch.rand(H, device="cuda").bfloat16()
+    up, down = (0.05 * torch.randn(n, k, device="cuda").bfloat16() for n, k in ((2 * F, H), (H, F)))
+
+    def chain(pause):
+        x = x0
+        for _ in range(6):
+            for step in (lambda t: ext.rmsnorm_fwd(t, w, 1e-5)[0], lambda t: ext.linear(t, up), ext.swiglu_fwd,
+                         lambda t: ext.linear(t, down)):
+                x = step(x)
+                if pause:
+                    torch.cuda.synchronize()
+        return x
+
+    want = chain(True)
+    assert torch.isfinite(want.float()).all()
+    for _ in range(5):
+        assert torch.equal(chain(False), want)
+
+
 def test_linear_autograd_matches_reference():
     from odc_b200 import ops
     x = torch.randn(3, 100, 512, device="cuda").bfloat16().requires_grad_()
