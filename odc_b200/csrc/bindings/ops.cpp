@@ -471,6 +471,59 @@ struct SwiGLUFn : Function<SwiGLUFn> {
 };
 Tensor swiglu(Tensor gate_up) { return SwiGLUFn::apply(gate_up.contiguous()); }
 
+// swiglu(x w^T) for w = [gate; up]: the activation is formed in the epilogue of the product where that kernel takes the
+// shape.  gate_up is only written when a gradient will need it.
+std::tuple<Tensor, Tensor> linear_swiglu_fwd(const Tensor& x, const Tensor& w, bool need_gate_up) {
+  c10::cuda::CUDAGuard g(x.device());
+  odc::bind_device(x.get_device());
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && w.size(0) % 2 == 0, "linear_swiglu: x [T,K], w [2F,K]");
+  TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "linear_swiglu: bf16 inputs");
+  TORCH_CHECK(x.stride(1) == 1 && w.stride(1) == 1, "linear_swiglu: innermost stride must be 1");
+  const int64_t T = x.size(0), F = w.size(0) / 2;
+  static const bool pairs = [] {
+    const char* e = std::getenv("ODC_GEMM_PAIR");
+    return e == nullptr || e[0] != '0';
+  }();
+  if (pairs && !library_gemm()) {
+    Tensor gate_up;
+    if (need_gate_up) gate_up = at::empty({T, 2 * F}, x.options());
+    auto act = at::empty({T, F}, x.options());
+    const cudaError_t e = odc::gemm_swiglu_pair(x.data_ptr(), w.data_ptr(), need_gate_up ? gate_up.data_ptr() : nullptr,
+                                                act.data_ptr(), static_cast<int>(T), static_cast<int>(F),
+                                                static_cast<int>(x.size(1)), x.stride(0), w.stride(0),
+                                                device_status(x.get_device()).data_ptr<int>(), sm_count(), cur_stream());
+    if (e != cudaErrorNotSupported) {
+      check(e, "linear_swiglu");
+      count();
+      return {act, gate_up};
+    }
+  }
+  const Tensor gate_up = product(x, w, kNT);
+  count();
+  return {swiglu_fwd(gate_up), gate_up};
+}
+
+struct LinearSwigluFn : Function<LinearSwigluFn> {
+  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor w, bool need_dx, bool need_dw) {
+    auto [act, gate_up] = linear_swiglu_fwd(rows2d(x), w, need_dx || need_dw);
+    ctx->saved_data["need"] = static_cast<int64_t>(need_dx | need_dw << 1);
+    if (need_dx || need_dw) ctx->save_for_backward({x, w, gate_up});
+    return like(act, x, w.size(0) / 2);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &w = saved[1];
+    const int64_t need = ctx->saved_data["need"].toInt();
+    const Tensor d = swiglu_bwd(rows2d(grads[0]).contiguous(), saved[2]);
+    count();
+    Tensor dx, dw;
+    if (need & 1) dx = product(d, w, kNN).view(x.sizes());
+    if (need & 2) dw = product(d, rows2d(x), kTN, {}, {}, w.scalar_type());
+    return {dx, dw, {}, {}};
+  }
+};
+Tensor linear_swiglu(Tensor x, Tensor w) { return LinearSwigluFn::apply(x, w, wants_grad(x), wants_grad(w)); }
+
 struct AttentionFn : Function<AttentionFn> {
   static Tensor forward(AutogradContext* ctx, Tensor q, Tensor k, Tensor v, Tensor cu, int64_t max_seqlen, bool causal,
                         double scale) {
@@ -783,6 +836,7 @@ void register_ops(py::module_& m) {
   m.def("rms_norm_residual", &rms_norm_residual, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());
   m.def("rope", &rope);
   m.def("swiglu", &swiglu);
+  m.def("linear_swiglu", &linear_swiglu, py::arg("x"), py::arg("w"));
   m.def("attention", &attention);
   m.def("attention_qkv", &attention_qkv);
   m.def("linear_cross_entropy", &linear_cross_entropy);

@@ -124,6 +124,9 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
                            int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0,
                            float* split_ws = nullptr);
 
+// act[M, F] = silu(x Wg^T) * (x Wu^T), w = [Wg; Wu]; gate_up [M, 2F] optional.  cudaErrorNotSupported: use the plain product.
+cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* act, int M, int F, int K, long long ldx,
+                             long long ldw, int* status, int sm_count, cudaStream_t stream);
 cudaError_t gemm_wgrad_scatter_pair(const void* dy, const void* x, int tokens, int n_out, int k_in, long long ld_dy,
                                     long long ld_x, const long long* acc_addrs_host, const long long* ctr_ptrs,
                                     long long acc_offset, int rows_per_rank, int nranks, float scale,

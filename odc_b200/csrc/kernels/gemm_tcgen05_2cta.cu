@@ -65,6 +65,8 @@ struct Params {
   const long long* shard_ptrs; // [nranks] base address of each owner's [rows_per_rank, w_cols] bf16 shard
   unsigned char* b_local;      // local [w_rows, w_cols] bf16 buffer the shards are gathered into (tensor map B covers it)
   unsigned int* panel_flags;   // [ceil(w_rows / 256)] chunks landed per 256-row group (zeroed before the launch)
+  // kModeSwiglu (N = F): tensor maps c: activation [M, F], owners.m[0] / [1]: gate / up half of the projection [M, 2F]
+  int store_gate_up;
   int w_rows, w_cols;          // gathered matrix: [N, K] when B is K-major (y = x W^T), [K, N] when MN-major (dx = dy W)
   // Rotation of the work order by this rank's position in the group.  Without it every rank would pull the first
   // owner's rows first (and push into the first owner's accumulator first): one GPU's links saturated, seven idle.
@@ -74,7 +76,11 @@ struct Params {
   long long fetch_rot;         // 64 KiB chunks by which the fetch order is rotated
 };
 
-constexpr int kModePlain = 0, kModeScatter = 1, kModeGather = 2;
+// kModeSwiglu: B holds the gate rows and, F rows further on, the up rows.  The even CTA stages 128 gate rows and the odd one
+// the matching 128 up rows, so a tile's accumulator holds both halves of 128 activations and the epilogue forms them: the
+// activation is not a pass of its own (16384 x 8192: 0.12 ms of reading and writing), and without gradients the
+// projection itself is never written.
+constexpr int kModePlain = 0, kModeScatter = 1, kModeGather = 2, kModeSwiglu = 3;
 constexpr int kFetchWarps = 4;
 constexpr int kFetchWarpBytes = 16384;                  // moved by one fetch warp between two flag updates
 constexpr int kFetchChunkBytes = kFetchWarps * kFetchWarpBytes;
@@ -223,7 +229,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         int kb0, k_blocks;
         k_range(tile, &kb0, &k_blocks);
         const int m0 = tm * 256 + static_cast<int>(cta) * BMH;   // this CTA's rows of A and C
-        const int n0 = tn * BN + static_cast<int>(cta) * BNH;    // this CTA's rows of B
+        const int n0 = kMode == kModeSwiglu ? tn * BNH + static_cast<int>(cta) * p.N
+                                            : tn * BN + static_cast<int>(cta) * BNH;    // this CTA's rows of B
         if constexpr (kMode == kModeGather) {
           // B K-major (forward): the 256 weight rows this tile multiplies must have landed in local memory first
           if (!p.b_mn && !(ok = wait_group(tn))) break;
@@ -364,6 +371,61 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const int row = m0 + my_row;
       const bool row_ok = row < p.M;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
+      if constexpr (kMode == kModeSwiglu) {
+        // one staged box of 64 bf16 columns: 32 packed registers per row
+        auto emit = [&](const uint32_t* v32, const CUtensorMap* map, int col0) -> bool {
+          const int buf = static_cast<int>(box_ctr & 1u);
+          const uint32_t use = box_ctr >> 1;
+          if (use >= 1 && !mbar_wait(sfree0 + 8 * buf, (use - 1) & 1, wc, 16)) return false;
+          uint8_t* srow = staging + buf * kStagingBytes + my_row * 128;
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<uint4*>(srow + ((v ^ (my_row & 7)) << 4)) =
+                make_uint4(v32[4 * v], v32[4 * v + 1], v32[4 * v + 2], v32[4 * v + 3]);
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(sready0 + 8 * buf);
+          if (warp == 2 && lane == 0 && mbar_wait(sready0 + 8 * buf, use & 1, wc, 17)) {
+            tma_store_2d(map, staging_u32 + buf * kStagingBytes, col0, m0);
+            bulk_commit_group();
+            if (box_ctr >= 1) {
+              bulk_wait_group_read1();
+              mbar_arrive(sfree0 + 8 * (buf ^ 1));
+            }
+          }
+          ++box_ctr;
+          return true;
+        };
+#pragma unroll 1
+        for (int bx = 0; bx < 2; ++bx) {
+          uint32_t gate[32], up[32];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t r[64];
+            tmem_ld_32x32(t_row + bx * 64 + 32 * h, r);
+            tmem_ld_32x32(t_row + BNH + bx * 64 + 32 * h, r + 32);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              gate[16 * h + i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+              up[16 * h + i] = pack2(__uint_as_float(r[32 + 2 * i]), __uint_as_float(r[32 + 2 * i + 1]));
+            }
+          }
+          const int col0 = tn * BNH + bx * 64;
+          if (col0 >= p.N || m0 >= p.M) continue;
+          if (p.store_gate_up) {
+            if (!(ok = emit(gate, &owners.m[0], col0))) break;
+            if (!(ok = emit(up, &owners.m[1], col0))) break;
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {   // from the rounded halves, as the stand-alone pass reads them
+            const float g0 = __uint_as_float(gate[i] << 16), g1 = __uint_as_float(gate[i] & 0xffff0000u);
+            const float u0 = __uint_as_float(up[i] << 16), u1 = __uint_as_float(up[i] & 0xffff0000u);
+            gate[i] = pack2(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1);
+          }
+          if (!(ok = emit(gate, &tmap_c, col0))) break;
+        }
+      } else {
       const int cols_per_box = p.c_is_f32 ? 32 : 64;
       const int n_boxes = BN / cols_per_box;
 #pragma unroll 1
@@ -438,6 +500,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           }
         }
         ++box_ctr;
+      }
       }
       if (!ok) break;
       tc_fence_before();
@@ -627,6 +690,49 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
         split_ws, static_cast<long long>(p.split_rows) * N, p.splits, static_cast<__nv_bfloat16*>(c), ldc,
         static_cast<const __nv_bfloat16*>(bias), static_cast<const __nv_bfloat16*>(residual), ldr, M, N);
   }
+  return cudaGetLastError();
+}
+
+// act[M, F] = silu(x Wg^T) * (x Wu^T) for w = [Wg; Wu], [2F, K]; gate_up [M, 2F] receives both products unless it is null.
+// cudaErrorNotSupported where the plain product followed by the activation is the better form: fewer rows than a tile, or a
+// reduction that is worth dividing.
+cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* act, int M, int F, int K, long long ldx,
+                             long long ldw, int* status, int sm_count, cudaStream_t stream) {
+  using namespace gemm_pair;
+  int kb_split;
+  if (M < 256 || F < BNH || K < BK || sm_count < 2 || plan_splits(M, 2 * F, K, sm_count, &kb_split) > 1) return cudaErrorNotSupported;
+  if ((ldx % 8) || (ldw % 8) || (F % 8) ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(gate_up) |
+        reinterpret_cast<uintptr_t>(act)) & 15))
+    return cudaErrorNotSupported;
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(gemm_bf16_pair_kernel<kModeSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    kSmemBytes);
+  });
+  if (attr_err != cudaSuccess) return attr_err;
+  CUtensorMap ta, tb, tc;
+  OwnerMaps halves{};
+  const uint64_t ld_gu = static_cast<uint64_t>(F) * 4;
+  if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, 2ull * F, ldw * 2, 64, BNH) ||
+      !encode_tile_map_2d(&tc, act, F, M, static_cast<uint64_t>(F) * 2, 64, BMH))
+    return cudaErrorInvalidValue;
+  if (gate_up != nullptr) {  // each half clipped at its own last column
+    if (!encode_tile_map_2d(&halves.m[0], gate_up, F, M, ld_gu, 64, BMH) ||
+        !encode_tile_map_2d(&halves.m[1], static_cast<__nv_bfloat16*>(gate_up) + F, F, M, ld_gu, 64, BMH))
+      return cudaErrorInvalidValue;
+  }
+  Params p{};
+  p.M = M; p.N = F; p.K = K;
+  p.splits = 1;
+  p.store_gate_up = gate_up != nullptr;
+  p.tiles_m = (M + 255) / 256;
+  p.tiles_n = (F + BNH - 1) / BNH;
+  p.status = status;
+  const int tiles = p.tiles_m * p.tiles_n;
+  const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
+  launch_after(gemm_bf16_pair_kernel<kModeSwiglu>, 2 * pairs, kThreads, kSmemBytes, stream, ta, tb, tc, halves, p);
   return cudaGetLastError();
 }
 

@@ -146,6 +146,13 @@ def swiglu(gate_up):
     return _ext().swiglu(gate_up)
 
 
+def linear_swiglu(x, w):
+    """``swiglu(linear(x, w))`` for ``w = [gate; up]``; on CUDA the activation is formed in the GEMM epilogue."""
+    if not x.is_cuda:
+        return ref.swiglu(ref.linear(x, w, None))
+    return _ext().linear_swiglu(x, w)
+
+
 # ------------------------------------------------------------------------------------------
 def varlen_attention_qkv(qkv, n_q: int, n_kv: int, head_dim: int, cu_seqlens, max_seqlen: int, causal: bool = True,
                          scale: Optional[float] = None):

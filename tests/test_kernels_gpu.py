@@ -316,6 +316,26 @@ def test_chained_kernels_see_their_predecessors(ext, T, H, F):
         assert torch.equal(chain(False), want)
 
 
+@pytest.mark.parametrize("T,K,F", [(256, 128, 128), (300, 264, 1000), (520, 2048, 136), (1000, 512, 4160), (16, 128, 256),
+                                   (765, 17920, 768)])
+def test_linear_swiglu_matches_the_two_passes(ext, T, K, F):
+    """Activation in the epilogue (ragged rows and columns of both halves) or, for few rows and divided reductions, behind it:
+    the bytes of product and activation one after the other, forward and backward, with and without gradients."""
+    torch.manual_seed(T + F)
+    x = torch.randn(2, T // 2, K, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(2 * F, K, device="cuda") / K ** 0.5).bfloat16().requires_grad_()
+    dy = torch.randn(2, T // 2, F, device="cuda").bfloat16()
+    y = ext.linear_swiglu(x, w)
+    want = ext.swiglu(ext.linear(x, w))
+    with torch.no_grad():
+        plain = ext.linear_swiglu(x, w)
+    torch.cuda.synchronize()
+    assert ext.kernel_status()[0].item() == 0, ext.kernel_status().tolist()
+    assert torch.equal(y, want) and torch.equal(plain, want)
+    for a, b in zip(torch.autograd.grad(y, [x, w], dy), torch.autograd.grad(want, [x, w], dy)):
+        assert torch.equal(a, b)
+
+
 def test_linear_autograd_matches_reference():
     from odc_b200 import ops
     x = torch.randn(3, 100, 512, device="cuda").bfloat16().requires_grad_()
