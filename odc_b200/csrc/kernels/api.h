@@ -118,7 +118,7 @@ cudaError_t gemm_bf16(const void* a, const void* b, void* c, int c_kind, const v
 size_t gemm_split_bytes(int M, int N, int K, int c_kind, int sm_count);
 
 // Same contract on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles).  Returns cudaErrorNotSupported for shapes it
-// does not take (M or N below 256, bf16 accumulation); gemm_bf16 tries it first unless ODC_GEMM_PAIR=0.
+// does not take (N below 256, M below 256 without split_ws, bf16 accumulation); gemm_bf16 tries it first unless ODC_GEMM_PAIR=0.
 cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, const void* bias, int M, int N, int K,
                            int layout, bool accumulate, long long lda, long long ldb, long long ldc, int* status,
                            int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0,

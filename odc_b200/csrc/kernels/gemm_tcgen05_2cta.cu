@@ -612,7 +612,7 @@ static int plan_splits(int M, int N, int K, int sm_count, int* kb_split) {
 
 size_t gemm_split_bytes(int M, int N, int K, int c_kind, int sm_count) {
   using namespace gemm_pair;
-  if (c_kind != kBF16 || M < 256 || N < 256 || K < BK || sm_count < 2) return 0;
+  if (c_kind != kBF16 || M < 1 || N < 256 || K < BK || sm_count < 2) return 0;
   int kb_split;
   const int splits = plan_splits(M, N, K, sm_count, &kb_split);
   return splits == 1 ? 0 : static_cast<size_t>(splits) * ((M + 255) / 256 * 256) * N * sizeof(float);
@@ -623,7 +623,9 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
                            int layout, bool accumulate, long long lda, long long ldb, long long ldc, int* status,
                            int sm_count, cudaStream_t stream, const void* residual, long long ldr, float* split_ws) {
   using namespace gemm_pair;
-  if (M < 256 || N < 256 || K < BK || sm_count < 2) return cudaErrorNotSupported;
+  // fewer rows than a tile are worth a pair only where several share the reduction (136 x 1536, K = 8960: 61 us on the
+  // single-CTA kernel, 23 us; 200 x 2048, K = 8192: 57 us, 25 us)
+  if ((M < 256 && split_ws == nullptr) || N < 256 || K < BK || sm_count < 2) return cudaErrorNotSupported;
   const bool a_mn = (layout == 2);
   const bool b_mn = (layout != 0);
   if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15)

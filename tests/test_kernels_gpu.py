@@ -270,7 +270,8 @@ def test_gemm_cta_pair_layouts(ext, layout, M, N, K):
 
 
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
-@pytest.mark.parametrize("M,N,K,divided", [(256, 256, 2048, True), (264, 264, 4040, True), (765, 1536, 17920, True),
+@pytest.mark.parametrize("M,N,K,divided", [(8, 256, 4096, True), (136, 1536, 8968, True), (255, 2048, 2048, False),
+                                           (256, 256, 2048, True), (264, 264, 4040, True), (765, 1536, 17920, True),
                                            (520, 1544, 8968, True), (768, 2048, 1536, False), (2304, 2304, 4096, False)])
 def test_gemm_divided_reduction(ext, layout, M, N, K, divided):
     """Few tiles and a long reduction: partial products and their sum, ragged tiles and a ragged last part included."""
