@@ -90,22 +90,28 @@ class SmallGroup:
         o, n = self.slots[name]
         return self.full[o:o + n].view(shape)
 
+    def _sinks(self, name: str):
+        """``(weight, fp32 buffer its kernel adds the gradient to)``.  The buffer counts as written from here on: the
+        kernels of a backward write it while it runs, and one that raises half way has written some of it."""
+        self.dirty = self.dirty or torch.is_grad_enabled()
+        return self._views[name]
+
     def norm(self, x, name: str, eps: float):
         if self.native:
-            w, sink = self._views[name]
+            w, sink = self._sinks(name)
             return ops._ext().rms_norm(x, w, eps, sink)
         return ops.rms_norm(x, self.view(name, (x.shape[-1],)), eps)
 
     def norm_residual(self, x, name: str, eps: float):
         if self.native:
-            w, sink = self._views[name]
+            w, sink = self._sinks(name)
             return ops._ext().rms_norm_residual(x, w, eps, sink)
         return ops.rms_norm_residual(x, self.view(name, (x.shape[-1],)), eps)
 
     def bias(self, name: str):
         """``(bias, fp32 buffer for its gradient or None)``"""
         if self.native:
-            return self._views[name]
+            return self._sinks(name)
         return self.view(name, (self.slots[name][1],)), None
 
     def flat(self):
@@ -118,6 +124,12 @@ class SmallGroup:
     def push(self) -> None:
         if self.dirty:
             L._service().scatter_accumulate(self.key, self.grad32, self.pg, scale=self.grad_scale)
+            self.clear()
+
+    @torch.no_grad()
+    def clear(self) -> None:
+        """Drop what has not been pushed (a pass that was given up)."""
+        if self.dirty:
             self.grad32.zero_()
             self.dirty = False
 
@@ -160,7 +172,6 @@ class _Embedding(torch.autograd.Function):
         model = ctx.model
         (ids,) = ctx.saved_tensors
         p = model.embed
-        model.small.dirty = True   # the lookup's backward is the last of a pass: every norm and bias has its gradient
         if _direct(p):
             service, reg = L._service(), SymmBufferRegistry.get_instance()
             ops._ext().embedding_scatter(ids.reshape(-1), dx.reshape(-1, dx.shape[-1]).contiguous(),
@@ -360,6 +371,7 @@ class FusedDecoderLM(nn.Module):
         """Zero the accumulators, publish this rank's freshly updated rows, pull the small group (collective)."""
         L.set_requires_gradient_sync(True)
         L.start_minibatch()
+        self.small.clear()
         self.small.refresh(self.gather)
 
     def set_requires_gradient_sync(self, flag: bool) -> None:

@@ -1,0 +1,91 @@
+"""The sharded decoder engine's gradients on one GPU, against the plain PyTorch decoder on the CPU (fp32)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = torch.device("cuda", 0)
+
+
+def _source(**over):
+    """A small decoder whose biases and norm weights are not their initial zeros and ones, every weight a bf16 value."""
+    from odc_b200.models import DecoderLM, get_config
+    cfg = get_config("tiny", **over)
+    src = DecoderLM(cfg)
+    src.reset_parameters(seed=0)
+    gen = torch.Generator().manual_seed(5)
+    with torch.no_grad():
+        for name, p in src.named_parameters():
+            if "norm" in name:
+                p.normal_(1.0, 0.1, generator=gen)
+            elif "bqkv" in name:
+                p.normal_(0.0, 0.05, generator=gen)
+            p.copy_(p.bfloat16())
+    return cfg, src
+
+
+def _batches(cfg, n=2, lo=16, hi=128, tokens=512, seed=0):
+    from odc_b200.data import LengthSpec, make_minibatch
+    return make_minibatch(0, 0, cfg.vocab_size, LengthSpec("uniform", lo=lo, hi=hi), n, tokens, seed=seed)
+
+
+def _args(mb):
+    return mb["input_ids"], mb["position_ids"], mb["cu_seqlens"], mb["max_seqlen"]
+
+
+class _Engine:
+    def __init__(self, **over):
+        import odc_b200 as odc
+        from odc_b200.parallel import FusedDecoderLM
+        self.cfg, self.src = _source(**over)
+        odc.init_nvshmem(DEV, 2 << 30)
+        self.model = FusedDecoderLM(self.cfg, device=DEV, source=self.src)
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.model.stop()
+
+    def minibatch(self, mbs, factor=1.0, sync=None):
+        """One minibatch; the accumulators by parameter name.  ``sync``: synchronisation on or off per microbatch."""
+        from odc_b200.data import to_device
+        self.model.start_minibatch()
+        for i, mb in enumerate(mbs):
+            if sync is not None:
+                self.model.set_requires_gradient_sync(sync[i])
+            mb = to_device(mb, DEV)
+            (factor * self.model(*_args(mb), labels=mb["labels"], loss_scale=mb["loss_scale"])).backward()
+        self.model.finish_minibatch()
+        return self.grads()
+
+    def grads(self):
+        out = {name: p.grad()[:p.out_features].clone() for name, p in self.model.matrices().items()}
+        out.update({name: self.model.small.acc[o:o + n].clone() for name, (o, n) in self.model.small.slots.items()})
+        return out
+
+
+def _rel(got, want):
+    want = want.double()
+    return ((got.double().to(want.device).reshape(want.shape) - want).norm() / want.norm()).item()
+
+
+def test_gradients_of_an_abandoned_pass_do_not_reach_the_next_minibatch():
+    """A backward that raised half way has already added the norm gradients of the layers behind it."""
+    from odc_b200.data import to_device
+    with _Engine() as e:
+        mbs = _batches(e.cfg)
+        clean = e.minibatch(mbs)
+        mb = to_device(mbs[0], DEV)
+
+        def fail(grad):
+            raise RuntimeError("abandoned")
+
+        handle = e.model.layers[0].register_forward_hook(lambda mod, args, out: out.register_hook(fail) and None)
+        e.model.start_minibatch()
+        with pytest.raises(RuntimeError, match="abandoned"):
+            e.model(*_args(mb), labels=mb["labels"], loss_scale=mb["loss_scale"]).backward()
+        handle.remove()
+        again = e.minibatch(mbs)
+        for name, want in clean.items():   # the same sums, in another order of additions
+            assert _rel(again[name], want) < 1e-3, name
