@@ -231,7 +231,7 @@ class ShardedParameter:
 
 class _OdcLinearFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, bias, residual, layer):
+    def forward(ctx, x, bias, residual, layer, bias_sink):
         p = layer.weight
         if p.world == 1:
             w_full = p.lowp[:p.out_features]      # the shard is the matrix: nothing to pull
@@ -247,6 +247,7 @@ class _OdcLinearFn(torch.autograd.Function):
             y, w_full = fused.gather_linear(x, p.lowp, p.out_features, p.pg, bias, residual)
         ctx.layer = layer
         ctx.has_bias = bias is not None
+        ctx.bias_sink = bias_sink
         if layer.keep_weight and p.world > 1:
             ctx.save_for_backward(x, w_full)
         else:
@@ -273,10 +274,12 @@ class _OdcLinearFn(torch.autograd.Function):
                 dx = fused.gather_dgrad(dy2, p.lowp, p.out_features, p.pg)[0].view(x.shape)
         accumulate_weight_grad(p, dy2, x2)
         db = None
-        if ctx.has_bias and ctx.needs_input_grad[1]:
+        if ctx.bias_sink is not None:
+            ctx.bias_sink.add_(dy2.float().sum(0))
+        elif ctx.has_bias and ctx.needs_input_grad[1]:
             db = dy2.float().sum(0).to(dy.dtype)
         dres = dy if ctx.needs_input_grad[2] else None
-        return dx, db, dres, None
+        return dx, db, dres, None, None
 
 
 def _deferred_weight_grad(i: int, dy2: torch.Tensor, x2: torch.Tensor) -> None:
@@ -321,15 +324,14 @@ class OdcLinear(nn.Module):
         return self.weight.grad_scale
 
     def forward(self, x, bias=None, residual=None, bias_sink=None):
-        """``bias_sink``: fp32 vector the kernel adds the bias gradient to (native layer only; the bias then gets none)."""
+        """``bias_sink``: fp32 vector the bias gradient is added to (the bias then gets none)."""
         bias = bias if bias is not None else self.bias
         m = self.weight._matrix
         if m is None:
             m = self.weight.matrix(self.keep_weight)
         if m and x.is_cuda and os.environ.get("ODC_WGRAD_SCATTER", "tma") == "tma":
             return ops._ext().sharded_linear(x, bias, residual, m, bias_sink)
-        assert bias_sink is None
-        return _OdcLinearFn.apply(x, bias, residual, self)
+        return _OdcLinearFn.apply(x, bias, residual, self, bias_sink)
 
 
 def sharded_parameters() -> List[ShardedParameter]:

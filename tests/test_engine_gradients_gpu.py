@@ -65,6 +65,11 @@ class _Engine:
         return out
 
 
+# About 20 values on the way through a layer and back are rounded to bf16 (2^-9 each, P and dS of the attention among them);
+# with two layers and the head some 50 independent roundings, sqrt(50) * 2^-9 = 1.4e-2 of a gradient's norm at most.
+CHAIN = 2e-2
+
+
 def _rel(got, want):
     want = want.double()
     return ((got.double().to(want.device).reshape(want.shape) - want).norm() / want.norm()).item()
@@ -89,3 +94,21 @@ def test_gradients_of_an_abandoned_pass_do_not_reach_the_next_minibatch():
         again = e.minibatch(mbs)
         for name, want in clean.items():   # the same sums, in another order of additions
             assert _rel(again[name], want) < 1e-3, name
+
+
+@pytest.mark.parametrize("route", ["tma", "red", "other nodes"])
+def test_qkv_bias_gradient_on_every_route(monkeypatch, route):
+    """The native layer adds the bias gradient in its kernel; the Python layer runs with per-thread reductions asked for,
+    and in groups whose rows are not all mapped here."""
+    from odc_b200.parallel import ShardedParameter
+    if route == "other nodes":
+        monkeypatch.setattr(ShardedParameter, "reaches_other_nodes", lambda self: True)
+    else:
+        monkeypatch.setenv("ODC_WGRAD_SCATTER", route)
+    with _Engine(qkv_bias=True, tie_embeddings=True) as e:
+        mbs = _batches(e.cfg)
+        got = e.minibatch(mbs)
+        for mb in mbs:
+            e.src(*_args(mb), labels=mb["labels"], loss_scale=mb["loss_scale"]).backward()
+        for name, p in e.src.named_parameters():
+            assert _rel(got[name], p.grad) < CHAIN, name
