@@ -77,8 +77,7 @@ class SmallGroup:
         if self.native:
             flat = self.full.detach()
             self._views = {name: (flat[o:o + n], self.grad32[o:o + n]) for name, (o, n) in self.slots.items()}
-        else:
-            self.full.register_post_accumulate_grad_hook(self._fold)
+        self.full.register_post_accumulate_grad_hook(self._fold)
 
     def _fold(self, leaf):
         # one low-precision gradient per backward pass; the running sum over microbatches is kept in fp32
@@ -90,29 +89,31 @@ class SmallGroup:
         o, n = self.slots[name]
         return self.full[o:o + n].view(shape)
 
-    def _sinks(self, name: str):
-        """``(weight, fp32 buffer its kernel adds the gradient to)``.  The buffer counts as written from here on: the
-        kernels of a backward write it while it runs, and one that raises half way has written some of it."""
+    def _sinks(self, x, name: str):
+        """``(weight, fp32 buffer its kernel adds the gradient to)``, or None for the weight as a part of the gathered leaf:
+        on CPU, and for an input that needs no gradient itself, where only the leaf makes autograd call the backward.
+        The buffer counts as written from here on: the kernels of a backward write it while it runs, and one that raises
+        half way has written some of it."""
+        if not self.native or (torch.is_grad_enabled() and not x.requires_grad):
+            return None
         self.dirty = self.dirty or torch.is_grad_enabled()
         return self._views[name]
 
     def norm(self, x, name: str, eps: float):
-        if self.native:
-            w, sink = self._sinks(name)
-            return ops._ext().rms_norm(x, w, eps, sink)
+        sinks = self._sinks(x, name)
+        if sinks is not None:
+            return ops._ext().rms_norm(x, sinks[0], eps, sinks[1])
         return ops.rms_norm(x, self.view(name, (x.shape[-1],)), eps)
 
     def norm_residual(self, x, name: str, eps: float):
-        if self.native:
-            w, sink = self._sinks(name)
-            return ops._ext().rms_norm_residual(x, w, eps, sink)
+        sinks = self._sinks(x, name)
+        if sinks is not None:
+            return ops._ext().rms_norm_residual(x, sinks[0], eps, sinks[1])
         return ops.rms_norm_residual(x, self.view(name, (x.shape[-1],)), eps)
 
-    def bias(self, name: str):
-        """``(bias, fp32 buffer for its gradient or None)``"""
-        if self.native:
-            return self._sinks(name)
-        return self.view(name, (self.slots[name][1],)), None
+    def bias(self, x, name: str):
+        """``(bias, fp32 buffer for its gradient or None)`` of a layer whose input is ``x``"""
+        return self._sinks(x, name) or (self.view(name, (self.slots[name][1],)), None)
 
     def flat(self):
         return self.master, self.acc, self.m, self.v, self.lowp
@@ -284,7 +285,7 @@ class FusedDecoderLayer(nn.Module):
         c, s, i = self.cfg, self.small, self.i
         T = x.shape[0]
         h, x = s.norm_residual(x, f"layers.{i}.attn_norm.weight", c.rms_eps)
-        bias, sink = s.bias(f"layers.{i}.attn.bqkv") if c.qkv_bias else (None, None)
+        bias, sink = s.bias(h, f"layers.{i}.attn.bqkv") if c.qkv_bias else (None, None)
         qkv = self.wqkv(h, bias=bias, bias_sink=sink)
         qkv = ops.rope_qkv(qkv, position_ids, c.num_heads, c.num_kv_heads, c.head_dim, c.rope_theta,
                            c.rope_inv_freq(qkv.device))

@@ -112,3 +112,22 @@ def test_qkv_bias_gradient_on_every_route(monkeypatch, route):
             e.src(*_args(mb), labels=mb["labels"], loss_scale=mb["loss_scale"]).backward()
         for name, p in e.src.named_parameters():
             assert _rel(got[name], p.grad) < CHAIN, name
+
+
+@pytest.mark.parametrize("leaf", [False, True])
+def test_a_layer_on_its_own(leaf):
+    """A layer that is called with activations of its own, which need a gradient or not, still gets all its gradients."""
+    with _Engine(qkv_bias=True) as e:
+        mb = _batches(e.cfg, n=1)[0]
+        where = tuple(t.to(DEV) if torch.is_tensor(t) else t for t in _args(mb)[1:])
+        T = mb["input_ids"].numel()
+        gen = torch.Generator().manual_seed(9)
+        x = torch.randn(T, e.cfg.hidden_size, generator=gen).bfloat16()
+        dy = torch.randn(T, e.cfg.hidden_size, generator=gen).bfloat16()
+        e.model.start_minibatch()
+        e.model.layers[0](x.to(DEV).requires_grad_(leaf), *where).backward(dy.to(DEV))
+        e.model.finish_minibatch()
+        got = e.grads()
+        e.src.layers[0](x.float(), *_args(mb)[1:]).backward(dy.float())
+        for name, p in e.src.layers[0].named_parameters():
+            assert _rel(got[f"layers.0.{name}"], p.grad) < CHAIN, name
