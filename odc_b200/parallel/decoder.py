@@ -77,15 +77,20 @@ class SmallGroup:
         if self.native:
             flat = self.full.detach()
             self._views = {name: (flat[o:o + n], self.grad32[o:o + n]) for name, (o, n) in self.slots.items()}
-        self.full.register_post_accumulate_grad_hook(self._fold)
+        self._folds = False
 
     def _fold(self, leaf):
         # one low-precision gradient per backward pass; the running sum over microbatches is kept in fp32
+        if leaf.grad is None:   # a pass that only the lookup tied to the leaf
+            return
         self.grad32.add_(leaf.grad)
         leaf.grad = None
         self.dirty = True
 
     def view(self, name: str, shape) -> torch.Tensor:
+        if not self._folds:
+            self._folds = True
+            self.full.register_post_accumulate_grad_hook(self._fold)
         o, n = self.slots[name]
         return self.full[o:o + n].view(shape)
 
