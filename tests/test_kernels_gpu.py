@@ -209,6 +209,17 @@ def test_adamw_accesses(ext, n, skip, grad):
     assert torch.equal(low, p.bfloat16())
 
 
+@pytest.mark.parametrize("n,skip", [(4096, 0), (4097, 0), (4099, 0), (4097, 1)])
+def test_adamw_is_one_launch(ext, n, skip):
+    """A remainder of four has no launch of its own (2 us, a fifth of the update of two million elements)."""
+    p, m, v, g = (torch.rand(n + skip, device="cuda")[skip:] for _ in range(4))
+    ext.adamw_step(p, g, m, v, None, 1e-2, 0.9, 0.95, 1e-8, 0.1, 1, 1.0)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ext.adamw_step(p, g, m, v, None, 1e-2, 0.9, 0.95, 1e-8, 0.1, 2, 1.0)
+        torch.cuda.synchronize()
+    assert sum("adamw" in e.name for e in prof.events()) == 1
+
+
 # ------------------------------------------------------------------------------------ GEMM
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (256, 512, 256), (300, 1376, 200), (1000, 264, 1032),
