@@ -156,8 +156,11 @@ class SmallGroup:
 
 
 def _direct(p: ShardedParameter) -> bool:
-    """True when a gradient of ``p`` can go straight to the owners: pushes are on, nothing waits in the local buffer and
-    all owners are mapped."""
+    """True when a gradient of ``p`` can go straight to the owners: pushes are on, nothing waits in the local buffer, all
+    owners are mapped, and the order of additions is free.  The head's push on the side stream and the lookup's atomic rows
+    meet in one accumulator in any order; in the local buffer they are added one after the other."""
+    if L._service().deterministic or torch.are_deterministic_algorithms_enabled():
+        return False
     return L.requires_gradient_sync() and not p.local_dirty and bool(p.matrix())
 
 

@@ -131,3 +131,22 @@ def test_a_layer_on_its_own(leaf):
         e.src.layers[0](x.float(), *_args(mb)[1:]).backward(dy.float())
         for name, p in e.src.layers[0].named_parameters():
             assert _rel(got[f"layers.0.{name}"], p.grad) < CHAIN, name
+
+
+@pytest.mark.parametrize("switch", ["ODC_DETERMINISTIC", "torch"])
+def test_embedding_gradient_is_reproducible_where_that_is_asked_for(monkeypatch, switch):
+    """A tied matrix gets the head's gradient and rows of the lookup, many for one token: with either switch they are
+    added in one order.  Sequences of one key tile: the attention's own sums over key tiles have no fixed order."""
+    if switch == "ODC_DETERMINISTIC":   # per-producer slots, and column sums in a fixed order
+        monkeypatch.setenv(switch, "1")
+    torch.use_deterministic_algorithms(True)
+    try:
+        with _Engine(tie_embeddings=True) as e:
+            mbs = _batches(e.cfg, lo=64, hi=128, tokens=2048)
+            for mb in mbs:
+                mb["input_ids"] = mb["input_ids"] % 3
+            runs = [e.minibatch(mbs)["embed.weight"] for _ in range(6)]
+            same = [torch.equal(runs[0], r) for r in runs[1:]]
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert all(same), same
