@@ -183,7 +183,8 @@ class _Embedding(torch.autograd.Function):
         p = model.embed
         if _direct(p):
             service, reg = L._service(), SymmBufferRegistry.get_instance()
-            ops._ext().embedding_scatter(ids.reshape(-1), dx.reshape(-1, dx.shape[-1]).contiguous(),
+            ops._ext().embedding_scatter(ids.reshape(-1).to(torch.int64).contiguous(),
+                                         dx.reshape(-1, dx.shape[-1]).contiguous(),
                                          reg.peer_ptr_table(service.scatter_target(p.key), p.ranks),
                                          reg.peer_ptr_table(service.counter, p.ranks), p.rows_per_rank, p.out_features,
                                          p.grad_scale)

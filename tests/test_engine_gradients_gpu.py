@@ -150,3 +150,23 @@ def test_embedding_gradient_is_reproducible_where_that_is_asked_for(monkeypatch,
     finally:
         torch.use_deterministic_algorithms(False)
     assert all(same), same
+
+
+@pytest.mark.parametrize("form", ["int32", "strided"])
+def test_token_ids_of_any_integer_form(form):
+    """Ids as 32-bit integers or as a column of a wider array: the gradients of plain contiguous ids."""
+    from odc_b200.data import to_device
+    with _Engine(tie_embeddings=True) as e:
+        mb = to_device(_batches(e.cfg, n=1)[0], DEV)
+        ids = mb["input_ids"]
+        other = {"int32": ids.int(), "strided": torch.stack([ids, ids + 1], 1)[:, 0]}[form]
+
+        def grads(ids):
+            e.model.start_minibatch()
+            x = e.model.hidden_states(ids, *_args(mb)[1:])
+            x.backward(torch.ones_like(x))
+            e.model.finish_minibatch()
+            return e.grads()["embed.weight"]
+
+        want, got = grads(ids), grads(other)
+        assert want.norm() > 0 and _rel(got, want) < 1e-3
