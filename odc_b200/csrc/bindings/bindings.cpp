@@ -249,6 +249,7 @@ void embedding_scatter(Tensor ids, Tensor dx, Tensor acc_table, Tensor ctr_table
   TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && dx.dim() == 2 && dx.is_contiguous() &&
                   dx.scalar_type() == at::kBFloat16 && ids.numel() == dx.size(0) && dx.size(1) % 8 == 0,
               "embedding_scatter: int64 ids [T], contiguous bf16 gradient [T, H], H a multiple of 8");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(dx.data_ptr()) % 16 == 0, "embedding_scatter: the gradient starts on 16 bytes");
   TORCH_CHECK(vocab <= rows_per_rank * acc_table.numel(), "embedding_scatter: more rows than the owners hold");
   check(odc::launch_embedding_scatter(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), dx.data_ptr(),
                                       static_cast<int>(dx.size(0)), static_cast<int>(dx.size(1)),

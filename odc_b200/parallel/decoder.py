@@ -183,8 +183,10 @@ class _Embedding(torch.autograd.Function):
         p = model.embed
         if _direct(p):
             service, reg = L._service(), SymmBufferRegistry.get_instance()
-            ops._ext().embedding_scatter(ids.reshape(-1).to(torch.int64).contiguous(),
-                                         dx.reshape(-1, dx.shape[-1]).contiguous(),
+            dx2 = dx.reshape(-1, dx.shape[-1]).contiguous()
+            if dx2.data_ptr() % 16:   # read 16 bytes at a time
+                dx2 = dx2.clone()
+            ops._ext().embedding_scatter(ids.reshape(-1).to(torch.int64).contiguous(), dx2,
                                          reg.peer_ptr_table(service.scatter_target(p.key), p.ranks),
                                          reg.peer_ptr_table(service.counter, p.ranks), p.rows_per_rank, p.out_features,
                                          p.grad_scale)
