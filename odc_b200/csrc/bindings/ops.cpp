@@ -329,10 +329,13 @@ bool env_on(const char* name) {
   return e != nullptr && *e != 0 && std::strcmp(e, "0") != 0 && std::strcmp(e, "false") != 0;
 }
 bool wants_grad(const Tensor& t) { return at::GradMode::is_enabled() && t.defined() && t.requires_grad(); }
-// sum over the rows of a bf16 gradient (the bias gradient), fp32 inside
+// sum over the rows of a gradient (the bias gradient), fp32 inside
 Tensor column_sum(const Tensor& x) {
   c10::cuda::CUDAGuard g(x.device());
-  TORCH_CHECK(x.dim() == 2 && x.is_contiguous() && x.scalar_type() == at::kBFloat16, "column_sum: contiguous bf16 [T,N]");
+  TORCH_CHECK(x.dim() == 2 && x.is_contiguous(), "column_sum: contiguous [T,N]");
+  // the kernel reads bf16, 16 bytes at a time; gradients of library products come in other types and widths too
+  if (x.scalar_type() != at::kBFloat16 || x.size(1) % 8 != 0 || reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 != 0)
+    return x.sum(0, false, at::kFloat).to(x.scalar_type());
   auto out = at::empty({x.size(1)}, x.options());
   check(odc::launch_column_sum(x.data_ptr(), out.data_ptr(), nullptr, x.size(0), static_cast<int>(x.size(1)), cur_stream()),
         "column_sum");

@@ -365,6 +365,32 @@ def test_linear_autograd_matches_reference():
     torch.testing.assert_close(b.grad.float(), br.grad, rtol=2e-2, atol=0.5)
 
 
+def test_bias_gradient_that_starts_off_a_16_byte_boundary():
+    """Only the bias is trained, so no product looks at the gradient's start; column sums of 700 small whole numbers."""
+    from odc_b200 import ops
+    x, w = torch.randn(700, 512, device="cuda").bfloat16(), torch.randn(264, 512, device="cuda").bfloat16()
+    b = torch.zeros(264, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    for skip in (0, 1, 4):
+        dy = torch.randint(-1, 2, (700 * 264 + skip,), device="cuda").bfloat16()[skip:].view(700, 264)
+        got, = torch.autograd.grad(ops.linear(x, w, b), [b], dy)
+        assert torch.equal(got, dy.float().sum(0).bfloat16())
+
+
+@pytest.mark.parametrize("dtype,N", [(torch.float32, 264), (torch.float16, 264), (torch.bfloat16, 12)])
+def test_linear_on_library_products_in_other_types_and_widths(monkeypatch, dtype, N):
+    """ODC_GEMM=cublas takes what the library takes; bias gradients of whole numbers are exact."""
+    from odc_b200 import ops
+    monkeypatch.setenv("ODC_GEMM", "cublas")
+    x, w = torch.randn(100, 64, device="cuda", dtype=dtype), torch.randn(N, 64, device="cuda", dtype=dtype, requires_grad=True)
+    b = torch.randn(N, device="cuda", dtype=dtype, requires_grad=True)
+    dy = torch.randint(-1, 2, (100, N), device="cuda").to(dtype)
+    y = ops.linear(x, w, b)
+    assert y.dtype == dtype
+    dw, db = torch.autograd.grad(y, [w, b], dy)
+    assert torch.equal(db, dy.float().sum(0).to(dtype))
+    assert torch.equal(dw, dy.t() @ x)
+
+
 def test_linear_cross_entropy_matches_reference():
     from odc_b200 import ops
     from odc_b200.ops import reference as ref
