@@ -586,6 +586,11 @@ Tensor attention_qkv(Tensor qkv, int64_t n_q, int64_t n_kv, int64_t d, Tensor cu
 }
 
 // ---- LM head ---------------------------------------------------------------------------------------------------------
+// bf16 logits of one chunk of tokens, whatever type a library product of the head is in
+Tensor chunk_logits(const Tensor& h, int64_t vocab, int64_t chunk) {
+  return at::empty({std::min(chunk, h.size(0)), vocab}, h.options().dtype(at::kBFloat16));
+}
+
 // Loss and both gradients (for a loss gradient of one) in one pass over token chunks; [T, vocab] logits never exist.
 // Same mathematics as the reference's chunked LM head (examples/llm_training/lm_head.py:7-59), but the gradients are
 // formed while the chunk's logits are at hand, so backward is a multiplication by the loss gradient.
@@ -594,7 +599,7 @@ std::tuple<Tensor, Tensor, Tensor> lm_head_loss(const Tensor& h, const Tensor& w
                                                 bool need_dh, bool need_dw, c10::optional<Tensor> dw_out) {
   const int64_t T = h.size(0), V = w.size(0), H = h.size(1);
   auto loss = at::zeros({}, h.options().dtype(at::kFloat));
-  auto logits = at::empty({std::min(chunk, T), V}, h.options());
+  auto logits = chunk_logits(h, V, chunk);
   Tensor dh, dw;
   if (need_dh) dh = at::empty_like(h);
   if (need_dw) dw = dw_out.has_value() ? *dw_out : at::empty({V, H}, h.options().dtype(at::kFloat));
@@ -645,7 +650,7 @@ struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
                         int64_t chunk, bool need_dh, bool need_dw) {
     const int64_t T = h.size(0);
     auto out = at::empty({T}, h.options().dtype(at::kFloat));
-    auto logits = at::empty({std::min(chunk, T), w.size(0)}, h.options());
+    auto logits = chunk_logits(h, w.size(0), chunk);
     for (int64_t s = 0; s < T; s += chunk) {
       const int64_t n = std::min(chunk, T - s);
       const Tensor lg = logits.narrow(0, 0, n);
@@ -671,7 +676,7 @@ struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
     if (T == 0 && cfg[3]) dw.zero_();
     const Tensor scale = (grads[0].reshape({-1}).to(at::kFloat) * (-1.0 / temperature)).contiguous();
     auto sink = at::zeros({}, scale.options());  // the kernel's loss output is not used here
-    auto logits = at::empty({std::min(chunk, T), w.size(0)}, h.options());
+    auto logits = chunk_logits(h, w.size(0), chunk);
     for (int64_t s = 0; s < T; s += chunk) {
       const int64_t n = std::min(chunk, T - s);
       const Tensor hs = h.narrow(0, s, n), lg = logits.narrow(0, 0, n);

@@ -391,6 +391,19 @@ def test_linear_on_library_products_in_other_types_and_widths(monkeypatch, dtype
     assert torch.equal(dw, dy.t() @ x)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_lm_head_on_library_products_in_other_types(monkeypatch, dtype):
+    """ODC_GEMM=cublas scores hidden states of any type; the logits are rounded to bf16 (2^-9 of values up to about 4)."""
+    from odc_b200 import ops
+    monkeypatch.setenv("ODC_GEMM", "cublas")
+    h, w = torch.randn(100, 64, device="cuda", dtype=dtype), (torch.randn(512, 64, device="cuda") / 8).to(dtype)
+    ids = torch.randint(0, 512, (100,), device="cuda")
+    want = (h.double() @ w.double().t()).log_softmax(-1).gather(-1, ids[:, None])[:, 0]
+    with torch.no_grad():
+        torch.testing.assert_close(ops.linear_token_logprobs(h, w, ids).double(), want, rtol=0, atol=2e-2)
+        torch.testing.assert_close(ops.linear_cross_entropy(h, w, ids).double(), -want.sum(), rtol=5e-3, atol=0)
+
+
 def test_linear_cross_entropy_matches_reference():
     from odc_b200 import ops
     from odc_b200.ops import reference as ref
