@@ -199,6 +199,8 @@ def linear_token_logprobs(h, w, ids, temperature: float = 1.0, ignore_index: int
     flat = ids.reshape(-1).to(torch.int64)
     if not h.is_cuda:
         return ref.linear_token_logprobs(h2, w, flat, temperature, ignore_index, chunk).view(shape)
+    if temperature == 0 and flat.numel():
+        raise ZeroDivisionError("temperature of zero")
     return _ext().linear_token_logprobs(h2, w, flat, float(temperature), ignore_index, chunk).view(shape)
 
 

@@ -493,6 +493,17 @@ def test_wgrad_scatter_emulated_ranks(ext, world, T, n_out, k_in):
         assert int(ctrs[r][0]) == 2
 
 
+def test_lm_head_refuses_a_chunk_or_temperature_of_zero():
+    from odc_b200 import ops
+    h, w = torch.randn(8, 64, device="cuda").bfloat16(), torch.randn(512, 64, device="cuda").bfloat16()
+    ids = torch.randint(0, 512, (8,), device="cuda")
+    for call in (ops.linear_cross_entropy, ops.linear_token_logprobs):
+        with pytest.raises(ValueError):
+            call(h, w, ids, chunk=0)
+    with pytest.raises(ZeroDivisionError):
+        ops.linear_token_logprobs(h, w, ids, temperature=0.0)
+
+
 @pytest.mark.parametrize("world", [1, 2, 8])
 @pytest.mark.parametrize("M,N,K", [(256, 512, 256), (1000, 1376, 512), (8192, 3072, 2048), (300, 264, 128)])
 def test_gemm_gather_emulated_ranks(ext, world, M, N, K):
