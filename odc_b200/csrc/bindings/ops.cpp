@@ -710,7 +710,6 @@ struct ShardedMatrix : torch::CustomClassHolder {
   std::vector<int64_t> acc_addrs;
   int64_t out_features = 0, rows_per_rank = 0, world = 1, index = 0;
   double grad_scale = 1.0;
-  bool keep_weight = false;
   bool local_pending = false;           // earlier microbatches left a gradient in the local buffer
   c10::intrusive_ptr<DispatchCounter> dispatched;
   Tensor whole() const { return shard.narrow(0, 0, out_features); }
@@ -723,8 +722,8 @@ py::object* g_deferred = nullptr;       // Python: (id, dy2, x2) of a gradient t
 // gradient is added into its owners from the epilogue of its product.  The weight is no autograd input.
 struct ShardedLinearFn : Function<ShardedLinearFn> {
   static Tensor forward(AutogradContext* ctx, Tensor x, c10::optional<Tensor> bias, c10::optional<Tensor> residual,
-                        c10::intrusive_ptr<ShardedMatrix> m, c10::optional<Tensor> bias_sink, bool need_dx, bool need_db,
-                        bool need_dres) {
+                        c10::intrusive_ptr<ShardedMatrix> m, c10::optional<Tensor> bias_sink, bool keep_weight, bool need_dx,
+                        bool need_db, bool need_dres) {
     const Tensor x2 = rows2d(x);
     c10::optional<Tensor> res;
     if (residual.has_value()) res = rows2d(*residual);
@@ -736,7 +735,7 @@ struct ShardedLinearFn : Function<ShardedLinearFn> {
       y = gemm_gather(x2, m->table, w_full, bias, m->rows_per_rank, m->index, res);
       count();
     }
-    if (!m->keep_weight) w_full = Tensor();  // dropped: backward pulls the shards again
+    if (!keep_weight) w_full = Tensor();  // dropped: backward pulls the shards again
     ctx->save_for_backward({x, w_full});
     ctx->saved_data["need"] = static_cast<int64_t>(need_dx | need_db << 1 | need_dres << 2);
     if (bias_sink.has_value()) ctx->saved_data["sink"] = *bias_sink;
@@ -782,13 +781,13 @@ struct ShardedLinearFn : Function<ShardedLinearFn> {
     } else if (need & 2) {
       db = column_sum(dy2);
     }
-    return {dx, db, (need & 4) ? grads[0] : Tensor(), {}, {}, {}, {}, {}};
+    return {dx, db, (need & 4) ? grads[0] : Tensor(), {}, {}, {}, {}, {}, {}};
   }
 };
 Tensor sharded_linear(Tensor x, c10::optional<Tensor> bias, c10::optional<Tensor> residual, c10::intrusive_ptr<ShardedMatrix> m,
-                      c10::optional<Tensor> bias_sink) {
+                      c10::optional<Tensor> bias_sink, bool keep_weight) {
   const bool db = bias.has_value() && wants_grad(*bias), dres = residual.has_value() && wants_grad(*residual);
-  return ShardedLinearFn::apply(x, bias, residual, m, bias_sink, wants_grad(x), db, dres);
+  return ShardedLinearFn::apply(x, bias, residual, m, bias_sink, keep_weight, wants_grad(x), db, dres);
 }
 
 }  // namespace
@@ -821,14 +820,13 @@ void register_ops(py::module_& m) {
       .def("take", &DispatchCounter::take);
   py::class_<ShardedMatrix, c10::intrusive_ptr<ShardedMatrix>>(m, "ShardedMatrix")
       .def(py::init([](int64_t id, Tensor shard, Tensor table, Tensor acc_table, Tensor ctr_table, std::vector<int64_t> acc_addrs,
-                       int64_t out_features, int64_t index, double grad_scale, bool keep_weight,
-                       c10::intrusive_ptr<DispatchCounter> dispatched) {
+                       int64_t out_features, int64_t index, double grad_scale, c10::intrusive_ptr<DispatchCounter> dispatched) {
         auto p = c10::make_intrusive<ShardedMatrix>();
         p->id = id; p->shard = shard; p->table = table; p->acc_table = acc_table; p->ctr_table = ctr_table;
         p->world = static_cast<int64_t>(acc_addrs.size());
         p->acc_addrs = std::move(acc_addrs);
         p->out_features = out_features; p->rows_per_rank = shard.size(0); p->index = index; p->grad_scale = grad_scale;
-        p->keep_weight = keep_weight; p->dispatched = dispatched;
+        p->dispatched = dispatched;
         return p;
       }))
       .def_readwrite("local_pending", &ShardedMatrix::local_pending);
@@ -839,7 +837,7 @@ void register_ops(py::module_& m) {
   });
   // differentiable forms
   m.def("sharded_linear", &sharded_linear, py::arg("x"), py::arg("bias"), py::arg("residual"), py::arg("matrix"),
-        py::arg("bias_sink") = py::none());
+        py::arg("bias_sink") = py::none(), py::arg("keep_weight") = false);
   m.def("linear", &linear, py::arg("x"), py::arg("w"), py::arg("bias") = py::none(), py::arg("residual") = py::none());
   m.def("rms_norm", &rms_norm, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());
   m.def("rms_norm_residual", &rms_norm_residual, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());

@@ -128,7 +128,7 @@ class ShardedParameter:
     def reaches_other_nodes(self) -> bool:
         return fused._spans_nodes(SymmBufferRegistry.get_instance(), self.ranks)
 
-    def matrix(self, keep_weight: bool = False):
+    def matrix(self):
         """What the native layer needs of this parameter (addresses of the owners' rows, accumulators and counters), or
         False where the data path is not the mapped heap alone (CPU ranks, groups that span nodes)."""
         if self._matrix is None:
@@ -143,7 +143,7 @@ class ShardedParameter:
                 self._matrix = ext.ShardedMatrix(
                     _params.index(self), self.lowp, reg.peer_ptr_table(self.lowp, self.ranks),
                     reg.peer_ptr_table(target, self.ranks), reg.peer_ptr_table(service.counter, self.ranks),
-                    reg.peer_ptrs(target, self.ranks), self.out_features, self.index, self.grad_scale, keep_weight,
+                    reg.peer_ptrs(target, self.ranks), self.out_features, self.index, self.grad_scale,
                     service.native_dispatches(self.ranks))
                 self._matrix.local_pending = self._local_dirty
                 ext.set_deferred_weight_grad(_deferred_weight_grad)
@@ -328,9 +328,9 @@ class OdcLinear(nn.Module):
         bias = bias if bias is not None else self.bias
         m = self.weight._matrix
         if m is None:
-            m = self.weight.matrix(self.keep_weight)
+            m = self.weight.matrix()
         if m and x.is_cuda and os.environ.get("ODC_WGRAD_SCATTER", "tma") == "tma":
-            return ops._ext().sharded_linear(x, bias, residual, m, bias_sink)
+            return ops._ext().sharded_linear(x, bias, residual, m, bias_sink, self.keep_weight)
         return _OdcLinearFn.apply(x, bias, residual, self, bias_sink)
 
 
