@@ -236,14 +236,16 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
         p = model.head_param()
         if _direct(p):
             p.push_direct(dw32, dloss)
-            return ops._ext().scale_to_bf16(dh, dloss), None, None, None, None, None
+            return gh, None, None, None, None, None
+        # one rounding from an fp32 factor, whether or not this microbatch's weight gradients are pushed now
+        gh = ops._ext().scale_to_bf16(dh, dloss) if dh.is_cuda and dh.dtype == torch.bfloat16 else dh * dloss.to(dh.dtype)
         p.wait_push()
         buf = p.local_buffer()
         buf[:p.out_features].addcmul_(dw32[:p.out_features], dloss.to(dw32.dtype))
         p.local_dirty = True
         if p is not model.embed and L.requires_gradient_sync():
             p.push_local(side_stream=True)   # a tied matrix is pushed by the lookup's backward, which runs last
-        return dh * dloss.to(dh.dtype), None, None, None, None, None
+        return gh, None, None, None, None, None
 
 
 class _FusedTokenLogProbs(torch.autograd.Function):

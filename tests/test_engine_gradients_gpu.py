@@ -170,3 +170,16 @@ def test_token_ids_of_any_integer_form(form):
 
         want, got = grads(ids), grads(other)
         assert want.norm() > 0 and _rel(got, want) < 1e-3
+
+
+@pytest.mark.parametrize("tied", [True, False])
+def test_activation_gradients_do_not_depend_on_deferral(tied):
+    """A loss factor that bf16 cannot hold (1/3, off by 2^-9 when rounded): the layers' gradients of a microbatch are the
+    same whether its weight gradients are pushed at once or held back.  Both forms round the same bf16 activations, so the
+    difference is that of fp32 sums."""
+    with _Engine(tie_embeddings=tied) as e:
+        mbs = _batches(e.cfg, n=2, lo=64, hi=128)   # one key tile per sequence: no sums in a free order
+        now = e.minibatch(mbs, factor=1 / 3)
+        held = e.minibatch(mbs, factor=1 / 3, sync=[False, True])
+        for name, want in now.items():
+            assert _rel(held[name], want) < 1e-4, name
