@@ -585,10 +585,10 @@ Tensor attention_qkv(Tensor qkv, int64_t n_q, int64_t n_kv, int64_t d, Tensor cu
   return AttentionQKVFn::apply(qkv, n_q, n_kv, d, cu, max_seqlen, causal, scale);
 }
 
-  if (chunk == 0) throw py::value_error("chunk must not be zero");   // the walk over the tokens would not end
 // ---- LM head ---------------------------------------------------------------------------------------------------------
 // bf16 logits of one chunk of tokens, whatever type a library product of the head is in
 Tensor chunk_logits(const Tensor& h, int64_t vocab, int64_t chunk) {
+  if (chunk == 0) throw py::value_error("chunk must not be zero");   // the walk over the tokens would not end
   return at::empty({std::min(chunk, h.size(0)), vocab}, h.options().dtype(at::kBFloat16));
 }
 

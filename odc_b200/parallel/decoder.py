@@ -234,11 +234,11 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
         dh, dw32 = ctx.saved_tensors
         model = ctx.model
         p = model.head_param()
+        # one rounding from an fp32 factor, whether or not this microbatch's weight gradients are pushed now
+        gh = ops._ext().scale_to_bf16(dh, dloss) if dh.is_cuda and dh.dtype == torch.bfloat16 else dh * dloss.to(dh.dtype)
         if _direct(p):
             p.push_direct(dw32, dloss)
             return gh, None, None, None, None, None
-        # one rounding from an fp32 factor, whether or not this microbatch's weight gradients are pushed now
-        gh = ops._ext().scale_to_bf16(dh, dloss) if dh.is_cuda and dh.dtype == torch.bfloat16 else dh * dloss.to(dh.dtype)
         p.wait_push()
         buf = p.local_buffer()
         buf[:p.out_features].addcmul_(dw32[:p.out_features], dloss.to(dw32.dtype))

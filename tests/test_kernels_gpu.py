@@ -404,6 +404,17 @@ def test_lm_head_on_library_products_in_other_types(monkeypatch, dtype):
         torch.testing.assert_close(ops.linear_cross_entropy(h, w, ids).double(), -want.sum(), rtol=5e-3, atol=0)
 
 
+def test_lm_head_refuses_a_chunk_or_temperature_of_zero():
+    from odc_b200 import ops
+    h, w = torch.randn(8, 64, device="cuda").bfloat16(), torch.randn(512, 64, device="cuda").bfloat16()
+    ids = torch.randint(0, 512, (8,), device="cuda")
+    for call in (ops.linear_cross_entropy, ops.linear_token_logprobs):
+        with pytest.raises(ValueError):
+            call(h, w, ids, chunk=0)
+    with pytest.raises(ZeroDivisionError):
+        ops.linear_token_logprobs(h, w, ids, temperature=0.0)
+
+
 def test_linear_cross_entropy_matches_reference():
     from odc_b200 import ops
     from odc_b200.ops import reference as ref
@@ -491,17 +502,6 @@ def test_wgrad_scatter_emulated_ranks(ext, world, T, n_out, k_in):
         torch.testing.assert_close(got, want[r * rows_per:r * rows_per + rows], rtol=2e-2, atol=2e-2 * math.sqrt(T))
         assert float(accs[r][:off].abs().sum()) == 0.0 and float(accs[r][off + rows_per * k_in:].abs().sum()) == 0.0
         assert int(ctrs[r][0]) == 2
-
-
-def test_lm_head_refuses_a_chunk_or_temperature_of_zero():
-    from odc_b200 import ops
-    h, w = torch.randn(8, 64, device="cuda").bfloat16(), torch.randn(512, 64, device="cuda").bfloat16()
-    ids = torch.randint(0, 512, (8,), device="cuda")
-    for call in (ops.linear_cross_entropy, ops.linear_token_logprobs):
-        with pytest.raises(ValueError):
-            call(h, w, ids, chunk=0)
-    with pytest.raises(ZeroDivisionError):
-        ops.linear_token_logprobs(h, w, ids, temperature=0.0)
 
 
 @pytest.mark.parametrize("world", [1, 2, 8])
