@@ -400,7 +400,7 @@ ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ label
                   float* __restrict__ loss, int vocab, long long ignore_index, float* __restrict__ per_token,
                   float inv_temp) {
   allow_next();
-  wait_previous(labels, loss_scale);
+  wait_previous(logits, labels, loss_scale);
   __shared__ float red[32];
   const int row = blockIdx.x;
   bf16* lr = logits + size_t(row) * vocab;

@@ -328,6 +328,69 @@ def test_chained_kernels_see_their_predecessors(ext, T, H, F):
         assert torch.equal(chain(False), want)
 
 
+def _same_bytes_without_pauses(steps, tries=5):
+    """``steps``: functions of the value before; a run that waits after each, then runs that do not."""
+    def run(pause):
+        x = None
+        for step in steps:
+            x = step(x)
+            if pause:
+                torch.cuda.synchronize()
+        return x
+    want = [t.clone() for t in run(True)]
+    assert all(torch.isfinite(t.float()).all() for t in want)
+    for _ in range(tries):
+        for got, exp in zip(run(False), want):
+            assert torch.equal(got, exp)
+
+
+@pytest.mark.parametrize("T,H,V", [(8, 256, 1024), (300, 512, 32000)])
+def test_chained_softmax_kernels_see_their_predecessors(ext, T, H, V):
+    """Product -> log-probabilities, product -> gradient of the logits -> product, in one logits buffer."""
+    torch.manual_seed(T)
+    hs = [torch.randn(T, H, device="cuda").bfloat16() for _ in range(4)]
+    w = (torch.randn(V, H, device="cuda") / 16).bfloat16()
+    ids, scale = torch.randint(0, V, (T,), device="cuda"), torch.rand(T, device="cuda")
+    logits = torch.empty(T, V, device="cuda", dtype=torch.bfloat16)
+    lp = torch.empty(len(hs), T, device="cuda")
+    dh = torch.empty(len(hs), T, H, device="cuda", dtype=torch.bfloat16)
+    loss = torch.zeros((), device="cuda")
+    steps = []
+    for i, h in enumerate(hs):
+        steps += [lambda _, h=h: ext.gemm(h, w, logits, "nt", None, False),
+                  lambda _, i=i: ext.token_logprobs(logits, ids, lp[i], -100),
+                  lambda _, h=h: ext.gemm(h, w, logits, "nt", None, False),
+                  lambda _: ext.ce_fwd_bwd(logits, ids, scale, loss, -100),
+                  lambda _, i=i: ext.gemm(logits, w, dh[i], "nn", None, False)]
+    _same_bytes_without_pauses(steps + [lambda _: (lp, dh)])
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_chained_attention_kernels_see_their_predecessors(ext, d):
+    """Rotation -> attention forward -> backward with reused memory; sequences of one key tile, whose gradients are sums in a
+    fixed order."""
+    lens, hq, hkv = [100, 128, 37], 4, 2
+    T = sum(lens)
+    torch.manual_seed(d)
+    qkvs = [torch.randn(T, (hq + 2 * hkv) * d, device="cuda").bfloat16() for _ in range(4)]
+    do = torch.randn(T, hq, d, device="cuda").bfloat16()
+    pos = torch.cat([torch.arange(n) for n in lens]).cuda()
+    cu = torch.tensor([0] + lens, device="cuda").cumsum(0).int()
+    out = torch.empty(len(qkvs), T, (hq + 2 * hkv) * d, device="cuda", dtype=torch.bfloat16)
+
+    def split(x):
+        return tuple(t.view(T, -1, d) for t in x.split([hq * d, hkv * d, hkv * d], dim=-1))
+
+    steps = []
+    for i, qkv in enumerate(qkvs):
+        steps += [lambda _, qkv=qkv: ext.rope_qkv(qkv, pos, hq, hkv, d, 10000.0, False),
+                  lambda x: (x, *ext.attn_fwd(*split(x), cu, max(lens), True, d ** -0.5)),
+                  lambda x: ext.attn_bwd(do, *split(x[0]), x[1], x[2], cu, max(lens), True, d ** -0.5, True)[3],
+                  lambda g: ext.rope_qkv(g, pos, hq, hkv, d, 10000.0, True),
+                  lambda g, i=i: out[i].copy_(g)]
+    _same_bytes_without_pauses(steps + [lambda _: (out,)])
+
+
 @pytest.mark.parametrize("T,K,F", [(256, 128, 128), (300, 264, 1000), (520, 2048, 136), (1000, 512, 4160), (16, 128, 256),
                                    (765, 17920, 768)])
 def test_linear_swiglu_matches_the_two_passes(ext, T, K, F):
