@@ -218,7 +218,7 @@ void gemm_into(const Tensor& a, const Tensor& b, const Tensor& c, int lay, const
     ldr = residual.stride(0);
   }
   Tensor parts;  // few tiles and a long reduction: scratch for the partial products
-  if (pair < 0 && !accumulate) {
+  if (pair < 0 && !accumulate && odc::gemm_pairs_enabled()) {
     const size_t bytes = odc::gemm_split_bytes(M, N, K, kind_of(c.scalar_type()), sm_count());
     if (bytes > 0) {
       parts = at::empty({static_cast<int64_t>(bytes / sizeof(float))}, a.options().dtype(at::kFloat));
@@ -483,11 +483,7 @@ std::tuple<Tensor, Tensor> linear_swiglu_fwd(const Tensor& x, const Tensor& w, b
   TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16, "linear_swiglu: bf16 inputs");
   TORCH_CHECK(x.stride(1) == 1 && w.stride(1) == 1, "linear_swiglu: innermost stride must be 1");
   const int64_t T = x.size(0), F = w.size(0) / 2;
-  static const bool pairs = [] {
-    const char* e = std::getenv("ODC_GEMM_PAIR");
-    return e == nullptr || e[0] != '0';
-  }();
-  if (pairs && !library_gemm()) {
+  if (odc::gemm_pairs_enabled() && !library_gemm()) {
     Tensor gate_up;
     if (need_gate_up) gate_up = at::empty({T, 2 * F}, x.options());
     auto act = at::empty({T, F}, x.options());

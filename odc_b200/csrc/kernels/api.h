@@ -114,6 +114,7 @@ cudaError_t gemm_bf16(const void* a, const void* b, void* c, int c_kind, const v
                       int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0,
                       int pair_mode = -1 /* -1: ODC_GEMM_PAIR decides, 0: single-CTA kernel, 1: CTA-pair kernel */,
                       float* split_ws = nullptr);
+bool gemm_pairs_enabled();   // ODC_GEMM_PAIR=0 (read once) keeps every product on the single-CTA kernel
 // Bytes of scratch (split_ws) with which the CTA-pair kernel would divide this product's reduction; 0: it would not.
 size_t gemm_split_bytes(int M, int N, int K, int c_kind, int sm_count);
 

@@ -39,16 +39,20 @@ using namespace gemm_impl;
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
+bool gemm_pairs_enabled() {
+  static const bool on = [] {
+    const char* e = getenv("ODC_GEMM_PAIR");
+    return e == nullptr || e[0] != '0';
+  }();
+  return on;
+}
+
 cudaError_t gemm_bf16(const void* a, const void* b, void* c, int c_kind, const void* bias, int M, int N, int K,
                       int layout, bool accumulate, long long lda, long long ldb, long long ldc, int* status,
                       int sm_count, cudaStream_t stream, const void* residual, long long ldr, int pair_mode, float* split_ws) {
   if (M == 0 || N == 0) return cudaSuccess;
   if (K == 0) return cudaErrorInvalidSymbol;
-  static const bool use_pairs = [] {
-    const char* e = getenv("ODC_GEMM_PAIR");
-    return e == nullptr || e[0] != '0';
-  }();
-  if (pair_mode == 1 || (pair_mode < 0 && use_pairs)) {
+  if (pair_mode == 1 || (pair_mode < 0 && gemm_pairs_enabled())) {
     const cudaError_t e = gemm_bf16_pair(a, b, c, c_kind, bias, M, N, K, layout, accumulate, lda, ldb, ldc, status,
                                          sm_count, stream, residual, ldr, split_ws);
     if (e != cudaErrorNotSupported || pair_mode == 1) return e;

@@ -391,6 +391,32 @@ def test_chained_attention_kernels_see_their_predecessors(ext, d):
     _same_bytes_without_pauses(steps + [lambda _: (out,)])
 
 
+_WITHOUT_PAIRS = """
+import torch
+from odc_b200 import ops, _ext
+ext = _ext.load()
+a, b = torch.randn(765, 17920, device="cuda").bfloat16(), torch.randn(1536, 17920, device="cuda").bfloat16()
+assert ext.gemm_split_bytes(765, 1536, 17920) > 0
+out = torch.empty(765, 1536, device="cuda", dtype=torch.bfloat16)
+ops.gemm(a, b, out=out)
+torch.cuda.synchronize()
+torch.cuda.reset_peak_memory_stats()
+before, held = ops.kernel_launches(), torch.cuda.memory_allocated()
+ops.gemm(a, b, out=out)
+assert ops.kernel_launches() - before == 1, ops.kernel_launches() - before
+assert torch.cuda.max_memory_allocated() == held, (torch.cuda.max_memory_allocated(), held)
+"""
+
+
+def test_single_cta_products_allocate_and_count_nothing_for_a_division():
+    """ODC_GEMM_PAIR=0 is read once per process: a process of its own."""
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", _WITHOUT_PAIRS], env={**os.environ, "ODC_GEMM_PAIR": "0"}, capture_output=True,
+                       text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr
+
+
 @pytest.mark.parametrize("T,K,F", [(256, 128, 128), (300, 264, 1000), (520, 2048, 136), (1000, 512, 4160), (16, 128, 256),
                                    (765, 17920, 768)])
 def test_linear_swiglu_matches_the_two_passes(ext, T, K, F):
