@@ -10,6 +10,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 
 namespace odc_bind {
 namespace {
@@ -711,6 +712,35 @@ struct ShardedMatrix : torch::CustomClassHolder {
   Tensor whole() const { return shard.narrow(0, 0, out_features); }
 };
 
+// Start of the last minibatch: an event behind its work, and the stream it ran on.  A pass on that stream is in order as it
+// is; any other waits for the event.  (A stream that is being captured cannot wait for work outside of the capture.)
+struct MinibatchStart {
+  std::mutex mu;
+  cudaEvent_t event = nullptr;
+  std::atomic<cudaStream_t> stream{nullptr};
+  std::atomic<bool> set{false};
+} g_start;
+
+void mark_start() {
+  std::lock_guard<std::mutex> lock(g_start.mu);
+  const cudaStream_t s = cur_stream();
+  if (g_start.event == nullptr) check(cudaEventCreateWithFlags(&g_start.event, cudaEventDisableTiming), "mark_start");
+  check(cudaEventRecord(g_start.event, s), "mark_start");
+  g_start.stream = s;
+  g_start.set = true;
+}
+
+void after_start() {
+  if (!g_start.set) return;
+  const cudaStream_t s = cur_stream();
+  if (s == g_start.stream) return;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  check(cudaStreamIsCapturing(s, &capture), "after_start");
+  if (capture != cudaStreamCaptureStatusNone) return;
+  std::lock_guard<std::mutex> lock(g_start.mu);
+  check(cudaStreamWaitEvent(s, g_start.event, 0), "after_start");
+}
+
 std::atomic<bool> g_sync_grads{true};   // false: weight gradients are accumulated on the producing rank
 py::object* g_deferred = nullptr;       // Python: (id, dy2, x2) of a gradient that is not pushed straight away
 
@@ -782,6 +812,7 @@ struct ShardedLinearFn : Function<ShardedLinearFn> {
 };
 Tensor sharded_linear(Tensor x, c10::optional<Tensor> bias, c10::optional<Tensor> residual, c10::intrusive_ptr<ShardedMatrix> m,
                       c10::optional<Tensor> bias_sink, bool keep_weight) {
+  after_start();
   const bool db = bias.has_value() && wants_grad(*bias), dres = residual.has_value() && wants_grad(*residual);
   return ShardedLinearFn::apply(x, bias, residual, m, bias_sink, keep_weight, wants_grad(x), db, dres);
 }
@@ -826,6 +857,8 @@ void register_ops(py::module_& m) {
         return p;
       }))
       .def_readwrite("local_pending", &ShardedMatrix::local_pending);
+  m.def("mark_start", &mark_start);
+  m.def("after_start", &after_start);
   m.def("set_sync_grads", [](bool on) { g_sync_grads = on; });
   m.def("set_deferred_weight_grad", [](py::object fn) {
     if (g_deferred == nullptr) g_deferred = new py::object();  // never destroyed: backward threads may outlive the module

@@ -387,6 +387,7 @@ class FusedDecoderLM(nn.Module):
         L.start_minibatch()
         self.small.clear()
         self.small.refresh(self.gather)
+        L.mark_start()
 
     def set_requires_gradient_sync(self, flag: bool) -> None:
         L.set_requires_gradient_sync(flag)
@@ -408,6 +409,8 @@ class FusedDecoderLM(nn.Module):
 
     # -- forward ------------------------------------------------------------------------------------------
     def hidden_states(self, input_ids, position_ids, cu_seqlens, max_seqlen):
+        if self.embed.lowp.is_cuda:
+            ops._ext().after_start()
         with torch.no_grad():
             # one pull per microbatch, like a root FSDP unit that stays unsharded from forward to backward
             if self.embed.world > 1:

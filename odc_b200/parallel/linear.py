@@ -331,6 +331,8 @@ class OdcLinear(nn.Module):
             m = self.weight.matrix()
         if m and x.is_cuda and os.environ.get("ODC_WGRAD_SCATTER", "tma") == "tma":
             return ops._ext().sharded_linear(x, bias, residual, m, bias_sink, self.keep_weight)
+        if x.is_cuda:
+            ops._ext().after_start()
         return _OdcLinearFn.apply(x, bias, residual, self, bias_sink)
 
 
@@ -345,6 +347,15 @@ def start_minibatch() -> None:
         if torch.cuda.is_available():
             torch.cuda.current_stream().synchronize()
         control.host_barrier()
+    mark_start()
+
+
+def mark_start() -> None:
+    """What is queued on the current stream so far belongs to the start of the minibatch: with one rank nothing else makes a
+    pass on another stream see cleared accumulators and the optimizer's weights.  Passes call ``after_start`` of the
+    extension (the native layer does so itself)."""
+    if _service().counter.is_cuda:
+        ops._ext().mark_start()
 
 
 def flush_local_grads() -> None:

@@ -172,6 +172,32 @@ def test_token_ids_of_any_integer_form(form):
         assert want.norm() > 0 and _rel(got, want) < 1e-3
 
 
+def test_passes_on_another_stream_than_the_start_of_their_minibatch():
+    """They find cleared accumulators and the weights of an optimizer step that was still running when it returned."""
+    from odc_b200.data import to_device
+    with _Engine(qkv_bias=True) as e:
+        mbs = _batches(e.cfg)
+        clean = e.minibatch(mbs)
+        on_device = [to_device(mb, DEV) for mb in mbs]
+        other = torch.cuda.Stream()
+        groups = e.model.optimizer_groups()
+        for g in groups:
+            g.flat()[4].zero_()
+        torch.cuda.synchronize()
+        torch.cuda._sleep(50_000_000)        # some 25 ms
+        for g in groups:                     # the optimizer's writes
+            g.flat()[4].copy_(g.flat()[0])
+        e.model.start_minibatch()
+        with torch.cuda.stream(other):
+            for mb in on_device:
+                e.model(*_args(mb), labels=mb["labels"], loss_scale=mb["loss_scale"]).backward()
+        torch.cuda.current_stream().wait_stream(other)
+        e.model.finish_minibatch()
+        got = e.grads()
+        for name, want in clean.items():     # the same sums, in another order of additions
+            assert _rel(got[name], want) < 1e-3, name
+
+
 @pytest.mark.parametrize("tied", [True, False])
 def test_activation_gradients_do_not_depend_on_deferral(tied):
     """A loss factor that bf16 cannot hold (1/3, off by 2^-9 when rounded): the layers' gradients of a microbatch are the
