@@ -99,9 +99,12 @@ class SmallGroup:
         on CPU, and for an input that needs no gradient itself, where only the leaf makes autograd call the backward.
         The buffer counts as written from here on: the kernels of a backward write it while it runs, and one that raises
         half way has written some of it."""
-        if not self.native or (torch.is_grad_enabled() and not x.requires_grad):
+        if not self.native:
             return None
-        self.dirty = self.dirty or torch.is_grad_enabled()
+        if torch.is_grad_enabled():
+            if not x.requires_grad:
+                return None
+            self.dirty = True
         return self._views[name]
 
     def norm(self, x, name: str, eps: float):

@@ -99,3 +99,29 @@ def test_attention_tile_edges(lens, hq, hkv, d, causal):
     for name, got, exp in (("o", o, want), ("dq", q.grad, qr.grad), ("dk", k.grad, kr.grad), ("dv", v.grad, vr.grad)):
         rel = ((got.double() - exp).norm() / exp.norm()).item()
         assert rel <= 4 * 2 ** -8, (name, rel)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_attention_of_many_sequences_and_heads_per_tile(d):
+    """More sequences than lanes of the warp that finds a tile, and key tiles for every SM: the backward then walks the heads
+    of a group one after the other and writes dK and dV itself.  Bounds as above."""
+    from odc_b200 import _ext, ops
+    from odc_b200.ops import reference as ref
+    hq, hkv = 8, 2
+    rng = torch.Generator().manual_seed(d)
+    lens = torch.randint(1, 200, (75,), generator=rng).tolist() + [700, 1, 1500, 129] + [128] * 20
+    lens = [lens[i] for i in torch.randperm(len(lens), generator=rng)]
+    T = sum(lens)
+    assert -(-T // 128) * hkv >= torch.cuda.get_device_properties(0).multi_processor_count and len(lens) > 64
+    q, k, v, cu = _case(lens, hq, hkv, d, seed=11)
+    q, k, v = (t.detach().clone().requires_grad_() for t in (q, k, v))
+    o = ops.varlen_attention(q, k, v, cu, max(lens))
+    do = torch.randn_like(o)
+    o.backward(do)
+    assert _ext.load().kernel_status()[0].item() == 0, _ext.load().kernel_status().tolist()
+    qr, kr, vr = (t.detach().double().requires_grad_() for t in (q, k, v))
+    want = ref.varlen_attention(qr, kr, vr, cu.cpu(), True, d ** -0.5)
+    want.backward(do.double())
+    for name, got, exp in (("o", o, want), ("dq", q.grad, qr.grad), ("dk", k.grad, kr.grad), ("dv", v.grad, vr.grad)):
+        rel = ((got.double() - exp).norm() / exp.norm()).item()
+        assert rel <= 4 * 2 ** -8, (name, rel)

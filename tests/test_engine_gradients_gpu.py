@@ -209,3 +209,19 @@ def test_activation_gradients_do_not_depend_on_deferral(tied):
         held = e.minibatch(mbs, factor=1 / 3, sync=[False, True])
         for name, want in now.items():
             assert _rel(held[name], want) < 1e-4, name
+
+
+@pytest.mark.parametrize("sync", [None, [False, True], [True, False]])
+@pytest.mark.parametrize("tied,bias", [(True, True), (False, False)])
+def test_every_accumulator_matches_the_plain_decoder(tied, bias, sync):
+    """Two microbatches with a loss factor, pushed at once, or held back and handed to the Python layer, tied and untied
+    heads: every accumulator after the minibatch is the gradient of the plain decoder."""
+    with _Engine(qkv_bias=bias, tie_embeddings=tied) as e:
+        mbs = _batches(e.cfg)
+        got = e.minibatch(mbs, factor=0.75, sync=sync)
+        for mb in mbs:
+            (0.75 * e.src(*_args(mb), labels=mb["labels"], loss_scale=mb["loss_scale"])).backward()
+        want = dict(e.src.named_parameters())
+        assert set(got) == set(want)
+        for name, p in want.items():
+            assert _rel(got[name], p.grad) < CHAIN, name

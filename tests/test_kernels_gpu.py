@@ -93,6 +93,62 @@ def test_scatter_accumulate_scale(ext):
     assert torch.equal(torch.stack(accs), x * 0.25)
 
 
+def test_scatter_accumulate_scale_on_the_device(ext):
+    """A factor the host has not seen, on top of the one it passes; both input types (exact: powers of two)."""
+    n, world = 4100, 3
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    for dtype in (torch.float32, torch.bfloat16):
+        accs = [torch.ones(n, device="cuda") for _ in range(world)]
+        ctrs = [torch.zeros(8, dtype=torch.int64, device="cuda") for _ in range(world)]
+        x = torch.randint(-8, 8, (world, n), device="cuda").to(dtype)
+        factor = torch.tensor(0.5, device="cuda")
+        ext.scatter_accumulate(x, _table(accs), _table(ctrs), n, torch.float32, 1, 0.25, True, status, n, factor)
+        assert torch.equal(torch.stack(accs), 1 + x.float() * 0.125)
+        assert [int(c[0]) for c in ctrs] == [1] * world
+    assert int(status[0]) == 0
+
+
+@pytest.mark.parametrize("world,tokens,width,vocab", [(1, 1, 8, 4), (1, 700, 264, 50), (3, 700, 64, 100), (8, 3000, 2048, 1001)])
+def test_embedding_scatter_emulated_ranks(ext, world, tokens, width, vocab):
+    """Rows of the lookup's gradient in the owners' accumulators: repeated ids, the first and the last row, ids outside of the
+    vocabulary skipped, padding rows untouched.  Whole numbers: exact in any order."""
+    rows = -(-vocab // world)
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    ids = torch.randint(0, vocab, (tokens,), device="cuda", generator=gen)
+    ids[: tokens // 3] = vocab - 1
+    if tokens > 3:
+        ids[-3:] = torch.tensor([0, -1, vocab], device="cuda")
+    dx = torch.randint(-4, 5, (tokens, width), device="cuda", generator=gen).bfloat16()
+    accs = [torch.ones(rows, width, device="cuda") for _ in range(world)]
+    ctrs = [torch.zeros(8, dtype=torch.int64, device="cuda") for _ in range(world)]
+    for _ in range(2):
+        ext.embedding_scatter(ids, dx, _table(accs), _table(ctrs), rows, vocab, 0.5)
+    want = torch.ones(world * rows, width, device="cuda", dtype=torch.float64)
+    keep = (ids >= 0) & (ids < vocab)
+    want.index_add_(0, ids[keep], dx[keep].double())
+    assert torch.equal(torch.cat(accs).double(), want)
+    assert [int(c[0]) for c in ctrs] == [2] * world
+
+
+def test_post_and_wait_runs_out(ext):
+    """The one launch of a synchronisation: posts and waits; a producer that never posts, and fewer arrivals than announced,
+    run into the short limit and are named, and the context stays usable."""
+    nprod = 3
+    slots, ctr = (torch.zeros(8, dtype=torch.int64, device="cuda") for _ in range(2))
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    host = torch.zeros(4, dtype=torch.int32).pin_memory()
+    addrs = [slots.data_ptr() + 8 * p for p in range(nprod)]
+    ctr[0] = 6
+    assert ext.post_and_wait(addrs, [1, 2, 3], 1, slots, nprod, ctr, 500, status, host) == (0, 0, 0)
+    assert [int(v) >> 32 for v in slots[:nprod]] == [1] * nprod
+    assert ext.post_and_wait(addrs[:2], [1, 2], 2, slots, nprod, ctr, 50, status, host) == (1, 1000 + nprod - 1, 1)
+    status.zero_()
+    assert ext.post_and_wait(addrs, [1, 2, 4], 3, slots, nprod, ctr, 50, status, host) == (1, 0, 6)
+    status.zero_()
+    ctr[0] = 7
+    assert ext.post_and_wait(addrs, [1, 2, 4], 4, slots, nprod, ctr, 500, status, host) == (0, 0, 0)
+
+
 # ------------------------------------------------------------------------------------ elementwise
 @pytest.mark.parametrize("rows,cols", [(1, 256), (333, 2048), (4096, 5120), (17, 8192)])
 def test_rmsnorm(rows, cols):
@@ -452,6 +508,19 @@ def test_linear_autograd_matches_reference():
     torch.testing.assert_close(x.grad.float(), xr.grad, rtol=2e-2, atol=5e-2)
     torch.testing.assert_close(w.grad.float(), wr.grad, rtol=2e-2, atol=0.5)
     torch.testing.assert_close(b.grad.float(), br.grad, rtol=2e-2, atol=0.5)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (127, 72), (129, 264), (1001, 2560), (4096, 64)])
+def test_bias_gradient_sums(ext, rows, cols):
+    """Column sums, ragged in rows and in the 64 columns of a CTA: rounded once to bf16 from fp32 sums."""
+    from odc_b200 import ops
+    x, w = torch.randn(rows, 64, device="cuda").bfloat16(), torch.randn(cols, 64, device="cuda").bfloat16()
+    b = torch.zeros(cols, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    dy = torch.randn(rows, cols, device="cuda").bfloat16()
+    db, = torch.autograd.grad(ops.linear(x, w, b), [b], dy)
+    exact = dy.double().sum(0)
+    # one rounding to bf16, and fp32 sums of `rows` terms of at most about 4
+    assert ((db.double() - exact).abs() <= 2 ** -8 * exact.abs() + rows * 4 * 2 ** -22).all()
 
 
 def test_bias_gradient_that_starts_off_a_16_byte_boundary():
