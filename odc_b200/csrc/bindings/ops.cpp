@@ -840,6 +840,11 @@ void register_ops(py::module_& m) {
   m.def("gemm_split_bytes", [](int M, int N, int K) { return odc::gemm_split_bytes(M, N, K, odc::kBF16, sm_count()); });
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
+  m.def("attn_plan", [](int tokens, int seqs, int longest, int n_q, int n_kv, int d, bool causal, int sms) {
+    return std::make_tuple(d == 128 && odc::attn_fwd_pairs(tokens, seqs, longest, n_q, n_kv, causal, sms),
+                           odc::attn_bwd_parts(tokens, n_q, n_kv, sms));
+  }, py::arg("tokens"), py::arg("seqs"), py::arg("longest"), py::arg("n_q"), py::arg("n_kv"), py::arg("head_dim"),
+        py::arg("causal"), py::arg("sms"));  // (forward in pairs of tiles, parts of the backward)
   m.def("kernel_status", &kernel_status);
   m.def("scale_to_bf16", &scale_to_bf16);
   py::class_<DispatchCounter, c10::intrusive_ptr<DispatchCounter>>(m, "DispatchCounter")

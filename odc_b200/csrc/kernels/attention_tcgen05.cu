@@ -20,6 +20,8 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "api.h"
@@ -112,18 +114,19 @@ __device__ __forceinline__ bool locate_tile(const int* cu, int num_seqs, int idx
 //            been read and runs under the exponentials of block j.
 //   D = 128: two tiles in one CTA that read the same K and V tiles: two heads of a key/value group, or with an odd number
 //            of heads per group two consecutive tiles of one head.  All 512 TMEM columns are taken: P(j) overwrites the
-//            scores it came from, and S(j+1) follows P V(j) in the tensor cores' issue order.
+//            scores it came from, and S(j+1) follows P V(j) in the tensor cores' issue order.  Where pairs would leave SMs
+//            without work (attn_fwd_pairs) a CTA takes one tile, with P in columns of its own as at D = 64.
 // Bound by the exponentials (16 per clock and SM) and the chain around them.  With one tile per CTA and P through shared
 // memory: 32768 tokens, 32/8 heads, D = 128: 10.4 ms (848 TFLOP/s), now 8.6 ms (1019); 16210 tokens in 12 sequences,
 // 32/8 heads, D = 64: 0.707 ms, now 0.600 ms.
-template <int D>
+template <int D, int Tiles>
 struct FwdCfg {
-  static constexpr int kTiles = (D == 64) ? 1 : 2;
-  static constexpr int kStages = (D == 64) ? 3 : 2;
-  static constexpr bool kPrivateP = (D == 64);
+  static constexpr int kTiles = Tiles;
+  static constexpr int kStages = (Tiles == 1) ? 3 : 2;
+  static constexpr bool kPrivateP = (Tiles == 1);
   static constexpr int kTmemCols = (D == 64) ? 256 : 512;
   static constexpr int kOCol = kTiles * 128;
-  static constexpr int kPCol = kPrivateP ? 192 : 0;
+  static constexpr int kPCol = kPrivateP ? 128 + D : 0;
   static constexpr int kCtasPerSm = (D == 64) ? 2 : 1;
   static constexpr int kThreads = 64 + 128 * kTiles;
   static constexpr int kQBytes = kBlockQ * D * 2;
@@ -152,12 +155,12 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   return d;
 }
 
-template <int D>
-__global__ void __launch_bounds__(FwdCfg<D>::kThreads, FwdCfg<D>::kCtasPerSm)
+template <int D, int Tiles>
+__global__ void __launch_bounds__(FwdCfg<D, Tiles>::kThreads, FwdCfg<D, Tiles>::kCtasPerSm)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
   wait_previous();
-  using C = FwdCfg<D>;
+  using C = FwdCfg<D, Tiles>;
   // the tiles of one CTA: heads_per_cta heads, or consecutive query tiles of one head
   const int rows = p.heads_per_cta == C::kTiles ? kBlockQ : kBlockQ * C::kTiles;
   // heads vary fastest: the longest tiles of all heads start first
@@ -931,12 +934,35 @@ narrow_grads_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ d
 
 }  // namespace
 
+// D = 128: whether a CTA takes a pair of query tiles, which share its K and V loads and hide each other's softmax, or one, of
+// which twice as many spread over the SMs.  Estimated time in us: as long as the longest tile or as an even share of all key
+// blocks, 1.3 us a key block for one tile and 1.7 for a pair, plus 1.5 us per wave of CTAs.  The host knows the number of
+// sequences and the longest; unless they are all about as long, each counts as half a tile more than it fills, and with
+// the key blocks of the longest.  (max_seqlen is the caller's word; a wrong one costs time only.)  Several waves of pairs
+// of one head that mostly lack their second tile are not worth it either.  Fitted to the times of 500 shapes, 100 to
+// 32000 tokens in 1 to 300 sequences, 1 to 40 heads: never slower than pairs throughout.  1000 tokens in one sequence,
+// 12/2 heads: pairs 24.6 us, single 15.3; 8000 tokens, 1 head: 138 and 82; 8000 tokens, 12/2 heads: 220 and 232; 12
+// sequences of 300 tokens, 14/2 heads: 36.5 and 31.1.
+bool attn_fwd_pairs(int total_tokens, int num_seqs, int max_seqlen, int n_q, int n_kv, bool causal, int sm_count) {
+  const double longest = std::min(std::max(max_seqlen, 1), total_tokens);
+  const double key_blocks = std::ceil(longest / kBlockKV);
+  const double per_tile = causal ? (key_blocks + 1) / 2 : key_blocks;
+  auto ctas = [&](double rows) {  // per head
+    return num_seqs * longest <= 1.1 * total_tokens ? num_seqs * std::ceil(longest / rows) : total_tokens / rows + num_seqs / 2.0;
+  };
+  const double tiles = n_q * ctas(kBlockQ);
+  const double pairs = (n_q / n_kv) % 2 == 0 ? tiles / 2 : n_q * ctas(2 * kBlockQ);
+  auto cost = [&](double n, double block_us) {
+    return block_us * std::max(key_blocks, n * per_tile / sm_count) + 1.5 * std::ceil(n / sm_count);
+  };
+  if (2 * pairs > 1.3 * tiles && pairs > sm_count) return false;
+  return cost(pairs, 1.7) <= cost(tiles, 1.3);
+}
+
 cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* cu_seqlens,
                      int num_seqs, int total_tokens, int max_seqlen, int n_q, int n_kv, int head_dim,
                      long long q_stride, long long kv_stride, long long o_stride, float scale, bool causal,
                      int* status, int sm_count, cudaStream_t stream) {
-  (void)max_seqlen;
-  (void)sm_count;
   if (total_tokens == 0 || num_seqs == 0) return cudaSuccess;
   if (head_dim != 64 && head_dim != 128) return cudaErrorInvalidValue;
   if (n_q % n_kv != 0) return cudaErrorInvalidValue;
@@ -953,25 +979,30 @@ cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float
   p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.n_q = n_q; p.n_kv = n_kv;
   p.o = static_cast<__nv_bfloat16*>(o); p.o_stride = o_stride; p.lse = lse; p.total_tokens = total_tokens;
   p.scale_log2 = scale * kLog2e; p.causal = causal ? 1 : 0; p.status = status;
-  // D = 128 takes two heads of a key/value group per CTA: both tiles then see the same keys, and a short sequence fills
-  // both.  An odd group is walked two query tiles at a time instead.
-  const int tiles = head_dim == 64 ? FwdCfg<64>::kTiles : FwdCfg<128>::kTiles;
+  const bool pairs = head_dim == 128 && attn_fwd_pairs(total_tokens, num_seqs, max_seqlen, n_q, n_kv, causal, sm_count);
+  // a pair takes two heads of a key/value group: both tiles then see the same keys, and a short sequence fills both.  An
+  // odd group is walked two query tiles at a time instead.
+  const int tiles = pairs ? 2 : 1;
   p.heads_per_cta = (n_q / n_kv) % tiles == 0 ? tiles : 1;
   const int rows = kBlockQ * tiles / p.heads_per_cta;
   const unsigned int grid = ((total_tokens + rows - 1) / rows + num_seqs) * (n_q / p.heads_per_cta);
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(attn_fwd_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<64>::kSmem);
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(attn_fwd_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      FwdCfg<128>::kSmem);
+    auto allow = [](auto kernel, int smem) {
+      if (attr_err == cudaSuccess) attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    };
+    allow(attn_fwd_kernel<64, 1>, FwdCfg<64, 1>::kSmem);
+    allow(attn_fwd_kernel<128, 1>, FwdCfg<128, 1>::kSmem);
+    allow(attn_fwd_kernel<128, 2>, FwdCfg<128, 2>::kSmem);
   });
   if (attr_err != cudaSuccess) return attr_err;
   if (head_dim == 64)
-    launch_after(attn_fwd_kernel<64>, grid, FwdCfg<64>::kThreads, FwdCfg<64>::kSmem, stream, tq, tk, tv, p);
+    launch_after(attn_fwd_kernel<64, 1>, grid, FwdCfg<64, 1>::kThreads, FwdCfg<64, 1>::kSmem, stream, tq, tk, tv, p);
+  else if (!pairs)
+    launch_after(attn_fwd_kernel<128, 1>, grid, FwdCfg<128, 1>::kThreads, FwdCfg<128, 1>::kSmem, stream, tq, tk, tv, p);
   else
-    launch_after(attn_fwd_kernel<128>, grid, FwdCfg<128>::kThreads, FwdCfg<128>::kSmem, stream, tq, tk, tv, p);
+    launch_after(attn_fwd_kernel<128, 2>, grid, FwdCfg<128, 2>::kThreads, FwdCfg<128, 2>::kSmem, stream, tq, tk, tv, p);
   return cudaGetLastError();
 }
 

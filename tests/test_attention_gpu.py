@@ -101,6 +101,33 @@ def test_attention_tile_edges(lens, hq, hkv, d, causal):
         assert rel <= 4 * 2 ** -8, (name, rel)
 
 
+def _plan(lens, hq, hkv, d, causal=True):
+    from odc_b200 import _ext
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return _ext.load().attn_plan(sum(lens), len(lens), max(lens), hq, hkv, d, causal, sms)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("lens,hq,hkv,pairs", [([765, 130], 12, 2, False), ([129, 1, 384], 10, 2, False), ([900], 1, 1, False),
+                                               ([513, 7, 1000, 128], 32, 8, True), ([129, 1, 384, 900], 40, 8, True)])
+def test_attention_forward_in_single_tiles_and_pairs(lens, hq, hkv, pairs, causal):
+    """D = 128: both forms of the forward, even and odd groups, ends of tiles.  Bound: P and the output are bf16 inside fp32
+    sums, as above."""
+    from odc_b200 import _ext
+    from odc_b200.ops import reference as ref
+    assert _plan(lens, hq, hkv, 128, causal)[0] == pairs
+    q, k, v, cu = _case(lens, hq, hkv, 128, seed=5)
+    o, lse = _ext.load().attn_fwd(q, k, v, cu, max(lens), causal, 128 ** -0.5)
+    assert _ext.load().kernel_status()[0].item() == 0, _ext.load().kernel_status().tolist()
+    want = ref.varlen_attention(q.double(), k.double(), v.double(), cu.cpu(), causal, 128 ** -0.5)
+    assert ((o.double() - want).norm() / want.norm()).item() <= 4 * 2 ** -8
+    n = lens[0]
+    s = (q[:n, -1].double() @ k[:n, -1].double().t()) * 128 ** -0.5
+    if causal:
+        s = s.masked_fill(~torch.ones(n, n, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    torch.testing.assert_close(lse[-1, :n].double(), torch.logsumexp(s, -1), rtol=1e-4, atol=1e-4)
+
+
 @pytest.mark.parametrize("d", [64, 128])
 def test_attention_of_many_sequences_and_heads_per_tile(d):
     """More sequences than lanes of the warp that finds a tile, and key tiles for every SM: the backward then walks the heads
@@ -111,8 +138,7 @@ def test_attention_of_many_sequences_and_heads_per_tile(d):
     rng = torch.Generator().manual_seed(d)
     lens = torch.randint(1, 200, (75,), generator=rng).tolist() + [700, 1, 1500, 129] + [128] * 20
     lens = [lens[i] for i in torch.randperm(len(lens), generator=rng)]
-    T = sum(lens)
-    assert -(-T // 128) * hkv >= torch.cuda.get_device_properties(0).multi_processor_count and len(lens) > 64
+    assert _plan(lens, hq, hkv, d)[1] == 1 and len(lens) > 64
     q, k, v, cu = _case(lens, hq, hkv, d, seed=11)
     q, k, v = (t.detach().clone().requires_grad_() for t in (q, k, v))
     o = ops.varlen_attention(q, k, v, cu, max(lens))
