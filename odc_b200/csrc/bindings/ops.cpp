@@ -311,13 +311,13 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(Tensor dout, Tensor q, Tenso
   }
   auto delta = at::empty({hq, T}, q.options().dtype(at::kFloat));
   auto dq_acc = at::empty({T, hq, d}, q.options().dtype(at::kFloat));
-  const int n_parts = hkv > 0 && hq % hkv == 0 ? odc::attn_bwd_parts(T, hq, hkv, sm_count()) : 1;
+  const int n_seqs = static_cast<int>(cu_seqlens.numel() - 1);
+  const int n_parts = hkv > 0 && hq % hkv == 0 ? odc::attn_bwd_parts(T, n_seqs, max_seqlen, hq, hkv, d, causal, sm_count()) : 1;
   Tensor kv_parts;
   if (n_parts > 1) kv_parts = at::empty({n_parts, 2, T, hkv, d}, q.options().dtype(at::kFloat));
   check(odc::attn_bwd(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
                       dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), dq_acc.data_ptr<float>(),
-                      n_parts > 1 ? kv_parts.data_ptr<float>() : nullptr,
-                      cu_seqlens.data_ptr<int>(), static_cast<int>(cu_seqlens.numel() - 1), T, max_seqlen, hq, hkv, d,
+                      n_parts > 1 ? kv_parts.data_ptr<float>() : nullptr, n_parts, cu_seqlens.data_ptr<int>(), n_seqs, T, max_seqlen, hq, hkv, d,
                       q.stride(0), k.stride(0), o.stride(0), dq.stride(0), dk.stride(0), static_cast<float>(scale),
                       causal, device_status(q.get_device()).data_ptr<int>(), sm_count(), cur_stream()),
         "attn_bwd");
@@ -842,7 +842,7 @@ void register_ops(py::module_& m) {
   m.def("attn_bwd", &attn_bwd);
   m.def("attn_plan", [](int tokens, int seqs, int longest, int n_q, int n_kv, int d, bool causal, int sms) {
     return std::make_tuple(d == 128 && odc::attn_fwd_pairs(tokens, seqs, longest, n_q, n_kv, causal, sms),
-                           odc::attn_bwd_parts(tokens, n_q, n_kv, sms));
+                           odc::attn_bwd_parts(tokens, seqs, longest, n_q, n_kv, d, causal, sms));
   }, py::arg("tokens"), py::arg("seqs"), py::arg("longest"), py::arg("n_q"), py::arg("n_kv"), py::arg("head_dim"),
         py::arg("causal"), py::arg("sms"));  // (forward in pairs of tiles, parts of the backward)
   m.def("kernel_status", &kernel_status);

@@ -175,9 +175,9 @@ cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float
 // head_dim 128: the forward takes query tiles in pairs, else (and with head_dim 64) one per CTA
 bool attn_fwd_pairs(int total_tokens, int num_seqs, int max_seqlen, int n_q, int n_kv, bool causal, int sm_count);
 // CTAs per (key tile, kv head) of the backward; above 1 it needs kv_parts, [parts][2][tokens, n_kv, head_dim] fp32 scratch
-int attn_bwd_parts(int total_tokens, int n_q, int n_kv, int sm_count);
+int attn_bwd_parts(int total_tokens, int num_seqs, int max_seqlen, int n_q, int n_kv, int head_dim, bool causal, int sm_count);
 cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const float* lse,
-                     void* dq, void* dk, void* dv, float* delta, float* dq_acc, float* kv_parts, const int* cu_seqlens, int num_seqs,
+                     void* dq, void* dk, void* dv, float* delta, float* dq_acc, float* kv_parts, int parts, const int* cu_seqlens, int num_seqs,
                      int total_tokens, int max_seqlen, int n_q, int n_kv, int head_dim, long long q_stride,
                      long long kv_stride, long long o_stride, long long dq_stride, long long dkv_stride, float scale,
                      bool causal, int* status, int sm_count, cudaStream_t stream);
