@@ -2,7 +2,7 @@
 //
 // A training step of a small model is bound by the host: a Python autograd function costs 15-25 us per direction, the
 // kernels behind it 3-10 us.  The native functions cost 3-5 us per direction and run their backward without the
-// interpreter lock (packed 2-layer, 512-wide decoder, two microbatches: see the figures at the Python wrappers).
+// interpreter lock (two layers, 512 wide, two microbatches: a training step 4579 -> 4004 us).
 #include "ops.h"
 
 #include <torch/csrc/autograd/custom_function.h>
@@ -157,7 +157,7 @@ void adamw_step(Tensor p, Tensor g, Tensor m, Tensor v, c10::optional<Tensor> p_
   check(odc::launch_adamw(p.data_ptr<float>(), g.data_ptr(), kind_of(g.scalar_type()), m.data_ptr<float>(),
                           v.data_ptr<float>(), lp, static_cast<size_t>(p.numel()), static_cast<float>(lr),
                           static_cast<float>(beta1), static_cast<float>(beta2), static_cast<float>(eps),
-                          static_cast<float>(wd), bc1, bc2, static_cast<float>(grad_scale), sm_count(), cur_stream()),
+                          static_cast<float>(wd), bc1, bc2, static_cast<float>(grad_scale), cur_stream()),
         "adamw");
 }
 

@@ -96,7 +96,7 @@ cudaError_t launch_token_logprobs(const void* logits, const long long* labels, f
                                   long long ignore_index, cudaStream_t stream, float inv_temp = 1.f);
 cudaError_t launch_adamw(float* p, const void* g, int g_kind, float* m, float* v, void* p_lowp, size_t n, float lr,
                          float beta1, float beta2, float eps, float wd, float bc1, float bc2, float grad_scale,
-                         int sm_count, cudaStream_t stream);
+                         cudaStream_t stream);
 // column sums of a bf16 [rows, cols] matrix, fp32 inside: rounded into out (bf16) or added to sink (fp32); cols % 8 == 0
 cudaError_t launch_column_sum(const void* x, void* out, float* sink, long long rows, int cols, cudaStream_t stream);
 // out (bf16) = in (fp32 or bf16) * *scale
