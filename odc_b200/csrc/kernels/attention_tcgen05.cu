@@ -91,7 +91,7 @@ __device__ __forceinline__ bool locate_tile(const int* cu, int num_seqs, int idx
     if (at_least(mid) > idx) lo = mid; else hi = mid - 1;
   }
   int rank = idx - at_least(lo + 1);
-  for (int first = 0;; first += 32) {  // the rank-th sequence with at least lo tiles
+  for (int first = 0; first < num_seqs; first += 32) {  // the rank-th sequence with at least lo tiles
     const bool has = (first == 0 ? own : tiles(first + lane)) >= lo;
     const unsigned int m = __ballot_sync(0xffffffffu, has);
     if (rank < __popc(m)) {
@@ -104,6 +104,7 @@ __device__ __forceinline__ bool locate_tile(const int* cu, int num_seqs, int idx
     }
     rank -= __popc(m);
   }
+  return false;  // not reached while cu_seqlens stays as it is
 }
 
 // Two 128-row query tiles per SM keep the exponential units and the tensor cores busy at the same time: while the softmax
