@@ -160,7 +160,6 @@ template <int D, int Tiles>
 __global__ void __launch_bounds__(FwdCfg<D, Tiles>::kThreads, FwdCfg<D, Tiles>::kCtasPerSm)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
-  wait_previous();
   using C = FwdCfg<D, Tiles>;
   // the tiles of one CTA: heads_per_cta heads, or consecutive query tiles of one head
   const int rows = p.heads_per_cta == C::kTiles ? kBlockQ : kBlockQ * C::kTiles;
@@ -228,7 +227,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  allow_next();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -493,7 +491,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
                 const __grid_constant__ CUtensorMap tmap_dq, const BwdParams p) {
-  wait_previous();
   using C = BwdCfg<D>;
   int seq_start, seq_len, work;
   if (!locate_tile(p.cu_seqlens, p.num_seqs, blockIdx.x / (p.n_kv * p.parts), 128, &seq_start, &seq_len, &work)) return;
@@ -562,7 +559,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  allow_next();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -868,8 +864,6 @@ template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o, float* __restrict__ delta,
                   int total_tokens, int n_q, long long do_stride, long long o_stride) {
-  allow_next();
-  wait_previous(dout, o);
   constexpr int kLanes = D / 8;               // threads per (token, head)
   constexpr int kTokens = 256 / kLanes;       // tokens per CTA
   const int part = threadIdx.x % kLanes;
@@ -906,8 +900,6 @@ __global__ void __launch_bounds__(256)
 narrow_grads_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, long long n8, int width8, long long dq_stride,
                     float scale, const float* __restrict__ kv_parts, int parts, __nv_bfloat16* __restrict__ dk,
                     __nv_bfloat16* __restrict__ dv, long long kv_n8, int kv_width8, long long dkv_stride) {
-  allow_next();
-  wait_previous(acc, kv_parts);
   const long long total = n8 + (parts > 1 ? 2 * kv_n8 : 0);
   for (long long v = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; v < total;
        v += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -999,11 +991,11 @@ cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float
   });
   if (attr_err != cudaSuccess) return attr_err;
   if (head_dim == 64)
-    launch_after(attn_fwd_kernel<64, 1>, grid, FwdCfg<64, 1>::kThreads, FwdCfg<64, 1>::kSmem, stream, tq, tk, tv, p);
+    launch(attn_fwd_kernel<64, 1>, grid, FwdCfg<64, 1>::kThreads, FwdCfg<64, 1>::kSmem, stream, tq, tk, tv, p);
   else if (!pairs)
-    launch_after(attn_fwd_kernel<128, 1>, grid, FwdCfg<128, 1>::kThreads, FwdCfg<128, 1>::kSmem, stream, tq, tk, tv, p);
+    launch(attn_fwd_kernel<128, 1>, grid, FwdCfg<128, 1>::kThreads, FwdCfg<128, 1>::kSmem, stream, tq, tk, tv, p);
   else
-    launch_after(attn_fwd_kernel<128, 2>, grid, FwdCfg<128, 2>::kThreads, FwdCfg<128, 2>::kSmem, stream, tq, tk, tv, p);
+    launch(attn_fwd_kernel<128, 2>, grid, FwdCfg<128, 2>::kThreads, FwdCfg<128, 2>::kSmem, stream, tq, tk, tv, p);
   return cudaGetLastError();
 }
 
@@ -1052,11 +1044,11 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
   const long long do_stride = static_cast<long long>(n_q) * head_dim;
   const unsigned int delta_y = (n_q + kDeltaHeads - 1) / kDeltaHeads;
   if (head_dim == 64) {
-    launch_after(attn_delta_kernel<64>, dim3((total_tokens + 31) / 32, delta_y), 256, 0, stream,
+    launch(attn_delta_kernel<64>, dim3((total_tokens + 31) / 32, delta_y), 256, 0, stream,
         static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, total_tokens, n_q,
         do_stride, o_stride);
   } else {
-    launch_after(attn_delta_kernel<128>, dim3((total_tokens + 15) / 16, delta_y), 256, 0, stream,
+    launch(attn_delta_kernel<128>, dim3((total_tokens + 15) / 16, delta_y), 256, 0, stream,
         static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, total_tokens, n_q,
         do_stride, o_stride);
   }
@@ -1089,14 +1081,14 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
   if (attr_err != cudaSuccess) return attr_err;
   const unsigned int grid = ((total_tokens + 127) / 128 + num_seqs) * n_kv * p.parts;
   if (head_dim == 64)
-    launch_after(attn_bwd_kernel<64>, grid, kBwdThreads, BwdCfg<64>::kSmem, stream, tq, tk, tv, tdo, tdq, p);
+    launch(attn_bwd_kernel<64>, grid, kBwdThreads, BwdCfg<64>::kSmem, stream, tq, tk, tv, tdo, tdq, p);
   else
-    launch_after(attn_bwd_kernel<128>, grid, kBwdThreads, BwdCfg<128>::kSmem, stream, tq, tk, tv, tdo, tdq, p);
+    launch(attn_bwd_kernel<128>, grid, kBwdThreads, BwdCfg<128>::kSmem, stream, tq, tk, tv, tdo, tdq, p);
   const long long n8 = static_cast<long long>(total_tokens) * n_q * head_dim / 8;
   const long long kv_n8 = static_cast<long long>(total_tokens) * n_kv * head_dim / 8;
   long long g = (n8 + (p.parts > 1 ? 2 * kv_n8 : 0) + 255) / 256;
   if (g > sm_count * 16) g = sm_count * 16;
-  launch_after(narrow_grads_kernel, static_cast<int>(g), 256, 0, stream,
+  launch(narrow_grads_kernel, static_cast<int>(g), 256, 0, stream,
       dq_acc, static_cast<__nv_bfloat16*>(dq), n8, n_q * head_dim / 8, dq_stride, scale, kv_parts, p.parts,
       static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), kv_n8, n_kv * head_dim / 8, dkv_stride);
   return cudaGetLastError();

@@ -86,8 +86,6 @@ template <int R>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y,
                    float* __restrict__ rstd_out, int rows, int cols, float eps) {
-  allow_next();
-  wait_previous(x, w);
   __shared__ float red[2][kNormWarps];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = warp % R;                       // which part of the row this warp covers
@@ -149,8 +147,6 @@ __global__ void __launch_bounds__(kNormThreads, 2)
 rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ w,
                    const float* __restrict__ rstd_in, bf16* __restrict__ dx, float* __restrict__ partial,
                    float* __restrict__ dw_out, int rows, int cols, const bf16* __restrict__ dres) {
-  allow_next();
-  wait_previous(dy, x, w, rstd_in, dres);
   extern __shared__ float dw_smem[];  // [cols]
   __shared__ float red[2][kNormWarps];  // alternating, so that a row's sums outlive the next row's first writer
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -254,8 +250,6 @@ __global__ void colsum_kernel(const float* __restrict__ partial, float* __restri
 constexpr int kColSumThreads = 1024;
 __global__ void __launch_bounds__(kColSumThreads)
 column_sum_kernel(const bf16* __restrict__ x, bf16* __restrict__ out, float* __restrict__ sink, long long rows, int cols) {
-  allow_next();
-  wait_previous(x);
   __shared__ float part[kColSumThreads / 32][64];
   const int vec = threadIdx.x & 7, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 64 + vec * 8;
@@ -295,8 +289,6 @@ column_sum_kernel(const bf16* __restrict__ x, bf16* __restrict__ out, float* __r
 __global__ void __launch_bounds__(128)
 rope_qkv_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, const long long* __restrict__ pos, int n_q,
                 int n_kv, int head_dim, float log2_theta, float sign) {
-  allow_next();
-  wait_previous(in, pos);
   extern __shared__ float cs[];  // [head_dim/2] cos, [head_dim/2] sin
   const int t = blockIdx.x;
   const int half = head_dim / 2;
@@ -340,8 +332,6 @@ rope_qkv_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, const long 
 // ------------------------------------------------------------------------- SwiGLU -----------
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long long rows, int f) {
-  allow_next();
-  wait_previous(gu);
   const int vec_per_row = f / 8;
   const long long total = rows * vec_per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -361,8 +351,6 @@ swiglu_fwd_kernel(const bf16* __restrict__ gu, bf16* __restrict__ out, long long
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ gu, bf16* __restrict__ dgu, long long rows,
                   int f) {
-  allow_next();
-  wait_previous(dy, gu);
   const int vec_per_row = f / 8;
   const long long total = rows * vec_per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -399,8 +387,6 @@ __global__ void __launch_bounds__(kCeThreads)
 ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ loss_scale,
                   float* __restrict__ loss, int vocab, long long ignore_index, float* __restrict__ per_token,
                   float inv_temp) {
-  allow_next();
-  wait_previous(logits, labels, loss_scale);
   __shared__ float red[32];
   const int row = blockIdx.x;
   bf16* lr = logits + size_t(row) * vocab;
@@ -594,7 +580,7 @@ cudaError_t rmsnorm_fwd_t(const void* x, const void* w, void* y, float* rstd, in
                           cudaStream_t stream) {
   const int want = (rows + kNormWarps / R - 1) / (kNormWarps / R);
   const int grid = want < sm_count * 8 ? want : sm_count * 8;
-  launch_after(rmsnorm_fwd_kernel<R>, grid, kNormThreads, 0, stream,
+  launch(rmsnorm_fwd_kernel<R>, grid, kNormThreads, 0, stream,
       static_cast<const bf16*>(x), static_cast<const bf16*>(w), static_cast<bf16*>(y), rstd, rows, cols, eps);
   return cudaGetLastError();
 }
@@ -603,11 +589,11 @@ template <int R, int V>
 cudaError_t rmsnorm_bwd_t(const void* dy, const void* x, const void* w, const float* rstd, void* dx, float* partial,
                           float* dw, int rows, int cols, int grid, cudaStream_t stream, const void* dres) {
   if (partial == nullptr) {
-    launch_after(rmsnorm_bwd_kernel<R, V, true>, grid, kNormThreads, cols * sizeof(float), stream,
+    launch(rmsnorm_bwd_kernel<R, V, true>, grid, kNormThreads, cols * sizeof(float), stream,
         static_cast<const bf16*>(dy), static_cast<const bf16*>(x), static_cast<const bf16*>(w), rstd,
         static_cast<bf16*>(dx), nullptr, dw, rows, cols, static_cast<const bf16*>(dres));
   } else {
-    launch_after(rmsnorm_bwd_kernel<R, V, false>, grid, kNormThreads, cols * sizeof(float), stream,
+    launch(rmsnorm_bwd_kernel<R, V, false>, grid, kNormThreads, cols * sizeof(float), stream,
         static_cast<const bf16*>(dy), static_cast<const bf16*>(x), static_cast<const bf16*>(w), rstd,
         static_cast<bf16*>(dx), partial, dw, rows, cols, static_cast<const bf16*>(dres));
   }
@@ -660,7 +646,7 @@ cudaError_t launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
 cudaError_t launch_column_sum(const void* x, void* out, float* sink, long long rows, int cols, cudaStream_t stream) {
   if (cols % 8 != 0 || (out == nullptr) == (sink == nullptr)) return cudaErrorInvalidValue;
   if (cols == 0) return cudaSuccess;
-  launch_after(column_sum_kernel, (cols + 63) / 64, kColSumThreads, 0, stream,
+  launch(column_sum_kernel, (cols + 63) / 64, kColSumThreads, 0, stream,
       static_cast<const bf16*>(x), static_cast<bf16*>(out), sink, rows, cols);
   return cudaGetLastError();
 }
@@ -669,7 +655,7 @@ cudaError_t launch_rope_qkv(const void* in, void* out, const long long* pos, int
                             int head_dim, float theta, bool inverse, cudaStream_t stream) {
   if (head_dim % 16 != 0) return cudaErrorInvalidValue;
   if (tokens == 0) return cudaSuccess;
-  launch_after(rope_qkv_kernel, tokens, 128, head_dim * sizeof(float), stream,
+  launch(rope_qkv_kernel, tokens, 128, head_dim * sizeof(float), stream,
       static_cast<const bf16*>(in), static_cast<bf16*>(out), pos, n_q, n_kv, head_dim, log2f(theta),
       inverse ? -1.f : 1.f);
   return cudaGetLastError();
@@ -679,7 +665,7 @@ cudaError_t launch_swiglu_fwd(const void* gate_up, void* out, long long rows, in
                               cudaStream_t stream) {
   if (f % 8 != 0) return cudaErrorInvalidValue;
   if (rows == 0) return cudaSuccess;
-  launch_after(swiglu_fwd_kernel, cap_grid(rows * (f / 8), 256, sm_count, 16), 256, 0, stream,
+  launch(swiglu_fwd_kernel, cap_grid(rows * (f / 8), 256, sm_count, 16), 256, 0, stream,
       static_cast<const bf16*>(gate_up), static_cast<bf16*>(out), rows, f);
   return cudaGetLastError();
 }
@@ -688,7 +674,7 @@ cudaError_t launch_swiglu_bwd(const void* dy, const void* gate_up, void* dgate_u
                               int sm_count, cudaStream_t stream) {
   if (f % 8 != 0) return cudaErrorInvalidValue;
   if (rows == 0) return cudaSuccess;
-  launch_after(swiglu_bwd_kernel, cap_grid(rows * (f / 8), 256, sm_count, 16), 256, 0, stream,
+  launch(swiglu_bwd_kernel, cap_grid(rows * (f / 8), 256, sm_count, 16), 256, 0, stream,
       static_cast<const bf16*>(dy), static_cast<const bf16*>(gate_up), static_cast<bf16*>(dgate_up), rows, f);
   return cudaGetLastError();
 }
@@ -697,7 +683,7 @@ cudaError_t launch_ce_fwd_bwd(void* logits, const long long* labels, const float
                               int rows, int vocab, long long ignore_index, cudaStream_t stream, float inv_temp) {
   if (rows == 0) return cudaSuccess;
   if (vocab % 8 != 0) return cudaErrorInvalidValue;  // rows must stay 16-byte aligned
-  launch_after(ce_fwd_bwd_kernel<false>, rows, kCeThreads, 0, stream,
+  launch(ce_fwd_bwd_kernel<false>, rows, kCeThreads, 0, stream,
       static_cast<bf16*>(logits), labels, loss_scale, loss, vocab, ignore_index, nullptr, inv_temp);
   return cudaGetLastError();
 }
@@ -707,7 +693,7 @@ cudaError_t launch_token_logprobs(const void* logits, const long long* labels, f
   if (rows == 0) return cudaSuccess;
   if (vocab % 8 != 0 || per_token == nullptr) return cudaErrorInvalidValue;
   // the forward-only instantiation never writes through the logits pointer
-  launch_after(ce_fwd_bwd_kernel<true>, rows, kCeThreads, 0, stream,
+  launch(ce_fwd_bwd_kernel<true>, rows, kCeThreads, 0, stream,
       static_cast<bf16*>(const_cast<void*>(logits)), labels, nullptr, nullptr, vocab, ignore_index, per_token, inv_temp);
   return cudaGetLastError();
 }

@@ -162,10 +162,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   cluster_sync_all();   // the partner's barriers exist before anything is reported to them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if constexpr (kMode != kModeGather) {  // that form polls flags of its own launch, cleared by a memset: plain order
-    allow_next();
-    wait_previous();
-  }
 
   const int splits = kMode == kModePlain ? p.splits : 1;
   const int num_tiles = p.tiles_m * p.tiles_n * splits;   // work items: (tile, split), the splits of a tile adjacent
@@ -542,8 +538,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 __global__ void __launch_bounds__(256)
 split_sum_kernel(const float* __restrict__ part, long long part_stride, int splits, __nv_bfloat16* __restrict__ c, long long ldc,
                  const __nv_bfloat16* __restrict__ bias, const __nv_bfloat16* __restrict__ residual, long long ldr, int M, int N) {
-  allow_next();
-  wait_previous(part, bias, residual);
   const int n8 = N / 8;
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= static_cast<long long>(M) * n8) return;
@@ -682,13 +676,13 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
   }
   const int tiles = p.tiles_m * p.tiles_n * p.splits;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
-  launch_after(gemm_bf16_pair_kernel<kModePlain>, 2 * pairs, kThreads, kSmemBytes, stream,
+  launch(gemm_bf16_pair_kernel<kModePlain>, 2 * pairs, kThreads, kSmemBytes, stream,
       ta, tb, tc, OwnerMaps{}, p);
   if (split) {
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const long long items = static_cast<long long>(M) * (N / 8);
-    launch_after(split_sum_kernel, static_cast<unsigned int>((items + 255) / 256), 256, 0, stream,
+    launch(split_sum_kernel, static_cast<unsigned int>((items + 255) / 256), 256, 0, stream,
         split_ws, static_cast<long long>(p.split_rows) * N, p.splits, static_cast<__nv_bfloat16*>(c), ldc,
         static_cast<const __nv_bfloat16*>(bias), static_cast<const __nv_bfloat16*>(residual), ldr, M, N);
   }
@@ -734,7 +728,7 @@ cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* 
   p.status = status;
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
-  launch_after(gemm_bf16_pair_kernel<kModeSwiglu>, 2 * pairs, kThreads, kSmemBytes, stream, ta, tb, tc, halves, p);
+  launch(gemm_bf16_pair_kernel<kModeSwiglu>, 2 * pairs, kThreads, kSmemBytes, stream, ta, tb, tc, halves, p);
   return cudaGetLastError();
 }
 
@@ -782,7 +776,7 @@ cudaError_t gemm_wgrad_scatter_pair(const void* dy, const void* x, int tokens, i
     p.rot_m = static_cast<int>((static_cast<long long>(start_rank) * rows_per_rank / 256) % p.tiles_m);
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
-  launch_after(gemm_bf16_pair_kernel<kModeScatter>, 2 * pairs, kThreads, kSmemBytes, stream, ta, tb, ta, owners, p);
+  launch(gemm_bf16_pair_kernel<kModeScatter>, 2 * pairs, kThreads, kSmemBytes, stream, ta, tb, ta, owners, p);
   return cudaGetLastError();
 }
 
