@@ -423,6 +423,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         l *= alpha;
         m_used = m_new;
+        // P of the first 64 keys alone starts a product into all columns of O, so the half 0 warp may say that it is there
+        // only when the half 1 warp has scaled its columns too.  Both hold the same rows and maxima: both come here.
+        tmem_st_wait();
+        tc_fence_before();
+        named_barrier_sync(pair_bar, 64);
+        tc_fence_after();
       }
       const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
       const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), sub2 = make_float2(-m_sub, -m_sub);
