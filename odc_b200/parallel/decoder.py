@@ -36,7 +36,7 @@ from ..primitives import GatherService
 from ..runtime import control
 from ..runtime.registry import SymmBufferRegistry
 from . import linear as L
-from .linear import OdcLinear, ShardedParameter
+from .linear import OdcLinear, ShardedParameter, plain_matrix
 
 
 class SmallGroup:
@@ -308,7 +308,7 @@ class FusedDecoderLayer(nn.Module):
         o = ops.varlen_attention_qkv(qkv, c.num_heads, c.num_kv_heads, c.head_dim, cu_seqlens, max_seqlen, causal=True)
         x = self.wo(o.reshape(T, c.num_heads * c.head_dim), residual=x)
         h, x = s.norm_residual(x, f"layers.{i}.mlp_norm.weight", c.rms_eps)
-        gate_up, down = self.w_gate_up.plain_matrix(h), self.w_down.plain_matrix(h)
+        gate_up, down = plain_matrix(self.w_gate_up, h), plain_matrix(self.w_down, h)
         if gate_up and down:
             return ops._ext().sharded_mlp(h, x, gate_up, down)
         return self.w_down(ops.swiglu(self.w_gate_up(h)), residual=x)

@@ -323,14 +323,6 @@ class OdcLinear(nn.Module):
     def grad_scale(self) -> float:
         return self.weight.grad_scale
 
-    def plain_matrix(self, x):
-        """The native handle where the whole matrix is this rank's and nobody watches the layer on its own: a caller may then
-        take it together with its neighbours.  Else None."""
-        if self.weight.world != 1 or not x.is_cuda or self.bias is not None or self._forward_hooks or self._forward_pre_hooks \
-                or self._backward_hooks or self._backward_pre_hooks or os.environ.get("ODC_WGRAD_SCATTER", "tma") != "tma":
-            return None
-        return (self.weight.matrix() if self.weight._matrix is None else self.weight._matrix) or None
-
     def forward(self, x, bias=None, residual=None, bias_sink=None):
         """``bias_sink``: fp32 vector the bias gradient is added to (the bias then gets none)."""
         bias = bias if bias is not None else self.bias
@@ -342,6 +334,21 @@ class OdcLinear(nn.Module):
         if x.is_cuda:
             ops._ext().after_start()
         return _OdcLinearFn.apply(x, bias, residual, self, bias_sink)
+
+
+_own_forward = OdcLinear.forward
+
+
+def plain_matrix(layer, x):
+    """The native handle of an ``OdcLinear`` whose whole matrix is this rank's and whose call nobody watches or replaces: its
+    caller may then take the matrix together with its neighbours.  Else None, and the layer has to be called."""
+    if not isinstance(layer, OdcLinear) or "forward" in layer.__dict__ or type(layer).forward is not _own_forward \
+            or type(layer).__call__ is not nn.Module.__call__:
+        return None
+    if layer.weight.world != 1 or not x.is_cuda or layer.bias is not None or layer._forward_hooks or layer._forward_pre_hooks \
+            or layer._backward_hooks or layer._backward_pre_hooks or os.environ.get("ODC_WGRAD_SCATTER", "tma") != "tma":
+        return None
+    return (layer.weight.matrix() if layer.weight._matrix is None else layer.weight._matrix) or None
 
 
 def sharded_parameters() -> List[ShardedParameter]:

@@ -225,3 +225,31 @@ def test_every_accumulator_matches_the_plain_decoder(tied, bias, sync):
         assert set(got) == set(want)
         for name, p in want.items():
             assert _rel(got[name], p.grad) < CHAIN, name
+
+
+class _Counting(torch.nn.Module):
+    def __init__(self, inner, calls):
+        super().__init__()
+        self.inner, self.calls, self.weight = inner, calls, inner.weight   # what the engine asks its layers for
+
+    def forward(self, *args, **kw):
+        self.calls.append(1)
+        return self.inner(*args, **kw)
+
+
+@pytest.mark.parametrize("form", ["hook", "replaced"])
+@pytest.mark.parametrize("name", ["w_gate_up", "w_down"])
+def test_layers_of_the_mlp_are_called_where_somebody_stands_between(form, name):
+    """The MLP takes its two matrices as one function, but not past a module hook or a module put in a layer's place."""
+    with _Engine() as e:
+        mbs = _batches(e.cfg, lo=64, hi=128)   # one key tile per sequence: no sums in a free order
+        clean = e.minibatch(mbs)
+        layer, calls = e.model.layers[1], []
+        if form == "hook":
+            getattr(layer, name).register_forward_hook(lambda *args: calls.append(1))
+        else:
+            setattr(layer, name, _Counting(getattr(layer, name), calls))
+        got = e.minibatch(mbs)
+        assert len(calls) == len(mbs)
+        for key, want in clean.items():   # the same roundings; fp32 sums of products in another order
+            assert _rel(got[key], want) < 1e-3, key

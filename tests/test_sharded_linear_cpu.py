@@ -1,4 +1,5 @@
 """Host side of the sharded linear layer: what it hands to the native extension (a stand-in here; no GPU)."""
+import pytest
 import torch
 
 from odc_b200.parallel import OdcLinear
@@ -29,3 +30,48 @@ def test_keep_weight_is_read_at_every_call(monkeypatch):
     layer.keep_weight = True
     layer(_OnGpu())
     assert ext.kept == [False, True]
+
+
+def _layer(cls=OdcLinear):
+    layer = cls.__new__(cls)
+    torch.nn.Module.__init__(layer)
+    layer.bias, layer.keep_weight = None, False
+    layer.weight = type("Weight", (), {"_matrix": object(), "world": 1})()
+    return layer
+
+
+class _Wrapped(torch.nn.Module):
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, x, **kw):
+        return self.inner(x, **kw)
+
+
+class _OwnForward(OdcLinear):
+    def forward(self, x, *args, **kw):
+        return super().forward(x, *args, **kw)
+
+
+def test_replaced_layers_are_called_and_not_passed_by(monkeypatch):
+    """The MLP takes both matrices at once only from layers that are what they were built as."""
+    layer = _layer()
+    assert L.plain_matrix(layer, _OnGpu()) is layer.weight._matrix
+    assert L.plain_matrix(_Wrapped(layer), _OnGpu()) is None
+    assert L.plain_matrix(_layer(_OwnForward), _OnGpu()) is None
+    patched = _layer()
+    patched.forward = lambda *args, **kw: None
+    assert L.plain_matrix(patched, _OnGpu()) is None
+    monkeypatch.setattr(OdcLinear, "forward", lambda self, x, **kw: x)
+    assert L.plain_matrix(layer, _OnGpu()) is None
+
+
+@pytest.mark.parametrize("register", ["register_forward_hook", "register_forward_pre_hook", "register_full_backward_hook",
+                                      "register_full_backward_pre_hook"])
+def test_watched_layers_are_called(register):
+    layer = _layer()
+    handle = getattr(layer, register)(lambda *args: None)
+    assert L.plain_matrix(layer, _OnGpu()) is None
+    handle.remove()
+    assert L.plain_matrix(layer, _OnGpu()) is layer.weight._matrix
