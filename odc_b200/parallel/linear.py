@@ -346,7 +346,8 @@ def plain_matrix(layer, x):
             or type(layer).__call__ is not nn.Module.__call__:
         return None
     if layer.weight.world != 1 or not x.is_cuda or layer.bias is not None or layer._forward_hooks or layer._forward_pre_hooks \
-            or layer._backward_hooks or layer._backward_pre_hooks or os.environ.get("ODC_WGRAD_SCATTER", "tma") != "tma":
+            or layer._backward_hooks or layer._backward_pre_hooks or nn.modules.module._has_any_global_hook() \
+            or os.environ.get("ODC_WGRAD_SCATTER", "tma") != "tma":
         return None
     return (layer.weight.matrix() if layer.weight._matrix is None else layer.weight._matrix) or None
 

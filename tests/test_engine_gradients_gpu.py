@@ -237,19 +237,26 @@ class _Counting(torch.nn.Module):
         return self.inner(*args, **kw)
 
 
-@pytest.mark.parametrize("form", ["hook", "replaced"])
+@pytest.mark.parametrize("form", ["hook", "global hook", "replaced"])
 @pytest.mark.parametrize("name", ["w_gate_up", "w_down"])
 def test_layers_of_the_mlp_are_called_where_somebody_stands_between(form, name):
     """The MLP takes its two matrices as one function, but not past a module hook or a module put in a layer's place."""
     with _Engine() as e:
         mbs = _batches(e.cfg, lo=64, hi=128)   # one key tile per sequence: no sums in a free order
         clean = e.minibatch(mbs)
-        layer, calls = e.model.layers[1], []
+        layer, calls, handle = e.model.layers[1], [], None
+        inner = getattr(layer, name)
         if form == "hook":
-            getattr(layer, name).register_forward_hook(lambda *args: calls.append(1))
+            inner.register_forward_hook(lambda *args: calls.append(1))
+        elif form == "global hook":
+            handle = torch.nn.modules.module.register_module_forward_hook(lambda m, *args: calls.append(1) if m is inner else None)
         else:
-            setattr(layer, name, _Counting(getattr(layer, name), calls))
-        got = e.minibatch(mbs)
+            setattr(layer, name, _Counting(inner, calls))
+        try:
+            got = e.minibatch(mbs)
+        finally:
+            if handle is not None:
+                handle.remove()
         assert len(calls) == len(mbs)
         for key, want in clean.items():   # the same roundings; fp32 sums of products in another order
             assert _rel(got[key], want) < 1e-3, key

@@ -67,11 +67,13 @@ def test_replaced_layers_are_called_and_not_passed_by(monkeypatch):
     assert L.plain_matrix(layer, _OnGpu()) is None
 
 
+@pytest.mark.parametrize("everywhere", [False, True])
 @pytest.mark.parametrize("register", ["register_forward_hook", "register_forward_pre_hook", "register_full_backward_hook",
                                       "register_full_backward_pre_hook"])
-def test_watched_layers_are_called(register):
+def test_watched_layers_are_called(register, everywhere):
     layer = _layer()
-    handle = getattr(layer, register)(lambda *args: None)
+    where, name = (torch.nn.modules.module, register.replace("register", "register_module")) if everywhere else (layer, register)
+    handle = getattr(where, name)(lambda *args: None)
     assert L.plain_matrix(layer, _OnGpu()) is None
     handle.remove()
     assert L.plain_matrix(layer, _OnGpu()) is layer.weight._matrix
