@@ -1203,7 +1203,16 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
   p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.n_q = n_q; p.n_kv = n_kv; p.lse = lse; p.delta = delta;
   p.dq_acc = dq_acc; p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv);
   p.total_tokens = total_tokens; p.scale = scale; p.causal = causal ? 1 : 0;
-  p.scale_log2 = scale * kLog2e; p.lse_scale = head_dim == 64 ? -1.f / scale : -kLog2e;
+  if (head_dim == 64) {
+    // The log-sum-exp joins the scores before they are scaled, divided by the scale.  A scale of zero (all keys alike), or one
+    // whose quotient could leave fp32, counts as 2^-100 here: no score below 2^76 shows beside a log-sum-exp then.
+    const float score_scale = std::fabs(scale) < 0x1p-100f ? 0x1p-100f : scale;
+    p.scale_log2 = score_scale * kLog2e;
+    p.lse_scale = -1.f / score_scale;
+  } else {
+    p.scale_log2 = scale * kLog2e;
+    p.lse_scale = -kLog2e;
+  }
   p.status = status; p.dkv_stride = dkv_stride;
   p.parts = parts;
   p.kv_parts = kv_parts;
