@@ -537,7 +537,8 @@ struct BwdParams {
 // is also the tensor cores' time for them; staging and loads add 256 KiB.  At D = 64 there is room to take traffic out:
 //   - Every thread needs the log-sum-exp and delta of all its queries: 581 of 3550 clocks per tile went to reading them.  They
 //     are 16-byte rows of an operand instead, each value in three bf16 terms (its 24 bits), and one more K step of S and dP with
-//     a selector of ones adds them to the whole tile.
+//     a selector of ones adds them to the whole tile.  Each has rows of its own: beside a selector of zeros in one row, a NaN or
+//     infinite delta would reach the scores as well.
 //   - dS^T is also written over dP^T in tensor memory, where dK reads it; from shared memory only dQ does.
 // 16321 tokens, lengths up to 8192, 32/8 heads: 1.27 ms, with the rows 1.23, with both 1.16; 8192 tokens in one sequence:
 // 0.95, 0.91, 0.83 ms.
@@ -548,11 +549,11 @@ struct BwdCfg {
   static constexpr int kTile = 128 * D * 2;                // one [128][D] bf16 operand
   static constexpr int kDsBytes = 128 * 128 * 2;
   static constexpr int kStageBytes = 2 * 16384;            // two [128][32] fp32 boxes of the dQ reduction
-  // Log-sum-exp and delta of the tile's queries.  D = 64: as rows of an operand (below), with the two row selectors;
+  // Log-sum-exp and delta of the tile's queries.  D = 64: as rows of an operand (below), with the row selector;
   // D = 128: two stages of plain values that every thread reads (as rows they would have to wait for dP of the tile before,
   // which is late there: 32768 tokens, 40/8 heads 27.4 ms, with rows 27.9)
   static constexpr bool kRows = (D == 64);
-  static constexpr int kStatBytes = kRows ? 2048 + 512 : kQStages * 2 * 128 * 4;
+  static constexpr int kStatBytes = kRows ? 2 * 2048 + 256 : kQStages * 2 * 128 * 4;
   static constexpr int kBarBytes = 256;
   // the dynamic window starts 1024-byte aligned in practice; the kernel checks and reports otherwise
   static constexpr int kAlignSlack = 768;
@@ -597,7 +598,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   constexpr int kQOff = 2 * C::kTile, kDoOff = kQOff + C::kQStages * C::kTile, kDsOff = kDoOff + C::kDoStages * C::kTile;
   constexpr int kStageOff = kDsOff + C::kDsBytes, kStatOff = kStageOff + C::kStageBytes, kBarOff = kStatOff + C::kStatBytes;
   const uint32_t k_smem = base, v_smem = base + C::kTile, ds_smem = base + kDsOff;
-  uint4* rows_smem = reinterpret_cast<uint4*>(smem + kStatOff);  // kRows: [128] queries, the selectors of S and dP, [2][16]
+  uint4* rows_smem = reinterpret_cast<uint4*>(smem + kStatOff);  // kRows: [lse, delta][128] queries, the selector, [2][8]
   float* stats = reinterpret_cast<float*>(smem + kStatOff);      // else [stage][-log2(e) * lse, delta][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kBarOff);
   const uint32_t bar0 = smem_u32(bars);
@@ -635,11 +636,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (C::kRows && warp == 2) {  // ones in the three places of a query's row that S or dP takes
-    uint4 sel = make_uint4(0, 0, 0, 0);
-    if (lane < 8) sel = make_uint4(0x3f803f80u, 0x00003f80u, 0, 0);
-    if (lane >= 16 && lane < 24) sel = make_uint4(0, 0x3f800000u, 0x3f803f80u, 0);
-    rows_smem[128 + lane] = sel;
+  if (C::kRows && warp == 2) {  // ones in the three places of a query's row
+    if (lane < 16) rows_smem[256 + lane] = lane < 8 ? make_uint4(0x3f803f80u, 0x00003f80u, 0, 0) : make_uint4(0, 0, 0, 0);
     fence_proxy_async();
   }
   if (warp == 1) {
@@ -688,15 +686,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (it > 0 && !__all_sync(0xffffffffu, mbar_wait(dp_full, (it - 1) & 1, wc, 25))) break;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {  // three bf16 terms hold the 24 bits of each value
-          uint32_t h[6];
           float rest[2] = {nl[e], dl[e]};
 #pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            const __nv_bfloat16 t = __float2bfloat16(rest[k / 3]);
-            rest[k / 3] -= __bfloat162float(t);
-            h[k] = __bfloat16_as_ushort(t);
+          for (int r = 0; r < 2; ++r) {
+            uint32_t h[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              const __nv_bfloat16 t = __float2bfloat16(rest[r]);
+              rest[r] -= __bfloat162float(t);
+              h[k] = __bfloat16_as_ushort(t);
+            }
+            rows_smem[128 * r + lane + 32 * e] = make_uint4(h[0] | h[1] << 16, h[2], 0, 0);
           }
-          rows_smem[lane + 32 * e] = make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, 0);
         }
         fence_proxy_async();
       } else {
@@ -734,15 +735,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
       };
       // rows of 16 bytes without swizzle: both halves of K read the same eight values, all keys the same eight selector rows
-      const uint64_t rows = make_plain_desc(base + kStatOff, 0, 128);
-      const uint64_t sel_s = make_plain_desc(base + kStatOff + 2048, 128, 0), sel_dp = make_plain_desc(base + kStatOff + 2304, 128, 0);
+      const uint64_t lse_rows = make_plain_desc(base + kStatOff, 0, 128), delta_rows = make_plain_desc(base + kStatOff + 2048, 0, 128);
+      const uint64_t sel = make_plain_desc(base + kStatOff + 4096, 128, 0);
       auto issue_s = [&](int it) -> bool {
         if (!mbar_wait(q_full0 + 8 * (it % C::kQStages), (it / C::kQStages) & 1, wc, 33)) return false;
         tc_fence_after();
         scores(C::kS, k_smem, base + kQOff + (it % C::kQStages) * C::kTile);
         if constexpr (C::kRows) {
           if (!mbar_wait(stat_full0, it & 1, wc, 26)) return false;
-          umma_f16(tmem_base + C::kS, sel_s, rows, idesc_s, 1u);      // - log-sum-exp of the query
+          umma_f16(tmem_base + C::kS, sel, lse_rows, idesc_s, 1u);      // - log-sum-exp of the query
         }
         umma_commit(s_full);
         return true;
@@ -751,7 +752,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (!mbar_wait(do_full0 + 8 * (it % C::kDoStages), (it / C::kDoStages) & 1, wc, 29)) return false;
         tc_fence_after();
         scores(C::kDp, v_smem, base + kDoOff + (it % C::kDoStages) * C::kTile);
-        if constexpr (C::kRows) umma_f16(tmem_base + C::kDp, sel_dp, rows, idesc_s, 1u);    // - delta of the query
+        if constexpr (C::kRows) umma_f16(tmem_base + C::kDp, sel, delta_rows, idesc_s, 1u);    // - delta of the query
         umma_commit(dp_full);
         return true;
       };
