@@ -643,16 +643,21 @@ Tensor attention_qkv(Tensor qkv, int64_t n_q, int64_t n_kv, int64_t d, Tensor cu
 }
 
 // ---- LM head ---------------------------------------------------------------------------------------------------------
+void check_chunk(int64_t chunk) {
+  if (chunk == 0) throw py::value_error("chunk must not be zero");   // the walk over the tokens would not end
+  TORCH_CHECK(chunk > 0, "chunk must be positive");
+}
 // bf16 logits of one chunk of tokens, whatever type a library product of the head is in
 Tensor chunk_logits(const Tensor& h, int64_t vocab, int64_t chunk) {
-  if (chunk == 0) throw py::value_error("chunk must not be zero");   // the walk over the tokens would not end
+  check_chunk(chunk);
   return at::empty({std::min(chunk, h.size(0)), vocab}, h.options().dtype(at::kBFloat16));
 }
 
-// One chunk of the head: logits = h w^T, then either the log-probability of every label (`per_token`; the logits are scratch) or
-// the logits turned in place into loss_scale * (softmax - onehot), with the summed loss added to `loss`.  Where the kernel takes
-// the product its epilogue leaves the softmax statistics, and one pass over the logits, or both, is saved.
-void head_chunk(const Tensor& h, const Tensor& w, const Tensor& logits, const Tensor& labels, const c10::optional<Tensor>& loss_scale,
+// One chunk of the head: logits = h w^T, then either the log-probability of every label (`per_token`; `logits` is scratch that the
+// first chunk to need it brings) or the logits turned in place into loss_scale * (softmax - onehot), with the summed loss added
+// to `loss`.  Where the kernel takes the product its epilogue leaves the softmax statistics, and one pass over the logits, or
+// both, is saved.
+void head_chunk(const Tensor& h, const Tensor& w, Tensor& logits, const Tensor& labels, const c10::optional<Tensor>& loss_scale,
                 const Tensor& loss, const Tensor& per_token, int64_t ignore_index, double inv_temp) {
   const int64_t n = h.size(0), V = w.size(0);
   if (!library_gemm() && odc::gemm_pairs_enabled() && h.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
@@ -687,11 +692,13 @@ void head_chunk(const Tensor& h, const Tensor& w, const Tensor& logits, const Te
       return;
     }
   }
-  product_into(h, w, logits, kNT);
+  if (!logits.defined()) logits = chunk_logits(h, V, n);
+  const Tensor lg = logits.narrow(0, 0, n);
+  product_into(h, w, lg, kNT);
   if (per_token.defined())
-    token_logprobs(logits, labels, per_token, ignore_index, inv_temp);
+    token_logprobs(lg, labels, per_token, ignore_index, inv_temp);
   else
-    ce_fwd_bwd(logits, labels, loss_scale, loss, ignore_index, inv_temp);
+    ce_fwd_bwd(lg, labels, loss_scale, loss, ignore_index, inv_temp);
   count();
 }
 
@@ -710,7 +717,8 @@ std::tuple<Tensor, Tensor, Tensor> lm_head_loss(const Tensor& h, const Tensor& w
   if (T == 0 && need_dw) dw.zero_();
   for (int64_t s = 0; s < T; s += chunk) {
     const int64_t n = std::min(chunk, T - s);
-    const Tensor hs = h.narrow(0, s, n), lg = logits.narrow(0, 0, n);
+    const Tensor hs = h.narrow(0, s, n);
+    Tensor lg = logits.narrow(0, 0, n);
     head_chunk(hs, w, lg, labels.narrow(0, s, n), loss_scale.has_value() ? c10::optional<Tensor>(loss_scale->narrow(0, s, n)) : c10::nullopt,
                loss, {}, ignore_index, 1.0);
     if (need_dh) product_into(lg, w, dh.narrow(0, s, n), kNN);
@@ -751,11 +759,11 @@ struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
                         int64_t chunk, bool need_dh, bool need_dw) {
     const int64_t T = h.size(0);
     auto out = at::empty({T}, h.options().dtype(at::kFloat));
-    auto logits = chunk_logits(h, w.size(0), chunk);
+    check_chunk(chunk);
+    Tensor logits;
     for (int64_t s = 0; s < T; s += chunk) {
       const int64_t n = std::min(chunk, T - s);
-      const Tensor lg = logits.narrow(0, 0, n);
-      head_chunk(h.narrow(0, s, n), w, lg, ids.narrow(0, s, n), c10::nullopt, {}, out.narrow(0, s, n), ignore_index, 1.0 / temperature);
+      head_chunk(h.narrow(0, s, n), w, logits, ids.narrow(0, s, n), c10::nullopt, {}, out.narrow(0, s, n), ignore_index, 1.0 / temperature);
     }
     ctx->save_for_backward({h, w, ids});
     ctx->saved_data["cfg"] = std::vector<int64_t>{ignore_index, chunk, need_dh, need_dw};
@@ -778,7 +786,8 @@ struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
     auto logits = chunk_logits(h, w.size(0), chunk);
     for (int64_t s = 0; s < T; s += chunk) {
       const int64_t n = std::min(chunk, T - s);
-      const Tensor hs = h.narrow(0, s, n), lg = logits.narrow(0, 0, n);
+      const Tensor hs = h.narrow(0, s, n);
+      Tensor lg = logits.narrow(0, 0, n);
       head_chunk(hs, w, lg, ids.narrow(0, s, n), scale.narrow(0, s, n), sink, {}, cfg[0], 1.0 / temperature);
       if (cfg[2]) product_into(lg, w, dh.narrow(0, s, n), kNN);
       if (cfg[3]) product_into(lg, hs, dw, kTN, {}, s > 0);

@@ -1022,3 +1022,29 @@ def test_mlp_matches_its_parts(ext, T, H, F):
     gate_up = ops.linear(x, gu).detach()
     one, two = ext.swiglu_product_bwd(dy, down.detach(), gate_up), ext.swiglu_bwd(dy @ down.detach(), gate_up)
     assert ((one.float() - two.float()).norm() / two.float().norm()).item() < 1e-2
+
+
+def test_log_probabilities_alone_hold_no_logits():
+    """Forward only, the product leaves row statistics (8 bytes per 256 words) and the logits are never written: no scratch for
+    them is held, except for a last chunk below a tile of rows, which takes the passes over logits."""
+    from odc_b200 import ops
+    T, V, H, chunk = 1100, 8192, 256, 512          # chunks of 512, 512 and 76 rows
+    h, w = torch.randn(T, H, device="cuda").bfloat16(), torch.randn(V, H, device="cuda").bfloat16()
+    ids = torch.randint(0, V, (T,), device="cuda")
+    run = lambda n: ops.linear_token_logprobs(h[:n], w, ids[:n], chunk=chunk)
+    with torch.no_grad():
+        for n, limit in ((1024, 1 << 20), (T, (1 << 20) + 76 * V * 2)):
+            run(n)
+            torch.cuda.synchronize()
+            torch.cuda.reset_peak_memory_stats()
+            held = torch.cuda.memory_allocated()
+            out = run(n)
+            torch.cuda.synchronize()
+            assert torch.cuda.max_memory_allocated() - held < limit
+            want = (h[:n].double() @ w.double().t()).log_softmax(-1).gather(1, ids[:n, None])[:, 0]
+            # logits around 100 are rounded to bf16: 2^-8 of their size
+            assert (out.double() - want).abs().max().item() < 2 ** -8 * 200
+        for chunk, error in ((0, ValueError), (-1, RuntimeError)):
+            for n in (0, T):
+                with pytest.raises(error):
+                    run(n)
