@@ -220,7 +220,7 @@ void gemm_into(const Tensor& a, const Tensor& b, const Tensor& c, int lay, const
   }
   Tensor parts;  // few tiles and a long reduction: scratch for the partial products
   if (pair < 0 && !accumulate && odc::gemm_pairs_enabled()) {
-    const size_t bytes = odc::gemm_split_bytes(M, N, K, kind_of(c.scalar_type()), sm_count());
+    const size_t bytes = odc::gemm_plan(M, N, K, kind_of(c.scalar_type()), sm_count()).scratch_bytes;
     if (bytes > 0) {
       parts = at::empty({static_cast<int64_t>(bytes / sizeof(float))}, a.options().dtype(at::kFloat));
       count();
@@ -990,7 +990,15 @@ void register_ops(py::module_& m) {
   m.def("sumsq", &sumsq);
   m.def("gemm", &gemm, py::arg("a"), py::arg("b"), py::arg("c"), py::arg("layout"), py::arg("bias"),
         py::arg("accumulate"), py::arg("residual") = py::none(), py::arg("pair") = -1);
-  m.def("gemm_split_bytes", [](int M, int N, int K) { return odc::gemm_split_bytes(M, N, K, odc::kBF16, sm_count(), true); });
+  m.def("gemm_plan", [](int M, int N, int K, int sms) {
+    const odc::GemmPlan p = odc::gemm_plan(M, N, K, odc::kBF16, sms);
+    return std::make_tuple(p.tiles, p.whole, p.parts, p.scratch_bytes);
+  }, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("sms"));  // (tiles, whole ones, parts of each other, scratch) in bf16
+  // scratch of a product of which every tile is divided; 0 for one of which some or all are whole
+  m.def("gemm_split_bytes", [](int M, int N, int K) {
+    const odc::GemmPlan p = odc::gemm_plan(M, N, K, odc::kBF16, sm_count());
+    return p.whole == 0 ? p.scratch_bytes : 0;
+  });
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
   m.def("attn_plan", [](int tokens, int seqs, int longest, int n_q, int n_kv, int d, bool causal, int sms) {

@@ -108,16 +108,19 @@ cudaError_t launch_sumsq(const void* x, int kind, size_t n, float* out, int sm_c
 // ---- tcgen05 GEMM ----------------------------------------------------------------------------
 // layout: 0 = "nt" C[M,N] = A[M,K] B[N,K]^T ; 1 = "nn" C = A[M,K] B[K,N] ; 2 = "tn" C = A[K,M]^T B[K,N]
 // All operands row-major bf16; C is bf16 or fp32; bias (bf16, length N) optional; accumulate adds into C.
-struct GemmPlan;
 cudaError_t gemm_bf16(const void* a, const void* b, void* c, int c_kind, const void* bias, int M, int N, int K,
                       int layout, bool accumulate, long long lda, long long ldb, long long ldc, int* status,
                       int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0,
                       int pair_mode = -1 /* -1: ODC_GEMM_PAIR decides, 0: single-CTA kernel, 1: CTA-pair kernel */,
                       float* split_ws = nullptr);
 bool gemm_pairs_enabled();   // ODC_GEMM_PAIR=0 (read once) keeps every product on the single-CTA kernel
-// Bytes of scratch (split_ws) with which the CTA-pair kernel would divide the reduction of some tiles of this product, or
-// (all_tiles) of every one; 0: it would not.
-size_t gemm_split_bytes(int M, int N, int K, int c_kind, int sm_count, bool all_tiles = false);
+// How the CTA-pair kernel takes a product that it is given scratch for (split_ws): the first `whole` of its 256 x 256 tiles as
+// they are, the reduction of every other in `parts`.  No scratch bytes: nothing is divided.
+struct GemmPlan {
+  int tiles, whole, parts;
+  size_t scratch_bytes;
+};
+GemmPlan gemm_plan(int M, int N, int K, int c_kind, int sm_count);
 
 // Same contract on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles).  Returns cudaErrorNotSupported for shapes it
 // does not take (N below 256, M below 256 without split_ws, bf16 accumulation); gemm_bf16 tries it first unless ODC_GEMM_PAIR=0.

@@ -794,12 +794,12 @@ static SplitPlan product_plan(int M, int N, int K, int sm_count) {
   return all.splits > 1 || M < 256 ? all : plan_splits(M, N, K, sm_count, true, true);
 }
 
-size_t gemm_split_bytes(int M, int N, int K, int c_kind, int sm_count, bool all_tiles) {
+GemmPlan gemm_plan(int M, int N, int K, int c_kind, int sm_count) {
   using namespace gemm_pair;
-  if (c_kind != kBF16 || M < 1 || N < 256 || K < BK || sm_count < 2) return 0;
-  const SplitPlan plan = all_tiles ? plan_splits(M, N, K, sm_count, true, false) : product_plan(M, N, K, sm_count);
-  const size_t tiles = static_cast<size_t>((M + 255) / 256) * ((N + BN - 1) / BN);
-  return plan.splits == 1 ? 0 : (tiles - plan.whole) * plan.splits * 256 * BN * sizeof(float);
+  const int tiles = (M + 255) / 256 * ((N + BN - 1) / BN);
+  if (c_kind != kBF16 || M < 1 || N < 256 || K < BK || sm_count < 2) return {tiles, tiles, 1, 0};
+  const SplitPlan plan = product_plan(M, N, K, sm_count);
+  return {tiles, plan.whole, plan.splits, static_cast<size_t>(tiles - plan.whole) * plan.splits * 256 * BN * sizeof(float)};
 }
 
 // Returns cudaErrorNotSupported when the shape is not worth a CTA pair (the caller then uses the single-CTA kernel).

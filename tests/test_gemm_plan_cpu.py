@@ -1,0 +1,30 @@
+"""Which tiles of a product are divided: host rules, checked without a GPU."""
+import pytest
+
+from odc_b200 import _ext
+
+SMS = 148
+
+
+def _plan(M, N, K):
+    return _ext.load().gemm_plan(M, N, K, SMS)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 256, 64), (24, 512, 512), (255, 2048, 8192), (765, 1536, 17920), (2304, 2304, 4096),
+                                   (3072, 2048, 8200), (5000, 1800, 8192), (16384, 2048, 8192), (30000, 4096, 14336)])
+def test_the_plan_covers_every_tile_and_its_scratch(M, N, K):
+    tiles, whole, parts, scratch = _plan(M, N, K)
+    assert tiles == -(-M // 256) * -(-N // 256) and 0 <= whole <= tiles
+    assert (whole == tiles) == (parts == 1) == (scratch == 0)
+    assert scratch == (tiles - whole) * parts * 256 * 256 * 4 and parts <= min(8, -(-K // 64))
+    if parts > 1 and whole:                # whole rounds of all pairs stay as they are
+        assert whole % (SMS // 2) == 0
+
+
+def test_full_rounds_and_short_reductions_are_not_divided():
+    assert _plan(74 * 256, 256, 8192)[2] == 1        # one tile for every pair
+    tiles, whole, parts, _ = _plan(2304, 2304, 4096)   # 7 tiles more than pairs
+    assert (tiles, whole) == (81, 74) and parts > 1
+    assert _plan(765, 1536, 512)[2] == 1
+    assert _plan(765, 1536, 17920)[1] == 0
+    assert _plan(300, 200, 4096)[2] == 1             # not a product for pairs

@@ -370,13 +370,16 @@ def test_gemm_divided_last_round(ext, layout, M, N, K):
     a = A.t().contiguous() if layout == "tn" else A
     b = B.t().contiguous() if layout == "nt" else B
     want = A.double() @ B.double()
-    assert ext.gemm_split_bytes(M, N, K) == 0
+    tiles, whole, parts, scratch = ext.gemm_plan(M, N, K, torch.cuda.get_device_properties(0).multi_processor_count)
+    assert 0 < whole < tiles and parts > 1 and ext.gemm_split_bytes(M, N, K) == 0
     c = torch.empty(M, N + 16, dtype=torch.bfloat16, device="cuda")[:, :N]
     for kw, exp in (((None, False), want), ((bias, False, res), want + bias.double() + res.double())):
-        before = ext.kernel_launches()
+        before, held = ext.kernel_launches(), torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
         ext.gemm(a, b, c, layout, *kw)
         torch.cuda.synchronize()
         assert ext.kernel_launches() - before == 1   # the sum of the parts
+        assert scratch <= torch.cuda.max_memory_allocated() - held < scratch + (2 << 20)
         assert ext.kernel_status()[0].item() == 0, ext.kernel_status().tolist()
         # fp32 sums of K products (sqrt(K) 2^-24 each way, far below) and one rounding to bf16
         assert ((c.double() - exp).abs() <= 2 ** -8 * exp.abs() + 1e-4 * K ** 0.5).all()
