@@ -994,6 +994,10 @@ void register_ops(py::module_& m) {
     const odc::GemmPlan p = odc::gemm_plan(M, N, K, odc::kBF16, sms);
     return std::make_tuple(p.tiles, p.whole, p.parts, p.scratch_bytes);
   }, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("sms"));  // (tiles, whole ones, parts of each other, scratch) in bf16
+  m.def("scatter_plan", [](int n_out, int k_in, int tokens, int ranks, int sms) {
+    const odc::GemmPlan p = odc::scatter_plan(n_out, k_in, tokens, ranks, sms);
+    return std::make_tuple(p.tiles, p.whole, p.parts);
+  }, py::arg("n_out"), py::arg("k_in"), py::arg("tokens"), py::arg("ranks"), py::arg("sms"));
   // scratch of a product of which every tile is divided; 0 for one of which some or all are whole
   m.def("gemm_split_bytes", [](int M, int N, int K) {
     const odc::GemmPlan p = odc::gemm_plan(M, N, K, odc::kBF16, sm_count());

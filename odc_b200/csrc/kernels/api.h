@@ -121,6 +121,8 @@ struct GemmPlan {
   size_t scratch_bytes;
 };
 GemmPlan gemm_plan(int M, int N, int K, int c_kind, int sm_count);
+// the same of a weight gradient that is added into its owners' accumulators (no scratch) and may be divided
+GemmPlan scatter_plan(int n_out, int k_in, int tokens, int nranks, int sm_count);
 
 // Same contract on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles).  Returns cudaErrorNotSupported for shapes it
 // does not take (N below 256, M below 256 without split_ws, bf16 accumulation); gemm_bf16 tries it first unless ODC_GEMM_PAIR=0.

@@ -758,15 +758,24 @@ static int rotate_mode() {
 // Which tiles are divided, and how many ways, where the last round of tiles (or the only one) leaves pairs idle.  In units of
 // a k-block (512 clocks of the tensor cores, 0.28 us): a product takes as many rounds as its items need, each as long as its
 // longest item.  Dividing a bf16 product adds a second launch (3 us: 11 units) and writes and reads the fp32 partials once
-// (at 5 TB/s, 1.4 MB per unit); a scattered one only adds the parts to the accumulators, once more each.  All tiles are
-// divided only where that is a tenth faster, those of the last rounds where it is a twentieth.
+// (at 5 TB/s, 1.4 MB per unit); a scattered one only adds the parts to the accumulators, once more each, and what other ranks
+// own crosses the link (770 GB/s, 0.216 MB per unit; priced as if nothing ran meanwhile, not measured on several GPUs).  All
+// tiles are divided only where that is a tenth faster, those of the last rounds where it is a twentieth.
 // All tiles: 765 x 1536 with K = 8960: 59 us whole, 29 us divided by four with the sum.  The last rounds, weight gradients
 // over 16321 rows: 3072 x 2048 (96 tiles on 74 pairs) 197 us whole, now 158; 2048 x 8192 410 and 370; over 30000 rows
 // 4096 x 4096 750 and 709.
 struct SplitPlan {
   int whole, splits, kb_split;
 };
-static SplitPlan plan_splits(int M, int N, int K, int sm_count, bool partials, bool tail) {
+struct SplitCost {   // in units: of dividing at all, and per MB of fp32 parts
+  double fixed, per_mb;
+};
+constexpr SplitCost kPartialsCost{11.0, 2 / 1.4};
+static SplitCost scatter_cost(int nranks) {
+  const double remote = static_cast<double>(nranks - 1) / nranks;
+  return {2.0, (1 - remote) / 1.4 + remote / 0.216};
+}
+static SplitPlan plan_splits(int M, int N, int K, int sm_count, const SplitCost& dividing, bool tail) {
   using namespace gemm_pair;
   const int tiles = (M + 255) / 256 * ((N + BN - 1) / BN), pairs = sm_count / 2;
   const int kb = (K + BK - 1) / BK, rounds = (tiles + pairs - 1) / pairs;
@@ -781,7 +790,7 @@ static SplitPlan plan_splits(int M, int N, int K, int sm_count, bool partials, b
       const long long items = static_cast<long long>(rest) * s;
       const double mb = items * 0.262144;
       const double cost = static_cast<double>(full) * kb + static_cast<double>((items + pairs - 1) / pairs) * each +
-                          (partials ? 11.0 + 2 * mb / 1.4 : 2.0 + mb / 1.4);
+                          dividing.fixed + mb * dividing.per_mb;
       if (cost < best) { best = cost; plan = SplitPlan{full * pairs, s, each}; }
     }
   }
@@ -790,8 +799,8 @@ static SplitPlan plan_splits(int M, int N, int K, int sm_count, bool partials, b
 
 // The plan of a bf16 product: all tiles divided where they are fewer than the pairs, else those of its last rounds.
 static SplitPlan product_plan(int M, int N, int K, int sm_count) {
-  const SplitPlan all = plan_splits(M, N, K, sm_count, true, false);
-  return all.splits > 1 || M < 256 ? all : plan_splits(M, N, K, sm_count, true, true);
+  const SplitPlan all = plan_splits(M, N, K, sm_count, kPartialsCost, false);
+  return all.splits > 1 || M < 256 ? all : plan_splits(M, N, K, sm_count, kPartialsCost, true);
 }
 
 GemmPlan gemm_plan(int M, int N, int K, int c_kind, int sm_count) {
@@ -880,7 +889,7 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
 cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* act, int M, int F, int K, long long ldx,
                              long long ldw, int* status, int sm_count, cudaStream_t stream) {
   using namespace gemm_pair;
-  if (M < 256 || F < BNH || K < BK || sm_count < 2 || plan_splits(M, 2 * F, K, sm_count, true, false).splits > 1)
+  if (M < 256 || F < BNH || K < BK || sm_count < 2 || plan_splits(M, 2 * F, K, sm_count, kPartialsCost, false).splits > 1)
     return cudaErrorNotSupported;
   if ((ldx % 8) || (ldw % 8) || (F % 8) ||
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(gate_up) |
@@ -922,7 +931,7 @@ cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* 
 cudaError_t gemm_swiglu_bwd_pair(const void* dy, const void* w, const void* gate_up, void* dgate_up, int M, int F, int K,
                                  long long lddy, long long ldw, int* status, int sm_count, cudaStream_t stream) {
   using namespace gemm_pair;
-  if (M < 256 || F < 256 || K < BK || sm_count < 2 || plan_splits(M, F, K, sm_count, true, false).splits > 1)
+  if (M < 256 || F < 256 || K < BK || sm_count < 2 || plan_splits(M, F, K, sm_count, kPartialsCost, false).splits > 1)
     return cudaErrorNotSupported;
   if ((lddy % 8) || (ldw % 8) || (F % 8) ||
       ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(gate_up) |
@@ -993,6 +1002,12 @@ cudaError_t gemm_logits_pair(const void* h, const void* w, void* logits, const l
   return cudaGetLastError();
 }
 
+GemmPlan scatter_plan(int n_out, int k_in, int tokens, int nranks, int sm_count) {
+  using namespace gemm_pair;
+  const SplitPlan plan = plan_splits(n_out, k_in, tokens, sm_count, scatter_cost(nranks), true);
+  return {(n_out + 255) / 256 * ((k_in + BN - 1) / BN), plan.whole, plan.splits, 0};
+}
+
 // dW[n_out, k_in] = dY^T X on CTA pairs; every 128 x 32 fp32 output box is added (x scale) into the accumulator of the
 // rank that owns its rows by the TMA unit, through the peer mapping; then one arrival per owner.  Same contract as
 // gemm_wgrad_scatter_tma; returns cudaErrorNotSupported for shapes it does not take.
@@ -1036,7 +1051,7 @@ cudaError_t gemm_wgrad_scatter_pair(const void* dy, const void* x, int tokens, i
   if (rotate_mode() >= 1)
     p.rot_m = static_cast<int>((static_cast<long long>(start_rank) * rows_per_rank / 256) % p.tiles_m);
   SplitPlan plan{p.tiles_m * p.tiles_n, 1, 0};
-  if (!fixed_order) plan = plan_splits(n_out, k_in, tokens, sm_count, false, true);
+  if (!fixed_order) plan = plan_splits(n_out, k_in, tokens, sm_count, scatter_cost(nranks), true);
   p.whole = plan.whole; p.splits = plan.splits; p.kb_split = plan.kb_split;
   const int items = p.whole + (p.tiles_m * p.tiles_n - p.whole) * p.splits;
   const int pairs = items < sm_count / 2 ? items : sm_count / 2;

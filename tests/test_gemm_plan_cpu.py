@@ -28,3 +28,26 @@ def test_full_rounds_and_short_reductions_are_not_divided():
     assert _plan(765, 1536, 512)[2] == 1
     assert _plan(765, 1536, 17920)[1] == 0
     assert _plan(300, 200, 4096)[2] == 1             # not a product for pairs
+
+
+@pytest.mark.parametrize("n_out,k_in,tokens", [(512, 512, 1900), (768, 520, 1900), (1536, 1536, 4099), (3072, 2048, 4099),
+                                               (3072, 2048, 16321), (2048, 8192, 16321), (4096, 4096, 30000)])
+def test_weight_gradients_are_divided_only_where_the_link_allows_it(n_out, k_in, tokens):
+    """Parts that other ranks own cost their way over the link: what is divided for one rank may be whole for several, and
+    the parts, sent one after the other at 770 GB/s, never take longer than the rounds of products that dividing saves."""
+    plan = lambda ranks: _ext.load().scatter_plan(n_out, k_in, tokens, ranks, SMS)
+    tiles, whole, parts = plan(1)
+    assert parts > 1 and whole < tiles
+    for ranks in (2, 8):
+        n, full, parts = plan(ranks)
+        assert n == tiles
+        if parts > 1:
+            kb, items = -(-tokens // 64), (tiles - full) * parts
+            saved = (-(-tiles // (SMS // 2)) - full // (SMS // 2)) * kb - -(-items // (SMS // 2)) * -(-kb // parts)
+            link = items * 256 * 256 * 4 * (ranks - 1) / ranks / 770e9
+            assert link < saved * 0.285e-6   # a k-block of a tile takes about 0.28 us
+
+
+def test_small_weight_gradients_stay_whole_across_ranks():
+    plan = lambda ranks: _ext.load().scatter_plan(512, 512, 765, ranks, SMS)
+    assert plan(1)[2] > 1 and plan(8) == (4, 4, 1)
