@@ -324,6 +324,16 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(Tensor dout, Tensor q, Tenso
   return {dq, dk, dv, fused_qkv ? dqkv : dq};  // 4th: the fused gradient when requested
 }
 
+Tensor exp2_poly(Tensor x) {
+  c10::cuda::CUDAGuard g(x.device());
+  odc::bind_device(x.get_device());
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.is_contiguous() && x.numel() % 2 == 0 &&
+                  reinterpret_cast<uintptr_t>(x.data_ptr()) % 8 == 0, "exp2_poly: pairs of fp32 values, contiguous");
+  auto y = at::empty_like(x);
+  check(odc::launch_exp2_poly(x.data_ptr<float>(), y.data_ptr<float>(), x.numel(), cur_stream()), "exp2_poly");
+  return y;
+}
+
 // ------------------------------------------------------------------------------------------------ differentiable ops
 bool env_on(const char* name) {
   const char* e = std::getenv(name);
@@ -1005,6 +1015,7 @@ void register_ops(py::module_& m) {
   });
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_bwd", &attn_bwd);
+  m.def("exp2_poly", &exp2_poly);
   m.def("attn_plan", [](int tokens, int seqs, int longest, int n_q, int n_kv, int d, bool causal, int sms) {
     return std::make_tuple(d == 128 && odc::attn_fwd_pairs(tokens, seqs, longest, n_q, n_kv, causal, sms),
                            odc::attn_bwd_parts(tokens, seqs, longest, n_q, n_kv, d, causal, sms));

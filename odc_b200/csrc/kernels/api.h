@@ -195,6 +195,8 @@ cudaError_t attn_fwd(const void* q, const void* k, const void* v, void* o, float
                      int* status, int sm_count, cudaStream_t stream);
 // head_dim 128: the forward takes query tiles in pairs, else (and with head_dim 64) one per CTA
 bool attn_fwd_pairs(int total_tokens, int num_seqs, int max_seqlen, int n_q, int n_kv, bool causal, int sm_count);
+// 2^x as the forward computes it on the FMA pipe, for tests; n is even, both 8-byte aligned
+cudaError_t launch_exp2_poly(const float* x, float* y, long long n, cudaStream_t stream);
 // CTAs per (key tile, kv head) of the backward; above 1 it needs kv_parts, [parts][2][tokens, n_kv, head_dim] fp32 scratch
 int attn_bwd_parts(int total_tokens, int num_seqs, int max_seqlen, int n_q, int n_kv, int head_dim, bool causal, int sm_count);
 cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o, const float* lse,

@@ -202,6 +202,12 @@ __device__ __forceinline__ float2 exp2_poly(float2 x) {
   return mul2(p, make_float2(__uint_as_float(__float_as_uint(t.x) << 23), __uint_as_float(__float_as_uint(t.y) << 23)));
 }
 
+// exp2_poly on its own, for tests of its error
+__global__ void __launch_bounds__(256) exp2_poly_kernel(const float2* x, float2* y, long long n2) {
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (i < n2) y[i] = exp2_poly(x[i]);
+}
+
 template <int D, int Tiles>
 __global__ void __launch_bounds__(FwdCfg<D, Tiles>::kThreads, FwdCfg<D, Tiles>::kCtasPerSm)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -1238,6 +1244,14 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
   launch(narrow_grads_kernel, static_cast<int>(g), 256, 0, stream,
       dq_acc, static_cast<__nv_bfloat16*>(dq), n8, n_q * head_dim / 8, dq_stride, scale, kv_parts, p.parts,
       static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), kv_n8, n_kv * head_dim / 8, dkv_stride);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_exp2_poly(const float* x, float* y, long long n, cudaStream_t stream) {
+  if (n % 2 != 0) return cudaErrorInvalidValue;
+  if (n == 0) return cudaSuccess;
+  launch(exp2_poly_kernel, static_cast<unsigned int>((n / 2 + 255) / 256), 256, 0, stream, reinterpret_cast<const float2*>(x),
+      reinterpret_cast<float2*>(y), n / 2);
   return cudaGetLastError();
 }
 

@@ -967,7 +967,7 @@ def test_rmsnorm_residual_backward_fuses_the_residual_gradient():
 @pytest.mark.parametrize("temperature", [1.0, 0.7])
 def test_head_statistics_from_the_product(ext, T, V, H, chunk, temperature):
     """Softmax statistics of ragged tiles, in chunks (a last one below a tile takes the other path): log-probabilities, loss and
-    both gradients; ignored and weightless rows; a row of -inf and one with NaN stay what they are."""
+    both gradients; ignored and weightless rows; a NaN row stays one row."""
     from odc_b200 import ops
     torch.manual_seed(T + V)
     h = (2 * torch.randn(T, H, device="cuda")).bfloat16().requires_grad_()
@@ -1000,6 +1000,46 @@ def test_head_statistics_from_the_product(ext, T, V, H, chunk, temperature):
     with torch.no_grad():
         out = ops.linear_token_logprobs(bad, w, ids, temperature, chunk=chunk)
     assert out[11].isnan() and out[12:].isfinite().all() and out[:11].isfinite().all()
+    bad.requires_grad_()
+    loss = ops.linear_cross_entropy(bad, w, ids, weight, chunk=chunk)
+    gh, = torch.autograd.grad(loss, bad)
+    assert loss.isnan() and gh[11].isnan().all() and gh[12:].isfinite().all() and gh[:11].isfinite().all()
+    assert ext.kernel_status()[0].item() == 0
+
+
+@pytest.mark.parametrize("T,V", [(256, 1000), (300, 2056)])
+def test_head_statistics_of_infinite_logits(ext, T, V):
+    """Logits of -inf beside finite ones, over a whole tile of 256 words and in single places: they have no weight, and nothing
+    else changes.  A row of nothing but -inf has no probabilities, as a softmax in 64 bits has none."""
+    from odc_b200 import ops
+    torch.manual_seed(T + V)
+    h = torch.randn(T, 64, device="cuda").bfloat16()
+    w = (torch.randn(V, 64, device="cuda") / 8).bfloat16()
+    gone = torch.zeros(V, dtype=torch.bool, device="cuda")
+    gone[256:512] = True
+    gone[torch.arange(3, V, 97, device="cuda")] = True
+    h[:, :2], w[:, :2] = 0.0, 0.0
+    h[5, 0], h[40, 0], h[7, 1] = 1e20, 1e20, 1e20     # their logits: -1e40 where a word has -1e20 in the same place
+    w[gone, 0], w[:, 1] = -1e20, -1e20
+    h.requires_grad_(), w.requires_grad_()
+    ids = (~gone).nonzero()[:, 0][torch.randint(0, int((~gone).sum()), (T,), device="cuda")]
+    lp = ops.linear_token_logprobs(h, w, ids)
+    logits = h.detach().double() @ w.detach().double().t()
+    logits = torch.where(logits < -1e38, float("-inf"), logits)
+    want = logits.log_softmax(-1)
+    keep = torch.arange(T, device="cuda") != 7
+    # logits up to about 6 are rounded to bf16 (2^-8 of their size)
+    assert (lp.double() - want[torch.arange(T), ids])[keep].abs().max().item() < 2 ** -8 * 12 and lp[7].isnan()
+    weight = torch.ones(T, device="cuda")
+    weight[7] = 0.0                                    # ignored in the loss: no NaN gets into it or the gradients
+    loss = ops.linear_cross_entropy(h, w, ids, weight)
+    gh, gw = torch.autograd.grad(loss, [h, w])
+    d = (want.exp() - torch.nn.functional.one_hot(ids, V).double()) * keep[:, None]
+    d = torch.where(keep[:, None], d, 0.0)
+    assert abs(loss.item() + want[torch.arange(T), ids][keep].sum().item()) < 1e-3 * loss.item()
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+    assert rel(gh[:, 2:], (d @ w.detach().double())[:, 2:]) < 1.5e-2
+    assert rel(gw[:, 2:], (d.t() @ h.detach().double())[:, 2:]) < 1.5e-2
     assert ext.kernel_status()[0].item() == 0
 
 
