@@ -677,8 +677,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       for (int e = 0; e < 4; ++e) {
         const int c = lane + 32 * e;
         const bool in = i * 128 + c < seq_len;
-        nl[e] = in ? p.lse_scale * p.lse[first + c] : 0.f;
-        dl[e] = in ? (C::kRows ? -p.delta[first + c] : p.delta[first + c]) : 0.f;
+        nl[e] = in ? p.lse[first + c] : 0.f;   // nothing that needs the values before Q is on its way
+        dl[e] = in ? p.delta[first + c] : 0.f;
       }
       if (!__all_sync(0xffffffffu, mbar_wait(q_empty0 + 8 * qs, ((it / C::kQStages) & 1) ^ 1, wc, 31))) break;
       if (leader) {
@@ -692,7 +692,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (it > 0 && !__all_sync(0xffffffffu, mbar_wait(dp_full, (it - 1) & 1, wc, 25))) break;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {  // three bf16 terms hold the 24 bits of each value
-          float rest[2] = {nl[e], dl[e]};
+          float rest[2] = {p.lse_scale * nl[e], -dl[e]};
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             uint32_t h[3];
@@ -710,7 +710,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         // a free Q stage also means that this slot's values have been read: dS was made from them
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          stats[qs * 256 + lane + 32 * e] = nl[e];
+          stats[qs * 256 + lane + 32 * e] = p.lse_scale * nl[e];
           stats[qs * 256 + 128 + lane + 32 * e] = dl[e];
         }
       }
