@@ -479,7 +479,7 @@ __device__ __forceinline__ float row_lse2(const float2* stats, int tiles, long l
   return gm + log2f(red ? block_sum(s, red) : warp_sum(s));
 }
 
-__global__ void __launch_bounds__(kCeThreads)
+__global__ void __launch_bounds__(256)
 ce_from_stats_kernel(bf16* __restrict__ logits, const long long* __restrict__ labels, const float* __restrict__ loss_scale,
                      const float2* __restrict__ stats, const float* __restrict__ label_logits, float* __restrict__ loss,
                      int rows, int vocab, int tiles, long long ignore_index, float inv_temp) {
@@ -778,8 +778,10 @@ cudaError_t launch_ce_from_stats(void* logits, const long long* labels, const fl
                                  cudaStream_t stream, float inv_temp) {
   if (rows == 0) return cudaSuccess;
   if (vocab % 8 != 0) return cudaErrorInvalidValue;
-  // a short row does not fill the threads of a long one (2000 x 4096: 31 us with 1024, 9.6 with 256)
-  launch(ce_from_stats_kernel, rows, vocab <= 16384 ? 256 : kCeThreads, 0, stream, static_cast<bf16*>(logits), labels, loss_scale,
+  // 256 threads a row at every length: more of them wait for one another over the tiles' statistics.  Head product of width 64
+  // and this pass, 4096 rows: 4096 words 49 us (512 threads 63, 1024 92), 32000 247 (262, 304), 128256 941 (944, 982), 151936
+  // 1109 (1122, 1155)
+  launch(ce_from_stats_kernel, rows, 256, 0, stream, static_cast<bf16*>(logits), labels, loss_scale,
       reinterpret_cast<const float2*>(row_stats), label_logits, loss, rows, vocab, tiles, ignore_index, inv_temp);
   return cudaGetLastError();
 }
