@@ -420,8 +420,9 @@ ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ label
       s *= __expf(m - mx);
       m = mx;
     }
+    const float m_sub = m == -INFINITY ? 0.f : m;   // nothing but -inf so far has no weight
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s += __expf(f[i] - m);
+    for (int i = 0; i < 8; ++i) s += __expf(f[i] - m_sub);
   }
   for (int j = nvec * 8 + threadIdx.x; j < vocab; j += blockDim.x) {
     const float f = __bfloat162float(lr[j]) * inv_temp;
@@ -429,7 +430,7 @@ ce_fwd_bwd_kernel(bf16* __restrict__ logits, const long long* __restrict__ label
       s *= __expf(m - f);
       m = f;
     }
-    s += __expf(f - m);
+    s += __expf(f - (m == -INFINITY ? 0.f : m));
   }
   const float gm = block_max(m, red);
   s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);

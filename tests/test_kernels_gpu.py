@@ -1007,6 +1007,24 @@ def test_head_statistics_from_the_product(ext, T, V, H, chunk, temperature):
     assert ext.kernel_status()[0].item() == 0
 
 
+def test_passes_over_logits_of_minus_infinity(ext):
+    """Eight logits of -inf in one thread's hands, at the start of its row or all of it, weigh nothing."""
+    torch.manual_seed(3)
+    T, V = 5, 16648
+    x = torch.randn(T, V, device="cuda").bfloat16()
+    x[0, 256:512], x[1, :8], x[2, 8:], x[3, 8192:8208] = (float("-inf"),) * 4
+    ids = torch.tensor([3, 9, 5, 8300, 7], device="cuda")
+    want = x.double().log_softmax(-1)
+    out, loss, grad = torch.empty(T, device="cuda"), torch.zeros((), device="cuda"), x.clone()
+    ext.token_logprobs(x, ids, out, -100, 1.0)
+    ext.ce_fwd_bwd(grad, ids, None, loss, -100, 1.0)
+    picked = want[torch.arange(T), ids]
+    # fp32 sums of V exponentials, each to a few 2^-22: far below 1e-4; gradients are rounded to bf16 (2^-8 of their size)
+    assert (out.double() - picked).abs().max().item() < 1e-4 and abs(loss.item() + picked.sum().item()) < 1e-3
+    d = want.exp() - torch.nn.functional.one_hot(ids, V)
+    assert ((grad.double() - d).abs() <= 2 ** -8 * d.abs() + 1e-6).all()
+
+
 @pytest.mark.parametrize("T,V", [(256, 1000), (300, 2056)])
 def test_head_statistics_of_infinite_logits(ext, T, V):
     """Logits of -inf beside finite ones, over a whole tile of 256 words and in single places: they have no weight, and nothing
