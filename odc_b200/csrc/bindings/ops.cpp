@@ -671,7 +671,8 @@ void head_chunk(const Tensor& h, const Tensor& w, Tensor& logits, const Tensor& 
                 const Tensor& loss, const Tensor& per_token, int64_t ignore_index, double inv_temp) {
   const int64_t n = h.size(0), V = w.size(0);
   if (!library_gemm() && odc::gemm_pairs_enabled() && h.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
-      labels.scalar_type() == at::kLong && labels.is_contiguous() && h.stride(1) == 1 && w.stride(1) == 1 && w.size(1) == h.size(1)) {
+      labels.scalar_type() == at::kLong && labels.is_contiguous() && h.stride(1) == 1 && w.stride(1) == 1 && w.size(1) == h.size(1) &&
+      odc::logits_stats_pay(static_cast<int>(n), static_cast<int>(V), static_cast<int>(h.size(1)), !per_token.defined(), sm_count())) {
     c10::cuda::CUDAGuard g(h.device());
     odc::bind_device(h.get_device());
     const int tiles = odc::logits_stat_tiles(static_cast<int>(V));
@@ -1008,6 +1009,9 @@ void register_ops(py::module_& m) {
     const odc::GemmPlan p = odc::scatter_plan(n_out, k_in, tokens, ranks, sms);
     return std::make_tuple(p.tiles, p.whole, p.parts);
   }, py::arg("n_out"), py::arg("k_in"), py::arg("tokens"), py::arg("ranks"), py::arg("sms"));
+  m.def("head_plan", [](int rows, int words, int width, bool gradient, int sms) {
+    return odc::logits_stats_pay(rows, words, width, gradient, sms);
+  }, py::arg("rows"), py::arg("words"), py::arg("width"), py::arg("gradient"), py::arg("sms"));  // statistics in the product
   // scratch of a product of which every tile is divided; 0 for one of which some or all are whole
   m.def("gemm_split_bytes", [](int M, int N, int K) {
     const odc::GemmPlan p = odc::gemm_plan(M, N, K, odc::kBF16, sm_count());

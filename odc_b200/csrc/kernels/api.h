@@ -145,6 +145,7 @@ cudaError_t gemm_swiglu_bwd_pair(const void* dy, const void* w, const void* gate
 // launches below take: row_stats [logits_stat_tiles(N), M, 2], label_logits [M].  cudaErrorNotSupported where a pair does not
 // take the product.
 int logits_stat_tiles(int N);
+bool logits_stats_pay(int M, int N, int K, bool store_logits, int sm_count);   // else the passes over plain logits
 cudaError_t gemm_logits_pair(const void* h, const void* w, void* logits, const long long* labels, float* row_stats,
                              float* label_logits, int M, int N, int K, long long ldh, long long ldw, long long ldl, float inv_temp,
                              int* status, int sm_count, cudaStream_t stream);

@@ -965,6 +965,24 @@ cudaError_t gemm_swiglu_bwd_pair(const void* dy, const void* w, const void* gate
   return cudaGetLastError();
 }
 
+// Where the statistics in the epilogue are the better form of a head of M rows, N words and width K.  Against the plain product
+// and the pass over its logits (times of that form over this one, log-probabilities / loss and its gradient):
+//   - They lengthen the last epilogue by 3 us, so there has to be more than one round of tiles, or enough rows to keep the pass
+//     busy for some waves: 256 rows and 4096 words, width 512: 0.81 / 0.77; 300 and 8192, 2048: 0.98 / 0.94; 800 and 4096: 1.07 /
+//     1.00; 300 and 32000, 2048: 1.07 / 1.05; 4096 and 4096: 1.52 / 1.23.
+//   - The product must not be one that is divided: 256 and 1024, width 4096: 0.52 / 0.51; 1200 and 1024: 0.87 / 0.84.
+//   - With the logits to be stored as well an epilogue takes as long as 16 k-blocks of the next tile's products.  Below that width
+//     the passes win where rows are long: 4096 and 128256, width 512: 0.94, 768 0.94, 1024 0.96, 1536 1.15; rows up to 16384 words
+//     gain at any width (1.03 to 1.7 from 2000 rows on).
+bool logits_stats_pay(int M, int N, int K, bool store_logits, int sm_count) {
+  using namespace gemm_pair;
+  if (M < 256 || N < 256 || K < BK || sm_count < 2) return false;
+  const long long tiles = static_cast<long long>((M + 255) / 256) * logits_stat_tiles(N);
+  if (tiles <= sm_count / 2 && M < 5 * sm_count) return false;
+  if (store_logits && K < 1024 && N > 16384) return false;
+  return product_plan(M, N, K, sm_count).splits == 1;
+}
+
 int logits_stat_tiles(int N) { return (N + gemm_pair::BN - 1) / gemm_pair::BN; }
 
 cudaError_t gemm_logits_pair(const void* h, const void* w, void* logits, const long long* labels, float* row_stats,

@@ -51,3 +51,13 @@ def test_weight_gradients_are_divided_only_where_the_link_allows_it(n_out, k_in,
 def test_small_weight_gradients_stay_whole_across_ranks():
     plan = lambda ranks: _ext.load().scatter_plan(512, 512, 765, ranks, SMS)
     assert plan(1)[2] > 1 and plan(8) == (4, 4, 1)
+
+
+def test_statistics_in_the_product_where_they_pay():
+    plan = lambda rows, words, width, gradient: _ext.load().head_plan(rows, words, width, gradient, SMS)
+    for gradient in (False, True):
+        for rows, words, width in ((4096, 128256, 2048), (300, 151936, 1536), (4096, 4096, 512), (2000, 1024, 512), (300, 32000, 2048)):
+            assert plan(rows, words, width, gradient), (rows, words, width)
+        for rows, words, width in ((255, 128256, 2048), (256, 4096, 512), (300, 8192, 2048), (1200, 1024, 4096), (4096, 200, 512)):
+            assert not plan(rows, words, width, gradient), (rows, words, width)
+    assert plan(4096, 128256, 512, False) and not plan(4096, 128256, 512, True)

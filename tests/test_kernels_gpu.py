@@ -963,10 +963,11 @@ def test_rmsnorm_residual_backward_fuses_the_residual_gradient():
     torch.testing.assert_close(x2.grad.float(), xg.grad, rtol=2e-2, atol=3e-2)
 
 
-@pytest.mark.parametrize("T,V,H,chunk", [(256, 264, 64, 4096), (700, 1000, 512, 300), (520, 8200, 256, 512)])
+@pytest.mark.parametrize("T,V,H,chunk", [(256, 264, 64, 4096), (700, 1000, 512, 300), (520, 8200, 256, 512), (900, 264, 64, 4096),
+                                         (1700, 1000, 512, 800), (1000, 8200, 256, 777)])
 @pytest.mark.parametrize("temperature", [1.0, 0.7])
 def test_head_statistics_from_the_product(ext, T, V, H, chunk, temperature):
-    """Softmax statistics of ragged tiles, in chunks (a last one below a tile takes the other path): log-probabilities, loss and
+    """Softmax statistics of ragged tiles, in chunks (short ones take the passes over logits): log-probabilities, loss and
     both gradients; ignored and weightless rows; a NaN row stays one row."""
     from odc_b200 import ops
     torch.manual_seed(T + V)
@@ -982,8 +983,10 @@ def test_head_statistics_from_the_product(ext, T, V, H, chunk, temperature):
     want = torch.where(keep, ((h64 @ w64.t()) / temperature).log_softmax(-1).gather(1, ids.clamp_min(0)[:, None])[:, 0], 0.0)
     wh, ww = torch.autograd.grad(want, [h64, w64], dlogp.double())
     rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
-    # logits are rounded to bf16 (2^-9 of values up to 10): 2e-2 of a log-probability, and of its gradient's weight
-    assert (lp.double() - want).abs().max().item() < 4e-2 / temperature and lp[3].item() == 0.0
+    # logits are rounded to bf16 (at most 2^-8 of each), the label's and those of the row's sum: 2e-2 of a gradient's weight
+    size = (h64 @ w64.t()).detach().abs()
+    bound = 2 ** -8 * (size.gather(1, ids.clamp_min(0)[:, None])[:, 0] + size.amax(1)) / temperature + 1e-4
+    assert ((lp.double() - want).abs() <= bound).all() and lp[3].item() == 0.0
     assert rel(dh, wh) < 1.5e-2 and rel(dw, ww) < 1.5e-2
     weight = torch.rand(T, device="cuda")
     weight[9] = 0.0
@@ -1025,7 +1028,7 @@ def test_passes_over_logits_of_minus_infinity(ext):
     assert ((grad.double() - d).abs() <= 2 ** -8 * d.abs() + 1e-6).all()
 
 
-@pytest.mark.parametrize("T,V", [(256, 1000), (300, 2056)])
+@pytest.mark.parametrize("T,V", [(256, 1000), (800, 1000), (1000, 2056)])
 def test_head_statistics_of_infinite_logits(ext, T, V):
     """Logits of -inf beside finite ones, over a whole tile of 256 words and in single places: they have no weight, and nothing
     else changes.  A row of nothing but -inf has no probabilities, as a softmax in 64 bits has none."""
@@ -1089,12 +1092,12 @@ def test_log_probabilities_alone_hold_no_logits():
     """Forward only, the product leaves row statistics (8 bytes per 256 words) and the logits are never written: no scratch for
     them is held, except for a last chunk below a tile of rows, which takes the passes over logits."""
     from odc_b200 import ops
-    T, V, H, chunk = 1100, 8192, 256, 512          # chunks of 512, 512 and 76 rows
+    T, V, H, chunk = 2124, 8192, 256, 1024         # chunks of 1024, 1024 and 76 rows
     h, w = torch.randn(T, H, device="cuda").bfloat16(), torch.randn(V, H, device="cuda").bfloat16()
     ids = torch.randint(0, V, (T,), device="cuda")
     run = lambda n: ops.linear_token_logprobs(h[:n], w, ids[:n], chunk=chunk)
     with torch.no_grad():
-        for n, limit in ((1024, 1 << 20), (T, (1 << 20) + 76 * V * 2)):
+        for n, limit in ((2048, 1 << 20), (T, (1 << 20) + 76 * V * 2)):
             run(n)
             torch.cuda.synchronize()
             torch.cuda.reset_peak_memory_stats()
