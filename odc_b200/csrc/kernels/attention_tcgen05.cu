@@ -679,6 +679,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
     }
     int head = first_head, i = i_first;
+    auto load_q = [&](int stage, int row) {
+      const uint32_t bar = q_full0 + 8 * stage, dst = base + kQOff + stage * C::kTile;
+      mbar_arrive_expect_tx(bar, C::kTile);
+#pragma unroll
+      for (int s = 0; s < D / 64; ++s) tma_load_2d(dst + s * 16384, &tmap_q, bar, head * D + 64 * s, row);
+    };
+    if (leader) load_q(0, seq_start + i * 128);   // not after the loads of log-sum-exp and delta below
     for (int it = 0; it < total_iters; ++it) {
       const int qs = it % C::kQStages, os = it % C::kDoStages;
       const int row = seq_start + i * 128;
@@ -688,22 +695,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       for (int e = 0; e < 4; ++e) {
         const int c = lane + 32 * e;
         const bool in = i * 128 + c < seq_len;
-        nl[e] = in ? p.lse[first + c] : 0.f;   // nothing that needs the values before Q is on its way
-        dl[e] = in ? p.delta[first + c] : 0.f;
+        nl[e] = in ? p.lse_scale * p.lse[first + c] : 0.f;
+        dl[e] = in ? (C::kRows ? -p.delta[first + c] : p.delta[first + c]) : 0.f;
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(q_empty0 + 8 * qs, ((it / C::kQStages) & 1) ^ 1, wc, 31))) break;
-      if (leader) {
-        const uint32_t bar = q_full0 + 8 * qs, dst = base + kQOff + qs * C::kTile;
-        mbar_arrive_expect_tx(bar, C::kTile);
-#pragma unroll
-        for (int s = 0; s < D / 64; ++s) tma_load_2d(dst + s * 16384, &tmap_q, bar, head * D + 64 * s, row);
+      if (it > 0) {
+        if (!__all_sync(0xffffffffu, mbar_wait(q_empty0 + 8 * qs, ((it / C::kQStages) & 1) ^ 1, wc, 31))) break;
+        if (leader) load_q(qs, row);
       }
       if constexpr (C::kRows) {
         // dP(it-1) has read the rows of the tile before
         if (it > 0 && !__all_sync(0xffffffffu, mbar_wait(dp_full, (it - 1) & 1, wc, 25))) break;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {  // three bf16 terms hold the 24 bits of each value
-          float rest[2] = {p.lse_scale * nl[e], -dl[e]};
+          float rest[2] = {nl[e], dl[e]};
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
             uint32_t h[3];
@@ -721,7 +725,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         // a free Q stage also means that this slot's values have been read: dS was made from them
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          stats[qs * 256 + lane + 32 * e] = p.lse_scale * nl[e];
+          stats[qs * 256 + lane + 32 * e] = nl[e];
           stats[qs * 256 + 128 + lane + 32 * e] = dl[e];
         }
       }
