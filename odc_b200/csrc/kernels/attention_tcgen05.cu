@@ -122,10 +122,10 @@ __device__ __forceinline__ bool locate_tile(const int* cu, int num_seqs, int idx
 //            without work (attn_fwd_pairs) a CTA takes one tile, with P in columns of its own as at D = 64.
 // Bound by the chain around the exponentials (scores out of TMEM, maximum, exponentials, P into TMEM): with none of them
 // computed at all a pass is only 12 (D = 128) to 18 % (D = 64) faster.  Two threads per row halve that chain, a few of the
-// exponentials go to the FMA pipe, and the first half of P V starts before the other half of P is there.  32768 tokens,
-// 40/8 heads, D = 128: 10.6 ms (1036 TFLOP/s) with one thread per row and MMAs issued by lane 0, now 9.8 ms (1120); 4096
-// tokens, 12/2 heads: 79 us, now 69; 27183 tokens, lengths up to 16384, 32/8 heads: 1.19 ms, now 1.11; 16321 tokens, lengths
-// up to 8192, 32/8 heads, D = 64: 519 us, now 513.
+// exponentials go to the FMA pipe, and the first half of P V starts before the other half of P is there.  Against one thread
+// per row and MMAs issued by lane 0: 32768 tokens, 40/8 heads, D = 128 9.65 ms, now 8.92 (1233 TFLOP/s), under the power cap
+// 10.77 and 10.05 (1094); 16 sequences of 1024 357 us, now 327; 40 of 300 297 and 299.  32/8 heads, D = 64: 16 sequences of
+// 1024 180 us, now 164; 40 of 300 125 and 112; one of 32768 5.53 ms and 5.56, under the power cap 5.83 and 5.94.
 template <int D, int Tiles>
 struct FwdCfg {
   static constexpr int kTiles = Tiles;
@@ -139,9 +139,10 @@ struct FwdCfg {
     return kPrivateP ? 128 + D + 32 * half : 128 * t + 64 * half;
   }
   // Of 16 pairs of exponentials, how many the FMA pipe takes instead of the special-function unit (13 instructions a pair).
-  // 4096 tokens, 12/2 heads, D = 128: none 72 us, two 69, four 70, six 74; 8192 tokens, 32/8 heads, D = 64: none 398 us,
-  // three 382, five 403, seven 441 (issue slots).
-  static constexpr int kPolyPairs = (D == 64) ? 3 : 2;
+  // 32768 tokens, 40/8 heads, D = 128: none 8974 us, one 9069, two 8916 (under the power cap 10076, 10184, 10047); 4096 tokens,
+  // 12/2 heads: none 72, two 69, four 70, six 74.  32/8 heads, D = 64, 32768 tokens: none 5756 us, one 5559, two 5646, three
+  // 5639 (under the power cap 6035, 5942, 6042, 6086); 16 sequences of 1024: 167, 164, 165, 166.
+  static constexpr int kPolyPairs = (D == 64) ? 1 : 2;
   static constexpr int kThreads = 64 + 256 * kTiles;
   static constexpr int kQBytes = kBlockQ * D * 2;
   static constexpr int kKBytes = kBlockKV * D * 2;
