@@ -94,13 +94,14 @@ struct Params {
 // kModeLogits: the epilogue leaves the softmax statistics of every row of a tile and the label's logit, so the log-sum-exp
 // needs no pass over the logits, and where no gradient follows they are not written at all.  From the logits as rounded to
 // bf16, as the pass that forms the gradient reads them.  The arithmetic (one exponential per logit) runs under the next tile's
-// products.  Log-probabilities of 6000 tokens, 151936 words, 1536 wide, forward and backward: 9.62 ms, now 8.99; forward only,
+// products, where these are long enough (logits_stats_pay).  Log-probabilities of 6000 tokens, 151936 words, 1536 wide, forward and backward: 9.62 ms, now 8.99; forward only,
 // 16321 tokens, 128256 words: four passes of 0.24 ms and as many writes of the logits less (36.6 -> 35.3 ms with the decoder).
 constexpr int kModePlain = 0, kModeScatter = 1, kModeGather = 2, kModeSwiglu = 3, kModeLogits = 4, kModeSwigluBwd = 5;
 // kModeSwigluBwd (N = F): the product is the gradient of the activations; the epilogue turns it, rounded to bf16, with the
 // projection [M, 2F] (tensor map c) into the projection's gradient (owners.m[0] / [1]: its halves).  A warp of its own brings
-// boxes of gate and up into two buffers, for which the ring gives up a stage.  30000 tokens, 4096 and 14336 wide, forward and
-// backward of a layer: 38.9 ms with the pass, now 36.5; 16321 tokens, 2048 and 8192 wide: 7.25, now 7.13.
+// boxes of gate and up into two buffers, for which the ring gives up a stage.  Forward and backward of a layer, both forms in
+// turn: 16321 tokens, 2048 and 8192 wide: 6.92 ms with the pass, 6.76 without; 30000 tokens, 4096 and 14336 wide, all under the
+// power cap: 34.4 and 34.6, the same within the spread of either.
 template <int kMode> struct Ring {
   static constexpr int kDepth = kMode == kModeSwigluBwd ? 5 : 6;
   static constexpr int kGateUpBytes = kMode == kModeSwigluBwd ? 2 * kStagingBytes : 0;
