@@ -265,6 +265,65 @@ Tensor product(const Tensor& a, const Tensor& b, int lay, const Tensor& bias = {
   return c;
 }
 
+// Products none of which reads what another writes: one launch where the kernel takes them together, else one by one.
+struct Product {
+  Tensor a, b, c;
+  int lay;
+  bool accumulate = false;
+  double scale = 1.0;   // with an arrival (products_into) only
+};
+bool fixed_order_asked() {
+  const char* e = std::getenv("ODC_DETERMINISTIC");
+  return at::globalContext().deterministicAlgorithms() ||
+         (e != nullptr && *e != 0 && std::strcmp(e, "0") != 0 && std::strcmp(e, "false") != 0);
+}
+// arrivals > 0: that many are reported to the counter behind ctr_table (one entry) when the results are in memory
+bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = {}, int arrivals = 0) {
+  const int n = static_cast<int>(products.size());
+  if (n < 1 || n > odc::kMaxGroupProducts || library_gemm() || !odc::gemm_pairs_enabled()) return false;
+  odc::GemmProduct g[odc::kMaxGroupProducts];
+  const bool fixed = fixed_order_asked();
+  for (int i = 0; i < n; ++i) {
+    const auto& [a, b, c, lay, accumulate, scale] = products[i];
+    if (a.dim() != 2 || b.dim() != 2 || c.dim() != 2 || a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16 ||
+        (c.scalar_type() != at::kBFloat16 && c.scalar_type() != at::kFloat) || a.stride(1) != 1 || b.stride(1) != 1 || c.stride(1) != 1)
+      return false;
+    const int64_t K = lay == kTN ? a.size(0) : a.size(1), M = lay == kTN ? a.size(1) : a.size(0), N = lay == kNT ? b.size(0) : b.size(1);
+    if ((lay == kNT ? b.size(1) : b.size(0)) != K || c.size(0) != M || c.size(1) != N) return false;
+    g[i] = odc::GemmProduct{a.data_ptr(), b.data_ptr(), c.data_ptr(), kind_of(c.scalar_type()), static_cast<int>(M), static_cast<int>(N),
+                            static_cast<int>(K), lay, accumulate, fixed, a.stride(0), b.stride(0), c.stride(0), static_cast<float>(scale)};
+  }
+  const Tensor& a = products[0].a;
+  c10::cuda::CUDAGuard guard(a.device());
+  odc::bind_device(a.get_device());
+  Tensor scratch;
+  if (const size_t bytes = odc::gemm_group_scratch(g, n, sm_count()))
+    scratch = at::empty({static_cast<int64_t>(bytes / sizeof(float))}, a.options().dtype(at::kFloat));
+  const cudaError_t e = odc::gemm_group(g, n, scratch.defined() ? scratch.data_ptr<float>() : nullptr,
+                                        ctr_table.defined() ? reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()) : nullptr,
+                                        arrivals, device_status(a.get_device()).data_ptr<int>(), sm_count(), cur_stream());
+  if (e == cudaErrorNotSupported) return false;
+  check(e, "group of products");
+  count();
+  return true;
+}
+void products_into(const std::vector<Product>& products) {
+  if (group_into(products)) return;
+  for (const auto& p : products) product_into(p.a, p.b, p.c, p.lay, {}, p.accumulate);
+}
+Tensor product_out(const Tensor& a, const Tensor& b, int lay, c10::optional<at::ScalarType> dtype = c10::nullopt) {
+  return at::empty({lay == kTN ? a.size(1) : a.size(0), lay == kNT ? b.size(0) : b.size(1)}, dtype ? a.options().dtype(*dtype) : a.options());
+}
+// the input gradient and the weight gradient of y = x w^T, what is wanted of them
+std::tuple<Tensor, Tensor> linear_grads(const Tensor& dy2, const Tensor& x2, const Tensor& w, bool need_dx, bool need_dw) {
+  Tensor dx, dw;
+  std::vector<Product> todo;
+  if (need_dx) todo.push_back({dy2, w, dx = product_out(dy2, w, kNN), kNN});
+  if (need_dw) todo.push_back({dy2, x2, dw = product_out(dy2, x2, kTN, w.scalar_type()), kTN});
+  products_into(todo);
+  return {dx, dw};
+}
+
 std::tuple<Tensor, Tensor> attn_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens, int max_seqlen, bool causal,
                                     double scale) {
   c10::cuda::CUDAGuard g(q.device());
@@ -389,9 +448,9 @@ struct LinearFn : Function<LinearFn> {
     const Tensor &x = saved[0], &w = saved[1], &dy = grads[0];
     const int64_t need = ctx->saved_data["need"].toInt();
     const Tensor dy2 = rows2d(dy).contiguous();
-    Tensor dx, dw, db;
-    if (need & 1) dx = product(dy2, w, kNN).view(x.sizes());
-    if (need & 2) dw = product(dy2, rows2d(x), kTN, {}, {}, w.scalar_type());
+    Tensor db;
+    auto [dx, dw] = linear_grads(dy2, rows2d(x), w, need & 1, need & 2);
+    if (dx.defined()) dx = dx.view(x.sizes());
     if (need & 4) db = column_sum(dy2);
     return {dx, dw, db, (need & 8) ? dy : Tensor(), {}, {}, {}, {}};
   }
@@ -526,9 +585,8 @@ struct LinearSwigluFn : Function<LinearSwigluFn> {
     const int64_t need = ctx->saved_data["need"].toInt();
     const Tensor d = swiglu_bwd(rows2d(grads[0]).contiguous(), saved[2]);
     count();
-    Tensor dx, dw;
-    if (need & 1) dx = product(d, w, kNN).view(x.sizes());
-    if (need & 2) dw = product(d, rows2d(x), kTN, {}, {}, w.scalar_type());
+    auto [dx, dw] = linear_grads(d, rows2d(x), w, need & 1, need & 2);
+    if (dx.defined()) dx = dx.view(x.sizes());
     return {dx, dw, {}, {}};
   }
 };
@@ -579,13 +637,14 @@ struct MlpFn : Function<MlpFn> {
     const Tensor &x = s[0], &w_gate_up = s[1], &w_down = s[2];
     const int64_t need = ctx->saved_data["need"].toInt();
     const Tensor dy2 = rows2d(grads[0]).contiguous();
-    Tensor dx, dgu, dd;
-    if (need & 3) {
-      const Tensor d = swiglu_product_bwd(dy2, w_down, s[3]);
-      if (need & 1) dx = product(d, w_gate_up, kNN).view(x.sizes());
-      if (need & 2) dgu = product(d, rows2d(x), kTN, {}, {}, w_gate_up.scalar_type());
-    }
-    if (need & 4) dd = product(dy2, s[4], kTN, {}, {}, w_down.scalar_type());
+    Tensor d, dx, dgu, dd;
+    if (need & 3) d = swiglu_product_bwd(dy2, w_down, s[3]);
+    std::vector<Product> todo;
+    if (need & 1) todo.push_back({d, w_gate_up, dx = product_out(d, w_gate_up, kNN), kNN});
+    if (need & 2) todo.push_back({d, rows2d(x), dgu = product_out(d, rows2d(x), kTN, w_gate_up.scalar_type()), kTN});
+    if (need & 4) todo.push_back({dy2, s[4], dd = product_out(dy2, s[4], kTN, w_down.scalar_type()), kTN});
+    products_into(todo);
+    if (dx.defined()) dx = dx.view(x.sizes());
     return {dx, dgu, dd, (need & 8) ? grads[0] : Tensor(), {}, {}, {}, {}};
   }
 };
@@ -732,8 +791,10 @@ std::tuple<Tensor, Tensor, Tensor> lm_head_loss(const Tensor& h, const Tensor& w
     Tensor lg = logits.narrow(0, 0, n);
     head_chunk(hs, w, lg, labels.narrow(0, s, n), loss_scale.has_value() ? c10::optional<Tensor>(loss_scale->narrow(0, s, n)) : c10::nullopt,
                loss, {}, ignore_index, 1.0);
-    if (need_dh) product_into(lg, w, dh.narrow(0, s, n), kNN);
-    if (need_dw) product_into(lg, hs, dw, kTN, {}, s > 0);
+    std::vector<Product> todo;
+    if (need_dh) todo.push_back({lg, w, dh.narrow(0, s, n), kNN});
+    if (need_dw) todo.push_back({lg, hs, dw, kTN, s > 0});
+    products_into(todo);
   }
   return {loss, dh, dw};
 }
@@ -800,8 +861,10 @@ struct LinearTokenLogProbsFn : Function<LinearTokenLogProbsFn> {
       const Tensor hs = h.narrow(0, s, n);
       Tensor lg = logits.narrow(0, 0, n);
       head_chunk(hs, w, lg, ids.narrow(0, s, n), scale.narrow(0, s, n), sink, {}, cfg[0], 1.0 / temperature);
-      if (cfg[2]) product_into(lg, w, dh.narrow(0, s, n), kNN);
-      if (cfg[3]) product_into(lg, hs, dw, kTN, {}, s > 0);
+      std::vector<Product> todo;
+      if (cfg[2]) todo.push_back({lg, w, dh.narrow(0, s, n), kNN});
+      if (cfg[3]) todo.push_back({lg, hs, dw, kTN, s > 0});
+      products_into(todo);
     }
     return {dh, dw.defined() ? dw.to(w.scalar_type()) : dw, {}, {}, {}, {}, {}, {}};
   }
@@ -861,7 +924,9 @@ void after_start() {
 }
 
 std::atomic<bool> g_sync_grads{true};   // false: weight gradients are accumulated on the producing rank
-py::object* g_deferred = nullptr;       // Python: (id, dy2, x2) of a gradient that is not pushed straight away
+// Python, by matrix: a gradient (id, dy2, x2) that is not pushed straight away; the local buffer, which has something to push from
+// here on; push it
+py::object *g_deferred = nullptr, *g_local_buffer = nullptr, *g_push_local = nullptr;
 
 // dy2^T x2 into the owners' accumulators, or, where pushes are off, into the local buffer
 void push_weight_grad(ShardedMatrix* m, const Tensor& dy2, const Tensor& x2) {
@@ -875,6 +940,44 @@ void push_weight_grad(ShardedMatrix* m, const Tensor& dy2, const Tensor& x2) {
     gemm_wgrad_scatter(dy2, x2, m->acc_table, m->ctr_table, 0, m->rows_per_rank, m->grad_scale);
   count();
   m->dispatched->n.fetch_add(1);
+}
+
+// What one backward forms from dy2: dx = dy2 w, and the gradients dy^T x of one or two matrices.  With one rank that is one launch:
+// the weight gradients are added to the accumulators, or to the local buffers where pushes are off, so that dx is summed in the
+// same order either way.
+struct WeightGrad {
+  ShardedMatrix* m;
+  Tensor dy2, x2;
+};
+Tensor sharded_grads(const Tensor& dy2, const ShardedMatrix* m, const std::vector<WeightGrad>& weights) {
+  const Tensor dx = product_out(dy2, m->whole(), kNN);
+  const bool pushes = g_sync_grads;
+  std::vector<Product> todo{{dy2, m->whole(), dx, kNN}};
+  for (const auto& w : weights) {
+    if (w.m->world != 1 || w.m->ctr_table.data_ptr() != m->ctr_table.data_ptr()) break;
+    Tensor to;
+    if (pushes) {
+      to = at::from_blob(reinterpret_cast<void*>(w.m->acc_addrs[0]), {w.m->out_features, w.m->shard.size(1)}, w.m->shard.options().dtype(at::kFloat));
+    } else {
+      py::gil_scoped_acquire gil;
+      to = (*g_local_buffer)(w.m->id).cast<Tensor>().narrow(0, 0, w.m->out_features);
+    }
+    todo.push_back({w.dy2, w.x2, to, kTN, true, pushes ? w.m->grad_scale : 1.0});
+  }
+  if (todo.size() == weights.size() + 1 && group_into(todo, m->ctr_table, pushes ? static_cast<int>(weights.size()) : 0)) {
+    for (const auto& w : weights) {
+      if (!pushes) continue;
+      w.m->dispatched->n.fetch_add(1);
+      if (w.m->local_pending) {   // what earlier microbatches accumulated locally follows
+        py::gil_scoped_acquire gil;
+        (*g_push_local)(w.m->id);
+      }
+    }
+    return dx;
+  }
+  product_into(dy2, m->whole(), dx, kNN);
+  for (const auto& w : weights) push_weight_grad(w.m, w.dy2, w.x2);
+  return dx;
 }
 
 // Forward is the plain product for one rank, else the product that pulls the owners' rows inside the kernel; the weight
@@ -909,10 +1012,10 @@ struct ShardedLinearFn : Function<ShardedLinearFn> {
     const int64_t need = ctx->saved_data["need"].toInt();
     const Tensor dy2 = rows2d(grads[0]).contiguous(), x2 = rows2d(x).contiguous();
     Tensor dx, db;
-    if (need & 1) {
-      if (m->world == 1) {
-        dx = product(dy2, m->whole(), kNN);
-      } else if (saved[1].defined()) {
+    if ((need & 1) && m->world == 1) {
+      dx = sharded_grads(dy2, m, {{m, dy2, x2}}).view(x.sizes());
+    } else if (need & 1) {
+      if (saved[1].defined()) {
         dx = product(dy2, saved[1], kNN);
       } else {
         auto w_full = at::empty({m->out_features, m->shard.size(1)}, m->shard.options());
@@ -921,7 +1024,7 @@ struct ShardedLinearFn : Function<ShardedLinearFn> {
       }
       dx = dx.view(x.sizes());
     }
-    push_weight_grad(m, dy2, x2);
+    if (!(need & 1) || m->world != 1) push_weight_grad(m, dy2, x2);
     auto sink = ctx->saved_data.find("sink");
     if (sink != ctx->saved_data.end()) {
       const Tensor s = sink->second.toTensor();
@@ -965,9 +1068,7 @@ struct ShardedMlpFn : Function<ShardedMlpFn> {
     Tensor dx;
     if (need & 1) {   // as layers one behind the other: without it only the last has anything to do
       const Tensor d = swiglu_product_bwd(dy2, down->whole(), s[1]);
-      push_weight_grad(down, dy2, s[2]);
-      dx = product(d, gu->whole(), kNN).view(x.sizes());
-      push_weight_grad(gu, d, x2);
+      dx = sharded_grads(d, gu, {{gu, d, x2}, {down, dy2, s[2]}}).view(x.sizes());
     } else {
       push_weight_grad(down, dy2, s[2]);
     }
@@ -1005,6 +1106,26 @@ void register_ops(py::module_& m) {
     const odc::GemmPlan p = odc::gemm_plan(M, N, K, odc::kBF16, sms);
     return std::make_tuple(p.tiles, p.whole, p.parts, p.scratch_bytes);
   }, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("sms"));  // (tiles, whole ones, parts of each other, scratch) in bf16
+  m.def("gemm_group", [](std::vector<std::tuple<Tensor, Tensor, Tensor, std::string, bool, double>> products) {
+    std::vector<Product> todo;
+    for (auto& [a, b, c, layout, accumulate, scale] : products) {
+      int lay = 0;
+      while (lay < 3 && layout != kLayoutNames[lay]) ++lay;
+      TORCH_CHECK(lay < 3, "gemm_group: unknown layout ", layout);
+      todo.push_back({a, b, c, lay, accumulate, scale});
+    }
+    return group_into(todo);
+  });  // (a, b, c, layout, accumulate, scale) each; False: not taken as a group, nothing done
+  m.def("gemm_group_plan", [](std::vector<std::tuple<int, int, int, bool, bool>> products, int sms) {
+    odc::GemmProduct g[odc::kMaxGroupProducts] = {};
+    int n = 0;
+    for (auto& [M, N, K, f32, accumulate] : products) {
+      TORCH_CHECK(n < odc::kMaxGroupProducts, "gemm_group_plan: too many products");
+      g[n].M = M; g[n].N = N; g[n].K = K; g[n].c_kind = f32 ? odc::kF32 : odc::kBF16; g[n].accumulate = accumulate; g[n++].scale = 1.f;
+    }
+    const auto plan = odc::gemm_group_plan(g, n, sms);
+    return std::vector<int>(plan.parts, plan.parts + n);
+  }, py::arg("products"), py::arg("sms"));  // parts of every tile of each (M, N, K, fp32, accumulate)
   m.def("scatter_plan", [](int n_out, int k_in, int tokens, int ranks, int sms) {
     const odc::GemmPlan p = odc::scatter_plan(n_out, k_in, tokens, ranks, sms);
     return std::make_tuple(p.tiles, p.whole, p.parts);
@@ -1045,9 +1166,15 @@ void register_ops(py::module_& m) {
   m.def("mark_start", &mark_start);
   m.def("after_start", &after_start);
   m.def("set_sync_grads", [](bool on) { g_sync_grads = on; });
-  m.def("set_deferred_weight_grad", [](py::object fn) {
-    if (g_deferred == nullptr) g_deferred = new py::object();  // never destroyed: backward threads may outlive the module
-    *g_deferred = fn;
+  m.def("set_deferred_weight_grad", [](py::object deferred, py::object local_buffer, py::object push_local) {
+    if (g_deferred == nullptr) {   // never destroyed: backward threads may outlive the module
+      g_deferred = new py::object();
+      g_local_buffer = new py::object();
+      g_push_local = new py::object();
+    }
+    *g_deferred = deferred;
+    *g_local_buffer = local_buffer;
+    *g_push_local = push_local;
   });
   // differentiable forms
   m.def("sharded_linear", &sharded_linear, py::arg("x"), py::arg("bias"), py::arg("residual"), py::arg("matrix"),

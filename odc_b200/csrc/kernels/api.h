@@ -131,6 +131,26 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
                            int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0,
                            float* split_ws = nullptr);
 
+// Up to three products of one layout each, none of which reads what another writes, as one launch on CTA pairs.  C is bf16, or fp32
+// (then times scale, and added to C if accumulate).  ctr_ptrs: device table whose first entry is an arrival counter that receives
+// `arrivals` once everything is in memory (0: none).  scratch: gemm_group_scratch() bytes.  cudaErrorNotSupported: one by one.
+constexpr int kMaxGroupProducts = 3;
+struct GemmProduct {
+  const void *a, *b;
+  void* c;
+  int c_kind, M, N, K, layout;
+  bool accumulate, fixed_order;   // fixed_order: the sum of an accumulating product is formed in one order
+  long long lda, ldb, ldc;
+  float scale;
+};
+struct GemmGroupPlan {
+  int parts[kMaxGroupProducts];   // of every tile; 0: not taken as a group
+};
+GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count);
+size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count);
+cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long long* ctr_ptrs, int arrivals, int* status, int sm_count,
+                       cudaStream_t stream);
+
 // act[M, F] = silu(x Wg^T) * (x Wu^T), w = [Wg; Wu]; gate_up [M, 2F] optional.  cudaErrorNotSupported: use the plain product.
 cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* act, int M, int F, int K, long long ldx,
                              long long ldw, int* status, int sm_count, cudaStream_t stream);

@@ -42,10 +42,11 @@ constexpr int kATile = BMH * BK * 2;                     // 16 KiB
 constexpr int kBTile = BNH * BK * 2;                     // 16 KiB
 constexpr int kStageBytes = kATile + kBTile;             // 32 KiB per CTA
 constexpr int kStagingBytes = 128 * 128;
-constexpr int kSmemBytes = kStages * kStageBytes + 2 * kStagingBytes + 1024 + 256;
+constexpr int kSmemBytes = kStages * kStageBytes + 2 * kStagingBytes + 1024 + 512;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint64_t kWaitBudgetNs = 4000000000ull;
 constexpr int kThreads = 192;
+constexpr int kMaxGroup = kMaxGroupProducts;
 
 struct Params {
   const __nv_bfloat16* bias;
@@ -96,7 +97,7 @@ struct Params {
 // bf16, as the pass that forms the gradient reads them.  The arithmetic (one exponential per logit) runs under the next tile's
 // products, where these are long enough (logits_stats_pay).  Log-probabilities of 6000 tokens, 151936 words, 1536 wide, forward and backward: 9.62 ms, now 8.99; forward only,
 // 16321 tokens, 128256 words: four passes of 0.24 ms and as many writes of the logits less (36.6 -> 35.3 ms with the decoder).
-constexpr int kModePlain = 0, kModeScatter = 1, kModeGather = 2, kModeSwiglu = 3, kModeLogits = 4, kModeSwigluBwd = 5;
+constexpr int kModePlain = 0, kModeScatter = 1, kModeGather = 2, kModeSwiglu = 3, kModeLogits = 4, kModeSwigluBwd = 5, kModeGroup = 6;
 // kModeSwigluBwd (N = F): the product is the gradient of the activations; the epilogue turns it, rounded to bf16, with the
 // projection [M, 2F] (tensor map c) into the projection's gradient (owners.m[0] / [1]: its halves).  A warp of its own brings
 // boxes of gate and up into two buffers, for which the ring gives up a stage.  Forward and backward of a layer, both forms in
@@ -118,20 +119,55 @@ struct OwnerMaps {   // one fp32 tensor map per owner's accumulator region (kMod
   CUtensorMap m[kMaxOwners];
 };
 
+// kModeGroup: up to three products that do not depend on one another (the input and weight gradients of a layer) in one launch.
+// Apart, each fills the machine by itself or not at all: 1000 tokens, 1536 and 8960 wide, are 24, 420 and 210 tiles of 280, 16
+// and 16 k-blocks on 74 pairs.  The items of the longest product come first and a pair takes the next one from a counter, so the
+// short ones fill what the long ones leave.  One by one / together, us: input and weight gradient of 1000 x 1536 x 2048 26.2 / 17.0,
+// of 1000 x 1536 x 1536 23.9 / 14.4, of 2000 x 512 x 512 (fp32 sum) 24.1 / 9.8; the three of an MLP over 2000 tokens, 512 and 1536
+// wide, 48.9 / 21.7, 300 tokens, 2048 and 8192 wide, 130 / 110, 1000 tokens, 1536 and 8960 wide, 112 / 109.  One product by itself
+// costs half a microsecond more than in kModePlain, and 0.5 us an item where items are short.
+struct GroupProblem {
+  int M, N, K, tiles_m, tiles_n;
+  int a_mn, b_mn;
+  int out;                  // 0: bf16, 1: fp32, 2: added to fp32
+  float scale;              // of an fp32 result
+  int first;                // its first item
+  int splits, kb_split;     // work items per tile, k-blocks of each
+  int first_split_tile, first_part;   // bf16 with splits > 1: of its first tile, among the divided tiles and parts of the launch
+};
+struct Group {
+  CUtensorMap a[kMaxGroup], b[kMaxGroup], c[kMaxGroup];
+  GroupProblem prob[kMaxGroup];
+  int count, items;
+  // bf16 tiles in parts: each part is left in fp32 scratch, and the CTA that finds its part to be the last of the tile adds them
+  // up in order.  arrived: parts that are there, per divided tile and CTA of a pair; zero before and after the launch.
+  float4* parts;
+  unsigned int* arrived;
+  unsigned int* next;       // items handed out so far beyond the first of every pair; zero before and after the launch
+  int arrivals;             // contributions to report to ctr_ptrs[0] when all is added
+};
+template <int kMode> struct Extra { using type = OwnerMaps; };
+template <> struct Extra<kModeGroup> { using type = Group; };
+constexpr uint32_t kItemSlots = 16;   // see the item loop
+
 // Tile order: groups of kGroupM tile rows are walked column by column (rows fastest inside a group), so the pairs
 // that run at the same time share a few A row panels and a few B column panels and both stay in L2 however large
 // the whole operands are.
 constexpr int kGroupM = 16;
-__device__ __forceinline__ void tile_coords(int tile, const Params& p, int* tm, int* tn) {
+template <typename P>
+__device__ __forceinline__ void tile_coords(int tile, const P& p, int rot_m, int rot_n, int* tm, int* tn) {
   const int per_group = kGroupM * p.tiles_n;
   const int group = tile / per_group;
   const int first_m = group * kGroupM;
   const int gsize = min(p.tiles_m - first_m, kGroupM);
   const int in_group = tile - group * per_group;
-  int m = first_m + in_group % gsize + p.rot_m;
-  int n = in_group / gsize + p.rot_n;
+  int m = first_m + in_group % gsize + rot_m;
+  int n = in_group / gsize + rot_n;
   *tm = m >= p.tiles_m ? m - p.tiles_m : m;
   *tn = n >= p.tiles_n ? n - p.tiles_n : n;
+}
+__device__ __forceinline__ void tile_coords(int tile, const Params& p, int* tm, int* tn) {
+  tile_coords(tile, p, p.rot_m, p.rot_n, tm, tn);
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -145,7 +181,7 @@ __device__ __forceinline__ float hi(uint32_t u) { return __uint_as_float(u & 0xf
 template <int kMode>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Roles<kMode>::kThreadsTotal, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                      const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ OwnerMaps owners,
+                      const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ typename Extra<kMode>::type owners,
                       const Params p) {
   constexpr int kStages = Ring<kMode>::kDepth;
   extern __shared__ uint8_t smem_raw[];
@@ -163,21 +199,49 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const uint32_t sfree0 = sready0 + 16;                     // [2]
   const uint32_t lready0 = sfree0 + 16;                     // [8]        a box of the last tile is staged in the ring
   const uint32_t gfull = lready0 + 64, gempty = gfull + 8;  // boxes of gate and up
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 18);
+  const uint32_t islot0 = gempty + 8;                       // [kItemSlots] per CTA: an item is written down
+  const uint32_t pready = islot0 + 8 * kItemSlots, pcounted = pready + 8;   // a part is in memory / has been counted
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 18 + kItemSlots + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* part_last = abort_flag + 1;
+  volatile int* item_slots = part_last + 1;                 // [kItemSlots]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();                   // 0: leader
   const WaitCtx wc{abort_flag, p.status, kWaitBudgetNs};
 
+  constexpr bool kDivides = kMode == kModePlain || kMode == kModeScatter;
+  const int num_tiles = p.tiles_m * p.tiles_n;
+  int num_items = kDivides ? p.whole + (num_tiles - p.whole) * p.splits : num_tiles;   // the parts of a tile are adjacent
+  if constexpr (kMode == kModeGroup) num_items = owners.items;
+  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  // kModeGroup, leader's producer: every pair asks until it is told that there is nothing left, `items` questions in all, and the
+  // last one clears the counter.  `taken` is apart from the question: looking at the answer waits for it.
+  [[maybe_unused]] auto take = [&]() -> int {
+    if constexpr (kMode == kModeGroup)
+      if (num_items > num_pairs && lane == 0) return num_pairs + static_cast<int>(atomicAdd(owners.next, 1u));
+    return num_items;
+  };
+  [[maybe_unused]] auto taken = [&](int i) {
+    if constexpr (kMode == kModeGroup)
+      if (num_items > num_pairs && lane == 0 && i == num_pairs + num_items - 1) *owners.next = 0;
+  };
+
   if (threadIdx.x == 0) {
-    prefetch_tmap(&tmap_a);   // the descriptors are on their way while the barriers are set up
-    prefetch_tmap(&tmap_b);
-    prefetch_tmap(&tmap_c);
+    if constexpr (kMode != kModeGroup) {
+      prefetch_tmap(&tmap_a);   // the descriptors are on their way while the barriers are set up
+      prefetch_tmap(&tmap_b);
+      prefetch_tmap(&tmap_c);
+    }
     for (int b = 0; b < 8; ++b) mbar_init(lready0 + 8 * b, 4);
     mbar_init(gfull, 1);
     mbar_init(gempty, 4);
+    if constexpr (kMode == kModeGroup) {
+      for (uint32_t s = 0; s < kItemSlots; ++s) mbar_init(islot0 + 8 * s, 1);
+      mbar_init(pready, 4);
+      mbar_init(pcounted, 1);
+    }
     for (int s = 0; s < kStages; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, 1);
@@ -191,9 +255,20 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     *abort_flag = 0;
     fence_barrier_init();
   }
+  if constexpr (kMode == kModeGroup) {
+    if (warp == 2 && lane < owners.count) {
+      prefetch_tmap(&owners.a[lane]);
+      prefetch_tmap(&owners.b[lane]);
+      prefetch_tmap(&owners.c[lane]);
+    }
+  }
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
     tmem_relinquish_pair();
+  }
+  [[maybe_unused]] int ahead = 0;   // kModeGroup: what the leader's producer (its lane 0) has asked for beyond the next item
+  if constexpr (kMode == kModeGroup) {
+    if (warp == 0 && cta == 0) ahead = take();
   }
   tc_fence_before();
   __syncthreads();
@@ -201,9 +276,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  constexpr bool kDivides = kMode == kModePlain || kMode == kModeScatter;
-  const int num_tiles = p.tiles_m * p.tiles_n;
-  const int num_items = kDivides ? p.whole + (num_tiles - p.whole) * p.splits : num_tiles;   // the parts of a tile are adjacent
   const int all_k_blocks = (p.K + BK - 1) / BK;
   auto is_part = [&](int item) { return kDivides && item >= p.whole; };
   auto tile_of = [&](int item) { return is_part(item) ? p.whole + (item - p.whole) / p.splits : item; };
@@ -215,9 +287,149 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       *kb1 = min(all_k_blocks, *kb0 + p.kb_split);
     }
   };
-  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  // Work items.  kModeGroup: the leader's producer takes them from a counter and writes the next one down for the other roles of
+  // both CTAs before it loads the current one.  A slot is written again kItemSlots items later.  By then all have read it: once the
+  // loads of an item have been issued, all but kStages (6) of the k-blocks so far have been multiplied, so at most 6 items are
+  // still to come for the multiplying thread, and at most two more (the accumulators) for the epilogues.
+  uint32_t item_seq = 0;
+  [[maybe_unused]] auto written_item = [&]() -> int {
+    if (num_items <= num_pairs) return num_items;   // one each, nothing is written down
+    const uint32_t slot = item_seq % kItemSlots, ph = (item_seq / kItemSlots) & 1;
+    ++item_seq;
+    const int item = mbar_wait_cluster(islot0 + 8 * slot, ph, wc, 22) ? item_slots[slot] : num_items;
+    return __shfl_sync(0xffffffffu, item, 0);   // the same in all lanes, also for the compiler
+  };
+  auto following = [&](int item) -> int {
+    if constexpr (kMode == kModeGroup) return written_item();
+    return item + num_pairs;
+  };
+  // where an item lies; group modes only
+  struct Place { int pi, tm, tn, kb0, kb1, part; };
+  [[maybe_unused]] auto place_of = [&](int item) -> Place {
+    Place w{};
+    if constexpr (kMode == kModeGroup) {
+      while (w.pi + 1 < owners.count && item >= owners.prob[w.pi + 1].first) ++w.pi;
+      const GroupProblem& q = owners.prob[w.pi];
+      const int local = item - q.first, tile = q.splits > 1 ? local / q.splits : local;
+      w.part = local - tile * q.splits;
+      tile_coords(tile, q, 0, 0, &w.tm, &w.tn);
+      w.kb0 = w.part * q.kb_split;
+      w.kb1 = min((q.K + BK - 1) / BK, w.kb0 + q.kb_split);
+    }
+    return w;
+  };
 
-  if (warp == 0) {
+  if (kMode == kModeGroup && warp == 0) {
+    // ------------------------------------------------------------------ TMA producer of a group (both CTAs)
+    // The whole warp walks the items, so that what depends on them stays in uniform registers, and one thread issues.
+    if constexpr (kMode == kModeGroup) {
+      uint32_t it = 0;
+      int item = pair, next = num_items;
+      Place w = place_of(item), w_next{};
+      for (; item < num_items; item = next, w = w_next) {
+        if (cta == 0 && num_items > num_pairs) {   // the next item is written down and the one after it asked for before this one is loaded
+          taken(ahead);
+          next = __shfl_sync(0xffffffffu, ahead, 0);
+          const uint32_t slot = item_seq++ % kItemSlots;
+          if (lane == 0) {
+            item_slots[slot] = next;
+            st_shared_cluster(mapa_shared(smem_u32(const_cast<int*>(item_slots + slot)), 1), next);
+            mbar_arrive(islot0 + 8 * slot);
+            mbar_arrive_cluster(mapa_shared(islot0 + 8 * slot, 1));
+          }
+          if (next < num_items) ahead = take();
+        }
+        const GroupProblem& q = owners.prob[w.pi];
+        const CUtensorMap *map_a = &owners.a[w.pi], *map_b = &owners.b[w.pi];
+        const int a_mn = q.a_mn, b_mn = q.b_mn;
+        const int m0 = w.tm * 256 + static_cast<int>(cta) * BMH, n0 = w.tn * BN + static_cast<int>(cta) * BNH;
+        bool ok = true;
+        auto load = [&](int kb0, int kb1) {
+          uint32_t step = it;
+          for (int kb = kb0; kb < kb1; ++kb, ++step) {
+            const int s = step % kStages;
+            const uint32_t ph = (step / kStages) & 1;
+            if (!(ok = mbar_wait(empty0 + 8 * s, ph ^ 1, wc, 11))) break;
+            const uint32_t sa = base + s * kStageBytes;
+            const uint32_t sb = sa + kATile;
+            if (cta == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * kStageBytes);
+            const uint32_t bar = mapa_shared(full0 + 8 * s, 0);
+            const int k0 = kb * BK;
+            if (!a_mn) {
+              tma_load_2d_pair(sa, map_a, bar, k0, m0);
+            } else {
+#pragma unroll
+              for (int i = 0; i < BMH / 64; ++i) tma_load_2d_pair(sa + i * 8192, map_a, bar, m0 + 64 * i, k0);
+            }
+            if (!b_mn) {
+              tma_load_2d_pair(sb, map_b, bar, k0, n0);
+            } else {
+#pragma unroll
+              for (int i = 0; i < BNH / 64; ++i) tma_load_2d_pair(sb + i * 8192, map_b, bar, n0 + 64 * i, k0);
+            }
+          }
+        };
+        const int head = min(w.kb1, w.kb0 + kStages);
+        if (elect_one()) load(w.kb0, head);
+        it += head - w.kb0;
+        __syncwarp();
+        // the rest of the item is loaded as the ring empties: time to find the place of the next one
+        if (cta != 0) next = written_item();
+        if (next < num_items) w_next = place_of(next);
+        if (elect_one() && ok) load(head, w.kb1);
+        it += w.kb1 - head;
+        if (!__all_sync(0xffffffffu, ok)) break;
+      }
+      if (cta == 0 && lane == 0 && item < num_items) {   // given up: the counter is left as the next launch expects it
+        for (; ahead < num_items; taken(ahead)) ahead = take();
+      }
+    }
+  } else if (kMode == kModeGroup && warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer of a group (leader only)
+    if constexpr (kMode == kModeGroup) {
+      if (cta == 0) {
+        uint32_t it = 0, local_tile = 0;
+        int item = pair, next;
+        Place w = place_of(item), w_next{};
+        for (; item < num_items; item = next, w = w_next, ++local_tile) {
+          next = written_item();   // ahead of the products: they are issued without a pause between two items
+          if (next < num_items) w_next = place_of(next);
+          const GroupProblem& q = owners.prob[w.pi];
+          const uint32_t acc = local_tile & 1, acc_ph = (local_tile >> 1) & 1;
+          const uint32_t idesc = make_idesc_bf16(256, 256, q.a_mn != 0, q.b_mn != 0);
+          const uint32_t a_lbo = q.a_mn ? 8192u : 16u, b_lbo = q.b_mn ? 8192u : 16u;
+          const uint64_t a_kstep = q.a_mn ? 128 : 2, b_kstep = q.b_mn ? 128 : 2;
+          const uint32_t d_tmem = tmem_base + acc * BN;
+          bool ok = true;
+          if (elect_one()) {
+            ok = mbar_wait(tempty0 + 8 * acc, acc_ph ^ 1, wc, 12);
+            tc_fence_after();
+            uint32_t step = it;
+            for (int kb = w.kb0; kb < w.kb1 && ok; ++kb, ++step) {
+              const int s = step % kStages;
+              const uint32_t ph = (step / kStages) & 1;
+              if (!(ok = mbar_wait(full0 + 8 * s, ph, wc, 13))) break;
+              tc_fence_after();
+              const uint32_t sa = base + s * kStageBytes;
+              const uint32_t sb = sa + kATile;
+              const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
+#pragma unroll
+              for (int j = 0; j < BK / 16; ++j)
+                umma_f16_pair(d_tmem, da + j * a_kstep, db + j * b_kstep, idesc, (kb > w.kb0 || j > 0) ? 1u : 0u);
+              umma_commit_pair(mapa_shared(empty0 + 8 * s, 0));
+              umma_commit_pair(mapa_shared(empty0 + 8 * s, 1));
+            }
+            if (ok) {
+              umma_commit_pair(mapa_shared(tfull0 + 8 * acc, 0));
+              umma_commit_pair(mapa_shared(tfull0 + 8 * acc, 1));
+            }
+          }
+          if (!__all_sync(0xffffffffu, ok)) break;
+          it += w.kb1 - w.kb0;
+        }
+      }
+    }
+  } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     if (elect_one()) {
       // gather mode: wait (bounded) until every chunk of 256-row group `g` of the gathered matrix is in local memory
@@ -411,13 +623,21 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     [[maybe_unused]] uint32_t gu_ctr = 0;
     bool ok = true;
     const uint32_t tempty_leader0 = mapa_shared(tempty0, 0);
-    for (int item = pair; item < num_items && ok; item += num_pairs, ++local_tile) {
+    [[maybe_unused]] uint32_t part_ctr = 0;
+    for (int item = pair, next_item; item < num_items && ok; item = next_item, ++local_tile) {
       int tm, tn;
-      tile_coords(tile_of(item), p, &tm, &tn);
+      [[maybe_unused]] Place place{};
+      if constexpr (kMode == kModeGroup) {
+        place = place_of(item);
+        tm = place.tm; tn = place.tn;
+      } else {
+        tile_coords(tile_of(item), p, &tm, &tn);
+      }
       const bool part = kMode == kModePlain && is_part(item), f32 = part || p.c_is_f32;
+      next_item = following(item);   // kModeGroup: written down when the loads of this one were issued
       // The ring is idle under the last epilogue of the CTA: every box gets a place of its own there and none waits for the
       // one before it to be read.
-      const bool last = item + num_pairs >= num_items;
+      const bool last = next_item >= num_items;
       const int m0 = tm * 256 + static_cast<int>(cta) * BMH;
       const int n0 = tn * BN;
       const uint32_t acc = local_tile & 1;
@@ -426,11 +646,15 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       tc_fence_after();
       const int my_row = quad * 32 + lane;
       const int row = m0 + my_row;
-      const bool row_ok = row < p.M;
+      [[maybe_unused]] const bool row_ok = row < p.M;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
-      if constexpr (kMode == kModeSwiglu || kMode == kModeLogits || kMode == kModeSwigluBwd) {
-        // one staged box of 64 bf16 columns: 32 packed registers per row
-        auto emit = [&](const uint32_t* v32, const CUtensorMap* map, int col0) -> bool {
+      if constexpr (kMode == kModeSwiglu || kMode == kModeLogits || kMode == kModeSwigluBwd || kMode == kModeGroup) {
+        // one staged box of 64 bf16 columns, or 32 of fp32: 32 registers per row
+        auto emit = [&](const uint32_t* v32, const CUtensorMap* map, int col0, bool add = false) -> bool {
+          auto send = [&](uint32_t src) {
+            if (kMode == kModeGroup && add) tma_reduce_add_2d(map, src, col0, m0);
+            else tma_store_2d(map, src, col0, m0);
+          };
           const int buf = static_cast<int>(box_ctr & 1u);
           const uint32_t use = box_ctr >> 1;
           if (!last && use >= 1 && !mbar_wait(sfree0 + 8 * buf, (use - 1) & 1, wc, 16)) return false;
@@ -444,13 +668,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           if (last) {
             if (lane == 0) mbar_arrive(lready0 + 8 * last_boxes);
             if (warp == 2 && elect_one() && mbar_wait(lready0 + 8 * last_boxes, 0, wc, 18))
-              tma_store_2d(map, base + last_boxes * kStagingBytes, col0, m0);
+              send(base + last_boxes * kStagingBytes);
             ++last_boxes;
             return true;
           }
           if (lane == 0) mbar_arrive(sready0 + 8 * buf);
           if (warp == 2 && elect_one() && mbar_wait(sready0 + 8 * buf, use & 1, wc, 17)) {
-            tma_store_2d(map, staging_u32 + buf * kStagingBytes, col0, m0);
+            send(staging_u32 + buf * kStagingBytes);
             bulk_commit_group();
             if (box_ctr >= 1) {
               bulk_wait_group_read1();
@@ -460,6 +684,96 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           ++box_ctr;
           return true;
         };
+        if constexpr (kMode == kModeGroup) {
+          const GroupProblem& q = owners.prob[place.pi];
+          const CUtensorMap* map = &owners.c[place.pi];
+          const int cols = m0 >= q.M ? 0 : min(BN, q.N - n0);
+          if (q.out != 0) {
+            const float scale = q.scale;
+            const bool add = q.out == 2;
+#pragma unroll 1
+            for (int col = 0; col < cols; col += 32) {
+              uint32_t r[32];
+              tmem_ld_32x32(t_row + col, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * scale);
+              if (!(ok = emit(r, map, n0 + col, add))) break;
+            }
+          } else {
+            // A part: 16 bytes of 128 rows next to one another, so that a warp writes and reads whole lines.
+            const float4* others = nullptr;
+            bool mine = true;
+            if (q.splits > 1) {
+              const int tile = q.first_split_tile + (item - q.first) / q.splits;
+              // parts of the tile, this CTA's half of each
+              float4* at = owners.parts + ((q.first_part + static_cast<long long>(item - q.first - place.part)) * 2 + cta) * (64 * 128) + my_row;
+              float4* own = at + static_cast<long long>(place.part) * (2 * 64 * 128);
+#pragma unroll 1
+              for (int col = 0; col < cols; col += 32) {
+                uint32_t r[32];
+                tmem_ld_32x32(t_row + col, r);
+                tmem_ld_wait();
+#pragma unroll
+                for (int v = 0; v < 8; ++v)
+                  __stcg(own + (col / 4 + v) * 128, make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
+                                                                __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3])));
+              }
+              __threadfence();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(pready);
+              if (warp == 2 && lane == 0 && mbar_wait(pready, part_ctr & 1, wc, 23)) {
+                __threadfence();
+                unsigned int* ctr = owners.arrived + 2 * tile + cta;
+                const bool all = atomicInc(ctr, q.splits - 1) == static_cast<unsigned int>(q.splits) - 1;   // and back to zero
+                __threadfence();
+                *part_last = all;
+                mbar_arrive(pcounted);
+              }
+              __syncwarp();
+              if (!(ok = mbar_wait(pcounted, part_ctr & 1, wc, 24))) break;
+              ++part_ctr;
+              mine = *part_last != 0;
+              others = at;
+            }
+            if (mine) {
+#pragma unroll 1
+              for (int col = 0; col < cols; col += 64) {
+                uint32_t r[64], v[32];
+                tmem_ld_32x32(t_row + col, r);
+                tmem_ld_32x32(t_row + col + 32, r + 32);
+                tmem_ld_wait();
+                if (others != nullptr) {
+                  // in the order of the parts; this one's from the accumulator
+                  float f[64];
+#pragma unroll
+                  for (int i = 0; i < 64; ++i) f[i] = 0.f;
+#pragma unroll 1
+                  for (int s = 0; s < q.splits; ++s) {
+                    if (s == place.part) {
+#pragma unroll
+                      for (int i = 0; i < 64; ++i) f[i] += __uint_as_float(r[i]);
+                    } else {
+                      const float4* src = others + static_cast<long long>(s) * (2 * 64 * 128) + (col / 4) * 128;
+                      float4 x[16];
+#pragma unroll
+                      for (int i = 0; i < 16; ++i) x[i] = __ldcg(src + i * 128);
+#pragma unroll
+                      for (int i = 0; i < 16; ++i) {
+                        f[4 * i] += x[i].x; f[4 * i + 1] += x[i].y; f[4 * i + 2] += x[i].z; f[4 * i + 3] += x[i].w;
+                      }
+                    }
+                  }
+#pragma unroll
+                  for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(f[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                if (!(ok = emit(v, map, n0 + col))) break;
+              }
+            }
+          }
+        } else
         if constexpr (kMode == kModeSwigluBwd) {
           const int n_boxes = m0 >= p.M ? 0 : min(BN, p.N - n0 + 63) / 64;
 #pragma unroll 1
@@ -677,6 +991,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       bulk_commit_group();
       bulk_wait_group0();  // all output boxes are in memory
       if constexpr (kMode == kModeScatter) __threadfence_system();
+      if constexpr (kMode == kModeGroup) {
+        if (owners.arrivals > 0) __threadfence_system();
+      }
     }
   }
 
@@ -688,9 +1005,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kTmemCols);
   }
-  if constexpr (kMode == kModeScatter) {
+  if constexpr (kMode == kModeScatter || kMode == kModeGroup) {
     // the last CTA to finish releases one arrival on every owner's counter, unless any CTA of the launch gave up
-    if (threadIdx.x == 0) {
+    unsigned long long arrivals = 1;
+    if constexpr (kMode == kModeGroup) arrivals = owners.arrivals;
+    if (threadIdx.x == 0 && arrivals > 0) {
       __threadfence_system();
       const unsigned int prev = atomicAdd(p.done_slot, 1u);
       if (prev == gridDim.x - 1) {
@@ -699,7 +1018,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const bool clean = !*abort_flag && (p.status == nullptr || *reinterpret_cast<volatile int*>(p.status) == 0);
         if (clean)
           for (int r = 0; r < p.nranks; ++r)
-            signal_add_release_sys(reinterpret_cast<unsigned long long*>(p.ctr_ptrs[r]), 1ull);
+            signal_add_release_sys(reinterpret_cast<unsigned long long*>(p.ctr_ptrs[r]), arrivals);
       }
     }
   }
@@ -1018,6 +1337,175 @@ cudaError_t gemm_logits_pair(const void* h, const void* w, void* logits, const l
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
   launch(gemm_bf16_pair_kernel<kModeLogits>, 2 * pairs, kThreads, kSmemBytes, stream, ta, tb, tc, OwnerMaps{}, p);
+  return cudaGetLastError();
+}
+
+// Words for the launches of groups, zero at load and left zero by each: the counter of items, the count of finished CTAs, and two
+// per divided tile.  They are handed out in turn and come round again after at least kGroupWords / (2 + 2 kMaxDivided) launches,
+// more than a device holds queued.
+constexpr unsigned int kGroupWords = 1u << 20;
+constexpr int kMaxDivided = 256;
+__device__ unsigned int g_group_words[kGroupWords];
+static unsigned int* group_words(int n) {
+  static std::mutex mu;
+  static unsigned int at = 0;
+  static unsigned int* base[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (base[dev] == nullptr) {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_group_words) != cudaSuccess) return nullptr;
+    base[dev] = static_cast<unsigned int*>(p);
+  }
+  if (at + n > kGroupWords) at = 0;
+  at += n;
+  return base[dev] + at - n;
+}
+
+// Into how many parts the tiles of each product are divided.  In units of a k-block (0.28 us): the items go to the pairs that are
+// free first, longest first, so the group takes the work per pair and half of its last item, but at least its longest item.  The
+// longest one is divided as long as that gains a twentieth.  An item takes at least what its epilogue does (6); a part of a bf16
+// tile writes and reads 256 KB of fp32 (3 each), the parts of an fp32 sum meet in memory.
+struct GroupShape {
+  int tiles, kb, splits, each;
+  bool may_divide, bf16;
+  double item() const { return std::max(6, each) + (splits > 1 ? (bf16 ? 6.0 : 1.0) : 0.0); }
+  double sum() const { return bf16 && splits > 1 ? 12.0 + 8.0 * (splits - 1) : 0.0; }
+};
+static void plan_group(GroupShape* g, int n, int pairs) {
+  auto cost = [&] {
+    int order[kMaxGroupProducts];
+    for (int i = 0; i < n; ++i) order[i] = i;
+    std::sort(order, order + n, [&](int a, int b) { return g[a].item() > g[b].item(); });
+    double work = 0, span = 0;
+    for (int i = 0; i < n; ++i) {
+      const GroupShape& q = g[order[i]];
+      const int items = q.tiles * q.splits;
+      work += items * q.item();
+      span = std::max(span, (i == 0 ? (items + pairs - 1) / pairs * q.item() : work / pairs + 0.5 * q.item()) + q.sum());
+    }
+    return span;
+  };
+  for (int i = 0; i < n; ++i) { g[i].splits = 1; g[i].each = g[i].kb; }
+  double best = cost();
+  while (true) {
+    int longest = 0;
+    for (int i = 1; i < n; ++i)
+      if (g[i].item() > g[longest].item()) longest = i;
+    GroupShape& q = g[longest];
+    const GroupShape before = q;
+    bool found = false;
+    for (int want = before.splits + 1; want <= 8 && !found && q.may_divide; ++want) {
+      const int each = (q.kb + want - 1) / want, s = (q.kb + each - 1) / each;   // no empty part
+      if (s <= before.splits || each < 4 || (q.bf16 && q.tiles > kMaxDivided)) continue;
+      q.splits = s; q.each = each;
+      const double c = cost();
+      if (c < 0.95 * best) { best = c; found = true; } else { q = before; }
+    }
+    if (!found) { q = before; return; }
+  }
+}
+
+static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* shapes) {
+  using namespace gemm_pair;
+  if (n < 1 || n > kMaxGroup || sm_count < 2) return false;
+  for (int i = 0; i < n; ++i) {
+    const GemmProduct& q = g[i];
+    if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate || q.scale != 1.f))) return false;
+    shapes[i] = GroupShape{(q.M + 255) / 256 * ((q.N + BN - 1) / BN), (q.K + BK - 1) / BK, 1, 0,
+                           q.c_kind == kBF16 || (q.accumulate && !q.fixed_order), q.c_kind == kBF16};
+  }
+  // A group saves the launches and last rounds of its products, 30 to 100 units.  With more work than this for a pair that is no
+  // gain any more, and pairs that are not in step with one another share less of L2 (16321 tokens, 2048 and 8192 wide, 4400 units:
+  // the layer 0.5 % slower together; 5120 and 13824 wide, 32000 units: 7.62 ms one by one, 7.83 together).  fp32 results, 256 KB a
+  // tile to be added to memory, run under the other products' arithmetic (head of 16384 tokens, 128256 words, 2048 wide, 7000
+  // units a chunk: 20.5 ms with its forward, 20.0 together).
+  long long work = 0;
+  bool f32 = false;
+  for (int i = 0; i < n; ++i) {
+    work += static_cast<long long>(shapes[i].tiles) * shapes[i].kb;
+    f32 = f32 || !shapes[i].bf16;
+  }
+  if (work > (f32 ? 12000ll : 3000ll) * (sm_count / 2)) return false;
+  plan_group(shapes, n, sm_count / 2);
+  return true;
+}
+
+size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count) {
+  GroupShape shapes[kMaxGroupProducts];
+  if (!group_shapes(g, n, sm_count, shapes)) return 0;
+  size_t parts = 0;
+  for (int i = 0; i < n; ++i)
+    if (shapes[i].bf16 && shapes[i].splits > 1) parts += static_cast<size_t>(shapes[i].tiles) * shapes[i].splits;
+  return parts * 256 * gemm_pair::BN * sizeof(float);
+}
+
+GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count) {
+  GroupShape shapes[kMaxGroupProducts];
+  GemmGroupPlan plan{};
+  if (!group_shapes(g, n, sm_count, shapes)) return plan;
+  for (int i = 0; i < n; ++i) plan.parts[i] = shapes[i].splits;
+  return plan;
+}
+
+cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long long* ctr_ptrs, int arrivals, int* status, int sm_count,
+                       cudaStream_t stream) {
+  using namespace gemm_pair;
+  GroupShape shapes[kMaxGroup];
+  if (!group_shapes(g, n, sm_count, shapes)) return cudaErrorNotSupported;
+  for (int i = 0; i < n; ++i) {
+    const GemmProduct& q = g[i];
+    if ((reinterpret_cast<uintptr_t>(q.a) | reinterpret_cast<uintptr_t>(q.b) | reinterpret_cast<uintptr_t>(q.c)) & 15)
+      return cudaErrorNotSupported;
+    if ((q.lda % 8) || (q.ldb % 8) || (q.N % 8) || (q.layout == 2 && q.M % 8) || (q.ldc % (q.c_kind == kF32 ? 4 : 8))) return cudaErrorNotSupported;
+  }
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(gemm_bf16_pair_kernel<kModeGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  });
+  if (attr_err != cudaSuccess) return attr_err;
+  int order[kMaxGroup];
+  for (int i = 0; i < n; ++i) order[i] = i;
+  std::stable_sort(order, order + n, [&](int x, int y) { return shapes[x].item() > shapes[y].item(); });
+  Group group{};
+  int divided = 0, parts = 0;
+  for (int i = 0; i < n; ++i) {
+    const GemmProduct& q = g[order[i]];
+    const GroupShape& shape = shapes[order[i]];
+    const bool a_mn = q.layout == 2, b_mn = q.layout != 0;
+    if (!(a_mn ? encode_tile_map_2d(&group.a[i], q.a, q.M, q.K, q.lda * 2, 64, 64) : encode_tile_map_2d(&group.a[i], q.a, q.K, q.M, q.lda * 2, 64, BMH)) ||
+        !(b_mn ? encode_tile_map_2d(&group.b[i], q.b, q.N, q.K, q.ldb * 2, 64, 64) : encode_tile_map_2d(&group.b[i], q.b, q.K, q.N, q.ldb * 2, 64, BNH)) ||
+        !(q.c_kind == kF32 ? encode_tile_map_2d_f32(&group.c[i], q.c, q.N, q.M, q.ldc * 4, 32, BMH) : encode_tile_map_2d(&group.c[i], q.c, q.N, q.M, q.ldc * 2, 64, BMH)))
+      return cudaErrorInvalidValue;
+    GroupProblem& t = group.prob[i];
+    t.M = q.M; t.N = q.N; t.K = q.K;
+    t.tiles_m = (q.M + 255) / 256; t.tiles_n = (q.N + BN - 1) / BN;
+    t.a_mn = a_mn; t.b_mn = b_mn;
+    t.out = q.c_kind == kBF16 ? 0 : q.accumulate ? 2 : 1;
+    t.scale = q.scale;
+    t.first = group.items;
+    t.splits = shape.splits; t.kb_split = shape.each;
+    if (shape.bf16 && shape.splits > 1) {
+      t.first_split_tile = divided; t.first_part = parts;
+      divided += shape.tiles; parts += shape.tiles * shape.splits;
+    }
+    group.items += shape.tiles * shape.splits;
+  }
+  group.count = n;
+  if (divided > kMaxDivided || (divided > 0 && scratch == nullptr)) return cudaErrorNotSupported;
+  group.parts = reinterpret_cast<float4*>(scratch);
+  unsigned int* words = group_words(2 + 2 * divided);
+  if (words == nullptr) return cudaErrorInvalidValue;
+  group.next = words;
+  group.arrived = words + 2;
+  group.arrivals = arrivals;
+  Params p{};
+  p.status = status;
+  p.ctr_ptrs = ctr_ptrs; p.nranks = 1; p.done_slot = words + 1;
+  const int pairs = group.items < sm_count / 2 ? group.items : sm_count / 2;
+  launch(gemm_bf16_pair_kernel<kModeGroup>, 2 * pairs, kThreads, kSmemBytes, stream, group.a[0], group.b[0], group.c[0], group, p);
   return cudaGetLastError();
 }
 

@@ -146,7 +146,7 @@ class ShardedParameter:
                     reg.peer_ptrs(target, self.ranks), self.out_features, self.index, self.grad_scale,
                     service.native_dispatches(self.ranks))
                 self._matrix.local_pending = self._local_dirty
-                ext.set_deferred_weight_grad(_deferred_weight_grad)
+                ext.set_deferred_weight_grad(_deferred_weight_grad, _pending_local_buffer, _push_local)
                 ext.set_sync_grads(_sync_grads)
                 _native = True
         return self._matrix
@@ -286,6 +286,18 @@ def _deferred_weight_grad(i: int, dy2: torch.Tensor, x2: torch.Tensor) -> None:
     """The native layer's way back for a gradient that is accumulated locally, or that follows one that was."""
     with torch.no_grad():
         accumulate_weight_grad(_params[i], dy2, x2)
+
+
+def _pending_local_buffer(i: int) -> torch.Tensor:
+    p = _params[i]
+    p.wait_push()
+    p.local_dirty = True
+    return p.local_buffer()
+
+
+def _push_local(i: int) -> None:
+    with torch.no_grad():
+        _params[i].push_local()
 
 
 def accumulate_weight_grad(p: ShardedParameter, dy2: torch.Tensor, x2: torch.Tensor) -> None:

@@ -53,6 +53,27 @@ def test_small_weight_gradients_stay_whole_across_ranks():
     assert plan(1)[2] > 1 and plan(8) == (4, 4, 1)
 
 
+@pytest.mark.parametrize("T", [64, 300, 1000, 4096, 16321])
+@pytest.mark.parametrize("H,F", [(512, 1536), (1536, 8960), (4096, 14336)])
+def test_groups_divide_what_would_outlast_them(T, H, F):
+    """No product keeps parts without k-blocks, products that overwrite fp32 stay whole, and only what is longer than the work
+    of a pair is divided; groups of very much work are not formed."""
+    plan = lambda *g: _ext.load().gemm_group_plan(list(g), SMS)
+    for acc in (False, True):
+        shapes = [(T, H, 2 * F, False, False), (2 * F, H, T, True, acc), (H, F, T, True, acc)]
+        kb = [-(-K // 64) for _, _, K, _, _ in shapes]
+        tiles = [-(-M // 256) * -(-N // 256) for M, N, *_ in shapes]
+        work = sum(k * t for k, t in zip(kb, tiles))
+        parts = plan(*shapes)
+        if work > 12000 * (SMS // 2):   # fp32 results
+            assert parts == [0, 0, 0]
+            continue
+        for s, k, shape in zip(parts, kb, shapes):
+            assert 1 <= s <= min(8, k) and (s == 1 or not shape[3] or acc)
+        if max(kb) <= work / (SMS // 2) / 2:
+            assert parts == [1, 1, 1]
+
+
 def test_statistics_in_the_product_where_they_pay():
     plan = lambda rows, words, width, gradient: _ext.load().head_plan(rows, words, width, gradient, SMS)
     for gradient in (False, True):

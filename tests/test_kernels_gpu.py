@@ -414,6 +414,81 @@ def test_wgrad_scatter_divided(ext, T, n_out, k_in):
     assert int(ctr[0]) == 5
 
 
+def _group_case(products, seed=0):
+    """Operands of (layout, M, N, K, output, added) each, row strides wider than the rows, and the result in 64 bits."""
+    torch.manual_seed(seed)
+    out = []
+    for lay, M, N, K, dtype, add, scale in products:
+        wide = lambda r, c: torch.randn(r, c + 8, device="cuda").bfloat16()[:, :c]
+        a, b = wide(*((K, M) if lay == "tn" else (M, K))), wide(*((N, K) if lay == "nt" else (K, N)))
+        c = torch.randn(M, N + 8, device="cuda").to(dtype)[:, :N]
+        A, B = (a.t() if lay == "tn" else a).double(), (b.t() if lay == "nt" else b).double()
+        want = (A @ B) * scale + (c.double() if add else 0)
+        # fp32 sums of K products: a few units in the last place of the sum of magnitudes; then one rounding to the output's type
+        bound = (A.abs() @ B.abs() * scale + c.double().abs()) * 2e-6 + want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23)
+        out.append((a, b, c, lay, add, scale, want, bound))
+    return out
+
+
+@pytest.mark.parametrize("parts,products", [
+    # (layout, M, N, K, output, added, scale); bf16 tiles in up to eight parts, edges in M, N and K, one to three products
+    ([1, 1], [("nn", 8, 256, 64, torch.bfloat16, False, 1.0), ("tn", 264, 520, 72, torch.bfloat16, False, 1.0)]),
+    (None, [("nn", 300, 264, 8200, torch.bfloat16, False, 1.0), ("tn", 776, 264, 300, torch.float32, False, 0.5)]),
+    (None, [("nn", 257, 512, 32768, torch.bfloat16, False, 1.0), ("tn", 256, 256, 257, torch.bfloat16, False, 1.0),
+            ("nt", 255, 264, 200, torch.float32, False, 2.0)]),
+    (None, [("tn", 512, 512, 4104, torch.float32, True, 0.25), ("tn", 1536, 264, 4104, torch.float32, True, 1.0)]),
+    (None, [("nn", 1000, 1536, 4096, torch.bfloat16, False, 1.0), ("tn", 4096, 1536, 1000, torch.float32, True, 1.0),
+            ("tn", 1536, 2048, 1000, torch.bfloat16, False, 1.0)]),
+    (None, [("nn", 64, 256, 5000, torch.bfloat16, False, 1.0)]),
+])
+def test_groups_of_products(ext, parts, products):
+    ops = _group_case(products)
+    plan = ext.gemm_group_plan([(M, N, K, d == torch.float32, add) for _, M, N, K, d, add, _ in products], ext.sm_count())
+    assert all(1 <= s <= 8 for s in plan) and (parts is None or plan == parts)
+    start = [c.clone() for _, _, c, *_ in ops]
+    for _ in range(3):   # the counters of one launch are as the next one expects them
+        for (_, _, c, *_), c0 in zip(ops, start):
+            c.copy_(c0)
+        assert ext.gemm_group([(a, b, c, lay, add, scale) for a, b, c, lay, add, scale, _, _ in ops])
+        for a, b, c, lay, add, scale, want, bound in ops:
+            assert ((c.double() - want).abs() <= bound).all(), (lay, plan)
+
+
+def test_parts_of_a_group_are_summed_in_one_order(ext):
+    """Eight parts and as many CTAs that may come last: the same bytes every time, in a replayed graph as well."""
+    torch.manual_seed(0)
+    a, b = torch.randn(300, 30000, device="cuda").bfloat16(), torch.randn(30000, 512, device="cuda").bfloat16()
+    x = torch.randn(300, 264, device="cuda").bfloat16()
+    outs = [torch.empty(300, 512, device="cuda", dtype=torch.bfloat16) for _ in range(6)]
+    dw = torch.empty(30000, 264, device="cuda", dtype=torch.bfloat16)
+    run = lambda o: ext.gemm_group([(a, b, o, "nn", False, 1.0), (a, x, dw, "tn", False, 1.0)])
+    for o in outs[:3]:
+        assert run(o)
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        for o in outs[3:]:
+            run(o)
+    for _ in range(3):
+        for o in outs[3:]:
+            o.zero_()
+        g.replay()
+        assert all(torch.equal(o, outs[0]) for o in outs)
+    assert ext.gemm_group_plan([(300, 512, 30000, False, False), (30000, 264, 300, False, False)], ext.sm_count())[0] > 1
+
+
+def test_groups_that_are_not_taken(ext):
+    """Types, widths and alignments the kernel does not read or write: nothing is done, the products go one by one."""
+    t = lambda *s, dtype=torch.bfloat16: torch.zeros(*s, device="cuda", dtype=dtype)
+    good = (t(300, 512), t(512, 256), t(300, 256), "nn", False, 1.0)
+    for bad in ((t(300, 512).float(), t(512, 256).float(), t(300, 256).float(), "nn", False, 1.0),
+                (t(300, 512), t(512, 200), t(300, 200), "nn", False, 1.0), (t(300, 512), t(512, 260), t(300, 260), "nn", False, 1.0),
+                (t(300, 32), t(32, 256), t(300, 256), "nn", False, 1.0), (t(300, 512), t(512, 256), t(300, 256), "nn", True, 1.0),
+                (t(300, 516)[:, 4:], t(512, 256), t(300, 256), "nn", False, 1.0)):
+        assert not ext.gemm_group([good, bad])
+    assert not ext.gemm_group([good] * 4)
+
+
 @pytest.mark.parametrize("T,H,F", [(24, 256, 512), (300, 512, 1536), (765, 1536, 8960)])
 def test_chained_kernels_see_their_predecessors(ext, T, H, F):
     """A kernel may start before the one ahead of it has ended: a chain queued without a pause gives the bytes of one that is
