@@ -464,6 +464,22 @@ Tensor linear(Tensor x, Tensor w, c10::optional<Tensor> bias, c10::optional<Tens
 // RMSNorm; with_residual also returns x, and backward forms d(norm) + d(residual) in one pass over the activation
 // instead of leaving a separate addition to autograd.  `sink` (fp32 [H]): the weight's gradient is added there by the
 // kernel and the weight itself gets none (engines that keep all small parameters in one flat accumulator).
+//
+// dx, and the weight's gradient unless it went to the sink
+std::tuple<Tensor, Tensor> norm_grads(const Tensor& dy2, const Tensor& x2, const Tensor& w, const Tensor& rstd,
+                                      const c10::optional<Tensor>& dres, const c10::optional<Tensor>& sink) {
+  const bool fixed = env_on("ODC_DETERMINISTIC");  // fixed-order column sums instead of in-kernel atomics
+  auto [dx, dw] = rmsnorm_bwd(dy2, x2, w, rstd, fixed, dres, fixed ? c10::nullopt : sink);
+  count(fixed ? 2 : 1);
+  if (sink.has_value()) {
+    if (fixed) sink->add_(dw);
+    dw = Tensor();
+  } else if (dw.scalar_type() != w.scalar_type()) {
+    dw = dw.to(w.scalar_type());
+  }
+  return {dx, dw};
+}
+
 struct RMSNormFn : Function<RMSNormFn> {
   static variable_list forward(AutogradContext* ctx, Tensor x, Tensor w, double eps, bool with_residual,
                                c10::optional<Tensor> sink) {
@@ -481,21 +497,13 @@ struct RMSNormFn : Function<RMSNormFn> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor &x2 = saved[0], &w = saved[1], &rstd = saved[2];
-    const bool fixed = env_on("ODC_DETERMINISTIC");  // fixed-order column sums instead of in-kernel atomics
     const Tensor dy2 = rows2d(grads[0]).contiguous();
     c10::optional<Tensor> dres;
     if (ctx->saved_data["residual"].toBool() && grads[1].defined()) dres = rows2d(grads[1]).contiguous();
     auto it = ctx->saved_data.find("sink");
     c10::optional<Tensor> sink;
     if (it != ctx->saved_data.end()) sink = it->second.toTensor();
-    auto [dx, dw] = rmsnorm_bwd(dy2, x2, w, rstd, fixed, dres, fixed ? c10::nullopt : sink);
-    count(fixed ? 2 : 1);
-    if (sink.has_value()) {
-      if (fixed) sink->add_(dw);
-      dw = Tensor();
-    } else if (dw.scalar_type() != w.scalar_type()) {
-      dw = dw.to(w.scalar_type());
-    }
+    auto [dx, dw] = norm_grads(dy2, x2, w, rstd, dres, sink);
     return {dx.view(ctx->saved_data["sizes"].toIntVector()), dw, {}, {}, {}};
   }
 };
@@ -891,7 +899,8 @@ struct ShardedMatrix : torch::CustomClassHolder {
   double grad_scale = 1.0;
   bool local_pending = false;           // earlier microbatches left a gradient in the local buffer
   c10::intrusive_ptr<DispatchCounter> dispatched;
-  Tensor whole() const { return shard.narrow(0, 0, out_features); }
+  Tensor matrix;                        // [out_features, K]: the shard of one rank without its padding rows
+  const Tensor& whole() const { return matrix; }
 };
 
 // Start of the last minibatch: an event behind its work, and the stream it ran on.  A pass on that stream is in order as it
@@ -1082,6 +1091,219 @@ Tensor sharded_mlp(Tensor x, c10::optional<Tensor> residual, c10::intrusive_ptr<
   return ShardedMlpFn::apply(x, residual, gu, down, wants_grad(x), residual.has_value() && wants_grad(*residual));
 }
 
+// ---- a decoder layer as one function -----------------------------------------------------------------------------------
+// norm, projection, rotary embedding, attention, output projection, norm, MLP.  Seven functions one behind the other cost the host
+// their interpreter calls, graph nodes and gradient hand-overs, and a small model's step waits for the host all the time.
+// Same kernels, same tensors kept for backward.  Two layers, 512 wide, two microbatches: a training step 2123 us in parts, 1685 as
+// one function a layer; a layer over 1000 tokens, 1536 wide, 373 and 365.
+struct LayerShape {
+  int64_t n_q, n_kv, d, max_seqlen;
+  double theta, eps1, eps2;
+  double scale() const { return 1.0 / std::sqrt(static_cast<double>(d)); }
+  std::vector<int64_t> ints() const { return {n_q, n_kv, d, max_seqlen}; }
+};
+struct LayerWeights {
+  Tensor norm1, wqkv, bqkv, wo, norm2, gate_up, down;   // bqkv may be undefined
+};
+enum LayerKept : int { kX1, kRstd1, kH1, kQkv, kO, kLse, kX2, kRstd2, kH2, kGateUp, kAct, kKept };
+
+// plain bf16 matrices and vectors of one layer; anything else takes the layer's modules one by one, which say what is wrong
+bool layer_takes(const Tensor& x, const Tensor& pos, const Tensor& cu, const LayerWeights& w, const LayerShape& c) {
+  const auto plain = [&](const Tensor& t, at::ScalarType type) {
+    return t.defined() && t.device() == x.device() && t.scalar_type() == type && t.layout() == at::kStrided && t.is_contiguous() &&
+           !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched,
+                                                     c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched}));
+  };
+  const auto matrix = [&](const Tensor& t, int64_t rows, int64_t cols) {
+    return plain(t, at::kBFloat16) && t.dim() == 2 && t.size(0) == rows && t.size(1) == cols;
+  };
+  const char* attention = std::getenv("ODC_ATTN");
+  if (!x.is_cuda() || x.dim() != 2 || !plain(x, at::kBFloat16) || x.size(0) == 0 || library_gemm() ||
+      (attention != nullptr && std::strcmp(attention, "native") != 0))
+    return false;
+  const int64_t T = x.size(0), H = x.size(1), qkv = (c.n_q + 2 * c.n_kv) * c.d;
+  return (c.d == 64 || c.d == 128) && c.n_kv > 0 && c.n_q % c.n_kv == 0 && H % 8 == 0 && plain(pos, at::kLong) && pos.numel() == T &&
+         plain(cu, at::kInt) && cu.numel() >= 2 && plain(w.norm1, at::kBFloat16) && w.norm1.numel() == H &&
+         plain(w.norm2, at::kBFloat16) && w.norm2.numel() == H && matrix(w.wqkv, qkv, H) && matrix(w.wo, H, c.n_q * c.d) &&
+         w.down.defined() && w.down.dim() == 2 && matrix(w.down, H, w.down.size(1)) && w.down.size(1) % 8 == 0 &&
+         matrix(w.gate_up, 2 * w.down.size(1), H) && (!w.bqkv.defined() || (plain(w.bqkv, at::kBFloat16) && w.bqkv.numel() == qkv));
+}
+
+// y, and what a backward needs (empty unless `keep`)
+std::tuple<Tensor, variable_list> layer_forward(const Tensor& x, const Tensor& pos, const Tensor& cu, const LayerWeights& w,
+                                                const LayerShape& c, bool keep) {
+  variable_list kept(keep ? kKept : 0);
+  const auto hold = [&](LayerKept i, const Tensor& t) { if (keep) kept[i] = t; };
+  Tensor qkv, x2, act;
+  {
+    auto [h, rstd] = rmsnorm_fwd(x, w.norm1, c.eps1);
+    hold(kX1, x); hold(kRstd1, rstd); hold(kH1, h);
+    qkv = product(h, w.wqkv, kNT, w.bqkv);
+  }
+  qkv = rope_qkv(qkv, pos, c.n_q, c.n_kv, c.d, c.theta, false);
+  hold(kQkv, qkv);
+  {
+    const auto [q, k, v] = AttentionQKVFn::parts(qkv, c.n_q, c.n_kv, c.d);
+    auto [o, lse] = attn_fwd(q, k, v, cu, c.max_seqlen, true, c.scale());
+    hold(kO, o); hold(kLse, lse);
+    qkv = Tensor();
+    x2 = product(o.view({x.size(0), c.n_q * c.d}), w.wo, kNT, {}, x);
+  }
+  hold(kX2, x2);
+  {
+    auto [h, rstd] = rmsnorm_fwd(x2, w.norm2, c.eps2);
+    hold(kRstd2, rstd); hold(kH2, h);
+    auto [a, gate_up] = linear_swiglu_fwd(h, w.gate_up, keep);
+    hold(kGateUp, gate_up); hold(kAct, a);
+    act = a;
+  }
+  count(4);
+  return {product(act, w.down, kNT, {}, x2), kept};
+}
+
+// dx; `sink` takes the gradients of the weights:
+//   linear(0: projection, 1: output projection; dy2, x2) -> dx;  mlp(d, x2, dy2, act) -> d gate_up;  norm(which, ...) -> dx;  bias(dqkv)
+template <typename Sink>
+Tensor layer_backward(const variable_list& kept, const Tensor& pos, const Tensor& cu, const LayerWeights& w, const LayerShape& c,
+                      const Tensor& dy, Sink& sink) {
+  const int64_t T = dy.size(0);
+  const Tensor d = swiglu_product_bwd(dy, w.down, kept[kGateUp]);
+  const Tensor dh2 = sink.mlp(d, kept[kH2], dy, kept[kAct]);
+  const Tensor dx2 = sink.norm(1, dh2, kept[kX2], w.norm2, kept[kRstd2], dy);
+  const Tensor o = kept[kO];
+  const Tensor dout = sink.linear(1, dx2, o.view({T, c.n_q * c.d})).view({T, c.n_q, c.d});
+  const auto [q, k, v] = AttentionQKVFn::parts(kept[kQkv], c.n_q, c.n_kv, c.d);
+  Tensor dqkv = std::get<3>(attn_bwd(dout, q, k, v, o, kept[kLse], cu, c.max_seqlen, true, c.scale(), true));
+  dqkv = rope_qkv(dqkv, pos, c.n_q, c.n_kv, c.d, c.theta, true);
+  count(4);
+  const Tensor dh1 = sink.linear(0, dqkv, kept[kH1]);
+  sink.bias(dqkv);
+  return sink.norm(0, dh1, kept[kX1], w.norm1, kept[kRstd1], dx2);
+}
+
+struct LayerFn : Function<LayerFn> {
+  struct Sink {
+    const LayerWeights& w;
+    Tensor norm_grad[2], matrix[2], d_gate_up, d_down, d_bias;
+    Tensor linear(int which, const Tensor& dy2, const Tensor& x2) {
+      const Tensor& m = which == 0 ? w.wqkv : w.wo;
+      Tensor dx;
+      std::tie(dx, matrix[which]) = linear_grads(dy2, x2, m, true, true);
+      return dx;
+    }
+    Tensor mlp(const Tensor& d, const Tensor& x2, const Tensor& dy2, const Tensor& act) {
+      const Tensor dx = product_out(d, w.gate_up, kNN);
+      d_gate_up = product_out(d, x2, kTN);
+      d_down = product_out(dy2, act, kTN);
+      products_into({{d, w.gate_up, dx, kNN}, {d, x2, d_gate_up, kTN}, {dy2, act, d_down, kTN}});
+      return dx;
+    }
+    Tensor norm(int which, const Tensor& dh, const Tensor& x, const Tensor& weight, const Tensor& rstd, const Tensor& dres) {
+      Tensor dx;
+      std::tie(dx, norm_grad[which]) = norm_grads(dh, x, weight, rstd, dres, c10::nullopt);
+      return dx;
+    }
+    void bias(const Tensor& dqkv) { if (w.bqkv.defined()) d_bias = column_sum(dqkv); }
+  };
+  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor norm1, Tensor wqkv, c10::optional<Tensor> bqkv, Tensor wo, Tensor norm2,
+                        Tensor gate_up, Tensor down, Tensor pos, Tensor cu, const LayerShape& c, bool keep) {
+    const LayerWeights w{norm1, wqkv, bqkv.value_or(Tensor()), wo, norm2, gate_up, down};
+    auto [y, kept] = layer_forward(x, pos, cu, w, c, keep);
+    if (keep) {
+      for (const Tensor& t : {w.norm1, w.wqkv, w.bqkv, w.wo, w.norm2, w.gate_up, w.down, pos, cu}) kept.push_back(t);
+      ctx->save_for_backward(std::move(kept));
+      ctx->saved_data["shape"] = c.ints();
+      ctx->saved_data["theta"] = c.theta;
+    }
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto kept = ctx->get_saved_variables();
+    const auto i = ctx->saved_data["shape"].toIntVector();
+    const LayerShape c{i[0], i[1], i[2], i[3], ctx->saved_data["theta"].toDouble(), 0, 0};
+    const LayerWeights w{kept[kKept], kept[kKept + 1], kept[kKept + 2], kept[kKept + 3], kept[kKept + 4], kept[kKept + 5], kept[kKept + 6]};
+    Sink sink{w};
+    const Tensor dx = layer_backward(kept, kept[kKept + 7], kept[kKept + 8], w, c, grads[0].contiguous(), sink);
+    return {dx, sink.norm_grad[0], sink.matrix[0], sink.d_bias, sink.matrix[1], sink.norm_grad[1], sink.d_gate_up, sink.d_down, {}, {}, {}, {}};
+  }
+};
+
+// None: not a layer of plain weights that all want a gradient, or none: its modules have to be called
+c10::optional<Tensor> decoder_layer(Tensor x, Tensor pos, Tensor cu, int64_t max_seqlen, int64_t n_q, int64_t n_kv, int64_t d, double theta,
+                                    double eps1, double eps2, Tensor norm1, Tensor wqkv, c10::optional<Tensor> bqkv, Tensor wo, Tensor norm2,
+                                    Tensor gate_up, Tensor down) {
+  const LayerShape c{n_q, n_kv, d, max_seqlen, theta, eps1, eps2};
+  if (!layer_takes(x, pos, cu, {norm1, wqkv, bqkv.value_or(Tensor()), wo, norm2, gate_up, down}, c)) return c10::nullopt;
+  const bool keep = wants_grad(x);
+  for (const Tensor& t : {norm1, wqkv, bqkv.value_or(x), wo, norm2, gate_up, down})
+    if (wants_grad(t) != keep) return c10::nullopt;
+  return LayerFn::apply(x, norm1, wqkv, bqkv, wo, norm2, gate_up, down, pos, cu, c, keep);
+}
+
+// The same for the sharded engine on one rank: the weights are no autograd inputs, their gradients go to the accumulators.
+struct ShardedLayer : torch::CustomClassHolder {
+  c10::intrusive_ptr<ShardedMatrix> wqkv, wo, gate_up, down;
+  LayerWeights w;
+  Tensor norm_sink[2], bias_sink;
+  LayerShape c;
+};
+struct ShardedLayerFn : Function<ShardedLayerFn> {
+  struct Sink {
+    const ShardedLayer& s;
+    Tensor linear(int which, const Tensor& dy2, const Tensor& x2) {
+      ShardedMatrix* m = which == 0 ? s.wqkv.get() : s.wo.get();
+      return sharded_grads(dy2, m, {{m, dy2, x2}});
+    }
+    Tensor mlp(const Tensor& d, const Tensor& x2, const Tensor& dy2, const Tensor& act) {
+      return sharded_grads(d, s.gate_up.get(), {{s.gate_up.get(), d, x2}, {s.down.get(), dy2, act}});
+    }
+    Tensor norm(int which, const Tensor& dh, const Tensor& x, const Tensor& weight, const Tensor& rstd, const Tensor& dres) {
+      return std::get<0>(norm_grads(dh, x, weight, rstd, dres, s.norm_sink[which]));
+    }
+    void bias(const Tensor& dqkv) {
+      if (!s.w.bqkv.defined()) return;
+      check(odc::launch_column_sum(dqkv.data_ptr(), nullptr, s.bias_sink.data_ptr<float>(), dqkv.size(0), static_cast<int>(dqkv.size(1)),
+                                   cur_stream()), "column_sum");
+      count();
+    }
+  };
+  static Tensor forward(AutogradContext* ctx, Tensor x, Tensor pos, Tensor cu, c10::intrusive_ptr<ShardedLayer> s, bool keep) {
+    auto [y, kept] = layer_forward(x, pos, cu, s->w, s->c, keep);
+    if (keep) {
+      kept.push_back(pos);
+      kept.push_back(cu);
+      ctx->save_for_backward(std::move(kept));
+      ctx->saved_data["layer"] = c10::IValue::make_capsule(s);
+    }
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto kept = ctx->get_saved_variables();
+    auto capsule = ctx->saved_data["layer"].toCapsule();
+    const auto& s = *static_cast<ShardedLayer*>(capsule.get());
+    Sink sink{s};
+    return {layer_backward(kept, kept[kKept], kept[kKept + 1], s.w, s.c, grads[0].contiguous(), sink), {}, {}, {}, {}};
+  }
+};
+// (view of the gathered vector, fp32 buffer its gradient is added to) for both norms and the bias
+using SmallWeight = std::tuple<Tensor, Tensor>;
+c10::optional<Tensor> sharded_layer(Tensor x, Tensor pos, Tensor cu, int64_t max_seqlen, int64_t n_q, int64_t n_kv, int64_t d, double theta,
+                                    double eps, SmallWeight norm1, c10::intrusive_ptr<ShardedMatrix> wqkv, c10::optional<SmallWeight> bqkv,
+                                    c10::intrusive_ptr<ShardedMatrix> wo, SmallWeight norm2, c10::intrusive_ptr<ShardedMatrix> gate_up,
+                                    c10::intrusive_ptr<ShardedMatrix> down) {
+  for (const auto* m : {wqkv.get(), wo.get(), gate_up.get(), down.get()}) TORCH_CHECK(m->world == 1, "sharded_layer: one rank");
+  auto s = c10::make_intrusive<ShardedLayer>();
+  s->wqkv = wqkv; s->wo = wo; s->gate_up = gate_up; s->down = down;
+  s->w = {std::get<0>(norm1), wqkv->whole(), bqkv.has_value() ? std::get<0>(*bqkv) : Tensor(), wo->whole(), std::get<0>(norm2),
+          gate_up->whole(), down->whole()};
+  s->norm_sink[0] = std::get<1>(norm1); s->norm_sink[1] = std::get<1>(norm2);
+  if (bqkv.has_value()) s->bias_sink = std::get<1>(*bqkv);
+  s->c = {n_q, n_kv, d, max_seqlen, theta, eps, eps};
+  if (!layer_takes(x, pos, cu, s->w, s->c)) return c10::nullopt;
+  after_start();
+  return ShardedLayerFn::apply(x, pos, cu, s, wants_grad(x));
+}
+
 }  // namespace
 
 void register_ops(py::module_& m) {
@@ -1160,6 +1382,7 @@ void register_ops(py::module_& m) {
         p->acc_addrs = std::move(acc_addrs);
         p->out_features = out_features; p->rows_per_rank = shard.size(0); p->index = index; p->grad_scale = grad_scale;
         p->dispatched = dispatched;
+        if (p->world == 1) p->matrix = shard.narrow(0, 0, out_features);
         return p;
       }))
       .def_readwrite("local_pending", &ShardedMatrix::local_pending);
@@ -1180,6 +1403,8 @@ void register_ops(py::module_& m) {
   m.def("sharded_linear", &sharded_linear, py::arg("x"), py::arg("bias"), py::arg("residual"), py::arg("matrix"),
         py::arg("bias_sink") = py::none(), py::arg("keep_weight") = false);
   m.def("sharded_mlp", &sharded_mlp, py::arg("x"), py::arg("residual"), py::arg("gate_up"), py::arg("down"));
+  m.def("decoder_layer", &decoder_layer);
+  m.def("sharded_layer", &sharded_layer);
   m.def("linear", &linear, py::arg("x"), py::arg("w"), py::arg("bias") = py::none(), py::arg("residual") = py::none());
   m.def("rms_norm", &rms_norm, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());
   m.def("rms_norm_residual", &rms_norm_residual, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());

@@ -161,6 +161,15 @@ def mlp(x, w_gate_up, w_down, residual=None):
     return _ext().mlp(x, w_gate_up, w_down, residual)
 
 
+def decoder_layer(x, position_ids, cu_seqlens, max_seqlen: int, n_q: int, n_kv: int, head_dim: int, theta: float, attn_eps: float,
+                  mlp_eps: float, attn_norm, wqkv, bqkv, wo, mlp_norm, w_gate_up, w_down):
+    """A pre-norm decoder layer (RMSNorm, rotary causal attention, RMSNorm, SwiGLU) on a CUDA tensor as one function; None where
+    its weights are not plain bf16 matrices that all want a gradient, or none of them: then it has to be put together from
+    the ops above."""
+    return _ext().decoder_layer(x, position_ids, cu_seqlens, max_seqlen, n_q, n_kv, head_dim, theta, attn_eps, mlp_eps, attn_norm,
+                                wqkv, bqkv, wo, mlp_norm, w_gate_up, w_down)
+
+
 # ------------------------------------------------------------------------------------------
 def varlen_attention_qkv(qkv, n_q: int, n_kv: int, head_dim: int, cu_seqlens, max_seqlen: int, causal: bool = True,
                          scale: Optional[float] = None):

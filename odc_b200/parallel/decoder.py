@@ -36,7 +36,7 @@ from ..primitives import GatherService
 from ..runtime import control
 from ..runtime.registry import SymmBufferRegistry
 from . import linear as L
-from .linear import OdcLinear, ShardedParameter, plain_matrix
+from .linear import OdcLinear, ShardedParameter, plain_matrices
 
 
 class SmallGroup:
@@ -300,6 +300,15 @@ class FusedDecoderLayer(nn.Module):
     def forward(self, x, position_ids, cu_seqlens, max_seqlen):
         c, s, i = self.cfg, self.small, self.i
         T = x.shape[0]
+        if s.native and not c.rope_scaling and (x.requires_grad or not torch.is_grad_enabled()):
+            m = plain_matrices((self.wqkv, self.wo, self.w_gate_up, self.w_down), x)
+            if m:
+                y = ops._ext().sharded_layer(x, position_ids, cu_seqlens, max_seqlen, c.num_heads, c.num_kv_heads, c.head_dim,
+                                             c.rope_theta, c.rms_eps, s._sinks(x, f"layers.{i}.attn_norm.weight"), m[0],
+                                             s._sinks(x, f"layers.{i}.attn.bqkv") if c.qkv_bias else None, m[1],
+                                             s._sinks(x, f"layers.{i}.mlp_norm.weight"), m[2], m[3])
+                if y is not None:
+                    return y
         h, x = s.norm_residual(x, f"layers.{i}.attn_norm.weight", c.rms_eps)
         bias, sink = s.bias(h, f"layers.{i}.attn.bqkv") if c.qkv_bias else (None, None)
         qkv = self.wqkv(h, bias=bias, bias_sink=sink)
@@ -308,9 +317,9 @@ class FusedDecoderLayer(nn.Module):
         o = ops.varlen_attention_qkv(qkv, c.num_heads, c.num_kv_heads, c.head_dim, cu_seqlens, max_seqlen, causal=True)
         x = self.wo(o.reshape(T, c.num_heads * c.head_dim), residual=x)
         h, x = s.norm_residual(x, f"layers.{i}.mlp_norm.weight", c.rms_eps)
-        gate_up, down = plain_matrix(self.w_gate_up, h), plain_matrix(self.w_down, h)
-        if gate_up and down:
-            return ops._ext().sharded_mlp(h, x, gate_up, down)
+        m = plain_matrices((self.w_gate_up, self.w_down), h)
+        if m:
+            return ops._ext().sharded_mlp(h, x, *m)
         return self.w_down(ops.swiglu(self.w_gate_up(h)), residual=x)
 
 

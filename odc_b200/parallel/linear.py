@@ -351,17 +351,30 @@ class OdcLinear(nn.Module):
 _own_forward = OdcLinear.forward
 
 
+def plain_matrices(layers, x):
+    """The native handles of ``OdcLinear`` s whose whole matrices are this rank's and whose calls nobody watches or replaces: their
+    caller may then take the matrices together.  Else None, and the layers have to be called."""
+    if not x.is_cuda or nn.modules.module._has_any_global_hook() or os.environ.get("ODC_WGRAD_SCATTER", "tma") != "tma":
+        return None
+    found = []
+    for layer in layers:
+        if not isinstance(layer, OdcLinear) or "forward" in layer.__dict__ or type(layer).forward is not _own_forward \
+                or type(layer).__call__ is not nn.Module.__call__:
+            return None
+        weight = layer.weight
+        if weight.world != 1 or layer.bias is not None or layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks \
+                or layer._backward_pre_hooks:
+            return None
+        m = weight.matrix() if weight._matrix is None else weight._matrix
+        if not m:
+            return None
+        found.append(m)
+    return found
+
+
 def plain_matrix(layer, x):
-    """The native handle of an ``OdcLinear`` whose whole matrix is this rank's and whose call nobody watches or replaces: its
-    caller may then take the matrix together with its neighbours.  Else None, and the layer has to be called."""
-    if not isinstance(layer, OdcLinear) or "forward" in layer.__dict__ or type(layer).forward is not _own_forward \
-            or type(layer).__call__ is not nn.Module.__call__:
-        return None
-    if layer.weight.world != 1 or not x.is_cuda or layer.bias is not None or layer._forward_hooks or layer._forward_pre_hooks \
-            or layer._backward_hooks or layer._backward_pre_hooks or nn.modules.module._has_any_global_hook() \
-            or os.environ.get("ODC_WGRAD_SCATTER", "tma") != "tma":
-        return None
-    return (layer.weight.matrix() if layer.weight._matrix is None else layer.weight._matrix) or None
+    found = plain_matrices((layer,), x)
+    return found[0] if found else None
 
 
 def sharded_parameters() -> List[ShardedParameter]:

@@ -260,3 +260,66 @@ def test_layers_of_the_mlp_are_called_where_somebody_stands_between(form, name):
         assert len(calls) == len(mbs)
         for key, want in clean.items():   # the same roundings; fp32 sums of products in another order
             assert _rel(got[key], want) < 1e-3, key
+
+
+@pytest.mark.parametrize("name,tokens", [("llama3.2-1b", [5, 128, 77]), ("qwen2.5-1.5b", [300, 64]), ("tiny", [1])])
+@pytest.mark.parametrize("grad", [True, False])
+def test_a_layer_as_one_function_is_its_parts(name, tokens, grad):
+    """Same kernels on the same operands: the same bytes forward; backward the additions of the norms' and the queries' gradients
+    come in any order (fp32, then rounded to bf16: 2^-8 of what a flipped rounding moves, far less in the norm)."""
+    from odc_b200 import ops
+    from odc_b200.models import DecoderLayer, get_config
+    cfg = get_config(name)
+    cfg.num_layers = 1
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        layer = DecoderLayer(cfg).bfloat16()
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.normal_(0.0 if p.dim() == 2 else 0.5, 0.05)
+    T = sum(tokens)
+    x = torch.randn(T, cfg.hidden_size, device="cuda").bfloat16().requires_grad_(grad)
+    for p in layer.parameters():
+        p.requires_grad_(grad)
+    dy = torch.randn(T, cfg.hidden_size, device="cuda").bfloat16()
+    pos = torch.cat([torch.arange(n) for n in tokens]).cuda()
+    cu = torch.tensor([0] + tokens).cumsum(0).int().cuda()
+    taken = []
+    whole = ops.decoder_layer
+    results = []
+    for parts in (False, True):
+        ops.decoder_layer = (lambda *a: None) if parts else (lambda *a: taken.append(whole(*a)) or taken[-1])
+        try:
+            y = layer(x, pos, cu, max(tokens))
+        finally:
+            ops.decoder_layer = whole
+        results.append([y] + (list(torch.autograd.grad(y, [x, *layer.parameters()], dy)) if grad else []))
+    assert len(taken) == 1 and taken[0] is not None
+    assert torch.equal(results[0][0], results[1][0])
+    for a, b in zip(*results):
+        assert a.dtype == b.dtype and a.shape == b.shape and _rel(a.float(), b.float()) < 3e-3
+
+
+def test_layers_that_are_not_taken_as_one_function():
+    """A frozen weight, weights of other types, strided activations and three dimensions go through the parts as before."""
+    from odc_b200 import ops
+    from odc_b200.models import DecoderLayer, get_config
+    cfg = get_config("llama3.2-1b")
+    with torch.device("cuda"):
+        layer = DecoderLayer(cfg).bfloat16()
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.normal_(0.0, 0.02)
+    x = torch.randn(300, cfg.hidden_size, device="cuda").bfloat16()
+    pos, cu = torch.arange(300, device="cuda"), torch.tensor([0, 300], dtype=torch.int32, device="cuda")
+    want = layer(x, pos, cu, 300)
+    layer.mlp.w_down.requires_grad_(False)
+    y = layer(x.requires_grad_(), pos, cu, 300)
+    assert torch.equal(y, want)
+    y.sum().backward()
+    assert layer.mlp.w_down.grad is None and layer.mlp.w_gate_up.grad is not None and x.grad is not None
+    layer.mlp.w_down.requires_grad_(True)
+    with torch.no_grad():
+        strided = torch.empty(300, 2 * cfg.hidden_size, device="cuda", dtype=torch.bfloat16)[:, :cfg.hidden_size]
+        strided.copy_(x)
+        assert torch.equal(layer(strided, pos, cu, 300), want)

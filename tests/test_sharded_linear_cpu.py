@@ -77,3 +77,36 @@ def test_watched_layers_are_called(register, everywhere):
     assert L.plain_matrix(layer, _OnGpu()) is None
     handle.remove()
     assert L.plain_matrix(layer, _OnGpu()) is layer.weight._matrix
+
+
+def _no_op(*args):
+    return None
+
+
+@pytest.mark.parametrize("part", ["attn_norm", "attn", "mlp_norm", "mlp"])
+def test_a_layer_is_one_function_only_as_it_was_built(part):
+    """Hooks, wrappers, other classes, another forward and hooks on all modules make the layer call its parts."""
+    from odc_b200.models import DecoderLayer, get_config
+    make = lambda: DecoderLayer(get_config("tiny"))
+    layer = make()
+    assert layer._as_built()
+    for register in ("register_forward_hook", "register_forward_pre_hook", "register_full_backward_hook", "register_full_backward_pre_hook"):
+        handle = getattr(getattr(layer, part), register)(_no_op)
+        assert not layer._as_built(), register
+        handle.remove()
+        assert layer._as_built()
+    handle = torch.nn.modules.module.register_module_forward_hook(_no_op)
+    assert not layer._as_built()
+    handle.remove()
+    setattr(getattr(layer, part), "forward", _no_op)
+    assert not layer._as_built()
+    layer = make()
+    setattr(layer, part, torch.nn.Identity())
+    assert not layer._as_built()
+    layer = make()
+    mod = getattr(layer, part)
+    mod.__class__ = type("Sub", (type(mod),), {})
+    assert not layer._as_built()
+    layer = make()
+    layer.attn.cfg.rope_scaling = {"rope_type": "linear", "factor": 2.0}
+    assert not layer._as_built()
