@@ -348,7 +348,7 @@ std::tuple<Tensor, Tensor> attn_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seql
 
 std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse,
                                                     Tensor cu_seqlens, int max_seqlen, bool causal, double scale,
-                                                    bool fused_qkv) {
+                                                    bool fused_qkv, const Tensor& rope_pos = {}, double rope_theta = 0) {
   c10::cuda::CUDAGuard g(q.device());
   odc::bind_device(q.get_device());
   const int T = q.size(0), hq = q.size(1), d = q.size(2), hkv = k.size(1);
@@ -378,7 +378,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> attn_bwd(Tensor dout, Tensor q, Tenso
                       dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta.data_ptr<float>(), dq_acc.data_ptr<float>(),
                       n_parts > 1 ? kv_parts.data_ptr<float>() : nullptr, n_parts, cu_seqlens.data_ptr<int>(), n_seqs, T, max_seqlen, hq, hkv, d,
                       q.stride(0), k.stride(0), o.stride(0), dq.stride(0), dk.stride(0), static_cast<float>(scale),
-                      causal, device_status(q.get_device()).data_ptr<int>(), sm_count(), cur_stream()),
+                      causal, device_status(q.get_device()).data_ptr<int>(), sm_count(), cur_stream(),
+                      rope_pos.defined() ? reinterpret_cast<const long long*>(rope_pos.data_ptr<int64_t>()) : nullptr,
+                      static_cast<float>(rope_theta)),
         "attn_bwd");
   return {dq, dk, dv, fused_qkv ? dqkv : dq};  // 4th: the fused gradient when requested
 }
@@ -551,6 +553,32 @@ struct SwiGLUFn : Function<SwiGLUFn> {
   }
 };
 Tensor swiglu(Tensor gate_up) { return SwiGLUFn::apply(gate_up.contiguous()); }
+
+// rope(x w^T + bias): rotated in the epilogue of the product where that kernel takes the shape
+Tensor linear_rope(const Tensor& x, const Tensor& w, const Tensor& bias, const Tensor& pos, int64_t n_q, int64_t n_kv, int64_t d,
+                   double theta) {
+  c10::cuda::CUDAGuard g(x.device());
+  odc::bind_device(x.get_device());
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && w.size(0) == (n_q + 2 * n_kv) * d, "linear_rope: x [T,K], w [(Hq+2Hkv)*D,K]");
+  TORCH_CHECK(pos.scalar_type() == at::kLong && pos.is_contiguous() && pos.numel() == x.size(0), "linear_rope: position_ids int64 [T]");
+  if (odc::gemm_pairs_enabled() && !library_gemm() && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+      x.stride(1) == 1 && w.stride(1) == 1 && (!bias.defined() || (bias.scalar_type() == at::kBFloat16 && bias.is_contiguous()))) {
+    auto out = at::empty({x.size(0), w.size(0)}, x.options());
+    const cudaError_t e = odc::gemm_rope_pair(
+        x.data_ptr(), w.data_ptr(), bias.defined() ? bias.data_ptr() : nullptr, out.data_ptr(),
+        reinterpret_cast<const long long*>(pos.data_ptr<int64_t>()), static_cast<int>(x.size(0)), static_cast<int>(w.size(0)),
+        static_cast<int>(x.size(1)), x.stride(0), w.stride(0), static_cast<int>((n_q + n_kv) * d), static_cast<int>(d),
+        static_cast<float>(theta), device_status(x.get_device()).data_ptr<int>(), sm_count(), cur_stream());
+    if (e != cudaErrorNotSupported) {
+      check(e, "linear_rope");
+      count();
+      return out;
+    }
+  }
+  const Tensor qkv = product(x, w, kNT, bias);
+  count();
+  return rope_qkv(qkv, pos, n_q, n_kv, d, theta, false);
+}
 
 // swiglu(x w^T) for w = [gate; up]: the activation is formed in the epilogue of the product where that kernel takes the
 // shape.  gate_up is only written when a gradient will need it.
@@ -1138,9 +1166,8 @@ std::tuple<Tensor, variable_list> layer_forward(const Tensor& x, const Tensor& p
   {
     auto [h, rstd] = rmsnorm_fwd(x, w.norm1, c.eps1);
     hold(kX1, x); hold(kRstd1, rstd); hold(kH1, h);
-    qkv = product(h, w.wqkv, kNT, w.bqkv);
+    qkv = linear_rope(h, w.wqkv, w.bqkv, pos, c.n_q, c.n_kv, c.d, c.theta);
   }
-  qkv = rope_qkv(qkv, pos, c.n_q, c.n_kv, c.d, c.theta, false);
   hold(kQkv, qkv);
   {
     const auto [q, k, v] = AttentionQKVFn::parts(qkv, c.n_q, c.n_kv, c.d);
@@ -1157,7 +1184,7 @@ std::tuple<Tensor, variable_list> layer_forward(const Tensor& x, const Tensor& p
     hold(kGateUp, gate_up); hold(kAct, a);
     act = a;
   }
-  count(4);
+  count(3);
   return {product(act, w.down, kNT, {}, x2), kept};
 }
 
@@ -1173,9 +1200,8 @@ Tensor layer_backward(const variable_list& kept, const Tensor& pos, const Tensor
   const Tensor o = kept[kO];
   const Tensor dout = sink.linear(1, dx2, o.view({T, c.n_q * c.d})).view({T, c.n_q, c.d});
   const auto [q, k, v] = AttentionQKVFn::parts(kept[kQkv], c.n_q, c.n_kv, c.d);
-  Tensor dqkv = std::get<3>(attn_bwd(dout, q, k, v, o, kept[kLse], cu, c.max_seqlen, true, c.scale(), true));
-  dqkv = rope_qkv(dqkv, pos, c.n_q, c.n_kv, c.d, c.theta, true);
-  count(4);
+  const Tensor dqkv = std::get<3>(attn_bwd(dout, q, k, v, o, kept[kLse], cu, c.max_seqlen, true, c.scale(), true, pos, c.theta));
+  count(3);
   const Tensor dh1 = sink.linear(0, dqkv, kept[kH1]);
   sink.bias(dqkv);
   return sink.norm(0, dh1, kept[kX1], w.norm1, kept[kRstd1], dx2);
@@ -1361,7 +1387,12 @@ void register_ops(py::module_& m) {
     return p.whole == 0 ? p.scratch_bytes : 0;
   });
   m.def("attn_fwd", &attn_fwd);
-  m.def("attn_bwd", &attn_bwd);
+  m.def("attn_bwd", [](Tensor dout, Tensor q, Tensor k, Tensor v, Tensor o, Tensor lse, Tensor cu_seqlens, int max_seqlen, bool causal,
+                       double scale, bool fused_qkv, c10::optional<Tensor> rope_pos, double rope_theta) {
+    return attn_bwd(dout, q, k, v, o, lse, cu_seqlens, max_seqlen, causal, scale, fused_qkv, rope_pos.value_or(Tensor()), rope_theta);
+  }, py::arg("dout"), py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("lse"), py::arg("cu_seqlens"),
+        py::arg("max_seqlen"), py::arg("causal"), py::arg("scale"), py::arg("fused_qkv"), py::arg("rope_pos") = py::none(),
+        py::arg("rope_theta") = 0.0);
   m.def("exp2_poly", &exp2_poly);
   m.def("attn_plan", [](int tokens, int seqs, int longest, int n_q, int n_kv, int d, bool causal, int sms) {
     return std::make_tuple(d == 128 && odc::attn_fwd_pairs(tokens, seqs, longest, n_q, n_kv, causal, sms),
@@ -1409,6 +1440,9 @@ void register_ops(py::module_& m) {
   m.def("rms_norm", &rms_norm, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());
   m.def("rms_norm_residual", &rms_norm_residual, py::arg("x"), py::arg("w"), py::arg("eps"), py::arg("sink") = py::none());
   m.def("rope", &rope);
+  m.def("linear_rope", [](Tensor x, Tensor w, c10::optional<Tensor> bias, Tensor pos, int64_t n_q, int64_t n_kv, int64_t d, double theta) {
+    return linear_rope(x, w, bias.value_or(Tensor()), pos, n_q, n_kv, d, theta);
+  });
   m.def("swiglu", &swiglu);
   m.def("linear_swiglu", &linear_swiglu, py::arg("x"), py::arg("w"));
   m.def("swiglu_product_bwd", &swiglu_product_bwd, py::arg("dy"), py::arg("w"), py::arg("gate_up"));

@@ -154,6 +154,11 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long l
 // act[M, F] = silu(x Wg^T) * (x Wu^T), w = [Wg; Wu]; gate_up [M, 2F] optional.  cudaErrorNotSupported: use the plain product.
 cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* act, int M, int F, int K, long long ldx,
                              long long ldw, int* status, int sm_count, cudaStream_t stream);
+// out[M, N] = x w^T + bias with the heads of the columns below rot_cols rotated by pos[row], as launch_rope_qkv does.
+// cudaErrorNotSupported: use the plain product and that.
+cudaError_t gemm_rope_pair(const void* x, const void* w, const void* bias, void* out, const long long* pos, int M, int N, int K,
+                           long long ldx, long long ldw, int rot_cols, int head_dim, float theta, int* status, int sm_count,
+                           cudaStream_t stream);
 cudaError_t gemm_wgrad_scatter_pair(const void* dy, const void* x, int tokens, int n_out, int k_in, long long ld_dy,
                                     long long ld_x, const long long* acc_addrs_host, const long long* ctr_ptrs,
                                     long long acc_offset, int rows_per_rank, int nranks, float scale,
@@ -224,6 +229,8 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
                      void* dq, void* dk, void* dv, float* delta, float* dq_acc, float* kv_parts, int parts, const int* cu_seqlens, int num_seqs,
                      int total_tokens, int max_seqlen, int n_q, int n_kv, int head_dim, long long q_stride,
                      long long kv_stride, long long o_stride, long long dq_stride, long long dkv_stride, float scale,
-                     bool causal, int* status, int sm_count, cudaStream_t stream);
+                     bool causal, int* status, int sm_count, cudaStream_t stream,
+                     // positions [tokens] by which q and k were rotated (rotary base rope_theta): their gradients are rotated back
+                     const long long* rope_pos = nullptr, float rope_theta = 0.f);
 
 }  // namespace odc

@@ -1022,7 +1022,7 @@ constexpr int kDeltaHeads = 4;
 template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o, float* __restrict__ delta,
-                  int total_tokens, int n_q, long long do_stride, long long o_stride) {
+                  float* __restrict__ dq_acc, int total_tokens, int n_q, long long do_stride, long long o_stride) {
   constexpr int kLanes = D / 8;               // threads per (token, head)
   constexpr int kTokens = 256 / kLanes;       // tokens per CTA
   const int part = threadIdx.x % kLanes;
@@ -1049,7 +1049,11 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* _
     }
 #pragma unroll
     for (int off = kLanes / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (live && part == 0 && h0 + k < n_q) delta[static_cast<long long>(h0 + k) * total_tokens + t] = s;
+    if (live && h0 + k < n_q) {
+      if (part == 0) delta[static_cast<long long>(h0 + k) * total_tokens + t] = s;
+      float4* acc = reinterpret_cast<float4*>(dq_acc + (static_cast<long long>(t) * n_q + h0 + k) * D + part * 8);
+      acc[0] = acc[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
 }
 
@@ -1081,6 +1085,92 @@ narrow_grads_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ d
     const float f = is_v ? 1.f : scale;
     *reinterpret_cast<uint4*>(dst + col) =
         make_uint4(pack2(a.x * f, a.y * f), pack2(a.z * f, a.w * f), pack2(b.x * f, b.y * f), pack2(b.z * f, b.w * f));
+  }
+}
+
+// The same for queries and keys that were rotated by their positions after the projection: the gradients are rotated back on the
+// way, rounded before as the pass over them finds them, and v's are left alone.  Bound by memory: fp32 dQ read once, dQ written and dK read
+// and written once, instead of a pass that narrows dQ and one over the whole of dqkv (16321 tokens, 32/8 heads of 64: 35 + 43 us).
+constexpr int kFinishTokens = 4;   // per CTA: their angles are as many as its threads
+template <int D>
+__global__ void __launch_bounds__(256)
+finish_rope_grads_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk,
+                         __nv_bfloat16* __restrict__ dv, int total_tokens, int n_q, int n_kv, long long dq_stride, long long dkv_stride,
+                         float scale, const float* __restrict__ kv_parts, int parts, const long long* __restrict__ pos, float log2_theta) {
+  constexpr int kHalf = D / 2, kVecs = kHalf / 8;
+  __shared__ float cs[kFinishTokens][2][kHalf];   // cosine and sine of the rotation back
+  const int t0 = blockIdx.x * kFinishTokens, tokens = min(kFinishTokens, total_tokens - t0);
+  for (int i = threadIdx.x; i < tokens * kHalf; i += blockDim.x) {
+    const int f = i % kHalf;
+    float sn, c;
+    sincosf(static_cast<float>(pos[t0 + i / kHalf]) * exp2f(-log2_theta * (2.0f * f) / D), &sn, &c);
+    cs[i / kHalf][0][f] = c;
+    cs[i / kHalf][1][f] = -sn;
+  }
+  __syncthreads();
+  const long long part_stride = 2ll * total_tokens * n_kv * D;
+  auto load8 = [&](const float* src, float* x, int n_parts) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = 0.f;
+    for (int s = 0; s < n_parts; ++s, src += part_stride) {
+      const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+      x[0] += a.x; x[1] += a.y; x[2] += a.z; x[3] += a.w;
+      x[4] += b.x; x[5] += b.y; x[6] += b.z; x[7] += b.w;
+    }
+  };
+  auto load8_bf16 = [&](const __nv_bfloat16* src, float* x) {
+    const uint4 u = *reinterpret_cast<const uint4*>(src);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[2 * i] = __uint_as_float(w[i] << 16);
+      x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  };
+  auto store8 = [&](__nv_bfloat16* dst, const float* x) {
+    *reinterpret_cast<uint4*>(dst) = make_uint4(pack2(x[0], x[1]), pack2(x[2], x[3]), pack2(x[4], x[5]), pack2(x[6], x[7]));
+  };
+  const int per_token = (n_q + n_kv) * kVecs;
+  for (int i = threadIdx.x; i < tokens * per_token; i += blockDim.x) {
+    const int tok = i / per_token, it = i - tok * per_token, head = it / kVecs, j = it % kVecs * 8;
+    const long long t = t0 + tok;
+    float x1[8], x2[8], o1[8], o2[8];
+    __nv_bfloat16* dst;
+    float f = scale;
+    if (head < n_q) {
+      const float* src = acc + (t * n_q + head) * D + j;
+      load8(src, x1, 1);
+      load8(src + kHalf, x2, 1);
+      dst = dq + t * dq_stride + head * D + j;
+    } else {
+      dst = dk + t * dkv_stride + (head - n_q) * D + j;
+      if (parts > 1) {
+        const float* src = kv_parts + (t * n_kv + head - n_q) * D + j;
+        load8(src, x1, parts);
+        load8(src + kHalf, x2, parts);
+      } else {   // scaled and rounded by the kernel that formed it
+        load8_bf16(dst, x1);
+        load8_bf16(dst + kHalf, x2);
+        f = 1.f;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float a = __bfloat162float(__float2bfloat16(x1[e] * f)), b = __bfloat162float(__float2bfloat16(x2[e] * f));
+      rotate_pair(a, b, cs[tok][0][j + e], cs[tok][1][j + e], &o1[e], &o2[e]);
+    }
+    store8(dst, o1);
+    store8(dst + kHalf, o2);
+  }
+  if (parts > 1) {
+    const int v_per_token = n_kv * D / 8;
+    for (int i = threadIdx.x; i < tokens * v_per_token; i += blockDim.x) {
+      const int tok = i / v_per_token, col = (i - tok * v_per_token) * 8;
+      const long long t = t0 + tok;
+      float x[8];
+      load8(kv_parts + (static_cast<long long>(total_tokens) + t) * n_kv * D + col, x, parts);
+      store8(dv + t * dkv_stride + col, x);
+    }
   }
 }
 
@@ -1191,7 +1281,7 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
                      const int* cu_seqlens, int num_seqs,
                      int total_tokens, int max_seqlen, int n_q, int n_kv, int head_dim, long long q_stride,
                      long long kv_stride, long long o_stride, long long dq_stride, long long dkv_stride, float scale,
-                     bool causal, int* status, int sm_count, cudaStream_t stream) {
+                     bool causal, int* status, int sm_count, cudaStream_t stream, const long long* rope_pos, float rope_theta) {
   (void)max_seqlen;
   if (total_tokens == 0 || num_seqs == 0) return cudaSuccess;
   if (head_dim != 64 && head_dim != 128) return cudaErrorInvalidValue;
@@ -1204,15 +1294,13 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
   const unsigned int delta_y = (n_q + kDeltaHeads - 1) / kDeltaHeads;
   if (head_dim == 64) {
     launch(attn_delta_kernel<64>, dim3((total_tokens + 31) / 32, delta_y), 256, 0, stream,
-        static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, total_tokens, n_q,
+        static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, dq_acc, total_tokens, n_q,
         do_stride, o_stride);
   } else {
     launch(attn_delta_kernel<128>, dim3((total_tokens + 15) / 16, delta_y), 256, 0, stream,
-        static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, total_tokens, n_q,
+        static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(o), delta, dq_acc, total_tokens, n_q,
         do_stride, o_stride);
   }
-  cudaError_t e = cudaMemsetAsync(dq_acc, 0, sizeof(float) * static_cast<size_t>(total_tokens) * n_q * head_dim, stream);
-  if (e != cudaSuccess) return e;
   CUtensorMap tq, tk, tv, tdo, tdq;
   if (!encode_tile_map_2d_f32(&tdq, dq_acc, static_cast<uint64_t>(n_q) * head_dim, total_tokens,
                               static_cast<uint64_t>(n_q) * head_dim * 4, 32, 128))
@@ -1253,6 +1341,13 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
     launch(attn_bwd_kernel<64>, grid, kBwdThreads, BwdCfg<64>::kSmem, stream, tq, tk, tv, tdo, tdq, p);
   else
     launch(attn_bwd_kernel<128>, grid, kBwdThreads, BwdCfg<128>::kSmem, stream, tq, tk, tv, tdo, tdq, p);
+  if (rope_pos != nullptr) {
+    const auto kernel = head_dim == 64 ? finish_rope_grads_kernel<64> : finish_rope_grads_kernel<128>;
+    launch(kernel, (total_tokens + kFinishTokens - 1) / kFinishTokens, 256, 0, stream, static_cast<const float*>(dq_acc),
+           static_cast<__nv_bfloat16*>(dq), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), total_tokens, n_q, n_kv,
+           dq_stride, dkv_stride, scale, static_cast<const float*>(kv_parts), p.parts, rope_pos, log2f(rope_theta));
+    return cudaGetLastError();
+  }
   const long long n8 = static_cast<long long>(total_tokens) * n_q * head_dim / 8;
   const long long kv_n8 = static_cast<long long>(total_tokens) * n_kv * head_dim / 8;
   long long g = (n8 + (p.parts > 1 ? 2 * kv_n8 : 0) + 255) / 256;

@@ -8,6 +8,7 @@
 
 #include "api.h"
 #include "launch.cuh"
+#include "odc_device.cuh"
 
 namespace odc {
 namespace {
@@ -319,9 +320,7 @@ rope_qkv_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, const long 
     unpack8(b, x2);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float c = cs[j + i], s = cs[half + j + i];
-      o1[i] = x1[i] * c - x2[i] * s;
-      o2[i] = x2[i] * c + x1[i] * s;
+      rotate_pair(x1[i], x2[i], cs[j + i], cs[half + j + i], &o1[i], &o2[i]);
     }
     *reinterpret_cast<uint4*>(orow + h * head_dim + j) = pack8(o1);
     *reinterpret_cast<uint4*>(orow + h * head_dim + half + j) = pack8(o2);

@@ -24,7 +24,9 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "api.h"
 #include "launch.cuh"
@@ -42,7 +44,7 @@ constexpr int kATile = BMH * BK * 2;                     // 16 KiB
 constexpr int kBTile = BNH * BK * 2;                     // 16 KiB
 constexpr int kStageBytes = kATile + kBTile;             // 32 KiB per CTA
 constexpr int kStagingBytes = 128 * 128;
-constexpr int kSmemBytes = kStages * kStageBytes + 2 * kStagingBytes + 1024 + 512;
+constexpr int kSmemBytes = kStages * kStageBytes + 2 * kStagingBytes + 1024 + 768;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint64_t kWaitBudgetNs = 4000000000ull;
 constexpr int kThreads = 192;
@@ -79,6 +81,10 @@ struct Params {
   float* label_logits;         // [M]
   float inv_temp;
   int store_logits;
+  // kModeRope: the columns below rot_cols are heads of head_dim, rotated by the row's position
+  const long long* pos;        // [M]
+  int rot_cols, head_dim;
+  float log2_theta;
   int w_rows, w_cols;          // gathered matrix: [N, K] when B is K-major (y = x W^T), [K, N] when MN-major (dx = dy W)
   // Rotation of the work order by this rank's position in the group.  Without it every rank would pull the first
   // owner's rows first (and push into the first owner's accumulator first): one GPU's links saturated, seven idle.
@@ -97,7 +103,7 @@ struct Params {
 // bf16, as the pass that forms the gradient reads them.  The arithmetic (one exponential per logit) runs under the next tile's
 // products, where these are long enough (logits_stats_pay).  Log-probabilities of 6000 tokens, 151936 words, 1536 wide, forward and backward: 9.62 ms, now 8.99; forward only,
 // 16321 tokens, 128256 words: four passes of 0.24 ms and as many writes of the logits less (36.6 -> 35.3 ms with the decoder).
-constexpr int kModePlain = 0, kModeScatter = 1, kModeGather = 2, kModeSwiglu = 3, kModeLogits = 4, kModeSwigluBwd = 5, kModeGroup = 6;
+constexpr int kModePlain = 0, kModeScatter = 1, kModeGather = 2, kModeSwiglu = 3, kModeLogits = 4, kModeSwigluBwd = 5, kModeGroup = 6, kModeRope = 7;
 // kModeSwigluBwd (N = F): the product is the gradient of the activations; the epilogue turns it, rounded to bf16, with the
 // projection [M, 2F] (tensor map c) into the projection's gradient (owners.m[0] / [1]: its halves).  A warp of its own brings
 // boxes of gate and up into two buffers, for which the ring gives up a stage.  Forward and backward of a layer, both forms in
@@ -205,6 +211,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* part_last = abort_flag + 1;
   volatile int* item_slots = part_last + 1;                 // [kItemSlots]
+  float* rope_freq = reinterpret_cast<float*>(const_cast<int*>(item_slots) + kItemSlots);   // [64]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -261,6 +268,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       prefetch_tmap(&owners.b[lane]);
       prefetch_tmap(&owners.c[lane]);
     }
+  }
+  if constexpr (kMode == kModeRope) {
+    if (threadIdx.x >= 128 && threadIdx.x < 128 + p.head_dim / 2)
+      rope_freq[threadIdx.x - 128] = exp2f(-p.log2_theta * (2.0f * (threadIdx.x - 128)) / p.head_dim);
   }
   if (warp == 1) {
     tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
@@ -648,7 +659,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const int row = m0 + my_row;
       [[maybe_unused]] const bool row_ok = row < p.M;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
-      if constexpr (kMode == kModeSwiglu || kMode == kModeLogits || kMode == kModeSwigluBwd || kMode == kModeGroup) {
+      if constexpr (kMode == kModeSwiglu || kMode == kModeLogits || kMode == kModeSwigluBwd || kMode == kModeGroup || kMode == kModeRope) {
         // one staged box of 64 bf16 columns, or 32 of fp32: 32 registers per row
         auto emit = [&](const uint32_t* v32, const CUtensorMap* map, int col0, bool add = false) -> bool {
           auto send = [&](uint32_t src) {
@@ -684,7 +695,72 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           ++box_ctr;
           return true;
         };
-        if constexpr (kMode == kModeGroup) {
+        if constexpr (kMode == kModeRope) {
+          const int cols = m0 >= p.M ? 0 : min(BN, p.N - n0);
+          const float at = row_ok ? static_cast<float>(p.pos[row]) : 0.f;
+          const __nv_bfloat16* bias = p.bias != nullptr ? p.bias + n0 : nullptr;
+          auto read16 = [&](int col, float* x) {   // 16 columns of this row, with their bias
+            uint32_t r[16];
+            tmem_ld_32x16(t_row + col, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]);
+            if (bias != nullptr) {
+#pragma unroll
+              for (int v = 0; v < 2; ++v) {
+                const uint4 u = *reinterpret_cast<const uint4*>(bias + col + 8 * v);
+                const uint32_t b4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) { x[8 * v + 2 * i] += lo(b4[i]); x[8 * v + 2 * i + 1] += hi(b4[i]); }
+              }
+            }
+          };
+          auto rounded = [](float x) { return __bfloat162float(__float2bfloat16(x)); };
+          // one head: halves of kHalf columns, packed next to one another
+          auto head = [&](auto half, int col, uint32_t* v) {
+            constexpr int kHalf = decltype(half)::value;
+#pragma unroll
+            for (int c = 0; c < kHalf; c += 16) {
+              float a[16], b[16];
+              read16(col + c, a);
+              read16(col + kHalf + c, b);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                float sn, cn;
+                sincosf(at * rope_freq[c + i], &sn, &cn);
+                rotate_pair(rounded(a[i]), rounded(b[i]), cn, sn, &a[i], &b[i]);   // as the stand-alone pass reads them
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                v[c / 2 + i] = pack2(a[2 * i], a[2 * i + 1]);
+                v[(kHalf + c) / 2 + i] = pack2(b[2 * i], b[2 * i + 1]);
+              }
+            }
+          };
+#pragma unroll 1
+          for (int col = 0; col < cols && ok;) {
+            uint32_t v[64];
+            if (n0 + col >= p.rot_cols) {   // v heads
+#pragma unroll
+              for (int c = 0; c < 64; c += 16) {
+                float a[16];
+                read16(col + c, a);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[c / 2 + i] = pack2(a[2 * i], a[2 * i + 1]);
+              }
+              ok = emit(v, &tmap_c, n0 + col);
+              col += 64;
+            } else if (p.head_dim == 64) {
+              head(std::integral_constant<int, 32>{}, col, v);
+              ok = emit(v, &tmap_c, n0 + col);
+              col += 64;
+            } else {
+              head(std::integral_constant<int, 64>{}, col, v);
+              ok = emit(v, &tmap_c, n0 + col) && emit(v + 32, &tmap_c, n0 + col + 64);
+              col += 128;
+            }
+          }
+        } else if constexpr (kMode == kModeGroup) {
           const GroupProblem& q = owners.prob[place.pi];
           const CUtensorMap* map = &owners.c[place.pi];
           const int cols = m0 >= q.M ? 0 : min(BN, q.N - n0);
@@ -1242,6 +1318,43 @@ cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* 
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
   launch(gemm_bf16_pair_kernel<kModeSwiglu>, 2 * pairs, kThreads, kSmemBytes, stream, ta, tb, tc, halves, p);
+  return cudaGetLastError();
+}
+
+// out[M, N] = x w^T (+ bias), w [N, K], with the columns below rot_cols, heads of 64 or 128, rotated by pos[row] (rotary base theta;
+// halves of a head are the pairs, as in launch_rope_qkv): the rotation is not a pass over the projection (16321 tokens, 32 + 16
+// heads of 64: 45 us), and runs while the next tile is multiplied.  The same bytes as the two passes: rounded, rotated, rounded.
+// cudaErrorNotSupported where the plain product and the pass are the better form.
+cudaError_t gemm_rope_pair(const void* x, const void* w, const void* bias, void* out, const long long* pos, int M, int N, int K,
+                           long long ldx, long long ldw, int rot_cols, int head_dim, float theta, int* status, int sm_count,
+                           cudaStream_t stream) {
+  using namespace gemm_pair;
+  if (M < 256 || N < 256 || K < BK || sm_count < 2 || plan_splits(M, N, K, sm_count, kPartialsCost, false).splits > 1)
+    return cudaErrorNotSupported;
+  if ((head_dim != 64 && head_dim != 128) || rot_cols % head_dim || N % 64 || rot_cols > N || (ldx % 8) || (ldw % 8) ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out) |
+        reinterpret_cast<uintptr_t>(bias)) & 15))
+    return cudaErrorNotSupported;
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  std::call_once(once, [] {
+    attr_err = cudaFuncSetAttribute(gemm_bf16_pair_kernel<kModeRope>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  });
+  if (attr_err != cudaSuccess) return attr_err;
+  CUtensorMap ta, tb, tc;
+  if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, N, ldw * 2, 64, BNH) ||
+      !encode_tile_map_2d(&tc, out, N, M, static_cast<uint64_t>(N) * 2, 64, BMH))
+    return cudaErrorNotSupported;
+  Params p{};
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.M = M; p.N = N; p.K = K;
+  p.pos = pos; p.rot_cols = rot_cols; p.head_dim = head_dim; p.log2_theta = log2f(theta);
+  p.tiles_m = (M + 255) / 256;
+  p.tiles_n = (N + BN - 1) / BN;
+  p.status = status;
+  const int tiles = p.tiles_m * p.tiles_n;
+  const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
+  launch(gemm_bf16_pair_kernel<kModeRope>, 2 * pairs, kThreads, kSmemBytes, stream, ta, tb, tc, OwnerMaps{}, p);
   return cudaGetLastError();
 }
 

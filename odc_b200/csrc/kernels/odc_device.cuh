@@ -119,4 +119,10 @@ __device__ __forceinline__ bool grid_barrier_bounded(unsigned int* counter, unsi
   return ok_flag != 0;
 }
 
+// One pair of a rotary embedding, with the operations spelled out: every kernel that rotates gives the same bytes.
+__device__ __forceinline__ void rotate_pair(float x1, float x2, float cos, float sin, float* y1, float* y2) {
+  *y1 = __fmaf_rn(x1, cos, -__fmul_rn(x2, sin));
+  *y2 = __fmaf_rn(x2, cos, __fmul_rn(x1, sin));
+}
+
 }  // namespace odc

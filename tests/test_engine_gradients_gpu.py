@@ -265,8 +265,8 @@ def test_layers_of_the_mlp_are_called_where_somebody_stands_between(form, name):
 @pytest.mark.parametrize("name,tokens", [("llama3.2-1b", [5, 128, 77]), ("qwen2.5-1.5b", [300, 64]), ("tiny", [1])])
 @pytest.mark.parametrize("grad", [True, False])
 def test_a_layer_as_one_function_is_its_parts(name, tokens, grad):
-    """Same kernels on the same operands: the same bytes forward; backward the additions of the norms' and the queries' gradients
-    come in any order (fp32, then rounded to bf16: 2^-8 of what a flipped rounding moves, far less in the norm)."""
+    """The same roundings: the same bytes forward; backward the additions of the norms' and the queries' gradients come in any
+    order (fp32, then rounded to bf16: 2^-8 of what a flipped rounding moves, far less in the norm)."""
     from odc_b200 import ops
     from odc_b200.models import DecoderLayer, get_config
     cfg = get_config(name)

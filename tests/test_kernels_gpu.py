@@ -603,6 +603,25 @@ def test_single_cta_products_allocate_and_count_nothing_for_a_division():
     assert r.returncode == 0, r.stderr
 
 
+def _linear(x, w, b):
+    from odc_b200 import ops
+    with torch.no_grad():
+        return ops.linear(x, w, b)
+
+
+@pytest.mark.parametrize("T,H,nq,nkv,d,bias", [(256, 64, 2, 1, 64, False), (300, 264, 5, 1, 64, True), (1000, 512, 8, 2, 64, False),
+                                               (256, 128, 1, 1, 128, True), (520, 200, 12, 2, 128, True), (16, 128, 4, 4, 64, True),
+                                               (300, 8960, 4, 1, 128, False), (2600, 2048, 32, 8, 64, False)])
+def test_projection_with_rotation(ext, T, H, nq, nkv, d, bias):
+    """The bytes of the product and the pass over it.  Fewer rows than a tile and divided products take those."""
+    torch.manual_seed(0)
+    x, w = torch.randn(T, H, device="cuda").bfloat16(), (torch.randn((nq + 2 * nkv) * d, H, device="cuda") * H ** -0.5).bfloat16()
+    b = torch.randn(w.shape[0], device="cuda").bfloat16() if bias else None
+    pos = torch.arange(T, device="cuda") % 777 * 3
+    out = ext.linear_rope(x, w, b, pos, nq, nkv, d, 10000.0)
+    assert torch.equal(out, ext.rope_qkv(_linear(x, w, b), pos, nq, nkv, d, 10000.0, False))
+
+
 @pytest.mark.parametrize("T,K,F", [(256, 128, 128), (300, 264, 1000), (520, 2048, 136), (1000, 512, 4160), (16, 128, 256),
                                    (765, 17920, 768)])
 def test_linear_swiglu_matches_the_two_passes(ext, T, K, F):
