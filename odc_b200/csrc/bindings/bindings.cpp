@@ -2,6 +2,8 @@
 // stream out to the launchers in kernels/api.h.  The decoder's differentiable ops are in ops.cpp.
 #include "ops.h"
 
+#include <atomic>
+#include <chrono>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -295,8 +297,8 @@ void post_counts(std::vector<int64_t> slot_addrs, std::vector<int64_t> counts, i
   check(odc::launch_post_counts(posted(slot_addrs, counts, epoch), cur_stream()), "post_counts launch");
 }
 
-// post_counts + wait_posted in one launch, then the current stream is synchronised; returns {code, detail, observed} of
-// the device's status word
+// post_counts + wait_posted in one launch; returns {code, detail, observed} of the device's status word once all that was queued on
+// the current stream before, and the waits, are done
 std::tuple<int, int, int> post_and_wait(std::vector<int64_t> slot_addrs, std::vector<int64_t> counts, int64_t epoch, Tensor slots,
                                         int64_t nprod, Tensor counter, int64_t timeout_ms, Tensor status, Tensor status_host) {
   c10::cuda::CUDAGuard g(counter.device());
@@ -304,21 +306,36 @@ std::tuple<int, int, int> post_and_wait(std::vector<int64_t> slot_addrs, std::ve
   TORCH_CHECK(slots.scalar_type() == at::kLong && slots.numel() >= nprod, "post_and_wait: int64 slots, one per producer");
   TORCH_CHECK(status_host.scalar_type() == at::kInt && status_host.numel() >= 4 && status_host.is_pinned(),
               "post_and_wait: four pinned ints");
-  int* host = status_host.data_ptr<int>();
-  int* mapped = nullptr;
-  check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&mapped), host, 0), "post_and_wait: status buffer");
+  auto* word = reinterpret_cast<volatile unsigned long long*>(status_host.data_ptr<int>());
+  unsigned long long* mapped = nullptr;
+  check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&mapped), status_host.data_ptr<int>(), 0), "post_and_wait: status buffer");
   const cudaStream_t stream = cur_stream();
+  *word = 0;
   check(odc::launch_post_and_wait(posted(slot_addrs, counts, epoch), slots.data_ptr(), static_cast<int>(nprod),
                                   static_cast<unsigned long long>(epoch), counter.data_ptr(),
                                   static_cast<unsigned long long>(timeout_ms) * 1000000ull, status.data_ptr<int>(), mapped, stream),
         "post_and_wait launch");
-  cudaError_t e;
+  const unsigned long long done = static_cast<unsigned long long>(epoch) << 8;
+  cudaError_t e = cudaSuccess;
+  int seen[4] = {0, 0, 0, 0};
   {
     py::gil_scoped_release nogil;
-    e = cudaStreamSynchronize(stream);
+    // The word is there some microseconds before the launch has retired and a synchronisation has returned.  A longer wait is the
+    // driver's, which also notices a stream that failed.
+    const auto t0 = std::chrono::steady_clock::now();
+    unsigned long long v = *word;
+    while (v != done && std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(200)) v = *word;
+    if (v != done) {
+      e = cudaStreamSynchronize(stream);
+      if (e == cudaSuccess && *word != done) {
+        e = cudaMemcpyAsync(seen, status.data_ptr<int>(), sizeof(seen), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+      }
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
   }
   check(e, "post_and_wait");
-  return {host[0], host[1], host[2]};
+  return {seen[0], seen[1], seen[2]};
 }
 
 void wait_posted(Tensor slots, int64_t nprod, int64_t epoch, Tensor counter, int64_t timeout_ms, Tensor status,

@@ -59,10 +59,10 @@ cudaError_t launch_post_counts(const PostedCounts& pc, cudaStream_t stream);
 cudaError_t launch_wait_posted(const void* slots, int nprod, unsigned long long epoch, const void* ctr,
                                unsigned long long budget_ns, int* status, unsigned long long* expected_out,
                                cudaStream_t stream);
-// Both in one launch: post to every owner, then wait; afterwards the status word is copied to status_host (four ints of
-// pinned host memory), so that the caller needs a stream synchronisation and no copy to look at it.
+// Both in one launch: post to every owner, then wait; then (epoch << 8) | status code is written to host_word (the device address of
+// pinned host memory), where the caller finds it without a copy or a synchronisation.
 cudaError_t launch_post_and_wait(const PostedCounts& pc, const void* slots, int nprod, unsigned long long epoch, const void* ctr,
-                                 unsigned long long budget_ns, int* status, int* status_host, cudaStream_t stream);
+                                 unsigned long long budget_ns, int* status, unsigned long long* host_word, cudaStream_t stream);
 
 // ---- single-primitive test kernels (device_prims.cu) ---------------------------------------------
 cudaError_t launch_put_block(void* remote_dst, const void* local_src, size_t bytes, cudaStream_t s);

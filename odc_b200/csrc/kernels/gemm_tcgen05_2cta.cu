@@ -1066,10 +1066,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     if (warp == 2 && elect_one()) {   // the thread that issued them
       bulk_commit_group();
       bulk_wait_group0();  // all output boxes are in memory
-      if constexpr (kMode == kModeScatter) __threadfence_system();
-      if constexpr (kMode == kModeGroup) {
-        if (owners.arrivals > 0) __threadfence_system();
-      }
     }
   }
 
@@ -1082,21 +1078,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     tmem_dealloc_pair(tmem_base, kTmemCols);
   }
   if constexpr (kMode == kModeScatter || kMode == kModeGroup) {
-    // the last CTA to finish releases one arrival on every owner's counter, unless any CTA of the launch gave up
+    // the last CTA to finish reports to every owner's counter, unless any CTA of the launch gave up
     unsigned long long arrivals = 1;
     if constexpr (kMode == kModeGroup) arrivals = owners.arrivals;
-    if (threadIdx.x == 0 && arrivals > 0) {
-      __threadfence_system();
-      const unsigned int prev = atomicAdd(p.done_slot, 1u);
-      if (prev == gridDim.x - 1) {
-        *p.done_slot = 0;
-        __threadfence_system();
-        const bool clean = !*abort_flag && (p.status == nullptr || *reinterpret_cast<volatile int*>(p.status) == 0);
-        if (clean)
-          for (int r = 0; r < p.nranks; ++r)
-            signal_add_release_sys(reinterpret_cast<unsigned long long*>(p.ctr_ptrs[r]), arrivals);
-      }
-    }
+    if (arrivals > 0)
+      finish_and_signal(p.ctr_ptrs, p.nranks, p.done_slot, arrivals,
+                        [&] { return !*abort_flag && (p.status == nullptr || *reinterpret_cast<volatile int*>(p.status) == 0); });
   }
 }
 

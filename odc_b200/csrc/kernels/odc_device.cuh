@@ -68,6 +68,35 @@ __device__ __forceinline__ void signal_add_release_sys(unsigned long long* p, un
   asm volatile("red.release.sys.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+__device__ __forceinline__ void signal_add_relaxed_sys(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.relaxed.sys.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// End of a launch that added to the owners' accumulators: when every CTA has come here, `arrivals` go to each owner's counter
+// (unless `ok` is false where the last one looks).  All threads of a CTA call it after their last addition.  The barrier puts a
+// CTA's additions before thread 0's fence, the counter theirs before the last CTA's, and one fence there stands for all owners.
+// With one rank the owner is this GPU, and so is whoever waits for the arrival: the fences need not reach beyond it.
+template <typename Ok>
+__device__ __forceinline__ void finish_and_signal(const long long* ctrs, int nranks, unsigned int* done_slot, unsigned long long arrivals,
+                                                  Ok ok) {
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const auto fence = [&] { if (nranks == 1) __threadfence(); else __threadfence_system(); };
+  fence();
+  if (gridDim.x > 1) {
+    if (atomicAdd(done_slot, 1u) != gridDim.x - 1) return;
+    *done_slot = 0;  // self-reset: the slot is reusable by a later launch
+    fence();
+  }
+  if (ok())
+    for (int p = 0; p < nranks; ++p) signal_add_relaxed_sys(reinterpret_cast<unsigned long long*>(ctrs[p]), arrivals);
+}
+
+__device__ __forceinline__ unsigned long long ld_relaxed_sys(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ unsigned long long ld_acquire_sys(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
