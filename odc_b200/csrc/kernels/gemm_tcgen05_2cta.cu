@@ -9,7 +9,7 @@
 //
 //   warp 0      : TMA producer of this CTA's halves; byte counts are reported to the leader's "full" barrier
 //   warp 1      : leader only: MMA issuer; completion is committed to BOTH CTAs' barriers (two commits, no multicast)
-//   warps 2..5  : epilogue of this CTA's 128 rows (tcgen05.ld -> bias / residual -> swizzled staging -> TMA store),
+//   warps 2..5  : epilogue of this CTA's 128 rows, 32 each (tcgen05.ld -> bias / residual -> swizzled staging -> TMA store),
 //                 then a (remote) arrive on the leader's "accumulator free" barrier
 // The issuing threads are elected with elect.sync: of a thread picked by its lane number the compiler does not know that it
 // is alone, and moves every descriptor to uniform registers by way of a loop, which the main loop then waits for (16321 x
@@ -44,6 +44,7 @@ constexpr int kATile = BMH * BK * 2;                     // 16 KiB
 constexpr int kBTile = BNH * BK * 2;                     // 16 KiB
 constexpr int kStageBytes = kATile + kBTile;             // 32 KiB per CTA
 constexpr int kStagingBytes = 128 * 128;
+constexpr int kOutRows = 32;                             // rows of an output box: those of one epilogue warp
 constexpr int kSmemBytes = kStages * kStageBytes + 2 * kStagingBytes + 1024 + 768;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint64_t kWaitBudgetNs = 4000000000ull;
@@ -130,8 +131,8 @@ struct OwnerMaps {   // one fp32 tensor map per owner's accumulator region (kMod
 // and 16 k-blocks on 74 pairs.  The items of the longest product come first and a pair takes the next one from a counter, so the
 // short ones fill what the long ones leave.  One by one / together, us: input and weight gradient of 1000 x 1536 x 2048 26.2 / 17.0,
 // of 1000 x 1536 x 1536 23.9 / 14.4, of 2000 x 512 x 512 (fp32 sum) 24.1 / 9.8; the three of an MLP over 2000 tokens, 512 and 1536
-// wide, 48.9 / 21.7, 300 tokens, 2048 and 8192 wide, 130 / 110, 1000 tokens, 1536 and 8960 wide, 112 / 109.  One product by itself
-// costs half a microsecond more than in kModePlain, and 0.5 us an item where items are short.
+// wide, 48.9 / 21.7, 300 tokens, 2048 and 8192 wide, 130 / 110, 1000 tokens, 1536 and 8960 wide, 109 / 104.  One product by itself
+// costs 0.7 us more than in kModePlain, and some 0.2 us an item where items are short.
 struct GroupProblem {
   int M, N, K, tiles_m, tiles_n;
   int a_mn, b_mn;
@@ -152,6 +153,8 @@ struct Group {
   unsigned int* next;       // items handed out so far beyond the first of every pair; zero before and after the launch
   int arrivals;             // contributions to report to ctr_ptrs[0] when all is added
 };
+__device__ __forceinline__ int owners_rows(const OwnerMaps&, int) { return 0; }
+__device__ __forceinline__ int owners_rows(const Group& g, int i) { return g.prob[i].M; }
 template <int kMode> struct Extra { using type = OwnerMaps; };
 template <> struct Extra<kModeGroup> { using type = Group; };
 constexpr uint32_t kItemSlots = 16;   // see the item loop
@@ -201,13 +204,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const uint32_t empty0 = full0 + 8 * kStages;              // [kStages]  per CTA: the MMAs have read this stage
   const uint32_t tfull0 = empty0 + 8 * kStages;             // [2]        per CTA: accumulator complete
   const uint32_t tempty0 = tfull0 + 16;                     // [2]        used in the leader: both epilogues drained it
-  const uint32_t sready0 = tempty0 + 16;                    // [2]
-  const uint32_t sfree0 = sready0 + 16;                     // [2]
-  const uint32_t lready0 = sfree0 + 16;                     // [8]        a box of the last tile is staged in the ring
-  const uint32_t gfull = lready0 + 64, gempty = gfull + 8;  // boxes of gate and up
+  const uint32_t gfull = tempty0 + 16, gempty = gfull + 8;  // boxes of gate and up
   const uint32_t islot0 = gempty + 8;                       // [kItemSlots] per CTA: an item is written down
   const uint32_t pready = islot0 + 8 * kItemSlots, pcounted = pready + 8;   // a part is in memory / has been counted
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 18 + kItemSlots + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 6 + kItemSlots + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* part_last = abort_flag + 1;
   volatile int* item_slots = part_last + 1;                 // [kItemSlots]
@@ -241,7 +241,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       prefetch_tmap(&tmap_b);
       prefetch_tmap(&tmap_c);
     }
-    for (int b = 0; b < 8; ++b) mbar_init(lready0 + 8 * b, 4);
     mbar_init(gfull, 1);
     mbar_init(gempty, 4);
     if constexpr (kMode == kModeGroup) {
@@ -256,8 +255,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     for (int a = 0; a < 2; ++a) {
       mbar_init(tfull0 + 8 * a, 1);
       mbar_init(tempty0 + 8 * a, 8);   // four epilogue warps in each CTA of the pair
-      mbar_init(sready0 + 8 * a, 4);
-      mbar_init(sfree0 + 8 * a, 1);
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -283,7 +280,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();   // the partner's barriers exist before anything is reported to them
+  cluster_sync_barriers();   // the partner's barriers exist before anything is reported to them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -307,7 +304,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     if (num_items <= num_pairs) return num_items;   // one each, nothing is written down
     const uint32_t slot = item_seq % kItemSlots, ph = (item_seq / kItemSlots) & 1;
     ++item_seq;
-    const int item = mbar_wait_cluster(islot0 + 8 * slot, ph, wc, 22) ? item_slots[slot] : num_items;
+    const bool there = cta == 0 ? mbar_wait(islot0 + 8 * slot, ph, wc, 22) : mbar_wait_cluster(islot0 + 8 * slot, ph, wc, 22);
+    const int item = there ? item_slots[slot] : num_items;
     return __shfl_sync(0xffffffffu, item, 0);   // the same in all lanes, also for the compiler
   };
   auto following = [&](int item) -> int {
@@ -344,9 +342,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           const uint32_t slot = item_seq++ % kItemSlots;
           if (lane == 0) {
             item_slots[slot] = next;
-            st_shared_cluster(mapa_shared(smem_u32(const_cast<int*>(item_slots + slot)), 1), next);
             mbar_arrive(islot0 + 8 * slot);
-            mbar_arrive_cluster(mapa_shared(islot0 + 8 * slot, 1));
+            st_async_arrive(mapa_shared(smem_u32(const_cast<int*>(item_slots + slot)), 1), next, mapa_shared(islot0 + 8 * slot, 1));
           }
           if (next < num_items) ahead = take();
         }
@@ -653,48 +650,65 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       const int n0 = tn * BN;
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
-      if (!(ok = mbar_wait(tfull0 + 8 * acc, acc_ph, wc, 14))) break;
-      tc_fence_after();
       const int my_row = quad * 32 + lane;
       const int row = m0 + my_row;
       [[maybe_unused]] const bool row_ok = row < p.M;
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
-      if constexpr (kMode == kModeSwiglu || kMode == kModeLogits || kMode == kModeSwigluBwd || kMode == kModeGroup || kMode == kModeRope) {
-        // one staged box of 64 bf16 columns, or 32 of fp32: 32 registers per row
-        auto emit = [&](const uint32_t* v32, const CUtensorMap* map, int col0, bool add = false) -> bool {
-          auto send = [&](uint32_t src) {
-            if (kMode == kModeGroup && add) tma_reduce_add_2d(map, src, col0, m0);
-            else tma_store_2d(map, src, col0, m0);
-          };
-          const int buf = static_cast<int>(box_ctr & 1u);
-          const uint32_t use = box_ctr >> 1;
-          if (!last && use >= 1 && !mbar_wait(sfree0 + 8 * buf, (use - 1) & 1, wc, 16)) return false;
-          uint8_t* srow = (last ? smem + last_boxes * kStagingBytes : staging + buf * kStagingBytes) + my_row * 128;
+      // the first `n` (a multiple of 8) of 64 values of a row, and their addition
+      [[maybe_unused]] auto load64 = [](const __nv_bfloat16* src, int n, uint4* v) {
 #pragma unroll
-          for (int v = 0; v < 8; ++v)
-            *reinterpret_cast<uint4*>(srow + ((v ^ (my_row & 7)) << 4)) =
-                make_uint4(v32[4 * v], v32[4 * v + 1], v32[4 * v + 2], v32[4 * v + 3]);
-          fence_proxy_async();
+        for (int i = 0; i < 8; ++i) v[i] = 8 * i < n ? *reinterpret_cast<const uint4*>(src + 8 * i) : make_uint4(0, 0, 0, 0);
+      };
+      [[maybe_unused]] auto add64 = [](uint32_t* r, const uint4* v) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t o[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            r[8 * i + 2 * k] = __float_as_uint(__uint_as_float(r[8 * i + 2 * k]) + lo(o[k]));
+            r[8 * i + 2 * k + 1] = __float_as_uint(__uint_as_float(r[8 * i + 2 * k + 1]) + hi(o[k]));
+          }
+        }
+      };
+      // the residual's first box is asked for while the products run (1000 x 1536 x 1536: 3 us more than without a residual, box by box)
+      [[maybe_unused]] const __nv_bfloat16* rrow = nullptr;
+      [[maybe_unused]] uint4 res[8];
+      if constexpr (kMode == kModePlain || kMode == kModeGather) {
+        if (p.residual != nullptr && !part && row_ok) rrow = p.residual + static_cast<long long>(row) * p.ldr + n0;
+        if (rrow != nullptr) load64(rrow, p.N - n0, res);
+      }
+      if (!(ok = mbar_wait(tfull0 + 8 * acc, acc_ph, wc, 14))) break;
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BN;
+      // A warp's 32 rows of one box, 64 columns of bf16 or 32 of fp32 (32 registers per row), are staged in shared memory of its own
+      // and handed to the TMA unit by the warp itself: no warp waits for another, as all four did at every box of 128 rows.  What
+      // a last epilogue waited for besides was the release of its accumulator to the other CTA (1500 clocks, and nobody takes it any
+      // more) and the residual and bias box by box.  From the first launch of a chain to the next, before and now: 1900 x 512 x 512
+      // 8.3 and 7.4 us, 1000 x 1536 x 1536 13.2 and 12.3, with a residual 16.1 and 13.7, with a bias 22.1 and 13.5; 16321 x 3072 x
+      // 2048 with a bias 167 and 133; fp32 sums of long rows 2 % slower (four times as many boxes; 16321 x 2048 x 2048: 101 and 104).
+      const bool rows_in = m0 + quad * 32 < (kMode == kModeGroup ? owners_rows(owners, place.pi) : p.M);
+      auto emit = [&](const uint32_t* v32, const CUtensorMap* map, int col0, int row0, bool add = false) {
+        uint8_t* slab = (last ? smem + last_boxes * kStagingBytes : staging + (box_ctr & 1u) * kStagingBytes) + quad * 4096;
+        if (!last && box_ctr >= 2) {   // the box before the last one has been read
+          if (elect_one()) bulk_wait_group_read1();
           __syncwarp();
-          if (last) {
-            if (lane == 0) mbar_arrive(lready0 + 8 * last_boxes);
-            if (warp == 2 && elect_one() && mbar_wait(lready0 + 8 * last_boxes, 0, wc, 18))
-              send(base + last_boxes * kStagingBytes);
-            ++last_boxes;
-            return true;
+        }
+        uint8_t* srow = slab + lane * 128;
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          *reinterpret_cast<uint4*>(srow + ((v ^ (lane & 7)) << 4)) =
+              make_uint4(v32[4 * v], v32[4 * v + 1], v32[4 * v + 2], v32[4 * v + 3]);
+        fence_proxy_async();
+        __syncwarp();
+        if (elect_one()) {
+          if (rows_in) {
+            if (add) tma_reduce_add_2d(map, smem_u32(slab), col0, row0 + quad * 32);
+            else tma_store_2d(map, smem_u32(slab), col0, row0 + quad * 32);
           }
-          if (lane == 0) mbar_arrive(sready0 + 8 * buf);
-          if (warp == 2 && elect_one() && mbar_wait(sready0 + 8 * buf, use & 1, wc, 17)) {
-            send(staging_u32 + buf * kStagingBytes);
-            bulk_commit_group();
-            if (box_ctr >= 1) {
-              bulk_wait_group_read1();
-              mbar_arrive(sfree0 + 8 * (buf ^ 1));
-            }
-          }
-          ++box_ctr;
-          return true;
-        };
+          bulk_commit_group();
+        }
+        if (last) ++last_boxes; else ++box_ctr;
+      };
+      if constexpr (kMode == kModeSwiglu || kMode == kModeLogits || kMode == kModeSwigluBwd || kMode == kModeGroup || kMode == kModeRope) {
         if constexpr (kMode == kModeRope) {
           const int cols = m0 >= p.M ? 0 : min(BN, p.N - n0);
           const float at = row_ok ? static_cast<float>(p.pos[row]) : 0.f;
@@ -738,7 +752,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             }
           };
 #pragma unroll 1
-          for (int col = 0; col < cols && ok;) {
+          for (int col = 0; col < cols;) {
             uint32_t v[64];
             if (n0 + col >= p.rot_cols) {   // v heads
 #pragma unroll
@@ -748,15 +762,16 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[c / 2 + i] = pack2(a[2 * i], a[2 * i + 1]);
               }
-              ok = emit(v, &tmap_c, n0 + col);
+              emit(v, &tmap_c, n0 + col, m0);
               col += 64;
             } else if (p.head_dim == 64) {
               head(std::integral_constant<int, 32>{}, col, v);
-              ok = emit(v, &tmap_c, n0 + col);
+              emit(v, &tmap_c, n0 + col, m0);
               col += 64;
             } else {
               head(std::integral_constant<int, 64>{}, col, v);
-              ok = emit(v, &tmap_c, n0 + col) && emit(v + 32, &tmap_c, n0 + col + 64);
+              emit(v, &tmap_c, n0 + col, m0);
+              emit(v + 32, &tmap_c, n0 + col + 64, m0);
               col += 128;
             }
           }
@@ -774,7 +789,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
               tmem_ld_wait();
 #pragma unroll
               for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * scale);
-              if (!(ok = emit(r, map, n0 + col, add))) break;
+              emit(r, map, n0 + col, m0, add);
             }
           } else {
             // A part: 16 bytes of 128 rows next to one another, so that a warp writes and reads whole lines.
@@ -845,7 +860,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 }
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-                if (!(ok = emit(v, map, n0 + col))) break;
+                emit(v, map, n0 + col, m0);
               }
             }
           }
@@ -887,8 +902,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
               g[i] = pack2(dg[0], dg[1]);
               u[i] = pack2(du[0], du[1]);
             }
-            if (!(ok = emit(g, &owners.m[0], n0 + bx * 64))) break;
-            if (!(ok = emit(u, &owners.m[1], n0 + bx * 64))) break;
+            emit(g, &owners.m[0], n0 + bx * 64, m0);
+            emit(u, &owners.m[1], n0 + bx * 64, m0);
           }
         } else if constexpr (kMode == kModeLogits) {
           const long long label = row_ok ? p.labels[row] - n0 : -1;
@@ -928,7 +943,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
               }
               p.label_logits[row] = x;
             }
-            if (p.store_logits && !(ok = emit(v, &tmap_c, n0 + bx * 64))) break;
+            if (p.store_logits) emit(v, &tmap_c, n0 + bx * 64, m0);
           }
           if (row_ok) p.row_stats[static_cast<long long>(tn) * p.M + row] = make_float2(m, s);
         } else {
@@ -950,8 +965,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           const int col0 = tn * BNH + bx * 64;
           if (col0 >= p.N || m0 >= p.M) continue;
           if (p.store_gate_up) {
-            if (!(ok = emit(gate, &owners.m[0], col0))) break;
-            if (!(ok = emit(up, &owners.m[1], col0))) break;
+            emit(gate, &owners.m[0], col0, m0);
+            emit(up, &owners.m[1], col0, m0);
           }
 #pragma unroll
           for (int i = 0; i < 32; ++i) {   // from the rounded halves, as the stand-alone pass reads them
@@ -959,113 +974,77 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             const float u0 = __uint_as_float(up[i] << 16), u1 = __uint_as_float(up[i] & 0xffff0000u);
             gate[i] = pack2(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1);
           }
-          if (!(ok = emit(gate, &tmap_c, col0))) break;
+          emit(gate, &tmap_c, col0, m0);
         }
         }
       } else {
-      const int cols_per_box = f32 ? 32 : 64;
-      // What the branches need is read before the loop, and bias and residual are off the path of a plain product: a box
-      // was staged 780 clocks after its accumulators were asked for with tests between its pieces, 300 without (765 x 1536
-      // x 1536: 15 us, now 13.2).
-      const int n_boxes = m0 >= p.M ? 0 : min(BN, p.N - n0 + cols_per_box - 1) / cols_per_box;
-      const __nv_bfloat16* bias = part ? nullptr : p.bias;
-      const __nv_bfloat16* rrow =
-          (p.residual != nullptr && !part && row_ok) ? p.residual + static_cast<long long>(row) * p.ldr + n0 : nullptr;
-#pragma unroll 1
-      for (int bx = 0; bx < n_boxes; ++bx) {
-        uint32_t r[64];
-        tmem_ld_32x32(t_row + bx * cols_per_box, r);
-        if (!f32) tmem_ld_32x32(t_row + bx * cols_per_box + 32, r + 32);
-        tmem_ld_wait();
-        const int col0 = n0 + bx * cols_per_box;
-        if constexpr (kMode == kModeScatter) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * p.scale);
-        }
-        if (bias != nullptr) {
-#pragma unroll
-          for (int i = 0; i < 64; ++i)
-            if (i < cols_per_box && col0 + i < p.N)
-              r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(bias[col0 + i]));
-        }
-        const int buf = static_cast<int>(box_ctr & 1u);
-        const uint32_t use = box_ctr >> 1;
-        if (!last && use >= 1) {
-          if (!(ok = mbar_wait(sfree0 + 8 * buf, (use - 1) & 1, wc, 16))) break;
-        }
-        uint8_t* srow = (last ? smem + last_boxes * kStagingBytes : staging + buf * kStagingBytes) + my_row * 128;
+        const int cols = m0 >= p.M ? 0 : min(BN, p.N - n0);
+        const __nv_bfloat16* bias = part ? nullptr : p.bias;   // the sum of the parts adds it
         if (f32) {
+          // a CTA's 128 rows never straddle two owners (rows_per_rank is a multiple of 128)
+          const int owner = kMode == kModeScatter ? m0 / p.rows_per_rank : 0;
+          const CUtensorMap* map = kMode == kModeScatter || part ? &owners.m[owner] : &tmap_c;
+          const int row0 = kMode == kModeScatter ? m0 - owner * p.rows_per_rank
+                           : part ? (item - p.whole) * 256 + static_cast<int>(cta) * BMH : m0;
+          const int first_col = part ? 0 : n0;
+          const bool add = kMode == kModeScatter || (!part && p.accumulate);
+#pragma unroll 1
+          for (int col = 0; col < cols; col += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32(t_row + col, r);
+            tmem_ld_wait();
+            if constexpr (kMode == kModeScatter) {
 #pragma unroll
-          for (int v = 0; v < 8; ++v)
-            *reinterpret_cast<uint4*>(srow + ((v ^ (my_row & 7)) << 4)) =
-                make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * p.scale);
+            }
+            if (bias != nullptr) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (n0 + col + i < p.N) r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(bias[n0 + col + i]));
+            }
+            emit(r, map, first_col + col, row0, add);
+          }
+        } else if (bias == nullptr && p.residual == nullptr) {
+#pragma unroll 1
+          for (int col = 0; col < cols; col += 64) {
+            uint32_t r[64];
+            tmem_ld_32x32(t_row + col, r);
+            tmem_ld_32x32(t_row + col + 32, r + 32);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+            emit(r, &tmap_c, n0 + col, m0);
+          }
         } else {
-          if (rrow != nullptr) {
-            const int left = p.N - col0;   // a multiple of 8
-            uint4 res[8];
-#pragma unroll
-            for (int v = 0; v < 8; ++v)
-              res[v] = 8 * v < left ? *reinterpret_cast<const uint4*>(rrow + bx * 64 + 8 * v) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-              const uint32_t o[4] = {res[v].x, res[v].y, res[v].z, res[v].w};
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                r[8 * v + 2 * i] = __float_as_uint(__uint_as_float(r[8 * v + 2 * i]) + __uint_as_float(o[i] << 16));
-                r[8 * v + 2 * i + 1] = __float_as_uint(__uint_as_float(r[8 * v + 2 * i + 1]) + __uint_as_float(o[i] & 0xffff0000u));
-              }
+#pragma unroll 1
+          for (int col = 0; col < cols; col += 64) {
+            uint32_t r[64];
+            tmem_ld_32x32(t_row + col, r);
+            tmem_ld_32x32(t_row + col + 32, r + 32);
+            tmem_ld_wait();
+            if (bias != nullptr) {
+              uint4 b[8];
+              load64(bias + n0 + col, cols - col, b);
+              add64(r, b);
             }
-          }
-#pragma unroll
-          for (int v = 0; v < 8; ++v) {
-            const uint32_t* x = r + 8 * v;
-            auto two = [&](int i) { return pack2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])); };
-            *reinterpret_cast<uint4*>(srow + ((v ^ (my_row & 7)) << 4)) = make_uint4(two(0), two(2), two(4), two(6));
-          }
-        }
-        fence_proxy_async();
-        __syncwarp();
-        auto send = [&](uint32_t src) {
-          if constexpr (kMode == kModeScatter) {
-            // a CTA's 128 rows never straddle two owners (rows_per_rank is a multiple of 128)
-            const int owner = m0 / p.rows_per_rank;
-            tma_reduce_add_2d(&owners.m[owner], src, col0, m0 - owner * p.rows_per_rank);
-          } else if (part) {
-            tma_store_2d(&owners.m[0], src, bx * cols_per_box, (item - p.whole) * 256 + static_cast<int>(cta) * BMH);
-          } else if (p.accumulate) {
-            tma_reduce_add_2d(&tmap_c, src, col0, m0);
-          } else {
-            tma_store_2d(&tmap_c, src, col0, m0);
-          }
-        };
-        if (last) {
-          if (lane == 0) mbar_arrive(lready0 + 8 * last_boxes);
-          if (warp == 2 && elect_one() && mbar_wait(lready0 + 8 * last_boxes, 0, wc, 18)) send(base + last_boxes * kStagingBytes);
-          ++last_boxes;
-          continue;
-        }
-        if (lane == 0) mbar_arrive(sready0 + 8 * buf);
-        if (warp == 2 && elect_one()) {
-          if (mbar_wait(sready0 + 8 * buf, use & 1, wc, 17)) {
-            send(staging_u32 + buf * kStagingBytes);
-            bulk_commit_group();
-            if (box_ctr >= 1) {
-              bulk_wait_group_read1();
-              mbar_arrive(sfree0 + 8 * (buf ^ 1));
+            if (rrow != nullptr) {
+              add64(r, res);
+              load64(rrow + col + 64, cols - col - 64, res);   // of the next box, under the rest of this one
             }
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+            emit(r, &tmap_c, n0 + col, m0);
           }
         }
-        ++box_ctr;
-      }
       }
       if (!ok) break;
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(tempty_leader0 + 8 * acc);   // the leader may overwrite this accumulator
+      if (lane == 0 && !last) mbar_arrive_cluster_tmem(tempty_leader0 + 8 * acc);   // the leader may overwrite this accumulator
     }
-    if (warp == 2 && elect_one()) {   // the thread that issued them
-      bulk_commit_group();
-      bulk_wait_group0();  // all output boxes are in memory
+    if (elect_one()) {   // the thread that issued them: all output boxes have been read, or are in memory before an arrival is reported
+      if constexpr (kMode == kModeScatter || kMode == kModeGroup) bulk_wait_group0();
+      else bulk_wait_group_read0();
     }
   }
 
@@ -1236,12 +1215,12 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
   p.whole = plan.whole; p.splits = plan.splits; p.kb_split = plan.kb_split;
   OwnerMaps scratch{};
   const int parts = (p.tiles_m * p.tiles_n - p.whole) * p.splits;
-  if (parts > 0 && !encode_tile_map_2d_f32(&scratch.m[0], split_ws, BN, static_cast<uint64_t>(parts) * 256, BN * 4, 32, BMH))
+  if (parts > 0 && !encode_tile_map_2d_f32(&scratch.m[0], split_ws, BN, static_cast<uint64_t>(parts) * 256, BN * 4, 32, kOutRows))
     return cudaErrorInvalidValue;
   if (c_kind == kF32) {
-    if (!encode_tile_map_2d_f32(&tc, c, N, M, ldc * 4, 32, BMH)) return cudaErrorInvalidValue;
+    if (!encode_tile_map_2d_f32(&tc, c, N, M, ldc * 4, 32, kOutRows)) return cudaErrorInvalidValue;
   } else {
-    if (!encode_tile_map_2d(&tc, c, N, M, ldc * 2, 64, BMH)) return cudaErrorInvalidValue;
+    if (!encode_tile_map_2d(&tc, c, N, M, ldc * 2, 64, kOutRows)) return cudaErrorInvalidValue;
   }
   p.bias = static_cast<const __nv_bfloat16*>(bias);   // the sum of the parts adds it where there are any
   p.M = M; p.N = N; p.K = K;
@@ -1289,11 +1268,11 @@ cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* 
   OwnerMaps halves{};
   const uint64_t ld_gu = static_cast<uint64_t>(F) * 4;
   if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, 2ull * F, ldw * 2, 64, BNH) ||
-      !encode_tile_map_2d(&tc, act, F, M, static_cast<uint64_t>(F) * 2, 64, BMH))
+      !encode_tile_map_2d(&tc, act, F, M, static_cast<uint64_t>(F) * 2, 64, kOutRows))
     return cudaErrorInvalidValue;
   if (gate_up != nullptr) {  // each half clipped at its own last column
-    if (!encode_tile_map_2d(&halves.m[0], gate_up, F, M, ld_gu, 64, BMH) ||
-        !encode_tile_map_2d(&halves.m[1], static_cast<__nv_bfloat16*>(gate_up) + F, F, M, ld_gu, 64, BMH))
+    if (!encode_tile_map_2d(&halves.m[0], gate_up, F, M, ld_gu, 64, kOutRows) ||
+        !encode_tile_map_2d(&halves.m[1], static_cast<__nv_bfloat16*>(gate_up) + F, F, M, ld_gu, 64, kOutRows))
       return cudaErrorInvalidValue;
   }
   Params p{};
@@ -1330,7 +1309,7 @@ cudaError_t gemm_rope_pair(const void* x, const void* w, const void* bias, void*
   if (attr_err != cudaSuccess) return attr_err;
   CUtensorMap ta, tb, tc;
   if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, N, ldw * 2, 64, BNH) ||
-      !encode_tile_map_2d(&tc, out, N, M, static_cast<uint64_t>(N) * 2, 64, BMH))
+      !encode_tile_map_2d(&tc, out, N, M, static_cast<uint64_t>(N) * 2, 64, kOutRows))
     return cudaErrorNotSupported;
   Params p{};
   p.bias = static_cast<const __nv_bfloat16*>(bias);
@@ -1369,8 +1348,8 @@ cudaError_t gemm_swiglu_bwd_pair(const void* dy, const void* w, const void* gate
   const uint64_t ld_gu = static_cast<uint64_t>(F) * 4;
   if (!encode_tile_map_2d(&ta, dy, K, M, lddy * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, F, K, ldw * 2, 64, 64) ||
       !encode_tile_map_2d(&tc, gate_up, 2ull * F, M, ld_gu, 64, BMH) ||
-      !encode_tile_map_2d(&halves.m[0], dgate_up, F, M, ld_gu, 64, BMH) ||   // each half clipped at its own last column
-      !encode_tile_map_2d(&halves.m[1], static_cast<__nv_bfloat16*>(dgate_up) + F, F, M, ld_gu, 64, BMH))
+      !encode_tile_map_2d(&halves.m[0], dgate_up, F, M, ld_gu, 64, kOutRows) ||   // each half clipped at its own last column
+      !encode_tile_map_2d(&halves.m[1], static_cast<__nv_bfloat16*>(dgate_up) + F, F, M, ld_gu, 64, kOutRows))
     return cudaErrorNotSupported;
   Params p{};
   p.M = M; p.N = F; p.K = K;
@@ -1424,7 +1403,7 @@ cudaError_t gemm_logits_pair(const void* h, const void* w, void* logits, const l
   if (!encode_tile_map_2d(&ta, h, K, M, ldh * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, N, ldw * 2, 64, BNH))
     return cudaErrorNotSupported;
   tc = ta;
-  if (logits != nullptr && !encode_tile_map_2d(&tc, logits, N, M, ldl * 2, 64, BMH)) return cudaErrorNotSupported;
+  if (logits != nullptr && !encode_tile_map_2d(&tc, logits, N, M, ldl * 2, 64, kOutRows)) return cudaErrorNotSupported;
   Params p{};
   p.M = M; p.N = N; p.K = K;
   p.labels = labels;
@@ -1577,7 +1556,7 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long l
     const bool a_mn = q.layout == 2, b_mn = q.layout != 0;
     if (!(a_mn ? encode_tile_map_2d(&group.a[i], q.a, q.M, q.K, q.lda * 2, 64, 64) : encode_tile_map_2d(&group.a[i], q.a, q.K, q.M, q.lda * 2, 64, BMH)) ||
         !(b_mn ? encode_tile_map_2d(&group.b[i], q.b, q.N, q.K, q.ldb * 2, 64, 64) : encode_tile_map_2d(&group.b[i], q.b, q.K, q.N, q.ldb * 2, 64, BNH)) ||
-        !(q.c_kind == kF32 ? encode_tile_map_2d_f32(&group.c[i], q.c, q.N, q.M, q.ldc * 4, 32, BMH) : encode_tile_map_2d(&group.c[i], q.c, q.N, q.M, q.ldc * 2, 64, BMH)))
+        !(q.c_kind == kF32 ? encode_tile_map_2d_f32(&group.c[i], q.c, q.N, q.M, q.ldc * 4, 32, kOutRows) : encode_tile_map_2d(&group.c[i], q.c, q.N, q.M, q.ldc * 2, 64, kOutRows)))
       return cudaErrorInvalidValue;
     GroupProblem& t = group.prob[i];
     t.M = q.M; t.N = q.N; t.K = q.K;
@@ -1643,7 +1622,7 @@ cudaError_t gemm_wgrad_scatter_pair(const void* dy, const void* x, int tokens, i
   OwnerMaps owners{};
   for (int r = 0; r < nranks; ++r) {
     float* base = reinterpret_cast<float*>(static_cast<uintptr_t>(acc_addrs_host[r])) + acc_offset;
-    if (!encode_tile_map_2d_f32(&owners.m[r], base, k_in, rows_per_rank, static_cast<uint64_t>(k_in) * 4, 32, BMH))
+    if (!encode_tile_map_2d_f32(&owners.m[r], base, k_in, rows_per_rank, static_cast<uint64_t>(k_in) * 4, 32, kOutRows))
       return cudaErrorInvalidValue;
   }
   Params p{};
@@ -1695,7 +1674,7 @@ cudaError_t gemm_gather_pair(bool dgrad, const void* a, const long long* shard_p
   } else {  // B is MN-major: rows = reduction index, box {64 output columns, 64 reduction rows}
     if (!encode_tile_map_2d(&tb, w_local, w_cols, w_rows, static_cast<uint64_t>(w_cols) * 2, 64, 64)) return cudaErrorInvalidValue;
   }
-  if (!encode_tile_map_2d(&tc, out, N, M, ldo * 2, 64, BMH)) return cudaErrorInvalidValue;
+  if (!encode_tile_map_2d(&tc, out, N, M, ldo * 2, 64, kOutRows)) return cudaErrorInvalidValue;
   Params p{};
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.M = M; p.N = N; p.K = K;

@@ -225,17 +225,27 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// the same after fence.mbarrier_init: the barriers of all CTAs exist, and nothing else is published (a release waits some 1000
+// clocks for the memory system)
+__device__ __forceinline__ void cluster_sync_barriers() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // address of the same shared-memory location in CTA `rank` of this cluster (a shared::cluster address)
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void st_shared_cluster(uint32_t cluster_addr, int v) {
-  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+// one word into another CTA's shared memory, with the arrival on a barrier of that CTA that makes it visible there (a store and a
+// release across the cluster would wait some 1000 clocks for the memory system)
+__device__ __forceinline__ void st_async_arrive(uint32_t cluster_addr, int v, uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], 4;" ::"r"(cluster_bar) : "memory");
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(cluster_addr), "r"(v), "r"(cluster_bar)
+               : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// for what has been read from tensor memory, which the tcgen05 fences order: a release beyond this CTA would wait for its stores
+__device__ __forceinline__ void mbar_arrive_cluster_tmem(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // 2-D tile load into THIS CTA's shared memory whose byte count is reported to the barrier at shared::cluster address
 // `bar_cluster` (this CTA's or its pair partner's)
