@@ -669,6 +669,38 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           }
         }
       };
+      // The tile's bias is asked for while the products run, eight columns a lane, and passed around by shuffles.
+      [[maybe_unused]] uint4 bias8 = make_uint4(0, 0, 0, 0);
+      constexpr bool kBias = kMode == kModePlain || kMode == kModeGather || kMode == kModeRope;
+      [[maybe_unused]] const bool biased = kBias && p.bias != nullptr && !part;
+      if constexpr (kBias) {
+        if (biased && n0 + 8 * lane < p.N) bias8 = *reinterpret_cast<const uint4*>(p.bias + n0 + 8 * lane);
+      }
+      // its values of `kCols` columns from `col` on (multiples of 16), added to accumulators
+      [[maybe_unused]] auto add_bias = [&](auto n_cols, int col, auto* r) {
+        const uint32_t b4[4] = {bias8.x, bias8.y, bias8.z, bias8.w};
+#pragma unroll
+        for (int i = 0; i < decltype(n_cols)::value / 2; ++i) {
+          const uint32_t b = __shfl_sync(0xffffffffu, b4[i & 3], (col >> 3) + (i >> 2));
+          if constexpr (sizeof(r[0]) == sizeof(uint32_t) && std::is_integral_v<std::remove_reference_t<decltype(r[0])>>) {
+            r[2 * i] = __float_as_uint(__uint_as_float(r[2 * i]) + lo(b));
+            r[2 * i + 1] = __float_as_uint(__uint_as_float(r[2 * i + 1]) + hi(b));
+          } else {
+            r[2 * i] += lo(b);
+            r[2 * i + 1] += hi(b);
+          }
+        }
+      };
+      // The angles of a row's heads: those of narrow heads, four of which share a tile, are worked out while the products run (for
+      // wide ones there are not the registers, and a row of a tile has only two heads).
+      [[maybe_unused]] float at = 0.f, cosines[kMode == kModeRope ? 32 : 1], sines[kMode == kModeRope ? 32 : 1];
+      if constexpr (kMode == kModeRope) {
+        at = row_ok ? static_cast<float>(p.pos[row]) : 0.f;
+        if (p.head_dim == 64) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sincosf(at * rope_freq[i], &sines[i], &cosines[i]);
+        }
+      }
       // the residual's first box is asked for while the products run (1000 x 1536 x 1536: 3 us more than without a residual, box by box)
       [[maybe_unused]] const __nv_bfloat16* rrow = nullptr;
       [[maybe_unused]] uint4 res[8];
@@ -711,27 +743,17 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       if constexpr (kMode == kModeSwiglu || kMode == kModeLogits || kMode == kModeSwigluBwd || kMode == kModeGroup || kMode == kModeRope) {
         if constexpr (kMode == kModeRope) {
           const int cols = m0 >= p.M ? 0 : min(BN, p.N - n0);
-          const float at = row_ok ? static_cast<float>(p.pos[row]) : 0.f;
-          const __nv_bfloat16* bias = p.bias != nullptr ? p.bias + n0 : nullptr;
           auto read16 = [&](int col, float* x) {   // 16 columns of this row, with their bias
             uint32_t r[16];
             tmem_ld_32x16(t_row + col, r);
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]);
-            if (bias != nullptr) {
-#pragma unroll
-              for (int v = 0; v < 2; ++v) {
-                const uint4 u = *reinterpret_cast<const uint4*>(bias + col + 8 * v);
-                const uint32_t b4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { x[8 * v + 2 * i] += lo(b4[i]); x[8 * v + 2 * i + 1] += hi(b4[i]); }
-              }
-            }
+            if (biased) add_bias(std::integral_constant<int, 16>{}, col, x);
           };
           auto rounded = [](float x) { return __bfloat162float(__float2bfloat16(x)); };
-          // one head: halves of kHalf columns, packed next to one another
-          auto head = [&](auto half, int col, uint32_t* v) {
+          // one head: halves of kHalf columns, packed next to one another; `angle` gives cosine and sine
+          auto head = [&](auto half, int col, uint32_t* v, auto angle) {
             constexpr int kHalf = decltype(half)::value;
 #pragma unroll
             for (int c = 0; c < kHalf; c += 16) {
@@ -741,7 +763,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
               for (int i = 0; i < 16; ++i) {
                 float sn, cn;
-                sincosf(at * rope_freq[c + i], &sn, &cn);
+                angle(c + i, &sn, &cn);
                 rotate_pair(rounded(a[i]), rounded(b[i]), cn, sn, &a[i], &b[i]);   // as the stand-alone pass reads them
               }
 #pragma unroll
@@ -765,11 +787,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
               emit(v, &tmap_c, n0 + col, m0);
               col += 64;
             } else if (p.head_dim == 64) {
-              head(std::integral_constant<int, 32>{}, col, v);
+              head(std::integral_constant<int, 32>{}, col, v, [&](int i, float* sn, float* cn) { *sn = sines[i]; *cn = cosines[i]; });
               emit(v, &tmap_c, n0 + col, m0);
               col += 64;
             } else {
-              head(std::integral_constant<int, 64>{}, col, v);
+              head(std::integral_constant<int, 64>{}, col, v, [&](int i, float* sn, float* cn) { sincosf(at * rope_freq[i], sn, cn); });
               emit(v, &tmap_c, n0 + col, m0);
               emit(v + 32, &tmap_c, n0 + col + 64, m0);
               col += 128;
@@ -979,7 +1001,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
       } else {
         const int cols = m0 >= p.M ? 0 : min(BN, p.N - n0);
-        const __nv_bfloat16* bias = part ? nullptr : p.bias;   // the sum of the parts adds it
         if (f32) {
           // a CTA's 128 rows never straddle two owners (rows_per_rank is a multiple of 128)
           const int owner = kMode == kModeScatter ? m0 / p.rows_per_rank : 0;
@@ -997,14 +1018,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
               for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * p.scale);
             }
-            if (bias != nullptr) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (n0 + col + i < p.N) r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(bias[n0 + col + i]));
-            }
+            if (biased) add_bias(std::integral_constant<int, 32>{}, col, r);
             emit(r, map, first_col + col, row0, add);
           }
-        } else if (bias == nullptr && p.residual == nullptr) {
+        } else if (!biased && p.residual == nullptr) {
 #pragma unroll 1
           for (int col = 0; col < cols; col += 64) {
             uint32_t r[64];
@@ -1022,11 +1039,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             tmem_ld_32x32(t_row + col, r);
             tmem_ld_32x32(t_row + col + 32, r + 32);
             tmem_ld_wait();
-            if (bias != nullptr) {
-              uint4 b[8];
-              load64(bias + n0 + col, cols - col, b);
-              add64(r, b);
-            }
+            if (biased) add_bias(std::integral_constant<int, 64>{}, col, r);
             if (rrow != nullptr) {
               add64(r, res);
               load64(rrow + col + 64, cols - col - 64, res);   // of the next box, under the rest of this one
