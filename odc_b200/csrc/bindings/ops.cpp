@@ -1374,6 +1374,16 @@ void register_ops(py::module_& m) {
     const auto plan = odc::gemm_group_plan(g, n, sms);
     return std::vector<int>(plan.parts, plan.parts + n);
   }, py::arg("products"), py::arg("sms"));  // parts of every tile of each (M, N, K, fp32, accumulate)
+  m.def("gemm_group_columns", [](std::vector<std::tuple<int, int, int, bool, bool>> products, int sms) {
+    odc::GemmProduct g[odc::kMaxGroupProducts] = {};
+    int n = 0;
+    for (auto& [M, N, K, f32, accumulate] : products) {
+      TORCH_CHECK(n < odc::kMaxGroupProducts, "gemm_group_columns: too many products");
+      g[n].M = M; g[n].N = N; g[n].K = K; g[n].c_kind = f32 ? odc::kF32 : odc::kBF16; g[n].accumulate = accumulate; g[n++].scale = 1.f;
+    }
+    const auto plan = odc::gemm_group_plan(g, n, sms);
+    return std::vector<int>(plan.columns, plan.columns + n);
+  }, py::arg("products"), py::arg("sms"));  // columns of a tile of each
   m.def("scatter_plan", [](int n_out, int k_in, int tokens, int ranks, int sms) {
     const odc::GemmPlan p = odc::scatter_plan(n_out, k_in, tokens, ranks, sms);
     return std::make_tuple(p.tiles, p.whole, p.parts);

@@ -144,7 +144,8 @@ struct GemmProduct {
   float scale;
 };
 struct GemmGroupPlan {
-  int parts[kMaxGroupProducts];   // of every tile; 0: not taken as a group
+  int parts[kMaxGroupProducts];     // of every tile; 0: not taken as a group
+  int columns[kMaxGroupProducts];   // of a tile
 };
 GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count);
 size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count);

@@ -58,7 +58,8 @@ struct Params {
   int M, N, K;
   int c_is_f32, accumulate;
   int a_mn, b_mn;
-  int tiles_m, tiles_n;   // in units of the pair's 256 x 256 tile
+  int tiles_m, tiles_n;   // in units of the pair's 256 x 256 tile (256 x 128 in half-width ones)
+  int bn;                 // modes with tiles of either width: columns of a tile
   // kModePlain, kModeScatter: the first `whole` tiles are work items of their own; the k-blocks of every other are divided
   // over `splits` items, kb_split each.  In kModePlain item whole + i writes its fp32 partial tile at row 256 * i of a
   // 256-column scratch (owners.m[0])
@@ -135,7 +136,7 @@ struct OwnerMaps {   // one fp32 tensor map per owner's accumulator region (kMod
 // costs 0.7 us more than in kModePlain, and some 0.2 us an item where items are short.
 struct GroupProblem {
   int M, N, K, tiles_m, tiles_n;
-  int a_mn, b_mn;
+  int a_mn, b_mn, bn;
   int out;                  // 0: bf16, 1: fp32, 2: added to fp32
   float scale;              // of an fp32 result
   int first;                // its first item
@@ -219,6 +220,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const WaitCtx wc{abort_flag, p.status, kWaitBudgetNs};
 
   constexpr bool kDivides = kMode == kModePlain || kMode == kModeScatter;
+  const int bn = kMode == kModePlain || kMode == kModeRope ? p.bn : BN;   // of a group: its products'
   const int num_tiles = p.tiles_m * p.tiles_n;
   int num_items = kDivides ? p.whole + (num_tiles - p.whole) * p.splits : num_tiles;   // the parts of a tile are adjacent
   if constexpr (kMode == kModeGroup) num_items = owners.items;
@@ -349,8 +351,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
         const GroupProblem& q = owners.prob[w.pi];
         const CUtensorMap *map_a = &owners.a[w.pi], *map_b = &owners.b[w.pi];
-        const int a_mn = q.a_mn, b_mn = q.b_mn;
-        const int m0 = w.tm * 256 + static_cast<int>(cta) * BMH, n0 = w.tn * BN + static_cast<int>(cta) * BNH;
+        const int a_mn = q.a_mn, b_mn = q.b_mn, q_bn = q.bn;
+        const int m0 = w.tm * 256 + static_cast<int>(cta) * BMH, n0 = w.tn * q_bn + static_cast<int>(cta) * (q_bn / 2);
         bool ok = true;
         auto load = [&](int kb0, int kb1) {
           uint32_t step = it;
@@ -360,7 +362,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             if (!(ok = mbar_wait(empty0 + 8 * s, ph ^ 1, wc, 11))) break;
             const uint32_t sa = base + s * kStageBytes;
             const uint32_t sb = sa + kATile;
-            if (cta == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * kStageBytes);
+            if (cta == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * kATile + q_bn * BK * 2);
             const uint32_t bar = mapa_shared(full0 + 8 * s, 0);
             const int k0 = kb * BK;
             if (!a_mn) {
@@ -372,8 +374,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             if (!b_mn) {
               tma_load_2d_pair(sb, map_b, bar, k0, n0);
             } else {
-#pragma unroll
-              for (int i = 0; i < BNH / 64; ++i) tma_load_2d_pair(sb + i * 8192, map_b, bar, n0 + 64 * i, k0);
+              tma_load_2d_pair(sb, map_b, bar, n0, k0);
+              if (q_bn == BN) tma_load_2d_pair(sb + 8192, map_b, bar, n0 + 64, k0);
             }
           }
         };
@@ -404,7 +406,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           if (next < num_items) w_next = place_of(next);
           const GroupProblem& q = owners.prob[w.pi];
           const uint32_t acc = local_tile & 1, acc_ph = (local_tile >> 1) & 1;
-          const uint32_t idesc = make_idesc_bf16(256, 256, q.a_mn != 0, q.b_mn != 0);
+          const uint32_t idesc = make_idesc_bf16(256, q.bn, q.a_mn != 0, q.b_mn != 0);
           const uint32_t a_lbo = q.a_mn ? 8192u : 16u, b_lbo = q.b_mn ? 8192u : 16u;
           const uint64_t a_kstep = q.a_mn ? 128 : 2, b_kstep = q.b_mn ? 128 : 2;
           const uint32_t d_tmem = tmem_base + acc * BN;
@@ -485,7 +487,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         k_range(item, &kb0, &k_blocks);
         const int m0 = tm * 256 + static_cast<int>(cta) * BMH;   // this CTA's rows of A and C
         const int n0 = kMode == kModeSwiglu ? tn * BNH + static_cast<int>(cta) * p.N
-                                            : tn * BN + static_cast<int>(cta) * BNH;    // this CTA's rows of B
+                                            : tn * bn + static_cast<int>(cta) * (bn / 2);   // this CTA's rows of B
         if constexpr (kMode == kModeGather) {
           // B K-major (forward): the 256 weight rows this tile multiplies must have landed in local memory first
           if (!p.b_mn && !(ok = wait_group(tn))) break;
@@ -500,7 +502,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           if (!(ok = mbar_wait(empty0 + 8 * s, ph ^ 1, wc, 11))) break;
           const uint32_t sa = base + s * kStageBytes;
           const uint32_t sb = sa + kATile;
-          if (cta == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * kStageBytes);   // bytes of both CTAs
+          if (cta == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * kATile + bn * BK * 2);   // bytes of both CTAs
           const uint32_t bar = mapa_shared(full0 + 8 * s, 0);
           const int k0 = (p.rot_kb ? (kb + p.rot_kb) % k_blocks : kb) * BK;
           if (!p.a_mn) {
@@ -510,10 +512,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             for (int i = 0; i < BMH / 64; ++i) tma_load_2d_pair(sa + i * 8192, &tmap_a, bar, m0 + 64 * i, k0);
           }
           if (!p.b_mn) {
-            tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);                 // box {64 k, 128 rows}
+            tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);                 // box {64 k, 128 (64) rows}
           } else {
-#pragma unroll
-            for (int i = 0; i < BNH / 64; ++i) tma_load_2d_pair(sb + i * 8192, &tmap_b, bar, n0 + 64 * i, k0);
+            tma_load_2d_pair(sb, &tmap_b, bar, n0, k0);
+            if (bn == BN) tma_load_2d_pair(sb + 8192, &tmap_b, bar, n0 + 64, k0);
           }
         }
       }
@@ -521,7 +523,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
     if (cta == 0 && elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(256, 256, p.a_mn != 0, p.b_mn != 0);
+      const uint32_t idesc = make_idesc_bf16(256, bn, p.a_mn != 0, p.b_mn != 0);
       const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
       const uint64_t a_kstep = p.a_mn ? 128 : 2, b_kstep = p.b_mn ? 128 : 2;  // 16-byte units per K = 16
       uint32_t it = 0, local_tile = 0;
@@ -647,7 +649,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       // one before it to be read.
       const bool last = next_item >= num_items;
       const int m0 = tm * 256 + static_cast<int>(cta) * BMH;
-      const int n0 = tn * BN;
+      int tile_cols = bn;
+      if constexpr (kMode == kModeGroup) tile_cols = owners.prob[place.pi].bn;
+      const int n0 = tn * tile_cols;
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
       const int my_row = quad * 32 + lane;
@@ -742,7 +746,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       };
       if constexpr (kMode == kModeSwiglu || kMode == kModeLogits || kMode == kModeSwigluBwd || kMode == kModeGroup || kMode == kModeRope) {
         if constexpr (kMode == kModeRope) {
-          const int cols = m0 >= p.M ? 0 : min(BN, p.N - n0);
+          const int cols = m0 >= p.M ? 0 : min(tile_cols, p.N - n0);
           auto read16 = [&](int col, float* x) {   // 16 columns of this row, with their bias
             uint32_t r[16];
             tmem_ld_32x16(t_row + col, r);
@@ -800,7 +804,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         } else if constexpr (kMode == kModeGroup) {
           const GroupProblem& q = owners.prob[place.pi];
           const CUtensorMap* map = &owners.c[place.pi];
-          const int cols = m0 >= q.M ? 0 : min(BN, q.N - n0);
+          const int cols = m0 >= q.M ? 0 : min(tile_cols, q.N - n0);
           if (q.out != 0) {
             const float scale = q.scale;
             const bool add = q.out == 2;
@@ -1000,7 +1004,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
         }
       } else {
-        const int cols = m0 >= p.M ? 0 : min(BN, p.N - n0);
+        const int cols = m0 >= p.M ? 0 : min(tile_cols, p.N - n0);
         if (f32) {
           // a CTA's 128 rows never straddle two owners (rows_per_rank is a multiple of 128)
           const int owner = kMode == kModeScatter ? m0 / p.rows_per_rank : 0;
@@ -1172,6 +1176,15 @@ static SplitPlan plan_splits(int M, int N, int K, int sm_count, const SplitCost&
   return plan;
 }
 
+// Whether an undivided product is taken in tiles of 256 x 128: where twice as many still have a pair each.  A k-block of one takes
+// 0.7 of the time (its operands arrive no faster) and its epilogue half, so that two rounds of them are slower than one of whole
+// tiles.  256 and 128 columns, us: 300 x 512 x 512 7.0 and 6.1, 1000 x 1536 x 1536 12.3 and 10.3, 512 x 4096 x 4096 25.1 and 20.3,
+// rotated projections 1.3 times as fast; with two rounds of half tiles 1000 x 3072 x 2048 15.6 and 19.6, with three for two whole
+// ones 3000 x 2048 x 2048 25.6 and 28.6.
+static bool half_tiles_pay(int M, int N, int sm_count) {
+  return (M + 255) / 256 * ((N + 127) / 128) <= sm_count / 2;
+}
+
 // The plan of a bf16 product: all tiles divided where they are fewer than the pairs, else those of its last rounds.
 static SplitPlan product_plan(int M, int N, int K, int sm_count) {
   const SplitPlan all = plan_splits(M, N, K, sm_count, kPartialsCost, false);
@@ -1215,16 +1228,19 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
   } else {
     if (!encode_tile_map_2d(&ta, a, M, K, lda * 2, 64, 64)) return cudaErrorInvalidPitchValue;
   }
+  SplitPlan plan{(M + 255) / 256 * ((N + BN - 1) / BN), 1, 0};
+  if (split_ws != nullptr) plan = product_plan(M, N, K, sm_count);
+  const int bn = plan.splits == 1 && half_tiles_pay(M, N, sm_count) ? BN / 2 : BN;
   if (!b_mn) {
-    if (!encode_tile_map_2d(&tb, b, K, N, ldb * 2, 64, BNH)) return cudaErrorInvalidTexture;
+    if (!encode_tile_map_2d(&tb, b, K, N, ldb * 2, 64, bn / 2)) return cudaErrorInvalidTexture;
   } else {
     if (!encode_tile_map_2d(&tb, b, N, K, ldb * 2, 64, 64)) return cudaErrorInvalidTexture;
   }
   Params p{};
   p.tiles_m = (M + 255) / 256;
-  p.tiles_n = (N + BN - 1) / BN;
-  SplitPlan plan{p.tiles_m * p.tiles_n, 1, 0};
-  if (split_ws != nullptr) plan = product_plan(M, N, K, sm_count);
+  p.tiles_n = (N + bn - 1) / bn;
+  p.bn = bn;
+  if (plan.splits == 1) plan.whole = p.tiles_m * p.tiles_n;
   p.whole = plan.whole; p.splits = plan.splits; p.kb_split = plan.kb_split;
   OwnerMaps scratch{};
   const int parts = (p.tiles_m * p.tiles_n - p.whole) * p.splits;
@@ -1321,7 +1337,8 @@ cudaError_t gemm_rope_pair(const void* x, const void* w, const void* bias, void*
   });
   if (attr_err != cudaSuccess) return attr_err;
   CUtensorMap ta, tb, tc;
-  if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, N, ldw * 2, 64, BNH) ||
+  const int bn = half_tiles_pay(M, N, sm_count) ? BN / 2 : BN;   // a head is 128 columns at most
+  if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, N, ldw * 2, 64, bn / 2) ||
       !encode_tile_map_2d(&tc, out, N, M, static_cast<uint64_t>(N) * 2, 64, kOutRows))
     return cudaErrorNotSupported;
   Params p{};
@@ -1329,7 +1346,8 @@ cudaError_t gemm_rope_pair(const void* x, const void* w, const void* bias, void*
   p.M = M; p.N = N; p.K = K;
   p.pos = pos; p.rot_cols = rot_cols; p.head_dim = head_dim; p.log2_theta = log2f(theta);
   p.tiles_m = (M + 255) / 256;
-  p.tiles_n = (N + BN - 1) / BN;
+  p.tiles_n = (N + bn - 1) / bn;
+  p.bn = bn;
   p.status = status;
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
@@ -1455,14 +1473,18 @@ static unsigned int* group_words(int n) {
   return base[dev] + at - n;
 }
 
-// Into how many parts the tiles of each product are divided.  In units of a k-block (0.28 us): the items go to the pairs that are
-// free first, longest first, so the group takes the work per pair and half of its last item, but at least its longest item.  The
-// longest one is divided as long as that gains a twentieth.  An item takes at least what its epilogue does (6); a part of a bf16
-// tile writes and reads 256 KB of fp32 (3 each), the parts of an fp32 sum meet in memory.
+// How wide the tiles of each product are and into how many parts they are divided.  In units of a k-block (0.28 us): the items go to
+// the pairs that are free first, longest first, so the group takes the work per pair and half of its last item, but at least its
+// longest item, and a second round besides costs 6 (the items are handed on from CTA to CTA, the first epilogues are in the way).
+// An item takes at least what its epilogue does (6) and 2 to begin with; a part of a bf16 tile writes and reads 256 KB of fp32 (6),
+// the parts of an fp32 sum meet in memory.  The longest item is made half as wide, or divided, as long as that gains a twentieth.
+// 300 tokens, 1536 wide: half as wide 15.3 -> 12.5 us (projection), MLP of 512 and 1536 19.5 -> 15.4.
+constexpr double kHalfTile = 0.7;   // time of a k-block of a 256 x 128 tile (half_tiles_pay)
 struct GroupShape {
   int tiles, kb, splits, each;
   bool may_divide, bf16;
-  double item() const { return std::max(6, each) + (splits > 1 ? (bf16 ? 6.0 : 1.0) : 0.0); }
+  int bn, half_tiles;   // columns of a tile; how many tiles of half the width there are
+  double item() const { return std::max(6.0, each * (bn == 128 ? kHalfTile : 1.0)) + 2 + (splits > 1 ? (bf16 ? 6.0 : 1.0) : 0.0); }
   double sum() const { return bf16 && splits > 1 ? 12.0 + 8.0 * (splits - 1) : 0.0; }
 };
 static void plan_group(GroupShape* g, int n, int pairs) {
@@ -1471,13 +1493,16 @@ static void plan_group(GroupShape* g, int n, int pairs) {
     for (int i = 0; i < n; ++i) order[i] = i;
     std::sort(order, order + n, [&](int a, int b) { return g[a].item() > g[b].item(); });
     double work = 0, span = 0;
+    int all = 0;
     for (int i = 0; i < n; ++i) {
       const GroupShape& q = g[order[i]];
       const int items = q.tiles * q.splits;
       work += items * q.item();
-      span = std::max(span, (i == 0 ? (items + pairs - 1) / pairs * q.item() : work / pairs + 0.5 * q.item()) + q.sum());
+      all += items;
+      const double end = all <= pairs ? q.item() : i == 0 ? (items + pairs - 1) / pairs * q.item() : work / pairs + 0.5 * q.item();
+      span = std::max(span, end + q.sum());
     }
-    return span;
+    return span + (all > pairs ? 6.0 : 0.0);
   };
   for (int i = 0; i < n; ++i) { g[i].splits = 1; g[i].each = g[i].kb; }
   double best = cost();
@@ -1487,15 +1512,26 @@ static void plan_group(GroupShape* g, int n, int pairs) {
       if (g[i].item() > g[longest].item()) longest = i;
     GroupShape& q = g[longest];
     const GroupShape before = q;
-    bool found = false;
-    for (int want = before.splits + 1; want <= 8 && !found && q.may_divide; ++want) {
+    GroupShape better = before;
+    double least = 0.95 * best;
+    const auto consider = [&] {
+      if (const double c = cost(); c < least) { least = c; better = q; }
+      q = before;
+    };
+    if (q.bn == 256 && q.splits == 1) {   // no sum of parts
+      q.bn = 128;
+      q.tiles = q.half_tiles;
+      consider();
+    }
+    for (int want = before.splits + 1; want <= 8 && q.may_divide; ++want) {
       const int each = (q.kb + want - 1) / want, s = (q.kb + each - 1) / each;   // no empty part
       if (s <= before.splits || each < 4 || (q.bf16 && q.tiles > kMaxDivided)) continue;
       q.splits = s; q.each = each;
-      const double c = cost();
-      if (c < 0.95 * best) { best = c; found = true; } else { q = before; }
+      consider();
     }
-    if (!found) { q = before; return; }
+    if (better.bn == before.bn && better.splits == before.splits) return;
+    q = better;
+    best = least;
   }
 }
 
@@ -1506,7 +1542,8 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
     const GemmProduct& q = g[i];
     if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate || q.scale != 1.f))) return false;
     shapes[i] = GroupShape{(q.M + 255) / 256 * ((q.N + BN - 1) / BN), (q.K + BK - 1) / BK, 1, 0,
-                           q.c_kind == kBF16 || (q.accumulate && !q.fixed_order), q.c_kind == kBF16};
+                           q.c_kind == kBF16 || (q.accumulate && !q.fixed_order), q.c_kind == kBF16,
+                           BN, (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2))};
   }
   // A group saves the launches and last rounds of its products, 30 to 100 units.  With more work than this for a pair that is no
   // gain any more, and pairs that are not in step with one another share less of L2 (16321 tokens, 2048 and 8192 wide, 4400 units:
@@ -1537,7 +1574,7 @@ GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count) {
   GroupShape shapes[kMaxGroupProducts];
   GemmGroupPlan plan{};
   if (!group_shapes(g, n, sm_count, shapes)) return plan;
-  for (int i = 0; i < n; ++i) plan.parts[i] = shapes[i].splits;
+  for (int i = 0; i < n; ++i) { plan.parts[i] = shapes[i].splits; plan.columns[i] = shapes[i].bn; }
   return plan;
 }
 
@@ -1568,13 +1605,13 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long l
     const GroupShape& shape = shapes[order[i]];
     const bool a_mn = q.layout == 2, b_mn = q.layout != 0;
     if (!(a_mn ? encode_tile_map_2d(&group.a[i], q.a, q.M, q.K, q.lda * 2, 64, 64) : encode_tile_map_2d(&group.a[i], q.a, q.K, q.M, q.lda * 2, 64, BMH)) ||
-        !(b_mn ? encode_tile_map_2d(&group.b[i], q.b, q.N, q.K, q.ldb * 2, 64, 64) : encode_tile_map_2d(&group.b[i], q.b, q.K, q.N, q.ldb * 2, 64, BNH)) ||
+        !(b_mn ? encode_tile_map_2d(&group.b[i], q.b, q.N, q.K, q.ldb * 2, 64, 64) : encode_tile_map_2d(&group.b[i], q.b, q.K, q.N, q.ldb * 2, 64, shape.bn / 2)) ||
         !(q.c_kind == kF32 ? encode_tile_map_2d_f32(&group.c[i], q.c, q.N, q.M, q.ldc * 4, 32, kOutRows) : encode_tile_map_2d(&group.c[i], q.c, q.N, q.M, q.ldc * 2, 64, kOutRows)))
       return cudaErrorInvalidValue;
     GroupProblem& t = group.prob[i];
     t.M = q.M; t.N = q.N; t.K = q.K;
-    t.tiles_m = (q.M + 255) / 256; t.tiles_n = (q.N + BN - 1) / BN;
-    t.a_mn = a_mn; t.b_mn = b_mn;
+    t.tiles_m = (q.M + 255) / 256; t.tiles_n = (q.N + shape.bn - 1) / shape.bn;
+    t.a_mn = a_mn; t.b_mn = b_mn; t.bn = shape.bn;
     t.out = q.c_kind == kBF16 ? 0 : q.accumulate ? 2 : 1;
     t.scale = q.scale;
     t.first = group.items;

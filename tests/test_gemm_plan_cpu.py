@@ -74,6 +74,13 @@ def test_groups_divide_what_would_outlast_them(T, H, F):
             assert parts == [1, 1, 1]
 
 
+def test_groups_halve_the_tiles_of_what_would_outlast_them():
+    columns = lambda *g: _ext.load().gemm_group_columns(list(g), SMS)
+    assert columns((300, 1536, 2048, False, False), (2048, 1536, 300, False, False)) == [128, 256]
+    assert columns((16321, 2048, 3072, False, False), (3072, 2048, 16321, True, True)) == [256, 256]
+    assert columns((1000, 1536, 2048, False, False), (2048, 1536, 1000, False, False)) == [256, 256]   # a second round of items
+
+
 def test_statistics_in_the_product_where_they_pay():
     plan = lambda rows, words, width, gradient: _ext.load().head_plan(rows, words, width, gradient, SMS)
     for gradient in (False, True):

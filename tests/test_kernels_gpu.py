@@ -337,6 +337,20 @@ def test_gemm_cta_pair_layouts(ext, layout, M, N, K):
 
 
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("M,N,K", [(512, 4736, 72), (512, 4744, 72), (264, 376, 136), (256, 264, 64), (776, 392, 1600)])
+def test_gemm_tiles_of_half_the_width(ext, layout, M, N, K):
+    """37 x 2 tiles of 256 x 128 have a pair each and are taken, 38 x 2 are not; edges in the last half tile.  Against 64 bits, with
+    bias and residual: fp32 sums (2e-6 of the magnitudes) and one rounding to bf16."""
+    for a, b, c, lay, _, _, want, bound in _group_case([(layout, M, N, K, torch.bfloat16, False, 1.0)]):
+        bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+        ext.gemm(a, b, c, lay, None, False, None, 1)
+        assert ((c.double() - want).abs() <= bound).all()
+        full = want + bias.double() + res.double()
+        ext.gemm(a, b, c, lay, bias, False, res, 1)
+        assert ((c.double() - full).abs() <= bound + 2e-6 * (bias.double().abs() + res.double().abs()) + full.abs() * 2.0 ** -8).all()
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K,divided", [(8, 256, 4096, True), (136, 1536, 8968, True), (255, 2048, 2048, False),
                                            (256, 256, 2048, True), (264, 264, 4040, True), (765, 1536, 17920, True),
                                            (520, 1544, 8968, True), (768, 2048, 1536, False), (2304, 2304, 4096, False)])
@@ -440,6 +454,9 @@ def _group_case(products, seed=0):
     (None, [("nn", 1000, 1536, 4096, torch.bfloat16, False, 1.0), ("tn", 4096, 1536, 1000, torch.float32, True, 1.0),
             ("tn", 1536, 2048, 1000, torch.bfloat16, False, 1.0)]),
     (None, [("nn", 64, 256, 5000, torch.bfloat16, False, 1.0)]),
+    # tiles of half the width next to whole ones
+    ([1, 1], [("nn", 300, 392, 2048, torch.bfloat16, False, 1.0), ("tn", 2048, 392, 304, torch.float32, True, 1.0)]),
+    (None, [("nt", 300, 1160, 1024, torch.float32, False, 1.0), ("nn", 264, 264, 512, torch.bfloat16, False, 1.0)]),
 ])
 def test_groups_of_products(ext, parts, products):
     ops = _group_case(products)
