@@ -270,7 +270,8 @@ struct Product {
   Tensor a, b, c;
   int lay;
   bool accumulate = false;
-  double scale = 1.0;   // with an arrival (products_into) only
+  double scale = 1.0;    // group_into only: of the result
+  Tensor times;          // group_into only: a further factor, one fp32 value on the device
 };
 bool fixed_order_asked() {
   const char* e = std::getenv("ODC_DETERMINISTIC");
@@ -284,14 +285,15 @@ bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = 
   odc::GemmProduct g[odc::kMaxGroupProducts];
   const bool fixed = fixed_order_asked();
   for (int i = 0; i < n; ++i) {
-    const auto& [a, b, c, lay, accumulate, scale] = products[i];
+    const auto& [a, b, c, lay, accumulate, scale, times] = products[i];
     if (a.dim() != 2 || b.dim() != 2 || c.dim() != 2 || a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16 ||
         (c.scalar_type() != at::kBFloat16 && c.scalar_type() != at::kFloat) || a.stride(1) != 1 || b.stride(1) != 1 || c.stride(1) != 1)
       return false;
     const int64_t K = lay == kTN ? a.size(0) : a.size(1), M = lay == kTN ? a.size(1) : a.size(0), N = lay == kNT ? b.size(0) : b.size(1);
     if ((lay == kNT ? b.size(1) : b.size(0)) != K || c.size(0) != M || c.size(1) != N) return false;
     g[i] = odc::GemmProduct{a.data_ptr(), b.data_ptr(), c.data_ptr(), kind_of(c.scalar_type()), static_cast<int>(M), static_cast<int>(N),
-                            static_cast<int>(K), lay, accumulate, fixed, a.stride(0), b.stride(0), c.stride(0), static_cast<float>(scale)};
+                            static_cast<int>(K), lay, accumulate, fixed, a.stride(0), b.stride(0), c.stride(0), static_cast<float>(scale),
+                            times.defined() ? times.data_ptr<float>() : nullptr};
   }
   const Tensor& a = products[0].a;
   c10::cuda::CUDAGuard guard(a.device());
@@ -835,9 +837,43 @@ std::tuple<Tensor, Tensor, Tensor> lm_head_loss(const Tensor& h, const Tensor& w
   return {loss, dh, dw};
 }
 
+// Tokens of one chunk: the gradient of their logits is kept for the backward instead of the fp32 gradient of the weight, which is
+// then formed with the loss gradient in its epilogue and rounded once.  The fp32 matrix is neither written nor read again by a pass
+// that multiplies it (128256 words, 2048 wide: 2.1 of 2.6 GB).  What waits for the backward is no larger than that matrix, or small.
+// Loss and gradients of 256 tokens 720 us with the matrix, 452 without, of 1000 1540 and 1255, 4096 wide 1380 and 830; 4096 tokens
+// the same.  Smallest training step, whose weight gradient goes straight to the accumulator: 1545 and 1367 us.
+bool keeps_logit_grads(const Tensor& h, const Tensor& w, int64_t chunk, bool need_dw) {
+  constexpr int64_t kSmall = 128 << 20;
+  const int64_t T = h.size(0), kept = T * w.size(0) * 2, instead = w.numel() * 4;
+  return need_dw && T > 0 && T <= chunk && (kept <= instead || kept <= kSmall) && h.scalar_type() == at::kBFloat16 &&
+         w.scalar_type() == at::kBFloat16 && !library_gemm();
+}
+std::tuple<Tensor, Tensor> loss_and_logit_grads(const Tensor& h, const Tensor& w, const Tensor& labels, const c10::optional<Tensor>& loss_scale,
+                                                int64_t ignore_index) {
+  auto loss = at::zeros({}, h.options().dtype(at::kFloat));
+  auto logits = chunk_logits(h, w.size(0), h.size(0));
+  head_chunk(h, w, logits, labels, loss_scale, loss, {}, ignore_index, 1.0);
+  return {loss, logits};
+}
+// (logits' gradient)^T h * *g, in the type of the weight
+Tensor head_weight_grad(const Tensor& dlogits, const Tensor& h, const Tensor& g) {
+  const Tensor g32 = g.to(at::kFloat);
+  Tensor dw = product_out(dlogits, h, kTN);
+  if (group_into({{dlogits, h, dw, kTN, false, 1.0, g32}})) return dw;
+  return scale_to_bf16(product(dlogits, h, kTN, {}, {}, at::kFloat), g32);
+}
+
 struct LinearCrossEntropyFn : Function<LinearCrossEntropyFn> {
   static Tensor forward(AutogradContext* ctx, Tensor h, Tensor w, Tensor labels, c10::optional<Tensor> loss_scale,
                         int64_t ignore_index, int64_t chunk, bool need_dh, bool need_dw) {
+    check_chunk(chunk);
+    if (keeps_logit_grads(h, w, chunk, need_dw)) {
+      auto [loss, dlogits] = loss_and_logit_grads(h, w, labels, loss_scale, ignore_index);
+      Tensor dh;
+      if (need_dh) dh = product(dlogits, w, kNN);
+      ctx->save_for_backward({dh, h, dlogits});
+      return loss;
+    }
     auto [loss, dh, dw] = lm_head_loss(h, w, labels, loss_scale, ignore_index, chunk, need_dh, need_dw, c10::nullopt);
     ctx->save_for_backward({dh, dw});
     return loss;
@@ -847,6 +883,7 @@ struct LinearCrossEntropyFn : Function<LinearCrossEntropyFn> {
     const Tensor& g = grads[0];
     Tensor gh, gw;
     if (s[0].defined()) gh = scale_to_bf16(s[0], g);
+    if (s.size() == 3) return {gh, head_weight_grad(s[2], s[1], g), {}, {}, {}, {}, {}, {}};
     if (s[1].defined()) gw = scale_to_bf16(s[1], g);
     return {gh, gw, {}, {}, {}, {}, {}, {}};
   }
@@ -1019,6 +1056,44 @@ Tensor sharded_grads(const Tensor& dy2, const ShardedMatrix* m, const std::vecto
 
 // Forward is the plain product for one rank, else the product that pulls the owners' rows inside the kernel; the weight
 // gradient is added into its owners from the epilogue of its product.  The weight is no autograd input.
+// Backward of the sharded engine's loss over tokens of one chunk: dh = dlogits w * *g, and dlogits^T h * scale * *g into the
+// accumulator of one rank (reported as an arrival), or added to `local`, or written to it without the factors.
+Tensor sharded_head_grads(const Tensor& dlogits, const Tensor& h, const Tensor& w, const Tensor& g, const c10::intrusive_ptr<ShardedMatrix>& m,
+                          c10::optional<Tensor> local, bool add) {
+  const Tensor g32 = g.to(at::kFloat);
+  const bool direct = !local.has_value();
+  TORCH_CHECK(!direct || m->world == 1, "sharded_head_grads: the accumulator of one rank");
+  const Tensor dw = direct ? at::from_blob(reinterpret_cast<void*>(m->acc_addrs[0]), {m->out_features, h.size(1)}, h.options().dtype(at::kFloat))
+                           : *local;
+  const Tensor dh = product_out(dlogits, w, kNN);
+  std::vector<Product> todo{{dlogits, w, dh, kNN, false, 1.0, g32},
+                            {dlogits, h, dw, kTN, direct || add, direct ? m->grad_scale : 1.0, direct || add ? g32 : Tensor()}};
+  if (group_into(todo, direct ? m->ctr_table : Tensor(), direct ? 1 : 0)) {
+    if (direct) m->dispatched->n.fetch_add(1);
+    return dh;
+  }
+  // one by one: dh rounded once more; the weight's gradient by way of a matrix of its own
+  product_into(dlogits, w, dh, kNN);
+  if (direct || add) {
+    const Tensor dw32 = product(dlogits, h, kTN, {}, {}, at::kFloat);
+    if (direct) {
+      const Tensor scaled = dw32.mul_(g32);
+      check(odc::launch_scatter_accumulate(scaled.data_ptr(), odc::kF32, reinterpret_cast<const long long*>(m->acc_table.data_ptr<int64_t>()),
+                                           odc::kF32, reinterpret_cast<const long long*>(m->ctr_table.data_ptr<int64_t>()),
+                                           static_cast<size_t>(scaled.numel()), 1, 0, static_cast<float>(m->grad_scale),
+                                           next_done_slot(h.get_device()), sm_count(), cur_stream(),
+                                           device_status(h.get_device()).data_ptr<int>(), 0, nullptr), "head gradient");
+      count();
+      m->dispatched->n.fetch_add(1);
+    } else {
+      dw.addcmul_(dw32, g32);
+    }
+  } else {
+    product_into(dlogits, h, dw, kTN);
+  }
+  return scale_to_bf16(dh, g32);
+}
+
 struct ShardedLinearFn : Function<ShardedLinearFn> {
   static Tensor forward(AutogradContext* ctx, Tensor x, c10::optional<Tensor> bias, c10::optional<Tensor> residual,
                         c10::intrusive_ptr<ShardedMatrix> m, c10::optional<Tensor> bias_sink, bool keep_weight, bool need_dx,
@@ -1461,6 +1536,10 @@ void register_ops(py::module_& m) {
   m.def("attention_qkv", &attention_qkv);
   m.def("linear_cross_entropy", &linear_cross_entropy);
   m.def("linear_token_logprobs", &linear_token_logprobs);
+  m.def("head_keeps_logit_grads", &keeps_logit_grads, py::arg("h"), py::arg("w"), py::arg("chunk"), py::arg("need_dw") = true);
+  m.def("loss_and_logit_grads", &loss_and_logit_grads);
+  m.def("sharded_head_grads", &sharded_head_grads, py::arg("dlogits"), py::arg("h"), py::arg("w"), py::arg("g"), py::arg("matrix"),
+        py::arg("local") = py::none(), py::arg("add") = false);
   m.def("lm_head_loss", &lm_head_loss, py::arg("h"), py::arg("w"), py::arg("labels"), py::arg("loss_scale"),
         py::arg("ignore_index"), py::arg("chunk"), py::arg("need_dh"), py::arg("need_dw"), py::arg("dw_out") = py::none());
 }

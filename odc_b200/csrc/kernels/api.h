@@ -131,8 +131,8 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
                            int sm_count, cudaStream_t stream, const void* residual = nullptr, long long ldr = 0,
                            float* split_ws = nullptr);
 
-// Up to three products of one layout each, none of which reads what another writes, as one launch on CTA pairs.  C is bf16, or fp32
-// (then times scale, and added to C if accumulate).  ctr_ptrs: device table whose first entry is an arrival counter that receives
+// Up to three products of one layout each, none of which reads what another writes, as one launch on CTA pairs.  C is bf16 or fp32,
+// times scale and, unless scale_ptr is null, the value there; an fp32 result is added to C if accumulate.  ctr_ptrs: device table whose first entry is an arrival counter that receives
 // `arrivals` once everything is in memory (0: none).  scratch: gemm_group_scratch() bytes.  cudaErrorNotSupported: one by one.
 constexpr int kMaxGroupProducts = 3;
 struct GemmProduct {
@@ -142,6 +142,7 @@ struct GemmProduct {
   bool accumulate, fixed_order;   // fixed_order: the sum of an accumulating product is formed in one order
   long long lda, ldb, ldc;
   float scale;
+  const float* scale_ptr;
 };
 struct GemmGroupPlan {
   int parts[kMaxGroupProducts];     // of every tile; 0: not taken as a group

@@ -138,7 +138,8 @@ struct GroupProblem {
   int M, N, K, tiles_m, tiles_n;
   int a_mn, b_mn, bn;
   int out;                  // 0: bf16, 1: fp32, 2: added to fp32
-  float scale;              // of an fp32 result
+  float scale;              // of the result, times *scale_ptr unless that is null
+  const float* scale_ptr;
   int first;                // its first item
   int splits, kb_split;     // work items per tile, k-blocks of each
   int first_split_tile, first_part;   // bf16 with splits > 1: of its first tile, among the divided tiles and parts of the launch
@@ -705,6 +706,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           for (int i = 0; i < 32; ++i) sincosf(at * rope_freq[i], &sines[i], &cosines[i]);
         }
       }
+      [[maybe_unused]] float result_scale = 1.f;
+      if constexpr (kMode == kModeGroup) {
+        const GroupProblem& q = owners.prob[place.pi];
+        result_scale = q.scale;
+        if (q.scale_ptr != nullptr) result_scale *= *q.scale_ptr;
+      }
       // the residual's first box is asked for while the products run (1000 x 1536 x 1536: 3 us more than without a residual, box by box)
       [[maybe_unused]] const __nv_bfloat16* rrow = nullptr;
       [[maybe_unused]] uint4 res[8];
@@ -806,7 +813,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           const CUtensorMap* map = &owners.c[place.pi];
           const int cols = m0 >= q.M ? 0 : min(tile_cols, q.N - n0);
           if (q.out != 0) {
-            const float scale = q.scale;
             const bool add = q.out == 2;
 #pragma unroll 1
             for (int col = 0; col < cols; col += 32) {
@@ -814,7 +820,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
               tmem_ld_32x32(t_row + col, r);
               tmem_ld_wait();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * scale);
+              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * result_scale);
               emit(r, map, n0 + col, m0, add);
             }
           } else {
@@ -883,6 +889,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                   }
 #pragma unroll
                   for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(f[i]);
+                }
+                if (result_scale != 1.f) {
+#pragma unroll
+                  for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * result_scale);
                 }
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
@@ -1540,7 +1550,7 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
   if (n < 1 || n > kMaxGroup || sm_count < 2) return false;
   for (int i = 0; i < n; ++i) {
     const GemmProduct& q = g[i];
-    if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate || q.scale != 1.f))) return false;
+    if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate))) return false;
     shapes[i] = GroupShape{(q.M + 255) / 256 * ((q.N + BN - 1) / BN), (q.K + BK - 1) / BK, 1, 0,
                            q.c_kind == kBF16 || (q.accumulate && !q.fixed_order), q.c_kind == kBF16,
                            BN, (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2))};
@@ -1613,7 +1623,7 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long l
     t.tiles_m = (q.M + 255) / 256; t.tiles_n = (q.N + shape.bn - 1) / shape.bn;
     t.a_mn = a_mn; t.b_mn = b_mn; t.bn = shape.bn;
     t.out = q.c_kind == kBF16 ? 0 : q.accumulate ? 2 : 1;
-    t.scale = q.scale;
+    t.scale = q.scale; t.scale_ptr = q.scale_ptr;
     t.first = group.items;
     t.splits = shape.splits; t.kb_split = shape.each;
     if (shape.bf16 && shape.splits > 1) {

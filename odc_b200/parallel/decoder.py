@@ -214,6 +214,11 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
     def forward(ctx, h, labels, loss_scale, model, ignore_index, chunk):
         p = model.head_param()
         w = model.head_full()[:p.out_features]
+        ctx.model, ctx.kept = model, h.is_cuda and bool(p.matrix()) and ops._ext().head_keeps_logit_grads(h, w, chunk)
+        if ctx.kept:   # the gradient of the logits; the products with it are left to the backward, which knows the loss gradient
+            loss, dlogits = ops._ext().loss_and_logit_grads(h, w, labels, loss_scale, ignore_index)
+            ctx.save_for_backward(h, dlogits)
+            return loss
         if h.is_cuda:
             # room for the owners' padding rows, so that the whole buffer can be pushed as it is
             dw32 = torch.empty(p.world * p.rows_per_rank, h.shape[1], dtype=torch.float32, device=h.device)
@@ -229,11 +234,36 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
                 dh, dw32 = torch.autograd.grad(loss, [h_, w_])
             loss = loss.detach()
         ctx.save_for_backward(dh, dw32)
-        ctx.model = model
         return loss
 
     @staticmethod
+    def _backward_kept(ctx, dloss):
+        h, dlogits = ctx.saved_tensors
+        model = ctx.model
+        p = model.head_param()
+        w = model.head_full()[:p.out_features]
+        grads = lambda *target: ops._ext().sharded_head_grads(dlogits, h, w, dloss, p.matrix(), *target)
+        if _direct(p):
+            if p.world == 1:
+                return grads()
+            # room for the owners' padding rows, so that the whole buffer can be pushed as it is
+            dw32 = torch.empty(p.world * p.rows_per_rank, h.shape[1], dtype=torch.float32, device=h.device)
+            if dw32.shape[0] > p.out_features:
+                dw32[p.out_features:].zero_()
+            gh = grads(dw32[:p.out_features], False)
+            p.push_direct(dw32, dloss)
+            return gh
+        p.wait_push()
+        gh = grads(p.local_buffer()[:p.out_features], True)
+        p.local_dirty = True
+        if p is not model.embed and L.requires_gradient_sync():
+            p.push_local(side_stream=True)   # a tied matrix is pushed by the lookup's backward, which runs last
+        return gh
+
+    @staticmethod
     def backward(ctx, dloss):
+        if ctx.kept:
+            return _FusedLinearCrossEntropy._backward_kept(ctx, dloss), None, None, None, None, None
         dh, dw32 = ctx.saved_tensors
         model = ctx.model
         p = model.head_param()

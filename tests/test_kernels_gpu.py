@@ -676,6 +676,32 @@ def test_linear_autograd_matches_reference():
     torch.testing.assert_close(b.grad.float(), br.grad, rtol=2e-2, atol=0.5)
 
 
+@pytest.mark.parametrize("T,H,V", [(1, 64, 256), (63, 264, 1000), (300, 512, 4096), (700, 256, 32000), (1000, 1536, 8192)])
+@pytest.mark.parametrize("factor", [1.0, 1 / 3])
+def test_loss_of_one_chunk_keeps_the_logit_gradients(T, H, V, factor):
+    """One chunk (the gradient of the logits waits for the backward) and several (the weight's gradient in fp32 does), both against
+    64 bits: the same loss, and gradients no further from it."""
+    from odc_b200 import ops
+    torch.manual_seed(0)
+    h, w = torch.randn(T, H, device="cuda").bfloat16(), (torch.randn(V, H, device="cuda") * H ** -0.5).bfloat16()
+    labels = torch.randint(0, V, (T,), device="cuda")
+    labels[:: 7] = -100
+    scale = torch.rand(T, device="cuda")
+    hd, wd = h.double().requires_grad_(), w.double().requires_grad_()
+    nll = torch.nn.functional.cross_entropy(hd @ wd.t(), labels, ignore_index=-100, reduction="none")
+    want = torch.autograd.grad((nll * scale.double()).sum() * factor, [hd, wd])
+    far = []
+    for chunk in (T, max(1, T - 1)):
+        a, b = h.clone().requires_grad_(), w.clone().requires_grad_()
+        loss = ops.linear_cross_entropy(a, b, labels, scale, chunk=chunk)
+        (loss * factor).backward()
+        far.append([float((g.double() - x).norm() / x.norm()) if float(x.norm()) else float(g.double().norm()) for g, x in zip((a.grad, b.grad), want)])
+        assert a.grad.dtype == b.grad.dtype == torch.bfloat16
+        # the logits and their gradients are bf16: 2^-8 each of them
+        assert abs(float(loss) - float((nll * scale).sum())) <= 2 ** -7 * float(nll.abs().sum()) and max(far[-1]) < 2 ** -6
+    assert far[0][0] <= 1.02 * far[1][0] + 1e-4 and far[0][1] <= 1.02 * far[1][1] + 1e-4
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 8), (127, 72), (129, 264), (1001, 2560), (4096, 64)])
 def test_bias_gradient_sums(ext, rows, cols):
     """Column sums, ragged in rows and in the 64 columns of a CTA: rounded once to bf16 from fp32 sums."""
