@@ -1091,9 +1091,11 @@ narrow_grads_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ d
 // The same for queries and keys that were rotated by their positions after the projection: the gradients are rotated back on the
 // way, rounded before as the pass over them finds them, and v's are left alone.  Bound by memory: fp32 dQ read once, dQ written and dK read
 // and written once, instead of a pass that narrows dQ and one over the whole of dqkv (16321 tokens, 32/8 heads of 64: 35 + 43 us).
-constexpr int kFinishTokens = 4;   // per CTA: their angles are as many as its threads
+// 128 threads for two tokens: 16321 tokens, 32/8 heads of 64, 40.3 us; 256 for four 41.9, for two 48.5, 128 for one 45.2; 1000 tokens,
+// 12/2 heads of 128, 6.1, 7.2, 6.0, 5.6.
+constexpr int kFinishTokens = 2, kFinishThreads = 128;
 template <int D>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kFinishThreads)
 finish_rope_grads_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk,
                          __nv_bfloat16* __restrict__ dv, int total_tokens, int n_q, int n_kv, long long dq_stride, long long dkv_stride,
                          float scale, const float* __restrict__ kv_parts, int parts, const long long* __restrict__ pos, float log2_theta) {
@@ -1343,7 +1345,7 @@ cudaError_t attn_bwd(const void* dout, const void* q, const void* k, const void*
     launch(attn_bwd_kernel<128>, grid, kBwdThreads, BwdCfg<128>::kSmem, stream, tq, tk, tv, tdo, tdq, p);
   if (rope_pos != nullptr) {
     const auto kernel = head_dim == 64 ? finish_rope_grads_kernel<64> : finish_rope_grads_kernel<128>;
-    launch(kernel, (total_tokens + kFinishTokens - 1) / kFinishTokens, 256, 0, stream, static_cast<const float*>(dq_acc),
+    launch(kernel, (total_tokens + kFinishTokens - 1) / kFinishTokens, kFinishThreads, 0, stream, static_cast<const float*>(dq_acc),
            static_cast<__nv_bfloat16*>(dq), static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), total_tokens, n_q, n_kv,
            dq_stride, dkv_stride, scale, static_cast<const float*>(kv_parts), p.parts, rope_pos, log2f(rope_theta));
     return cudaGetLastError();
