@@ -132,7 +132,8 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
                            float* split_ws = nullptr);
 
 // Up to three products of one layout each, none of which reads what another writes, as one launch on CTA pairs.  C is bf16 or fp32,
-// times scale and, unless scale_ptr is null, the value there; an fp32 result is added to C if accumulate.  ctr_ptrs: device table whose first entry is an arrival counter that receives
+// times scale and, unless scale_ptr is null, the value there; an fp32 result is added to C if accumulate, and to a bf16
+// one an fp32 matrix may be added.  ctr_ptrs: device table whose first entry is an arrival counter that receives
 // `arrivals` once everything is in memory (0: none).  scratch: gemm_group_scratch() bytes.  cudaErrorNotSupported: one by one.
 constexpr int kMaxGroupProducts = 3;
 struct GemmProduct {
@@ -143,6 +144,7 @@ struct GemmProduct {
   long long lda, ldb, ldc;
   float scale;
   const float* scale_ptr;
+  const float* addend;   // bf16 C: fp32 [M, N], joins the sum before scale and rounding
 };
 struct GemmGroupPlan {
   int parts[kMaxGroupProducts];     // of every tile; 0: not taken as a group

@@ -140,6 +140,7 @@ struct GroupProblem {
   int out;                  // 0: bf16, 1: fp32, 2: added to fp32
   float scale;              // of the result, times *scale_ptr unless that is null
   const float* scale_ptr;
+  const float* addend;      // bf16 results: fp32 [M, N] that joins the sum before it is rounded, or null
   int first;                // its first item
   int splits, kb_split;     // work items per tile, k-blocks of each
   int first_split_tile, first_part;   // bf16 with splits > 1: of its first tile, among the divided tiles and parts of the launch
@@ -890,6 +891,23 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
                   for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(f[i]);
                 }
+                if (q.addend != nullptr) {
+                  if (row < q.M) {
+                    const float* from = q.addend + static_cast<long long>(row) * q.N + n0 + col;
+                    const int left = cols - col;   // a multiple of 8
+                    float4 x[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                      x[i] = 4 * i < left ? *reinterpret_cast<const float4*>(from + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                      r[4 * i] = __float_as_uint(__uint_as_float(r[4 * i]) + x[i].x);
+                      r[4 * i + 1] = __float_as_uint(__uint_as_float(r[4 * i + 1]) + x[i].y);
+                      r[4 * i + 2] = __float_as_uint(__uint_as_float(r[4 * i + 2]) + x[i].z);
+                      r[4 * i + 3] = __float_as_uint(__uint_as_float(r[4 * i + 3]) + x[i].w);
+                    }
+                  }
+                }
                 if (result_scale != 1.f) {
 #pragma unroll
                   for (int i = 0; i < 64; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * result_scale);
@@ -1550,9 +1568,9 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
   if (n < 1 || n > kMaxGroup || sm_count < 2) return false;
   for (int i = 0; i < n; ++i) {
     const GemmProduct& q = g[i];
-    if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate))) return false;
+    if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate)) || (q.addend != nullptr && q.c_kind != kBF16)) return false;
     shapes[i] = GroupShape{(q.M + 255) / 256 * ((q.N + BN - 1) / BN), (q.K + BK - 1) / BK, 1, 0,
-                           q.c_kind == kBF16 || (q.accumulate && !q.fixed_order), q.c_kind == kBF16,
+                           q.c_kind == kBF16 ? q.addend == nullptr : q.accumulate && !q.fixed_order, q.c_kind == kBF16,
                            BN, (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2))};
   }
   // A group saves the launches and last rounds of its products, 30 to 100 units.  With more work than this for a pair that is no
@@ -1564,7 +1582,7 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
   bool f32 = false;
   for (int i = 0; i < n; ++i) {
     work += static_cast<long long>(shapes[i].tiles) * shapes[i].kb;
-    f32 = f32 || !shapes[i].bf16;
+    f32 = f32 || !shapes[i].bf16 || g[i].addend != nullptr;
   }
   if (work > (f32 ? 12000ll : 3000ll) * (sm_count / 2)) return false;
   plan_group(shapes, n, sm_count / 2);
@@ -1597,6 +1615,7 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long l
     const GemmProduct& q = g[i];
     if ((reinterpret_cast<uintptr_t>(q.a) | reinterpret_cast<uintptr_t>(q.b) | reinterpret_cast<uintptr_t>(q.c)) & 15)
       return cudaErrorNotSupported;
+    if (reinterpret_cast<uintptr_t>(q.addend) & 15) return cudaErrorNotSupported;
     if ((q.lda % 8) || (q.ldb % 8) || (q.N % 8) || (q.layout == 2 && q.M % 8) || (q.ldc % (q.c_kind == kF32 ? 4 : 8))) return cudaErrorNotSupported;
   }
   static std::once_flag once;
@@ -1623,7 +1642,7 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long l
     t.tiles_m = (q.M + 255) / 256; t.tiles_n = (q.N + shape.bn - 1) / shape.bn;
     t.a_mn = a_mn; t.b_mn = b_mn; t.bn = shape.bn;
     t.out = q.c_kind == kBF16 ? 0 : q.accumulate ? 2 : 1;
-    t.scale = q.scale; t.scale_ptr = q.scale_ptr;
+    t.scale = q.scale; t.scale_ptr = q.scale_ptr; t.addend = q.addend;
     t.first = group.items;
     t.splits = shape.splits; t.kb_split = shape.each;
     if (shape.bf16 && shape.splits > 1) {
