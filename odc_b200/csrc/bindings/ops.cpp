@@ -1297,7 +1297,7 @@ Tensor layer_backward(const variable_list& kept, const Tensor& pos, const Tensor
 struct LayerFn : Function<LayerFn> {
   struct Sink {
     const LayerWeights& w;
-    Tensor norm_grad[2], matrix[2], d_gate_up, d_down, d_bias;
+    Tensor norm_grad[2], norm_sums, matrix[2], d_gate_up, d_down, d_bias;
     Tensor linear(int which, const Tensor& dy2, const Tensor& x2) {
       const Tensor& m = which == 0 ? w.wqkv : w.wo;
       Tensor dx;
@@ -1312,9 +1312,14 @@ struct LayerFn : Function<LayerFn> {
       return dx;
     }
     Tensor norm(int which, const Tensor& dh, const Tensor& x, const Tensor& weight, const Tensor& rstd, const Tensor& dres) {
-      Tensor dx;
-      std::tie(dx, norm_grad[which]) = norm_grads(dh, x, weight, rstd, dres, c10::nullopt);
-      return dx;
+      if (!norm_sums.defined()) norm_sums = at::zeros({2, x.size(1)}, x.options().dtype(at::kFloat));   // of both norms
+      return std::get<0>(norm_grads(dh, x, weight, rstd, dres, norm_sums.select(0, which)));
+    }
+    void narrow_norms() {
+      for (int i = 0; i < 2; ++i) norm_grad[i] = at::empty({norm_sums.size(1)}, w.norm1.options());
+      check(odc::launch_narrow_pair(norm_sums.data_ptr<float>(), norm_grad[0].data_ptr(), norm_grad[1].data_ptr(),
+                                    static_cast<int>(norm_sums.size(1)), cur_stream()), "layer backward");
+      count();
     }
     void bias(const Tensor& dqkv) { if (w.bqkv.defined()) d_bias = column_sum(dqkv); }
   };
@@ -1337,6 +1342,7 @@ struct LayerFn : Function<LayerFn> {
     const LayerWeights w{kept[kKept], kept[kKept + 1], kept[kKept + 2], kept[kKept + 3], kept[kKept + 4], kept[kKept + 5], kept[kKept + 6]};
     Sink sink{w};
     const Tensor dx = layer_backward(kept, kept[kKept + 7], kept[kKept + 8], w, c, grads[0].contiguous(), sink);
+    sink.narrow_norms();
     return {dx, sink.norm_grad[0], sink.matrix[0], sink.d_bias, sink.matrix[1], sink.norm_grad[1], sink.d_gate_up, sink.d_down, {}, {}, {}, {}};
   }
 };

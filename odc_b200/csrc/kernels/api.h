@@ -99,6 +99,8 @@ cudaError_t launch_adamw(float* p, const void* g, int g_kind, float* m, float* v
                          cudaStream_t stream);
 // column sums of a bf16 [rows, cols] matrix, fp32 inside: rounded into out (bf16) or added to sink (fp32); cols % 8 == 0
 cudaError_t launch_column_sum(const void* x, void* out, float* sink, long long rows, int cols, cudaStream_t stream);
+// a, b (bf16 [n]) = the halves of in (fp32 [2, n])
+cudaError_t launch_narrow_pair(const float* in, void* a, void* b, int n, cudaStream_t stream);
 // out (bf16) = in (fp32 or bf16) * *scale
 cudaError_t launch_scale_to_bf16(const void* in, int in_kind, void* out, const float* scale, size_t n, int sm_count,
                                  cudaStream_t stream);

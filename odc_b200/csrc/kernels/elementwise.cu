@@ -718,6 +718,19 @@ cudaError_t launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
   return e;
 }
 
+// Two fp32 vectors next to one another, in bf16, each into a tensor of its own: what a layer's norms sum up in its backward.  Cleared
+// and narrowed together they take two launches of the layer's backward instead of four, 8 us of 331 over 1000 tokens (narrowing them in
+// the CTA that adds last instead lengthened that kernel by 5 us each).
+__global__ void __launch_bounds__(256) narrow_pair_kernel(const float* __restrict__ in, bf16* __restrict__ a, bf16* __restrict__ b, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 2 * n) (i < n ? a[i] : b[i - n]) = __float2bfloat16(in[i]);
+}
+cudaError_t launch_narrow_pair(const float* in, void* a, void* b, int n, cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  launch(narrow_pair_kernel, (2 * n + 255) / 256, 256, 0, stream, in, static_cast<bf16*>(a), static_cast<bf16*>(b), n);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_column_sum(const void* x, void* out, float* sink, long long rows, int cols, cudaStream_t stream) {
   if (cols % 8 != 0 || (out == nullptr) == (sink == nullptr)) return cudaErrorInvalidValue;
   if (cols == 0) return cudaSuccess;
