@@ -190,6 +190,62 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 __device__ __forceinline__ float lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
+// One thread's walk over the k-blocks of an item.  What a k-block takes is instructions one behind the other: with the stage's
+// number, address and parity worked out from a running count, the operands' layouts asked for and the leader's barrier looked up
+// at each, loading one took 465 clocks, nearly as much as multiplying a whole tile's (512) and more than a half tile's (256).
+// Stepped, with the layouts as types and the first tile worked out before the pair meets: 1900 x 512 x 512 6.3 us, now 5.3, 1000 x
+// 1536 x 1536 10.2 and 8.1, with K = 8960 and an fp32 result 38.5 and 28.0; whole tiles gain half a microsecond a launch.
+template <int kStages, bool kAMn, bool kBMn>
+__device__ __forceinline__ bool load_blocks(const CUtensorMap* map_a, const CUtensorMap* map_b, int kb0, int kb1, int m0, int n0, bool whole_b,
+                                            uint32_t it, uint32_t base, uint32_t empty0, uint32_t full0, uint32_t leader_full0, bool leader,
+                                            uint32_t bytes, const WaitCtx& wc) {
+  uint32_t s = it % kStages, parity = ((it / kStages) & 1) ^ 1;
+  for (int k0 = kb0 * BK; k0 < kb1 * BK; k0 += BK) {
+    if (!mbar_wait(empty0 + 8 * s, parity, wc, 11)) return false;
+    const uint32_t sa = base + s * kStageBytes, sb = sa + kATile, bar = leader_full0 + 8 * s;
+    if (leader) mbar_arrive_expect_tx(full0 + 8 * s, bytes);   // of both CTAs
+    if constexpr (!kAMn) {
+      tma_load_2d_pair(sa, map_a, bar, k0, m0);                 // box {64 k, 128 rows}
+    } else {
+      tma_load_2d_pair(sa, map_a, bar, m0, k0);
+      tma_load_2d_pair(sa + 8192, map_a, bar, m0 + 64, k0);
+    }
+    if constexpr (!kBMn) {
+      tma_load_2d_pair(sb, map_b, bar, k0, n0);                 // box {64 k, 128 (64) rows}
+    } else {
+      tma_load_2d_pair(sb, map_b, bar, n0, k0);
+      if (whole_b) tma_load_2d_pair(sb + 8192, map_b, bar, n0 + 64, k0);
+    }
+    if (++s == kStages) { s = 0; parity ^= 1; }
+  }
+  return true;
+}
+template <int kStages, typename... Rest>
+__device__ __forceinline__ bool load_blocks(int a_mn, int b_mn, Rest... rest) {
+  if (a_mn) return load_blocks<kStages, true, true>(rest...);   // "tn"
+  return b_mn ? load_blocks<kStages, false, true>(rest...) : load_blocks<kStages, false, false>(rest...);
+}
+// The products of an item's k-blocks into the accumulator at d_tmem; the stages are reusable in BOTH CTAs once they have been read.
+template <int kStages>
+__device__ __forceinline__ bool multiply_blocks(int blocks, uint32_t it, uint32_t d_tmem, uint32_t idesc, int a_mn, int b_mn, uint32_t base,
+                                                uint32_t full0, uint32_t empty0, const WaitCtx& wc) {
+  const uint32_t leader_empty0 = mapa_shared(empty0, 0), partner_empty0 = mapa_shared(empty0, 1);
+  const uint64_t da0 = make_smem_desc(base, a_mn ? 8192u : 16u, 1024), db0 = make_smem_desc(base + kATile, b_mn ? 8192u : 16u, 1024);
+  const uint64_t a_kstep = a_mn ? 128 : 2, b_kstep = b_mn ? 128 : 2;  // 16-byte units per K = 16
+  uint32_t s = it % kStages, parity = (it / kStages) & 1;
+  for (int n = 0; n < blocks; ++n) {
+    if (!mbar_wait(full0 + 8 * s, parity, wc, 13)) return false;
+    tc_fence_after();
+    const uint64_t da = da0 + s * (kStageBytes / 16), db = db0 + s * (kStageBytes / 16);
+#pragma unroll
+    for (int j = 0; j < BK / 16; ++j) umma_f16_pair(d_tmem, da + j * a_kstep, db + j * b_kstep, idesc, (n > 0 || j > 0) ? 1u : 0u);
+    umma_commit_pair(leader_empty0 + 8 * s);
+    umma_commit_pair(partner_empty0 + 8 * s);
+    if (++s == kStages) { s = 0; parity ^= 1; }
+  }
+  return true;
+}
+
 template <int kMode>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Roles<kMode>::kThreadsTotal, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -278,16 +334,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     tmem_alloc_pair(smem_u32(tmem_slot), kTmemCols);
     tmem_relinquish_pair();
   }
-  [[maybe_unused]] int ahead = 0;   // kModeGroup: what the leader's producer (its lane 0) has asked for beyond the next item
-  if constexpr (kMode == kModeGroup) {
-    if (warp == 0 && cta == 0) ahead = take();
-  }
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync_barriers();   // the partner's barriers exist before anything is reported to them
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
   const int all_k_blocks = (p.K + BK - 1) / BK;
   auto is_part = [&](int item) { return kDivides && item >= p.whole; };
   auto tile_of = [&](int item) { return is_part(item) ? p.whole + (item - p.whole) / p.splits : item; };
@@ -298,23 +344,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       *kb0 = (item - p.whole) % p.splits * p.kb_split;
       *kb1 = min(all_k_blocks, *kb0 + p.kb_split);
     }
-  };
-  // Work items.  kModeGroup: the leader's producer takes them from a counter and writes the next one down for the other roles of
-  // both CTAs before it loads the current one.  A slot is written again kItemSlots items later.  By then all have read it: once the
-  // loads of an item have been issued, all but kStages (6) of the k-blocks so far have been multiplied, so at most 6 items are
-  // still to come for the multiplying thread, and at most two more (the accumulators) for the epilogues.
-  uint32_t item_seq = 0;
-  [[maybe_unused]] auto written_item = [&]() -> int {
-    if (num_items <= num_pairs) return num_items;   // one each, nothing is written down
-    const uint32_t slot = item_seq % kItemSlots, ph = (item_seq / kItemSlots) & 1;
-    ++item_seq;
-    const bool there = cta == 0 ? mbar_wait(islot0 + 8 * slot, ph, wc, 22) : mbar_wait_cluster(islot0 + 8 * slot, ph, wc, 22);
-    const int item = there ? item_slots[slot] : num_items;
-    return __shfl_sync(0xffffffffu, item, 0);   // the same in all lanes, also for the compiler
-  };
-  auto following = [&](int item) -> int {
-    if constexpr (kMode == kModeGroup) return written_item();
-    return item + num_pairs;
   };
   // where an item lies; group modes only
   struct Place { int pi, tm, tn, kb0, kb1, part; };
@@ -332,13 +361,48 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     return w;
   };
 
+  // the producer's first tile, worked out before the CTAs of the pair meet
+  [[maybe_unused]] int first_tm = 0, first_tn = 0;
+  [[maybe_unused]] Place first_place{};
+  if (warp == 0) {
+    if constexpr (kMode == kModeGroup) first_place = place_of(pair);
+    else tile_coords(tile_of(pair), p, &first_tm, &first_tn);
+  }
+  [[maybe_unused]] int ahead = 0;   // kModeGroup: what the leader's producer (its lane 0) has asked for beyond the next item
+  if constexpr (kMode == kModeGroup) {
+    if (warp == 0 && cta == 0) ahead = take();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_barriers();   // the partner's barriers exist before anything is reported to them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  // Work items.  kModeGroup: the leader's producer takes them from a counter and writes the next one down for the other roles of
+  // both CTAs before it loads the current one.  A slot is written again kItemSlots items later.  By then all have read it: once the
+  // loads of an item have been issued, all but kStages (6) of the k-blocks so far have been multiplied, so at most 6 items are
+  // still to come for the multiplying thread, and at most two more (the accumulators) for the epilogues.
+  uint32_t item_seq = 0;
+  [[maybe_unused]] auto written_item = [&]() -> int {
+    if (num_items <= num_pairs) return num_items;   // one each, nothing is written down
+    const uint32_t slot = item_seq % kItemSlots, ph = (item_seq / kItemSlots) & 1;
+    ++item_seq;
+    const bool there = cta == 0 ? mbar_wait(islot0 + 8 * slot, ph, wc, 22) : mbar_wait_cluster(islot0 + 8 * slot, ph, wc, 22);
+    const int item = there ? item_slots[slot] : num_items;
+    return __shfl_sync(0xffffffffu, item, 0);   // the same in all lanes, also for the compiler
+  };
+  auto following = [&](int item) -> int {
+    if constexpr (kMode == kModeGroup) return written_item();
+    return item + num_pairs;
+  };
   if (kMode == kModeGroup && warp == 0) {
     // ------------------------------------------------------------------ TMA producer of a group (both CTAs)
     // The whole warp walks the items, so that what depends on them stays in uniform registers, and one thread issues.
     if constexpr (kMode == kModeGroup) {
       uint32_t it = 0;
       int item = pair, next = num_items;
-      Place w = place_of(item), w_next{};
+      Place w = first_place, w_next{};
+      const uint32_t leader_full0 = mapa_shared(full0, 0);
       for (; item < num_items; item = next, w = w_next) {
         if (cta == 0 && num_items > num_pairs) {   // the next item is written down and the one after it asked for before this one is loaded
           taken(ahead);
@@ -357,29 +421,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const int m0 = w.tm * 256 + static_cast<int>(cta) * BMH, n0 = w.tn * q_bn + static_cast<int>(cta) * (q_bn / 2);
         bool ok = true;
         auto load = [&](int kb0, int kb1) {
-          uint32_t step = it;
-          for (int kb = kb0; kb < kb1; ++kb, ++step) {
-            const int s = step % kStages;
-            const uint32_t ph = (step / kStages) & 1;
-            if (!(ok = mbar_wait(empty0 + 8 * s, ph ^ 1, wc, 11))) break;
-            const uint32_t sa = base + s * kStageBytes;
-            const uint32_t sb = sa + kATile;
-            if (cta == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * kATile + q_bn * BK * 2);
-            const uint32_t bar = mapa_shared(full0 + 8 * s, 0);
-            const int k0 = kb * BK;
-            if (!a_mn) {
-              tma_load_2d_pair(sa, map_a, bar, k0, m0);
-            } else {
-#pragma unroll
-              for (int i = 0; i < BMH / 64; ++i) tma_load_2d_pair(sa + i * 8192, map_a, bar, m0 + 64 * i, k0);
-            }
-            if (!b_mn) {
-              tma_load_2d_pair(sb, map_b, bar, k0, n0);
-            } else {
-              tma_load_2d_pair(sb, map_b, bar, n0, k0);
-              if (q_bn == BN) tma_load_2d_pair(sb + 8192, map_b, bar, n0 + 64, k0);
-            }
-          }
+          ok = load_blocks<kStages>(a_mn, b_mn, map_a, map_b, kb0, kb1, m0, n0, q_bn == BN, it, base, empty0, full0, leader_full0, cta == 0,
+                                    static_cast<uint32_t>(2 * kATile + q_bn * BK * 2), wc);
         };
         const int head = min(w.kb1, w.kb0 + kStages);
         if (elect_one()) load(w.kb0, head);
@@ -409,28 +452,12 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           const GroupProblem& q = owners.prob[w.pi];
           const uint32_t acc = local_tile & 1, acc_ph = (local_tile >> 1) & 1;
           const uint32_t idesc = make_idesc_bf16(256, q.bn, q.a_mn != 0, q.b_mn != 0);
-          const uint32_t a_lbo = q.a_mn ? 8192u : 16u, b_lbo = q.b_mn ? 8192u : 16u;
-          const uint64_t a_kstep = q.a_mn ? 128 : 2, b_kstep = q.b_mn ? 128 : 2;
           const uint32_t d_tmem = tmem_base + acc * BN;
           bool ok = true;
           if (elect_one()) {
             ok = mbar_wait(tempty0 + 8 * acc, acc_ph ^ 1, wc, 12);
             tc_fence_after();
-            uint32_t step = it;
-            for (int kb = w.kb0; kb < w.kb1 && ok; ++kb, ++step) {
-              const int s = step % kStages;
-              const uint32_t ph = (step / kStages) & 1;
-              if (!(ok = mbar_wait(full0 + 8 * s, ph, wc, 13))) break;
-              tc_fence_after();
-              const uint32_t sa = base + s * kStageBytes;
-              const uint32_t sb = sa + kATile;
-              const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
-#pragma unroll
-              for (int j = 0; j < BK / 16; ++j)
-                umma_f16_pair(d_tmem, da + j * a_kstep, db + j * b_kstep, idesc, (kb > w.kb0 || j > 0) ? 1u : 0u);
-              umma_commit_pair(mapa_shared(empty0 + 8 * s, 0));
-              umma_commit_pair(mapa_shared(empty0 + 8 * s, 1));
-            }
+            ok = ok && multiply_blocks<kStages>(w.kb1 - w.kb0, it, d_tmem, idesc, q.a_mn, q.b_mn, base, full0, empty0, wc);
             if (ok) {
               umma_commit_pair(mapa_shared(tfull0 + 8 * acc, 0));
               umma_commit_pair(mapa_shared(tfull0 + 8 * acc, 1));
@@ -482,9 +509,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       };
       uint32_t it = 0;
       bool ok = true;
+      const uint32_t leader_full0 = mapa_shared(full0, 0);
+      int tm = first_tm, tn = first_tn;
       for (int item = pair; item < num_items && ok; item += num_pairs) {
-        int tm, tn;
-        tile_coords(tile_of(item), p, &tm, &tn);
         int kb0, k_blocks;
         k_range(item, &kb0, &k_blocks);
         const int m0 = tm * 256 + static_cast<int>(cta) * BMH;   // this CTA's rows of A and C
@@ -493,41 +520,25 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if constexpr (kMode == kModeGather) {
           // B K-major (forward): the 256 weight rows this tile multiplies must have landed in local memory first
           if (!p.b_mn && !(ok = wait_group(tn))) break;
-        }
-        for (int kb = kb0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
-          if constexpr (kMode == kModeGather) {
+          for (int kb = kb0; kb < k_blocks; ++kb, ++it) {
             // B MN-major (input gradient): the gathered rows are the reduction dimension, 4 k-blocks per group
-            if (p.b_mn && !(ok = wait_group(((p.rot_kb ? (kb + p.rot_kb) % k_blocks : kb) * BK) / BN))) break;
+            const int at = p.rot_kb ? (kb + p.rot_kb) % k_blocks : kb;
+            if (p.b_mn && !(ok = wait_group(at * BK / BN))) break;
+            if (!(ok = load_blocks<kStages>(p.a_mn, p.b_mn, &tmap_a, &tmap_b, at, at + 1, m0, n0, true, it, base, empty0, full0, leader_full0,
+                                            cta == 0, static_cast<uint32_t>(2 * kStageBytes), wc))) break;
           }
-          if (!(ok = mbar_wait(empty0 + 8 * s, ph ^ 1, wc, 11))) break;
-          const uint32_t sa = base + s * kStageBytes;
-          const uint32_t sb = sa + kATile;
-          if (cta == 0) mbar_arrive_expect_tx(full0 + 8 * s, 2 * kATile + bn * BK * 2);   // bytes of both CTAs
-          const uint32_t bar = mapa_shared(full0 + 8 * s, 0);
-          const int k0 = (p.rot_kb ? (kb + p.rot_kb) % k_blocks : kb) * BK;
-          if (!p.a_mn) {
-            tma_load_2d_pair(sa, &tmap_a, bar, k0, m0);                 // box {64 k, 128 rows}
-          } else {
-#pragma unroll
-            for (int i = 0; i < BMH / 64; ++i) tma_load_2d_pair(sa + i * 8192, &tmap_a, bar, m0 + 64 * i, k0);
-          }
-          if (!p.b_mn) {
-            tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);                 // box {64 k, 128 (64) rows}
-          } else {
-            tma_load_2d_pair(sb, &tmap_b, bar, n0, k0);
-            if (bn == BN) tma_load_2d_pair(sb + 8192, &tmap_b, bar, n0 + 64, k0);
-          }
+        } else {
+          ok = load_blocks<kStages>(p.a_mn, p.b_mn, &tmap_a, &tmap_b, kb0, k_blocks, m0, n0, bn == BN, it, base, empty0, full0, leader_full0,
+                                    cta == 0, static_cast<uint32_t>(2 * kATile + bn * BK * 2), wc);
+          it += k_blocks - kb0;
         }
+        if (item + num_pairs < num_items) tile_coords(tile_of(item + num_pairs), p, &tm, &tn);
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
     if (cta == 0 && elect_one()) {
       const uint32_t idesc = make_idesc_bf16(256, bn, p.a_mn != 0, p.b_mn != 0);
-      const uint32_t a_lbo = p.a_mn ? 8192u : 16u, b_lbo = p.b_mn ? 8192u : 16u;
-      const uint64_t a_kstep = p.a_mn ? 128 : 2, b_kstep = p.b_mn ? 128 : 2;  // 16-byte units per K = 16
       uint32_t it = 0, local_tile = 0;
       bool ok = true;
       for (int item = pair; item < num_items && ok; item += num_pairs, ++local_tile) {
@@ -538,21 +549,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const uint32_t d_tmem = tmem_base + acc * BN;
         int kb0, k_blocks;
         k_range(item, &kb0, &k_blocks);
-        for (int kb = kb0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
-          if (!(ok = mbar_wait(full0 + 8 * s, ph, wc, 13))) break;
-          tc_fence_after();
-          const uint32_t sa = base + s * kStageBytes;
-          const uint32_t sb = sa + kATile;
-          const uint64_t da = make_smem_desc(sa, a_lbo, 1024), db = make_smem_desc(sb, b_lbo, 1024);
-#pragma unroll
-          for (int j = 0; j < BK / 16; ++j)
-            umma_f16_pair(d_tmem, da + j * a_kstep, db + j * b_kstep, idesc, (kb > kb0 || j > 0) ? 1u : 0u);
-          // the stage is reusable in BOTH CTAs once these MMAs have read it
-          umma_commit_pair(mapa_shared(empty0 + 8 * s, 0));
-          umma_commit_pair(mapa_shared(empty0 + 8 * s, 1));
-        }
+        ok = multiply_blocks<kStages>(k_blocks - kb0, it, d_tmem, idesc, p.a_mn, p.b_mn, base, full0, empty0, wc);
+        it += k_blocks - kb0;
         if (ok) {
           umma_commit_pair(mapa_shared(tfull0 + 8 * acc, 0));
           umma_commit_pair(mapa_shared(tfull0 + 8 * acc, 1));
@@ -1085,7 +1083,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       if (!ok) break;
       tc_fence_before();
       __syncwarp();
-      if (lane == 0 && !last) mbar_arrive_cluster_tmem(tempty_leader0 + 8 * acc);   // the leader may overwrite this accumulator
+      // the leader may overwrite this accumulator, if it has a use for it
+      if (lane == 0 && (kMode == kModeGroup ? !last : item + 2 * num_pairs < num_items)) mbar_arrive_cluster_tmem(tempty_leader0 + 8 * acc);
     }
     if (elect_one()) {   // the thread that issued them: all output boxes have been read, or are in memory before an arrival is reported
       if constexpr (kMode == kModeScatter || kMode == kModeGroup) bulk_wait_group0();
@@ -1096,7 +1095,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   // ---------------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();   // nothing is reported to the partner's barriers, or read from its shared memory, after this
+  // Nothing is reported to the partner's barriers, or read from its shared memory, after this.  Where all that a thread reported has
+  // been waited for, nothing is left to be ordered (a release waits 1000 clocks for the memory system); in a group with further
+  // items the last accumulator but one is given back to nobody.
+  if (kMode != kModeGroup || num_items <= num_pairs) cluster_sync_exit();
+  else cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, kTmemCols);

@@ -230,6 +230,10 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void cluster_sync_barriers() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// before the exit of CTAs whose words to one another have all been waited for: nothing is published
+__device__ __forceinline__ void cluster_sync_exit() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 // address of the same shared-memory location in CTA `rank` of this cluster (a shared::cluster address)
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
   uint32_t r;
