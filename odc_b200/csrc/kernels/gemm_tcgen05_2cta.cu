@@ -278,7 +278,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const WaitCtx wc{abort_flag, p.status, kWaitBudgetNs};
 
   constexpr bool kDivides = kMode == kModePlain || kMode == kModeScatter;
-  const int bn = kMode == kModePlain || kMode == kModeRope ? p.bn : BN;   // of a group: its products'
+  const int bn = kMode == kModePlain || kMode == kModeRope || kMode == kModeSwiglu ? p.bn : BN;   // of a group: its products'
   const int num_tiles = p.tiles_m * p.tiles_n;
   int num_items = kDivides ? p.whole + (num_tiles - p.whole) * p.splits : num_tiles;   // the parts of a tile are adjacent
   if constexpr (kMode == kModeGroup) num_items = owners.items;
@@ -515,7 +515,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         int kb0, k_blocks;
         k_range(item, &kb0, &k_blocks);
         const int m0 = tm * 256 + static_cast<int>(cta) * BMH;   // this CTA's rows of A and C
-        const int n0 = kMode == kModeSwiglu ? tn * BNH + static_cast<int>(cta) * p.N
+        const int n0 = kMode == kModeSwiglu ? tn * (bn / 2) + static_cast<int>(cta) * p.N
                                             : tn * bn + static_cast<int>(cta) * (bn / 2);   // this CTA's rows of B
         if constexpr (kMode == kModeGather) {
           // B K-major (forward): the 256 weight rows this tile multiplies must have landed in local memory first
@@ -1000,13 +1000,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           if (row_ok) p.row_stats[static_cast<long long>(tn) * p.M + row] = make_float2(m, s);
         } else {
 #pragma unroll 1
-        for (int bx = 0; bx < 2; ++bx) {
+        for (int bx = 0; bx < bn / 128; ++bx) {
           uint32_t gate[32], up[32];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t r[64];
             tmem_ld_32x32(t_row + bx * 64 + 32 * h, r);
-            tmem_ld_32x32(t_row + BNH + bx * 64 + 32 * h, r + 32);
+            tmem_ld_32x32(t_row + bn / 2 + bx * 64 + 32 * h, r + 32);
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
@@ -1014,7 +1014,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
               up[16 * h + i] = pack2(__uint_as_float(r[32 + 2 * i]), __uint_as_float(r[32 + 2 * i + 1]));
             }
           }
-          const int col0 = tn * BNH + bx * 64;
+          const int col0 = tn * (bn / 2) + bx * 64;
           if (col0 >= p.N || m0 >= p.M) continue;
           if (p.store_gate_up) {
             emit(gate, &owners.m[0], col0, m0);
@@ -1207,13 +1207,19 @@ static SplitPlan plan_splits(int M, int N, int K, int sm_count, const SplitCost&
   return plan;
 }
 
-// Whether an undivided product is taken in tiles of 256 x 128: where twice as many still have a pair each.  A k-block of one takes
-// 0.7 of the time (its operands arrive no faster) and its epilogue half, so that two rounds of them are slower than one of whole
-// tiles.  256 and 128 columns, us: 300 x 512 x 512 7.0 and 6.1, 1000 x 1536 x 1536 12.3 and 10.3, 512 x 4096 x 4096 25.1 and 20.3,
-// rotated projections 1.3 times as fast; with two rounds of half tiles 1000 x 3072 x 2048 15.6 and 19.6, with three for two whole
-// ones 3000 x 2048 x 2048 25.6 and 28.6.
-static bool half_tiles_pay(int M, int N, int sm_count) {
-  return (M + 255) / 256 * ((N + 127) / 128) <= sm_count / 2;
+// Whether an undivided product is taken in tiles of 256 x 128: a k-block of one takes 0.6 of the time, its epilogue half, so it is
+// where as many rounds of them are shorter.  Twice as many tiles that still have a pair each: 300 x 512 x 512 6.8 us, half as wide
+// 5.1, 1000 x 1536 x 1536 11.9 and 8.0, 512 x 4096 x 4096 24.3 and 15.1; three rounds instead of two: 1500 x 4096 x 4096 45.0 and
+// 38.4, 4000 x 1536 x 1536 20.0 and 17.9; two instead of one 1900 x 2048 x 2048 15.5 and 15.8, six instead of three 6000 x 2048 x
+// 2048 36.4 and 40.0.  Weight gradients, whose two operands take three loads a k-block, 0.75: 3000 x 2048 x 2048 26.1 and 30.0.
+static double half_tile_time(int layout) { return layout == 2 ? 0.75 : 0.6; }
+static bool half_tiles_pay(int tiles, int half_tiles, int layout, int sm_count) {
+  const int pairs = sm_count / 2;
+  return (half_tiles + pairs - 1) / pairs * half_tile_time(layout) < 0.95 * ((tiles + pairs - 1) / pairs);
+}
+static bool half_tiles_pay_for(int M, int N, int layout, int sm_count) {
+  const int rows = (M + 255) / 256;
+  return half_tiles_pay(rows * ((N + 255) / 256), rows * ((N + 127) / 128), layout, sm_count);
 }
 
 // The plan of a bf16 product: all tiles divided where they are fewer than the pairs, else those of its last rounds.
@@ -1261,7 +1267,7 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
   }
   SplitPlan plan{(M + 255) / 256 * ((N + BN - 1) / BN), 1, 0};
   if (split_ws != nullptr) plan = product_plan(M, N, K, sm_count);
-  const int bn = plan.splits == 1 && half_tiles_pay(M, N, sm_count) ? BN / 2 : BN;
+  const int bn = plan.splits == 1 && half_tiles_pay_for(M, N, layout, sm_count) ? BN / 2 : BN;
   if (!b_mn) {
     if (!encode_tile_map_2d(&tb, b, K, N, ldb * 2, 64, bn / 2)) return cudaErrorInvalidTexture;
   } else {
@@ -1326,8 +1332,10 @@ cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* 
   if (attr_err != cudaSuccess) return attr_err;
   CUtensorMap ta, tb, tc;
   OwnerMaps halves{};
+  const int row_tiles = (M + 255) / 256;   // 128 activations a tile, or 64
+  const int bn = half_tiles_pay(row_tiles * ((F + 127) / 128), row_tiles * ((F + 63) / 64), 0, sm_count) ? BN / 2 : BN;
   const uint64_t ld_gu = static_cast<uint64_t>(F) * 4;
-  if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, 2ull * F, ldw * 2, 64, BNH) ||
+  if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, 2ull * F, ldw * 2, 64, bn / 2) ||
       !encode_tile_map_2d(&tc, act, F, M, static_cast<uint64_t>(F) * 2, 64, kOutRows))
     return cudaErrorInvalidValue;
   if (gate_up != nullptr) {  // each half clipped at its own last column
@@ -1339,7 +1347,8 @@ cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* 
   p.M = M; p.N = F; p.K = K;
   p.store_gate_up = gate_up != nullptr;
   p.tiles_m = (M + 255) / 256;
-  p.tiles_n = (F + BNH - 1) / BNH;
+  p.tiles_n = (F + bn / 2 - 1) / (bn / 2);
+  p.bn = bn;
   p.status = status;
   const int tiles = p.tiles_m * p.tiles_n;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
@@ -1368,7 +1377,7 @@ cudaError_t gemm_rope_pair(const void* x, const void* w, const void* bias, void*
   });
   if (attr_err != cudaSuccess) return attr_err;
   CUtensorMap ta, tb, tc;
-  const int bn = half_tiles_pay(M, N, sm_count) ? BN / 2 : BN;   // a head is 128 columns at most
+  const int bn = half_tiles_pay_for(M, N, 0, sm_count) ? BN / 2 : BN;   // a head is 128 columns at most
   if (!encode_tile_map_2d(&ta, x, K, M, ldx * 2, 64, BMH) || !encode_tile_map_2d(&tb, w, K, N, ldw * 2, 64, bn / 2) ||
       !encode_tile_map_2d(&tc, out, N, M, static_cast<uint64_t>(N) * 2, 64, kOutRows))
     return cudaErrorNotSupported;
@@ -1510,12 +1519,11 @@ static unsigned int* group_words(int n) {
 // An item takes at least what its epilogue does (6) and 2 to begin with; a part of a bf16 tile writes and reads 256 KB of fp32 (6),
 // the parts of an fp32 sum meet in memory.  The longest item is made half as wide, or divided, as long as that gains a twentieth.
 // 300 tokens, 1536 wide: half as wide 15.3 -> 12.5 us (projection), MLP of 512 and 1536 19.5 -> 15.4.
-constexpr double kHalfTile = 0.7;   // time of a k-block of a 256 x 128 tile (half_tiles_pay)
 struct GroupShape {
   int tiles, kb, splits, each;
   bool may_divide, bf16;
-  int bn, half_tiles;   // columns of a tile; how many tiles of half the width there are
-  double item() const { return std::max(6.0, each * (bn == 128 ? kHalfTile : 1.0)) + 2 + (splits > 1 ? (bf16 ? 6.0 : 1.0) : 0.0); }
+  int bn, half_tiles, layout;   // columns of a tile; how many tiles of half the width there are
+  double item() const { return std::max(6.0, each * (bn == 128 ? half_tile_time(layout) : 1.0)) + 2 + (splits > 1 ? (bf16 ? 6.0 : 1.0) : 0.0); }
   double sum() const { return bf16 && splits > 1 ? 12.0 + 8.0 * (splits - 1) : 0.0; }
 };
 static void plan_group(GroupShape* g, int n, int pairs) {
@@ -1574,7 +1582,7 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
     if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate)) || (q.addend != nullptr && q.c_kind != kBF16)) return false;
     shapes[i] = GroupShape{(q.M + 255) / 256 * ((q.N + BN - 1) / BN), (q.K + BK - 1) / BK, 1, 0,
                            q.c_kind == kBF16 ? q.addend == nullptr : q.accumulate && !q.fixed_order, q.c_kind == kBF16,
-                           BN, (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2))};
+                           BN, (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
   }
   // A group saves the launches and last rounds of its products, 30 to 100 units.  With more work than this for a pair that is no
   // gain any more, and pairs that are not in step with one another share less of L2 (16321 tokens, 2048 and 8192 wide, 4400 units:

@@ -339,7 +339,7 @@ def test_gemm_cta_pair_layouts(ext, layout, M, N, K):
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K", [(512, 4736, 72), (512, 4744, 72), (264, 376, 136), (256, 264, 64), (776, 392, 1600)])
 def test_gemm_tiles_of_half_the_width(ext, layout, M, N, K):
-    """37 x 2 tiles of 256 x 128 have a pair each and are taken, 38 x 2 are not; edges in the last half tile.  Against 64 bits, with
+    """37 x 2 tiles of 256 x 128 have a pair each and are taken, 38 x 2 would take two rounds; edges in the last half tile.  Against 64 bits, with
     bias and residual: fp32 sums (2e-6 of the magnitudes) and one rounding to bf16."""
     for a, b, c, lay, _, _, want, bound in _group_case([(layout, M, N, K, torch.bfloat16, False, 1.0)]):
         bias, res = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
