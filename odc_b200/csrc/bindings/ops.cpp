@@ -2,7 +2,7 @@
 //
 // A training step of a small model is bound by the host: a Python autograd function costs 15-25 us per direction, the
 // kernels behind it 3-10 us.  The native functions cost 3-5 us per direction and run their backward without the
-// interpreter lock (two layers, 512 wide, two microbatches: a training step 4579 -> 4004 us).
+// interpreter lock.
 #include "ops.h"
 
 #include <torch/csrc/autograd/custom_function.h>
@@ -186,6 +186,20 @@ Tensor kernel_status() {
   return device_status(dev);
 }
 
+// The host read an error there.  A launch that gave up may have left counters of a group half way, so from here on a group brings
+// its own (one more launch, 2 us); nothing waits for what other streams have in flight.
+std::atomic<bool> g_gave_up{false};
+void clear_kernel_status() {
+  kernel_status().zero_();
+  g_gave_up = true;
+}
+
+bool capturing() {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  check(cudaStreamIsCapturing(cur_stream(), &capture), "capture");
+  return capture != cudaStreamCaptureStatusNone;
+}
+
 // ODC_GEMM=cublas: library products, to measure the hand-written kernels against (read at every call)
 bool library_gemm() {
   const char* e = std::getenv("ODC_GEMM");
@@ -302,7 +316,11 @@ bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = 
   Tensor scratch;
   if (const size_t bytes = odc::gemm_group_scratch(g, n, sm_count()))
     scratch = at::empty({static_cast<int64_t>(bytes / sizeof(float))}, a.options().dtype(at::kFloat));
+  Tensor words;
+  if (capturing() || g_gave_up)   // a graph's are cleared at each replay
+    words = at::zeros({odc::kGroupLaunchWords}, a.options().dtype(at::kInt));
   const cudaError_t e = odc::gemm_group(g, n, scratch.defined() ? scratch.data_ptr<float>() : nullptr,
+                                        words.defined() ? reinterpret_cast<unsigned int*>(words.data_ptr<int>()) : nullptr,
                                         ctr_table.defined() ? reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()) : nullptr,
                                         arrivals, device_status(a.get_device()).data_ptr<int>(), sm_count(), cur_stream());
   if (e == cudaErrorNotSupported) return false;
@@ -1002,9 +1020,7 @@ void after_start() {
   if (!g_start.set) return;
   const cudaStream_t s = cur_stream();
   if (s == g_start.stream) return;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  check(cudaStreamIsCapturing(s, &capture), "after_start");
-  if (capture != cudaStreamCaptureStatusNone) return;
+  if (capturing()) return;
   std::lock_guard<std::mutex> lock(g_start.mu);
   check(cudaStreamWaitEvent(s, g_start.event, 0), "after_start");
 }
@@ -1066,8 +1082,6 @@ Tensor sharded_grads(const Tensor& dy2, const ShardedMatrix* m, const std::vecto
   return dx;
 }
 
-// Forward is the plain product for one rank, else the product that pulls the owners' rows inside the kernel; the weight
-// gradient is added into its owners from the epilogue of its product.  The weight is no autograd input.
 // Backward of the sharded engine's loss over tokens of one chunk: dh = dlogits w * *g, and dlogits^T h * scale * *g into the
 // accumulator of one rank (reported as an arrival), or added to `local`, or written to it without the factors.
 Tensor sharded_head_grads(const Tensor& dlogits, const Tensor& h, const Tensor& w, const Tensor& g, const c10::intrusive_ptr<ShardedMatrix>& m,
@@ -1106,6 +1120,8 @@ Tensor sharded_head_grads(const Tensor& dlogits, const Tensor& h, const Tensor& 
   return scale_to_bf16(dh, g32);
 }
 
+// Forward is the plain product for one rank, else the product that pulls the owners' rows inside the kernel; the weight
+// gradient is added into its owners from the epilogue of its product.  The weight is no autograd input.
 struct ShardedLinearFn : Function<ShardedLinearFn> {
   static Tensor forward(AutogradContext* ctx, Tensor x, c10::optional<Tensor> bias, c10::optional<Tensor> residual,
                         c10::intrusive_ptr<ShardedMatrix> m, c10::optional<Tensor> bias_sink, bool keep_weight, bool need_dx,
@@ -1503,6 +1519,7 @@ void register_ops(py::module_& m) {
   }, py::arg("tokens"), py::arg("seqs"), py::arg("longest"), py::arg("n_q"), py::arg("n_kv"), py::arg("head_dim"),
         py::arg("causal"), py::arg("sms"));  // (forward in pairs of tiles, parts of the backward)
   m.def("kernel_status", &kernel_status);
+  m.def("clear_kernel_status", &clear_kernel_status);
   m.def("scale_to_bf16", &scale_to_bf16);
   py::class_<DispatchCounter, c10::intrusive_ptr<DispatchCounter>>(m, "DispatchCounter")
       .def(py::init([] { return c10::make_intrusive<DispatchCounter>(); }))

@@ -136,8 +136,13 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
 // Up to three products of one layout each, none of which reads what another writes, as one launch on CTA pairs.  C is bf16 or fp32,
 // times scale and, unless scale_ptr is null, the value there; an fp32 result is added to C if accumulate, and to a bf16
 // one an fp32 matrix may be added.  ctr_ptrs: device table whose first entry is an arrival counter that receives
-// `arrivals` once everything is in memory (0: none).  scratch: gemm_group_scratch() bytes.  cudaErrorNotSupported: one by one.
+// `arrivals` once everything is in memory (0: none).  scratch: gemm_group_scratch() bytes.  words: kGroupLaunchWords zeros that are
+// this launch's alone, left zero by it unless a wait runs out, or null for some of the device's own (not for a captured launch, which
+// keeps what it got, nor after a wait has run out).
+// cudaErrorNotSupported: one by one.
 constexpr int kMaxGroupProducts = 3;
+constexpr int kMaxGroupDivided = 256;   // divided tiles of a launch
+constexpr int kGroupLaunchWords = 2 + 2 * kMaxGroupDivided;
 struct GemmProduct {
   const void *a, *b;
   void* c;
@@ -154,8 +159,8 @@ struct GemmGroupPlan {
 };
 GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count);
 size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count);
-cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long long* ctr_ptrs, int arrivals, int* status, int sm_count,
-                       cudaStream_t stream);
+cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,
+                       int* status, int sm_count, cudaStream_t stream);
 
 // act[M, F] = silu(x Wg^T) * (x Wu^T), w = [Wg; Wu]; gate_up [M, 2F] optional.  cudaErrorNotSupported: use the plain product.
 cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* act, int M, int F, int K, long long ldx,

@@ -1,4 +1,5 @@
-// bf16 GEMM on CTA pairs (tcgen05 cta_group::2) for sm_100a: one 256 x 256 output tile per pair of SMs.
+// bf16 GEMM on CTA pairs (tcgen05 cta_group::2) for sm_100a: one 256 x 256 output tile per pair of SMs, or one of 256 x 128 where
+// that is the shorter way (half_tiles_pay), with half of B and of the accumulator.
 //
 // Two CTAs of a cluster work on one tile.  Each CTA stages ITS half of the A tile (128 rows) and ITS half of the B
 // tile (128 rows of B, i.e. 128 output columns) with ordinary per-CTA TMA loads, and holds the accumulator rows
@@ -15,8 +16,8 @@
 // is alone, and moves every descriptor to uniform registers by way of a loop, which the main loop then waits for (16321 x
 // 16384 x 2048: 760 us, elected 679; the twelve products of a 2048-wide layer over 16321 tokens: 4.40 ms, now 4.05).
 // Two accumulators (all 512 TMEM columns of each CTA) alternate, so the epilogue of one tile overlaps the main
-// loop of the next.  Every copy in this file is an ordinary per-CTA TMA copy into that CTA's own shared memory.  Every wait is bounded and reports through the
-// status word; a pair whose partner gave up runs into its own bounded waits and leaves the same way.
+// loop of the next.  Every copy in this file is an ordinary per-CTA TMA copy into that CTA's own shared memory.  Every wait is
+// bounded and reports through the status word; a pair whose partner gave up runs into its own bounded waits and leaves the same way.
 //
 // Operand layouts, edge handling and the epilogue are those of the single-CTA kernel (gemm_tcgen05.cu).
 #include <cuda.h>
@@ -1491,10 +1492,9 @@ cudaError_t gemm_logits_pair(const void* h, const void* w, void* logits, const l
 }
 
 // Words for the launches of groups, zero at load and left zero by each: the counter of items, the count of finished CTAs, and two
-// per divided tile.  They are handed out in turn and come round again after at least kGroupWords / (2 + 2 kMaxDivided) launches,
-// more than a device holds queued.
+// per divided tile.  They are handed out in turn and come round again after at least kGroupWords / kGroupLaunchWords (2040)
+// launches, more than a device holds queued; a captured launch runs again at any time and brings its own.
 constexpr unsigned int kGroupWords = 1u << 20;
-constexpr int kMaxDivided = 256;
 __device__ unsigned int g_group_words[kGroupWords];
 static unsigned int* group_words(int n) {
   static std::mutex mu;
@@ -1564,7 +1564,7 @@ static void plan_group(GroupShape* g, int n, int pairs) {
     }
     for (int want = before.splits + 1; want <= 8 && q.may_divide; ++want) {
       const int each = (q.kb + want - 1) / want, s = (q.kb + each - 1) / each;   // no empty part
-      if (s <= before.splits || each < 4 || (q.bf16 && q.tiles > kMaxDivided)) continue;
+      if (s <= before.splits || each < 4 || (q.bf16 && q.tiles > kMaxGroupDivided)) continue;
       q.splits = s; q.each = each;
       consider();
     }
@@ -1617,8 +1617,8 @@ GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count) {
   return plan;
 }
 
-cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long long* ctr_ptrs, int arrivals, int* status, int sm_count,
-                       cudaStream_t stream) {
+cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,
+                       int* status, int sm_count, cudaStream_t stream) {
   using namespace gemm_pair;
   GroupShape shapes[kMaxGroup];
   if (!group_shapes(g, n, sm_count, shapes)) return cudaErrorNotSupported;
@@ -1663,9 +1663,9 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, const long l
     group.items += shape.tiles * shape.splits;
   }
   group.count = n;
-  if (divided > kMaxDivided || (divided > 0 && scratch == nullptr)) return cudaErrorNotSupported;
+  if (divided > kMaxGroupDivided || (divided > 0 && scratch == nullptr)) return cudaErrorNotSupported;
   group.parts = reinterpret_cast<float4*>(scratch);
-  unsigned int* words = group_words(2 + 2 * divided);
+  if (words == nullptr) words = group_words(2 + 2 * divided);
   if (words == nullptr) return cudaErrorInvalidValue;
   group.next = words;
   group.arrived = words + 2;

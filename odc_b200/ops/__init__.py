@@ -47,7 +47,7 @@ def check_status() -> None:
     word = _ext().kernel_status()
     host = word.cpu()
     if int(host[0]) != 0:
-        word.zero_()
+        _ext().clear_kernel_status()
         check_status_word(int(host[0]), int(host[1]), int(host[2]))
 
 

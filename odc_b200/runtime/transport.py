@@ -228,8 +228,12 @@ class NvlinkP2PTransport(Transport):
                                                     config.wait_timeout_ms(), self.status, self._status_host)
         self.launches += 1
         if code != 0:
-            self.status.zero_()
+            self._clear_status()
             check_status_word(code, detail, seen)
+
+    def _clear_status(self) -> None:
+        with torch.cuda.device(self.heap.device):
+            self.ext.clear_kernel_status()
 
     def check(self) -> None:
         """Read the device status word (one small D2H copy + stream sync) and raise if a kernel gave up.
@@ -242,7 +246,7 @@ class NvlinkP2PTransport(Transport):
         code = int(self._status_host[0])
         if code != 0:
             detail, seen = int(self._status_host[1]), int(self._status_host[2])
-            self.status.zero_()
+            self._clear_status()
             check_status_word(code, detail, seen)
 
 

@@ -193,3 +193,22 @@ def test_pipeline_status_surfaces_at_the_next_sync(single_rank_pg):
         red.stop()
     finally:
         odc.finalize_distributed()
+
+
+def test_groups_after_a_reported_error():
+    """Once a wait has run out, launches of several products bring their own counters, which the one that gave up cannot have left
+    half way.  The word is pre-set by hand again."""
+    from odc_b200 import _ext, ops
+    from odc_b200.runtime.status import ERR_PIPELINE_TIMEOUT, OdcTimeoutError
+    ext = _ext.load()
+    a, b = torch.randn(300, 4096, device="cuda").bfloat16(), torch.randn(4096, 512, device="cuda").bfloat16()
+    outs = [torch.empty(300, 512, device="cuda", dtype=torch.bfloat16) for _ in range(4)]
+    assert ext.gemm_group([(a, b, outs[0], "nn", False, 1.0)])
+    ext.kernel_status().copy_(torch.tensor([ERR_PIPELINE_TIMEOUT, 3, 17, 0], dtype=torch.int32))
+    with pytest.raises(OdcTimeoutError, match="pipeline"):
+        ops.check_status()
+    ops.check_status()
+    for o in outs[1:]:
+        assert ext.gemm_group([(a, b, o, "nn", False, 1.0)])
+        assert torch.equal(o, outs[0])
+    ops.check_status()
