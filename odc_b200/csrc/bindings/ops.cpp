@@ -890,7 +890,7 @@ struct LinearCrossEntropyFn : Function<LinearCrossEntropyFn> {
       auto [loss, dlogits] = loss_and_logit_grads(h, w, labels, loss_scale, ignore_index);
       Tensor dh;
       if (need_dh) dh = product(dlogits, w, kNN);
-      ctx->save_for_backward({dh, h, dlogits});
+      ctx->save_for_backward({dh, h.clone(), dlogits});   // a copy: the caller may write to h before the backward, as with several chunks
       return loss;
     }
     auto [loss, dh, dw] = lm_head_loss(h, w, labels, loss_scale, ignore_index, chunk, need_dh, need_dw, c10::nullopt);

@@ -702,6 +702,25 @@ def test_loss_of_one_chunk_keeps_the_logit_gradients(T, H, V, factor):
     assert far[0][0] <= 1.02 * far[1][0] + 1e-4 and far[0][1] <= 1.02 * far[1][1] + 1e-4
 
 
+@pytest.mark.parametrize("chunk", [96, 300])
+def test_loss_lets_its_input_be_written_to(chunk):
+    """Whatever waits for the backward is the loss's own: overwriting the hidden states before it changes no gradient."""
+    from odc_b200 import ops
+    torch.manual_seed(0)
+    h0, w = torch.randn(300, 256, device="cuda").bfloat16(), torch.randn(1032, 256, device="cuda").bfloat16().requires_grad_()
+    labels = torch.randint(0, 1032, (300,), device="cuda")
+    grads = []
+    for write in (False, True):
+        leaf = h0.clone().requires_grad_()
+        h = leaf * 1
+        loss = ops.linear_cross_entropy(h, w, labels, chunk=chunk)
+        if write:
+            h.data.zero_()
+            h.add_(1)
+        grads.append(torch.autograd.grad(loss, [leaf, w]))
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 8), (127, 72), (129, 264), (1001, 2560), (4096, 64)])
 def test_bias_gradient_sums(ext, rows, cols):
     """Column sums, ragged in rows and in the 64 columns of a CTA: rounded once to bf16 from fp32 sums."""
