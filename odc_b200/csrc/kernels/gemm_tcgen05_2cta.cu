@@ -1595,7 +1595,21 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
     work += static_cast<long long>(shapes[i].tiles) * shapes[i].kb;
     f32 = f32 || !shapes[i].bf16 || g[i].addend != nullptr;
   }
-  if (work > (f32 ? 12000ll : 3000ll) * (sm_count / 2)) return false;
+  if (work > (f32 ? 12000ll : 2700ll) * (sm_count / 2)) return false;
+  // Handing an item on costs 0.2 to 0.5 us that a product of its own does not pay, and in many rounds of items that is more than the
+  // launches and last rounds are, the sooner the shorter the items.  Products one by one and together, us, in bf16 (k-blocks of the
+  // weight gradients, rounds of items): MLP of 4096 and 14336, 256 tokens (4, 36) 164 and 167, 768 (12, 36) 333 and 325; of 5120
+  // and 13824, 64 (1, 44) 161 and 171, 1000 (16, 44) 493 and 494, 2000 (32, 44) 925 and 971; of 2048 and 8192, 64 (1, 10) 57 and 53;
+  // head of 128256 words, 2048 wide, 256 (4, 54) 253 and 271, 1500 (24, 54) 1070 and 1133, of 32000, 4096 wide, 400 (7, 27) 198 and
+  // 202, 768 (12, 27) 296 and 288.  fp32 gradients gain at all of them (first head 547 and 458): their additions to memory run
+  // under the other items.
+  int rounds = 0, shortest = shapes[0].kb;
+  for (int i = 0; i < n; ++i) {
+    rounds += shapes[i].tiles;
+    shortest = std::min(shortest, shapes[i].kb);
+  }
+  rounds /= sm_count / 2;
+  if (n > 1 && !f32 && rounds >= std::min(40, std::max(20, 7 * shortest / 2))) return false;
   plan_group(shapes, n, sm_count / 2);
   return true;
 }

@@ -74,6 +74,19 @@ def test_groups_divide_what_would_outlast_them(T, H, F):
             assert parts == [1, 1, 1]
 
 
+def test_groups_are_not_formed_of_many_items():
+    """Products in bf16 with many rounds of items go one by one, the sooner the fewer the tokens; fp32 ones are taken together."""
+    plan = lambda T, H, F, f32: _ext.load().gemm_group_plan([(T, H, 2 * F, False, False), (2 * F, H, T, f32, f32), (H, F, T, f32, f32)], SMS)
+    for T, H, F, taken in ((64, 5120, 13824, False), (256, 4096, 14336, False), (512, 4096, 14336, False), (768, 4096, 14336, True), (2000, 5120, 13824, False),
+                           (64, 2048, 8192, True), (256, 1536, 8960, True)):
+        assert (plan(T, H, F, False) != [0, 0, 0]) == taken, (T, H, F)
+        assert plan(T, H, F, True) != [0, 0, 0]
+    head = lambda T, f32: _ext.load().gemm_group_plan([(T, 2048, 128256, False, False), (128256, 2048, T, f32, f32)], SMS)
+    for T in (300, 1500):
+        assert head(T, False) == [0, 0] != head(T, True)
+    assert _ext.load().gemm_group_plan([(128256, 2048, 300, False, False)], SMS) != [0]   # nothing else gives it its factor
+
+
 def test_groups_halve_the_tiles_of_what_would_outlast_them():
     columns = lambda *g: _ext.load().gemm_group_columns(list(g), SMS)
     assert columns((300, 1536, 2048, False, False), (2048, 1536, 300, False, False)) == [128, 256]
