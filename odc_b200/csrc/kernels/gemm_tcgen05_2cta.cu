@@ -679,7 +679,18 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       constexpr bool kBias = kMode == kModePlain || kMode == kModeGather || kMode == kModeRope;
       [[maybe_unused]] const bool biased = kBias && p.bias != nullptr && !part;
       if constexpr (kBias) {
-        if (biased && n0 + 8 * lane < p.N) bias8 = *reinterpret_cast<const uint4*>(p.bias + n0 + 8 * lane);
+        if (biased && n0 + 8 * lane < p.N) {
+          const __nv_bfloat16* from = p.bias + n0 + 8 * lane;
+          // a bias may be a view of anything; kModeRope is only launched with one that starts on a 16-byte boundary
+          if (kMode == kModeRope || (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
+            bias8 = *reinterpret_cast<const uint4*>(from);
+          } else {
+            const auto two = [&](int i) {
+              return static_cast<uint32_t>(__bfloat16_as_ushort(from[i])) | static_cast<uint32_t>(__bfloat16_as_ushort(from[i + 1])) << 16;
+            };
+            bias8 = make_uint4(two(0), two(2), two(4), two(6));
+          }
+        }
       }
       // its values of `kCols` columns from `col` on (multiples of 16), added to accumulators
       [[maybe_unused]] auto add_bias = [&](auto n_cols, int col, auto* r) {

@@ -639,6 +639,32 @@ def test_projection_with_rotation(ext, T, H, nq, nkv, d, bias):
     assert torch.equal(out, ext.rope_qkv(_linear(x, w, b), pos, nq, nkv, d, 10000.0, False))
 
 
+@pytest.mark.parametrize("M,N,K", [(300, 264, 128), (1000, 520, 256), (1000, 512, 128), (765, 1536, 8960), (2304, 2304, 4096), (16, 264, 128)])
+@pytest.mark.parametrize("offset", [1, 4])
+def test_bias_that_starts_off_a_16_byte_boundary(ext, M, N, K, offset):
+    """A view of a larger vector, in bf16 and fp32 results, with a residual, in half-width, divided and single-CTA products, gathered
+    weights and the rotary projection: the bytes that the same bias gives at the start of an allocation."""
+    torch.manual_seed(0)
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    bias, res = torch.randn(N + 8, device="cuda").bfloat16()[offset:offset + N], torch.randn(M, N, device="cuda").bfloat16()
+    whole = bias.clone()
+    assert bias.data_ptr() % 16 and whole.data_ptr() % 16 == 0
+
+    def results(b):
+        c, c32 = torch.empty_like(res), torch.ones(M, N, device="cuda")
+        ext.gemm(x, w, c, "nt", b, False, res)
+        ext.gemm(x, w, c32, "nt", b, True)
+        out = [_linear(x, w, b), c, c32]
+        if M >= 256:
+            out.append(ext.gemm_gather(x, _table([w]), torch.empty_like(w), b, N, 0, res))
+        if N == 512:
+            out.append(ext.linear_rope(x, w, b, torch.arange(M, device="cuda"), N // 64 - 4, 2, 64, 10000.0))
+        return out
+    for got, want in zip(results(bias), results(whole)):
+        assert torch.equal(got, want)
+    assert ext.kernel_status()[0].item() == 0, ext.kernel_status().tolist()
+
+
 @pytest.mark.parametrize("T,K,F", [(256, 128, 128), (300, 264, 1000), (520, 2048, 136), (1000, 512, 4160), (16, 128, 256),
                                    (765, 17920, 768)])
 def test_linear_swiglu_matches_the_two_passes(ext, T, K, F):
