@@ -287,6 +287,7 @@ struct Product {
   double scale = 1.0;    // group_into only: of the result
   Tensor times;          // group_into only: a further factor, one fp32 value on the device
   Tensor addend;         // group_into only: contiguous fp32 that joins a bf16 result before it is rounded
+  bool any_order = false;   // group_into only: an accumulating product may add its parts in any order
 };
 bool fixed_order_asked() {
   const char* e = std::getenv("ODC_DETERMINISTIC");
@@ -300,14 +301,14 @@ bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = 
   odc::GemmProduct g[odc::kMaxGroupProducts];
   const bool fixed = fixed_order_asked();
   for (int i = 0; i < n; ++i) {
-    const auto& [a, b, c, lay, accumulate, scale, times, addend] = products[i];
+    const auto& [a, b, c, lay, accumulate, scale, times, addend, any_order] = products[i];
     if (a.dim() != 2 || b.dim() != 2 || c.dim() != 2 || a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16 ||
         (c.scalar_type() != at::kBFloat16 && c.scalar_type() != at::kFloat) || a.stride(1) != 1 || b.stride(1) != 1 || c.stride(1) != 1)
       return false;
     const int64_t K = lay == kTN ? a.size(0) : a.size(1), M = lay == kTN ? a.size(1) : a.size(0), N = lay == kNT ? b.size(0) : b.size(1);
     if ((lay == kNT ? b.size(1) : b.size(0)) != K || c.size(0) != M || c.size(1) != N) return false;
     g[i] = odc::GemmProduct{a.data_ptr(), b.data_ptr(), c.data_ptr(), kind_of(c.scalar_type()), static_cast<int>(M), static_cast<int>(N),
-                            static_cast<int>(K), lay, accumulate, fixed, a.stride(0), b.stride(0), c.stride(0), static_cast<float>(scale),
+                            static_cast<int>(K), lay, accumulate, fixed || !any_order, a.stride(0), b.stride(0), c.stride(0), static_cast<float>(scale),
                             times.defined() ? times.data_ptr<float>() : nullptr, addend.defined() ? addend.data_ptr<float>() : nullptr};
   }
   const Tensor& a = products[0].a;
@@ -1064,7 +1065,8 @@ Tensor sharded_grads(const Tensor& dy2, const ShardedMatrix* m, const std::vecto
       py::gil_scoped_acquire gil;
       to = (*g_local_buffer)(w.m->id).cast<Tensor>().narrow(0, 0, w.m->out_features);
     }
-    todo.push_back({w.dy2, w.x2, to, kTN, true, pushes ? w.m->grad_scale : 1.0});
+    // several parts meet in the accumulator as they do in a launch of its own; the local buffer is a sum in one order
+    todo.push_back({w.dy2, w.x2, to, kTN, true, pushes ? w.m->grad_scale : 1.0, {}, {}, pushes});
   }
   if (todo.size() == weights.size() + 1 && group_into(todo, m->ctr_table, pushes ? static_cast<int>(weights.size()) : 0)) {
     for (const auto& w : weights) {
@@ -1469,30 +1471,34 @@ void register_ops(py::module_& m) {
       int lay = 0;
       while (lay < 3 && layout != kLayoutNames[lay]) ++lay;
       TORCH_CHECK(lay < 3, "gemm_group: unknown layout ", layout);
-      todo.push_back({a, b, c, lay, accumulate, scale});
+      todo.push_back({a, b, c, lay, accumulate, scale, {}, {}, accumulate});
     }
     return group_into(todo);
   });  // (a, b, c, layout, accumulate, scale) each; False: not taken as a group, nothing done
-  m.def("gemm_group_plan", [](std::vector<std::tuple<int, int, int, bool, bool>> products, int sms) {
+  using Shape = std::tuple<int, int, int, bool, bool>;   // (M, N, K, fp32, accumulate)
+  static const auto group_plan = [](const std::vector<Shape>& products, int sms) {
+    TORCH_CHECK(products.size() <= odc::kMaxGroupProducts, "group plan: too many products");
     odc::GemmProduct g[odc::kMaxGroupProducts] = {};
     int n = 0;
     for (auto& [M, N, K, f32, accumulate] : products) {
-      TORCH_CHECK(n < odc::kMaxGroupProducts, "gemm_group_plan: too many products");
       g[n].M = M; g[n].N = N; g[n].K = K; g[n].c_kind = f32 ? odc::kF32 : odc::kBF16; g[n].accumulate = accumulate; g[n++].scale = 1.f;
     }
-    const auto plan = odc::gemm_group_plan(g, n, sms);
-    return std::vector<int>(plan.parts, plan.parts + n);
-  }, py::arg("products"), py::arg("sms"));  // parts of every tile of each (M, N, K, fp32, accumulate)
-  m.def("gemm_group_columns", [](std::vector<std::tuple<int, int, int, bool, bool>> products, int sms) {
-    odc::GemmProduct g[odc::kMaxGroupProducts] = {};
-    int n = 0;
-    for (auto& [M, N, K, f32, accumulate] : products) {
-      TORCH_CHECK(n < odc::kMaxGroupProducts, "gemm_group_columns: too many products");
-      g[n].M = M; g[n].N = N; g[n].K = K; g[n].c_kind = f32 ? odc::kF32 : odc::kBF16; g[n].accumulate = accumulate; g[n++].scale = 1.f;
-    }
-    const auto plan = odc::gemm_group_plan(g, n, sms);
-    return std::vector<int>(plan.columns, plan.columns + n);
+    return odc::gemm_group_plan(g, n, sms);
+  };
+  m.def("gemm_group_plan", [](std::vector<Shape> products, int sms) {
+    const auto plan = group_plan(products, sms);
+    return std::vector<int>(plan.parts, plan.parts + products.size());
+  }, py::arg("products"), py::arg("sms"));  // parts of every tile of each product
+  m.def("gemm_group_columns", [](std::vector<Shape> products, int sms) {
+    const auto plan = group_plan(products, sms);
+    return std::vector<int>(plan.columns, plan.columns + products.size());
   }, py::arg("products"), py::arg("sms"));  // columns of a tile of each
+  m.def("gemm_group_tiles", [](std::vector<Shape> products, int sms) {
+    const auto plan = group_plan(products, sms);
+    std::vector<std::tuple<int, int, int>> out;
+    for (size_t i = 0; i < products.size(); ++i) out.emplace_back(plan.tiles[i].tiles, plan.tiles[i].whole, plan.tiles[i].parts);
+    return out;
+  }, py::arg("products"), py::arg("sms"));  // (tiles, whole ones, parts of each other) of each
   m.def("scatter_plan", [](int n_out, int k_in, int tokens, int ranks, int sms) {
     const odc::GemmPlan p = odc::scatter_plan(n_out, k_in, tokens, ranks, sms);
     return std::make_tuple(p.tiles, p.whole, p.parts);

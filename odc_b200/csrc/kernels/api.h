@@ -141,7 +141,7 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
 // keeps what it got, nor after a wait has run out).
 // cudaErrorNotSupported: one by one.
 constexpr int kMaxGroupProducts = 3;
-constexpr int kMaxGroupDivided = 256;   // divided tiles of a launch
+constexpr int kMaxGroupDivided = 512;   // divided tiles of a launch: those of two rounds of pairs for each product, at most
 constexpr int kGroupLaunchWords = 2 + 2 * kMaxGroupDivided;
 struct GemmProduct {
   const void *a, *b;
@@ -154,8 +154,9 @@ struct GemmProduct {
   const float* addend;   // bf16 C: fp32 [M, N], joins the sum before scale and rounding
 };
 struct GemmGroupPlan {
-  int parts[kMaxGroupProducts];     // of every tile; 0: not taken as a group
+  int parts[kMaxGroupProducts];     // of every tile (1 where some are whole); 0: not taken as a group
   int columns[kMaxGroupProducts];   // of a tile
+  GemmPlan tiles[kMaxGroupProducts];
 };
 GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count);
 size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count);

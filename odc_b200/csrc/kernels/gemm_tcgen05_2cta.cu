@@ -143,8 +143,8 @@ struct GroupProblem {
   const float* scale_ptr;
   const float* addend;      // bf16 results: fp32 [M, N] that joins the sum before it is rounded, or null
   int first;                // its first item
-  int splits, kb_split;     // work items per tile, k-blocks of each
-  int first_split_tile, first_part;   // bf16 with splits > 1: of its first tile, among the divided tiles and parts of the launch
+  int whole, splits, kb_split;   // the first `whole` tiles are items, every other tile is `splits` of kb_split k-blocks each
+  int first_split_tile, first_part;   // bf16 with divided tiles: of the first of them, among the divided tiles and parts of the launch
 };
 struct Group {
   CUtensorMap a[kMaxGroup], b[kMaxGroup], c[kMaxGroup];
@@ -347,17 +347,19 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     }
   };
   // where an item lies; group modes only
-  struct Place { int pi, tm, tn, kb0, kb1, part; };
+  struct Place { int pi, tm, tn, kb0, kb1, part, divided; };   // divided: which of its product's divided tiles, or -1
   [[maybe_unused]] auto place_of = [&](int item) -> Place {
     Place w{};
     if constexpr (kMode == kModeGroup) {
       while (w.pi + 1 < owners.count && item >= owners.prob[w.pi + 1].first) ++w.pi;
       const GroupProblem& q = owners.prob[w.pi];
-      const int local = item - q.first, tile = q.splits > 1 ? local / q.splits : local;
-      w.part = local - tile * q.splits;
-      tile_coords(tile, q, 0, 0, &w.tm, &w.tn);
+      const int local = item - q.first, beyond = local - q.whole;
+      w.divided = beyond < 0 ? -1 : beyond / q.splits;
+      w.part = beyond < 0 ? 0 : beyond - w.divided * q.splits;
+      tile_coords(beyond < 0 ? local : q.whole + w.divided, q, 0, 0, &w.tm, &w.tn);
       w.kb0 = w.part * q.kb_split;
-      w.kb1 = min((q.K + BK - 1) / BK, w.kb0 + q.kb_split);
+      w.kb1 = (q.K + BK - 1) / BK;
+      if (beyond >= 0) w.kb1 = min(w.kb1, w.kb0 + q.kb_split);
     }
     return w;
   };
@@ -838,10 +840,10 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             // A part: 16 bytes of 128 rows next to one another, so that a warp writes and reads whole lines.
             const float4* others = nullptr;
             bool mine = true;
-            if (q.splits > 1) {
-              const int tile = q.first_split_tile + (item - q.first) / q.splits;
+            if (place.divided >= 0) {
+              const int tile = q.first_split_tile + place.divided;
               // parts of the tile, this CTA's half of each
-              float4* at = owners.parts + ((q.first_part + static_cast<long long>(item - q.first - place.part)) * 2 + cta) * (64 * 128) + my_row;
+              float4* at = owners.parts + ((q.first_part + static_cast<long long>(place.divided) * q.splits) * 2 + cta) * (64 * 128) + my_row;
               float4* own = at + static_cast<long long>(place.part) * (2 * 64 * 128);
 #pragma unroll 1
               for (int col = 0; col < cols; col += 32) {
@@ -1503,7 +1505,7 @@ cudaError_t gemm_logits_pair(const void* h, const void* w, void* logits, const l
 }
 
 // Words for the launches of groups, zero at load and left zero by each: the counter of items, the count of finished CTAs, and two
-// per divided tile.  They are handed out in turn and come round again after at least kGroupWords / kGroupLaunchWords (2040)
+// per divided tile.  They are handed out in turn and come round again after at least kGroupWords / kGroupLaunchWords (1022)
 // launches, more than a device holds queued; a captured launch runs again at any time and brings its own.
 constexpr unsigned int kGroupWords = 1u << 20;
 __device__ unsigned int g_group_words[kGroupWords];
@@ -1524,19 +1526,40 @@ static unsigned int* group_words(int n) {
   return base[dev] + at - n;
 }
 
-// How wide the tiles of each product are and into how many parts they are divided.  In units of a k-block (0.28 us): the items go to
-// the pairs that are free first, longest first, so the group takes the work per pair and half of its last item, but at least its
-// longest item, and a second round besides costs 6 (the items are handed on from CTA to CTA, the first epilogues are in the way).
-// An item takes at least what its epilogue does (6) and 2 to begin with; a part of a bf16 tile writes and reads 256 KB of fp32 (6),
-// the parts of an fp32 sum meet in memory.  The longest item is made half as wide, or divided, as long as that gains a twentieth.
-// 300 tokens, 1536 wide: half as wide 15.3 -> 12.5 us (projection), MLP of 512 and 1536 19.5 -> 15.4.
+// How wide the tiles of each product are, in units of a k-block (0.28 us): the items go to the pairs that are free first, longest
+// first, so the group takes the work per pair and half of its last item, but at least its longest item, and a second round besides
+// costs 6 (the items are handed on from CTA to CTA, the first epilogues are in the way).  An item takes at least what its epilogue
+// does (6) and 2 to begin with; a part of a bf16 tile writes and reads 256 KB of fp32 (6), the parts of an fp32 sum meet in memory.
+// The longest item is made half as wide as long as that gains a twentieth.  300 tokens, 1536 wide: half as wide 15.3 -> 12.5 us
+// (projection), MLP of 512 and 1536 19.5 -> 15.4.
 struct GroupShape {
-  int tiles, kb, splits, each;
-  bool may_divide, bf16;
+  int tiles, kb;
+  SplitPlan plan;
+  bool bf16;
   int bn, half_tiles, layout;   // columns of a tile; how many tiles of half the width there are
-  double item() const { return std::max(6.0, each * (bn == 128 ? half_tile_time(layout) : 1.0)) + 2 + (splits > 1 ? (bf16 ? 6.0 : 1.0) : 0.0); }
-  double sum() const { return bf16 && splits > 1 ? 12.0 + 8.0 * (splits - 1) : 0.0; }
+  int divided() const { return tiles - plan.whole; }
+  int parts() const { return divided() * plan.splits; }
+  double time(int k_blocks, bool part) const {
+    return std::max(6.0, k_blocks * (bn == 128 ? half_tile_time(layout) : 1.0)) + 2 + (part ? (bf16 ? 6.0 : 1.0) : 0.0);
+  }
+  double item() const { return plan.whole > 0 ? time(kb, false) : time(plan.kb_split, true); }   // the longest
+  double sum() const { return bf16 && parts() > 0 ? 12.0 + 8.0 * (plan.splits - 1) : 0.0; }
+  double work() const { return plan.whole * time(kb, false) + (parts() > 0 ? parts() * time(plan.kb_split, true) : 0.0); }
 };
+// Into how many parts: as the product by itself would be, so that a sum is no longer than there, and the bytes of a bf16 result are
+// the same either way.  The tensor cores drop what does not fit behind an accumulator's last bit, 1e-9 of the result for every product in
+// one sum: 1.8e-6 over 2048, 1.8e-5 over 17920, 1.3e-4 over 131072.  Left whole under the other products' arithmetic, as three
+// parts had not been, the hidden states' gradient over 151936 words went from 8.3e-5 to 1.2e-4 (2.3526e-3 to 2.3602e-3 from 64
+// bits in all).  Sums over no more than 2048 (1.8e-6) stay whole: there a product by itself divides its last one to eight tiles at most.
+// What is added to fp32 in any order is divided as in a launch of its own (scatter_plan); addends and sums in one order are not.
+constexpr int kGroupShortSum = 2048 / gemm_pair::BK;
+static SplitPlan group_split(const GemmProduct& q, int tiles, int sm_count) {
+  using namespace gemm_pair;
+  const int kb = (q.K + BK - 1) / BK;
+  if (q.c_kind == kBF16 && q.addend == nullptr && kb > kGroupShortSum) return product_plan(q.M, q.N, q.K, sm_count);
+  if (q.c_kind == kF32 && q.accumulate && !q.fixed_order) return plan_splits(q.M, q.N, q.K, sm_count, scatter_cost(1), true);
+  return {tiles, 1, kb};
+}
 static void plan_group(GroupShape* g, int n, int pairs) {
   auto cost = [&] {
     int order[kMaxGroupProducts];
@@ -1546,42 +1569,29 @@ static void plan_group(GroupShape* g, int n, int pairs) {
     int all = 0;
     for (int i = 0; i < n; ++i) {
       const GroupShape& q = g[order[i]];
-      const int items = q.tiles * q.splits;
-      work += items * q.item();
+      const int items = q.plan.whole + q.parts();
+      work += q.work();
       all += items;
-      const double end = all <= pairs ? q.item() : i == 0 ? (items + pairs - 1) / pairs * q.item() : work / pairs + 0.5 * q.item();
+      const double end = all <= pairs ? q.item() : i == 0 ? (items + pairs - 1) / pairs * (q.work() / items) : work / pairs + 0.5 * q.item();
       span = std::max(span, end + q.sum());
     }
     return span + (all > pairs ? 6.0 : 0.0);
   };
-  for (int i = 0; i < n; ++i) { g[i].splits = 1; g[i].each = g[i].kb; }
-  double best = cost();
-  while (true) {
+  for (double best = cost();;) {
     int longest = 0;
     for (int i = 1; i < n; ++i)
       if (g[i].item() > g[longest].item()) longest = i;
     GroupShape& q = g[longest];
+    if (q.bn != 256 || q.parts() > 0) return;
     const GroupShape before = q;
-    GroupShape better = before;
-    double least = 0.95 * best;
-    const auto consider = [&] {
-      if (const double c = cost(); c < least) { least = c; better = q; }
+    q.bn = 128;
+    q.tiles = q.plan.whole = q.half_tiles;
+    const double c = cost();
+    if (c >= 0.95 * best) {
       q = before;
-    };
-    if (q.bn == 256 && q.splits == 1) {   // no sum of parts
-      q.bn = 128;
-      q.tiles = q.half_tiles;
-      consider();
+      return;
     }
-    for (int want = before.splits + 1; want <= 8 && q.may_divide; ++want) {
-      const int each = (q.kb + want - 1) / want, s = (q.kb + each - 1) / each;   // no empty part
-      if (s <= before.splits || each < 4 || (q.bf16 && q.tiles > kMaxGroupDivided)) continue;
-      q.splits = s; q.each = each;
-      consider();
-    }
-    if (better.bn == before.bn && better.splits == before.splits) return;
-    q = better;
-    best = least;
+    best = c;
   }
 }
 
@@ -1591,9 +1601,9 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
   for (int i = 0; i < n; ++i) {
     const GemmProduct& q = g[i];
     if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate)) || (q.addend != nullptr && q.c_kind != kBF16)) return false;
-    shapes[i] = GroupShape{(q.M + 255) / 256 * ((q.N + BN - 1) / BN), (q.K + BK - 1) / BK, 1, 0,
-                           q.c_kind == kBF16 ? q.addend == nullptr : q.accumulate && !q.fixed_order, q.c_kind == kBF16,
-                           BN, (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
+    const int tiles = (q.M + 255) / 256 * ((q.N + BN - 1) / BN);
+    shapes[i] = GroupShape{tiles, (q.K + BK - 1) / BK, group_split(q, tiles, sm_count), q.c_kind == kBF16, BN,
+                           (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
   }
   // A group saves the launches and last rounds of its products, 30 to 100 units.  With more work than this for a pair that is no
   // gain any more, and pairs that are not in step with one another share less of L2 (16321 tokens, 2048 and 8192 wide, 4400 units:
@@ -1630,7 +1640,7 @@ size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count) {
   if (!group_shapes(g, n, sm_count, shapes)) return 0;
   size_t parts = 0;
   for (int i = 0; i < n; ++i)
-    if (shapes[i].bf16 && shapes[i].splits > 1) parts += static_cast<size_t>(shapes[i].tiles) * shapes[i].splits;
+    if (shapes[i].bf16) parts += static_cast<size_t>(shapes[i].parts());
   return parts * 256 * gemm_pair::BN * sizeof(float);
 }
 
@@ -1638,7 +1648,12 @@ GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count) {
   GroupShape shapes[kMaxGroupProducts];
   GemmGroupPlan plan{};
   if (!group_shapes(g, n, sm_count, shapes)) return plan;
-  for (int i = 0; i < n; ++i) { plan.parts[i] = shapes[i].splits; plan.columns[i] = shapes[i].bn; }
+  for (int i = 0; i < n; ++i) {
+    const SplitPlan& split = shapes[i].plan;
+    plan.parts[i] = split.whole > 0 ? 1 : split.splits;
+    plan.columns[i] = shapes[i].bn;
+    plan.tiles[i] = {shapes[i].tiles, split.whole, split.splits, 0};
+  }
   return plan;
 }
 
@@ -1680,12 +1695,12 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int
     t.out = q.c_kind == kBF16 ? 0 : q.accumulate ? 2 : 1;
     t.scale = q.scale; t.scale_ptr = q.scale_ptr; t.addend = q.addend;
     t.first = group.items;
-    t.splits = shape.splits; t.kb_split = shape.each;
-    if (shape.bf16 && shape.splits > 1) {
+    t.whole = shape.plan.whole; t.splits = shape.plan.splits; t.kb_split = shape.plan.kb_split;
+    if (shape.bf16) {
       t.first_split_tile = divided; t.first_part = parts;
-      divided += shape.tiles; parts += shape.tiles * shape.splits;
+      divided += shape.divided(); parts += shape.parts();
     }
-    group.items += shape.tiles * shape.splits;
+    group.items += shape.plan.whole + shape.parts();
   }
   group.count = n;
   if (divided > kMaxGroupDivided || (divided > 0 && scratch == nullptr)) return cudaErrorNotSupported;

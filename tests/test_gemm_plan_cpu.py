@@ -74,6 +74,19 @@ def test_groups_divide_what_would_outlast_them(T, H, F):
             assert parts == [1, 1, 1]
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 256, 4096), (765, 1536, 17920), (1904, 1536, 151936), (4096, 1536, 151936), (3072, 2048, 8200),
+                                   (2304, 2304, 4096), (4096, 4096, 28672), (16321, 2048, 16384), (300, 392, 2112)])
+def test_sums_are_as_short_in_a_group_as_in_a_launch_of_their_own(M, N, K):
+    """A bf16 product keeps its own parts whatever stands next to it, and so does a weight gradient that is added in any order."""
+    ext = _ext.load()
+    for neighbours in ([], [(N, 512, M, True, True)], [(4096, 512, M, False, False), (512, 2048, M, False, False)]):
+        got = ext.gemm_group_tiles([(M, N, K, False, False)] + neighbours, SMS)
+        assert got[0][1:] == _plan(M, N, K)[1:3] or (_plan(M, N, K)[2] == 1 and got[0][2] == 1)
+        if neighbours and neighbours[0][3]:
+            tiles, whole, parts = ext.scatter_plan(N, 512, M, 1, SMS)
+            assert got[1][2] == parts and (parts == 1 or got[1] == (tiles, whole, parts))
+
+
 def test_groups_are_not_formed_of_many_items():
     """Products in bf16 with many rounds of items go one by one, the sooner the fewer the tokens; fp32 ones are taken together."""
     plan = lambda T, H, F, f32: _ext.load().gemm_group_plan([(T, H, 2 * F, False, False), (2 * F, H, T, f32, f32), (H, F, T, f32, f32)], SMS)

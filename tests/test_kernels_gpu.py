@@ -471,6 +471,22 @@ def test_groups_of_products(ext, parts, products):
             assert ((c.double() - want).abs() <= bound).all(), (lay, plan)
 
 
+@pytest.mark.parametrize("products", [
+    # all tiles in parts, those of the last round, none; ragged edges; next to products of other kinds
+    [("nn", 765, 1536, 17920), ("tn", 17920, 1536, 765), ("tn", 1536, 8960, 765)],
+    [("nn", 4090, 1544, 20000), ("tn", 1024, 1544, 4090)],
+    [("tn", 3072, 2056, 8200), ("nn", 2304, 2304, 4096), ("nt", 300, 264, 8200)],
+    [("nn", 2304, 2304, 4096)], [("tn", 264, 264, 4040)], [("nn", 600, 520, 200), ("tn", 520, 200 * 8, 600)]])
+def test_groups_give_the_bytes_of_single_products(ext, products):
+    """A bf16 result does not depend on what is formed in the same launch: its sum is divided as in a launch of its own."""
+    ops = [case[:4] for case in _group_case([(lay, M, N, K, torch.bfloat16, False, 1.0) for lay, M, N, K in products])]
+    assert ext.gemm_group([(a, b, c, lay, False, 1.0) for a, b, c, lay in ops])
+    for a, b, c, lay in ops:
+        alone = torch.empty_like(c)
+        ext.gemm(a, b, alone, lay, None, False)
+        assert torch.equal(c, alone), (lay, *c.shape)
+
+
 def test_parts_of_a_group_are_summed_in_one_order(ext):
     """Eight parts and as many CTAs that may come last: the same bytes every time, in a replayed graph as well."""
     torch.manual_seed(0)
@@ -744,6 +760,21 @@ def test_loss_lets_its_input_be_written_to(chunk):
             h.data.zero_()
             h.add_(1)
         grads.append(torch.autograd.grad(loss, [leaf, w]))
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+def test_weight_gradient_of_several_chunks_is_summed_in_one_order(monkeypatch):
+    """Chunks are added to the fp32 matrix one after the other, each as one sum: the same bytes with and without a fixed order asked for."""
+    from odc_b200 import ops
+    torch.manual_seed(0)
+    T, H, V = 6000, 256, 1024
+    h = torch.randn(T, H, device="cuda").bfloat16().requires_grad_()
+    w = (0.05 * torch.randn(V, H, device="cuda")).bfloat16().requires_grad_()
+    labels = torch.randint(0, V, (T,), device="cuda")
+    grads = []
+    for fixed in ("0", "1"):
+        monkeypatch.setenv("ODC_DETERMINISTIC", fixed)
+        grads.append(torch.autograd.grad(ops.linear_cross_entropy(h, w, labels, chunk=3000), [h, w]))
     assert all(torch.equal(a, b) for a, b in zip(*grads))
 
 
