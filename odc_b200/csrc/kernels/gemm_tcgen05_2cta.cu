@@ -1373,13 +1373,13 @@ cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* 
 // out[M, N] = x w^T (+ bias), w [N, K], with the columns below rot_cols, heads of 64 or 128, rotated by pos[row] (rotary base theta;
 // halves of a head are the pairs, as in launch_rope_qkv): the rotation is not a pass over the projection (16321 tokens, 32 + 16
 // heads of 64: 45 us), and runs while the next tile is multiplied.  The same bytes as the two passes: rounded, rotated, rounded.
-// cudaErrorNotSupported where the plain product and the pass are the better form.
+// cudaErrorNotSupported where the product by itself would be divided, all of it or its last round (528 to 608 x 7168 x 5120): then the
+// product and the pass.
 cudaError_t gemm_rope_pair(const void* x, const void* w, const void* bias, void* out, const long long* pos, int M, int N, int K,
                            long long ldx, long long ldw, int rot_cols, int head_dim, float theta, int* status, int sm_count,
                            cudaStream_t stream) {
   using namespace gemm_pair;
-  if (M < 256 || N < 256 || K < BK || sm_count < 2 || plan_splits(M, N, K, sm_count, kPartialsCost, false).splits > 1)
-    return cudaErrorNotSupported;
+  if (M < 256 || N < 256 || K < BK || sm_count < 2 || product_plan(M, N, K, sm_count).splits > 1) return cudaErrorNotSupported;
   if ((head_dim != 64 && head_dim != 128) || rot_cols % head_dim || N % 64 || rot_cols > N || (ldx % 8) || (ldw % 8) ||
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out) |
         reinterpret_cast<uintptr_t>(bias)) & 15))

@@ -644,9 +644,10 @@ def _linear(x, w, b):
 
 @pytest.mark.parametrize("T,H,nq,nkv,d,bias", [(256, 64, 2, 1, 64, False), (300, 264, 5, 1, 64, True), (1000, 512, 8, 2, 64, False),
                                                (256, 128, 1, 1, 128, True), (520, 200, 12, 2, 128, True), (16, 128, 4, 4, 64, True),
-                                               (300, 8960, 4, 1, 128, False), (2600, 2048, 32, 8, 64, False)])
+                                               (300, 8960, 4, 1, 128, False), (2600, 2048, 32, 8, 64, False), (560, 5120, 40, 8, 128, True)])
 def test_projection_with_rotation(ext, T, H, nq, nkv, d, bias):
-    """The bytes of the product and the pass over it.  Fewer rows than a tile and divided products take those."""
+    """The bytes of the product and the pass over it.  Fewer rows than a tile and products divided as a whole or in their last round take
+    those."""
     torch.manual_seed(0)
     x, w = torch.randn(T, H, device="cuda").bfloat16(), (torch.randn((nq + 2 * nkv) * d, H, device="cuda") * H ** -0.5).bfloat16()
     b = torch.randn(w.shape[0], device="cuda").bfloat16() if bias else None
