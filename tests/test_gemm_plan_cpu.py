@@ -79,12 +79,18 @@ def test_groups_divide_what_would_outlast_them(T, H, F):
 def test_sums_are_as_short_in_a_group_as_in_a_launch_of_their_own(M, N, K):
     """A bf16 product keeps its own parts whatever stands next to it, and so does a weight gradient that is added in any order."""
     ext = _ext.load()
-    for neighbours in ([], [(N, 512, M, True, True)], [(4096, 512, M, False, False), (512, 2048, M, False, False)]):
-        got = ext.gemm_group_tiles([(M, N, K, False, False)] + neighbours, SMS)
+    taken = 0
+    for neighbours in ([], [(N, 512, max(M, 64), True, True)], [(4096, 512, 300, False, False), (512, 2048, 300, False, False)]):
+        products = [(M, N, K, False, False)] + neighbours
+        got = ext.gemm_group_tiles(products, SMS)
+        if 0 in ext.gemm_group_plan(products, SMS):   # much work in bf16
+            continue
+        taken += 1
         assert got[0][1:] == _plan(M, N, K)[1:3] or (_plan(M, N, K)[2] == 1 and got[0][2] == 1)
         if neighbours and neighbours[0][3]:
-            tiles, whole, parts = ext.scatter_plan(N, 512, M, 1, SMS)
+            tiles, whole, parts = ext.scatter_plan(N, 512, max(M, 64), 1, SMS)
             assert got[1][2] == parts and (parts == 1 or got[1] == (tiles, whole, parts))
+    assert taken
 
 
 def test_groups_are_not_formed_of_many_items():
