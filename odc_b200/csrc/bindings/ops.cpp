@@ -862,11 +862,24 @@ std::tuple<Tensor, Tensor, Tensor> lm_head_loss(const Tensor& h, const Tensor& w
 // that multiplies it (128256 words, 2048 wide: 2.1 of 2.6 GB).  What waits for the backward is no larger than that matrix, or small.
 // Loss and gradients of 256 tokens 720 us with the matrix, 452 without, of 1000 1540 and 1255, 4096 wide 1380 and 830; 4096 tokens
 // the same.  Smallest training step, whose weight gradient goes straight to the accumulator: 1545 and 1367 us.
-bool keeps_logit_grads(const Tensor& h, const Tensor& w, int64_t chunk, bool need_dw) {
+// Only where the kernel takes the products that are to gain by it, the weight's gradient alone or, `sharded`, both gradients: else the
+// fp32 matrix would be formed after all, next to what has been kept (4000 tokens, 128256 words, 2048 wide: a peak of 3.0 GB instead of 2.0).
+bool logit_grads_pay(int64_t T, int64_t V, int64_t H, int64_t chunk, bool sharded, int sms) {
   constexpr int64_t kSmall = 128 << 20;
-  const int64_t T = h.size(0), kept = T * w.size(0) * 2, instead = w.numel() * 4;
-  return need_dw && T > 0 && T <= chunk && (kept <= instead || kept <= kSmall) && h.scalar_type() == at::kBFloat16 &&
-         w.scalar_type() == at::kBFloat16 && !library_gemm();
+  const int64_t kept = T * V * 2, instead = V * H * 4;
+  if (T < 1 || T > chunk || (kept > instead && kept > kSmall)) return false;
+  odc::GemmProduct g[2] = {};
+  g[0].M = static_cast<int>(V); g[0].N = static_cast<int>(H); g[0].K = static_cast<int>(T);
+  g[0].layout = kTN; g[0].lda = V; g[0].ldb = g[0].ldc = H;
+  g[0].c_kind = sharded ? odc::kF32 : odc::kBF16;
+  g[1].M = static_cast<int>(T); g[1].N = static_cast<int>(H); g[1].K = static_cast<int>(V);
+  g[1].layout = kNN; g[1].lda = V; g[1].ldb = g[1].ldc = H;
+  g[1].c_kind = odc::kBF16;
+  return odc::gemm_group_takes(g, sharded ? 2 : 1, sms);
+}
+bool keeps_logit_grads(const Tensor& h, const Tensor& w, int64_t chunk, bool need_dw, bool sharded) {
+  return need_dw && h.dim() == 2 && h.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && !library_gemm() &&
+         odc::gemm_pairs_enabled() && logit_grads_pay(h.size(0), w.size(0), h.size(1), chunk, sharded, sm_count());
 }
 std::tuple<Tensor, Tensor> loss_and_logit_grads(const Tensor& h, const Tensor& w, const Tensor& labels, const c10::optional<Tensor>& loss_scale,
                                                 int64_t ignore_index) {
@@ -887,7 +900,7 @@ struct LinearCrossEntropyFn : Function<LinearCrossEntropyFn> {
   static Tensor forward(AutogradContext* ctx, Tensor h, Tensor w, Tensor labels, c10::optional<Tensor> loss_scale,
                         int64_t ignore_index, int64_t chunk, bool need_dh, bool need_dw) {
     check_chunk(chunk);
-    if (keeps_logit_grads(h, w, chunk, need_dw)) {
+    if (keeps_logit_grads(h, w, chunk, need_dw, false)) {
       auto [loss, dlogits] = loss_and_logit_grads(h, w, labels, loss_scale, ignore_index);
       Tensor dh;
       if (need_dh) dh = product(dlogits, w, kNN);
@@ -1105,12 +1118,11 @@ Tensor sharded_head_grads(const Tensor& dlogits, const Tensor& h, const Tensor& 
   if (direct || add) {
     const Tensor dw32 = product(dlogits, h, kTN, {}, {}, at::kFloat);
     if (direct) {
-      const Tensor scaled = dw32.mul_(g32);
-      check(odc::launch_scatter_accumulate(scaled.data_ptr(), odc::kF32, reinterpret_cast<const long long*>(m->acc_table.data_ptr<int64_t>()),
+      check(odc::launch_scatter_accumulate(dw32.data_ptr(), odc::kF32, reinterpret_cast<const long long*>(m->acc_table.data_ptr<int64_t>()),
                                            odc::kF32, reinterpret_cast<const long long*>(m->ctr_table.data_ptr<int64_t>()),
-                                           static_cast<size_t>(scaled.numel()), 1, 0, static_cast<float>(m->grad_scale),
+                                           static_cast<size_t>(dw32.numel()), 1, 0, static_cast<float>(m->grad_scale),
                                            next_done_slot(h.get_device()), sm_count(), cur_stream(),
-                                           device_status(h.get_device()).data_ptr<int>(), 0, nullptr), "head gradient");
+                                           device_status(h.get_device()).data_ptr<int>(), 0, g32.data_ptr<float>()), "head gradient");
       count();
       m->dispatched->n.fetch_add(1);
     } else {
@@ -1577,7 +1589,10 @@ void register_ops(py::module_& m) {
   m.def("attention_qkv", &attention_qkv);
   m.def("linear_cross_entropy", &linear_cross_entropy);
   m.def("linear_token_logprobs", &linear_token_logprobs);
-  m.def("head_keeps_logit_grads", &keeps_logit_grads, py::arg("h"), py::arg("w"), py::arg("chunk"), py::arg("need_dw") = true);
+  m.def("head_keeps_logit_grads", &keeps_logit_grads, py::arg("h"), py::arg("w"), py::arg("chunk"), py::arg("need_dw") = true,
+        py::arg("sharded") = true);
+  m.def("logit_grads_pay", &logit_grads_pay, py::arg("tokens"), py::arg("words"), py::arg("width"), py::arg("chunk"), py::arg("sharded"),
+        py::arg("sms"));
   m.def("loss_and_logit_grads", &loss_and_logit_grads);
   m.def("sharded_head_grads", &sharded_head_grads, py::arg("dlogits"), py::arg("h"), py::arg("w"), py::arg("g"), py::arg("matrix"),
         py::arg("local") = py::none(), py::arg("add") = false);

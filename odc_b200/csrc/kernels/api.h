@@ -159,6 +159,7 @@ struct GemmGroupPlan {
   GemmPlan tiles[kMaxGroupProducts];
 };
 GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count);
+bool gemm_group_takes(const GemmProduct* g, int n, int sm_count);   // what gemm_group answers with cudaErrorNotSupported is false
 size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count);
 cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,
                        int* status, int sm_count, cudaStream_t stream);

@@ -1657,18 +1657,27 @@ GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count) {
   return plan;
 }
 
+static bool group_takes(const GemmProduct* g, int n, int sm_count, GroupShape* shapes) {
+  if (!group_shapes(g, n, sm_count, shapes)) return false;
+  for (int i = 0; i < n; ++i) {
+    const GemmProduct& q = g[i];
+    if ((reinterpret_cast<uintptr_t>(q.a) | reinterpret_cast<uintptr_t>(q.b) | reinterpret_cast<uintptr_t>(q.c) |
+         reinterpret_cast<uintptr_t>(q.addend)) & 15)
+      return false;
+    if ((q.lda % 8) || (q.ldb % 8) || (q.N % 8) || (q.layout == 2 && q.M % 8) || (q.ldc % (q.c_kind == kF32 ? 4 : 8))) return false;
+  }
+  return true;
+}
+bool gemm_group_takes(const GemmProduct* g, int n, int sm_count) {
+  GroupShape shapes[kMaxGroupProducts];
+  return group_takes(g, n, sm_count, shapes);
+}
+
 cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,
                        int* status, int sm_count, cudaStream_t stream) {
   using namespace gemm_pair;
   GroupShape shapes[kMaxGroup];
-  if (!group_shapes(g, n, sm_count, shapes)) return cudaErrorNotSupported;
-  for (int i = 0; i < n; ++i) {
-    const GemmProduct& q = g[i];
-    if ((reinterpret_cast<uintptr_t>(q.a) | reinterpret_cast<uintptr_t>(q.b) | reinterpret_cast<uintptr_t>(q.c)) & 15)
-      return cudaErrorNotSupported;
-    if (reinterpret_cast<uintptr_t>(q.addend) & 15) return cudaErrorNotSupported;
-    if ((q.lda % 8) || (q.ldb % 8) || (q.N % 8) || (q.layout == 2 && q.M % 8) || (q.ldc % (q.c_kind == kF32 ? 4 : 8))) return cudaErrorNotSupported;
-  }
+  if (!group_takes(g, n, sm_count, shapes)) return cudaErrorNotSupported;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {

@@ -121,3 +121,25 @@ def test_statistics_in_the_product_where_they_pay():
         for rows, words, width in ((255, 128256, 2048), (256, 4096, 512), (300, 8192, 2048), (1200, 1024, 4096), (4096, 200, 512)):
             assert not plan(rows, words, width, gradient), (rows, words, width)
     assert plan(4096, 128256, 512, False) and not plan(4096, 128256, 512, True)
+
+
+@pytest.mark.parametrize("sharded", [False, True])
+@pytest.mark.parametrize("words,width", [(128256, 2048), (128256, 4096), (152064, 5120), (4096, 512), (32000, 4096), (1000, 200), (1001, 256)])
+def test_the_loss_keeps_what_its_products_are_going_to_read(words, width, sharded):
+    """The logits' gradient waits for the backward only where the launch that is to read it will be taken, alone or with the input
+    gradient; where it is not, the fp32 matrix would be formed next to it."""
+    ext, kept = _ext.load(), []
+    for tokens in (1, 64, 300, 1000, 1600, 2400, 3300, 3600, 4096, 5000):
+        products = [(words, width, tokens, sharded, False)] + ([(tokens, width, words, False, False)] if sharded else [])
+        taken = 0 not in ext.gemm_group_plan(products, SMS) and words % 8 == 0
+        fits = tokens <= 4096 and (tokens * words * 2 <= words * width * 4 or tokens * words * 2 <= 128 << 20)
+        kept.append(ext.logit_grads_pay(tokens, words, width, 4096, sharded, SMS))
+        assert kept[-1] == (taken and fits), tokens
+    assert (True in kept) == (words % 8 == 0 and width >= 256) and not kept[-1]
+
+
+def test_the_loss_forms_the_weight_gradient_at_once_where_its_product_is_refused():
+    pays = lambda *a: _ext.load().logit_grads_pay(*a, 4096, sharded, SMS)
+    for sharded, first, last in ((False, (1600, 128256, 2048), (3300, 128256, 2048)), (False, (800, 152064, 5120), (1200, 152064, 5120)),
+                                 (True, (3300, 128256, 4096), (3600, 128256, 4096)), (True, (2200, 152064, 5120), (2500, 152064, 5120))):
+        assert pays(*first) and not pays(*last)
