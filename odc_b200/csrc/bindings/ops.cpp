@@ -288,6 +288,7 @@ struct Product {
   Tensor times;          // group_into only: a further factor, one fp32 value on the device
   Tensor addend;         // group_into only: contiguous fp32 that joins a bf16 result before it is rounded
   bool any_order = false;   // group_into only: an accumulating product may add its parts in any order
+  bool whole = false;       // group_into only: a bf16 product is one sum
 };
 bool fixed_order_asked() {
   const char* e = std::getenv("ODC_DETERMINISTIC");
@@ -301,14 +302,15 @@ bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = 
   odc::GemmProduct g[odc::kMaxGroupProducts];
   const bool fixed = fixed_order_asked();
   for (int i = 0; i < n; ++i) {
-    const auto& [a, b, c, lay, accumulate, scale, times, addend, any_order] = products[i];
+    const auto& [a, b, c, lay, accumulate, scale, times, addend, any_order, whole] = products[i];
     if (a.dim() != 2 || b.dim() != 2 || c.dim() != 2 || a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16 ||
         (c.scalar_type() != at::kBFloat16 && c.scalar_type() != at::kFloat) || a.stride(1) != 1 || b.stride(1) != 1 || c.stride(1) != 1)
       return false;
     const int64_t K = lay == kTN ? a.size(0) : a.size(1), M = lay == kTN ? a.size(1) : a.size(0), N = lay == kNT ? b.size(0) : b.size(1);
     if ((lay == kNT ? b.size(1) : b.size(0)) != K || c.size(0) != M || c.size(1) != N) return false;
     g[i] = odc::GemmProduct{a.data_ptr(), b.data_ptr(), c.data_ptr(), kind_of(c.scalar_type()), static_cast<int>(M), static_cast<int>(N),
-                            static_cast<int>(K), lay, accumulate, fixed || !any_order, a.stride(0), b.stride(0), c.stride(0), static_cast<float>(scale),
+                            static_cast<int>(K), lay, accumulate,
+                            c.scalar_type() == at::kFloat ? fixed || !any_order : whole, a.stride(0), b.stride(0), c.stride(0), static_cast<float>(scale),
                             times.defined() ? times.data_ptr<float>() : nullptr, addend.defined() ? addend.data_ptr<float>() : nullptr};
   }
   const Tensor& a = products[0].a;
@@ -892,7 +894,7 @@ std::tuple<Tensor, Tensor> loss_and_logit_grads(const Tensor& h, const Tensor& w
 Tensor head_weight_grad(const Tensor& dlogits, const Tensor& h, const Tensor& g) {
   const Tensor g32 = g.to(at::kFloat);
   Tensor dw = product_out(dlogits, h, kTN);
-  if (group_into({{dlogits, h, dw, kTN, false, 1.0, g32}})) return dw;
+  if (group_into({{dlogits, h, dw, kTN, false, 1.0, g32, {}, false, true}})) return dw;   // one sum, as the fp32 matrix is
   return scale_to_bf16(product(dlogits, h, kTN, {}, {}, at::kFloat), g32);
 }
 

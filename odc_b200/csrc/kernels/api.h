@@ -147,7 +147,7 @@ struct GemmProduct {
   const void *a, *b;
   void* c;
   int c_kind, M, N, K, layout;
-  bool accumulate, fixed_order;   // fixed_order: the sum of an accumulating product is formed in one order
+  bool accumulate, whole;   // whole: the sum is not divided, as a bf16 product by itself or one that is added in any order may be
   long long lda, ldb, ldc;
   float scale;
   const float* scale_ptr;

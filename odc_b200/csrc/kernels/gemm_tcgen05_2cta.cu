@@ -1526,16 +1526,17 @@ static unsigned int* group_words(int n) {
   return base[dev] + at - n;
 }
 
-// How wide the tiles of each product are, in units of a k-block (0.28 us): the items go to the pairs that are free first, longest
-// first, so the group takes the work per pair and half of its last item, but at least its longest item, and a second round besides
-// costs 6 (the items are handed on from CTA to CTA, the first epilogues are in the way).  An item takes at least what its epilogue
-// does (6) and 2 to begin with; a part of a bf16 tile writes and reads 256 KB of fp32 (6), the parts of an fp32 sum meet in memory.
-// The longest item is made half as wide as long as that gains a twentieth.  300 tokens, 1536 wide: half as wide 15.3 -> 12.5 us
-// (projection), MLP of 512 and 1536 19.5 -> 15.4.
+// How wide the tiles of each product are, and into how many parts short sums that may be added in any order are divided.  In units of a
+// k-block (0.28 us): the items go to the pairs that are free first, longest first, so the group takes the work per pair and half of
+// its last item, but at least its longest item, and a second round besides costs 6 (the items are handed on from CTA to CTA, the
+// first epilogues are in the way).  An item takes at least what its epilogue does (6) and 2 to begin with; a part of a bf16 tile
+// writes and reads 256 KB of fp32 (6), the parts of an fp32 sum meet in memory.  The longest item is made half as wide, or
+// divided, as long as that gains a twentieth.  300 tokens, 1536 wide: half as wide 15.3 -> 12.5 us (projection), MLP of 512 and 1536
+// 19.5 -> 15.4.
 struct GroupShape {
   int tiles, kb;
   SplitPlan plan;
-  bool bf16;
+  bool bf16, may_divide;        // may_divide: into other parts than the plan's
   int bn, half_tiles, layout;   // columns of a tile; how many tiles of half the width there are
   int divided() const { return tiles - plan.whole; }
   int parts() const { return divided() * plan.splits; }
@@ -1546,18 +1547,21 @@ struct GroupShape {
   double sum() const { return bf16 && parts() > 0 ? 12.0 + 8.0 * (plan.splits - 1) : 0.0; }
   double work() const { return plan.whole * time(kb, false) + (parts() > 0 ? parts() * time(plan.kb_split, true) : 0.0); }
 };
-// Into how many parts: as the product by itself would be, so that a sum is no longer than there, and the bytes of a bf16 result are
-// the same either way.  The tensor cores drop what does not fit behind an accumulator's last bit, 1e-9 of the result for every product in
-// one sum: 1.8e-6 over 2048, 1.8e-5 over 17920, 1.3e-4 over 131072.  Left whole under the other products' arithmetic, as three
+// Long sums are divided as in a launch of their own, so that they are no longer than there, and the bytes of a bf16 result are the
+// same either way.  The tensor cores drop what does not fit behind an accumulator's last bit, 1e-9 of the result for every product in
+// one sum: 3.8e-6 over 4096, 1.8e-5 over 17920, 1.3e-4 over 131072.  Left whole under the other products' arithmetic, as three
 // parts had not been, the hidden states' gradient over 151936 words went from 8.3e-5 to 1.2e-4 (2.3526e-3 to 2.3602e-3 from 64
-// bits in all).  Sums over no more than 2048 (1.8e-6) stay whole: there a product by itself divides its last one to eight tiles at most.
-// What is added to fp32 in any order is divided as in a launch of its own (scatter_plan); addends and sums in one order are not.
-constexpr int kGroupShortSum = 2048 / gemm_pair::BK;
+// bits in all).  Over no more than 4096 there is next to nothing to lose (one rounding to bf16: 1.7e-3), and parts of a product's own
+// are too many here: MLP of 512 and 1536, fp32 sums, 2000 tokens 35 us with them and 20 without, 300 tokens 25 and 16; projection of
+// 3072 x 2048, 300 tokens, 28 and 21.5.  What is added to fp32 in any order may be divided there, everything else stays whole; so
+// do addends and sums in one order over any length.
+constexpr int kGroupShortSum = 4096 / gemm_pair::BK;
 static SplitPlan group_split(const GemmProduct& q, int tiles, int sm_count) {
   using namespace gemm_pair;
   const int kb = (q.K + BK - 1) / BK;
-  if (q.c_kind == kBF16 && q.addend == nullptr && kb > kGroupShortSum) return product_plan(q.M, q.N, q.K, sm_count);
-  if (q.c_kind == kF32 && q.accumulate && !q.fixed_order) return plan_splits(q.M, q.N, q.K, sm_count, scatter_cost(1), true);
+  if (q.whole || kb <= kGroupShortSum) return {tiles, 1, kb};
+  if (q.c_kind == kBF16 && q.addend == nullptr) return product_plan(q.M, q.N, q.K, sm_count);
+  if (q.c_kind == kF32 && q.accumulate) return plan_splits(q.M, q.N, q.K, sm_count, scatter_cost(1), true);
   return {tiles, 1, kb};
 }
 static void plan_group(GroupShape* g, int n, int pairs) {
@@ -1582,16 +1586,27 @@ static void plan_group(GroupShape* g, int n, int pairs) {
     for (int i = 1; i < n; ++i)
       if (g[i].item() > g[longest].item()) longest = i;
     GroupShape& q = g[longest];
-    if (q.bn != 256 || q.parts() > 0) return;
     const GroupShape before = q;
-    q.bn = 128;
-    q.tiles = q.plan.whole = q.half_tiles;
-    const double c = cost();
-    if (c >= 0.95 * best) {
+    GroupShape better = before;
+    double least = 0.95 * best;
+    const auto consider = [&] {
+      if (const double c = cost(); c < least) { least = c; better = q; }
       q = before;
-      return;
+    };
+    if (q.bn == 256 && q.parts() == 0) {
+      q.bn = 128;
+      q.tiles = q.plan.whole = q.half_tiles;
+      consider();
     }
-    best = c;
+    for (int want = before.plan.splits + 1; want <= 8 && q.may_divide; ++want) {
+      const int each = (q.kb + want - 1) / want, s = (q.kb + each - 1) / each;   // no empty part
+      if (s <= before.plan.splits || each < 4) continue;
+      q.plan = {0, s, each};
+      consider();
+    }
+    if (better.bn == before.bn && better.plan.splits == before.plan.splits) return;
+    q = better;
+    best = least;
   }
 }
 
@@ -1602,8 +1617,8 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
     const GemmProduct& q = g[i];
     if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate)) || (q.addend != nullptr && q.c_kind != kBF16)) return false;
     const int tiles = (q.M + 255) / 256 * ((q.N + BN - 1) / BN);
-    shapes[i] = GroupShape{tiles, (q.K + BK - 1) / BK, group_split(q, tiles, sm_count), q.c_kind == kBF16, BN,
-                           (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
+    shapes[i] = GroupShape{tiles, (q.K + BK - 1) / BK, group_split(q, tiles, sm_count), q.c_kind == kBF16,
+                           q.c_kind == kF32 && q.accumulate && !q.whole && q.K <= kGroupShortSum * BK, BN, (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
   }
   // A group saves the launches and last rounds of its products, 30 to 100 units.  With more work than this for a pair that is no
   // gain any more, and pairs that are not in step with one another share less of L2 (16321 tokens, 2048 and 8192 wide, 4400 units:

@@ -74,10 +74,11 @@ def test_groups_divide_what_would_outlast_them(T, H, F):
             assert parts == [1, 1, 1]
 
 
-@pytest.mark.parametrize("M,N,K", [(8, 256, 4096), (765, 1536, 17920), (1904, 1536, 151936), (4096, 1536, 151936), (3072, 2048, 8200),
-                                   (2304, 2304, 4096), (4096, 4096, 28672), (16321, 2048, 16384), (300, 392, 2112)])
+@pytest.mark.parametrize("M,N,K", [(8, 256, 4160), (765, 1536, 17920), (1904, 1536, 151936), (4096, 1536, 151936), (3072, 2048, 8200),
+                                   (2304, 2304, 4160), (4096, 4096, 28672), (16321, 2048, 16384), (300, 392, 8192)])
 def test_sums_are_as_short_in_a_group_as_in_a_launch_of_their_own(M, N, K):
-    """A bf16 product keeps its own parts whatever stands next to it, and so does a weight gradient that is added in any order."""
+    """Over more than 4096, a bf16 product keeps its own parts whatever stands next to it, and so does a weight gradient that is added
+    in any order; over less it stays whole."""
     ext = _ext.load()
     taken = 0
     for neighbours in ([], [(N, 512, max(M, 64), True, True)], [(4096, 512, 300, False, False), (512, 2048, 300, False, False)]):
@@ -87,7 +88,8 @@ def test_sums_are_as_short_in_a_group_as_in_a_launch_of_their_own(M, N, K):
             continue
         taken += 1
         assert got[0][1:] == _plan(M, N, K)[1:3] or (_plan(M, N, K)[2] == 1 and got[0][2] == 1)
-        if neighbours and neighbours[0][3]:
+        assert ext.gemm_group_tiles([(M, N, 4096, False, False)] + neighbours, SMS)[0][2] == 1
+        if neighbours and neighbours[0][3] and M > 4096:
             tiles, whole, parts = ext.scatter_plan(N, 512, max(M, 64), 1, SMS)
             assert got[1][2] == parts and (parts == 1 or got[1] == (tiles, whole, parts))
     assert taken
