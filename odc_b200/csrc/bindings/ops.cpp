@@ -186,12 +186,11 @@ Tensor kernel_status() {
   return device_status(dev);
 }
 
-// The host read an error there.  A launch that gave up may have left counters of a group half way, so from here on a group brings
-// its own (one more launch, 2 us); nothing waits for what other streams have in flight.
-std::atomic<bool> g_gave_up{false};
+// The host read an error there.  A launch that gave up may have left the counters of its stream's groups half way: the next ones get
+// others; nothing waits for what other streams have in flight.
 void clear_kernel_status() {
   kernel_status().zero_();
-  g_gave_up = true;
+  odc::gemm_group_new_words();
 }
 
 bool capturing() {
@@ -199,6 +198,9 @@ bool capturing() {
   check(cudaStreamIsCapturing(cur_stream(), &capture), "capture");
   return capture != cudaStreamCaptureStatusNone;
 }
+
+// the counters of the current stream's groups, or null where a launch has to bring its own
+unsigned int* group_words() { return capturing() ? nullptr : odc::gemm_group_words(cur_stream()); }
 
 // ODC_GEMM=cublas: library products, to measure the hand-written kernels against (read at every call)
 bool library_gemm() {
@@ -319,11 +321,13 @@ bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = 
   Tensor scratch;
   if (const size_t bytes = odc::gemm_group_scratch(g, n, sm_count()))
     scratch = at::empty({static_cast<int64_t>(bytes / sizeof(float))}, a.options().dtype(at::kFloat));
-  Tensor words;
-  if (capturing() || g_gave_up)   // a graph's are cleared at each replay
-    words = at::zeros({odc::kGroupLaunchWords}, a.options().dtype(at::kInt));
-  const cudaError_t e = odc::gemm_group(g, n, scratch.defined() ? scratch.data_ptr<float>() : nullptr,
-                                        words.defined() ? reinterpret_cast<unsigned int*>(words.data_ptr<int>()) : nullptr,
+  unsigned int* words = group_words();
+  Tensor own;
+  if (words == nullptr) {   // a graph's are cleared at each replay
+    own = at::zeros({odc::kGroupLaunchWords}, a.options().dtype(at::kInt));
+    words = reinterpret_cast<unsigned int*>(own.data_ptr<int>());
+  }
+  const cudaError_t e = odc::gemm_group(g, n, scratch.defined() ? scratch.data_ptr<float>() : nullptr, words,
                                         ctr_table.defined() ? reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()) : nullptr,
                                         arrivals, device_status(a.get_device()).data_ptr<int>(), sm_count(), cur_stream());
   if (e == cudaErrorNotSupported) return false;
@@ -1489,6 +1493,11 @@ void register_ops(py::module_& m) {
     }
     return group_into(todo);
   });  // (a, b, c, layout, accumulate, scale) each; False: not taken as a group, nothing done
+  m.def("group_words", []() -> c10::optional<Tensor> {
+    unsigned int* words = group_words();
+    if (words == nullptr) return c10::nullopt;
+    return at::from_blob(words, {odc::kGroupLaunchWords}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, at::cuda::current_device()));
+  });  // counters of the current stream's groups; None where every launch brings its own
   using Shape = std::tuple<int, int, int, bool, bool>;   // (M, N, K, fp32, accumulate)
   static const auto group_plan = [](const std::vector<Shape>& products, int sms) {
     TORCH_CHECK(products.size() <= odc::kMaxGroupProducts, "group plan: too many products");

@@ -137,8 +137,8 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
 // times scale and, unless scale_ptr is null, the value there; an fp32 result is added to C if accumulate, and to a bf16
 // one an fp32 matrix may be added.  ctr_ptrs: device table whose first entry is an arrival counter that receives
 // `arrivals` once everything is in memory (0: none).  scratch: gemm_group_scratch() bytes.  words: kGroupLaunchWords zeros that are
-// this launch's alone, left zero by it unless a wait runs out, or null for some of the device's own (not for a captured launch, which
-// keeps what it got, nor after a wait has run out).
+// this launch's alone while it runs, left zero by it unless a wait runs out: gemm_group_words() of its stream (null: no more of
+// them), but not for a captured launch, which may run on another stream.  gemm_group_new_words(): a launch on this device has given up.
 // cudaErrorNotSupported: one by one.
 constexpr int kMaxGroupProducts = 3;
 constexpr int kMaxGroupDivided = 512;   // divided tiles of a launch: those of two rounds of pairs for each product, at most
@@ -160,6 +160,8 @@ struct GemmGroupPlan {
 };
 GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count);
 bool gemm_group_takes(const GemmProduct* g, int n, int sm_count);   // what gemm_group answers with cudaErrorNotSupported is false
+unsigned int* gemm_group_words(cudaStream_t stream);
+void gemm_group_new_words();
 size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count);
 cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,
                        int* status, int sm_count, cudaStream_t stream);

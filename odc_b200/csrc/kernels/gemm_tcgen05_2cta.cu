@@ -28,6 +28,7 @@
 #include <cmath>
 #include <mutex>
 #include <type_traits>
+#include <unordered_map>
 
 #include "api.h"
 #include "launch.cuh"
@@ -1505,25 +1506,44 @@ cudaError_t gemm_logits_pair(const void* h, const void* w, void* logits, const l
 }
 
 // Words for the launches of groups, zero at load and left zero by each: the counter of items, the count of finished CTAs, and two
-// per divided tile.  They are handed out in turn and come round again after at least kGroupWords / kGroupLaunchWords (1022)
-// launches, more than a device holds queued; a captured launch runs again at any time and brings its own.
-constexpr unsigned int kGroupWords = 1u << 20;
-__device__ unsigned int g_group_words[kGroupWords];
-static unsigned int* group_words(int n) {
-  static std::mutex mu;
-  static unsigned int at = 0;
-  static unsigned int* base[64] = {};
+// per divided tile.  Every stream has a set of its own, so the order of its launches keeps one from the words of another that still
+// runs.  A launch that gives up may leave some as they are: from then on the streams of the device get new sets.  Who comes
+// after kGroupSets of them gets none.
+constexpr int kGroupSets = 1000;
+__device__ unsigned int g_group_words[kGroupSets * kGroupLaunchWords];
+struct GroupSets {
+  std::mutex mu;
+  unsigned int* base = nullptr;
+  int used = 0;
+  std::unordered_map<unsigned long long, int> of_stream;   // by a number that no other stream of the process ever has
+};
+static GroupSets* group_sets() {
+  static GroupSets sets[64];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  if (base[dev] == nullptr) {
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? &sets[dev] : nullptr;
+}
+unsigned int* gemm_group_words(cudaStream_t stream) {
+  GroupSets* sets = group_sets();
+  unsigned long long id = 0;
+  if (sets == nullptr || cudaStreamGetId(stream, &id) != cudaSuccess) return nullptr;
+  std::lock_guard<std::mutex> lock(sets->mu);
+  if (sets->base == nullptr) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_group_words) != cudaSuccess) return nullptr;
-    base[dev] = static_cast<unsigned int*>(p);
+    sets->base = static_cast<unsigned int*>(p);
   }
-  if (at + n > kGroupWords) at = 0;
-  at += n;
-  return base[dev] + at - n;
+  auto set = sets->of_stream.find(id);
+  if (set == sets->of_stream.end()) {
+    if (sets->used == kGroupSets) return nullptr;
+    set = sets->of_stream.emplace(id, sets->used++).first;
+  }
+  return sets->base + static_cast<size_t>(set->second) * kGroupLaunchWords;
+}
+void gemm_group_new_words() {
+  if (GroupSets* sets = group_sets()) {
+    std::lock_guard<std::mutex> lock(sets->mu);
+    sets->of_stream.clear();
+  }
 }
 
 // How wide the tiles of each product are, and into how many parts short sums that may be added in any order are divided.  In units of a
@@ -1729,7 +1749,6 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int
   group.count = n;
   if (divided > kMaxGroupDivided || (divided > 0 && scratch == nullptr)) return cudaErrorNotSupported;
   group.parts = reinterpret_cast<float4*>(scratch);
-  if (words == nullptr) words = group_words(2 + 2 * divided);
   if (words == nullptr) return cudaErrorInvalidValue;
   group.next = words;
   group.arrived = words + 2;

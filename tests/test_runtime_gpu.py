@@ -195,20 +195,51 @@ def test_pipeline_status_surfaces_at_the_next_sync(single_rank_pg):
         odc.finalize_distributed()
 
 
+def test_every_stream_has_counters_of_its_own_for_groups():
+    """The order of a stream's launches is what keeps two of them from one set of counters; a captured launch brings its own."""
+    from odc_b200 import _ext
+    ext = _ext.load()
+    a, b = torch.randn(300, 8192, device="cuda").bfloat16(), torch.randn(8192, 512, device="cuda").bfloat16()
+    x = torch.randn(300, 2048, device="cuda").bfloat16()
+    streams, words, outs = [torch.cuda.current_stream()] + [torch.cuda.Stream() for _ in range(3)], [], []
+    torch.cuda.synchronize()
+    for _ in range(40):
+        for s in streams:
+            with torch.cuda.stream(s):
+                words.append(ext.group_words().data_ptr())
+                o, dw = torch.empty(300, 512, device="cuda", dtype=torch.bfloat16), torch.empty(8192, 2048, device="cuda", dtype=torch.bfloat16)
+                assert ext.gemm_group([(a, b, o, "nn", False, 1.0), (a, x, dw, "tn", False, 1.0)])
+                outs.append((o, dw))
+    torch.cuda.synchronize()
+    assert len(set(words)) == len(streams) and words[:len(streams)] * 40 == words
+    assert all(torch.equal(o, outs[0][0]) and torch.equal(dw, outs[0][1]) for o, dw in outs)
+    assert not any(ext.group_words().tolist())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        assert ext.group_words() is None
+
+
 def test_groups_after_a_reported_error():
-    """Once a wait has run out, launches of several products bring their own counters, which the one that gave up cannot have left
-    half way.  The word is pre-set by hand again."""
+    """Once a wait has run out, launches of several products get other counters than the one that gave up, which may have left its own
+    half way.  The word and the counters are set by hand."""
     from odc_b200 import _ext, ops
     from odc_b200.runtime.status import ERR_PIPELINE_TIMEOUT, OdcTimeoutError
     ext = _ext.load()
-    a, b = torch.randn(300, 4096, device="cuda").bfloat16(), torch.randn(4096, 512, device="cuda").bfloat16()
-    outs = [torch.empty(300, 512, device="cuda", dtype=torch.bfloat16) for _ in range(4)]
-    assert ext.gemm_group([(a, b, outs[0], "nn", False, 1.0)])
+    a, b = torch.randn(300, 8192, device="cuda").bfloat16(), torch.randn(8192, 512, device="cuda").bfloat16()
+    x = torch.randn(300, 2048, device="cuda").bfloat16()
+
+    def run():
+        o, dw = torch.empty(300, 512, device="cuda", dtype=torch.bfloat16), torch.empty(8192, 2048, device="cuda", dtype=torch.bfloat16)
+        assert ext.gemm_group([(a, b, o, "nn", False, 1.0), (a, x, dw, "tn", False, 1.0)])
+        return o, dw
+    want, left = run(), ext.group_words()
+    left.fill_(1)
     ext.kernel_status().copy_(torch.tensor([ERR_PIPELINE_TIMEOUT, 3, 17, 0], dtype=torch.int32))
     with pytest.raises(OdcTimeoutError, match="pipeline"):
         ops.check_status()
     ops.check_status()
-    for o in outs[1:]:
-        assert ext.gemm_group([(a, b, o, "nn", False, 1.0)])
-        assert torch.equal(o, outs[0])
+    assert ext.group_words().data_ptr() != left.data_ptr()
+    for _ in range(3):
+        assert all(torch.equal(p, q) for p, q in zip(run(), want))
+    assert left.min() == 1 and not any(ext.group_words().tolist())
     ops.check_status()
