@@ -440,7 +440,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (!__all_sync(0xffffffffu, ok)) break;
       }
       if (cta == 0 && lane == 0 && item < num_items) {   // given up: the counter is left as the next launch expects it
-        for (; ahead < num_items; taken(ahead)) ahead = take();
+        taken(ahead);   // the answer that had not been looked at may be the last one
+        while (ahead < num_items) taken(ahead = take());
       }
     }
   } else if (kMode == kModeGroup && warp == 1) {
