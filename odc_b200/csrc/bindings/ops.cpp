@@ -589,6 +589,7 @@ Tensor linear_rope(const Tensor& x, const Tensor& w, const Tensor& bias, const T
   odc::bind_device(x.get_device());
   TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && w.size(0) == (n_q + 2 * n_kv) * d, "linear_rope: x [T,K], w [(Hq+2Hkv)*D,K]");
   TORCH_CHECK(pos.scalar_type() == at::kLong && pos.is_contiguous() && pos.numel() == x.size(0), "linear_rope: position_ids int64 [T]");
+  TORCH_CHECK(!bias.defined() || bias.numel() == w.size(0), "linear_rope: bias [(Hq+2Hkv)*D]");
   if (odc::gemm_pairs_enabled() && !library_gemm() && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
       x.stride(1) == 1 && w.stride(1) == 1 && (!bias.defined() || (bias.scalar_type() == at::kBFloat16 && bias.is_contiguous()))) {
     auto out = at::empty({x.size(0), w.size(0)}, x.options());

@@ -682,6 +682,14 @@ def test_bias_that_starts_off_a_16_byte_boundary(ext, M, N, K, offset):
     assert ext.kernel_status()[0].item() == 0, ext.kernel_status().tolist()
 
 
+@pytest.mark.parametrize("T", [16, 300])
+def test_projection_with_rotation_refuses_a_bias_of_another_length(ext, T):
+    x, w = torch.randn(T, 128, device="cuda").bfloat16(), torch.randn(512, 128, device="cuda").bfloat16()
+    for n in (8, 504, 520):
+        with pytest.raises(RuntimeError, match="linear_rope: bias"):
+            ext.linear_rope(x, w, torch.randn(n, device="cuda").bfloat16(), torch.arange(T, device="cuda"), 4, 2, 64, 10000.0)
+
+
 @pytest.mark.parametrize("T,K,F", [(256, 128, 128), (300, 264, 1000), (520, 2048, 136), (1000, 512, 4160), (16, 128, 256),
                                    (765, 17920, 768)])
 def test_linear_swiglu_matches_the_two_passes(ext, T, K, F):
