@@ -217,7 +217,7 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
         ctx.model, ctx.kept = model, h.is_cuda and bool(p.matrix()) and ops._ext().head_keeps_logit_grads(h, w, chunk)
         if ctx.kept:   # the gradient of the logits; the products with it are left to the backward, which knows the loss gradient
             loss, dlogits = ops._ext().loss_and_logit_grads(h, w, labels, loss_scale, ignore_index)
-            ctx.save_for_backward(h, dlogits)
+            ctx.save_for_backward(h.clone(), dlogits)   # a copy: whoever holds h may write to it, as with several chunks
             return loss
         if h.is_cuda:
             # room for the owners' padding rows, so that the whole buffer can be pushed as it is

@@ -227,6 +227,36 @@ def test_every_accumulator_matches_the_plain_decoder(tied, bias, sync):
             assert _rel(got[name], p.grad) < CHAIN, name
 
 
+@pytest.mark.parametrize("chunk,kept", [(4096, True), (300, False)])
+def test_hidden_states_may_be_written_to_after_the_loss(chunk, kept):
+    """One chunk, whose products wait for the backward, and several: what the loss needs of the hidden states is its own."""
+    from odc_b200 import ops
+    with _Engine() as e:
+        e.cfg.ce_chunk = e.model.cfg.ce_chunk = chunk
+        mbs = _batches(e.cfg, n=1, lo=64, hi=128)   # one key tile per sequence: no sums in a free order
+        states, calls = [], []
+        plain, loss = e.model.hidden_states, ops._ext().loss_and_logit_grads
+        e.model.hidden_states = lambda *a: states.append(plain(*a)) or states[-1]
+        want = e.minibatch(mbs)
+        whole = type(e.model).forward
+
+        def forward(*args, **kw):
+            out = whole(e.model, *args, **kw)
+            states[-1].data.zero_()
+            with torch.no_grad():
+                states[-1].add_(1)
+            return out
+        e.model.forward = forward
+        ops._ext().loss_and_logit_grads = lambda *a: calls.append(1) or loss(*a)
+        try:
+            got = e.minibatch(mbs)
+        finally:
+            ops._ext().loss_and_logit_grads = loss
+        assert len(states) == 2 and bool(calls) == kept
+        for name in want:   # the same sums, in another order of additions
+            assert _rel(got[name], want[name]) < 1e-3, name
+
+
 class _Counting(torch.nn.Module):
     def __init__(self, inner, calls):
         super().__init__()
