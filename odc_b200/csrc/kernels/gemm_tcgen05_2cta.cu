@@ -1547,7 +1547,7 @@ void gemm_group_new_words() {
   }
 }
 
-// How wide the tiles of each product are, and into how many parts short sums that may be added in any order are divided.  In units of a
+// How wide the tiles of each product are, and into how many parts its sum is divided unless that is given (group_split).  In units of a
 // k-block (0.28 us): the items go to the pairs that are free first, longest first, so the group takes the work per pair and half of
 // its last item, but at least its longest item, and a second round besides costs 6 (the items are handed on from CTA to CTA, the
 // first epilogues are in the way).  An item takes at least what its epilogue does (6) and 2 to begin with; a part of a bf16 tile
@@ -1570,20 +1570,20 @@ struct GroupShape {
 };
 // Long sums are divided as in a launch of their own, so that they are no longer than there, and the bytes of a bf16 result are the
 // same either way.  The tensor cores drop what does not fit behind an accumulator's last bit, 1e-9 of the result for every product in
-// one sum: 3.8e-6 over 4096, 1.8e-5 over 17920, 1.3e-4 over 131072.  Left whole under the other products' arithmetic, as three
-// parts had not been, the hidden states' gradient over 151936 words went from 8.3e-5 to 1.2e-4 (2.3526e-3 to 2.3602e-3 from 64
-// bits in all).  Over no more than 4096 there is next to nothing to lose (one rounding to bf16: 1.7e-3), and parts of a product's own
-// are too many here: MLP of 512 and 1536, fp32 sums, 2000 tokens 35 us with them and 20 without, 300 tokens 25 and 16; projection of
-// 3072 x 2048, 300 tokens, 28 and 21.5.  What is added to fp32 in any order may be divided there, everything else stays whole; so
-// do addends and sums in one order over any length.
-constexpr int kGroupShortSum = 4096 / gemm_pair::BK;
+// one sum: 8e-6 over 8192, 1.8e-5 over 17920, 1.3e-4 over 131072.  Left whole under the other products' arithmetic, as three parts
+// had not been, the hidden states' gradient over 151936 words went from 8.3e-5 to 1.2e-4 (2.3526e-3 to 2.3602e-3 from 64 bits in
+// all), the input gradient of a layer of 4096 and 14336 from 7.3445e-3 to 7.3461e-3; of one of 2048 and 8192, a sum over 16384, it
+// stayed at 4.190e-3.  Shorter sums are divided as the group needs it: parts of a product's own are too many here (MLP of 512 and
+// 1536, fp32 sums, 2000 tokens 35 us with them and 20 without; projection of 6144 x 4096, 300 tokens, 48 and 45).  Sums in one
+// order and addends stay whole over any length.
+constexpr int kGroupShortSum = 16384;
 static SplitPlan group_split(const GemmProduct& q, int tiles, int sm_count) {
   using namespace gemm_pair;
-  const int kb = (q.K + BK - 1) / BK;
-  if (q.whole || kb <= kGroupShortSum) return {tiles, 1, kb};
-  if (q.c_kind == kBF16 && q.addend == nullptr) return product_plan(q.M, q.N, q.K, sm_count);
-  if (q.c_kind == kF32 && q.accumulate) return plan_splits(q.M, q.N, q.K, sm_count, scatter_cost(1), true);
-  return {tiles, 1, kb};
+  if (q.K > kGroupShortSum && !q.whole) {
+    if (q.c_kind == kBF16 && q.addend == nullptr) return product_plan(q.M, q.N, q.K, sm_count);
+    if (q.c_kind == kF32 && q.accumulate) return plan_splits(q.M, q.N, q.K, sm_count, scatter_cost(1), true);
+  }
+  return {tiles, 1, (q.K + BK - 1) / BK};
 }
 static void plan_group(GroupShape* g, int n, int pairs) {
   auto cost = [&] {
@@ -1621,7 +1621,7 @@ static void plan_group(GroupShape* g, int n, int pairs) {
     }
     for (int want = before.plan.splits + 1; want <= 8 && q.may_divide; ++want) {
       const int each = (q.kb + want - 1) / want, s = (q.kb + each - 1) / each;   // no empty part
-      if (s <= before.plan.splits || each < 4) continue;
+      if (s <= before.plan.splits || each < 4 || (q.bf16 && q.tiles > kMaxGroupDivided / kMaxGroupProducts)) continue;
       q.plan = {0, s, each};
       consider();
     }
@@ -1639,7 +1639,8 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
     if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate)) || (q.addend != nullptr && q.c_kind != kBF16)) return false;
     const int tiles = (q.M + 255) / 256 * ((q.N + BN - 1) / BN);
     shapes[i] = GroupShape{tiles, (q.K + BK - 1) / BK, group_split(q, tiles, sm_count), q.c_kind == kBF16,
-                           q.c_kind == kF32 && q.accumulate && !q.whole && q.K <= kGroupShortSum * BK, BN, (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
+                           !q.whole && q.K <= kGroupShortSum && (q.c_kind == kBF16 ? q.addend == nullptr : q.accumulate), BN,
+                           (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
   }
   // A group saves the launches and last rounds of its products, 30 to 100 units.  With more work than this for a pair that is no
   // gain any more, and pairs that are not in step with one another share less of L2 (16321 tokens, 2048 and 8192 wide, 4400 units:
@@ -1707,6 +1708,29 @@ static bool group_takes(const GemmProduct* g, int n, int sm_count, GroupShape* s
 bool gemm_group_takes(const GemmProduct* g, int n, int sm_count) {
   GroupShape shapes[kMaxGroupProducts];
   return group_takes(g, n, sm_count, shapes);
+}
+
+// A long sum of a few tiles, whose eight parts a product by itself has added up by 32 CTAs a tile, is not hidden by products of few
+// k-blocks.  One by one and together, us: MLP of 1024 and 4096, 64 tokens 24.5 and 32.5, 512 tokens 33.2 and 37.5; of 2048 and 8192,
+// 200 tokens 58.8 and 62.0; of 1536 and 8960, 64 tokens, in eight parts together as well, 47.7 and 59.2.  With fp32 sums, whose
+// launches cost more, the others have to take 1.5 times as long as the parts (12 + 8 units for each but the first): 64 tokens 29.0 and
+// 34.3, 95.6 and 106.8 (1536 and 8960), but 109.7 and 98.0 (2048 and 8192).
+bool gemm_group_pays(const GemmProduct* g, int n, int sm_count) {
+  GroupShape shapes[kMaxGroupProducts];
+  if (!group_shapes(g, n, sm_count, shapes)) return false;
+  double work = 0;
+  bool f32 = false;
+  for (int i = 0; i < n; ++i) {
+    work += (g[i].M + 255) / 256 * ((g[i].N + 255) / 256) * std::max(8.0, shapes[i].kb + 2.0);
+    f32 = f32 || g[i].c_kind == kF32;
+  }
+  for (int i = 0; i < n && n > 1; ++i) {
+    const GemmProduct& q = g[i];
+    if (q.c_kind != kBF16 || q.whole || q.addend != nullptr || q.K <= 4096) continue;
+    const SplitPlan alone = product_plan(q.M, q.N, q.K, sm_count);
+    if (alone.whole == 0 && alone.splits == 8 && (!f32 || work / (sm_count / 2) < 1.5 * (12.0 + 8.0 * 7))) return false;
+  }
+  return true;
 }
 
 cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,

@@ -74,11 +74,11 @@ def test_groups_divide_what_would_outlast_them(T, H, F):
             assert parts == [1, 1, 1]
 
 
-@pytest.mark.parametrize("M,N,K", [(8, 256, 4160), (765, 1536, 17920), (1904, 1536, 151936), (4096, 1536, 151936), (3072, 2048, 8200),
-                                   (2304, 2304, 4160), (4096, 4096, 28672), (16321, 2048, 16384), (300, 392, 8192)])
+@pytest.mark.parametrize("M,N,K", [(765, 1536, 17920), (1904, 1536, 151936), (4096, 1536, 151936), (3072, 2048, 16400),
+                                   (2304, 2304, 16400), (4096, 4096, 28672), (16321, 2048, 16640), (1000, 392, 20000)])
 def test_sums_are_as_short_in_a_group_as_in_a_launch_of_their_own(M, N, K):
-    """Over more than 4096, a bf16 product keeps its own parts whatever stands next to it, and so does a weight gradient that is added
-    in any order; over less it stays whole."""
+    """Over more than 16384, a bf16 product keeps its own parts whatever stands next to it, and so does a weight gradient that is added
+    in any order."""
     ext = _ext.load()
     taken = 0
     for neighbours in ([], [(N, 512, max(M, 64), True, True)], [(4096, 512, 300, False, False), (512, 2048, 300, False, False)]):
@@ -88,8 +88,7 @@ def test_sums_are_as_short_in_a_group_as_in_a_launch_of_their_own(M, N, K):
             continue
         taken += 1
         assert got[0][1:] == _plan(M, N, K)[1:3] or (_plan(M, N, K)[2] == 1 and got[0][2] == 1)
-        assert ext.gemm_group_tiles([(M, N, 4096, False, False)] + neighbours, SMS)[0][2] == 1
-        if neighbours and neighbours[0][3] and M > 4096:
+        if neighbours and neighbours[0][3] and M > 16384:
             tiles, whole, parts = ext.scatter_plan(N, 512, max(M, 64), 1, SMS)
             assert got[1][2] == parts and (parts == 1 or got[1] == (tiles, whole, parts))
     assert taken
@@ -106,6 +105,15 @@ def test_groups_are_not_formed_of_many_items():
     for T in (300, 1500):
         assert head(T, False) == [0, 0] != head(T, True)
     assert _ext.load().gemm_group_plan([(128256, 2048, 300, False, False)], SMS) != [0]   # nothing else gives it its factor
+
+
+def test_groups_are_not_formed_around_a_sum_of_many_parts():
+    """A few tiles in eight parts by themselves go alone where the other products are over before they are added up."""
+    pays = lambda T, H, F, f32: _ext.load().gemm_group_pays([(T, H, 2 * F, False, False), (2 * F, H, T, f32, f32), (H, F, T, f32, f32)], SMS)
+    for T, H, F, bf16, fp32 in ((64, 1024, 4096, False, False), (512, 1024, 4096, False, False), (765, 1024, 4096, True, True),
+                                (64, 1536, 8960, False, False), (300, 1536, 8960, True, True), (256, 2048, 8192, False, True),
+                                (300, 2048, 8192, True, True), (64, 512, 1536, True, True), (256, 4096, 14336, False, True)):
+        assert pays(T, H, F, False) == bf16 and pays(T, H, F, True) == fp32, (T, H, F)
 
 
 def test_groups_halve_the_tiles_of_what_would_outlast_them():

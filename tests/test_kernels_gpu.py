@@ -475,10 +475,10 @@ def test_groups_of_products(ext, parts, products):
     # all tiles in parts, those of the last round, none; ragged edges; next to products of other kinds
     [("nn", 765, 1536, 17920), ("tn", 17920, 1536, 765), ("tn", 1536, 8960, 765)],
     [("nn", 4090, 1544, 20000), ("tn", 1024, 1544, 4090)],
-    [("tn", 3072, 2056, 8200), ("nn", 2304, 2304, 4104), ("nt", 300, 264, 8200)],
-    [("nn", 2304, 2304, 4104)], [("tn", 264, 264, 5040)], [("nn", 600, 520, 200), ("tn", 520, 200 * 8, 600)]])
+    [("tn", 3072, 2056, 16400), ("nn", 2304, 2304, 16400), ("nt", 1000, 264, 17000)],
+    [("nn", 2304, 2304, 16400)], [("tn", 264, 264, 17000)], [("nn", 600, 520, 200), ("tn", 520, 200 * 8, 600)]])
 def test_groups_give_the_bytes_of_single_products(ext, products):
-    """A bf16 result does not depend on what is formed in the same launch: a sum over more than 4096 is divided as in a launch of its own."""
+    """A bf16 result does not depend on what is formed in the same launch: a sum over more than 16384 is divided as in a launch of its own."""
     ops = [case[:4] for case in _group_case([(lay, M, N, K, torch.bfloat16, False, 1.0) for lay, M, N, K in products])]
     assert ext.gemm_group([(a, b, c, lay, False, 1.0) for a, b, c, lay in ops])
     for a, b, c, lay in ops:
