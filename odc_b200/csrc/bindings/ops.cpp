@@ -297,9 +297,8 @@ bool fixed_order_asked() {
   return at::globalContext().deterministicAlgorithms() ||
          (e != nullptr && *e != 0 && std::strcmp(e, "0") != 0 && std::strcmp(e, "false") != 0);
 }
-// arrivals > 0: that many are reported to the counter behind ctr_table (one entry) when the results are in memory.  `anyway`: also where
-// one by one is faster.
-bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = {}, int arrivals = 0, bool anyway = false) {
+// arrivals > 0: that many are reported to the counter behind ctr_table (one entry) when the results are in memory
+bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = {}, int arrivals = 0) {
   const int n = static_cast<int>(products.size());
   if (n < 1 || n > odc::kMaxGroupProducts || library_gemm() || !odc::gemm_pairs_enabled()) return false;
   odc::GemmProduct g[odc::kMaxGroupProducts];
@@ -319,7 +318,6 @@ bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = 
   const Tensor& a = products[0].a;
   c10::cuda::CUDAGuard guard(a.device());
   odc::bind_device(a.get_device());
-  if (!anyway && !odc::gemm_group_pays(g, n, sm_count())) return false;
   Tensor scratch;
   if (const size_t bytes = odc::gemm_group_scratch(g, n, sm_count()))
     scratch = at::empty({static_cast<int64_t>(bytes / sizeof(float))}, a.options().dtype(at::kFloat));
@@ -338,7 +336,7 @@ bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = 
   return true;
 }
 void products_into(const std::vector<Product>& products) {
-  if (products.size() > 1 && group_into(products)) return;
+  if (group_into(products)) return;
   for (const auto& p : products) product_into(p.a, p.b, p.c, p.lay, {}, p.accumulate);
 }
 Tensor product_out(const Tensor& a, const Tensor& b, int lay, c10::optional<at::ScalarType> dtype = c10::nullopt) {
@@ -1118,7 +1116,7 @@ Tensor sharded_head_grads(const Tensor& dlogits, const Tensor& h, const Tensor& 
   const Tensor dh = product_out(dlogits, w, kNN);
   std::vector<Product> todo{{dlogits, w, dh, kNN, false, 1.0, g32},
                             {dlogits, h, dw, kTN, direct || add, direct ? m->grad_scale : 1.0, direct || add ? g32 : Tensor()}};
-  if (group_into(todo, direct ? m->ctr_table : Tensor(), direct ? 1 : 0, true)) {
+  if (group_into(todo, direct ? m->ctr_table : Tensor(), direct ? 1 : 0)) {
     if (direct) m->dispatched->n.fetch_add(1);
     return dh;
   }
@@ -1494,7 +1492,7 @@ void register_ops(py::module_& m) {
       TORCH_CHECK(lay < 3, "gemm_group: unknown layout ", layout);
       todo.push_back({a, b, c, lay, accumulate, scale, {}, {}, accumulate});
     }
-    return group_into(todo, {}, 0, true);
+    return group_into(todo);
   });  // (a, b, c, layout, accumulate, scale) each; False: not taken as a group, nothing done
   m.def("group_words", []() -> c10::optional<Tensor> {
     unsigned int* words = group_words();
@@ -1523,10 +1521,6 @@ void register_ops(py::module_& m) {
     const auto plan = group_plan(products, sms);
     return std::vector<int>(plan.columns, plan.columns + products.size());
   }, py::arg("products"), py::arg("sms"));  // columns of a tile of each
-  m.def("gemm_group_pays", [](std::vector<Shape> products, int sms) {
-    const auto g = shapes_of(products);
-    return odc::gemm_group_pays(g.data(), static_cast<int>(g.size()), sms);
-  }, py::arg("products"), py::arg("sms"));
   m.def("gemm_group_tiles", [](std::vector<Shape> products, int sms) {
     const auto plan = group_plan(products, sms);
     std::vector<std::tuple<int, int, int>> out;

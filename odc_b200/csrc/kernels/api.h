@@ -160,7 +160,6 @@ struct GemmGroupPlan {
 };
 GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count);
 bool gemm_group_takes(const GemmProduct* g, int n, int sm_count);   // what gemm_group answers with cudaErrorNotSupported is false
-bool gemm_group_pays(const GemmProduct* g, int n, int sm_count);    // false: refused, or slower than one by one
 unsigned int* gemm_group_words(cudaStream_t stream);
 void gemm_group_new_words();
 size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count);

@@ -1710,29 +1710,6 @@ bool gemm_group_takes(const GemmProduct* g, int n, int sm_count) {
   return group_takes(g, n, sm_count, shapes);
 }
 
-// A long sum of a few tiles, whose eight parts a product by itself has added up by 32 CTAs a tile, is not hidden by products of few
-// k-blocks.  One by one and together, us: MLP of 1024 and 4096, 64 tokens 24.5 and 32.5, 512 tokens 33.2 and 37.5; of 2048 and 8192,
-// 200 tokens 58.8 and 62.0; of 1536 and 8960, 64 tokens, in eight parts together as well, 47.7 and 59.2.  With fp32 sums, whose
-// launches cost more, the others have to take 1.5 times as long as the parts (12 + 8 units for each but the first): 64 tokens 29.0 and
-// 34.3, 95.6 and 106.8 (1536 and 8960), but 109.7 and 98.0 (2048 and 8192).
-bool gemm_group_pays(const GemmProduct* g, int n, int sm_count) {
-  GroupShape shapes[kMaxGroupProducts];
-  if (!group_shapes(g, n, sm_count, shapes)) return false;
-  double work = 0;
-  bool f32 = false;
-  for (int i = 0; i < n; ++i) {
-    work += (g[i].M + 255) / 256 * ((g[i].N + 255) / 256) * std::max(8.0, shapes[i].kb + 2.0);
-    f32 = f32 || g[i].c_kind == kF32;
-  }
-  for (int i = 0; i < n && n > 1; ++i) {
-    const GemmProduct& q = g[i];
-    if (q.c_kind != kBF16 || q.whole || q.addend != nullptr || q.K <= 4096) continue;
-    const SplitPlan alone = product_plan(q.M, q.N, q.K, sm_count);
-    if (alone.whole == 0 && alone.splits == 8 && (!f32 || work / (sm_count / 2) < 1.5 * (12.0 + 8.0 * 7))) return false;
-  }
-  return true;
-}
-
 cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,
                        int* status, int sm_count, cudaStream_t stream) {
   using namespace gemm_pair;

@@ -107,15 +107,6 @@ def test_groups_are_not_formed_of_many_items():
     assert _ext.load().gemm_group_plan([(128256, 2048, 300, False, False)], SMS) != [0]   # nothing else gives it its factor
 
 
-def test_groups_are_not_formed_around_a_sum_of_many_parts():
-    """A few tiles in eight parts by themselves go alone where the other products are over before they are added up."""
-    pays = lambda T, H, F, f32: _ext.load().gemm_group_pays([(T, H, 2 * F, False, False), (2 * F, H, T, f32, f32), (H, F, T, f32, f32)], SMS)
-    for T, H, F, bf16, fp32 in ((64, 1024, 4096, False, False), (512, 1024, 4096, False, False), (765, 1024, 4096, True, True),
-                                (64, 1536, 8960, False, False), (300, 1536, 8960, True, True), (256, 2048, 8192, False, True),
-                                (300, 2048, 8192, True, True), (64, 512, 1536, True, True), (256, 4096, 14336, False, True)):
-        assert pays(T, H, F, False) == bf16 and pays(T, H, F, True) == fp32, (T, H, F)
-
-
 def test_groups_halve_the_tiles_of_what_would_outlast_them():
     columns = lambda *g: _ext.load().gemm_group_columns(list(g), SMS)
     assert columns((300, 1536, 2048, False, False), (2048, 1536, 300, False, False)) == [128, 256]
