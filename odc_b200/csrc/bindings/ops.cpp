@@ -77,6 +77,7 @@ Tensor rope_qkv(Tensor qkv, Tensor pos, int n_q, int n_kv, int head_dim, double 
   TORCH_CHECK(qkv.dim() == 2 && qkv.is_contiguous() && qkv.scalar_type() == at::kBFloat16, "rope: qkv [T,W] bf16");
   TORCH_CHECK(qkv.size(1) == int64_t(n_q + 2 * n_kv) * head_dim, "rope: width mismatch");
   TORCH_CHECK(pos.scalar_type() == at::kLong && pos.numel() == qkv.size(0), "rope: position_ids int64 [T]");
+  TORCH_CHECK(pos.device() == qkv.device(), "rope: position_ids on ", pos.device(), ", qkv on ", qkv.device());
   auto out = at::empty_like(qkv);
   check(odc::launch_rope_qkv(qkv.data_ptr(), out.data_ptr(), reinterpret_cast<const long long*>(pos.data_ptr<int64_t>()),
                              static_cast<int>(qkv.size(0)), n_q, n_kv, head_dim, static_cast<float>(theta), inverse,
@@ -364,6 +365,7 @@ std::tuple<Tensor, Tensor> attn_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seql
                   v.stride(1) == d, "attention: heads must be packed within a token");
   TORCH_CHECK(k.stride(0) == v.stride(0), "attention: k and v must share a row stride");
   TORCH_CHECK(cu_seqlens.scalar_type() == at::kInt && cu_seqlens.is_contiguous(), "attention: cu_seqlens int32");
+  TORCH_CHECK(cu_seqlens.device() == q.device(), "attention: cu_seqlens on ", cu_seqlens.device(), ", q on ", q.device());
   auto o = at::empty({T, hq, d}, q.options());
   auto lse = at::empty({hq, T}, q.options().dtype(at::kFloat));
   check(odc::attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(),
@@ -590,6 +592,7 @@ Tensor linear_rope(const Tensor& x, const Tensor& w, const Tensor& bias, const T
   TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.size(1) == w.size(1) && w.size(0) == (n_q + 2 * n_kv) * d, "linear_rope: x [T,K], w [(Hq+2Hkv)*D,K]");
   TORCH_CHECK(pos.scalar_type() == at::kLong && pos.is_contiguous() && pos.numel() == x.size(0), "linear_rope: position_ids int64 [T]");
   TORCH_CHECK(!bias.defined() || bias.numel() == w.size(0), "linear_rope: bias [(Hq+2Hkv)*D]");
+  TORCH_CHECK(pos.device() == x.device(), "linear_rope: position_ids on ", pos.device(), ", x on ", x.device());
   if (odc::gemm_pairs_enabled() && !library_gemm() && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
       x.stride(1) == 1 && w.stride(1) == 1 && (!bias.defined() || (bias.scalar_type() == at::kBFloat16 && bias.is_contiguous()))) {
     auto out = at::empty({x.size(0), w.size(0)}, x.options());

@@ -682,6 +682,21 @@ def test_bias_that_starts_off_a_16_byte_boundary(ext, M, N, K, offset):
     assert ext.kernel_status()[0].item() == 0, ext.kernel_status().tolist()
 
 
+def test_positions_and_offsets_on_the_host_are_refused(ext):
+    """A layer, its projection, rotation and attention name the device instead of handing a host address to a kernel."""
+    from odc_b200 import ops
+    from odc_b200.models import DecoderLayer, get_config
+    with torch.device("cuda"):
+        layer = DecoderLayer(get_config("tiny")).bfloat16()
+    x = torch.randn(300, 256, device="cuda").bfloat16()
+    pos, cu = torch.arange(300), torch.tensor([0, 300], dtype=torch.int32)
+    qkv = torch.randn(300, 768, device="cuda").bfloat16()
+    for call in (lambda: layer(x, pos, cu.cuda(), 300), lambda: layer(x, pos.cuda(), cu, 300), lambda: ops.rope_qkv(qkv, pos, 4, 4, 64, 10000.0),
+                 lambda: ext.linear_rope(x, qkv.t()[:, :256].contiguous(), None, pos, 4, 4, 64, 10000.0), lambda: ops.varlen_attention_qkv(qkv, 4, 4, 64, cu, 300)):
+        with pytest.raises(RuntimeError, match="on cpu"):
+            call()
+
+
 @pytest.mark.parametrize("T", [16, 300])
 def test_projection_with_rotation_refuses_a_bias_of_another_length(ext, T):
     x, w = torch.randn(T, 128, device="cuda").bfloat16(), torch.randn(512, 128, device="cuda").bfloat16()
