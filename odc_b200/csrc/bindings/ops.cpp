@@ -74,6 +74,7 @@ std::tuple<Tensor, Tensor> rmsnorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor rst
 Tensor rope_qkv(Tensor qkv, Tensor pos, int n_q, int n_kv, int head_dim, double theta, bool inverse) {
   c10::cuda::CUDAGuard g(qkv.device());
   odc::bind_device(qkv.get_device());
+  pos = pos.contiguous();
   TORCH_CHECK(qkv.dim() == 2 && qkv.is_contiguous() && qkv.scalar_type() == at::kBFloat16, "rope: qkv [T,W] bf16");
   TORCH_CHECK(qkv.size(1) == int64_t(n_q + 2 * n_kv) * head_dim, "rope: width mismatch");
   TORCH_CHECK(pos.scalar_type() == at::kLong && pos.numel() == qkv.size(0), "rope: position_ids int64 [T]");

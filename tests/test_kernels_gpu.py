@@ -682,6 +682,27 @@ def test_bias_that_starts_off_a_16_byte_boundary(ext, M, N, K, offset):
     assert ext.kernel_status()[0].item() == 0, ext.kernel_status().tolist()
 
 
+def test_positions_that_are_a_strided_view(ext):
+    """Every second value of a larger vector: what the same values give next to one another, in the op, its backward and a layer."""
+    from odc_b200 import ops
+    from odc_b200.models import DecoderLayer, get_config
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        layer = DecoderLayer(get_config("tiny")).bfloat16()
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.normal_(0.0 if p.dim() == 2 else 1.0, 0.05)
+    x = torch.randn(300, 256, device="cuda").bfloat16()
+    cu = torch.tensor([0, 300], dtype=torch.int32, device="cuda")
+    pos = torch.arange(600, device="cuda")[::2]
+    qkv, dy = torch.randn(300, 768, device="cuda").bfloat16().requires_grad_(), torch.randn(300, 768, device="cuda").bfloat16()
+    rotated = [ops.rope_qkv(qkv, p, 4, 4, 64, 10000.0) for p in (pos, pos.clone(memory_format=torch.contiguous_format))]
+    assert not pos.is_contiguous() and torch.equal(*rotated)
+    assert torch.equal(*(torch.autograd.grad(y, [qkv], dy)[0] for y in rotated))
+    with torch.no_grad():
+        assert torch.equal(layer(x, pos, cu, 300), layer(x, pos.contiguous(), cu, 300))
+
+
 def test_positions_and_offsets_on_the_host_are_refused(ext):
     """A layer, its projection, rotation and attention name the device instead of handing a host address to a kernel."""
     from odc_b200 import ops
