@@ -132,10 +132,11 @@ struct OwnerMaps {   // one fp32 tensor map per owner's accumulator region (kMod
 // kModeGroup: up to three products that do not depend on one another (the input and weight gradients of a layer) in one launch.
 // Apart, each fills the machine by itself or not at all: 1000 tokens, 1536 and 8960 wide, are 24, 420 and 210 tiles of 280, 16
 // and 16 k-blocks on 74 pairs.  The items of the longest product come first and a pair takes the next one from a counter, so the
-// short ones fill what the long ones leave.  One by one / together, us: input and weight gradient of 1000 x 1536 x 2048 26.2 / 17.0,
-// of 1000 x 1536 x 1536 23.9 / 14.4, of 2000 x 512 x 512 (fp32 sum) 24.1 / 9.8; the three of an MLP over 2000 tokens, 512 and 1536
-// wide, 48.9 / 21.7, 300 tokens, 2048 and 8192 wide, 130 / 110, 1000 tokens, 1536 and 8960 wide, 109 / 104.  One product by itself
-// costs 0.7 us more than in kModePlain, and some 0.2 us an item where items are short.
+// short ones fill what the long ones leave.  One by one / together, us on the GPU: input and weight gradient of 1000 x 1536 x 2048
+// 19.0 / 17.5, of 1000 x 1536 x 1536 14.9 / 14.9, of 2000 x 512 x 512 (fp32 sum) 14.5 / 10.1; the three of an MLP over 2000 tokens, 512
+// and 1536 wide, 32.0 / 18.3, 300 tokens, 2048 and 8192 wide, 70 / 67 (fp32 sums 123 / 106), 1000 tokens, 1536 and 8960 wide,
+// 109 / 106 (134 / 130).  Called from a program, smaller ones gain the launches: MLP of 512 and 1536, 300 tokens, forward and backward,
+// 93 / 85.  One product by itself costs 0.7 us more than in kModePlain, and some 0.2 us an item where items are short.
 struct GroupProblem {
   int M, N, K, tiles_m, tiles_n;
   int a_mn, b_mn, bn;
@@ -742,7 +743,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       // a last epilogue waited for besides was the release of its accumulator to the other CTA (1500 clocks, and nobody takes it any
       // more) and the residual and bias box by box.  From the first launch of a chain to the next, before and now: 1900 x 512 x 512
       // 8.3 and 7.4 us, 1000 x 1536 x 1536 13.2 and 12.3, with a residual 16.1 and 13.7, with a bias 22.1 and 13.5; 16321 x 3072 x
-      // 2048 with a bias 167 and 133; fp32 sums of long rows 2 % slower (four times as many boxes; 16321 x 2048 x 2048: 101 and 104).
+      // 2048 with a bias 167 and 133; fp32 results, in four times as many boxes, 16320 x 2048 x 2048 96 and 96, K = 512 47 and 38, added
+      // 102 and 103, 68 and 64, 2048 x 2048 x 8192 53 and 52.
       const bool rows_in = m0 + quad * 32 < (kMode == kModeGroup ? owners_rows(owners, place.pi) : p.M);
       auto emit = [&](const uint32_t* v32, const CUtensorMap* map, int col0, int row0, bool add = false) {
         uint8_t* slab = (last ? smem + last_boxes * kStagingBytes : staging + (box_ctr & 1u) * kStagingBytes) + quad * 4096;
@@ -1228,6 +1230,8 @@ static SplitPlan plan_splits(int M, int N, int K, int sm_count, const SplitCost&
 // 5.1, 1000 x 1536 x 1536 11.9 and 8.0, 512 x 4096 x 4096 24.3 and 15.1; three rounds instead of two: 1500 x 4096 x 4096 45.0 and
 // 38.4, 4000 x 1536 x 1536 20.0 and 17.9; two instead of one 1900 x 2048 x 2048 15.5 and 15.8, six instead of three 6000 x 2048 x
 // 2048 36.4 and 40.0.  Weight gradients, whose two operands take three loads a k-block, 0.75: 3000 x 2048 x 2048 26.1 and 30.0.
+// The logits have many rounds of tiles at any number of tokens; the SwiGLU backward, scattered weight gradients and gathered weights
+// were not tried in half tiles and keep whole ones.
 static double half_tile_time(int layout) { return layout == 2 ? 0.75 : 0.6; }
 static bool half_tiles_pay(int tiles, int half_tiles, int layout, int sm_count) {
   const int pairs = sm_count / 2;
@@ -1372,6 +1376,8 @@ cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* 
   return cudaGetLastError();
 }
 
+// The kernel is at the limit of 255 registers and spills 60 bytes of stores and 100 of loads a thread; what these cost was not measured
+// apart (with the angles of all heads of a tile in registers it was 340 bytes and a tenth of its time, 10.4 -> 11.5 us).
 // out[M, N] = x w^T (+ bias), w [N, K], with the columns below rot_cols, heads of 64 or 128, rotated by pos[row] (rotary base theta;
 // halves of a head are the pairs, as in launch_rope_qkv): the rotation is not a pass over the projection (16321 tokens, 32 + 16
 // heads of 64: 45 us), and runs while the next tile is multiplied.  The same bytes as the two passes: rounded, rotated, rounded.
@@ -1659,8 +1665,8 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
   // weight gradients, rounds of items): MLP of 4096 and 14336, 256 tokens (4, 36) 164 and 167, 768 (12, 36) 333 and 325; of 5120
   // and 13824, 64 (1, 44) 161 and 171, 1000 (16, 44) 493 and 494, 2000 (32, 44) 925 and 971; of 2048 and 8192, 64 (1, 10) 57 and 53;
   // head of 128256 words, 2048 wide, 256 (4, 54) 253 and 271, 1500 (24, 54) 1070 and 1133, of 32000, 4096 wide, 400 (7, 27) 198 and
-  // 202, 768 (12, 27) 296 and 288.  fp32 gradients gain at all of them (first head 547 and 458): their additions to memory run
-  // under the other items.
+  // 202, 768 (12, 27) 296 and 288.  (All with long sums whole; with parts of their own the two that gained are level, 323 and 325, 285 and
+  // 288.)  fp32 gradients gain at all of them: their additions to memory run under the other items.
   int rounds = 0, shortest = shapes[0].kb;
   for (int i = 0; i < n; ++i) {
     rounds += shapes[i].tiles;
