@@ -145,7 +145,8 @@ struct GroupProblem {
   const float* scale_ptr;
   const float* addend;      // bf16 results: fp32 [M, N] that joins the sum before it is rounded, or null
   int first;                // its first item
-  int whole, splits, kb_split;   // the first `whole` tiles are items, every other tile is `splits` of kb_split k-blocks each
+  // the first `whole` tiles are items, each of the `divided` others is `splits` of kb_split k-blocks each
+  int whole, divided, splits, kb_split;
   int first_split_tile, first_part;   // bf16 with divided tiles: of the first of them, among the divided tiles and parts of the launch
 };
 struct Group {
@@ -356,8 +357,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       while (w.pi + 1 < owners.count && item >= owners.prob[w.pi + 1].first) ++w.pi;
       const GroupProblem& q = owners.prob[w.pi];
       const int local = item - q.first, beyond = local - q.whole;
-      w.divided = beyond < 0 ? -1 : beyond / q.splits;
-      w.part = beyond < 0 ? 0 : beyond - w.divided * q.splits;
+      // the first parts of all tiles, then the second ones: what runs at the same time reads the same k-blocks of A and B
+      w.part = beyond < 0 ? 0 : beyond / q.divided;
+      w.divided = beyond < 0 ? -1 : beyond - w.part * q.divided;
       tile_coords(beyond < 0 ? local : q.whole + w.divided, q, 0, 0, &w.tm, &w.tn);
       w.kb0 = w.part * q.kb_split;
       w.kb1 = (q.K + BK - 1) / BK;
@@ -1747,7 +1749,7 @@ cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int
     t.out = q.c_kind == kBF16 ? 0 : q.accumulate ? 2 : 1;
     t.scale = q.scale; t.scale_ptr = q.scale_ptr; t.addend = q.addend;
     t.first = group.items;
-    t.whole = shape.plan.whole; t.splits = shape.plan.splits; t.kb_split = shape.plan.kb_split;
+    t.whole = shape.plan.whole; t.divided = shape.divided(); t.splits = shape.plan.splits; t.kb_split = shape.plan.kb_split;
     if (shape.bf16) {
       t.first_split_tile = divided; t.first_part = parts;
       divided += shape.divided(); parts += shape.parts();
