@@ -211,13 +211,13 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
     producing rank's fp32 buffer instead of to autograd."""
 
     @staticmethod
-    def forward(ctx, h, labels, loss_scale, model, ignore_index, chunk):
+    def forward(ctx, h, labels, loss_scale, model, ignore_index, chunk, held):
         p = model.head_param()
         w = model.head_full()[:p.out_features]
         ctx.model, ctx.kept = model, h.is_cuda and bool(p.matrix()) and ops._ext().head_keeps_logit_grads(h, w, chunk)
         if ctx.kept:   # the gradient of the logits; the products with it are left to the backward, which knows the loss gradient
             loss, dlogits = ops._ext().loss_and_logit_grads(h, w, labels, loss_scale, ignore_index)
-            ctx.save_for_backward(h.clone(), dlogits)   # a copy: whoever holds h may write to it, as with several chunks
+            ctx.save_for_backward(h.clone() if held else h, dlogits)   # whoever holds h may write to it, as with several chunks
             return loss
         if h.is_cuda:
             # room for the owners' padding rows, so that the whole buffer can be pushed as it is
@@ -263,7 +263,7 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         if ctx.kept:
-            return _FusedLinearCrossEntropy._backward_kept(ctx, dloss), None, None, None, None, None
+            return _FusedLinearCrossEntropy._backward_kept(ctx, dloss), None, None, None, None, None, None
         dh, dw32 = ctx.saved_tensors
         model = ctx.model
         p = model.head_param()
@@ -271,14 +271,14 @@ class _FusedLinearCrossEntropy(torch.autograd.Function):
         gh = ops._ext().scale_to_bf16(dh, dloss) if dh.is_cuda and dh.dtype == torch.bfloat16 else dh * dloss.to(dh.dtype)
         if _direct(p):
             p.push_direct(dw32, dloss)
-            return gh, None, None, None, None, None
+            return gh, None, None, None, None, None, None
         p.wait_push()
         buf = p.local_buffer()
         buf[:p.out_features].addcmul_(dw32[:p.out_features], dloss.to(dw32.dtype))
         p.local_dirty = True
         if p is not model.embed and L.requires_gradient_sync():
             p.push_local(side_stream=True)   # a tied matrix is pushed by the lookup's backward, which runs last
-        return gh, None, None, None, None, None
+        return gh, None, None, None, None, None, None
 
 
 class _FusedTokenLogProbs(torch.autograd.Function):
@@ -482,8 +482,10 @@ class FusedDecoderLM(nn.Module):
                                              self.cfg.ce_chunk)
         if loss_scale is not None and loss_scale.dtype != torch.float32:
             loss_scale = loss_scale.float()
+        # the states of this class's own method are in nobody's hands but autograd's
+        held = "hidden_states" in self.__dict__ or type(self).hidden_states is not _own_hidden_states
         return _FusedLinearCrossEntropy.apply(h.contiguous(), labels.contiguous(), loss_scale, self, -100,
-                                              self.cfg.ce_chunk)
+                                              self.cfg.ce_chunk, held)
 
     @torch.no_grad()
     def logits(self, input_ids, position_ids, cu_seqlens, max_seqlen):
@@ -507,6 +509,9 @@ class FusedDecoderLM(nn.Module):
             p.load_full(sd[name].to(p.master.device, torch.float32))
         self.small.load_flat(self.small.master, {n: sd[n].to(self.device, torch.float32) for n in self.small.slots})
         self.small.lowp.copy_(self.small.master)
+
+
+_own_hidden_states = FusedDecoderLM.hidden_states
 
 
 class FusedOptimizer:

@@ -227,8 +227,9 @@ def test_every_accumulator_matches_the_plain_decoder(tied, bias, sync):
             assert _rel(got[name], p.grad) < CHAIN, name
 
 
+@pytest.mark.parametrize("subclass", [False, True])
 @pytest.mark.parametrize("chunk,kept", [(4096, True), (300, False)])
-def test_hidden_states_may_be_written_to_after_the_loss(chunk, kept):
+def test_hidden_states_may_be_written_to_after_the_loss(chunk, kept, subclass):
     """One chunk, whose products wait for the backward, and several: what the loss needs of the hidden states is its own."""
     from odc_b200 import ops
     with _Engine() as e:
@@ -236,7 +237,11 @@ def test_hidden_states_may_be_written_to_after_the_loss(chunk, kept):
         mbs = _batches(e.cfg, n=1, lo=64, hi=128)   # one key tile per sequence: no sums in a free order
         states, calls = [], []
         plain, loss = e.model.hidden_states, ops._ext().loss_and_logit_grads
-        e.model.hidden_states = lambda *a: states.append(plain(*a)) or states[-1]
+        holds = lambda *a: states.append(plain(*a)) or states[-1]
+        if subclass:
+            e.model.__class__ = type("Holds", (type(e.model),), {"hidden_states": lambda self, *a: holds(*a)})
+        else:
+            e.model.hidden_states = holds
         want = e.minibatch(mbs)
         whole = type(e.model).forward
 
