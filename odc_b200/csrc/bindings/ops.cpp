@@ -320,16 +320,18 @@ bool group_into(const std::vector<Product>& products, const Tensor& ctr_table = 
   const Tensor& a = products[0].a;
   c10::cuda::CUDAGuard guard(a.device());
   odc::bind_device(a.get_device());
+  const odc::GemmGroupPlan plan = odc::gemm_group_plan(g, n, sm_count());
+  if (!plan.taken) return false;
   Tensor scratch;
-  if (const size_t bytes = odc::gemm_group_scratch(g, n, sm_count()))
-    scratch = at::empty({static_cast<int64_t>(bytes / sizeof(float))}, a.options().dtype(at::kFloat));
+  if (plan.scratch_bytes > 0)
+    scratch = at::empty({static_cast<int64_t>(plan.scratch_bytes / sizeof(float))}, a.options().dtype(at::kFloat));
   unsigned int* words = group_words();
   Tensor own;
   if (words == nullptr) {   // a graph's are cleared at each replay
     own = at::zeros({odc::kGroupLaunchWords}, a.options().dtype(at::kInt));
     words = reinterpret_cast<unsigned int*>(own.data_ptr<int>());
   }
-  const cudaError_t e = odc::gemm_group(g, n, scratch.defined() ? scratch.data_ptr<float>() : nullptr, words,
+  const cudaError_t e = odc::gemm_group(g, n, plan, scratch.defined() ? scratch.data_ptr<float>() : nullptr, words,
                                         ctr_table.defined() ? reinterpret_cast<const long long*>(ctr_table.data_ptr<int64_t>()) : nullptr,
                                         arrivals, device_status(a.get_device()).data_ptr<int>(), sm_count(), cur_stream());
   if (e == cudaErrorNotSupported) return false;

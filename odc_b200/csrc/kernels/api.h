@@ -136,7 +136,7 @@ cudaError_t gemm_bf16_pair(const void* a, const void* b, void* c, int c_kind, co
 // Up to three products of one layout each, none of which reads what another writes, as one launch on CTA pairs.  C is bf16 or fp32,
 // times scale and, unless scale_ptr is null, the value there; an fp32 result is added to C if accumulate, and to a bf16
 // one an fp32 matrix may be added.  ctr_ptrs: device table whose first entry is an arrival counter that receives
-// `arrivals` once everything is in memory (0: none).  scratch: gemm_group_scratch() bytes.  words: kGroupLaunchWords zeros that are
+// `arrivals` once everything is in memory (0: none).  scratch: the plan's scratch_bytes.  words: kGroupLaunchWords zeros that are
 // this launch's alone while it runs, left zero by it unless a wait runs out: gemm_group_words() of its stream (null: no more of
 // them), but not for a captured launch, which may run on another stream.  gemm_group_new_words(): a launch on this device has given up.
 // cudaErrorNotSupported: one by one.
@@ -154,17 +154,20 @@ struct GemmProduct {
   const float* addend;   // bf16 C: fp32 [M, N], joins the sum before scale and rounding
 };
 struct GemmGroupPlan {
+  bool taken;
   int parts[kMaxGroupProducts];     // of every tile (1 where some are whole); 0: not taken as a group
   int columns[kMaxGroupProducts];   // of a tile
   GemmPlan tiles[kMaxGroupProducts];
+  int kb_split[kMaxGroupProducts];  // k-blocks of a part
+  int order[kMaxGroupProducts];     // longest items first
+  size_t scratch_bytes;
 };
 GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count);
 bool gemm_group_takes(const GemmProduct* g, int n, int sm_count);   // what gemm_group answers with cudaErrorNotSupported is false
 unsigned int* gemm_group_words(cudaStream_t stream);
 void gemm_group_new_words();
-size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count);
-cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,
-                       int* status, int sm_count, cudaStream_t stream);
+cudaError_t gemm_group(const GemmProduct* g, int n, const GemmGroupPlan& plan, float* scratch, unsigned int* words,
+                       const long long* ctr_ptrs, int arrivals, int* status, int sm_count, cudaStream_t stream);
 
 // act[M, F] = silu(x Wg^T) * (x Wu^T), w = [Wg; Wu]; gate_up [M, 2F] optional.  cudaErrorNotSupported: use the plain product.
 cudaError_t gemm_swiglu_pair(const void* x, const void* w, void* gate_up, void* act, int M, int F, int K, long long ldx,

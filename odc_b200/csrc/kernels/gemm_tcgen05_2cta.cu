@@ -1639,17 +1639,10 @@ static void plan_group(GroupShape* g, int n, int pairs) {
   }
 }
 
-static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* shapes) {
+// What is taken together, by types and sizes.
+static bool group_admits(const GemmProduct* g, int n, int sm_count) {
   using namespace gemm_pair;
   if (n < 1 || n > kMaxGroup || sm_count < 2) return false;
-  for (int i = 0; i < n; ++i) {
-    const GemmProduct& q = g[i];
-    if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate)) || (q.addend != nullptr && q.c_kind != kBF16)) return false;
-    const int tiles = (q.M + 255) / 256 * ((q.N + BN - 1) / BN);
-    shapes[i] = GroupShape{tiles, (q.K + BK - 1) / BK, group_split(q, tiles, sm_count), q.c_kind == kBF16,
-                           !q.whole && q.K <= kGroupShortSum && (q.c_kind == kBF16 ? q.addend == nullptr : q.accumulate), BN,
-                           (q.M + 255) / 256 * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
-  }
   // A group saves the launches and last rounds of its products, 30 to 100 units.  With more work than this for a pair that is no
   // gain any more, and pairs that are not in step with one another share less of L2 (16321 tokens, 2048 and 8192 wide, 4400 units:
   // the layer 0.5 % slower together; 5120 and 13824 wide, 32000 units: 7.62 ms one by one, 7.83 together).  fp32 results, 256 KB a
@@ -1657,9 +1650,15 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
   // units a chunk: 20.5 ms with its forward, 20.0 together).
   long long work = 0;
   bool f32 = false;
+  int rounds = 0, shortest = (g[0].K + BK - 1) / BK;
   for (int i = 0; i < n; ++i) {
-    work += static_cast<long long>(shapes[i].tiles) * shapes[i].kb;
-    f32 = f32 || !shapes[i].bf16 || g[i].addend != nullptr;
+    const GemmProduct& q = g[i];
+    if (q.M < 1 || q.N < 256 || q.K < BK || (q.c_kind != kF32 && (q.c_kind != kBF16 || q.accumulate)) || (q.addend != nullptr && q.c_kind != kBF16)) return false;
+    const int tiles = (q.M + 255) / 256 * ((q.N + BN - 1) / BN), kb = (q.K + BK - 1) / BK;
+    work += static_cast<long long>(tiles) * kb;
+    f32 = f32 || q.c_kind == kF32 || q.addend != nullptr;
+    rounds += tiles;
+    shortest = std::min(shortest, kb);
   }
   if (work > (f32 ? 12000ll : 2700ll) * (sm_count / 2)) return false;
   // Handing an item on costs 0.2 to 0.5 us that a product of its own does not pay, and in many rounds of items that is more than the
@@ -1669,41 +1668,39 @@ static bool group_shapes(const GemmProduct* g, int n, int sm_count, GroupShape* 
   // head of 128256 words, 2048 wide, 256 (4, 54) 253 and 271, 1500 (24, 54) 1070 and 1133, of 32000, 4096 wide, 400 (7, 27) 198 and
   // 202, 768 (12, 27) 296 and 288.  (All with long sums whole; with parts of their own the two that gained are level, 323 and 325, 285 and
   // 288.)  fp32 gradients gain at all of them: their additions to memory run under the other items.
-  int rounds = 0, shortest = shapes[0].kb;
-  for (int i = 0; i < n; ++i) {
-    rounds += shapes[i].tiles;
-    shortest = std::min(shortest, shapes[i].kb);
-  }
   rounds /= sm_count / 2;
-  if (n > 1 && !f32 && rounds >= std::min(40, std::max(20, 7 * shortest / 2))) return false;
-  plan_group(shapes, n, sm_count / 2);
-  return true;
-}
-
-size_t gemm_group_scratch(const GemmProduct* g, int n, int sm_count) {
-  GroupShape shapes[kMaxGroupProducts];
-  if (!group_shapes(g, n, sm_count, shapes)) return 0;
-  size_t parts = 0;
-  for (int i = 0; i < n; ++i)
-    if (shapes[i].bf16) parts += static_cast<size_t>(shapes[i].parts());
-  return parts * 256 * gemm_pair::BN * sizeof(float);
+  return n == 1 || f32 || rounds < std::min(40, std::max(20, 7 * shortest / 2));
 }
 
 GemmGroupPlan gemm_group_plan(const GemmProduct* g, int n, int sm_count) {
-  GroupShape shapes[kMaxGroupProducts];
+  using namespace gemm_pair;
   GemmGroupPlan plan{};
-  if (!group_shapes(g, n, sm_count, shapes)) return plan;
+  if (!group_admits(g, n, sm_count)) return plan;
+  plan.taken = true;
+  GroupShape shapes[kMaxGroup];
+  for (int i = 0; i < n; ++i) {
+    const GemmProduct& q = g[i];
+    const int rows = (q.M + 255) / 256, tiles = rows * ((q.N + BN - 1) / BN);
+    shapes[i] = GroupShape{tiles, (q.K + BK - 1) / BK, group_split(q, tiles, sm_count), q.c_kind == kBF16,
+                           !q.whole && q.K <= kGroupShortSum && (q.c_kind == kBF16 ? q.addend == nullptr : q.accumulate), BN,
+                           rows * ((q.N + BN / 2 - 1) / (BN / 2)), q.layout};
+  }
+  plan_group(shapes, n, sm_count / 2);
   for (int i = 0; i < n; ++i) {
     const SplitPlan& split = shapes[i].plan;
+    plan.order[i] = i;
     plan.parts[i] = split.whole > 0 ? 1 : split.splits;
     plan.columns[i] = shapes[i].bn;
     plan.tiles[i] = {shapes[i].tiles, split.whole, split.splits, 0};
+    plan.kb_split[i] = split.kb_split;
+    if (shapes[i].bf16) plan.scratch_bytes += static_cast<size_t>(shapes[i].parts()) * 256 * BN * sizeof(float);
   }
+  std::stable_sort(plan.order, plan.order + n, [&](int x, int y) { return shapes[x].item() > shapes[y].item(); });
   return plan;
 }
 
-static bool group_takes(const GemmProduct* g, int n, int sm_count, GroupShape* shapes) {
-  if (!group_shapes(g, n, sm_count, shapes)) return false;
+// what the tensor maps and the epilogue ask for
+static bool group_aligned(const GemmProduct* g, int n) {
   for (int i = 0; i < n; ++i) {
     const GemmProduct& q = g[i];
     if ((reinterpret_cast<uintptr_t>(q.a) | reinterpret_cast<uintptr_t>(q.b) | reinterpret_cast<uintptr_t>(q.c) |
@@ -1713,48 +1710,42 @@ static bool group_takes(const GemmProduct* g, int n, int sm_count, GroupShape* s
   }
   return true;
 }
-bool gemm_group_takes(const GemmProduct* g, int n, int sm_count) {
-  GroupShape shapes[kMaxGroupProducts];
-  return group_takes(g, n, sm_count, shapes);
-}
+bool gemm_group_takes(const GemmProduct* g, int n, int sm_count) { return group_admits(g, n, sm_count) && group_aligned(g, n); }
 
-cudaError_t gemm_group(const GemmProduct* g, int n, float* scratch, unsigned int* words, const long long* ctr_ptrs, int arrivals,
-                       int* status, int sm_count, cudaStream_t stream) {
+cudaError_t gemm_group(const GemmProduct* g, int n, const GemmGroupPlan& plan, float* scratch, unsigned int* words,
+                       const long long* ctr_ptrs, int arrivals, int* status, int sm_count, cudaStream_t stream) {
   using namespace gemm_pair;
-  GroupShape shapes[kMaxGroup];
-  if (!group_takes(g, n, sm_count, shapes)) return cudaErrorNotSupported;
+  if (!plan.taken || !group_aligned(g, n)) return cudaErrorNotSupported;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
     attr_err = cudaFuncSetAttribute(gemm_bf16_pair_kernel<kModeGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   });
   if (attr_err != cudaSuccess) return attr_err;
-  int order[kMaxGroup];
-  for (int i = 0; i < n; ++i) order[i] = i;
-  std::stable_sort(order, order + n, [&](int x, int y) { return shapes[x].item() > shapes[y].item(); });
   Group group{};
   int divided = 0, parts = 0;
   for (int i = 0; i < n; ++i) {
-    const GemmProduct& q = g[order[i]];
-    const GroupShape& shape = shapes[order[i]];
+    const GemmProduct& q = g[plan.order[i]];
+    const GemmPlan& tiles = plan.tiles[plan.order[i]];
+    const int bn = plan.columns[plan.order[i]];
     const bool a_mn = q.layout == 2, b_mn = q.layout != 0;
     if (!(a_mn ? encode_tile_map_2d(&group.a[i], q.a, q.M, q.K, q.lda * 2, 64, 64) : encode_tile_map_2d(&group.a[i], q.a, q.K, q.M, q.lda * 2, 64, BMH)) ||
-        !(b_mn ? encode_tile_map_2d(&group.b[i], q.b, q.N, q.K, q.ldb * 2, 64, 64) : encode_tile_map_2d(&group.b[i], q.b, q.K, q.N, q.ldb * 2, 64, shape.bn / 2)) ||
+        !(b_mn ? encode_tile_map_2d(&group.b[i], q.b, q.N, q.K, q.ldb * 2, 64, 64) : encode_tile_map_2d(&group.b[i], q.b, q.K, q.N, q.ldb * 2, 64, bn / 2)) ||
         !(q.c_kind == kF32 ? encode_tile_map_2d_f32(&group.c[i], q.c, q.N, q.M, q.ldc * 4, 32, kOutRows) : encode_tile_map_2d(&group.c[i], q.c, q.N, q.M, q.ldc * 2, 64, kOutRows)))
       return cudaErrorInvalidValue;
     GroupProblem& t = group.prob[i];
     t.M = q.M; t.N = q.N; t.K = q.K;
-    t.tiles_m = (q.M + 255) / 256; t.tiles_n = (q.N + shape.bn - 1) / shape.bn;
-    t.a_mn = a_mn; t.b_mn = b_mn; t.bn = shape.bn;
+    t.tiles_m = (q.M + 255) / 256; t.tiles_n = (q.N + bn - 1) / bn;
+    t.a_mn = a_mn; t.b_mn = b_mn; t.bn = bn;
     t.out = q.c_kind == kBF16 ? 0 : q.accumulate ? 2 : 1;
     t.scale = q.scale; t.scale_ptr = q.scale_ptr; t.addend = q.addend;
     t.first = group.items;
-    t.whole = shape.plan.whole; t.divided = shape.divided(); t.splits = shape.plan.splits; t.kb_split = shape.plan.kb_split;
-    if (shape.bf16) {
+    t.whole = tiles.whole; t.divided = tiles.tiles - tiles.whole; t.splits = tiles.parts; t.kb_split = plan.kb_split[plan.order[i]];
+    if (q.c_kind == kBF16) {
       t.first_split_tile = divided; t.first_part = parts;
-      divided += shape.divided(); parts += shape.parts();
+      divided += t.divided; parts += t.divided * t.splits;
     }
-    group.items += shape.plan.whole + shape.parts();
+    group.items += t.whole + t.divided * t.splits;
   }
   group.count = n;
   if (divided > kMaxGroupDivided || (divided > 0 && scratch == nullptr)) return cudaErrorNotSupported;
