@@ -262,6 +262,34 @@ def test_hidden_states_may_be_written_to_after_the_loss(chunk, kept, subclass):
             assert _rel(got[name], want[name]) < 1e-3, name
 
 
+@pytest.mark.parametrize("library", [False, True])
+@pytest.mark.parametrize("add", [False, True])
+def test_head_gradients_for_a_buffer_that_is_pushed_later(monkeypatch, add, library):
+    """What several ranks push, the matrix without the loss gradient, and what is held back, the sum with it; together in one launch,
+    and one by one with library products.  Against 64 bits."""
+    from odc_b200 import ops
+    with _Engine() as e:
+        p = e.model.head_param()
+        w = e.model.head_full()[:p.out_features]
+        torch.manual_seed(0)
+        T, V, H = 300, w.shape[0], w.shape[1]
+        d, h = (0.01 * torch.randn(T, V, device=DEV)).bfloat16(), torch.randn(T, H, device=DEV).bfloat16()
+        g = torch.tensor(1 / 3, device=DEV)
+        local = torch.randn(V, H, device=DEV)
+        start = local.double()
+        matrix = p.matrix()
+        if library:
+            monkeypatch.setenv("ODC_GEMM", "cublas")
+        dh = ops._ext().sharded_head_grads(d, h, w, g, matrix, local, add)
+        want_dh, want = d.double() @ w.double() / 3, d.double().t() @ h.double()
+        term = want / 3 if add else want
+        want = start + term if add else term
+        # one rounding to bf16 (one by one, two), fp32 sums of 300 to 1024 products; a library product is rounded to bf16 whatever it is for
+        assert ((dh.double() - want_dh).abs() <= 2 ** -7 * want_dh.abs() + 1e-5).all()
+        rounded = 2 ** -8 if library else 2 ** -20
+        assert ((local.double() - want).abs() <= rounded * term.abs() + 2 ** -20 * start.abs() + 1e-5).all()
+
+
 class _Counting(torch.nn.Module):
     def __init__(self, inner, calls):
         super().__init__()

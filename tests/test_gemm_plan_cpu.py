@@ -57,7 +57,7 @@ def test_small_weight_gradients_stay_whole_across_ranks():
 @pytest.mark.parametrize("H,F", [(512, 1536), (1536, 8960), (4096, 14336)])
 def test_groups_divide_what_would_outlast_them(T, H, F):
     """No product keeps parts without k-blocks, products that overwrite fp32 stay whole, and only what is longer than the work
-    of a pair is divided; groups of very much work are not formed."""
+    of a pair is divided altogether; groups of very much work are not formed."""
     plan = lambda *g: _ext.load().gemm_group_plan(list(g), SMS)
     for acc in (False, True):
         shapes = [(T, H, 2 * F, False, False), (2 * F, H, T, True, acc), (H, F, T, True, acc)]
