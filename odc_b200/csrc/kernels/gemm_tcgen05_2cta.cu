@@ -1534,7 +1534,11 @@ static GroupSets* group_sets() {
 unsigned int* gemm_group_words(cudaStream_t stream) {
   GroupSets* sets = group_sets();
   unsigned long long id = 0;
-  if (sets == nullptr || cudaStreamGetId(stream, &id) != cudaSuccess) return nullptr;
+  if (sets == nullptr) return nullptr;
+  if (cudaStreamGetId(stream, &id) != cudaSuccess) {
+    (void)cudaGetLastError();   // the launch that follows, with counters of its own, is not to answer for it
+    return nullptr;
+  }
   std::lock_guard<std::mutex> lock(sets->mu);
   if (sets->base == nullptr) {
     void* p = nullptr;
